@@ -173,10 +173,17 @@ typedef struct b200spSpmmShape {
     int32_t kahan;      /* 1 = compensated fp32 accumulation */
     int32_t block_units; /* from b200sp_spmm_analyze_blocks: units of the column-block path, 0 = not in use */
     int32_t long_rows;  /* from b200sp_spmm_analyze_blocks: rows the analysis listed as long */
+    int64_t repack_bytes; /* bytes of the plan buffer beyond b200sp_spmm_plan_bytes that a repacked B may use
+                           * (b200sp_spmm_repack_bytes), 0 = none */
 } b200spSpmmShape;
 
 /* Bytes of workspace for the SpMM analysis + long-row partial sums. */
 size_t b200sp_spmm_plan_bytes(int64_t rows, int64_t nnz, int64_t n);
+
+/* Bytes wanted after the plan for a copy of B in rows the kernels can read with 16-byte loads: 0 when B lies in
+ * such rows already, or when it is read too seldom for a copy to pay.  Without them (shape.repack_bytes smaller) the
+ * product runs a slower kernel that takes any layout.  Only the sizes and the layout of B are read. */
+size_t b200sp_spmm_repack_bytes(const b200spSpmmShape *shape, int val_type);
 
 /* Analysis pass: finds rows too long for one warp, cuts them into segments and writes
  * the segment table into `plan`.  This call synchronises `stream` once to read back

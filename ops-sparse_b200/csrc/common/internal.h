@@ -61,6 +61,7 @@ struct ActivePlan {
     int32_t longRows = 0;   // SpMM only: rows listed as long
     const void *colInd = nullptr;  // SpMM with column blocks: the cut table was made from these column indices
     int32_t valueType = -1;        // ... and for B rows of this element type
+    int64_t repackBytes = 0;       // SpMM only: bytes after the plan that a repacked B may use
     int32_t spmvInfo[B200SP_SPMV_PLAN_INFO_INTS] = {};  // SpMV only: plan_info written by b200sp_spmv_analyze
     uint64_t generation = 0;  // BufferGeneration(buffer) when the analysis was written
 };

@@ -49,6 +49,7 @@ aclsparseStatus_t ValidateSpmm(aclsparseOperation_t opA, aclsparseOperation_t op
 
 struct Analysis {
     int32_t segments = 0, blockUnits = 0, longRows = 0;
+    int64_t repackBytes = 0;
 };
 
 size_t ElemBytes(aclDataType t)
@@ -85,6 +86,30 @@ aclsparseStatus_t Analyse(const aclsparseSpMatDescr *A, int64_t n, void *buffer,
     return ACL_SPARSE_STATUS_SUCCESS;
 }
 
+b200spSpmmShape ShapeOf(const aclsparseSpMatDescr *A, const aclsparseDnMatDescr *B, const aclsparseDnMatDescr *C,
+                        aclsparseOperation_t opB)
+{
+    b200spSpmmShape sh{};
+    sh.m = A->rows;
+    sh.k = A->cols;
+    sh.n = C->cols;
+    sh.nnz = A->nnz;
+    sh.ldb = B->ld;
+    sh.ldc = C->ld;
+    sh.order_b = (B->order == ACL_SPARSE_ORDER_COL) ? 1 : 0;
+    sh.order_c = (C->order == ACL_SPARSE_ORDER_COL) ? 1 : 0;
+    sh.op_b = (opB == ACL_SPARSE_OP_TRANSPOSE) ? 1 : 0;
+    return sh;
+}
+
+// What a buffer analysed for these operands holds after the plan: room for a copy of B in the kernels' layout.
+size_t RepackBytes(const aclsparseSpMatDescr *A, const aclsparseDnMatDescr *B, const aclsparseDnMatDescr *C,
+                   aclsparseOperation_t opB)
+{
+    const b200spSpmmShape sh = ShapeOf(A, B, C, opB);
+    return b200sp_spmm_repack_bytes(&sh, b200sp::KernelTypeOf(A->valueType));
+}
+
 bool PlanMatches(const ActivePlan &p, const void *buffer, const aclsparseSpMatDescr *A, int64_t n)
 {
     return p.kind == PlanKind::kSpmm && p.buffer == buffer && p.rowPtr == A->offsets && p.rows == A->rows &&
@@ -108,7 +133,7 @@ aclsparseStatus_t aclsparseSpMMGetBufferSize(aclsparseHandle_t handle, aclsparse
     if (size == nullptr) return ACL_SPARSE_STATUS_INVALID_VALUE;
     const aclsparseStatus_t st = ValidateSpmm(opA, opB, matA, matB, matC, computeType, alg);
     if (st != ACL_SPARSE_STATUS_SUCCESS) return st;
-    *size = b200sp_spmm_plan_bytes(matA->rows, matA->nnz, matC->cols);
+    *size = b200sp_spmm_plan_bytes(matA->rows, matA->nnz, matC->cols) + RepackBytes(matA, matB, matC, opB);
     return ACL_SPARSE_STATUS_SUCCESS;
 }
 
@@ -147,6 +172,7 @@ aclsparseStatus_t aclsparseSpMMPreprocess(aclsparseHandle_t handle, aclsparseOpe
     p.longRows = found.longRows;
     p.colInd = matA->indices;
     p.valueType = (int32_t)matA->valueType;
+    p.repackBytes = (int64_t)RepackBytes(matA, matB, matC, opB);  // the buffer holds what GetBufferSize said for these operands
     p.generation = b200sp::BufferGeneration(buffer);
     matA->active = p;
     return ACL_SPARSE_STATUS_SUCCESS;
@@ -169,6 +195,7 @@ aclsparseStatus_t aclsparseSpMM(aclsparseHandle_t handle, aclsparseOperation_t o
         found.segments = matA->active.segments;
         found.blockUnits = matA->active.blockUnits;
         found.longRows = matA->active.longRows;
+        found.repackBytes = matA->active.repackBytes;
     } else {
         // Not the active buffer: analyse into it now, as the reference rebuilds its tiling
         // in place (spmm_host.cpp:310-321).  This path synchronises the stream once.
@@ -188,16 +215,8 @@ aclsparseStatus_t aclsparseSpMM(aclsparseHandle_t handle, aclsparseOperation_t o
         if (beta != nullptr) sc.beta_f = *static_cast<const float *>(beta);
     }
 
-    b200spSpmmShape sh{};
-    sh.m = matA->rows;
-    sh.k = matA->cols;
-    sh.n = matC->cols;
-    sh.nnz = matA->nnz;
-    sh.ldb = matB->ld;
-    sh.ldc = matC->ld;
-    sh.order_b = (matB->order == ACL_SPARSE_ORDER_COL) ? 1 : 0;
-    sh.order_c = (matC->order == ACL_SPARSE_ORDER_COL) ? 1 : 0;
-    sh.op_b = (opB == ACL_SPARSE_OP_TRANSPOSE) ? 1 : 0;
+    b200spSpmmShape sh = ShapeOf(matA, matB, matC, opB);
+    sh.repack_bytes = found.repackBytes;
     sh.block_units = found.blockUnits;
     sh.long_rows = found.longRows;
     sh.kahan = (alg == ACL_SPARSE_SPMM_CSR_FP32_HIGH_PRECISION_ALG && matA->valueType == ACL_FLOAT) ? 1 : 0;

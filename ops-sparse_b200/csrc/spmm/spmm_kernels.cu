@@ -18,15 +18,18 @@
 //                                          finishes last: it adds the stored partial rows in
 //                                          segment order, so no CTA ever waits and the sum
 //                                          order is fixed.
-// Layouts other than "B rows contiguous, C row-major, 16-byte aligned", and the int8 path,
-// go through a generic one-thread-per-output kernel that uses the reference's index
-// formulas verbatim in meaning (spmm_kernel.cpp:156-168, 215-219).
+// The kernels want contiguous, 16-byte aligned rows of B.  A B in any other layout (column-major, odd N or
+// ldb) is first repacked into such rows in the caller's buffer (SpmmRepack*Kernel); a C that is column-major
+// or unaligned is written through a shared-memory tile, with the index formulas of the reference
+// (spmm_kernel.cpp:156-168, 215-219).  Products whose buffer was not analysed for the layout, or whose B is hardly
+// reused, go through a generic one-thread-per-output kernel.
 //
 // Numerics follow the golden SpmmCpuFp32 / SpmmCpuInt8 (test/spmm/arch35/spmm_test.cpp:
 // 125-200): inputs widened to fp32 (int32), products accumulated in fp32 (int32),
 // C = alpha*acc + beta*C with C not read when beta == 0; fp16 output is clamped to
 // +-65504 before rounding; int32 output is computed in int64 and saturated.
 #include <cstdint>
+#include <type_traits>
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -45,7 +48,6 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kLongRow = 1024;          // rows longer than this are handled by segment CTAs
 constexpr int kSegNnz = 4096;           // non-zeros per segment
 constexpr int kWarpSegNnz = kSegNnz / kWarps;
-constexpr int kMaxTileCols = 256;       // widest column tile one warp pass covers (32 lanes x 8)
 
 inline size_t AlignUp(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -207,6 +209,38 @@ template <> struct Pack<__nv_bfloat16> {
     }
 };
 
+template <> struct Pack<int8_t> {
+    static constexpr int kElems = 16;
+};
+
+// What a product of ValT operands accumulates in, and the scalars that go with it.
+template <typename ValT> struct Arith {
+    using Acc = float;
+    using Scalars = ScalarsF;
+};
+template <> struct Arith<int8_t> {
+    using Acc = int32_t;
+    using Scalars = ScalarsI;
+};
+
+// alpha * acc + beta * old, rounded (or saturated: int64 epilogue, reference spmm_kernel.cpp:251-266) to OutT.
+template <typename OutT>
+__device__ __forceinline__ OutT Finish(float acc, float alpha, float beta, const OutT *old)
+{
+    float z = __fmul_rn(alpha, acc);
+    if (beta != 0.0f) z = __fadd_rn(z, __fmul_rn(beta, ToF32(*old)));
+    return FromF32<OutT>(z);
+}
+template <typename OutT>
+__device__ __forceinline__ OutT Finish(int32_t acc, int32_t alpha, int32_t beta, const OutT *old)
+{
+    long long wide = (long long)alpha * (long long)acc;
+    if (beta != 0) wide += (long long)beta * (long long)*old;
+    if (wide > 2147483647LL) wide = 2147483647LL;
+    if (wide < -2147483648LL) wide = -2147483648LL;
+    return (OutT)wide;
+}
+
 // ---------------------------------------------------------------- analysis
 
 __global__ void SpmmFindLongRowsKernel(const int32_t *__restrict__ rowPtr, int rows, int32_t *counts,
@@ -366,14 +400,16 @@ struct FastArgs {
     OutT *C;
     int m;
     int n;
+    int nB;               // columns of a row of B as laid out: n, padded to whole 16-byte pieces when repacked
     long long ldb;
-    long long ldc;
-    ScalarsF sc;
+    long long ldc;        // element (r, j) of C lies at r * ldc + j, or (kGenC) at r * cRow + j * cCol
+    long long cRow, cCol;
+    typename Arith<ValT>::Scalars sc;
     int nsegs;
     const LongRow *longRows;
     const SegEntry *segs;
     int32_t *counters;
-    float *partials;      // [partial slot][n]
+    void *partials;       // [partial slot][n] of the accumulator's type
 };
 
 // One accumulation step, in the golden's arithmetic: the product is rounded, then added
@@ -465,6 +501,51 @@ __device__ __forceinline__ void RowDot(const int32_t *__restrict__ colInd, const
     }
 }
 
+// The int8 form: four entries at a time.  A lane holds 16 columns of four rows of B; each 4 x 4 block of bytes is
+// transposed (eight byte permutes) so that one __dp4a adds four products: 12 instructions for 16 products instead
+// of 32 (16 extractions and 16 multiply-adds).  Entries past a row's end carry value 0 and column 0, which adds
+// nothing.  int32 addition wraps the same in any order, so the result is the golden's whatever the grouping.
+template <int kLanes>
+__device__ __forceinline__ void RowDot8(const int32_t *__restrict__ colInd, const int8_t *__restrict__ val,
+                                        const int8_t *__restrict__ Bslice, long long ldb, int s, int e, int trips,
+                                        int32_t (&acc)[16])
+{
+    static_assert(kLanes >= 4, "a lane group holds whole quads of entries");
+    const int li = threadIdx.x & (kLanes - 1);
+    for (int chunk = 0; chunk < trips; ++chunk) {
+        const int p0 = s + chunk * kLanes;
+        const int rem = e - p0;
+        int myCol = 0, quad = 0;
+        if (li < rem) {
+            myCol = __ldcs(colInd + p0 + li);
+            quad = (int)(unsigned char)__ldcs(reinterpret_cast<const signed char *>(val) + p0 + li);
+        }
+        quad |= __shfl_down_sync(0xffffffffu, quad, 1, kLanes) << 8;
+        quad = (quad & 0xffff) | (__shfl_down_sync(0xffffffffu, quad, 2, kLanes) << 16);  // lanes 0, 4, 8, ...: four values
+#pragma unroll
+        for (int q0 = 0; q0 < kLanes; q0 += 4) {
+            if (!__any_sync(0xffffffffu, q0 < rem)) break;
+            uint32_t w[4][4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int c = __shfl_sync(0xffffffffu, myCol, q0 + u, kLanes);
+                const uint4 q = LoadB16(Bslice + (long long)c * ldb);
+                w[u][0] = q.x; w[u][1] = q.y; w[u][2] = q.z; w[u][3] = q.w;
+            }
+            const int v = __shfl_sync(0xffffffffu, quad, q0, kLanes);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t lo01 = __byte_perm(w[0][j], w[1][j], 0x5140), lo23 = __byte_perm(w[2][j], w[3][j], 0x5140);
+                const uint32_t hi01 = __byte_perm(w[0][j], w[1][j], 0x7362), hi23 = __byte_perm(w[2][j], w[3][j], 0x7362);
+                acc[4 * j] = __dp4a((int)__byte_perm(lo01, lo23, 0x5410), v, acc[4 * j]);
+                acc[4 * j + 1] = __dp4a((int)__byte_perm(lo01, lo23, 0x7632), v, acc[4 * j + 1]);
+                acc[4 * j + 2] = __dp4a((int)__byte_perm(hi01, hi23, 0x5410), v, acc[4 * j + 2]);
+                acc[4 * j + 3] = __dp4a((int)__byte_perm(hi01, hi23, 0x7632), v, acc[4 * j + 3]);
+            }
+        }
+    }
+}
+
 #ifndef B200SP_SPMM_C_STREAMED
 #define B200SP_SPMM_C_STREAMED 1
 #endif
@@ -505,53 +586,123 @@ __device__ __forceinline__ void StoreRowSlice(OutT *dst, const float (&acc)[E], 
     }
 }
 
+template <typename OutT>
+__device__ __forceinline__ void StoreRowSlice(OutT *dst, const int32_t (&acc)[16], int32_t alpha, int32_t beta)
+{
+    static_assert(sizeof(OutT) == 4, "int8 products are stored as int32");
+#pragma unroll
+    for (int i = 0; i < 16; i += 4) {
+        alignas(16) int32_t old[4] = {0, 0, 0, 0}, z[4];
+        if (beta != 0) *reinterpret_cast<int4 *>(old) = __ldcs(reinterpret_cast<const int4 *>(dst + i));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) z[k] = Finish<int32_t>(acc[i + k], alpha, beta, old + k);
+        __stcs(reinterpret_cast<int4 *>(dst + i), *reinterpret_cast<const int4 *>(z));
+    }
+}
+
 // kLanes lanes lie side by side on one row of B (16 bytes each); a warp therefore carries
 // 32 / kLanes rows of A at once.  Rows of up to kLongRow entries are summed by their group in
 // CSR order; longer rows belong to the segment CTAs at the front of the grid.
-template <typename ValT, typename OutT, bool kKahan, int kLanes>
+//
+// kGenC: C is column-major or not 16-byte aligned.  A CTA then takes kGenRows rows, parks their sums in a
+// shared-memory tile and writes C along its contiguous direction (of column-major fp16 C, 32 rows are 64 bytes;
+// straight from registers every element would be a 32-byte sector of its own).
+template <typename ValT, int kLanes> struct FastShape {
+    static constexpr int kTileCols = kLanes * Pack<ValT>::kElems;
+    static constexpr int kCtaRows = kWarps * (32 / kLanes);                   // rows of A per pass of the CTA
+    static constexpr int kFit = 8192 / kTileCols < 32 ? 8192 / kTileCols : 32;  // at most 32 KB of tile
+    static constexpr int kGenRows = kCtaRows > kFit ? kCtaRows : kFit;
+};
+
+template <typename ValT, typename OutT, bool kKahan, int kLanes, bool kGenC>
 __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, OutT> a)
 {
+    using Acc = typename Arith<ValT>::Acc;
+    using Shape = FastShape<ValT, kLanes>;
+    constexpr bool kInt8 = std::is_same_v<ValT, int8_t>;
     constexpr int E = Pack<ValT>::kElems;
     constexpr int kRowsPerWarp = 32 / kLanes;
-    constexpr int kTileCols = kLanes * E;
-    __shared__ float sAcc[kWarps][kMaxTileCols];
+    constexpr int kTileCols = Shape::kTileCols;
+    constexpr int kTileStride = kTileCols + 1;
+    constexpr int kSegWords = kWarps * 32 * E;  // the segment CTAs' sums, one slice per warp
+    constexpr int kTileWords = kGenC ? Shape::kGenRows * kTileStride : 0;
+    __shared__ Acc sBuf[kSegWords > kTileWords ? kSegWords : kTileWords];
+    __shared__ unsigned char sSkip[kGenC ? Shape::kGenRows : 1];
     __shared__ int sLast;
 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int li = lane & (kLanes - 1);
-    const float alpha = a.sc.Alpha();
-    const float beta = a.sc.Beta();
+    const auto alpha = a.sc.Alpha();
+    const auto beta = a.sc.Beta();
+    // one element of C at a time, whatever its layout
+    auto storeOne = [&](long long row, int col, Acc v) {
+        OutT *dst = a.C + row * a.cRow + col * a.cCol;
+        *dst = Finish<OutT>(v, alpha, beta, dst);
+    };
 
     if ((int)blockIdx.x >= a.nsegs) {
         // ---- one lane group per row ----
-        const long long row = ((long long)(blockIdx.x - a.nsegs) * kWarps + warp) * kRowsPerWarp + lane / kLanes;
-        int s = 0, e = 0;
-        if (row < a.m) {
-            s = a.rowPtr[row];
-            e = a.rowPtr[row + 1];
-            if (e - s > kLongRow) e = s;  // owned by segment CTAs
-        }
-        int trips = (e - s + kLanes - 1) / kLanes;
+        constexpr int kBlockRows = kGenC ? Shape::kGenRows : Shape::kCtaRows;
+        const long long row0 = (long long)(blockIdx.x - a.nsegs) * kBlockRows;
+        for (int col0 = 0; col0 < (kGenC ? a.n : 1); col0 += kTileCols) {  // kGenC: a tile of columns at a time
+#pragma unroll 1
+            for (int pass = 0; pass < kBlockRows; pass += Shape::kCtaRows) {
+                const int rowIn = pass + warp * kRowsPerWarp + lane / kLanes;
+                const long long row = row0 + rowIn;
+                int s = 0, e = 0;
+                bool skip = row >= a.m;
+                if (row < a.m) {
+                    s = a.rowPtr[row];
+                    e = a.rowPtr[row + 1];
+                    if (e - s > kLongRow) {  // owned by segment CTAs
+                        e = s;
+                        skip = true;
+                    }
+                }
+                int trips = (e - s + kLanes - 1) / kLanes;
 #pragma unroll
-        for (int off = kLanes; off < 32; off <<= 1) {
-            const int other = __shfl_xor_sync(0xffffffffu, trips, off);
-            trips = other > trips ? other : trips;
-        }
-        const bool skip = row >= a.m || (a.rowPtr[row + 1] - a.rowPtr[row] > kLongRow);
-        for (int col0 = 0; col0 < a.n; col0 += kTileCols) {
-            const int col = col0 + li * E;
-            const bool colLive = col < a.n;
-            const bool allLive = col0 + kTileCols <= a.n;
-            float acc[E], comp[E];
+                for (int off = kLanes; off < 32; off <<= 1) {
+                    const int other = __shfl_xor_sync(0xffffffffu, trips, off);
+                    trips = other > trips ? other : trips;
+                }
+                const int colFirst = kGenC ? col0 : 0, colLast = kGenC ? col0 + 1 : a.n;
+                for (int colT = colFirst; colT < colLast; colT += kTileCols) {
+                    const int col = colT + li * E;
+                    const bool colLive = col < a.nB;
+                    const bool allLive = colT + kTileCols <= a.nB;
+                    Acc acc[E], comp[E];
 #pragma unroll
-            for (int i = 0; i < E; ++i) acc[i] = comp[i] = 0.0f;
-            RowDot<ValT, kKahan, kLanes>(a.colInd, a.val, a.B + col, a.ldb, s, e, trips, colLive, allLive, acc, comp);
-            if (kKahan) {
+                    for (int i = 0; i < E; ++i) acc[i] = comp[i] = Acc(0);
+                    if constexpr (kInt8) {
+                        RowDot8<kLanes>(a.colInd, a.val, a.B + (colLive ? col : 0), a.ldb, s, e, trips, acc);
+                    } else {
+                        RowDot<ValT, kKahan, kLanes>(a.colInd, a.val, a.B + col, a.ldb, s, e, trips, colLive, allLive, acc,
+                                                     comp);
+                    }
+                    if (kKahan) {
 #pragma unroll
-                for (int i = 0; i < E; ++i) acc[i] -= comp[i];
+                        for (int i = 0; i < E; ++i) acc[i] -= comp[i];
+                    }
+                    if constexpr (kGenC) {
+#pragma unroll
+                        for (int i = 0; i < E; ++i) sBuf[rowIn * kTileStride + li * E + i] = acc[i];
+                        if (li == 0) sSkip[rowIn] = skip;
+                    } else {
+                        if (!skip && colLive) StoreRowSlice(a.C + row * a.ldc + col, acc, alpha, beta);
+                    }
+                }
             }
-            if (!skip && colLive) StoreRowSlice<OutT, E>(a.C + row * a.ldc + col, acc, alpha, beta);
+            if constexpr (kGenC) {
+                __syncthreads();
+                const bool rowsRun = a.cRow == 1;  // column-major C: consecutive threads on consecutive rows
+                for (int i = threadIdx.x; i < Shape::kGenRows * kTileCols; i += kThreads) {
+                    const int r = rowsRun ? i % Shape::kGenRows : i / kTileCols;
+                    const int c = rowsRun ? i / Shape::kGenRows : i % kTileCols;
+                    if (col0 + c < a.n && !sSkip[r]) storeOne(row0 + r, col0 + c, sBuf[r * kTileStride + c]);
+                }
+                __syncthreads();
+            }
         }
         return;
     }
@@ -569,22 +720,32 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
     if (ws > segEnd) ws = segEnd;
     if (we > segEnd) we = segEnd;
     const int g = lane / kLanes;
-    float *partial = a.partials + (long long)(lr.partBase + seg.seg) * a.n;
+    Acc *partial = static_cast<Acc *>(a.partials) + (long long)(lr.partBase + seg.seg) * a.n;
+    auto storeSlice = [&](int col, const Acc (&v)[E]) {
+        if constexpr (kGenC) {
+#pragma unroll
+            for (int i = 0; i < E; ++i)
+                if (col + i < a.n) storeOne(seg.row, col + i, v[i]);
+        } else {
+            StoreRowSlice(a.C + (long long)seg.row * a.ldc + col, v, alpha, beta);
+        }
+    };
 
     for (int col0 = 0; col0 < a.n; col0 += kTileCols) {
         const int col = col0 + li * E;
-        const bool colLive = col < a.n;
-        const bool allLive = col0 + kTileCols <= a.n;
-        float acc[E], comp[E];
+        const bool colLive = col < a.nB;
+        const bool allLive = col0 + kTileCols <= a.nB;
+        Acc acc[E], comp[E];
 #pragma unroll
-        for (int i = 0; i < E; ++i) acc[i] = comp[i] = 0.0f;
+        for (int i = 0; i < E; ++i) acc[i] = comp[i] = Acc(0);
         // group g walks chunks g, g + kRowsPerWarp, ... of [ws, we)
         const int nChunks = (we - ws + kLanes - 1) / kLanes;
         for (int ch0 = 0; ch0 < nChunks; ch0 += kRowsPerWarp) {  // same trip count in every group
             const int ch = ch0 + g;
             const int cs = ws + ch * kLanes < we ? ws + ch * kLanes : we;
             const int ce = cs + kLanes < we ? cs + kLanes : we;
-            RowDot<ValT, kKahan, kLanes>(a.colInd, a.val, a.B + col, a.ldb, cs, ce, 1, colLive, allLive, acc, comp);
+            if constexpr (kInt8) RowDot8<kLanes>(a.colInd, a.val, a.B + (colLive ? col : 0), a.ldb, cs, ce, 1, acc);
+            else RowDot<ValT, kKahan, kLanes>(a.colInd, a.val, a.B + col, a.ldb, cs, ce, 1, colLive, allLive, acc, comp);
         }
 #pragma unroll
         for (int i = 0; i < E; ++i) {
@@ -594,23 +755,24 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
         }
         if (lane < kLanes) {
 #pragma unroll
-            for (int i = 0; i < E; ++i) sAcc[warp][li * E + i] = acc[i];
+            for (int i = 0; i < E; ++i) sBuf[warp * 32 * E + li * E + i] = acc[i];
         }
         __syncthreads();
         // warp 0 adds the four warps' slices in warp order
         if (warp == 0 && lane < kLanes && colLive) {
-            float tot[E];
+            Acc tot[E];
 #pragma unroll
             for (int i = 0; i < E; ++i) {
-                tot[i] = sAcc[0][li * E + i];
+                tot[i] = sBuf[li * E + i];
 #pragma unroll
-                for (int w = 1; w < kWarps; ++w) tot[i] += sAcc[w][li * E + i];
+                for (int w = 1; w < kWarps; ++w) tot[i] += sBuf[w * 32 * E + li * E + i];
             }
             if (lr.nseg == 1) {
-                StoreRowSlice<OutT, E>(a.C + (long long)seg.row * a.ldc + col, tot, alpha, beta);
+                storeSlice(col, tot);
             } else {
 #pragma unroll
-                for (int i = 0; i < E; ++i) partial[col + i] = tot[i];
+                for (int i = 0; i < E; ++i)
+                    if (!kGenC || col + i < a.n) partial[col + i] = tot[i];
             }
         }
         __syncthreads();
@@ -628,16 +790,17 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
     __syncthreads();
     if (!sLast) return;
     __threadfence();
-    const float *first = a.partials + (long long)lr.partBase * a.n;
+    const Acc *first = static_cast<const Acc *>(a.partials) + (long long)lr.partBase * a.n;
     for (int col = threadIdx.x * E; col < a.n; col += kThreads * E) {
-        float tot[E];
+        Acc tot[E];
 #pragma unroll
-        for (int i = 0; i < E; ++i) tot[i] = 0.0f;
+        for (int i = 0; i < E; ++i) tot[i] = Acc(0);
         for (int sgi = 0; sgi < lr.nseg; ++sgi) {
 #pragma unroll
-            for (int i = 0; i < E; ++i) tot[i] += __ldcg(first + (long long)sgi * a.n + col + i);
+            for (int i = 0; i < E; ++i)
+                if (!kGenC || col + i < a.n) tot[i] += __ldcg(first + (long long)sgi * a.n + col + i);
         }
-        StoreRowSlice<OutT, E>(a.C + (long long)seg.row * a.ldc + col, tot, alpha, beta);
+        storeSlice(col, tot);
     }
 }
 
@@ -1162,6 +1325,56 @@ __global__ void __launch_bounds__(kStreamThreads) SpmmRowStreamKernel(const Stre
     }
 }
 
+// ---------------------------------------------------------------- repacking B
+
+// Copies op(B) (k rows of n elements, any layout) into rows of `vecs` 16-byte pieces, zeros after element n.  One
+// pass over B; worth it when B is read back often enough (see WorthRepacking).
+template <typename ValT>
+__global__ void __launch_bounds__(256) SpmmRepackRowsKernel(const ValT *__restrict__ B, long long ldb, long long k, int n,
+                                                            int vecs, uint4 *__restrict__ out)
+{
+    constexpr int E = 16 / (int)sizeof(ValT);
+    const long long total = k * vecs;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+        const long long r = i / vecs;
+        const int c = (int)(i - r * vecs) * E;
+        alignas(16) ValT v[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e) v[e] = c + e < n ? __ldcs(B + r * ldb + c + e) : ValT(0);
+        out[i] = *reinterpret_cast<const uint4 *>(v);
+    }
+}
+
+// The same from a B whose columns are contiguous (element (r, j) at j * ldb + r), through a tile of 64 rows.
+constexpr int kRepackRows = 64;
+template <typename ValT>
+__global__ void __launch_bounds__(256) SpmmRepackColsKernel(const ValT *__restrict__ B, long long ldb, long long k, int n,
+                                                            int vecs, uint4 *__restrict__ out)
+{
+    constexpr int E = 16 / (int)sizeof(ValT);
+    constexpr int kCols = 64;                            // columns per step
+    constexpr int kVecs = kCols / E;
+    __shared__ ValT tile[kCols][kRepackRows + 2 * 4 / sizeof(ValT)];  // rows two words apart: no bank is hit twice on the way out
+    const long long r0 = (long long)blockIdx.x * kRepackRows;
+    const int rIn = threadIdx.x & (kRepackRows - 1);
+    for (int c0 = 0; c0 < vecs * E; c0 += kCols) {
+#pragma unroll
+        for (int c = threadIdx.x / kRepackRows; c < kCols; c += 256 / kRepackRows)
+            tile[c][rIn] = (c0 + c < n && r0 + rIn < k) ? __ldcs(B + (c0 + c) * ldb + r0 + rIn) : ValT(0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < kRepackRows * kVecs; i += 256) {
+            const int v = i % kVecs, r = i / kVecs;
+            if (r0 + r < k && c0 / E + v < vecs) {
+                alignas(16) ValT w[E];
+#pragma unroll
+                for (int e = 0; e < E; ++e) w[e] = tile[v * E + e][r];
+                out[(r0 + r) * vecs + c0 / E + v] = *reinterpret_cast<const uint4 *>(w);
+            }
+        }
+        __syncthreads();
+    }
+}
+
 // ---------------------------------------------------------------- generic path
 
 struct GenericShape {
@@ -1234,11 +1447,12 @@ __global__ void __launch_bounds__(256) SpmmGenericInt8Kernel(const int32_t *__re
 
 // ---------------------------------------------------------------- host dispatch
 
-ScalarsF MakeF(const b200spScalars *s)
+template <typename S> S MakeScalars(const b200spScalars *s);
+template <> ScalarsF MakeScalars<ScalarsF>(const b200spScalars *s)
 {
     return {s->alpha_f, s->beta_f, static_cast<const float *>(s->alpha_dev), static_cast<const float *>(s->beta_dev)};
 }
-ScalarsI MakeI(const b200spScalars *s)
+template <> ScalarsI MakeScalars<ScalarsI>(const b200spScalars *s)
 {
     return {s->alpha_i, s->beta_i, static_cast<const int32_t *>(s->alpha_dev),
             static_cast<const int32_t *>(s->beta_dev)};
@@ -1273,100 +1487,169 @@ int LaunchRowStream(const StreamArgs<ValT, OutT> &sa, cudaStream_t stream)
     return (int)cudaGetLastError();
 }
 
+// B rows contiguous in memory: (N, row-major) or (T, column-major).
+bool RowsContiguous(int opB, int orderB) { return (opB != 0) == (orderB != 0); }
+
+// Bytes of a repacked B, 0 when its layout is the kernels' own.  From sizes and layout alone, never from the pointer:
+// a caller may size the buffer before B exists (an unaligned B then goes to the generic kernel).
+size_t RepackBytes(const b200spSpmmShape *sh, int valBytes)
+{
+    const int E = 16 / valBytes;
+    if (RowsContiguous(sh->op_b, sh->order_b) && sh->n % E == 0 && sh->ldb % E == 0) return 0;
+    return (size_t)sh->k * (size_t)((sh->n + E - 1) / E) * 16;
+}
+
+// Repacking reads and writes k * n elements; the generic kernel touches nnz * n of them, a sector each when the
+// columns of B are the contiguous ones and otherwise with one load per product instead of one per 16 bytes.  From
+// two entries per row of B on the copy is the cheaper side by far (65,537 x 50,001 with 24 entries a row, fp16,
+// N = 40 in column-major order: generic 257 us, copy + product 22 us).
+bool WorthRepacking(const b200spSpmmShape *sh) { return sh->nnz >= 2 * sh->k; }
+
 template <typename ValT, typename OutT>
-int LaunchFloat(const int32_t *rowPtr, const int32_t *colInd, const void *val, const void *B, void *C,
+int LaunchGeneric(const int32_t *rowPtr, const int32_t *colInd, const void *val, const void *B, void *C,
+                  const b200spSpmmShape *sh, const b200spScalars *s, cudaStream_t stream)
+{
+    GenericShape g{sh->m, sh->n, sh->ldb, sh->ldc, sh->order_b == 0, sh->order_c == 0, sh->op_b, sh->kahan};
+    const long long total = sh->m * sh->n;
+    if (total == 0) return 0;
+    const long long want = (total + 255) / 256;
+    const long long cap = (long long)b200sp_sm_count() * 32;
+    const unsigned grid = (unsigned)(want < cap ? want : cap);
+    const auto sc = MakeScalars<typename Arith<ValT>::Scalars>(s);
+    if constexpr (std::is_same_v<ValT, int8_t>)
+        SpmmGenericInt8Kernel<<<grid, 256, 0, stream>>>(rowPtr, colInd, static_cast<const ValT *>(val),
+                                                        static_cast<const ValT *>(B), static_cast<OutT *>(C), g, sc);
+    else
+        SpmmGenericFloatKernel<ValT, OutT><<<grid, 256, 0, stream>>>(rowPtr, colInd, static_cast<const ValT *>(val),
+                                                                     static_cast<const ValT *>(B),
+                                                                     static_cast<OutT *>(C), g, sc);
+    b200sp_note_launches(1);
+    return (int)cudaGetLastError();
+}
+
+template <typename ValT, typename OutT>
+int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, const void *B, void *C,
                 const b200spSpmmShape *sh, const b200spScalars *s, void *plan, int32_t segments,
                 cudaStream_t stream)
 {
+    constexpr bool kInt8 = std::is_same_v<ValT, int8_t>;
     constexpr int E = Pack<ValT>::kElems;
-    // B rows contiguous in memory: (N, row-major) or (T, column-major).
-    const bool bRowsContig = (sh->op_b == 0 && sh->order_b == 0) || (sh->op_b == 1 && sh->order_b == 1);
-    const bool fast = plan != nullptr && bRowsContig && sh->order_c == 0 && sh->n % E == 0 && sh->ldb % E == 0 &&
-                      sh->ldc % E == 0 && Aligned16(B) && Aligned16(C);
-    if (fast) {
-        const PlanLayout L = LayoutFor(sh->m, sh->nnz, sh->n);
-        char *p = static_cast<char *>(plan);
-        FastArgs<ValT, OutT> a;
-        a.rowPtr = rowPtr;
-        a.colInd = colInd;
-        a.val = static_cast<const ValT *>(val);
-        a.B = static_cast<const ValT *>(B);
-        a.C = static_cast<OutT *>(C);
-        a.m = (int)sh->m;
-        a.n = (int)sh->n;
-        a.ldb = sh->ldb;
-        a.ldc = sh->ldc;
-        a.sc = MakeF(s);
-        a.longRows = reinterpret_cast<const LongRow *>(p + L.offLong);
-        a.segs = reinterpret_cast<const SegEntry *>(p + L.offSegs);
-        a.counters = reinterpret_cast<int32_t *>(p + L.offCounters);
-        a.partials = reinterpret_cast<float *>(p + L.offPartials);
-        int lanes_ = 1;  // lanes side by side on a row of B
-        while (lanes_ < 32 && lanes_ * E < sh->n) lanes_ <<= 1;
-        const long long rowsPerBlock = (long long)kWarps * (32 / lanes_);
-        // B rows of 128 / 256 / 512 bytes: rows of up to kLongRow entries go to the row-stream kernel,
+    const size_t repack = RepackBytes(sh, (int)sizeof(ValT));
+    const bool bReady = repack == 0 ? Aligned16(B) : (sh->repack_bytes >= (int64_t)repack && WorthRepacking(sh));
+    if (plan == nullptr || !bReady)
+        return LaunchGeneric<ValT, OutT>(rowPtr, colInd, val, B, C, sh, s, stream);
+    if (sh->m == 0 || sh->n == 0) return 0;
+    const bool cPlain = sh->order_c == 0 && sh->n % E == 0 && sh->ldc % E == 0 && Aligned16(C);
+    const PlanLayout L = LayoutFor(sh->m, sh->nnz, sh->n);
+    char *p = static_cast<char *>(plan);
+    FastArgs<ValT, OutT> a;
+    a.rowPtr = rowPtr;
+    a.colInd = colInd;
+    a.val = static_cast<const ValT *>(val);
+    a.B = static_cast<const ValT *>(B);
+    a.C = static_cast<OutT *>(C);
+    a.m = (int)sh->m;
+    a.n = (int)sh->n;
+    a.nB = a.n;
+    a.ldb = sh->ldb;
+    a.ldc = sh->ldc;
+    a.cRow = sh->order_c == 0 ? sh->ldc : 1;
+    a.cCol = sh->order_c == 0 ? 1 : sh->ldc;
+    a.sc = MakeScalars<typename Arith<ValT>::Scalars>(s);
+    a.longRows = reinterpret_cast<const LongRow *>(p + L.offLong);
+    a.segs = reinterpret_cast<const SegEntry *>(p + L.offSegs);
+    a.counters = reinterpret_cast<int32_t *>(p + L.offCounters);
+    a.partials = p + L.offPartials;
+    a.nsegs = segments;
+    if (repack > 0) {
+        const int vecs = (int)((sh->n + E - 1) / E);
+        auto *out = reinterpret_cast<uint4 *>(p + L.total);
+        if (RowsContiguous(sh->op_b, sh->order_b)) {
+            const long long want = (sh->k * vecs + 255) / 256;
+            const long long cap = (long long)b200sp_sm_count() * 32;
+            SpmmRepackRowsKernel<ValT><<<(unsigned)(want < cap ? want : cap), 256, 0, stream>>>(a.B, sh->ldb, sh->k, a.n,
+                                                                                              vecs, out);
+        } else {
+            SpmmRepackColsKernel<ValT><<<(unsigned)((sh->k + kRepackRows - 1) / kRepackRows), 256, 0, stream>>>(
+                a.B, sh->ldb, sh->k, a.n, vecs, out);
+        }
+        b200sp_note_launches(1);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return (int)e;
+        a.B = reinterpret_cast<const ValT *>(out);
+        a.ldb = (long long)vecs * E;
+        a.nB = vecs * E;
+    }
+    constexpr int kMinLanes = kInt8 ? 4 : 1;
+    int lanes_ = kMinLanes;  // lanes side by side on a row of B
+    while (lanes_ < 32 && lanes_ * E < sh->n) lanes_ <<= 1;
+    // Grid of SpmmFastKernel: `segs` segment CTAs, then CTAs for all rows when `rowCtas` is set.
+    auto launchFast = [&](int segs, bool rowCtas, cudaStream_t st) {
+        a.nsegs = segs;
+        auto launch = [&]<int kLanes>() {
+            using Shape = FastShape<ValT, kLanes>;
+            const long long rows = cPlain ? Shape::kCtaRows : Shape::kGenRows;
+            const long long grid = segs + (rowCtas ? (sh->m + rows - 1) / rows : 0);
+            if (grid == 0) return;
+            if constexpr (std::is_same_v<ValT, float>) {
+                if (sh->kahan && cPlain) SpmmFastKernel<ValT, OutT, true, kLanes, false><<<(unsigned)grid, kThreads, 0, st>>>(a);
+                else if (sh->kahan) SpmmFastKernel<ValT, OutT, true, kLanes, true><<<(unsigned)grid, kThreads, 0, st>>>(a);
+            }
+            if (!sh->kahan && cPlain) SpmmFastKernel<ValT, OutT, false, kLanes, false><<<(unsigned)grid, kThreads, 0, st>>>(a);
+            else if (!sh->kahan) SpmmFastKernel<ValT, OutT, false, kLanes, true><<<(unsigned)grid, kThreads, 0, st>>>(a);
+            b200sp_note_launches(1);
+        };
+        switch (lanes_) {
+            case 1: if constexpr (kMinLanes <= 1) launch.template operator()<1>(); break;
+            case 2: if constexpr (kMinLanes <= 2) launch.template operator()<2>(); break;
+            case 4: launch.template operator()<4>(); break;
+            case 8: launch.template operator()<8>(); break;
+            case 16: launch.template operator()<16>(); break;
+            default: launch.template operator()<32>(); break;
+        }
+        return cudaGetLastError();
+    };
+    if constexpr (kInt8) {
+        return (int)launchFast(segments, true, stream);
+    } else {
+        if (!cPlain) return (int)launchFast(segments, true, stream);
+        // B rows of 512 / 1024 bytes: rows of up to kLongRow entries go to the row-stream kernel,
         // and SpmmFastKernel is launched for its segment CTAs only.
         const long long rowBytes = sh->n * (long long)sizeof(ValT);
-        const bool stream_ = !sh->kahan && (rowBytes == 512 || rowBytes == 1024) && sh->m > 0 && B200SP_SPMM_USE_STREAM;
+        const bool stream_ = !sh->kahan && (rowBytes == 512 || rowBytes == 1024);
         // Long rows by column blocks of B (found applicable by b200sp_spmm_analyze_blocks) instead of by segments.
         const bool byBlocks = sh->block_units > 0 && sh->long_rows > 0 && !sh->kahan && rowBytes >= kBlockMinRowBytes &&
                               sh->block_units <= L.capBlockSlots;
         if (byBlocks) segments = 0;
-        a.nsegs = segments;
-        BlockArgs ba{};
-        if (byBlocks) {
-            ba.nUnits = sh->block_units;
-            ba.units = reinterpret_cast<const BlockUnit *>(p + L.offUnits);
-            ba.rowSlots = reinterpret_cast<const int2 *>(p + L.offRowSlots);
-            ba.counters = reinterpret_cast<int32_t *>(p + L.offBlockCounters);
-            ba.partials = reinterpret_cast<float *>(p + L.offBlockPartials);
-        }
-        const long long blockUnits = byBlocks ? (long long)ba.nUnits : 0;
-        // With both kernels to run, the segment CTAs (the long rows: few CTAs, each with much work) are forked
-        // onto the side stream first and the row-stream kernel shares the SMs with them.
+        // With both kernels to run, the long rows (few CTAs, each with much work) are forked onto the side stream
+        // first and the other rows' kernel shares the SMs with them.
         b200sp::SideLanes *lanes = nullptr;
-        cudaStream_t segStream = stream;
-#ifndef B200SP_SPMM_FORK_SEGMENTS
-#define B200SP_SPMM_FORK_SEGMENTS 1
-#endif
-        if (B200SP_SPMM_FORK_SEGMENTS && ((stream_ && segments > 0) || byBlocks)) {
+        cudaStream_t longStream = stream;
+        if ((stream_ && segments > 0) || byBlocks) {
             lanes = b200sp::GetSideLanes();
             if (lanes != nullptr) {
                 if (cudaEventRecord(lanes->fork, stream) != cudaSuccess ||
                     cudaStreamWaitEvent(lanes->stream[0], lanes->fork, 0) != cudaSuccess)
                     return (int)cudaGetLastError();
-                segStream = lanes->stream[0];
+                longStream = lanes->stream[0];
             }
-        }
-        auto launchFast = [&](unsigned grid, cudaStream_t st) {
-            auto launch = [&]<int kLanes>() {
-                if (sh->kahan) SpmmFastKernel<ValT, OutT, true, kLanes><<<grid, kThreads, 0, st>>>(a);
-                else SpmmFastKernel<ValT, OutT, false, kLanes><<<grid, kThreads, 0, st>>>(a);
+            if (byBlocks) {
+                BlockArgs ba{};
+                ba.nUnits = sh->block_units;
+                ba.units = reinterpret_cast<const BlockUnit *>(p + L.offUnits);
+                ba.rowSlots = reinterpret_cast<const int2 *>(p + L.offRowSlots);
+                ba.counters = reinterpret_cast<int32_t *>(p + L.offBlockCounters);
+                ba.partials = reinterpret_cast<float *>(p + L.offBlockPartials);
+                const unsigned grid = (unsigned)(((long long)ba.nUnits + kWarps - 1) / kWarps);
+                SpmmLongBlockKernel<ValT, OutT><<<grid, kThreads, 0, longStream>>>(a, ba);
                 b200sp_note_launches(1);
-            };
-            switch (lanes_) {
-                case 1: launch.template operator()<1>(); break;
-                case 2: launch.template operator()<2>(); break;
-                case 4: launch.template operator()<4>(); break;
-                case 8: launch.template operator()<8>(); break;
-                case 16: launch.template operator()<16>(); break;
-                default: launch.template operator()<32>(); break;
+                if (cudaGetLastError() != cudaSuccess) return (int)cudaErrorLaunchFailure;
+            } else if (lanes != nullptr) {
+                if (launchFast(segments, false, longStream) != cudaSuccess) return (int)cudaErrorLaunchFailure;
+                segments = 0;
             }
-        };
-        auto launchBlocks = [&](cudaStream_t st) {
-            const long long want = (blockUnits + kWarps - 1) / kWarps;
-            const long long fixed = B200SP_SPMM_BLOCK_CTAS > 0 ? (long long)b200sp_sm_count() * B200SP_SPMM_BLOCK_CTAS : want;
-            SpmmLongBlockKernel<ValT, OutT><<<(unsigned)(want < fixed ? want : fixed), kThreads, 0, st>>>(a, ba);
-            b200sp_note_launches(1);
-        };
-        if (lanes != nullptr) {
-            if (byBlocks) launchBlocks(segStream);
-            else launchFast((unsigned)segments, segStream);
-            if (cudaGetLastError() != cudaSuccess || cudaEventRecord(lanes->join[0], segStream) != cudaSuccess)
+            if (lanes != nullptr && cudaEventRecord(lanes->join[0], longStream) != cudaSuccess)
                 return (int)cudaErrorLaunchFailure;
-        } else if (byBlocks) {
-            launchBlocks(stream);
-            if (cudaGetLastError() != cudaSuccess) return (int)cudaErrorLaunchFailure;
         }
         if (stream_) {
             StreamArgs<ValT, OutT> sa;
@@ -1376,7 +1659,7 @@ int LaunchFloat(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             sa.B = a.B;
             sa.C = a.C;
             sa.m = a.m;
-            sa.ldb = sh->ldb;
+            sa.ldb = a.ldb;
             sa.ldc = sh->ldc;
             sa.sc = a.sc;
             sa.waitCycles = gHostStreamWaitCycles;
@@ -1388,27 +1671,11 @@ int LaunchFloat(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
         // What is left for SpmmFastKernel on the caller's stream: the segment CTAs unless they were forked (or
         // replaced by the column-block kernel), and the rows of up to kLongRow entries unless the row-stream
         // kernel took them.
-        const long long blocks = (lanes != nullptr ? 0 : (long long)segments) +
-                                 (stream_ ? 0 : (sh->m + rowsPerBlock - 1) / rowsPerBlock);
-        if (lanes != nullptr && !stream_) a.nsegs = 0;  // the forked launch had them; these CTAs are all row CTAs
-        if (blocks > 0) {
-            launchFast((unsigned)blocks, stream);
-            if (cudaGetLastError() != cudaSuccess) return (int)cudaErrorLaunchFailure;
-        }
+        if (launchFast(segments, !stream_, stream) != cudaSuccess) return (int)cudaErrorLaunchFailure;
         if (lanes != nullptr)  // the long rows are already running beside: join them
             return (int)cudaStreamWaitEvent(stream, lanes->join[0], 0);
         return 0;
     }
-    GenericShape g{sh->m, sh->n, sh->ldb, sh->ldc, sh->order_b == 0, sh->order_c == 0, sh->op_b, sh->kahan};
-    const long long total = sh->m * sh->n;
-    if (total == 0) return 0;
-    const long long want = (total + 255) / 256;
-    const long long cap = (long long)b200sp_sm_count() * 32;
-    SpmmGenericFloatKernel<ValT, OutT><<<(unsigned)(want < cap ? want : cap), 256, 0, stream>>>(
-        rowPtr, colInd, static_cast<const ValT *>(val), static_cast<const ValT *>(B), static_cast<OutT *>(C), g,
-        MakeF(s));
-    b200sp_note_launches(1);
-    return (int)cudaGetLastError();
 }
 
 }  // namespace
@@ -1435,6 +1702,12 @@ void b200sp_spmm_stream_wait_test(long long wait_cycles, unsigned extra_tx)
 }
 
 size_t b200sp_spmm_plan_bytes(int64_t rows, int64_t nnz, int64_t n) { return LayoutFor(rows, nnz, n).total; }
+
+size_t b200sp_spmm_repack_bytes(const b200spSpmmShape *shape, int val_type)
+{
+    const int bytes = val_type == B200SP_F32 ? 4 : val_type == B200SP_I8 ? 1 : 2;
+    return WorthRepacking(shape) ? RepackBytes(shape, bytes) : 0;
+}
 
 int b200sp_spmm_analyze(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,
                         size_t plan_bytes, int32_t *segments, void *stream)
@@ -1518,28 +1791,14 @@ int b200sp_spmm_launch(const int32_t *row_ptr, const int32_t *col_ind, const voi
                        void *plan, int32_t segments, void *stream)
 {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (val_type == B200SP_F32 && out_type == B200SP_F32)
-        return LaunchFloat<float, float>(row_ptr, col_ind, val, B, C, shape, scalars, plan, segments, st);
-    if (val_type == B200SP_F16 && out_type == B200SP_F16)
-        return LaunchFloat<__half, __half>(row_ptr, col_ind, val, B, C, shape, scalars, plan, segments, st);
-    if (val_type == B200SP_BF16 && out_type == B200SP_BF16)
-        return LaunchFloat<__nv_bfloat16, __nv_bfloat16>(row_ptr, col_ind, val, B, C, shape, scalars, plan,
-                                                         segments, st);
-    if (val_type == B200SP_BF16 && out_type == B200SP_F32)
-        return LaunchFloat<__nv_bfloat16, float>(row_ptr, col_ind, val, B, C, shape, scalars, plan, segments, st);
-    if (val_type == B200SP_I8 && out_type == B200SP_I32) {
-        GenericShape g{shape->m, shape->n, shape->ldb, shape->ldc, shape->order_b == 0, shape->order_c == 0,
-                       shape->op_b, 0};
-        const long long total = shape->m * shape->n;
-        if (total == 0) return 0;
-        const long long want = (total + 255) / 256;
-        const long long cap = (long long)b200sp_sm_count() * 32;
-        SpmmGenericInt8Kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, st>>>(
-            row_ptr, col_ind, static_cast<const int8_t *>(val), static_cast<const int8_t *>(B),
-            static_cast<int32_t *>(C), g, MakeI(scalars));
-        b200sp_note_launches(1);
-        return (int)cudaGetLastError();
-    }
+    auto go = [&]<typename ValT, typename OutT>() {
+        return LaunchTyped<ValT, OutT>(row_ptr, col_ind, val, B, C, shape, scalars, plan, segments, st);
+    };
+    if (val_type == B200SP_F32 && out_type == B200SP_F32) return go.template operator()<float, float>();
+    if (val_type == B200SP_F16 && out_type == B200SP_F16) return go.template operator()<__half, __half>();
+    if (val_type == B200SP_BF16 && out_type == B200SP_BF16) return go.template operator()<__nv_bfloat16, __nv_bfloat16>();
+    if (val_type == B200SP_BF16 && out_type == B200SP_F32) return go.template operator()<__nv_bfloat16, float>();
+    if (val_type == B200SP_I8 && out_type == B200SP_I32) return go.template operator()<int8_t, int32_t>();
     return (int)cudaErrorInvalidValue;
 }
 
