@@ -170,22 +170,26 @@ __device__ __forceinline__ uint4 LoadB16(const void *p)
 #endif
 }
 
+// The same for lanes with `on` set; the others keep what q held (and request nothing).
+__device__ __forceinline__ void LoadB16If(bool on, const void *p, uint4 &q)
+{
+    if (on) q = LoadB16(p);
+}
+
 // 16 bytes of a B row as fp32 values: 4 floats, or 8 half / bf16.
 template <typename T> struct Pack;
 template <> struct Pack<float> {
     static constexpr int kElems = 4;
-    static __device__ __forceinline__ void Load(const float *p, float (&out)[4])
+    static __device__ __forceinline__ void Convert(const uint4 &q, float (&out)[4])
     {
-        const uint4 q = LoadB16(p);
         out[0] = __uint_as_float(q.x); out[1] = __uint_as_float(q.y);
         out[2] = __uint_as_float(q.z); out[3] = __uint_as_float(q.w);
     }
 };
 template <> struct Pack<__half> {
     static constexpr int kElems = 8;
-    static __device__ __forceinline__ void Load(const __half *p, float (&out)[8])
+    static __device__ __forceinline__ void Convert(const uint4 &q, float (&out)[8])
     {
-        const uint4 q = LoadB16(p);
         const __half2 *h = reinterpret_cast<const __half2 *>(&q);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -197,9 +201,8 @@ template <> struct Pack<__half> {
 };
 template <> struct Pack<__nv_bfloat16> {
     static constexpr int kElems = 8;
-    static __device__ __forceinline__ void Load(const __nv_bfloat16 *p, float (&out)[8])
+    static __device__ __forceinline__ void Convert(const uint4 &q, float (&out)[8])
     {
-        const uint4 q = LoadB16(p);
         const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {  // bf16 -> fp32 is a 16-bit shift
@@ -404,33 +407,54 @@ struct FastArgs {
     long long ldb;
     long long ldc;        // element (r, j) of C lies at r * ldc + j, or (kGenC) at r * cRow + j * cCol
     long long cRow, cCol;
+    unsigned long long negZeros;
     typename Arith<ValT>::Scalars sc;
     int nsegs;
+    int splitRows;        // int8 only: a CTA per row
     const LongRow *longRows;
     const SegEntry *segs;
     int32_t *counters;
     void *partials;       // [partial slot][n] of the accumulator's type
 };
 
-// One accumulation step, in the golden's arithmetic: the product is rounded, then added
-// (no fused multiply-add), so a row summed in CSR order reproduces the golden bit for bit.
-template <bool kKahan>
-__device__ __forceinline__ void Accumulate(float v, float b, float &acc, float &comp)
+// Accumulation in the golden's arithmetic: the product is rounded, then added (no fused multiply-add), so a row
+// summed in CSR order reproduces the golden bit for bit.  Two of a lane's outputs share an instruction (packed fp32
+// of sm_100): 8 instead of 16 per 16-byte piece of a half-precision B row.  The product is an fma with -0, which rounds
+// it and keeps its sign, and the -0 comes from the launch (kNegZeros), out of the assembler's sight: it fuses a
+// packed mul.rn, or an fma with a constant -0, with the addition that follows.
+constexpr unsigned long long kNegZeros = 0x8000000080000000ull;
+__device__ __forceinline__ void MulAdd2(float &a0, float &a1, float b0, float b1, float v,
+                                        unsigned long long negZeros)
 {
-    const float prod = __fmul_rn(v, b);
-    if (kKahan) {  // compensated summation, the reference's high-precision algorithm
-        const float y = __fsub_rn(prod, comp);
-        const float t = __fadd_rn(acc, y);
-        comp = __fsub_rn(__fsub_rn(t, acc), y);
-        acc = t;
-    } else {
-        acc = __fadd_rn(acc, prod);
-    }
+    asm("{\n\t.reg .b64 x, y, z;\n\t"
+        "mov.b64 x, {%2, %3};\n\t"
+        "mov.b64 y, {%4, %4};\n\t"
+        "mov.b64 z, {%0, %1};\n\t"
+        "fma.rn.f32x2 x, x, y, %5;\n\t"
+        "add.rn.f32x2 z, z, x;\n\t"
+        "mov.b64 {%0, %1}, z;\n\t}"
+        : "+f"(a0), "+f"(a1)
+        : "f"(b0), "f"(b1), "f"(v), "l"(negZeros));
+}
+template <int E>
+__device__ __forceinline__ void Accumulate(float v, const float (&b)[E], float (&acc)[E], unsigned long long negZeros)
+{
+#pragma unroll
+    for (int i = 0; i < E; i += 2) MulAdd2(acc[i], acc[i + 1], b[i], b[i + 1], v, negZeros);
+}
+// Compensated summation, the reference's high-precision algorithm.
+__device__ __forceinline__ void AccumulateKahan(float v, float b, float &acc, float &comp)
+{
+    const float y = __fsub_rn(__fmul_rn(v, b), comp);
+    const float t = __fadd_rn(acc, y);
+    comp = __fsub_rn(__fsub_rn(t, acc), y);
+    acc = t;
 }
 
 // Adds sum_{p in [s, e)} val[p] * B[col[p], slice] to acc, p ascending.  The kLanes lanes of a
 // group call it together with the same s, e (groups of one warp may differ); `trips` is the
-// warp-uniform number of kLanes-wide chunks to walk (>= this group's own need).
+// warp-uniform number of kLanes-wide chunks to walk (>= this group's own need).  A lane whose columns lie past the
+// end of the row (colLive false) loads nothing; what it accumulates is never stored.
 #ifndef B200SP_SPMM_BATCH
 #define B200SP_SPMM_BATCH 4
 #endif
@@ -438,7 +462,7 @@ __device__ __forceinline__ void Accumulate(float v, float b, float &acc, float &
 template <typename ValT, bool kKahan, int kLanes>
 __device__ __forceinline__ void RowDot(const int32_t *__restrict__ colInd, const ValT *__restrict__ val,
                                        const ValT *__restrict__ Bslice, long long ldb, int s, int e, int trips,
-                                       bool colLive, bool allColsLive, float (&acc)[Pack<ValT>::kElems],
+                                       bool colLive, bool allColsLive, unsigned long long negZeros, float (&acc)[Pack<ValT>::kElems],
                                        float (&comp)[Pack<ValT>::kElems])
 {
     constexpr int E = Pack<ValT>::kElems;
@@ -453,48 +477,57 @@ __device__ __forceinline__ void RowDot(const int32_t *__restrict__ colInd, const
             myCol = __ldcs(colInd + p0 + li);
             myVal = ToF32(__ldcs(val + p0 + li));
         }
-        // Whole warp on full chunks and live columns: straight-line code without predicates.
+        // Whole warp on full chunks and live columns: straight-line code, no predicate per entry.
         if (allColsLive && __all_sync(0xffffffffu, rem >= kLanes)) {
 #pragma unroll
             for (int q0 = 0; q0 < kLanes; q0 += kBatch) {
-                float b[kBatch][E];
+                uint4 q[kBatch];
                 float v[kBatch];
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u) {
                     const int c = __shfl_sync(0xffffffffu, myCol, q0 + u, kLanes);
                     v[u] = __shfl_sync(0xffffffffu, myVal, q0 + u, kLanes);
-                    Pack<ValT>::Load(Bslice + (long long)c * ldb, b[u]);
+                    q[u] = LoadB16(Bslice + (long long)c * ldb);
                 }
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u) {
+                    float b[E];
+                    Pack<ValT>::Convert(q[u], b);
+                    if constexpr (kKahan) {
 #pragma unroll
-                    for (int i = 0; i < E; ++i) Accumulate<kKahan>(v[u], b[u][i], acc[i], comp[i]);
+                        for (int i = 0; i < E; ++i) AccumulateKahan(v[u], b[i], acc[i], comp[i]);
+                    } else {
+                        Accumulate<E>(v[u], b, acc, negZeros);
+                    }
                 }
             }
             continue;
         }
+        // Entries past the end of this group's row count as 0 * 0: adding +0 to a sum that began at +0 changes no
+        // bit of it.  (The compensated sum is not indifferent to zeros and skips them.)
 #pragma unroll
         for (int q0 = 0; q0 < kLanes; q0 += kBatch) {
-            float b[kBatch][E];
+            if (!__any_sync(0xffffffffu, q0 < rem)) break;
+            uint4 q[kBatch];
             float v[kBatch];
-            bool live[kBatch];
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
                 const int c = __shfl_sync(0xffffffffu, myCol, q0 + u, kLanes);
                 v[u] = __shfl_sync(0xffffffffu, myVal, q0 + u, kLanes);
-                live[u] = colLive && (q0 + u < rem);
-                if (live[u]) {
-                    Pack<ValT>::Load(Bslice + (long long)c * ldb, b[u]);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < E; ++i) b[u][i] = 0.0f;
-                }
+                q[u] = make_uint4(0, 0, 0, 0);
+                LoadB16If(colLive && q0 + u < rem, Bslice + (long long)c * ldb, q[u]);
             }
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
-                if (live[u]) {
+                float b[E];
+                Pack<ValT>::Convert(q[u], b);
+                if constexpr (kKahan) {
+                    if (q0 + u < rem) {
 #pragma unroll
-                    for (int i = 0; i < E; ++i) Accumulate<kKahan>(v[u], b[u][i], acc[i], comp[i]);
+                        for (int i = 0; i < E; ++i) AccumulateKahan(v[u], b[i], acc[i], comp[i]);
+                    }
+                } else {
+                    Accumulate<E>(v[u], b, acc, negZeros);
                 }
             }
         }
@@ -522,25 +555,30 @@ __device__ __forceinline__ void RowDot8(const int32_t *__restrict__ colInd, cons
         }
         quad |= __shfl_down_sync(0xffffffffu, quad, 1, kLanes) << 8;
         quad = (quad & 0xffff) | (__shfl_down_sync(0xffffffffu, quad, 2, kLanes) << 16);  // lanes 0, 4, 8, ...: four values
+        constexpr int kQuads = kLanes >= 8 ? 2 : 1;  // quads of B rows in flight per lane
 #pragma unroll
-        for (int q0 = 0; q0 < kLanes; q0 += 4) {
+        for (int q0 = 0; q0 < kLanes; q0 += 4 * kQuads) {
             if (!__any_sync(0xffffffffu, q0 < rem)) break;
-            uint32_t w[4][4];
+            uint32_t w[4 * kQuads][4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < 4 * kQuads; ++u) {
                 const int c = __shfl_sync(0xffffffffu, myCol, q0 + u, kLanes);
                 const uint4 q = LoadB16(Bslice + (long long)c * ldb);
                 w[u][0] = q.x; w[u][1] = q.y; w[u][2] = q.z; w[u][3] = q.w;
             }
-            const int v = __shfl_sync(0xffffffffu, quad, q0, kLanes);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t lo01 = __byte_perm(w[0][j], w[1][j], 0x5140), lo23 = __byte_perm(w[2][j], w[3][j], 0x5140);
-                const uint32_t hi01 = __byte_perm(w[0][j], w[1][j], 0x7362), hi23 = __byte_perm(w[2][j], w[3][j], 0x7362);
-                acc[4 * j] = __dp4a((int)__byte_perm(lo01, lo23, 0x5410), v, acc[4 * j]);
-                acc[4 * j + 1] = __dp4a((int)__byte_perm(lo01, lo23, 0x7632), v, acc[4 * j + 1]);
-                acc[4 * j + 2] = __dp4a((int)__byte_perm(hi01, hi23, 0x5410), v, acc[4 * j + 2]);
-                acc[4 * j + 3] = __dp4a((int)__byte_perm(hi01, hi23, 0x7632), v, acc[4 * j + 3]);
+            for (int h = 0; h < kQuads; ++h) {
+                const int v = __shfl_sync(0xffffffffu, quad, q0 + 4 * h, kLanes);
+                uint32_t(&x)[4] = w[4 * h], (&y)[4] = w[4 * h + 1], (&z)[4] = w[4 * h + 2], (&t)[4] = w[4 * h + 3];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t lo01 = __byte_perm(x[j], y[j], 0x5140), lo23 = __byte_perm(z[j], t[j], 0x5140);
+                    const uint32_t hi01 = __byte_perm(x[j], y[j], 0x7362), hi23 = __byte_perm(z[j], t[j], 0x7362);
+                    acc[4 * j] = __dp4a((int)__byte_perm(lo01, lo23, 0x5410), v, acc[4 * j]);
+                    acc[4 * j + 1] = __dp4a((int)__byte_perm(lo01, lo23, 0x7632), v, acc[4 * j + 1]);
+                    acc[4 * j + 2] = __dp4a((int)__byte_perm(hi01, hi23, 0x5410), v, acc[4 * j + 2]);
+                    acc[4 * j + 3] = __dp4a((int)__byte_perm(hi01, hi23, 0x7632), v, acc[4 * j + 3]);
+                }
             }
         }
     }
@@ -641,7 +679,8 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
         *dst = Finish<OutT>(v, alpha, beta, dst);
     };
 
-    if ((int)blockIdx.x >= a.nsegs) {
+    const bool splitRow = kInt8 && a.splitRows && (int)blockIdx.x >= a.nsegs;
+    if ((int)blockIdx.x >= a.nsegs && !splitRow) {
         // ---- one lane group per row ----
         constexpr int kBlockRows = kGenC ? Shape::kGenRows : Shape::kCtaRows;
         const long long row0 = (long long)(blockIdx.x - a.nsegs) * kBlockRows;
@@ -677,7 +716,7 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
                     if constexpr (kInt8) {
                         RowDot8<kLanes>(a.colInd, a.val, a.B + (colLive ? col : 0), a.ldb, s, e, trips, acc);
                     } else {
-                        RowDot<ValT, kKahan, kLanes>(a.colInd, a.val, a.B + col, a.ldb, s, e, trips, colLive, allLive, acc,
+                        RowDot<ValT, kKahan, kLanes>(a.colInd, a.val, a.B + col, a.ldb, s, e, trips, colLive, allLive, a.negZeros, acc,
                                                      comp);
                     }
                     if (kKahan) {
@@ -708,15 +747,18 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
     }
 
     // ---- one CTA per long-row segment: the four warps take a quarter each ----
-    const SegEntry seg = a.segs[blockIdx.x];
-    const LongRow lr = a.longRows[seg.longIdx];
+    // (int8 with split rows: every row of up to kLongRow entries is such a segment)
+    const SegEntry seg = splitRow ? SegEntry{(int)blockIdx.x - a.nsegs, 0, 0, 0} : a.segs[blockIdx.x];
+    const LongRow lr = splitRow ? LongRow{seg.row, 0, 1, 0} : a.longRows[seg.longIdx];
     const int rowStart = a.rowPtr[seg.row];
     const int rowEnd = a.rowPtr[seg.row + 1];
+    if (splitRow && rowEnd - rowStart > kLongRow) return;
     const int segStart = rowStart + seg.seg * kSegNnz;
     const int segEnd = segStart + kSegNnz < rowEnd ? segStart + kSegNnz : rowEnd;
     // inside a warp the lane groups take interleaved kLanes-wide chunks of the warp's quarter
-    int ws = segStart + warp * kWarpSegNnz;
-    int we = ws + kWarpSegNnz;
+    const int quarter = splitRow ? ((segEnd - segStart + 4 * kWarps - 1) / (4 * kWarps)) * 4 : kWarpSegNnz;
+    int ws = segStart + warp * quarter;
+    int we = ws + quarter;
     if (ws > segEnd) ws = segEnd;
     if (we > segEnd) we = segEnd;
     const int g = lane / kLanes;
@@ -745,7 +787,8 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
             const int cs = ws + ch * kLanes < we ? ws + ch * kLanes : we;
             const int ce = cs + kLanes < we ? cs + kLanes : we;
             if constexpr (kInt8) RowDot8<kLanes>(a.colInd, a.val, a.B + (colLive ? col : 0), a.ldb, cs, ce, 1, acc);
-            else RowDot<ValT, kKahan, kLanes>(a.colInd, a.val, a.B + col, a.ldb, cs, ce, 1, colLive, allLive, acc, comp);
+            else RowDot<ValT, kKahan, kLanes>(a.colInd, a.val, a.B + col, a.ldb, cs, ce, 1, colLive, allLive, a.negZeros, acc,
+                                                     comp);
         }
 #pragma unroll
         for (int i = 0; i < E; ++i) {
@@ -1155,6 +1198,7 @@ struct StreamArgs {
     long long ldc;
     ScalarsF sc;
     long long waitCycles;   // limit of every wait on a copy barrier, in SM clocks
+    unsigned long long negZeros;
     unsigned extraTx;       // bytes expected on every barrier beyond those copied (0 outside the wait test)
 };
 
@@ -1304,7 +1348,7 @@ __global__ void __launch_bounds__(kStreamThreads) SpmmRowStreamKernel(const Stre
             float b[E];
             WordsToF32<ValT, kWords>::Convert(w, b);
 #pragma unroll
-            for (int i = 0; i < E; ++i) acc[i] = __fadd_rn(acc[i], __fmul_rn(v, b[i]));
+            for (int i = 0; i < E; i += 2) MulAdd2(acc[i], acc[i + 1], b[i], b[i + 1], v, a.negZeros);
             if (meta & 0x100) {  // last entry of its row (warp-uniform)
                 const int l = meta & 0xff;
                 StoreSlice<OutT, E>(cRow0 + (long long)l * a.ldc, acc, old, alpha, beta);
@@ -1407,8 +1451,8 @@ __global__ void __launch_bounds__(256) SpmmGenericFloatKernel(const int32_t *__r
         const int e = rowPtr[r + 1];
         for (int p = rowPtr[r]; p < e; ++p) {
             const float b = ToF32(B[BIndex(g, colInd[p], j)]);
-            if (g.kahan) Accumulate<true>(ToF32(val[p]), b, acc, comp);
-            else Accumulate<false>(ToF32(val[p]), b, acc, comp);
+            if (g.kahan) AccumulateKahan(ToF32(val[p]), b, acc, comp);
+            else acc = __fadd_rn(acc, __fmul_rn(ToF32(val[p]), b));
         }
         if (g.kahan) acc -= comp;
         const long long ci = g.cRowMajor ? r * g.ldc + j : j * g.ldc + r;
@@ -1561,6 +1605,8 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
     a.counters = reinterpret_cast<int32_t *>(p + L.offCounters);
     a.partials = p + L.offPartials;
     a.nsegs = segments;
+    a.splitRows = 0;
+    a.negZeros = kNegZeros;
     if (repack > 0) {
         const int vecs = (int)((sh->n + E - 1) / E);
         auto *out = reinterpret_cast<uint4 *>(p + L.total);
@@ -1588,7 +1634,7 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
         a.nsegs = segs;
         auto launch = [&]<int kLanes>() {
             using Shape = FastShape<ValT, kLanes>;
-            const long long rows = cPlain ? Shape::kCtaRows : Shape::kGenRows;
+            const long long rows = a.splitRows ? 1 : cPlain ? Shape::kCtaRows : Shape::kGenRows;
             const long long grid = segs + (rowCtas ? (sh->m + rows - 1) / rows : 0);
             if (grid == 0) return;
             if constexpr (std::is_same_v<ValT, float>) {
@@ -1610,6 +1656,9 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
         return cudaGetLastError();
     };
     if constexpr (kInt8) {
+        // Integer sums may be regrouped: where a warp per row would not fill the SMs and rows are long enough to be
+        // shared, a CTA takes a row (4096 rows of 410 entries, N = 512: B200SP_SPLIT_NOTE).
+        a.splitRows = cPlain && sh->nnz >= 128 * sh->m && sh->m * lanes_ / 32 < 64ll * b200sp_sm_count();
         return (int)launchFast(segments, true, stream);
     } else {
         if (!cPlain) return (int)launchFast(segments, true, stream);
@@ -1662,6 +1711,7 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             sa.ldb = a.ldb;
             sa.ldc = sh->ldc;
             sa.sc = a.sc;
+            sa.negZeros = kNegZeros;
             sa.waitCycles = gHostStreamWaitCycles;
             sa.extraTx = gHostStreamExtraTx;
             const int rc = rowBytes == 512 ? LaunchRowStream<ValT, OutT, 512>(sa, stream)
