@@ -8,8 +8,7 @@ Preprocess -> compute.  All arithmetic happens inside libops_sparse.so.
 """
 from __future__ import annotations
 
-import ctypes
-from ctypes import byref, c_float, c_int, c_int32, c_size_t, c_void_p
+from ctypes import Structure, addressof, byref, c_float, c_int, c_int32, c_size_t, c_void_p
 
 import torch
 
@@ -36,6 +35,28 @@ def acl_type_of(dtype: torch.dtype) -> int:
 def _ptr(t: torch.Tensor | None) -> c_void_p | None:
     """Device pointer of a tensor as a C void* (None -> NULL)."""
     return None if t is None else c_void_p(t.data_ptr())
+
+
+class _PackedCall(Structure):
+    """b200spPackedCall (include/b200sp_packed.h)."""
+
+    _fields_ = [("handle", c_void_p), ("a", c_void_p), ("x", c_void_p), ("y", c_void_p), ("out", c_void_p),
+                ("buffer", c_void_p), ("opA", c_int), ("opB", c_int), ("alg", c_int)]
+
+
+class _PackedCalls(dict):
+    """Packed argument structs of the products a matrix (or plan) was used in, by the very values they hold: an entry
+    can not go stale, it is found only by a call with the same arguments.  Converting ten arguments costs an
+    interpreter more than launching a small product; with these a repeated call converts three."""
+
+    MOST = 64
+
+    def pack(self, key, **fields) -> tuple:
+        if len(self) >= self.MOST:
+            self.clear()
+        struct = _PackedCall(**fields)
+        self[key] = struct, addressof(struct)
+        return self[key]
 
 
 class Handle:
@@ -73,6 +94,7 @@ class Handle:
 class DnVec:
     def __init__(self, values: torch.Tensor, size: int | None = None):
         self.values = values
+        self.is_i32 = values.dtype == torch.int32
         self._d = c_void_p()
         n = values.numel() if size is None else size
         check(lib().aclsparseCreateDnVec(byref(self._d), n, _ptr(values), acl_type_of(values.dtype)),
@@ -100,6 +122,7 @@ class DnMat:
 
     def __init__(self, values: torch.Tensor, rows: int, cols: int, ld: int, order: str = "row"):
         self.values = values
+        self.is_i32 = values.dtype == torch.int32
         self.rows, self.cols, self.ld, self.order = rows, cols, ld, order
         self._d = c_void_p()
         check(lib().aclsparseCreateDnMat(byref(self._d), rows, cols, ld, _ptr(values), acl_type_of(values.dtype),
@@ -133,6 +156,7 @@ class CsrMatrix:
         """row_ptr is int32, or int64 for the SpMVOp plan API; index_base 1 likewise is SpMVOp only."""
         assert row_ptr.dtype in (torch.int32, torch.int64) and col_ind.dtype == torch.int32
         self.row_ptr, self.col_ind, self.values = row_ptr, col_ind, values
+        self.is_whole = values.dtype in (torch.int32, torch.int8)
         self.rows, self.cols = rows, cols
         self.nnz = col_ind.numel() if nnz is None else nnz
         self._d = c_void_p()
@@ -142,6 +166,7 @@ class CsrMatrix:
                                        acl_type_of(values.dtype)),
               "aclsparseCreateCsr")
         self.buffer: torch.Tensor | None = None  # workspace recorded by preprocess_*()
+        self._calls = _PackedCalls()
 
     @property
     def raw(self) -> c_void_p:
@@ -149,6 +174,7 @@ class CsrMatrix:
 
     def close(self) -> None:
         if self._d:
+            self._calls.clear()
             lib().aclsparseDestroySpMat(self._d)
             self._d = c_void_p()
 
@@ -160,21 +186,27 @@ class CsrMatrix:
 
 
 def _scalars(handle: Handle, alpha, beta, compute_type: int):
-    """Returns (alpha_arg, beta_arg, keepalive) for the C call."""
+    """The scalar arguments of the C call: pointers to host copies that live as long as the arguments do, or the
+    device pointers themselves.  (byref of a fresh object: a cast to c_void_p costs as much as the rest of a call.)"""
     if handle.device_scalars:
-        return _ptr(alpha), _ptr(beta), (alpha, beta)
-    ctype = c_int32 if compute_type == ACL_INT32 else c_float
-    a, b = ctype(alpha), ctype(beta)
-    return ctypes.cast(byref(a), c_void_p), ctypes.cast(byref(b), c_void_p), (a, b)
+        return _ptr(alpha), _ptr(beta)
+    if compute_type == ACL_INT32:
+        return byref(c_int32(alpha)), byref(c_int32(beta))
+    return byref(c_float(alpha)), byref(c_float(beta))
 
 
 def _compute_type(values: torch.Tensor, out: torch.Tensor) -> int:
     return ACL_INT32 if (values.dtype in (torch.int32, torch.int8) and out.dtype == torch.int32) else ACL_FLOAT
 
 
+def _product_type(A: CsrMatrix, out: DnVec | DnMat) -> int:
+    """The same from what the descriptors were created with."""
+    return ACL_INT32 if A.is_whole and out.is_i32 else ACL_FLOAT
+
+
 def spmv_buffer_size(handle: Handle, A: CsrMatrix, x: DnVec, y: DnVec, op: int = ACL_SPARSE_OP_NON_TRANSPOSE) -> int:
     size = c_size_t()
-    ct = _compute_type(A.values, y.values)
+    ct = _product_type(A, y)
     check(lib().aclsparseSpMVGetBufferSize(handle.raw, op, None, A.raw, x.raw, None, y.raw, ct,
                                            ACL_SPARSE_SPMV_ALG_DEFAULT, byref(size)), "aclsparseSpMVGetBufferSize")
     return size.value
@@ -184,7 +216,7 @@ def spmv_preprocess(handle: Handle, A: CsrMatrix, x: DnVec, y: DnVec, op: int = 
     """GetBufferSize + device allocation + Preprocess; the buffer is kept on A.buffer."""
     nbytes = spmv_buffer_size(handle, A, x, y, op)
     A.buffer = torch.empty(nbytes, dtype=torch.uint8, device=A.row_ptr.device)
-    ct = _compute_type(A.values, y.values)
+    ct = _product_type(A, y)
     check(lib().aclsparseSpMVPreprocess(handle.raw, op, None, A.raw, x.raw, None, y.raw, ct,
                                         ACL_SPARSE_SPMV_ALG_DEFAULT, _ptr(A.buffer)), "aclsparseSpMVPreprocess")
     return A.buffer
@@ -193,18 +225,27 @@ def spmv_preprocess(handle: Handle, A: CsrMatrix, x: DnVec, y: DnVec, op: int = 
 def spmv(handle: Handle, A: CsrMatrix, x: DnVec, y: DnVec, alpha=1.0, beta=0.0,
          op: int = ACL_SPARSE_OP_NON_TRANSPOSE, buffer: torch.Tensor | None = None) -> None:
     """y = alpha * op(A) x + beta * y, enqueued on the handle's stream."""
-    ct = _compute_type(A.values, y.values)
-    a, b, keep = _scalars(handle, alpha, beta, ct)
-    buf = _ptr(buffer) if buffer is not None else None
-    check(lib().aclsparseSpMV(handle.raw, op, a, A.raw, x.raw, b, y.raw, ct, ACL_SPARSE_SPMV_ALG_DEFAULT, buf),
-          "aclsparseSpMV")
-    del keep
+    ct = _product_type(A, y)
+    buf = buffer.data_ptr() if buffer is not None else None
+    if ct == ACL_FLOAT and not handle.device_scalars:
+        h, xd, yd = handle._h.value, x._d.value, y._d.value
+        key = (h, xd, yd, buf, op)
+        call = A._calls.get(key) or A._calls.pack(key, handle=h, a=A._d.value, x=xd, out=yd, buffer=buf, opA=op,
+                                                  alg=ACL_SPARSE_SPMV_ALG_DEFAULT)
+        status = lib().b200spPackedSpMV(call[1], alpha, beta)
+        if status:
+            check(status, "aclsparseSpMV")
+        return
+    a, b = _scalars(handle, alpha, beta, ct)
+    status = lib().aclsparseSpMV(handle._h, op, a, A._d, x._d, b, y._d, ct, ACL_SPARSE_SPMV_ALG_DEFAULT, buf)
+    if status:
+        check(status, "aclsparseSpMV")
 
 
 def spmm_buffer_size(handle: Handle, A: CsrMatrix, B: DnMat, C: DnMat, op_b: int = ACL_SPARSE_OP_NON_TRANSPOSE,
                      alg: int = ACL_SPARSE_SPMM_ALG_DEFAULT) -> int:
     size = c_size_t()
-    ct = _compute_type(A.values, C.values)
+    ct = _product_type(A, C)
     check(lib().aclsparseSpMMGetBufferSize(handle.raw, ACL_SPARSE_OP_NON_TRANSPOSE, op_b, None, A.raw, B.raw, None,
                                            C.raw, ct, alg, byref(size)), "aclsparseSpMMGetBufferSize")
     return size.value
@@ -214,7 +255,7 @@ def spmm_preprocess(handle: Handle, A: CsrMatrix, B: DnMat, C: DnMat, op_b: int 
                     alg: int = ACL_SPARSE_SPMM_ALG_DEFAULT):
     nbytes = spmm_buffer_size(handle, A, B, C, op_b, alg)
     A.buffer = torch.empty(nbytes, dtype=torch.uint8, device=A.row_ptr.device)
-    ct = _compute_type(A.values, C.values)
+    ct = _product_type(A, C)
     check(lib().aclsparseSpMMPreprocess(handle.raw, ACL_SPARSE_OP_NON_TRANSPOSE, op_b, None, A.raw, B.raw, None,
                                         C.raw, ct, alg, _ptr(A.buffer)), "aclsparseSpMMPreprocess")
     return A.buffer
@@ -224,14 +265,24 @@ def spmm(handle: Handle, A: CsrMatrix, B: DnMat, C: DnMat, alpha=1.0, beta=0.0,
          op_b: int = ACL_SPARSE_OP_NON_TRANSPOSE, alg: int = ACL_SPARSE_SPMM_ALG_DEFAULT,
          buffer: torch.Tensor | None = None) -> None:
     """C = alpha * A op(B) + beta * C, enqueued on the handle's stream."""
-    ct = _compute_type(A.values, C.values)
-    a, b, keep = _scalars(handle, alpha, beta, ct)
+    ct = _product_type(A, C)
     buf = buffer if buffer is not None else A.buffer
     if buf is None:
         buf = spmm_preprocess(handle, A, B, C, op_b, alg)
-    check(lib().aclsparseSpMM(handle.raw, ACL_SPARSE_OP_NON_TRANSPOSE, op_b, a, A.raw, B.raw, b, C.raw, ct, alg,
-                              _ptr(buf)), "aclsparseSpMM")
-    del keep
+    if ct == ACL_FLOAT and not handle.device_scalars:
+        h, bd, cd, ptr = handle._h.value, B._d.value, C._d.value, buf.data_ptr()
+        key = (h, bd, cd, ptr, op_b, alg)
+        call = A._calls.get(key) or A._calls.pack(key, handle=h, a=A._d.value, x=bd, out=cd, buffer=ptr,
+                                                  opA=ACL_SPARSE_OP_NON_TRANSPOSE, opB=op_b, alg=alg)
+        status = lib().b200spPackedSpMM(call[1], alpha, beta)
+        if status:
+            check(status, "aclsparseSpMM")
+        return
+    a, b = _scalars(handle, alpha, beta, ct)
+    status = lib().aclsparseSpMM(handle._h, ACL_SPARSE_OP_NON_TRANSPOSE, op_b, a, A._d, B._d, b, C._d, ct, alg,
+                                 buf.data_ptr())
+    if status:
+        check(status, "aclsparseSpMM")
 
 
 class SpMVOpPlan:
@@ -251,6 +302,7 @@ class SpMVOpPlan:
         self.buffer = (torch.empty(max(size.value, 1), dtype=torch.uint8, device=A.col_ind.device)
                        if alg == ACL_SPARSE_SPMVOP_ALG2 else None)
         self._descr, self._plan = c_void_p(), c_void_p()
+        self._calls = _PackedCalls()
         check(lib().aclsparseSpMVOp_createDescr(handle.raw, byref(self._descr), ACL_SPARSE_OP_NON_TRANSPOSE, A.raw,
                                                 x.raw, y.raw, z.raw, ACL_FLOAT, alg,
                                                 _ptr(self.buffer) if self.buffer is not None else None),
@@ -259,11 +311,21 @@ class SpMVOpPlan:
               "aclsparseSpMVOp_createPlan")
 
     def run(self, x: DnVec, y: DnVec, z: DnVec, alpha=1.0, beta=0.0) -> None:
-        a, b, keep = _scalars(self.handle, alpha, beta, ACL_FLOAT)
-        check(lib().aclsparseSpMVOp(self.handle.raw, self._plan, a, b, x.raw, y.raw, z.raw), "aclsparseSpMVOp")
-        del keep
+        if not self.handle.device_scalars:
+            h, xd, yd, zd = self.handle._h.value, x._d.value, y._d.value, z._d.value
+            key = (h, xd, yd, zd)
+            call = self._calls.get(key) or self._calls.pack(key, handle=h, a=self._plan.value, x=xd, y=yd, out=zd)
+            status = lib().b200spPackedSpMVOp(call[1], alpha, beta)
+            if status:
+                check(status, "aclsparseSpMVOp")
+            return
+        a, b = _scalars(self.handle, alpha, beta, ACL_FLOAT)
+        status = lib().aclsparseSpMVOp(self.handle._h, self._plan, a, b, x._d, y._d, z._d)
+        if status:
+            check(status, "aclsparseSpMVOp")
 
     def close(self) -> None:
+        self._calls.clear()
         if self._plan:
             lib().aclsparseSpMVOp_destroyPlan(self._plan)
             self._plan = c_void_p()

@@ -24,6 +24,7 @@ LIB_PATH = LIB_DIR / "libops_sparse.so"
 SOURCES = [
     "common/context.cpp",
     "common/descr.cpp",
+    "common/packed.cpp",
     "common/repeat.cpp",
     "common/host_product.cpp",
     "spmv/spmv_host.cpp",

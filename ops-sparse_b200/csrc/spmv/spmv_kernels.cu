@@ -52,6 +52,7 @@
 #include <cuda_runtime.h>
 
 #include "b200sp_kernels.h"
+#include "../common/chained.cuh"
 #include "../common/side_stream.h"
 
 namespace {
@@ -180,6 +181,8 @@ __device__ __forceinline__ CompT GroupSum(CompT v, int lanes)
 __global__ void SpmvTileSearchKernel(const int32_t *__restrict__ rowPtr, int rows, int nnz, int ntiles,
                                      int32_t *__restrict__ tileRow, int32_t *__restrict__ counters)
 {
+    b200sp::WaitForPrevious();
+    b200sp::AllowNext();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t > ntiles) return;
     const long long total = (long long)rows + nnz;
@@ -228,6 +231,8 @@ __global__ void __launch_bounds__(kTileThreads, B200SP_SPMV_MIN_BLOCKS) SpmvTile
     const int lane = tid & 31;
     const int warp = tid >> 5;
     const int t = blockIdx.x;
+    b200sp::WaitForPrevious();
+    b200sp::AllowNext();
     const int i0 = a.tileRow[t];
     const int i1 = a.tileRow[t + 1];
     const long long total = (long long)a.rows + a.nnz;
@@ -948,6 +953,8 @@ __global__ void __launch_bounds__(256) SpmvShortRowsKernel(const int32_t *__rest
                                                             const ValT *__restrict__ x, OutT *__restrict__ y,
                                                             int rows, Scalars<CompT> sc)
 {
+    b200sp::WaitForPrevious();
+    b200sp::AllowNext();
     ShortRowsBody<CompT, ValT, OutT, G>(blockIdx.x, rowPtr, colInd, val, x, y, rows, sc);
 }
 
@@ -963,6 +970,8 @@ __global__ void __launch_bounds__(256) SpmvMediumShortKernel(const int32_t *__re
                                                               const int4 *__restrict__ listM, int nM, int rows,
                                                               Scalars<CompT> sc)
 {
+    b200sp::WaitForPrevious();
+    b200sp::AllowNext();
     const unsigned wpc = blockDim.x >> 5;
     const unsigned mediumBlocks = ((unsigned)nM + wpc - 1u) / wpc;
     if (blockIdx.x < mediumBlocks) MediumRowsBody<CompT, ValT, OutT>(blockIdx.x, colInd, val, x, y, listM, nM, sc);
@@ -992,6 +1001,8 @@ __global__ void __launch_bounds__(256, 6) SpmvAllBinsKernel(const int32_t *__res
                                                              Scalars<CompT> sc)
 {
     __shared__ CompT sWarp[8];
+    b200sp::WaitForPrevious();
+    b200sp::AllowNext();
     unsigned b = blockIdx.x;
     if (b < (unsigned)nL) {  // nL counts segments here
         LongRowBody<CompT, ValT, OutT, kVec, 2>(b, colInd, val, x, y, ls, sc, sWarp);
@@ -1257,19 +1268,17 @@ int LaunchBinned(const int32_t *rowPtr, const int32_t *colInd, const ValT *val, 
     // such products pipelined on three streams with their host copies took 329 us fused against 287 us forked.
     if (nL > 0 && nnz <= (4ll << 20) && !(info[kInfoKind] == kPlanBinnedBlocked && L.xBlocks > 0)) {
         const unsigned blocks = (unsigned)nS + (unsigned)((nM + 7) / 8) + (unsigned)((rows * G + 255) / 256);
+        b200sp_note_launches(1);
         auto launch = [&]<int GG>() {
-            if (vec) SpmvAllBinsKernel<CompT, ValT, OutT, GG, true><<<blocks, 256, 0, stream>>>(
-                rowPtr, colInd, val, x, y, listM, ls, nM, nS, (int)rows, sc);
-            else SpmvAllBinsKernel<CompT, ValT, OutT, GG, false><<<blocks, 256, 0, stream>>>(
-                rowPtr, colInd, val, x, y, listM, ls, nM, nS, (int)rows, sc);
+            return b200sp::LaunchChained(vec ? SpmvAllBinsKernel<CompT, ValT, OutT, GG, true>
+                                             : SpmvAllBinsKernel<CompT, ValT, OutT, GG, false>,
+                                         blocks, 256, 0, stream, rowPtr, colInd, val, x, y, listM, ls, nM, nS, (int)rows, sc);
         };
         switch (G) {
-            case 2: launch.template operator()<2>(); break;
-            case 8: launch.template operator()<8>(); break;
-            default: launch.template operator()<4>(); break;
+            case 2: return (int)launch.template operator()<2>();
+            case 8: return (int)launch.template operator()<8>();
+            default: return (int)launch.template operator()<4>();
         }
-        b200sp_note_launches(1);
-        return (int)cudaGetLastError();
     }
 #endif
     // The kernels write disjoint rows of y.  The long rows go first, to a side stream forked from
@@ -1321,20 +1330,21 @@ int LaunchBinned(const int32_t *rowPtr, const int32_t *colInd, const ValT *val, 
         constexpr int kMsThreads = 128;
         constexpr int kWpc = kMsThreads / 32;
         const unsigned shortBlocks = (unsigned)((rows * G + kMsThreads - 1) / kMsThreads);
-        if (nM > 0) {
-            const unsigned blocks = (unsigned)((nM + kWpc - 1) / kWpc) + shortBlocks;
-            switch (G) {
-                case 2: SpmvMediumShortKernel<CompT, ValT, OutT, 2><<<blocks, kMsThreads, 0, stream>>>(rowPtr, colInd, val, x, y, listM, nM, (int)rows, sc); break;
-                case 8: SpmvMediumShortKernel<CompT, ValT, OutT, 8><<<blocks, kMsThreads, 0, stream>>>(rowPtr, colInd, val, x, y, listM, nM, (int)rows, sc); break;
-                default: SpmvMediumShortKernel<CompT, ValT, OutT, 4><<<blocks, kMsThreads, 0, stream>>>(rowPtr, colInd, val, x, y, listM, nM, (int)rows, sc); break;
-            }
-        } else {
-            switch (G) {
-                case 2: SpmvShortRowsKernel<CompT, ValT, OutT, 2><<<shortBlocks, kMsThreads, 0, stream>>>(rowPtr, colInd, val, x, y, (int)rows, sc); break;
-                case 8: SpmvShortRowsKernel<CompT, ValT, OutT, 8><<<shortBlocks, kMsThreads, 0, stream>>>(rowPtr, colInd, val, x, y, (int)rows, sc); break;
-                default: SpmvShortRowsKernel<CompT, ValT, OutT, 4><<<shortBlocks, kMsThreads, 0, stream>>>(rowPtr, colInd, val, x, y, (int)rows, sc); break;
-            }
+        auto launch = [&]<int GG>() {
+            if (nM > 0)
+                return b200sp::LaunchChained(SpmvMediumShortKernel<CompT, ValT, OutT, GG>,
+                                             (unsigned)((nM + kWpc - 1) / kWpc) + shortBlocks, kMsThreads, 0, stream, rowPtr,
+                                             colInd, val, x, y, listM, nM, (int)rows, sc);
+            return b200sp::LaunchChained(SpmvShortRowsKernel<CompT, ValT, OutT, GG>, shortBlocks, kMsThreads, 0, stream,
+                                         rowPtr, colInd, val, x, y, (int)rows, sc);
+        };
+        cudaError_t rc = cudaSuccess;
+        switch (G) {
+            case 2: rc = launch.template operator()<2>(); break;
+            case 8: rc = launch.template operator()<8>(); break;
+            default: rc = launch.template operator()<4>(); break;
         }
+        if (rc != cudaSuccess) return (int)rc;
         b200sp_note_launches(1);
     }
     cudaError_t e = cudaGetLastError();
@@ -1372,10 +1382,10 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
         a.partTail = reinterpret_cast<CompT *>(p + L.offTail);
         const bool vec = (reinterpret_cast<uintptr_t>(colInd) % 16 == 0) &&
                          (reinterpret_cast<uintptr_t>(val) % (4 * sizeof(ValT)) == 0);
-        if (vec) SpmvTileKernel<CompT, ValT, OutT, true><<<(unsigned)L.ntiles, kTileThreads, 0, stream>>>(a);
-        else SpmvTileKernel<CompT, ValT, OutT, false><<<(unsigned)L.ntiles, kTileThreads, 0, stream>>>(a);
         b200sp_note_launches(1);
-        return (int)cudaGetLastError();
+        return (int)b200sp::LaunchChained(vec ? SpmvTileKernel<CompT, ValT, OutT, true>
+                                              : SpmvTileKernel<CompT, ValT, OutT, false>,
+                                          (unsigned)L.ntiles, kTileThreads, 0, stream, a);
     }
     if (rows == 0) return 0;
     const int G = GroupWidthFor(rows, nnz);
@@ -1499,11 +1509,10 @@ int b200sp_spmv_analyze(const int32_t *row_ptr, const int32_t *col_ind, int64_t 
         const PlanLayout L = LayoutFor(rows, nnz);
         if (L.ntiles == 0) return 0;
         const unsigned blocks = (unsigned)((L.ntiles + 1 + 255) / 256);
-        SpmvTileSearchKernel<<<blocks, 256, 0, st>>>(row_ptr, (int)rows, (int)nnz, (int)L.ntiles,
-                                                     reinterpret_cast<int32_t *>(p + L.offTileRow),
-                                                     reinterpret_cast<int32_t *>(p + L.offCounters));
         b200sp_note_launches(1);
-        return (int)cudaGetLastError();
+        return (int)b200sp::LaunchChained(SpmvTileSearchKernel, blocks, 256, 0, st, row_ptr, (int)rows, (int)nnz,
+                                          (int)L.ntiles, reinterpret_cast<int32_t *>(p + L.offTileRow),
+                                          reinterpret_cast<int32_t *>(p + L.offCounters));
     }
     // Binned plan: list the medium and the long rows, then read the counts back (one sync).
     const BinLayout L = BinLayoutFor(rows, cols, nnz);
