@@ -5,6 +5,7 @@
 // 660-764).  The reference reorders rows greedily over its cores in Preprocess; here the work is cut by
 // non-zeros (a warp per 32 consecutive entries of C, the lanes splitting k), which needs no analysis:
 // BufferSize reports a token 256 bytes (the API wants a buffer), Preprocess only checks its arguments.
+#include <atomic>
 #include <climits>
 #include <cstdint>
 
@@ -12,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include "b200sp_kernels.h"
+#include "common/chained.cuh"
 #include "common/internal.h"
 
 namespace {
@@ -69,111 +71,254 @@ __global__ void __launch_bounds__(256) SddmmKernel(const int32_t *__restrict__ r
     }
 }
 
-// 16 bytes of both operands per lane and step: 4 fp32 or 8 fp16 products.
-__device__ __forceinline__ float Dot16(const uint4 &x, const uint4 &y, float acc, float)
+// The same product when k runs along the contiguous direction of both operands.  An entry of C is the dot product of
+// two short rows, so the work is fetching a row of Y per entry; what counts is how many of them an SM has in flight
+// and how few instructions go into each.
+//   - kLanes lanes lie side by side on a row, kBytes bytes each (the widest the rows' alignment allows) and kSlabs pieces
+//     apart; a warp therefore works on 32 / kLanes entries at a time, and rows wider than 32 * kSlabs pieces take
+//     several turns.
+//   - Rows come through shared memory by cp.async, kStages batches of kBatch entries deep per lane group: no registers
+//     hold data in flight.  A row of X is copied only when it differs from the entry before.
+//   - A warp owns a tile of consecutive entries.  What is done once per entry (row, column, old value, store) is done
+//     for the whole tile with coalesced accesses; lane group g works on the tile's g-th part.
+//   - The kBatch sums of a batch are reduced together: every butterfly step that halves the number of values a lane
+//     carries costs as many shuffles as values are left (6 instead of 20 for four sums over 32 lanes).
+// fp16 rows that start on odd 2-byte addresses (kBytes = 2) are copied as the 4-byte words that cover them and
+// realigned when they are read from shared memory.
+// Measured (1 M nodes, 16.0 M entries, fp16, k = 256): 2091 us with the rows in registers, four entries in flight and a full butterfly per
+// entry; 1384 us here, 8.2 GB of Y rows at 5.9 TB/s.
+template <int kBytes> struct Words { using Type = uint32_t; };  // 4, and the words of kBytes = 2
+template <> struct Words<16> { using Type = uint4; };
+template <> struct Words<8> { using Type = uint2; };
+
+__device__ __forceinline__ float DotWord(uint32_t x, uint32_t y, float acc, float)
 {
-    acc = fmaf(__uint_as_float(x.x), __uint_as_float(y.x), acc);
-    acc = fmaf(__uint_as_float(x.y), __uint_as_float(y.y), acc);
-    acc = fmaf(__uint_as_float(x.z), __uint_as_float(y.z), acc);
-    return fmaf(__uint_as_float(x.w), __uint_as_float(y.w), acc);
+    return fmaf(__uint_as_float(x), __uint_as_float(y), acc);
 }
-__device__ __forceinline__ float Dot16(const uint4 &x, const uint4 &y, float acc, __half)
+__device__ __forceinline__ float DotWord(uint32_t x, uint32_t y, float acc, __half)
 {
-    const __half2 *hx = reinterpret_cast<const __half2 *>(&x);
-    const __half2 *hy = reinterpret_cast<const __half2 *>(&y);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float2 a = __half22float2(hx[i]), b = __half22float2(hy[i]);
-        acc = fmaf(a.x, b.x, acc);
-        acc = fmaf(a.y, b.y, acc);
-    }
-    return acc;
+    const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&x)), b = __half22float2(*reinterpret_cast<const __half2 *>(&y));
+    return fmaf(a.y, b.y, fmaf(a.x, b.x, acc));
+}
+template <typename T> __device__ __forceinline__ float DotPiece(const uint4 &x, const uint4 &y, float acc)
+{
+    acc = DotWord(x.x, y.x, acc, T());
+    acc = DotWord(x.y, y.y, acc, T());
+    acc = DotWord(x.z, y.z, acc, T());
+    return DotWord(x.w, y.w, acc, T());
+}
+template <typename T> __device__ __forceinline__ float DotPiece(const uint2 &x, const uint2 &y, float acc)
+{
+    acc = DotWord(x.x, y.x, acc, T());
+    return DotWord(x.y, y.y, acc, T());
+}
+template <typename T> __device__ __forceinline__ float DotPiece(uint32_t x, uint32_t y, float acc)
+{
+    return DotWord(x, y, acc, T());
 }
 
-// The same product when k runs along the contiguous direction of both operands and rows are 16-byte
-// aligned: 128-bit loads.  The first 16-byte piece of the X row of every lane stays in registers while
-// consecutive entries of C share their row (rows of up to 32 pieces -- 128 fp32 or 256 fp16 -- are then
-// read once per row and chunk).
-constexpr int kSddmmBatch = 4;  // entries of C a warp works on at once
-template <typename T>
-__global__ void __launch_bounds__(256) SddmmVecKernel(const int32_t *__restrict__ rowPtr, const int32_t *__restrict__ colInd,
-                                                      T *__restrict__ cVal, const T *__restrict__ X,
-                                                      const T *__restrict__ Y, int m, int pieces, long long nnz,
-                                                      long long xRow16, long long yRow16, float alpha, float beta,
-                                                      const T *alphaDev, const T *betaDev)
+// kSize bytes from global to shared memory; `bytes` of them are read, the rest is zero.
+template <int kSize> __device__ __forceinline__ void CopyAsync(void *dst, const void *src, int bytes)
 {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if constexpr (kSize == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(kSize), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void CopyCommit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kPending> __device__ __forceinline__ void CopyWait() { asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory"); }
+
+// Row of every lane's entry p (p0 + lane), given a row r0 with rowPtr[r0] <= p0: largest r with rowPtr[r] <= p.
+__device__ __forceinline__ int RowOfLane(const int32_t *__restrict__ rowPtr, int m, int r0, int p, int lane)
+{
+    const int last = 0x7fffffff;
+    const int end = r0 + 1 + lane <= m - 1 ? __ldg(rowPtr + r0 + 1 + lane) : last;  // starts of the 32 rows after r0
+    int n = 0;  // how many of them are <= p: they ascend
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1) {
+        const int at = __shfl_sync(0xffffffffu, end, n + step - 1);
+        if (at <= p) n += step;
+    }
+    const int end31 = __shfl_sync(0xffffffffu, end, 31);
+    if (n == 31 && end31 <= p) n = 32;
+    int r = r0 + n;
+    if (n == 32) {  // more than 32 rows within 32 entries: go on alone
+        int hi = m - 1;
+        while (r < hi) {
+            const int mid = r + ((hi - r + 1) >> 1);
+            if (__ldg(rowPtr + mid) <= p) r = mid;
+            else hi = mid - 1;
+        }
+    }
+    return r;
+}
+
+// 1384 us with 4 warps and tiles of 128, 1286 with 2 and 64 on the same GPU; one warp or longer tiles gain nothing more.
+constexpr int kSddmmWarps = 2;
+constexpr int kSddmmTile = 64;  // entries a warp owns at most
+template <int kBytes, int kLanes, int kSlabs> struct SddmmShape {
+    static constexpr int kBatch = kSlabs >= 4 ? 2 : 4;
+    static constexpr int kStages = 2;
+    static constexpr int kCopy = kBytes == 2 ? 4 : kBytes;
+    static constexpr int kSlotBytes = 32 * kSlabs * kCopy;                       // one entry of every lane group
+    static constexpr int kRing = 2 * kStages * kBatch * kSlotBytes;              // rows of Y, rows of X
+    static constexpr int kWarpBytes = kRing + kSddmmTile * 12;                   // and row, column, sum per entry
+    static constexpr int kCtaBytes = kSddmmWarps * kWarpBytes;
+};
+
+template <typename T, int kBytes, int kLanes, int kSlabs>
+__global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(
+    const int32_t *__restrict__ rowPtr, const int32_t *__restrict__ colInd, T *__restrict__ cVal, const char *__restrict__ X,
+    const char *__restrict__ Y, int m, int k, int nnz, int tile, long long xRowBytes, long long yRowBytes, float alpha,
+    float beta, const T *alphaDev, const T *betaDev)
+{
+    using Shape = SddmmShape<kBytes, kLanes, kSlabs>;
+    using Piece = typename Words<kBytes>::Type;
+    constexpr int kBatch = Shape::kBatch;
+    constexpr int kStages = Shape::kStages;
+    constexpr int kCopy = Shape::kCopy;
+    constexpr bool kOdd = kBytes == 2;
+    static_assert(kLanes >= 4, "the sums of a batch are spread over four lanes");
+    extern __shared__ __align__(16) unsigned char sRaw[];
+    b200sp::WaitForPrevious();
+    b200sp::AllowNext();
     const float a = alphaDev ? Load<T>(alphaDev) : alpha;
     const float b = betaDev ? Load<T>(betaDev) : beta;
     const int lane = threadIdx.x & 31;
-    const uint4 *X16 = reinterpret_cast<const uint4 *>(X);
-    const uint4 *Y16 = reinterpret_cast<const uint4 *>(Y);
-    const long long warpsTotal = (long long)gridDim.x * (blockDim.x >> 5);
-    const long long chunks = (nnz + 31) / 32;
-    for (long long c = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < chunks; c += warpsTotal) {
-        const long long p0 = c * 32;
-        const long long p1 = p0 + 32 < nnz ? p0 + 32 : nnz;
-        // The row of the chunk's first entry (largest r with rowPtr[r] <= p0): the 32 lanes probe 32 places
-        // per round, so a million rows take four dependent loads instead of twenty.
-        int lo = 0, hi = m;
-        while (hi - lo > 1) {
-            const int step = (hi - lo + 31) / 32;
-            const long long idx = (long long)lo + (long long)(lane + 1) * step;
-            const bool ok = idx < hi && (long long)__ldg(rowPtr + idx) <= p0;
-            const int k = __popc(__ballot_sync(0xffffffffu, ok));  // offsets ascend: the lanes that pass are a prefix
-            lo += k * step;
-            hi = hi < lo + step ? hi : lo + step;
-        }
-        int r = lo, cachedRow = -1;
-        uint4 x0 = make_uint4(0, 0, 0, 0);
-        const int myCol = p0 + lane < p1 ? __ldg(colInd + p0 + lane) : 0;  // the chunk's columns, one per lane
-        // Four entries at a time: their Y rows are requested together, so that a warp has four rows in flight
-        // instead of one (the gather of Y rows from DRAM is what this kernel waits for).
-        for (long long p = p0; p < p1; p += kSddmmBatch) {
-            int rows[kSddmmBatch];
-            uint4 y[kSddmmBatch];
+    const int li = lane & (kLanes - 1);
+    const int group = lane / kLanes;
+    const long long p0 = ((long long)blockIdx.x * kSddmmWarps + (threadIdx.x >> 5)) * tile;
+    if (p0 >= nnz) return;
+    unsigned char *sWarp = sRaw + (threadIdx.x >> 5) * Shape::kWarpBytes;
+    Piece *sY = reinterpret_cast<Piece *>(sWarp), *sX = sY + kStages * kBatch * kSlabs * 32;
+    int *sRow = reinterpret_cast<int *>(sWarp + Shape::kRing), *sCol = sRow + kSddmmTile;
+    float *sDot = reinterpret_cast<float *>(sCol + kSddmmTile);
+
+    // The row of the first entry (largest r with rowPtr[r] <= p0): the 32 lanes probe 32 places per round.
+    int r0 = 0;
+    for (int hi = m; hi - r0 > 1;) {
+        const int step = (hi - r0 + 31) / 32;
+        const long long idx = (long long)r0 + (long long)(lane + 1) * step;
+        const bool ok = idx < hi && (long long)__ldg(rowPtr + idx) <= p0;
+        const int n = __popc(__ballot_sync(0xffffffffu, ok));  // offsets ascend: the lanes that pass are a prefix
+        r0 += n * step;
+        hi = hi < r0 + step ? hi : r0 + step;
+    }
+    for (int t = lane; t < tile; t += 32) {
+        const int p = p0 + t < nnz ? (int)p0 + t : nnz - 1;  // past the end: the last entry again, not stored
+        const int r = RowOfLane(rowPtr, m, r0, p, lane);
+        sRow[t] = r;
+        sCol[t] = __ldg(colInd + p);
+        sDot[t] = 0.0f;
+        r0 = __shfl_sync(0xffffffffu, r, 31);
+    }
+    __syncwarp();
+
+    const int pieces = kOdd ? (k + 1) / 2 : k * (int)sizeof(T) / kBytes;
+    const int perGroup = tile / (32 / kLanes);
+    const int t0 = group * perGroup;
+    const int batches = perGroup / kBatch;
+    for (int piece0 = 0; piece0 < pieces; piece0 += kLanes * kSlabs - (kOdd ? 1 : 0)) {
+        const int width = kLanes * kSlabs - (kOdd ? 1 : 0);
+        auto copyRow = [&](Piece *slot, const char *row) {
 #pragma unroll
-            for (int u = 0; u < kSddmmBatch; ++u) {
-                const bool live = p + u < p1;
-                if (live) {
-                    while ((long long)__ldg(rowPtr + r + 1) <= p + u) ++r;
+            for (int s = 0; s < kSlabs; ++s) {
+                const int q = piece0 + s * kLanes + li;
+                if constexpr (kOdd) {  // words from the one that holds the first element on, zeros after the row's last
+                    const int off = (int)(reinterpret_cast<uintptr_t>(row) & 2);
+                    const int left = 2 * k + off - 4 * q;
+                    const int bytes = left >= 4 ? 4 : left > 0 ? left : 0;
+                    CopyAsync<4>(slot + s * 32 + lane, row - off + (bytes > 0 ? 4 * q : 0), bytes);
+                } else {
+                    const bool in = q < pieces;
+                    CopyAsync<kCopy>(slot + s * 32 + lane, row + (in ? (long long)q * kBytes : 0), in ? kCopy : 0);
                 }
-                rows[u] = r;
-                const int j = __shfl_sync(0xffffffffu, myCol, (int)(p + u - p0) & 31);
-                y[u] = make_uint4(0, 0, 0, 0);
-                if (live && lane < pieces) y[u] = __ldg(Y16 + (long long)j * yRow16 + lane);
             }
-            float acc[kSddmmBatch];
+        };
+        auto request = [&](int batch) {
+            if (batch < batches) {
+                const int stage = batch % kStages;
+                int before = batch > 0 ? sRow[t0 + batch * kBatch - 1] : -1;
 #pragma unroll
-            for (int u = 0; u < kSddmmBatch; ++u) {
+                for (int u = 0; u < kBatch; ++u) {
+                    const int t = t0 + batch * kBatch + u;
+                    const int row = sRow[t];
+                    copyRow(sY + (stage * kBatch + u) * kSlabs * 32, Y + sCol[t] * yRowBytes);
+                    if (row != before) copyRow(sX + (stage * kBatch + u) * kSlabs * 32, X + row * xRowBytes);
+                    before = row;
+                }
+            }
+            CopyCommit();
+        };
+        // A lane's pieces of a row: its own words, or (kOdd) the elements 2 q and 2 q + 1 wherever they lie.
+        auto read = [&](const Piece *slot, const char *row, int s) -> Piece {
+            if constexpr (kOdd) {
+                const int i = s * kLanes + li;  // word of the turn; the last one only completes its neighbour
+                const int next = i + 1 < kLanes * kSlabs ? i + 1 : i;
+                const uint32_t w0 = slot[s * 32 + lane];
+                const uint32_t w1 = slot[(next / kLanes) * 32 + group * kLanes + (next & (kLanes - 1))];
+                const uint32_t v = __funnelshift_r(w0, w1, (uint32_t)(reinterpret_cast<uintptr_t>(row) & 2) * 8);
+                return i < width ? v : 0u;
+            } else {
+                return slot[s * 32 + lane];
+            }
+        };
+        Piece x[kSlabs];
+#pragma unroll
+        for (int s = 0; s < kSlabs; ++s) x[s] = Piece{};
+        int before = -1;
+#pragma unroll
+        for (int i = 0; i < kStages - 1; ++i) request(i);
+#pragma unroll 1
+        for (int batch = 0; batch < batches; ++batch) {
+            request(batch + kStages - 1);
+            CopyWait<kStages - 1>();
+            __syncwarp();
+            const int stage = batch % kStages;
+            float acc[kBatch];
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+                const int t = t0 + batch * kBatch + u;
+                const int row = sRow[t];
+                if (row != before) {
+#pragma unroll
+                    for (int s = 0; s < kSlabs; ++s) x[s] = read(sX + (stage * kBatch + u) * kSlabs * 32, X + row * xRowBytes, s);
+                    before = row;
+                }
                 acc[u] = 0.0f;
-                if (p + u >= p1) continue;
-                const uint4 *xr = X16 + (long long)rows[u] * xRow16;
-                if (rows[u] != cachedRow) {
-                    if (lane < pieces) x0 = __ldg(xr + lane);
-                    cachedRow = rows[u];
-                }
-                if (lane < pieces) acc[u] = Dot16(x0, y[u], acc[u], T());
-                if (pieces > 32) {
-                    const int j = __shfl_sync(0xffffffffu, myCol, (int)(p + u - p0) & 31);
-                    const uint4 *yc = Y16 + (long long)j * yRow16;
-                    for (int q = lane + 32; q < pieces; q += 32) acc[u] = Dot16(__ldg(xr + q), __ldg(yc + q), acc[u], T());
-                }
-            }
 #pragma unroll
-            for (int u = 0; u < kSddmmBatch; ++u) {
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], off);
+                for (int s = 0; s < kSlabs; ++s)
+                    acc[u] = DotPiece<T>(x[s], read(sY + (stage * kBatch + u) * kSlabs * 32, Y + sCol[t] * yRowBytes, s), acc[u]);
             }
-            // every lane holds all sums now: lane u writes entry p + u
-            float mine = 0.0f;
+            // Lanes with bit kLanes/2 set keep the upper half of the values, then those with bit kLanes/4 the odd ones.
+            const bool up = (li & (kLanes / 2)) != 0;
+            float v;
+            int u;  // the value this lane ends up with
+            if constexpr (kBatch == 4) {
+                const bool odd = (li & (kLanes / 4)) != 0;
+                const float k0 = (up ? acc[2] : acc[0]) + __shfl_xor_sync(0xffffffffu, up ? acc[0] : acc[2], kLanes / 2);
+                const float k1 = (up ? acc[3] : acc[1]) + __shfl_xor_sync(0xffffffffu, up ? acc[1] : acc[3], kLanes / 2);
+                v = (odd ? k1 : k0) + __shfl_xor_sync(0xffffffffu, odd ? k0 : k1, kLanes / 4);
 #pragma unroll
-            for (int u = 0; u < kSddmmBatch; ++u) mine = lane == u ? acc[u] : mine;
-            if (lane < kSddmmBatch && p + lane < p1) {
-                float z = a * mine;
-                if (b != 0.0f) z += b * Load<T>(cVal + p + lane);
-                cVal[p + lane] = Store<T>(z);
+                for (int off = kLanes / 8; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+                u = (up ? 2 : 0) + (odd ? 1 : 0);
+            } else {
+                v = (up ? acc[1] : acc[0]) + __shfl_xor_sync(0xffffffffu, up ? acc[0] : acc[1], kLanes / 2);
+#pragma unroll
+                for (int off = kLanes / 4; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+                u = up ? 1 : 0;
             }
+            if ((li & (kLanes / kBatch - 1)) == 0) sDot[t0 + batch * kBatch + u] += v;
+            __syncwarp();  // this stage's slots may be written again
         }
+        CopyWait<0>();
+        __syncwarp();
+    }
+    for (int t = lane; t < tile && p0 + t < nnz; t += 32) {
+        float z = a * sDot[t];
+        if (b != 0.0f) z += b * Load<T>(cVal + p0 + t);
+        cVal[p0 + t] = Store<T>(z);
     }
 }
 
@@ -245,28 +390,71 @@ aclsparseStatus_t ValidateCall(aclsparseHandle_t handle, const aclsparseDnMatDes
     return ACL_SPARSE_STATUS_SUCCESS;
 }
 
+template <typename T, int kBytes, int kLanes, int kSlabs, typename... Args>
+int LaunchRowsShape(int nnz, int tile, cudaStream_t stream, Args... args)
+{
+    using Shape = SddmmShape<kBytes, kLanes, kSlabs>;
+    static std::atomic<bool> configured[64] = {};  // per device: this instantiation may use kCtaBytes of shared memory
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
+    if (!configured[dev].load(std::memory_order_relaxed)) {
+        const cudaError_t e = cudaFuncSetAttribute(SddmmRowsKernel<T, kBytes, kLanes, kSlabs>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::kCtaBytes);
+        if (e != cudaSuccess) return (int)e;
+        configured[dev].store(true, std::memory_order_relaxed);
+    }
+    const long long warps = ((long long)nnz + tile - 1) / tile;
+    b200sp_note_launches(1);
+    return (int)b200sp::LaunchChained(SddmmRowsKernel<T, kBytes, kLanes, kSlabs>,
+                                      (unsigned)((warps + kSddmmWarps - 1) / kSddmmWarps), 32 * kSddmmWarps, Shape::kCtaBytes,
+                                      stream, args...);
+}
+
+template <typename T, int kBytes>
+int LaunchRows(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const aclsparseDnMatDescr *Y, int k, Strides st,
+               float alpha, float beta, const void *alphaDev, const void *betaDev, cudaStream_t stream)
+{
+    const int nnz = (int)C->nnz;
+    // pieces of a row, one more where they start in the middle of a word
+    const int pieces = kBytes == 2 ? (k + 1) / 2 + 1 : (int)((long long)k * (long long)sizeof(T) / kBytes);
+    // The longer the tile the longer the runs of copies in flight, as long as every SM gets some 16 warps.
+    int tile = 32;
+    while (tile < kSddmmTile && nnz / (2 * tile) >= 16 * b200sp_sm_count()) tile *= 2;
+    auto launch = [&]<int kLanes, int kSlabs>() {
+        return LaunchRowsShape<T, kBytes, kLanes, kSlabs>(
+            nnz, tile, stream, static_cast<const int32_t *>(C->offsets), static_cast<const int32_t *>(C->indices),
+            static_cast<T *>(C->values), static_cast<const char *>(X->values), static_cast<const char *>(Y->values),
+            (int)C->rows, k, nnz, tile, st.xi * (long long)sizeof(T), st.yj * (long long)sizeof(T), alpha, beta,
+            static_cast<const T *>(alphaDev), static_cast<const T *>(betaDev));
+    };
+    if (pieces <= 4) return launch.template operator()<4, 1>();
+    if (pieces <= 8) return launch.template operator()<8, 1>();
+    if (pieces <= 16) return launch.template operator()<16, 1>();
+    if (pieces <= 32) return launch.template operator()<32, 1>();
+    if (pieces <= 64) return launch.template operator()<32, 2>();
+    return launch.template operator()<32, 4>();
+}
+
 template <typename T>
 int Launch(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const aclsparseDnMatDescr *Y, int k, Strides st,
            float alpha, float beta, const void *alphaDev, const void *betaDev, cudaStream_t stream)
 {
+    if (st.xk == 1 && st.yk == 1) {
+        // the widest piece that every row starts and ends on
+        const unsigned long long all = (unsigned long long)k * sizeof(T) | (unsigned long long)st.xi * sizeof(T) |
+                                       (unsigned long long)st.yj * sizeof(T) | reinterpret_cast<uintptr_t>(X->values) |
+                                       reinterpret_cast<uintptr_t>(Y->values);
+        if (all % 16 == 0) return LaunchRows<T, 16>(C, X, Y, k, st, alpha, beta, alphaDev, betaDev, stream);
+        if (all % 8 == 0) return LaunchRows<T, 8>(C, X, Y, k, st, alpha, beta, alphaDev, betaDev, stream);
+        if (all % 4 == 0) return LaunchRows<T, 4>(C, X, Y, k, st, alpha, beta, alphaDev, betaDev, stream);
+        if constexpr (sizeof(T) == 2)  // the covering words of the first rows start at the arrays
+            if (reinterpret_cast<uintptr_t>(X->values) % 4 == 0 && reinterpret_cast<uintptr_t>(Y->values) % 4 == 0)
+                return LaunchRows<T, 2>(C, X, Y, k, st, alpha, beta, alphaDev, betaDev, stream);
+    }
     const long long chunks = (C->nnz + 31) / 32;
     const long long want = (chunks + 7) / 8;
     const long long cap = (long long)b200sp_sm_count() * 32;
     const unsigned grid = (unsigned)(want < cap ? want : cap);
-    const long long rowBytes = (long long)k * (long long)sizeof(T);
-    const bool vec = st.xk == 1 && st.yk == 1 && rowBytes % 16 == 0 && (st.xi * (long long)sizeof(T)) % 16 == 0 &&
-                     (st.yj * (long long)sizeof(T)) % 16 == 0 && reinterpret_cast<uintptr_t>(X->values) % 16 == 0 &&
-                     reinterpret_cast<uintptr_t>(Y->values) % 16 == 0;
-    if (vec) {
-        SddmmVecKernel<T><<<grid, 256, 0, stream>>>(
-            static_cast<const int32_t *>(C->offsets), static_cast<const int32_t *>(C->indices),
-            static_cast<T *>(C->values), static_cast<const T *>(X->values), static_cast<const T *>(Y->values),
-            (int)C->rows, (int)(rowBytes / 16), (long long)C->nnz, st.xi * (long long)sizeof(T) / 16,
-            st.yj * (long long)sizeof(T) / 16, alpha, beta, static_cast<const T *>(alphaDev),
-            static_cast<const T *>(betaDev));
-        b200sp_note_launches(1);
-        return (int)cudaGetLastError();
-    }
     SddmmKernel<T><<<grid, 256, 0, stream>>>(
         static_cast<const int32_t *>(C->offsets), static_cast<const int32_t *>(C->indices), static_cast<T *>(C->values),
         static_cast<const T *>(X->values), static_cast<const T *>(Y->values), (int)C->rows, k, (long long)C->nnz, st,

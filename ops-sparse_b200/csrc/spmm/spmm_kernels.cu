@@ -1546,7 +1546,7 @@ size_t RepackBytes(const b200spSpmmShape *sh, int valBytes)
 // Repacking reads and writes k * n elements; the generic kernel touches nnz * n of them, a sector each when the
 // columns of B are the contiguous ones and otherwise with one load per product instead of one per 16 bytes.  From
 // two entries per row of B on the copy is the cheaper side by far (65,537 x 50,001 with 24 entries a row, fp16,
-// N = 40 in column-major order: generic 257 us, copy + product 22 us).
+// N = 40 in column-major order: generic 257 us, copy + product 57 us).
 bool WorthRepacking(const b200spSpmmShape *sh) { return sh->nnz >= 2 * sh->k; }
 
 template <typename ValT, typename OutT>
@@ -1657,7 +1657,7 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
     };
     if constexpr (kInt8) {
         // Integer sums may be regrouped: where a warp per row would not fill the SMs and rows are long enough to be
-        // shared, a CTA takes a row (4096 rows of 410 entries, N = 512: B200SP_SPLIT_NOTE).
+        // shared, a CTA takes a row (4096 rows of 410 entries, N = 512: 104 us with a warp per row, 74 us so).
         a.splitRows = cPlain && sh->nnz >= 128 * sh->m && sh->m * lanes_ / 32 < 64ll * b200sp_sm_count();
         return (int)launchFast(segments, true, stream);
     } else {
