@@ -15,6 +15,7 @@
 #include "b200sp_kernels.h"
 #include "common/chained.cuh"
 #include "common/internal.h"
+#include "common/rows.cuh"
 
 namespace {
 
@@ -129,31 +130,6 @@ template <int kSize> __device__ __forceinline__ void CopyAsync(void *dst, const 
 __device__ __forceinline__ void CopyCommit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int kPending> __device__ __forceinline__ void CopyWait() { asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory"); }
 
-// Row of every lane's entry p (p0 + lane), given a row r0 with rowPtr[r0] <= p0: largest r with rowPtr[r] <= p.
-__device__ __forceinline__ int RowOfLane(const int32_t *__restrict__ rowPtr, int m, int r0, int p, int lane)
-{
-    const int last = 0x7fffffff;
-    const int end = r0 + 1 + lane <= m - 1 ? __ldg(rowPtr + r0 + 1 + lane) : last;  // starts of the 32 rows after r0
-    int n = 0;  // how many of them are <= p: they ascend
-#pragma unroll
-    for (int step = 16; step > 0; step >>= 1) {
-        const int at = __shfl_sync(0xffffffffu, end, n + step - 1);
-        if (at <= p) n += step;
-    }
-    const int end31 = __shfl_sync(0xffffffffu, end, 31);
-    if (n == 31 && end31 <= p) n = 32;
-    int r = r0 + n;
-    if (n == 32) {  // more than 32 rows within 32 entries: go on alone
-        int hi = m - 1;
-        while (r < hi) {
-            const int mid = r + ((hi - r + 1) >> 1);
-            if (__ldg(rowPtr + mid) <= p) r = mid;
-            else hi = mid - 1;
-        }
-    }
-    return r;
-}
-
 // 1384 us with 4 warps and tiles of 128, 1286 with 2 and 64 on the same GPU; one warp or longer tiles gain nothing more.
 constexpr int kSddmmWarps = 2;
 constexpr int kSddmmTile = 64;  // entries a warp owns at most
@@ -195,19 +171,10 @@ __global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(
     int *sRow = reinterpret_cast<int *>(sWarp + Shape::kRing), *sCol = sRow + kSddmmTile;
     float *sDot = reinterpret_cast<float *>(sCol + kSddmmTile);
 
-    // The row of the first entry (largest r with rowPtr[r] <= p0): the 32 lanes probe 32 places per round.
-    int r0 = 0;
-    for (int hi = m; hi - r0 > 1;) {
-        const int step = (hi - r0 + 31) / 32;
-        const long long idx = (long long)r0 + (long long)(lane + 1) * step;
-        const bool ok = idx < hi && (long long)__ldg(rowPtr + idx) <= p0;
-        const int n = __popc(__ballot_sync(0xffffffffu, ok));  // offsets ascend: the lanes that pass are a prefix
-        r0 += n * step;
-        hi = hi < r0 + step ? hi : r0 + step;
-    }
+    int r0 = b200sp::WarpRowOf(rowPtr, m, p0, lane);
     for (int t = lane; t < tile; t += 32) {
         const int p = p0 + t < nnz ? (int)p0 + t : nnz - 1;  // past the end: the last entry again, not stored
-        const int r = RowOfLane(rowPtr, m, r0, p, lane);
+        const int r = b200sp::RowOfLane(rowPtr, m, r0, p, lane);
         sRow[t] = r;
         sCol[t] = __ldg(colInd + p);
         sDot[t] = 0.0f;
