@@ -2,14 +2,11 @@
 // carried along; and the legacy matrix descriptor it takes its index base from.
 // Checks, their order and status codes follow the reference host layer
 // (sparse/csrsort/arch35/csrsort_host.cpp:52-74, 146-222; sparse/common/aclsparse_matdescr.cpp:25-108).
-// The sort: every entry becomes a 64-bit key (column in the high word, position inside its row in the low word),
-// which makes keys unique and the ascending order of keys exactly the stable order the golden defines
-// (test/csrsort/arch35/csrsort_golden.h:38-70); the rows are sorted by the segmented sort of segsort.cuh
-// (registers for rows of up to 256 entries, shared memory up to 2048, chunk sort + merge passes beyond), which
-// forms the keys while it loads a row and splits them while it stores it: the high word is the sorted column, the
-// low word says which entry of P moves here.  Two launches, no pass of its own over the arrays.
-// Workspace: 8 bytes per entry for the keys and 8 for the merge scratch (both touched only for rows of more than
-// 2048 entries) and a list of the rows too long for a warp.
+// The rows are sorted by the kernels of rowsort.cuh, each row by the method its length asks for; the order is
+// (column, place in the row), which is the stable order the golden defines
+// (test/csrsort/arch35/csrsort_golden.h:38-70).
+// Workspace: 16 bytes per entry (touched only for rows of more than 16384 entries) and a list of the rows too long for
+// a warp.
 #include <cstdint>
 #include <limits>
 #include <new>
@@ -18,7 +15,7 @@
 
 #include "b200sp_kernels.h"
 #include "common/internal.h"
-#include "convert/segsort.cuh"
+#include "convert/rowsort.cuh"
 
 struct aclsparseMatDescr {  // aclsparse_descr_internal.h:131-136
     aclsparseMatrixType_t type = ACL_SPARSE_MATRIX_TYPE_GENERAL;
@@ -50,30 +47,9 @@ SortLayout SortLayoutFor(int m, int nnz)
     L.offKeys = 0;
     L.offScratch = keys;
     L.offList = 2 * keys;
-    L.total = 2 * keys + b200sp_segsort::ListBytes(m);
+    L.total = 2 * keys + b200sp_rowsort::ListBytes(m);
     return L;
 }
-
-// How the sort reads and writes this operator's arrays: the key of entry i of a row is (column << 32 | i), made on
-// the fly from csrColInd; a sorted key puts its high word back into csrColInd and moves P[row start + low word] to
-// its place (read for the whole row before any of it is written: the sort is in place in both arrays).
-struct CsrsortIo {
-    int *colInd;
-    int *P;
-    using Payload = int;
-    __device__ __forceinline__ unsigned long long Load(int a, int i) const
-    {
-        return ((unsigned long long)(unsigned)colInd[a + i] << 32) | (unsigned)i;
-    }
-    __device__ __forceinline__ int Fetch(int a, unsigned long long key) const { return P[a + (int)(unsigned)(key & 0xffffffffu)]; }
-    __device__ __forceinline__ void Commit(int a, int i, unsigned long long key, int moved) const
-    {
-        colInd[a + i] = (int)(unsigned)(key >> 32);
-        P[a + i] = moved;
-    }
-    static __device__ __forceinline__ unsigned Pack(int v) { return (unsigned)v; }
-    static __device__ __forceinline__ int Unpack(unsigned v) { return (int)v; }
-};
 
 }  // namespace
 
@@ -138,7 +114,7 @@ aclsparseStatus_t aclsparseXcsrsort(aclsparseHandle_t handle, int m, int n, int 
     auto *scratch = reinterpret_cast<unsigned long long *>(w + L.offScratch);
     auto *list = reinterpret_cast<int *>(w + L.offList);
     const int b = base == ACL_SPARSE_INDEX_BASE_ONE ? 1 : 0;
-    const cudaError_t e = b200sp_segsort::Sort(csrRowPtr, b, m, CsrsortIo{csrColInd, P}, keys, scratch, list, stream);
+    const cudaError_t e = b200sp_rowsort::Sort(csrRowPtr, b, m, n, nnz, csrColInd, P, keys, scratch, list, stream);
     if (e != cudaSuccess) {
         B200SP_LOGE("aclsparseXcsrsort: sort failed (%s)", cudaGetErrorString(e));
         (void)cudaGetLastError();
