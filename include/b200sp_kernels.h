@@ -84,6 +84,15 @@ int b200sp_spmv_launch(const int32_t *row_ptr, const int32_t *col_ind, const voi
                        int64_t rows, int64_t cols, int64_t nnz, const b200spScalars *scalars, int comp_type,
                        int val_type, int out_type, void *plan, const int32_t *plan_info, void *stream);
 
+/* The same product for a matrix that was not analysed, with nothing to analyse first: a kernel over the rows and a second
+ * one for the segments of the rows above 1024 entries, which the first lists in `scratch`
+ * (b200sp_spmv_rows_bytes(nnz) bytes, contents arbitrary).  `state` is two ints of device memory that are zero before the
+ * first product; every product leaves them zero.  Two products that can overlap need a scratch and a state each. */
+size_t b200sp_spmv_rows_bytes(int64_t nnz);
+int b200sp_spmv_rows_launch(const int32_t *row_ptr, const int32_t *col_ind, const void *val, const void *x, void *y, int64_t rows,
+                            int64_t nnz, const b200spScalars *scalars, int comp_type, int val_type, int out_type, void *scratch,
+                            int32_t *state, void *stream);
+
 /* Longest row of A, read back to *max_len (synchronises `stream` once).  scratch4 is any 4 bytes of
  * device memory.  The analysis of the transposed product: it decides `by_nnz` below. */
 int b200sp_spmv_max_row_length(const int32_t *row_ptr, int64_t rows, void *scratch4, int32_t *max_len, void *stream);

@@ -288,12 +288,33 @@ aclsparseStatus_t aclsparseSpMV(aclsparseHandle_t handle, aclsparseOperation_t o
             plan = externalBuffer;  // analysed by Preprocess: nothing to redo
             info = matA->active.spmvInfo;
         } else {
-            // Per-call analysis stays asynchronous: a tile plan, in the caller's buffer or the handle workspace.
+            // Without a plan: two kernels that need no analysis, with their list of long rows in the caller's buffer
+            // (as large as GetBufferSize says, which is more) or the handle workspace; where that is too small, the tile
+            // kernel with a plan per call.
+            const size_t listBytes = b200sp_spmv_rows_bytes(matA->nnz);
+            char *scratch = static_cast<char *>(externalBuffer);
+            int32_t *state = handle->productState;
+            if (scratch != nullptr) {  // nothing of the handle is shared then: its stream may change between products
+                state = reinterpret_cast<int32_t *>(scratch);
+                scratch += b200sp::kStateBytes;
+                if (cudaMemsetAsync(state, 0, b200sp::kStateBytes, stream) != cudaSuccess) return ACL_SPARSE_STATUS_EXECUTION_FAILED;
+            } else if (handle->WorkspaceBytes() >= listBytes) {
+                scratch = static_cast<char *>(handle->Workspace());
+            }
+            if (scratch != nullptr) {
+                (void)b200sp::NoteBufferWrite(externalBuffer != nullptr ? externalBuffer : scratch);  // a plan recorded for this buffer, of any matrix, is stale now
+                rc = b200sp_spmv_rows_launch(rowPtr, colInd, matA->values, vecX->values, vecY->values, matA->rows, matA->nnz, &sc,
+                                             c.compType, c.valType, c.outType, scratch, state, stream);
+                if (rc != 0) {
+                    B200SP_LOGE("aclsparseSpMV: kernel launch failed (cuda error %d)", rc);
+                    return ACL_SPARSE_STATUS_EXECUTION_FAILED;
+                }
+                return ACL_SPARSE_STATUS_SUCCESS;
+            }
             const size_t bytes = b200sp_spmv_tile_plan_bytes(matA->rows, matA->nnz);
-            if (externalBuffer != nullptr) plan = externalBuffer;
-            else if (handle->WorkspaceBytes() >= bytes) plan = handle->Workspace();
-            if (plan != nullptr) {
-                (void)b200sp::NoteBufferWrite(plan);  // a plan recorded for this buffer, of any matrix, is stale now
+            if (handle->WorkspaceBytes() >= bytes) {
+                plan = handle->Workspace();
+                (void)b200sp::NoteBufferWrite(plan);
                 rc = b200sp_spmv_analyze(rowPtr, colInd, matA->rows, matA->cols, matA->nnz, plan, bytes, nullptr, stream);
                 if (rc != 0) {
                     B200SP_LOGE("aclsparseSpMV: analysis launch failed (cuda error %d)", rc);

@@ -1,0 +1,73 @@
+"""GPU: aclsparseSpMV without an analysed buffer where its kernels change hands, against the CPU golden."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+import helpers
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mean", [2, 12, 40, 100, 300])  # one per width of the lane groups
+@pytest.mark.parametrize("vt,ot", [("f32", "f32"), ("bf16", "bf16"), ("i32", "i32")])
+@pytest.mark.parametrize("own_buffer", [False, True])
+def test_row_lengths_around_every_limit(handle, device, oracle, mean, vt, ot, own_buffer):
+    """Rows on both sides of a lane group's, a warp's and a segment's limit; twice, so that what the first product left
+    behind is met by the second."""
+    from ops_sparse_b200 import api, synth
+    rng = np.random.default_rng(mean)
+    edges = [16 * g for g in (2, 4, 8, 16, 32)] + [1024, 8192, 16384]
+    lengths = np.concatenate([rng.integers(0, 2 * mean + 1, 5000), [e + d for e in edges for d in (0, 1)], [0, 40000]])
+    rng.shuffle(lengths)
+    m, n = lengths.size, 60000
+    whole = vt == "i32"
+    A = synth.csr_from_lengths(rng, lengths, n, (lambda r, k: r.integers(-9, 10, k)) if whole else synth.normal)
+    x = rng.integers(-9, 10, n).astype(np.int32) if whole else oracle.to_storage(rng.standard_normal(n).astype(np.float32), vt)
+    y = rng.integers(-9, 10, m).astype(np.int32) if whole else oracle.to_storage(rng.standard_normal(m).astype(np.float32), ot)
+    val = A.values.astype(np.int32) if whole else oracle.to_storage(A.values, vt)
+    alpha, beta = (2, -3) if whole else (1.5, -0.5)
+    dA = helpers.make_csr(device, A.row_ptr, A.col_ind, val, vt, m, n)
+    dx = api.DnVec(helpers.to_device(x, vt, device))
+    for _ in range(2):
+        dy = api.DnVec(helpers.to_device(y, ot, device))
+        buf = torch.full((api.spmv_buffer_size(handle, dA, dx, dy),), 0x5A, dtype=torch.uint8, device=device) if own_buffer else None
+        api.spmv(handle, dA, dx, dy, alpha, beta, buffer=buf)
+        torch.cuda.synchronize()
+        got = helpers.to_host(dy.values, ot)
+        if whole:
+            prod = val.astype(np.int64) * x[A.col_ind].astype(np.int64)
+            total = np.concatenate([[0], np.cumsum(prod)])
+            want = alpha * (total[A.row_ptr[1:]] - total[A.row_ptr[:-1]]) + beta * y.astype(np.int64)
+            assert np.array_equal(got, want.astype(np.int32))
+            continue
+        f = lambda a, t: oracle.from_storage(a, t).astype(np.float64)
+        prod = f(val, vt) * f(x, vt)[A.col_ind]
+        add = lambda p: np.diff(np.concatenate([[0.0], np.cumsum(p)])[A.row_ptr])
+        want, scale = alpha * add(prod) + beta * f(y, ot), abs(alpha) * add(np.abs(prod)) + np.abs(beta * f(y, ot))
+        if ot == "bf16":  # the one rounding of the result, 8 bits
+            scale = scale + np.abs(want) * 2.0 ** -8 / helpers.TOL[vt]
+        helpers.assert_rowwise(f(got, ot), want, scale + 1e-12, helpers.TOL[vt], f"unplanned {vt} mean {mean}")
+
+
+@pytest.mark.parametrize("items", [1 << 18, (1 << 18) + 1, 1 << 23, (1 << 23) + 1])
+def test_tile_sizes_of_the_entry_point_without_scratch(pkg, device, oracle, items):
+    """rows + entries at which the tiles change size; rows that span tiles, empty rows, a ragged last tile."""
+    from ctypes import c_float, c_int, c_int64, c_void_p
+    rng = np.random.default_rng(items)
+    m, n = items // 40, 50000
+    nnz = items - m
+    rp = np.concatenate([[0], np.sort(rng.integers(0, nnz + 1, m - 1)), [nnz]]).astype(np.int32)
+    rp[m // 2:m // 2 + m // 50] = rp[m // 2]  # a long row after a stretch of empty ones
+    ci = rng.integers(0, n, nnz).astype(np.int32)
+    val, x, y = (rng.standard_normal(k).astype(np.float32) for k in (nnz, n, m))
+    f = pkg.lib().b200sp_spmv_f32_noalloc
+    f.restype, f.argtypes = c_int, [c_void_p] * 5 + [c_int64] * 3 + [c_float] * 2 + [c_void_p]
+    d = [torch.from_numpy(a).to(device) for a in (rp, ci, val, x, y)]
+    assert f(*(c_void_p(t.data_ptr()) for t in d), m, n, nnz, 1.5, -0.5,
+             c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    torch.cuda.synchronize()
+    want = oracle.spmv(rp, ci, val, x, y, 1.5, -0.5)
+    scale = 1.5 * oracle.spmv_abs_rowsum(rp, ci, val, x) + 0.5 * np.abs(y) + 1e-12
+    helpers.assert_rowwise(d[4].cpu().numpy().astype(np.float64), want.astype(np.float64), scale, helpers.TOL["f32"], "tiles")
