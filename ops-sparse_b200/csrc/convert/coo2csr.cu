@@ -21,7 +21,6 @@ __global__ void __launch_bounds__(256) Coo2CsrKernel(const int *__restrict__ coo
                                                      int *__restrict__ csrRowPtr, int base)
 {
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     for (long long i0 = (long long)blockIdx.x * 256; i0 <= m; i0 += (long long)gridDim.x * 256)
         b200sp::OffsetsOfSorted(cooRowInd, nnz, i0, m, base, base, csrRowPtr);
 }

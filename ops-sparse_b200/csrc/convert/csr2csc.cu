@@ -87,7 +87,6 @@ __global__ void __launch_bounds__(256) ColumnOffsetsKernel(const int *__restrict
                                                            int *__restrict__ cscColPtr)
 {
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     for (long long i0 = (long long)blockIdx.x * 256; i0 <= n; i0 += (long long)gridDim.x * 256)
         b200sp::OffsetsOfSorted(sortedCols, nnz, i0, n, 0, base, cscColPtr);
 }

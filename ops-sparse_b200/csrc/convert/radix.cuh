@@ -74,7 +74,6 @@ static __global__ void __launch_bounds__(kThreads) HistogramKernel(const int *__
 {
     __shared__ int sHist[kMaxBins];
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     for (int i = threadIdx.x; i < bins; i += kThreads) sHist[i] = 0;
     __syncthreads();
     const long long first = (long long)blockIdx.x * kThreads * kItems;
@@ -127,7 +126,6 @@ inline int ChunksFor(long long tiles) { return (int)((tiles + kChunk - 1) / kChu
 static __global__ void __launch_bounds__(128) ScanTilesKernel(int *__restrict__ counts, int tiles, int bins, int *__restrict__ chunks)
 {
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     const int digitBlocks = (bins + 127) / 128;
     const int d = (int)(blockIdx.x % digitBlocks) * 128 + threadIdx.x, chunk = blockIdx.x / digitBlocks;
     if (d >= bins) return;
@@ -152,7 +150,6 @@ static __global__ void __launch_bounds__(kMaxBins) ScanChunksKernel(int *__restr
 {
     __shared__ int sWarp[32];
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     const int d = threadIdx.x;
     int run = 0;
     if (d < bins) {
@@ -269,7 +266,6 @@ static __global__ void __launch_bounds__(kThreads, 2) ScatterKernel(const PassAr
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int bins = a.bins;
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     const long long first = (long long)blockIdx.x * kTile;
     const int live = a.nnz - first < kTile ? (int)(a.nnz - first) : kTile;
 
@@ -393,7 +389,6 @@ static __global__ void __launch_bounds__(256) OffsetsFromCountsKernel(const int 
     constexpr int kTile = kThreads * kItems;
     __shared__ int sHist[kMaxBins];
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     const int bins = 1 << digitBits, lo = blockIdx.x;
     if (lo == 0 && threadIdx.x == 0) colPtr[n] = nnz + base;
     if (passes == 1) {

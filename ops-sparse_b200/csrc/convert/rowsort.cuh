@@ -100,7 +100,6 @@ static __global__ void __launch_bounds__(128) RowSortWarpKernel(const int *__res
                                                                 const int *__restrict__ list)
 {
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     const int lane = threadIdx.x & 31;
     const int count = list[kCountWarp];
     for (int i = blockIdx.x * 4 + (threadIdx.x >> 5); i < count; i += gridDim.x * 4) {
@@ -117,7 +116,6 @@ static __global__ void __launch_bounds__(256) RowSortShortKernel(const int *__re
                                                                  int *colInd, int *P, int *__restrict__ list)
 {
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     const int lane = threadIdx.x & 31;
     const long long row0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * rowsPerWarp;
     if (row0 >= m) return;
@@ -390,7 +388,6 @@ static __global__ void __launch_bounds__(kThreads, 2048 / kThreads > 227 * 1024 
     __shared__ unsigned sCost;
     __shared__ int sTake;
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     const int count = list[kClass];
     const int *rows = list + kListHead + (kClass == kCountMid ? 0 : m);
     for (;;) {
@@ -418,7 +415,6 @@ static __global__ void __launch_bounds__(kHugeThreads) RowSortHugeKernel(const i
     __shared__ int sWarp[kHugeWarps];
     __shared__ int sTake, sWord;
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     if (list[kCountHuge] == 0) return;
     const int count = list[kCountLong];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

@@ -158,7 +158,6 @@ __global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(
     static_assert(kLanes >= 4, "the sums of a batch are spread over four lanes");
     extern __shared__ __align__(16) unsigned char sRaw[];
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     const float a = alphaDev ? Load<T>(alphaDev) : alpha;
     const float b = betaDev ? Load<T>(betaDev) : beta;
     const int lane = threadIdx.x & 31;

@@ -184,7 +184,6 @@ __global__ void __launch_bounds__(256) SpmvTileSearchKernel(const int32_t *__res
                                                             int32_t *__restrict__ counters)
 {
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (t > ntiles) return;
@@ -247,7 +246,6 @@ __global__ void __launch_bounds__(TileThreads(kSize)) SpmvTileKernel(const TileA
     const int warp = tid >> 5;
     const int t = blockIdx.x;
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     const int i0 = a.tileRow[t];
     const int i1 = a.tileRow[t + 1];
     const long long total = (long long)a.rows + a.nnz;
@@ -479,11 +477,8 @@ struct BinHeader {  // first 256 bytes of the binned plan
 #endif
 constexpr int kXBlockElems = B200SP_SPMV_XBLOCK_ELEMS;  // 128 KB of fp32 x, 64 KB of 16-bit x
 constexpr int kMaxXBlocks = 64;      // wider matrices use SpmvLongListKernel
-constexpr int kMaxLongGroups = 64;   // CTAs per column block
+constexpr int kMaxLongGroups = 160;  // CTAs per column block
 constexpr int kLongBlockThreads = B200SP_SPMV_LONG_BLOCK_THREADS;
-#ifndef B200SP_SPMV_PIECE_LANES
-#define B200SP_SPMV_PIECE_LANES 8    // lanes that share one (long row, x block) piece
-#endif
 #ifndef B200SP_SPMV_FUSE_LIST
 #define B200SP_SPMV_FUSE_LIST 1      // long rows that keep a CTA each share one grid with the other bins
 #endif
@@ -653,7 +648,7 @@ struct LongBlockArgs {
 
 // CTA (b, g) keeps block b of x in shared memory and sums, for every long row of its group,
 // the entries whose column falls in that block -- a contiguous piece of the row, because the
-// column indices ascend.  kPieceLanes lanes share a piece; x comes from shared memory, so the
+// column indices ascend.  kPieceLanes lanes share a piece (8, 32 or 256: see LongBlockShapeFor); x comes from shared memory, so the
 // only global traffic is the col_ind / values stream.  The last CTA of a row group to finish
 // adds each row's partial sums in block order (no wait, fixed order) and writes y.
 // Registers are capped at 48 (not at the 64 a 1024-thread CTA could have): while this kernel holds an SM, the
@@ -661,7 +656,7 @@ struct LongBlockArgs {
 // occupancy.  Timestamps taken inside the kernels on the power-law matrix: these CTAs run 30-43 us, all done 47 us
 // after the first started; the medium rows beside them finish at 68 us instead of 35 alone, the short rows at
 // 91.  Product time with 56 / 46 / 40 registers here: 90.2 / 86.4 / 89.2 us.
-template <typename CompT, typename ValT, typename OutT, bool kVec>
+template <typename CompT, typename ValT, typename OutT, bool kVec, int kPieceLanes>
 __global__ void __maxnreg__(48) SpmvLongBlockKernel(const LongBlockArgs<CompT, ValT, OutT> a)
 {
     extern __shared__ __align__(16) unsigned char sRaw[];
@@ -687,7 +682,6 @@ __global__ void __maxnreg__(48) SpmvLongBlockKernel(const LongBlockArgs<CompT, V
     __syncthreads();
 
     const ValT *xrel = xs - x0;  // xrel[col] is x[col] for the columns of this block
-    constexpr int kPieceLanes = B200SP_SPMV_PIECE_LANES;
     constexpr int kUnroll = B200SP_SPMV_LONG_BLOCK_UNROLL;  // quads in flight per lane
     constexpr int kPiecesPerCta = kLongBlockThreads / kPieceLanes;
     const int pl = tid & (kPieceLanes - 1);
@@ -756,7 +750,17 @@ __global__ void __maxnreg__(48) SpmvLongBlockKernel(const LongBlockArgs<CompT, V
         }
         sCur = sNext;
         eCur = eNext;
-        sum = GroupSum(sum, kPieceLanes);
+        sum = GroupSum(sum, kPieceLanes < 32 ? kPieceLanes : 32);
+        if constexpr (kPieceLanes > 32) {  // the piece's warps, in order
+            __shared__ CompT sWarp[kLongBlockThreads / 32];
+            if ((tid & 31) == 0) sWarp[tid >> 5] = sum;
+            __syncthreads();
+            if (pl == 0) {
+#pragma unroll
+                for (int w = 1; w < kPieceLanes / 32; ++w) sum += sWarp[(tid >> 5) + w];
+            }
+            __syncthreads();
+        }
         if (pl == 0 && slot < nLong) a.partials[(long long)slot * a.xBlocks + b] = sum;
     }
 
@@ -974,7 +978,6 @@ __global__ void __launch_bounds__(256) SpmvShortRowsKernel(const int32_t *__rest
                                                             int rows, Scalars<CompT> sc)
 {
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     ShortRowsBody<CompT, ValT, OutT, G>(blockIdx.x, rowPtr, colInd, val, x, y, rows, sc);
 }
 
@@ -991,7 +994,6 @@ __global__ void __launch_bounds__(256) SpmvMediumShortKernel(const int32_t *__re
                                                               Scalars<CompT> sc)
 {
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     const unsigned wpc = blockDim.x >> 5;
     const unsigned mediumBlocks = ((unsigned)nM + wpc - 1u) / wpc;
     if (blockIdx.x < mediumBlocks) MediumRowsBody<CompT, ValT, OutT>(blockIdx.x, colInd, val, x, y, listM, nM, sc);
@@ -1022,7 +1024,6 @@ __global__ void __launch_bounds__(256, 6) SpmvAllBinsKernel(const int32_t *__res
 {
     __shared__ CompT sWarp[8];
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     unsigned b = blockIdx.x;
     if (b < (unsigned)nL) {  // nL counts segments here
         LongRowBody<CompT, ValT, OutT, kVec, 2>(b, colInd, val, x, y, ls, sc, sWarp);
@@ -1062,7 +1063,8 @@ inline RowList RowListIn(void *scratch, int32_t *state, int64_t nnz)
     return {state, reinterpret_cast<int2 *>(p), reinterpret_cast<int32_t *>(p + n), p + n + (size_t)RowListItems(nnz) * 4};
 }
 
-template <typename CompT, typename ValT, typename OutT, int G>
+// kList false: rows of kLongLen entries and more are somebody else's and not listed.
+template <typename CompT, typename ValT, typename OutT, int G, bool kList>
 __global__ void __launch_bounds__(128, 16) SpmvRowsKernel(const int32_t *__restrict__ rowPtr, const int32_t *__restrict__ colInd,
                                                           const ValT *__restrict__ val, const ValT *__restrict__ x,
                                                           OutT *__restrict__ y, int rows, Scalars<CompT> sc, RowList list)
@@ -1070,7 +1072,6 @@ __global__ void __launch_bounds__(128, 16) SpmvRowsKernel(const int32_t *__restr
     constexpr int kGroupMax = kGroupTrips * 4 * G;
     const int lane = threadIdx.x & 31, li = lane & (G - 1);
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     const long long r = ((long long)blockIdx.x * 128 + threadIdx.x) / G;
     int s = 0, e = 0;
     if (r < rows) {
@@ -1079,13 +1080,14 @@ __global__ void __launch_bounds__(128, 16) SpmvRowsKernel(const int32_t *__restr
     }
     const CompT beta = sc.Beta();
     const int len = e - s;
-    if (len > kListedRow && li == 0) {
+    if (kList && len > kListedRow && li == 0) {
         const int n = (len + kSegLen - 1) / kSegLen;
         const int at = atomicAdd(list.state, n);
         list.counters[at] = 0;
         for (int k = 0; k < n; ++k) list.items[at + k] = make_int2((int)r, k);
     }
-    const bool mine = r < rows && len <= kListedRow;
+    const bool mine = r < rows && (kList ? len <= kListedRow : len < kLongLen);
+    if (!mine) e = s;
     CompT yOld = CompT(0);
     if (mine && li == 0 && beta != CompT(0)) yOld = Widen<CompT>(y[r]);  // requested now, used at the end
     CompT sum = CompT(0);
@@ -1148,7 +1150,6 @@ __global__ void __launch_bounds__(256) SpmvListedKernel(const int32_t *__restric
     __shared__ int sCount;
     const int tid = threadIdx.x;
     b200sp::WaitForPrevious();
-    b200sp::AllowNext();
     const int count = *static_cast<volatile int32_t *>(list.state);
     if (count == 0) return;
     const CompT beta = sc.Beta();
@@ -1385,6 +1386,13 @@ int GroupWidthFor(int64_t rows, int64_t nnz)
     return G;
 }
 
+// Lanes per row of SpmvRowsKernel, which gives a row of up to 16 times as many entries to them.
+int RowsGroup(int64_t rows, int64_t nnz)
+{
+    const int64_t avg = rows > 0 ? nnz / rows : 0;
+    return avg <= 6 ? 2 : avg <= 28 ? 4 : avg <= 64 ? 8 : avg <= 128 ? 16 : 32;
+}
+
 // Binned plan in the caller's buffer: header, list of medium rows, list of long rows and, when
 // the matrix is narrow enough for the blocked long-row kernel, that kernel's tables.
 struct BinLayout {
@@ -1423,7 +1431,38 @@ enum { kInfoKind = 0, kInfoMedium = 1, kInfoLong = 2, kInfoGroup = 3, kInfoXBloc
        kInfoSegments = 7 };
 enum { kPlanTiles = 0, kPlanBinned = 1, kPlanBinnedBlocked = 2 };  // blocked: long rows go to SpmvLongBlockKernel
 
-template <typename CompT, typename ValT, typename OutT, bool kVec>
+// How SpmvLongBlockKernel shares out the long rows: groups of them, a CTA for each on every block of x (one CTA per SM at
+// most: it holds half of the SM's threads and a block of x), and lanes per piece.  With many blocks the groups are
+// few and large, and eight lanes per piece keep 128 pieces going; with few blocks a group is a handful of rows,
+// and more lanes share a piece.  Estimated per trip: about a microsecond, and a round trip to memory per eight entries
+// of a lane, for the 2048 entries a long row has on average.  (765,345 rows, one block of x, 5,000 long rows: 59 us
+// with eight lanes and 40 groups, 40 us with 32 lanes; 25,544 rows of mean 26: 40 and 10 us.)
+struct LongBlockShape {
+    int groups, lanes;
+};
+LongBlockShape LongBlockShapeFor(int xBlocks, int nLong)
+{
+    LongBlockShape best{1, 8};
+    int groups = b200sp_sm_count() / xBlocks;
+    groups = groups < 1 ? 1 : groups > kMaxLongGroups ? kMaxLongGroups : groups;
+    if (groups > nLong) groups = nLong;
+    const int rows = (nLong + groups - 1) / groups, piece = 2048 / xBlocks;
+    double least = 1e30;
+    for (int lanes : {8, 32, 256}) {
+        const int slots = kLongBlockThreads / lanes;
+        const double cost = ((rows + slots - 1) / slots) * (1.0 + 0.6 * ((piece + 8 * lanes - 1) / (8 * lanes)));
+        if (cost < least) {
+            least = cost;
+            best.lanes = lanes;
+        }
+    }
+    const int slots = kLongBlockThreads / best.lanes;
+    const int useful = (nLong + slots - 1) / slots;
+    best.groups = groups < useful ? groups : useful;
+    return best;
+}
+
+template <typename CompT, typename ValT, typename OutT, bool kVec, int kPieceLanes>
 int LaunchLongBlock(const LongBlockArgs<CompT, ValT, OutT> &la, int blocks, cudaStream_t stream)
 {
     constexpr int kSmem = kXBlockElems * (int)sizeof(ValT);
@@ -1431,12 +1470,12 @@ int LaunchLongBlock(const LongBlockArgs<CompT, ValT, OutT> &la, int blocks, cuda
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= b200sp::kMaxDevices) return (int)cudaErrorInvalidDevice;
     if (!configured[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(SpmvLongBlockKernel<CompT, ValT, OutT, kVec>,
+        const cudaError_t e = cudaFuncSetAttribute(SpmvLongBlockKernel<CompT, ValT, OutT, kVec, kPieceLanes>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
         if (e != cudaSuccess) return (int)e;
         configured[dev] = true;
     }
-    SpmvLongBlockKernel<CompT, ValT, OutT, kVec><<<(unsigned)blocks, kLongBlockThreads, kSmem, stream>>>(la);
+    SpmvLongBlockKernel<CompT, ValT, OutT, kVec, kPieceLanes><<<(unsigned)blocks, kLongBlockThreads, kSmem, stream>>>(la);
     b200sp_note_launches(1);
     return (int)cudaGetLastError();
 }
@@ -1503,16 +1542,14 @@ int LaunchBinned(const int32_t *rowPtr, const int32_t *colInd, const ValT *val, 
             la.partials = reinterpret_cast<CompT *>(p + L.offPartials);
             la.nLong = nL;
             la.xBlocks = L.xBlocks;
-            // one CTA per SM at most (it holds half of the SM's threads and a block of x)
-            constexpr int kPiecesPerCta = kLongBlockThreads / B200SP_SPMV_PIECE_LANES;
-            int groups = b200sp_sm_count() / L.xBlocks;
-            const int useful = (nL + kPiecesPerCta - 1) / kPiecesPerCta;
-            if (groups > useful) groups = useful;
-            if (groups > kMaxLongGroups) groups = kMaxLongGroups;
-            if (groups < 1) groups = 1;
-            la.groups = groups;
-            const int rcL = vec ? LaunchLongBlock<CompT, ValT, OutT, true>(la, L.xBlocks * groups, sL)
-                                : LaunchLongBlock<CompT, ValT, OutT, false>(la, L.xBlocks * groups, sL);
+            const LongBlockShape shape = LongBlockShapeFor(L.xBlocks, nL);
+            la.groups = shape.groups;
+            auto launchLong = [&]<int kPieceLanes>() {
+                return vec ? LaunchLongBlock<CompT, ValT, OutT, true, kPieceLanes>(la, L.xBlocks * la.groups, sL)
+                           : LaunchLongBlock<CompT, ValT, OutT, false, kPieceLanes>(la, L.xBlocks * la.groups, sL);
+            };
+            const int rcL = shape.lanes == 8 ? launchLong.template operator()<8>()
+                          : shape.lanes == 32 ? launchLong.template operator()<32>() : launchLong.template operator()<256>();
             if (rcL != 0) return rcL;
         } else {
             if (vec) SpmvLongListKernel<CompT, ValT, OutT, true><<<(unsigned)nS, 256, 0, sL>>>(colInd, val, x, y, ls, sc);
@@ -1528,6 +1565,12 @@ int LaunchBinned(const int32_t *rowPtr, const int32_t *colInd, const ValT *val, 
         constexpr int kWpc = kMsThreads / 32;
         const unsigned shortBlocks = (unsigned)((rows * G + kMsThreads - 1) / kMsThreads);
         auto launch = [&]<int GG>() {
+            // Where many rows are medium, a lane group that takes them too beats a warp each (fixed rows of 53 entries,
+            // 169,574 of them: 47 us with a warp, 38 with 8 lanes); where they are few (power-law rows, one in seventeen to eight),
+            // they start first and the lane groups stay narrow.
+            if (nM >= rows / 4)
+                return b200sp::LaunchChained(SpmvRowsKernel<CompT, ValT, OutT, GG, false>, (unsigned)((rows * GG + 127) / 128), 128, 0,
+                                             stream, rowPtr, colInd, val, x, y, (int)rows, sc, RowList{});
             if (nM > 0)
                 return b200sp::LaunchChained(SpmvMediumShortKernel<CompT, ValT, OutT, GG>,
                                              (unsigned)((nM + kWpc - 1) / kWpc) + shortBlocks, kMsThreads, 0, stream, rowPtr,
@@ -1536,7 +1579,9 @@ int LaunchBinned(const int32_t *rowPtr, const int32_t *colInd, const ValT *val, 
                                          rowPtr, colInd, val, x, y, (int)rows, sc);
         };
         cudaError_t rc = cudaSuccess;
-        switch (G) {
+        switch (nM >= rows / 4 ? RowsGroup(rows, nnz) : G) {
+            case 16: rc = launch.template operator()<16>(); break;
+            case 32: rc = launch.template operator()<32>(); break;
             case 2: rc = launch.template operator()<2>(); break;
             case 8: rc = launch.template operator()<8>(); break;
             default: rc = launch.template operator()<4>(); break;
@@ -1665,13 +1710,17 @@ int LaunchRows(const int32_t *rowPtr, const int32_t *colInd, const void *val, co
     if (rows == 0) return 0;
     auto launch = [&]<int G>() {
         b200sp_note_launches(1);
-        return b200sp::LaunchChained(SpmvRowsKernel<CompT, ValT, OutT, G>, (unsigned)((rows * G + 127) / 128), 128, 0, stream, rowPtr,
+        return b200sp::LaunchChained(SpmvRowsKernel<CompT, ValT, OutT, G, true>, (unsigned)((rows * G + 127) / 128), 128, 0, stream, rowPtr,
                                      colInd, v, xv, yv, (int)rows, sc, list);
     };
-    const int64_t avg = nnz / rows;
-    cudaError_t e = avg <= 6 ? launch.template operator()<2>() : avg <= 32 ? launch.template operator()<4>()
-                  : avg <= 64 ? launch.template operator()<8>() : avg <= 128 ? launch.template operator()<16>()
-                  : launch.template operator()<32>();
+    cudaError_t e;
+    switch (RowsGroup(rows, nnz)) {
+        case 2: e = launch.template operator()<2>(); break;
+        case 4: e = launch.template operator()<4>(); break;
+        case 8: e = launch.template operator()<8>(); break;
+        case 16: e = launch.template operator()<16>(); break;
+        default: e = launch.template operator()<32>(); break;
+    }
     if (e != cudaSuccess || nnz <= kListedRow) return (int)e;
     const int64_t most = nnz / (kListedRow + 1), cap = (int64_t)b200sp_sm_count() * 4;
     b200sp_note_launches(1);
