@@ -150,8 +150,7 @@ b200spScalars ReadScalars(const aclsparseContext *h, const void *alpha, const vo
     return s;
 }
 
-constexpr int32_t kTransPlan = 3;       // ActivePlan::spmvInfo[0] of a transposed-product analysis ([1] = longest row)
-constexpr int32_t kTransLongRow = 2048;  // a lane group walks at most this many entries of one row alone
+constexpr int32_t kTransPlan = 3;  // ActivePlan::spmvInfo[0] of a matrix preprocessed for the transposed product
 
 bool PlanMatches(const ActivePlan &p, const void *buffer, const aclsparseSpMatDescr *A)
 {
@@ -196,23 +195,15 @@ aclsparseStatus_t aclsparseSpMVPreprocess(aclsparseHandle_t handle, aclsparseOpe
     if (st != ACL_SPARSE_STATUS_SUCCESS) return st;
     if (externalBuffer == nullptr) return ACL_SPARSE_STATUS_INSUFFICIENT_RESOURCES;
     if (c.trans) {
-        // The scatter path only wants to know whether some row is far longer than a warp should walk alone.
+        // The scatter needs no analysis; the record keeps a plain product from taking this buffer for one of its own.
         ActivePlan t;
-        int32_t maxLen = 0;
         t.generation = b200sp::NoteBufferWrite(externalBuffer);
-        const int rcT = b200sp_spmv_max_row_length(static_cast<const int32_t *>(matA->offsets), matA->rows,
-                                                   externalBuffer, &maxLen, handle->stream);
-        if (rcT != 0) {
-            B200SP_LOGE("aclsparseSpMVPreprocess: analysis failed (cuda error %d)", rcT);
-            return ACL_SPARSE_STATUS_EXECUTION_FAILED;
-        }
         t.buffer = externalBuffer;
         t.kind = PlanKind::kSpmv;
         t.rowPtr = matA->offsets;
         t.rows = matA->rows;
         t.nnz = matA->nnz;
         t.spmvInfo[0] = kTransPlan;
-        t.spmvInfo[1] = maxLen;
         matA->active = t;
         return ACL_SPARSE_STATUS_SUCCESS;
     }
@@ -261,18 +252,16 @@ aclsparseStatus_t aclsparseSpMV(aclsparseHandle_t handle, aclsparseOperation_t o
                 return ACL_SPARSE_STATUS_INSUFFICIENT_RESOURCES;
             }
         }
-        // Preprocess'ed and a row of kTransLongRow entries or more: cut the scatter by non-zeros.  (A transposed
-        // plan is host-side knowledge only, so it survives the accumulator written into the buffer below.)
-        const bool byNnz = PlanMatches(matA->active, externalBuffer, matA) &&
-                           matA->active.spmvInfo[0] == kTransPlan && matA->active.spmvInfo[1] >= kTransLongRow;
-        // A 16-bit y accumulates in the buffer: whatever analysis any matrix had in it is gone.
+        // A 16-bit y accumulates in the buffer: whatever analysis any matrix had in it is gone.  (A transposed record is
+        // host-side knowledge only, so it survives.)
+        const bool mine = PlanMatches(matA->active, externalBuffer, matA) && matA->active.spmvInfo[0] == kTransPlan;
         if (scratch == externalBuffer && scratchBytes > 0) {
             const uint64_t gen = b200sp::NoteBufferWrite(externalBuffer);
-            if (byNnz) matA->active.generation = gen;
+            if (mine) matA->active.generation = gen;
         }
         rc = b200sp_spmv_trans_launch(rowPtr, colInd, matA->values, vecX->values, vecY->values, matA->rows,
                                       matA->cols, matA->nnz, &sc, c.compType, c.valType, c.outType, scratch,
-                                      scratchBytes, byNnz ? 1 : 0, stream);
+                                      scratchBytes, /*by_nnz=*/1, stream);
     } else {
         void *plan = nullptr;
         const int32_t *info = nullptr;
