@@ -758,7 +758,7 @@ def aux_arm(args, synth, oracle):
         ok = bool(np.all(np.abs(got - gold.astype(np.float64)) <= 1e-6 * scale + 1e-30))
         alg = synth.algorithmic_bytes_spmv(m, n, nnz, 4, 4, cfg["beta"])
         workload = {"workload": f"aclsparseSpMVOp ({args.op[-4:]}) on the c2 matrix", "rows": m, "nnz": nnz}
-        kernels = ("SpmvOpLongRowsKernel + SpmvOpRowsKernel per length class" if args.op.endswith("2") else "SpmvOpRowsKernel")
+        kernels = ("SpmvOpClassesKernel" if args.op.endswith("2") else "SpmvOpRowsKernel")
         plan.close()
     else:  # sddmm: the pattern of a 1 M-node power-law graph, X and Y^T of 256 fp16 per row (the backward of c5's layer)
         cfg = synth.config5(rows=1 << 20)

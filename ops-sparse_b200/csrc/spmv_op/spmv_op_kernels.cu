@@ -11,23 +11,24 @@
 // the same bits on every run; the final combination is the reference's.  With G = 1 the arithmetic
 // is the reference's, operation for operation.
 //
-// Two ways to pick G:
-//   no plan (ALG1)   one G for the whole matrix, from nnz / rows; nothing is analysed;
-//   plan (ALG2)      the analysis orders the rows by descending length class (class c: lengths that
-//                    need c bits); rows of 1024 entries and more get a CTA each, rows of 64 and more
-//                    a warp, the rest four lanes, longest rows first -- the
-//                    counterpart of the reference's reorder / bin_edge tables
-//                    (spmv_op_kernel.cpp:425-540), built here by a histogram and a scatter.
+// SpmvOpRowsKernel (ALG1, and ALG2 where row lengths are alike): rows up to 16 * G entries get G lanes, longer ones a
+// warp, in row order; G comes from the mean length.
+// SpmvOpClassesKernel (ALG2 on skewed lengths): the plan orders the rows by descending length class (class c: lengths that
+// need c bits; a histogram and a scatter, the counterpart of the reference's reorder / bin_edge tables,
+// spmv_op_kernel.cpp:425-540), and a class gets as many lanes per row as leave each of them four to eight entries; rows of
+// 512 entries and more get a CTA.  One grid, longest rows first.
 #include <cstdint>
 
 #include <cuda_runtime.h>
 
 #include "b200sp_kernels.h"
-#include "../common/side_stream.h"
+#include "../common/chained.cuh"
 
 namespace {
 
 constexpr int kClasses = B200SP_SPMVOP_CLASSES;
+constexpr int kLongBits = 10;  // rows of this many bits of length and more (512 entries) are long
+constexpr int kThreads = 128;
 
 inline size_t AlignUp(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -46,7 +47,6 @@ inline OpPlanLayout OpLayoutFor(int64_t rows)
 struct Triple {
     float hi, md, lo;
 };
-
 // One step of the reference recurrence (spmv_op_kernel.cpp:101-122).
 __device__ __forceinline__ void PriestStep(Triple &t, float val, float xv)
 {
@@ -95,128 +95,162 @@ struct OpArgs {
     const float *x;
     const float *y;
     float *z;
-    const int32_t *reorder;  // NULL: row i is row i
-    long long first;         // first position of this launch in the row sequence
-    long long count;         // positions in this launch
+    const int32_t *reorder;  // rows by descending length class (SpmvOpClassesKernel)
+    long long rows;
     int indexBase;
     float alpha, beta;
     const float *alphaDev, *betaDev;
 };
 
-template <int G, bool kIs64>
-__global__ void __launch_bounds__(256) SpmvOpRowsKernel(const OpArgs a)
+__device__ __forceinline__ float Combine(const Triple &t, float alpha, float betaY)  // spmv_op_kernel.cpp:172-176
 {
-    const float alpha = a.alphaDev ? *a.alphaDev : a.alpha;
-    const float beta = a.betaDev ? *a.betaDev : a.beta;
-    const int lane = threadIdx.x & (G - 1);
-    const long long groupsTotal = (long long)gridDim.x * blockDim.x / G;
-    const long long firstGroup = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / G;
-    // every lane of a warp makes the same number of trips, so the shuffles below are full-warp
-    const long long padded = (a.count + groupsTotal - 1) / groupsTotal * groupsTotal;
-    for (long long i = firstGroup; i < padded; i += groupsTotal) {
-        const bool live = i < a.count;
-        long long row = 0, s = 0, e = 0;
-        if (live) {
-            row = a.reorder ? (long long)a.reorder[a.first + i] : a.first + i;
-            s = LoadOffset(a.rowOffsets, kIs64, row) - a.indexBase;
-            e = LoadOffset(a.rowOffsets, kIs64, row + 1) - a.indexBase;
-        }
-        float yOld = 0.0f;
-        if (live && lane == 0 && beta != 0.0f) yOld = a.y[row];  // requested now, used at the end
-        Triple t{0.0f, 0.0f, 0.0f};
-        // Four entries are requested before the first of them is used; the steps run in entry order.
-        long long p = s + lane;
-        for (; p + 3 * G < e; p += 4 * G) {
-            float v[4], xv[4];
+    const float corr = __fadd_rn(t.md, t.lo);
+    return __fmaf_rn(alpha, t.hi, __fmaf_rn(alpha, corr, betaY));
+}
+
+// Entries first, first + step, ... below e, in that order; four are requested before the first of them is used.
+__device__ __forceinline__ Triple SumEntries(const OpArgs &a, long long first, long long e, int step)
+{
+    Triple t{0.0f, 0.0f, 0.0f};
+    for (long long p = first; p < e; p += 4 * step) {
+        int c[4];
+        float v[4], xv[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int col = __ldcs(a.colInd + p + u * G) - a.indexBase;
-                v[u] = __ldcs(a.val + p + u * G);
-                xv[u] = __ldg(a.x + col);
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) PriestStep(t, v[u], xv[u]);
-        }
-        for (; p < e; p += G) {
-            const int col = __ldcs(a.colInd + p) - a.indexBase;
-            PriestStep(t, __ldcs(a.val + p), __ldg(a.x + col));
+        for (int u = 0; u < 4; ++u) {
+            const bool in = p + u * step < e;
+            c[u] = in ? __ldcs(a.colInd + p + u * step) - a.indexBase : 0;
+            v[u] = in ? __ldcs(a.val + p + u * step) : 0.0f;
         }
 #pragma unroll
-        for (int off = G >> 1; off > 0; off >>= 1) {
-            Triple o;
-            o.hi = __shfl_down_sync(0xffffffffu, t.hi, off, G);
-            o.md = __shfl_down_sync(0xffffffffu, t.md, off, G);
-            o.lo = __shfl_down_sync(0xffffffffu, t.lo, off, G);
-            JoinTriples(t, o);  // lanes >= off of a group compute values nobody reads
+        for (int u = 0; u < 4; ++u) xv[u] = p + u * step < e ? __ldg(a.x + c[u]) : 0.0f;
+        // a step that no lane needs is branched over: rows are short, a step is some twenty instructions
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (u > 0 && !__any_sync(__activemask(), p + u * step < e)) break;
+            if (p + u * step < e) PriestStep(t, v[u], xv[u]);
         }
-        if (live && lane == 0) {
-            // spmv_op_kernel.cpp:172-176
-            const float corr = __fadd_rn(t.md, t.lo);
-            const float step1 = __fmaf_rn(alpha, corr, __fmul_rn(beta, yOld));
-            a.z[row] = __fmaf_rn(alpha, t.hi, step1);
-        }
+    }
+    return t;
+}
+template <int kLanes> __device__ __forceinline__ void JoinLanes(Triple &t)  // lane 0 of every group gets the sum
+{
+#pragma unroll
+    for (int off = kLanes >> 1; off > 0; off >>= 1) {
+        Triple o;
+        o.hi = __shfl_down_sync(0xffffffffu, t.hi, off, kLanes);
+        o.md = __shfl_down_sync(0xffffffffu, t.md, off, kLanes);
+        o.lo = __shfl_down_sync(0xffffffffu, t.lo, off, kLanes);
+        JoinTriples(t, o);  // lanes >= off of a group compute values nobody reads
     }
 }
 
-// Rows of kLongBits bits or more (1024 entries and up): one CTA per row.  Thread t runs the recurrence on
-// entries t, t + 256, ...; the lanes of a warp are joined on the butterfly, then warp 0 joins the eight
-// warp triples the same way: a fixed shape again.
-constexpr int kLongBits = 11;
+// A row per CTA: thread t runs the recurrence on entries t, t + kThreads, ...; the lanes of a warp are joined on the butterfly,
+// then warp 0 joins the warps' triples the same way: a fixed shape again.
 template <bool kIs64>
-__global__ void __launch_bounds__(256) SpmvOpLongRowsKernel(const OpArgs a)
+__device__ __forceinline__ void LongRow(const OpArgs &a, long long row, float alpha, float beta)
 {
-    __shared__ Triple sWarp[8];
-    const float alpha = a.alphaDev ? *a.alphaDev : a.alpha;
-    const float beta = a.betaDev ? *a.betaDev : a.beta;
+    __shared__ Triple sWarp[kThreads / 32];
     const int tid = threadIdx.x;
-    const long long row = a.reorder ? (long long)a.reorder[a.first + blockIdx.x] : a.first + blockIdx.x;
     const long long s = LoadOffset(a.rowOffsets, kIs64, row) - a.indexBase;
     const long long e = LoadOffset(a.rowOffsets, kIs64, row + 1) - a.indexBase;
     float yOld = 0.0f;
     if (tid == 0 && beta != 0.0f) yOld = a.y[row];
-    Triple t{0.0f, 0.0f, 0.0f};
-    long long p = s + tid;
-    for (; p + 3 * 256 < e; p += 4 * 256) {
-        float v[4], xv[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int col = __ldcs(a.colInd + p + u * 256) - a.indexBase;
-            v[u] = __ldcs(a.val + p + u * 256);
-            xv[u] = __ldg(a.x + col);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) PriestStep(t, v[u], xv[u]);
-    }
-    for (; p < e; p += 256) {
-        const int col = __ldcs(a.colInd + p) - a.indexBase;
-        PriestStep(t, __ldcs(a.val + p), __ldg(a.x + col));
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        Triple o;
-        o.hi = __shfl_down_sync(0xffffffffu, t.hi, off);
-        o.md = __shfl_down_sync(0xffffffffu, t.md, off);
-        o.lo = __shfl_down_sync(0xffffffffu, t.lo, off);
-        JoinTriples(t, o);
-    }
+    Triple t = SumEntries(a, s + tid, e, kThreads);
+    JoinLanes<32>(t);
     if ((tid & 31) == 0) sWarp[tid >> 5] = t;
     __syncthreads();
     if (tid < 32) {
-        Triple w = tid < 8 ? sWarp[tid] : Triple{0.0f, 0.0f, 0.0f};
-#pragma unroll
-        for (int off = 4; off > 0; off >>= 1) {
-            Triple o;
-            o.hi = __shfl_down_sync(0xffffffffu, w.hi, off);
-            o.md = __shfl_down_sync(0xffffffffu, w.md, off);
-            o.lo = __shfl_down_sync(0xffffffffu, w.lo, off);
-            JoinTriples(w, o);
-        }
-        if (tid == 0) {
-            const float corr = __fadd_rn(w.md, w.lo);
-            const float step1 = __fmaf_rn(alpha, corr, __fmul_rn(beta, yOld));
-            a.z[row] = __fmaf_rn(alpha, w.hi, step1);
-        }
+        Triple w = tid < kThreads / 32 ? sWarp[tid] : Triple{0.0f, 0.0f, 0.0f};
+        JoinLanes<kThreads / 32>(w);
+        if (tid == 0) a.z[row] = Combine(w, alpha, __fmul_rn(beta, yOld));
     }
+}
+
+// Light on registers and without barriers: it lives on warps in flight (the gathers of x go to L2, one sector per clock and
+// SM).  CTAs of 128 threads: 466,673 rows of 51 entries 69 us, with 256 threads 78.
+template <int G, bool kIs64>
+__global__ void __launch_bounds__(kThreads, 12) SpmvOpRowsKernel(const OpArgs a)
+{
+    b200sp::WaitForPrevious();
+    const float alpha = a.alphaDev ? *a.alphaDev : a.alpha;
+    const float beta = a.betaDev ? *a.betaDev : a.beta;
+    const int lane = threadIdx.x & 31, li = lane & (G - 1);
+    const long long row = ((long long)blockIdx.x * kThreads + threadIdx.x) / G;
+    const bool mine = row < a.rows;
+    long long s = 0, e = 0;
+    if (mine) {
+        s = LoadOffset(a.rowOffsets, kIs64, row) - a.indexBase;
+        e = LoadOffset(a.rowOffsets, kIs64, row + 1) - a.indexBase;
+    }
+    const bool wide = e - s > 16 * G;
+    float yOld = 0.0f;
+    if (mine && li == 0 && beta != 0.0f) yOld = a.y[row];  // requested now, used at the end
+    Triple t{0.0f, 0.0f, 0.0f};
+    if (!wide) t = SumEntries(a, s + li, e, G);
+    JoinLanes<G>(t);
+    unsigned todo = __ballot_sync(0xffffffffu, wide && li == 0);
+    while (todo != 0) {
+        const int owner = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const long long ws = __shfl_sync(0xffffffffu, s, owner), we = __shfl_sync(0xffffffffu, e, owner);
+        Triple w = SumEntries(a, ws + lane, we, 32);
+        JoinLanes<32>(w);
+        w.hi = __shfl_sync(0xffffffffu, w.hi, 0);
+        w.md = __shfl_sync(0xffffffffu, w.md, 0);
+        w.lo = __shfl_sync(0xffffffffu, w.lo, 0);
+        if (lane == owner) t = w;
+    }
+    if (mine && li == 0) a.z[row] = Combine(t, alpha, __fmul_rn(beta, yOld));
+}
+
+// Places first .. first + count of the row order, from block firstBlock on, with G lanes per row (0: a CTA).
+struct Range {
+    int firstBlock, first, count;
+};
+// long rows; 128 to 511 entries; 64 to 127; 32 to 63; 16 to 31; 4 to 15; up to 3
+constexpr int kRanges = 7;
+constexpr int kRangeLanes[kRanges] = {0, 32, 16, 8, 4, 2, 1};
+constexpr int kRangeBits[kRanges] = {kLongBits, 8, 7, 6, 5, 3, 0};  // fewest bits of a length in the range
+struct Ranges {
+    Range r[kRanges];
+};
+
+template <int G, bool kIs64>
+__device__ __forceinline__ void ClassRow(const OpArgs &a, const Range &range, float alpha, float beta)
+{
+    const int li = threadIdx.x & (G - 1);
+    const int i = ((int)blockIdx.x - range.firstBlock) * (kThreads / G) + (int)threadIdx.x / G;
+    const bool mine = i < range.count;
+    long long row = 0, s = 0, e = 0;
+    if (mine) {
+        row = a.reorder[range.first + i];
+        s = LoadOffset(a.rowOffsets, kIs64, row) - a.indexBase;
+        e = LoadOffset(a.rowOffsets, kIs64, row + 1) - a.indexBase;
+    }
+    float yOld = 0.0f;
+    if (mine && li == 0 && beta != 0.0f) yOld = a.y[row];
+    Triple t = SumEntries(a, s + li, e, G);
+    JoinLanes<G>(t);
+    if (mine && li == 0) a.z[row] = Combine(t, alpha, __fmul_rn(beta, yOld));
+}
+
+// 31.2 M entries in 1 M power-law rows: a warp per row from 64 entries and four lanes below, long rows on a side stream:
+// 165 us; 133 us so.  The long rows wait for their gathers (L2 delivers one sector per clock and SM), the others
+// for issue slots: an entry is some twenty instructions and a join of two lanes' sums as many, so lanes must not idle.
+template <bool kIs64>
+__global__ void __launch_bounds__(kThreads, 12) SpmvOpClassesKernel(const OpArgs a, const Ranges ranges)
+{
+    b200sp::WaitForPrevious();
+    const float alpha = a.alphaDev ? *a.alphaDev : a.alpha;
+    const float beta = a.betaDev ? *a.betaDev : a.beta;
+    const int b = blockIdx.x;
+    if (b < ranges.r[1].firstBlock) LongRow<kIs64>(a, a.reorder[b], alpha, beta);
+    else if (b < ranges.r[2].firstBlock) ClassRow<32, kIs64>(a, ranges.r[1], alpha, beta);
+    else if (b < ranges.r[3].firstBlock) ClassRow<16, kIs64>(a, ranges.r[2], alpha, beta);
+    else if (b < ranges.r[4].firstBlock) ClassRow<8, kIs64>(a, ranges.r[3], alpha, beta);
+    else if (b < ranges.r[5].firstBlock) ClassRow<4, kIs64>(a, ranges.r[4], alpha, beta);
+    else if (b < ranges.r[6].firstBlock) ClassRow<2, kIs64>(a, ranges.r[5], alpha, beta);
+    else ClassRow<1, kIs64>(a, ranges.r[6], alpha, beta);
 }
 
 __global__ void SpmvOpScaleKernel(const float *__restrict__ y, float *__restrict__ z, long long rows, float beta,
@@ -283,26 +317,35 @@ __global__ void SpmvOpScatterKernel(const void *rowOffsets, long long rows, int3
     }
 }
 
-// Lanes for rows whose length needs `bits` bits.  Two ranges only: a launch per class of short rows cost
-// 15 us each for a few hundred thousand entries (five launches, 81 us on the power-law matrix).
-inline int LanesForClass(int bits) { return bits >= 7 ? 32 : 4; }  // 64 entries and more: a warp per row
-
 template <bool kIs64>
-void LaunchRows(const OpArgs &a, int G, cudaStream_t st)
+cudaError_t LaunchRows(const OpArgs &a, double mean, cudaStream_t st)
 {
-    if (a.count <= 0) return;
-    const long long want = (a.count * G + 255) / 256;
-    const long long cap = (long long)b200sp_sm_count() * 64;
-    const unsigned blocks = (unsigned)(want < cap ? want : cap);
-    switch (G) {
-        case 1: SpmvOpRowsKernel<1, kIs64><<<blocks, 256, 0, st>>>(a); break;
-        case 2: SpmvOpRowsKernel<2, kIs64><<<blocks, 256, 0, st>>>(a); break;
-        case 4: SpmvOpRowsKernel<4, kIs64><<<blocks, 256, 0, st>>>(a); break;
-        case 8: SpmvOpRowsKernel<8, kIs64><<<blocks, 256, 0, st>>>(a); break;
-        case 16: SpmvOpRowsKernel<16, kIs64><<<blocks, 256, 0, st>>>(a); break;
-        default: SpmvOpRowsKernel<32, kIs64><<<blocks, 256, 0, st>>>(a); break;
+    auto launch = [&]<int G>() {
+        b200sp_note_launches(1);
+        return b200sp::LaunchChained(SpmvOpRowsKernel<G, kIs64>, (unsigned)((a.rows * G + kThreads - 1) / kThreads), kThreads, 0, st, a);
+    };
+    // lanes for which rows of the mean length give each of them four to eight entries: fewer idle the memory, more the lanes
+    if (mean <= 6) return launch.template operator()<2>();
+    if (mean <= 28) return launch.template operator()<4>();
+    if (mean <= 64) return launch.template operator()<8>();
+    if (mean <= 128) return launch.template operator()<16>();
+    return launch.template operator()<32>();
+}
+
+// Entries in rows four times as long as the mean and longer, as a share: from the classes, whose lengths lie between
+// 2^(c-1) and 2^c - 1.  Ragged rows (up to twice the mean) have none, power-law rows more than half.  Below 15 % the rows
+// in their own order win: their offsets and results coalesce, and the few long ones cost less than the indirection.
+bool Skewed(const int32_t *class_start, double mean)
+{
+    double all = 0.0, heavy = 0.0;
+    for (int i = 0; i < kClasses; ++i) {
+        const int c = kClasses - 1 - i;
+        if (c == 0) continue;
+        const double entries = (class_start[i + 1] - class_start[i]) * 0.75 * (double)(1ll << c);
+        all += entries;
+        if ((double)(1ll << (c - 1)) >= 4 * mean) heavy += entries;
     }
-    b200sp_note_launches(1);
+    return heavy > 0.15 * all;
 }
 
 }  // namespace
@@ -375,52 +418,24 @@ int b200sp_spmvop_launch(const void *row_offsets, int offsets_are_64, const int3
     a.beta = beta;
     a.alphaDev = alpha_dev;
     a.betaDev = beta_dev;
-    if (plan == nullptr || class_start == nullptr) {
-        a.reorder = nullptr;
-        a.first = 0;
-        a.count = rows;
-        const long long avg = nnz / rows;
-        int G = 1;
-        while (G < 32 && 4 * G < avg) G <<= 1;
-        if (offsets_are_64) LaunchRows<true>(a, G, st);
-        else LaunchRows<false>(a, G, st);
-        return (int)cudaGetLastError();
-    }
     a.reorder = static_cast<const int32_t *>(plan);
-    // Classes of kLongBits bits and more: a CTA per row.
-    int k = kClasses - kLongBits;  // class_start index of class kLongBits - 1
-    a.first = class_start[0];
-    a.count = (long long)class_start[k] - class_start[0];
-    // The rows of the ranges are disjoint, so the long-row grid goes onto the side stream and runs beside the
-    // other ranges (each of them is bound by latency, not by a throughput the others would take away).
-    b200sp::SideLanes *lanes = nullptr;
-    if (a.count > 0) {
-        cudaStream_t sL = st;
-        lanes = b200sp::GetSideLanes();
-        if (lanes != nullptr) {
-            if (cudaEventRecord(lanes->fork, st) != cudaSuccess ||
-                cudaStreamWaitEvent(lanes->stream[0], lanes->fork, 0) != cudaSuccess)
-                return (int)cudaGetLastError();
-            sL = lanes->stream[0];
-        }
-        if (offsets_are_64) SpmvOpLongRowsKernel<true><<<(unsigned)a.count, 256, 0, sL>>>(a);
-        else SpmvOpLongRowsKernel<false><<<(unsigned)a.count, 256, 0, sL>>>(a);
-        b200sp_note_launches(1);
-        if (lanes != nullptr && cudaEventRecord(lanes->join[0], sL) != cudaSuccess) return (int)cudaGetLastError();
+    a.rows = rows;
+    const double mean = (double)nnz / (double)rows;
+    if (plan == nullptr || class_start == nullptr || !Skewed(class_start, mean))
+        return (int)(offsets_are_64 ? LaunchRows<true>(a, mean, st) : LaunchRows<false>(a, mean, st));
+    Ranges ranges;
+    long long blocks = 0;
+    for (int i = 0; i < kRanges; ++i) {
+        Range &r = ranges.r[i];
+        r.firstBlock = (int)blocks;
+        r.first = i == 0 ? 0 : ranges.r[i - 1].first + ranges.r[i - 1].count;
+        r.count = class_start[kClasses - kRangeBits[i]] - r.first;
+        const int perBlock = kRangeLanes[i] == 0 ? 1 : kThreads / kRangeLanes[i];
+        blocks += (r.count + perBlock - 1) / perBlock;
     }
-    // Then one launch per run of classes that share a lane count, longest rows first.
-    while (k < kClasses) {
-        const int G = LanesForClass(kClasses - 1 - k);
-        int k2 = k;
-        while (k2 < kClasses && LanesForClass(kClasses - 1 - k2) == G) ++k2;
-        a.first = class_start[k];
-        a.count = (long long)class_start[k2] - class_start[k];
-        if (offsets_are_64) LaunchRows<true>(a, G, st);
-        else LaunchRows<false>(a, G, st);
-        k = k2;
-    }
-    if (lanes != nullptr && cudaStreamWaitEvent(st, lanes->join[0], 0) != cudaSuccess) return (int)cudaGetLastError();
-    return (int)cudaGetLastError();
+    b200sp_note_launches(1);
+    return (int)(offsets_are_64 ? b200sp::LaunchChained(SpmvOpClassesKernel<true>, (unsigned)blocks, kThreads, 0, st, a, ranges)
+                                : b200sp::LaunchChained(SpmvOpClassesKernel<false>, (unsigned)blocks, kThreads, 0, st, a, ranges));
 }
 
 int b200sp_spmvop_scale(const float *y, float *z, int64_t rows, float beta, const float *beta_dev, void *stream)
