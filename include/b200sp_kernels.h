@@ -184,6 +184,7 @@ typedef struct b200spSpmmShape {
     int32_t long_rows;  /* from b200sp_spmm_analyze_blocks: rows the analysis listed as long */
     int64_t repack_bytes; /* bytes of the plan buffer beyond b200sp_spmm_plan_bytes that a repacked B may use
                            * (b200sp_spmm_repack_bytes), 0 = none */
+    int32_t mid_units;  /* from b200sp_spmm_analyze_units; 0 = rows of up to 1024 entries are all treated alike */
 } b200spSpmmShape;
 
 /* Bytes of workspace for the SpMM analysis + long-row partial sums. */
@@ -195,8 +196,12 @@ size_t b200sp_spmm_plan_bytes(int64_t rows, int64_t nnz, int64_t n);
 size_t b200sp_spmm_repack_bytes(const b200spSpmmShape *shape, int val_type);
 
 /* Analysis pass: finds rows too long for one warp, cuts them into segments and writes
- * the segment table into `plan`.  This call synchronises `stream` once to read back
- * the segment count (4 bytes), returned in *segments. */
+ * the segment table into `plan`, and lists the rows that are better summed apart from
+ * their neighbours.  This call synchronises `stream` once to read back the two counts,
+ * returned in *segments and *mid_units. */
+int b200sp_spmm_analyze_units(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,
+                              size_t plan_bytes, int32_t *segments, int32_t *mid_units, void *stream);
+/* The same without the second count. */
 int b200sp_spmm_analyze(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,
                         size_t plan_bytes, int32_t *segments, void *stream);
 

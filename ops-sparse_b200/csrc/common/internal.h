@@ -58,6 +58,7 @@ struct ActivePlan {
     int64_t nnz = 0;
     int64_t n = 0;         // SpMM only: dense column count the partial-sum area was sized for
     int32_t segments = 0;  // SpMM only: long-row segments found by the analysis
+    int32_t midUnits = 0;  // SpMM only: shorter rows summed apart from their neighbours
     int32_t blockUnits = 0;  // SpMM only: units of the column-block path for the long rows (0 = summed by segments)
     int32_t longRows = 0;   // SpMM only: rows listed as long
     const void *colInd = nullptr;  // SpMM with column blocks: the cut table was made from these column indices

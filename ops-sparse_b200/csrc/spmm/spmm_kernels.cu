@@ -11,12 +11,12 @@
 // bit-identical to the golden.
 //
 // Row-length routing (the analysis pass fills the workspace):
-//     rows <= 1024 non-zeros            -> one lane group per row;
-//     longer rows                       -> cut into segments of 4096 non-zeros, one CTA
-//                                          (4 warps) per segment.  A row of several
-//                                          segments is completed by whichever segment CTA
-//                                          finishes last: it adds the stored partial rows in
-//                                          segment order, so no CTA ever waits and the sum
+//     ordinary rows                     -> one lane group per row;
+//     longer ones (MidRowLimit)         -> a unit each, rows above 1024 non-zeros one per 1024 of them.  The fp kernels
+//                                          give a unit a warp per 64 bytes of a B row, which keeps some fifty
+//                                          entries in flight and sums them in CSR order all the same (UnitSum); int8
+//                                          a CTA.  A row of several units is completed by whichever comes last: it
+//                                          adds the stored partial rows in order, so nobody ever waits and the sum
 //                                          order is fixed.
 // The kernels want contiguous, 16-byte aligned rows of B.  A B in any other layout (column-major, odd N or
 // ldb) is first repacked into such rows in the caller's buffer (SpmmRepack*Kernel); a C that is column-major
@@ -36,6 +36,7 @@
 #include <cuda_runtime.h>
 
 #include "b200sp_kernels.h"
+#include "../common/chained.cuh"
 #include "../common/side_stream.h"
 
 namespace {
@@ -45,16 +46,15 @@ namespace {
 #endif
 constexpr int kThreads = B200SP_SPMM_THREADS;  // warps of a CTA: one lane-group set each, or one long-row segment
 constexpr int kWarps = kThreads / 32;
-constexpr int kLongRow = 1024;          // rows longer than this are handled by segment CTAs
-constexpr int kSegNnz = 4096;           // non-zeros per segment
-constexpr int kWarpSegNnz = kSegNnz / kWarps;
+constexpr int kLongRow = 1024;          // rows longer than this are cut
+constexpr int kSegNnz = 1024;           // non-zeros per unit of theirs
 
 inline size_t AlignUp(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 struct SegEntry {
     int32_t row;
-    int32_t seg;      // index of this segment inside its row
-    int32_t longIdx;  // index into the long-row table
+    int32_t seg;      // index of this unit inside its row
+    int32_t longIdx;  // index into the long-row table, -1: the unit is the whole row
     int32_t pad;
 };
 struct LongRow {
@@ -78,23 +78,36 @@ constexpr int kBlockMinRowBytes = 512;            // B rows narrower than a warp
 #endif
 constexpr int kUnitNnz = B200SP_SPMM_UNIT_NNZ;   // a (row, block) piece longer than this is cut into several units
 
+// Rows longer than this are summed apart from their neighbours: a lane group has four entries in flight and lets the
+// other groups of its warp wait.  Four times the mean leaves rows of like lengths together; where the rows do not fill
+// the SMs anyway every row of more than a few entries is better off as a unit.
+// 2,759 power-law rows of up to 4,245 entries, bf16, N = 12: 216 us with the limit at 1024, 19 us so; 597,812 rows of
+// up to 16,384, N = 16: 694 and 362 us.
+inline int MidRowLimit(int64_t rows, int64_t nnz, int64_t n)
+{
+    if (rows * n < 148ll * 2048) return 16;
+    const int64_t four = 4 * (nnz / (rows > 0 ? rows : 1));
+    return (int)(four < 64 ? 64 : four > kLongRow ? kLongRow : four);
+}
+
 struct PlanLayout {
     int64_t capLong, capSegs, capBlockSlots;
     size_t offCounts, offLong, offSegs, offCounters, offPartials;
     size_t offCuts, offRowSlots, offBlockCounters, offBlockMeta, offUnits, offBlockPartials, total;
 };
 
+inline int64_t ArrivalsPerRow(int64_t n) { return (n + 15) / 16; }  // slices of 64 bytes in a B row, at most
+
 inline PlanLayout LayoutFor(int64_t rows, int64_t nnz, int64_t n)
 {
-    (void)rows;
     PlanLayout L;
     L.capLong = nnz / (kLongRow + 1) + 1;
-    L.capSegs = nnz / kSegNnz + L.capLong + 1;
+    L.capSegs = nnz / kSegNnz + L.capLong + nnz / (MidRowLimit(rows, nnz, n) + 1) + 1;
     L.offCounts = 0;
     L.offLong = 256;
     L.offSegs = AlignUp(L.offLong + sizeof(LongRow) * (size_t)L.capLong, 256);
     L.offCounters = AlignUp(L.offSegs + sizeof(SegEntry) * (size_t)L.capSegs, 256);
-    L.offPartials = AlignUp(L.offCounters + sizeof(int32_t) * (size_t)L.capLong, 256);
+    L.offPartials = AlignUp(L.offCounters + sizeof(int32_t) * (size_t)(L.capLong * ArrivalsPerRow(n)), 256);
     // Only rows of two or more segments store partial rows; those have > kSegNnz entries.
     const int64_t capPartialSegs = 2 * (nnz / kSegNnz) + 1;
     L.offCuts = AlignUp(L.offPartials + sizeof(float) * (size_t)capPartialSegs * (size_t)n, 256);
@@ -246,19 +259,23 @@ __device__ __forceinline__ OutT Finish(int32_t acc, int32_t alpha, int32_t beta,
 
 // ---------------------------------------------------------------- analysis
 
-__global__ void SpmmFindLongRowsKernel(const int32_t *__restrict__ rowPtr, int rows, int32_t *counts,
+__global__ void SpmmFindLongRowsKernel(const int32_t *__restrict__ rowPtr, int rows, int limit, int arrivals, int capSegs, int32_t *counts,
                                        LongRow *longRows, SegEntry *segs, int32_t *counters)
 {
     for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < rows;
          r += (long long)gridDim.x * blockDim.x) {
         const int len = rowPtr[r + 1] - rowPtr[r];
-        if (len <= kLongRow) continue;
+        if (len <= limit) continue;
+        if (len <= kLongRow) {
+            segs[capSegs - 1 - atomicAdd(&counts[5], 1)] = {(int32_t)r, 0, -1, 0};
+            continue;
+        }
         const int nseg = (len + kSegNnz - 1) / kSegNnz;
         const int li = atomicAdd(&counts[0], 1);
         const int sb = atomicAdd(&counts[1], nseg);
-        const int pb = nseg > 1 ? atomicAdd(&counts[2], nseg) : 0;
+        const int pb = atomicAdd(&counts[2], nseg);
         longRows[li] = {(int32_t)r, sb, nseg, pb};
-        counters[li] = 0;
+        for (int s = 0; s < arrivals; ++s) counters[(long long)li * arrivals + s] = 0;
         for (int s = 0; s < nseg; ++s) segs[sb + s] = {(int32_t)r, s, li, 0};
     }
 }
@@ -409,11 +426,17 @@ struct FastArgs {
     long long cRow, cCol;
     unsigned long long negZeros;
     typename Arith<ValT>::Scalars sc;
-    int nsegs;
+    int rowLimit;         // longer rows are units
+    int longUnits;        // units of rows above kLongRow, from the front of the table, ...
+    int nUnits;           // ... then those of one row each, from its end
+    int unitCtas;         // CTAs at the front of the grid that work on them
+    int slices;           // fp: warps a unit takes, 64 bytes of a B row each
     int splitRows;        // int8 only: a CTA per row
+    int genRows;          // column-major C: rows of a CTA
     const LongRow *longRows;
-    const SegEntry *segs;
-    int32_t *counters;
+    const SegEntry *segs, *segsEnd;
+    int32_t *counters;    // [long row][ArrivalsPerRow]
+    int arrivals;
     void *partials;       // [partial slot][n] of the accumulator's type
 };
 
@@ -453,40 +476,50 @@ __device__ __forceinline__ void AccumulateKahan(float v, float b, float &acc, fl
 
 // Adds sum_{p in [s, e)} val[p] * B[col[p], slice] to acc, p ascending.  The kLanes lanes of a
 // group call it together with the same s, e (groups of one warp may differ); `trips` is the
-// warp-uniform number of kLanes-wide chunks to walk (>= this group's own need).  A lane whose columns lie past the
-// end of the row (colLive false) loads nothing; what it accumulates is never stored.
+// warp-uniform number of kChunk-wide chunks to walk (>= this group's own need).
 #ifndef B200SP_SPMM_BATCH
 #define B200SP_SPMM_BATCH 4
 #endif
+template <int kLanes> struct Chunk {
+    static constexpr int kHold = kLanes >= 8 ? 1 : 8 / kLanes;  // entries a lane holds, so that narrow groups have work in flight
+    static constexpr int kChunk = kLanes * kHold;
+};
 
 template <typename ValT, bool kKahan, int kLanes>
 __device__ __forceinline__ void RowDot(const int32_t *__restrict__ colInd, const ValT *__restrict__ val,
                                        const ValT *__restrict__ Bslice, long long ldb, int s, int e, int trips,
-                                       bool colLive, bool allColsLive, unsigned long long negZeros, float (&acc)[Pack<ValT>::kElems],
+                                       unsigned long long negZeros, float (&acc)[Pack<ValT>::kElems],
                                        float (&comp)[Pack<ValT>::kElems])
 {
     constexpr int E = Pack<ValT>::kElems;
-    constexpr int kBatch = kLanes < B200SP_SPMM_BATCH ? kLanes : B200SP_SPMM_BATCH;  // B rows in flight per lane
+    constexpr int kHold = Chunk<kLanes>::kHold;
+    constexpr int kChunk = Chunk<kLanes>::kChunk;
+    constexpr int kBatch = kChunk < B200SP_SPMM_BATCH ? kChunk : B200SP_SPMM_BATCH;  // B rows in flight per lane
     const int li = threadIdx.x & (kLanes - 1);
     for (int chunk = 0; chunk < trips; ++chunk) {
-        const int p0 = s + chunk * kLanes;
+        const int p0 = s + chunk * kChunk;
         const int rem = e - p0;  // entries of this group's row left; <= 0 once the row is done
-        int myCol = 0;
-        float myVal = 0.0f;
-        if (li < rem) {
-            myCol = __ldcs(colInd + p0 + li);
-            myVal = ToF32(__ldcs(val + p0 + li));
-        }
-        // Whole warp on full chunks and live columns: straight-line code, no predicate per entry.
-        if (allColsLive && __all_sync(0xffffffffu, rem >= kLanes)) {
+        int myCol[kHold];
+        float myVal[kHold];
 #pragma unroll
-            for (int q0 = 0; q0 < kLanes; q0 += kBatch) {
+        for (int h = 0; h < kHold; ++h) {
+            myCol[h] = 0;
+            myVal[h] = 0.0f;
+            if (h * kLanes + li < rem) {
+                myCol[h] = __ldcs(colInd + p0 + h * kLanes + li);
+                myVal[h] = ToF32(__ldcs(val + p0 + h * kLanes + li));
+            }
+        }
+        // Whole warp on full chunks: straight-line code, no predicate per entry.
+        if (__all_sync(0xffffffffu, rem >= kChunk)) {
+#pragma unroll
+            for (int q0 = 0; q0 < kChunk; q0 += kBatch) {
                 uint4 q[kBatch];
                 float v[kBatch];
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u) {
-                    const int c = __shfl_sync(0xffffffffu, myCol, q0 + u, kLanes);
-                    v[u] = __shfl_sync(0xffffffffu, myVal, q0 + u, kLanes);
+                    const int c = __shfl_sync(0xffffffffu, myCol[(q0 + u) / kLanes], (q0 + u) % kLanes, kLanes);
+                    v[u] = __shfl_sync(0xffffffffu, myVal[(q0 + u) / kLanes], (q0 + u) % kLanes, kLanes);
                     q[u] = LoadB16(Bslice + (long long)c * ldb);
                 }
 #pragma unroll
@@ -506,16 +539,16 @@ __device__ __forceinline__ void RowDot(const int32_t *__restrict__ colInd, const
         // Entries past the end of this group's row count as 0 * 0: adding +0 to a sum that began at +0 changes no
         // bit of it.  (The compensated sum is not indifferent to zeros and skips them.)
 #pragma unroll
-        for (int q0 = 0; q0 < kLanes; q0 += kBatch) {
+        for (int q0 = 0; q0 < kChunk; q0 += kBatch) {
             if (!__any_sync(0xffffffffu, q0 < rem)) break;
             uint4 q[kBatch];
             float v[kBatch];
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
-                const int c = __shfl_sync(0xffffffffu, myCol, q0 + u, kLanes);
-                v[u] = __shfl_sync(0xffffffffu, myVal, q0 + u, kLanes);
+                const int c = __shfl_sync(0xffffffffu, myCol[(q0 + u) / kLanes], (q0 + u) % kLanes, kLanes);
+                v[u] = __shfl_sync(0xffffffffu, myVal[(q0 + u) / kLanes], (q0 + u) % kLanes, kLanes);
                 q[u] = make_uint4(0, 0, 0, 0);
-                LoadB16If(colLive && q0 + u < rem, Bslice + (long long)c * ldb, q[u]);
+                LoadB16If(q0 + u < rem, Bslice + (long long)c * ldb, q[u]);
             }
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
@@ -638,13 +671,188 @@ __device__ __forceinline__ void StoreRowSlice(OutT *dst, const int32_t (&acc)[16
     }
 }
 
+__device__ __forceinline__ void CopyAsync16(void *dst, const void *src, bool on)  // zeros where not `on`
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(on ? 16 : 0) : "memory");
+}
+
+// A unit: a row of up to kLongRow entries, or that many of a longer one.  A warp sums kPieces * 16 bytes of the B rows of
+// its entries, in CSR order.  What bounds it is the latency of the gathers: they come through shared memory by cp.async,
+// kStages rounds in flight, requested by all lanes whatever the number of columns; the columns and values of a round are
+// loaded kStages rounds before its request.  Then lane l adds up word l of the B rows, one entry after the other.
+// 64 bytes per warp at most: wide rows are shared by more warps, and the shared memory (some 18 KB a CTA) leaves the
+// ordinary rows of the same grid their occupancy.
+template <int kLanes> struct UnitShape {
+    static constexpr int kPieces = kLanes < 4 ? kLanes : 4;
+    static constexpr int kRound = kPieces == 4 ? 16 : 32;            // entries per round
+    static constexpr int kStages = 4;
+    static constexpr int kCopies = kRound * kPieces / 32;            // of a lane per round
+    static constexpr int kStageBytes = kRound * kPieces * 16;
+    static constexpr int kWarpBytes = kStages * (kStageBytes + kRound * 4);
+};
+
+template <typename ValT, typename OutT, bool kKahan, int kLanes>
+__device__ void UnitSum(const FastArgs<ValT, OutT> &a, unsigned char *sWarp)
+{
+    using Shape = UnitShape<kLanes>;
+    constexpr int kPieces = Shape::kPieces, kRound = Shape::kRound, kStages = Shape::kStages, kCopies = Shape::kCopies;
+    constexpr int E = Pack<ValT>::kElems;
+    constexpr int kCols = 4 / (int)sizeof(ValT);  // columns of a word
+    const int lane = threadIdx.x & 31;
+    const long long at = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
+    const int unit = (int)(at / a.slices), slice = (int)(at - (long long)unit * a.slices);
+    if (unit >= a.nUnits) return;
+    const SegEntry seg = unit < a.longUnits ? a.segs[unit] : a.segsEnd[a.longUnits - 1 - unit];
+    const int rowEnd = a.rowPtr[seg.row + 1];
+    const int s = a.rowPtr[seg.row] + seg.seg * kSegNnz;
+    const int length = rowEnd - s > kSegNnz ? kSegNnz : rowEnd - s;
+    const int rounds = (length + kRound - 1) / kRound;
+    unsigned char *sData = sWarp;                                                                     // [kStages][kStageBytes]
+    float *sVal = reinterpret_cast<float *>(sWarp + kStages * Shape::kStageBytes);                    // [kStages][kRound]
+    const int piece = lane & (kPieces - 1);
+    const bool live = (slice * kPieces + piece) * E < a.nB;
+    const ValT *Bs = a.B + (live ? (slice * kPieces + piece) * E : 0);
+
+    struct Batch {  // of kStages rounds; lane l holds entry l of each
+        int col[kStages];
+        float val[kStages];
+    };
+    auto load = [&](Batch &b, int round0) {
+#pragma unroll
+        for (int i = 0; i < kStages; ++i) {
+            const int p = (round0 + i) * kRound + lane;
+            const bool in = lane < kRound && p < length;
+            b.col[i] = in ? __ldcs(a.colInd + s + p) : 0;
+            b.val[i] = in ? ToF32(__ldcs(a.val + s + p)) : 0.0f;
+        }
+    };
+    auto request = [&](const Batch &b, int i, int round) {
+        if (round < rounds) {
+#pragma unroll
+            for (int u = 0; u < kCopies; ++u) {
+                const int entry = u * (32 / kPieces) + lane / kPieces;
+                const int c = __shfl_sync(0xffffffffu, b.col[i], entry);
+                CopyAsync16(sData + i * Shape::kStageBytes + (u * 32 + lane) * 16, Bs + c * a.ldb,
+                            live && round * kRound + entry < length);
+            }
+            if (lane < kRound) sVal[i * kRound + lane] = b.val[i];
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    Batch now, next;
+    load(now, 0);
+    load(next, kStages);
+#pragma unroll
+    for (int i = 0; i < kStages; ++i) request(now, i, i);
+    const int word = lane & (4 * kPieces - 1);  // lanes past the last word repeat others' work
+    float acc[kCols] = {}, comp[kCols] = {};
+#pragma unroll 1
+    for (int r0 = 0; r0 < rounds; r0 += kStages) {
+        Batch after;
+        load(after, r0 + 2 * kStages);
+#pragma unroll
+        for (int i = 0; i < kStages; ++i) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 1) : "memory");
+            __syncwarp();
+            const uint32_t *data = reinterpret_cast<const uint32_t *>(sData + i * Shape::kStageBytes) + word;
+            const int left = length - (r0 + i) * kRound;
+            // Entries past the end count as 0 * 0 (the compensated sum skips them).
+#pragma unroll
+            for (int t0 = 0; t0 < kRound; t0 += 8) {
+                if (t0 >= left) break;
+                alignas(16) float v[8];
+                uint32_t w[8];
+                *reinterpret_cast<float4 *>(v) = *reinterpret_cast<const float4 *>(sVal + i * kRound + t0);
+                *reinterpret_cast<float4 *>(v + 4) = *reinterpret_cast<const float4 *>(sVal + i * kRound + t0 + 4);
+#pragma unroll
+                for (int t = 0; t < 8; ++t) w[t] = data[(t0 + t) * 4 * kPieces];
+#pragma unroll
+                for (int t = 0; t < 8; ++t) {
+                    if constexpr (kKahan) {
+                        if (t0 + t < left) AccumulateKahan(v[t], __uint_as_float(w[t]), acc[0], comp[0]);
+                    } else if constexpr (kCols == 1) {
+                        acc[0] = __fadd_rn(acc[0], __fmul_rn(v[t], __uint_as_float(w[t])));
+                    } else {
+                        float lo, hi;
+                        if constexpr (std::is_same_v<ValT, __half>) {
+                            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[t]));
+                            lo = f.x;
+                            hi = f.y;
+                        } else {
+                            lo = __uint_as_float(w[t] << 16);
+                            hi = __uint_as_float(w[t] & 0xffff0000u);
+                        }
+                        MulAdd2(acc[0], acc[1], lo, hi, v[t], a.negZeros);
+                    }
+                }
+            }
+            __syncwarp();
+            request(next, i, r0 + kStages + i);
+        }
+        next = after;
+    }
+    if (kKahan) acc[0] -= comp[0];
+    const float alpha = a.sc.Alpha();
+    const float beta = a.sc.Beta();
+    const int col = (slice * kPieces * 4 + word) * kCols;
+    const bool owner = lane < 4 * kPieces;
+    auto store = [&](const float (&v)[kCols]) {
+#pragma unroll
+        for (int i = 0; i < kCols; ++i) {
+            if (owner && col + i < a.n) {
+                OutT *dst = a.C + seg.row * a.cRow + (col + i) * a.cCol;
+                *dst = Finish<OutT>(v[i], alpha, beta, dst);
+            }
+        }
+    };
+    if (seg.longIdx < 0) {
+        store(acc);
+        return;
+    }
+    // The unit that comes last adds the row's partial sums of these columns in order.
+    const LongRow lr = a.longRows[seg.longIdx];
+    float *partial = static_cast<float *>(a.partials) + (long long)lr.partBase * a.n + col;
+#pragma unroll
+    for (int i = 0; i < kCols; ++i)
+        if (owner && col + i < a.n) __stcg(partial + (long long)seg.seg * a.n + i, acc[i]);
+    __threadfence();
+    __syncwarp();
+    int last = 0;
+    if (lane == 0) {
+        int32_t *counter = a.counters + (long long)seg.longIdx * a.arrivals + slice;
+        last = atomicAdd(counter, 1) == lr.nseg - 1;
+        if (last) *counter = 0;  // ready for the next launch
+    }
+    if (__shfl_sync(0xffffffffu, last, 0) == 0) return;
+    __threadfence();
+    float tot[kCols] = {};
+    for (int g0 = 0; g0 < lr.nseg; g0 += 8) {
+        float v[8][kCols];
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+#pragma unroll
+            for (int i = 0; i < kCols; ++i)
+                v[g][i] = g0 + g < lr.nseg && col + i < a.n ? __ldcg(partial + (long long)(g0 + g) * a.n + i) : 0.0f;
+        }
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+#pragma unroll
+            for (int i = 0; i < kCols; ++i) tot[i] += v[g][i];
+        }
+    }
+    store(tot);
+}
+
 // kLanes lanes lie side by side on one row of B (16 bytes each); a warp therefore carries
-// 32 / kLanes rows of A at once.  Rows of up to kLongRow entries are summed by their group in
-// CSR order; longer rows belong to the segment CTAs at the front of the grid.
+// 32 / kLanes rows of A at once.  Rows of up to a.rowLimit entries are summed by their group in
+// CSR order; longer rows are units, at the front of the grid.  A lane past the end of a B row works on the
+// row's first columns once more and stores nothing.
 //
-// kGenC: C is column-major or not 16-byte aligned.  A CTA then takes kGenRows rows, parks their sums in a
-// shared-memory tile and writes C along its contiguous direction (of column-major fp16 C, 32 rows are 64 bytes;
-// straight from registers every element would be a 32-byte sector of its own).
+// kGenC: C is column-major or not 16-byte aligned.  Sums then go through shared memory and are written along the
+// contiguous direction of C: by a warp where that is the row's, else by the CTA, which takes a.genRows rows (of
+// column-major fp16 C, 32 rows are 64 bytes; straight from registers every element would be a 32-byte sector of its
+// own) unless there are too few rows to give every SM a CTA.
 template <typename ValT, int kLanes> struct FastShape {
     static constexpr int kTileCols = kLanes * Pack<ValT>::kElems;
     static constexpr int kCtaRows = kWarps * (32 / kLanes);                   // rows of A per pass of the CTA
@@ -662,15 +870,23 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
     constexpr int kRowsPerWarp = 32 / kLanes;
     constexpr int kTileCols = Shape::kTileCols;
     constexpr int kTileStride = kTileCols + 1;
-    constexpr int kSegWords = kWarps * 32 * E;  // the segment CTAs' sums, one slice per warp
-    constexpr int kTileWords = kGenC ? Shape::kGenRows * kTileStride : 0;
-    __shared__ Acc sBuf[kSegWords > kTileWords ? kSegWords : kTileWords];
+    constexpr int kWarpWords = kInt8 ? 32 * E : UnitShape<kLanes>::kWarpBytes / 4;  // what a warp keeps of a unit
+    constexpr int kTileWords = kGenC ? (Shape::kGenRows * kTileStride > kThreads * E ? Shape::kGenRows * kTileStride : kThreads * E) : 0;
+    __shared__ __align__(16) Acc sBuf[kWarps * kWarpWords > kTileWords ? kWarps * kWarpWords : kTileWords];
     __shared__ unsigned char sSkip[kGenC ? Shape::kGenRows : 1];
     __shared__ int sLast;
 
+    b200sp::WaitForPrevious();
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int li = lane & (kLanes - 1);
+    const bool isUnit = (int)blockIdx.x < a.unitCtas;
+    if constexpr (!kInt8) {
+        if (isUnit) {
+            UnitSum<ValT, OutT, kKahan, kLanes>(a, reinterpret_cast<unsigned char *>(sBuf + warp * kWarpWords));
+            return;
+        }
+    }
     const auto alpha = a.sc.Alpha();
     const auto beta = a.sc.Beta();
     // one element of C at a time, whatever its layout
@@ -679,14 +895,16 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
         *dst = Finish<OutT>(v, alpha, beta, dst);
     };
 
-    const bool splitRow = kInt8 && a.splitRows && (int)blockIdx.x >= a.nsegs;
-    if ((int)blockIdx.x >= a.nsegs && !splitRow) {
+    const bool splitRow = kInt8 && a.splitRows && !isUnit;
+    if (!isUnit && !splitRow) {
         // ---- one lane group per row ----
-        constexpr int kBlockRows = kGenC ? Shape::kGenRows : Shape::kCtaRows;
-        const long long row0 = (long long)(blockIdx.x - a.nsegs) * kBlockRows;
-        for (int col0 = 0; col0 < (kGenC ? a.n : 1); col0 += kTileCols) {  // kGenC: a tile of columns at a time
+        constexpr int kChunk = kInt8 ? kLanes : Chunk<kLanes>::kChunk;
+        const bool rowsRun = kGenC && a.cCol != 1;  // column-major C
+        const int blockRows = rowsRun ? a.genRows : Shape::kCtaRows;
+        const long long row0 = (long long)(blockIdx.x - a.unitCtas) * blockRows;
+        for (int col0 = 0; col0 < (rowsRun ? a.n : 1); col0 += kTileCols) {  // column-major C: a tile of columns at a time
 #pragma unroll 1
-            for (int pass = 0; pass < kBlockRows; pass += Shape::kCtaRows) {
+            for (int pass = 0; pass < blockRows; pass += Shape::kCtaRows) {
                 const int rowIn = pass + warp * kRowsPerWarp + lane / kLanes;
                 const long long row = row0 + rowIn;
                 int s = 0, e = 0;
@@ -694,50 +912,58 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
                 if (row < a.m) {
                     s = a.rowPtr[row];
                     e = a.rowPtr[row + 1];
-                    if (e - s > kLongRow) {  // owned by segment CTAs
+                    if (e - s > a.rowLimit) {  // a unit
                         e = s;
                         skip = true;
                     }
                 }
-                int trips = (e - s + kLanes - 1) / kLanes;
+                int trips = (e - s + kChunk - 1) / kChunk;
 #pragma unroll
                 for (int off = kLanes; off < 32; off <<= 1) {
                     const int other = __shfl_xor_sync(0xffffffffu, trips, off);
                     trips = other > trips ? other : trips;
                 }
-                const int colFirst = kGenC ? col0 : 0, colLast = kGenC ? col0 + 1 : a.n;
+                const int colFirst = rowsRun ? col0 : 0, colLast = rowsRun ? col0 + 1 : a.n;
                 for (int colT = colFirst; colT < colLast; colT += kTileCols) {
                     const int col = colT + li * E;
                     const bool colLive = col < a.nB;
-                    const bool allLive = colT + kTileCols <= a.nB;
                     Acc acc[E], comp[E];
 #pragma unroll
                     for (int i = 0; i < E; ++i) acc[i] = comp[i] = Acc(0);
-                    if constexpr (kInt8) {
-                        RowDot8<kLanes>(a.colInd, a.val, a.B + (colLive ? col : 0), a.ldb, s, e, trips, acc);
-                    } else {
-                        RowDot<ValT, kKahan, kLanes>(a.colInd, a.val, a.B + col, a.ldb, s, e, trips, colLive, allLive, a.negZeros, acc,
-                                                     comp);
-                    }
+                    const ValT *Bs = a.B + (colLive ? col : 0);
+                    if constexpr (kInt8) RowDot8<kLanes>(a.colInd, a.val, Bs, a.ldb, s, e, trips, acc);
+                    else RowDot<ValT, kKahan, kLanes>(a.colInd, a.val, Bs, a.ldb, s, e, trips, a.negZeros, acc, comp);
                     if (kKahan) {
 #pragma unroll
                         for (int i = 0; i < E; ++i) acc[i] -= comp[i];
                     }
                     if constexpr (kGenC) {
+                        if (rowsRun) {
 #pragma unroll
-                        for (int i = 0; i < E; ++i) sBuf[rowIn * kTileStride + li * E + i] = acc[i];
-                        if (li == 0) sSkip[rowIn] = skip;
+                            for (int i = 0; i < E; ++i) sBuf[rowIn * kTileStride + li * E + i] = acc[i];
+                            if (li == 0) sSkip[rowIn] = skip;
+                        } else {
+                            Acc *sWarp = sBuf + warp * 32 * E;
+                            const unsigned skipped = __ballot_sync(0xffffffffu, skip);
+                            __syncwarp();
+#pragma unroll
+                            for (int i = 0; i < E; ++i) sWarp[lane * E + i] = acc[i];
+                            __syncwarp();
+#pragma unroll
+                            for (int i = lane; i < 32 * E; i += 32) {
+                                const int g = i / kTileCols, c = colT + i % kTileCols;
+                                if (c < a.n && !(skipped >> (g * kLanes) & 1)) storeOne(row0 + warp * kRowsPerWarp + g, c, sWarp[i]);
+                            }
+                        }
                     } else {
                         if (!skip && colLive) StoreRowSlice(a.C + row * a.ldc + col, acc, alpha, beta);
                     }
                 }
             }
-            if constexpr (kGenC) {
+            if (rowsRun) {
                 __syncthreads();
-                const bool rowsRun = a.cRow == 1;  // column-major C: consecutive threads on consecutive rows
-                for (int i = threadIdx.x; i < Shape::kGenRows * kTileCols; i += kThreads) {
-                    const int r = rowsRun ? i % Shape::kGenRows : i / kTileCols;
-                    const int c = rowsRun ? i / Shape::kGenRows : i % kTileCols;
+                for (int i = threadIdx.x; i < blockRows * kTileCols; i += kThreads) {  // consecutive threads on consecutive rows
+                    const int c = i / blockRows, r = i - c * blockRows;
                     if (col0 + c < a.n && !sSkip[r]) storeOne(row0 + r, col0 + c, sBuf[r * kTileStride + c]);
                 }
                 __syncthreads();
@@ -746,104 +972,104 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
         return;
     }
 
-    // ---- one CTA per long-row segment: the four warps take a quarter each ----
-    // (int8 with split rows: every row of up to kLongRow entries is such a segment)
-    const SegEntry seg = splitRow ? SegEntry{(int)blockIdx.x - a.nsegs, 0, 0, 0} : a.segs[blockIdx.x];
-    const LongRow lr = splitRow ? LongRow{seg.row, 0, 1, 0} : a.longRows[seg.longIdx];
-    const int rowStart = a.rowPtr[seg.row];
-    const int rowEnd = a.rowPtr[seg.row + 1];
-    if (splitRow && rowEnd - rowStart > kLongRow) return;
-    const int segStart = rowStart + seg.seg * kSegNnz;
-    const int segEnd = segStart + kSegNnz < rowEnd ? segStart + kSegNnz : rowEnd;
-    // inside a warp the lane groups take interleaved kLanes-wide chunks of the warp's quarter
-    const int quarter = splitRow ? ((segEnd - segStart + 4 * kWarps - 1) / (4 * kWarps)) * 4 : kWarpSegNnz;
-    int ws = segStart + warp * quarter;
-    int we = ws + quarter;
-    if (ws > segEnd) ws = segEnd;
-    if (we > segEnd) we = segEnd;
-    const int g = lane / kLanes;
-    Acc *partial = static_cast<Acc *>(a.partials) + (long long)(lr.partBase + seg.seg) * a.n;
-    auto storeSlice = [&](int col, const Acc (&v)[E]) {
-        if constexpr (kGenC) {
-#pragma unroll
-            for (int i = 0; i < E; ++i)
-                if (col + i < a.n) storeOne(seg.row, col + i, v[i]);
-        } else {
-            StoreRowSlice(a.C + (long long)seg.row * a.ldc + col, v, alpha, beta);
-        }
-    };
-
-    for (int col0 = 0; col0 < a.n; col0 += kTileCols) {
-        const int col = col0 + li * E;
-        const bool colLive = col < a.nB;
-        const bool allLive = col0 + kTileCols <= a.nB;
-        Acc acc[E], comp[E];
-#pragma unroll
-        for (int i = 0; i < E; ++i) acc[i] = comp[i] = Acc(0);
-        // group g walks chunks g, g + kRowsPerWarp, ... of [ws, we)
-        const int nChunks = (we - ws + kLanes - 1) / kLanes;
-        for (int ch0 = 0; ch0 < nChunks; ch0 += kRowsPerWarp) {  // same trip count in every group
-            const int ch = ch0 + g;
-            const int cs = ws + ch * kLanes < we ? ws + ch * kLanes : we;
-            const int ce = cs + kLanes < we ? cs + kLanes : we;
-            if constexpr (kInt8) RowDot8<kLanes>(a.colInd, a.val, a.B + (colLive ? col : 0), a.ldb, cs, ce, 1, acc);
-            else RowDot<ValT, kKahan, kLanes>(a.colInd, a.val, a.B + col, a.ldb, cs, ce, 1, colLive, allLive, a.negZeros, acc,
-                                                     comp);
-        }
-#pragma unroll
-        for (int i = 0; i < E; ++i) {
-            if (kKahan) acc[i] -= comp[i];
-#pragma unroll
-            for (int off = kLanes; off < 32; off <<= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], off);
-        }
-        if (lane < kLanes) {
-#pragma unroll
-            for (int i = 0; i < E; ++i) sBuf[warp * 32 * E + li * E + i] = acc[i];
-        }
-        __syncthreads();
-        // warp 0 adds the four warps' slices in warp order
-        if (warp == 0 && lane < kLanes && colLive) {
-            Acc tot[E];
-#pragma unroll
-            for (int i = 0; i < E; ++i) {
-                tot[i] = sBuf[li * E + i];
-#pragma unroll
-                for (int w = 1; w < kWarps; ++w) tot[i] += sBuf[w * 32 * E + li * E + i];
-            }
-            if (lr.nseg == 1) {
-                storeSlice(col, tot);
-            } else {
+    // ---- int8: one CTA per unit (with split rows also per row), the four warps take a quarter each ----
+    if constexpr (kInt8) {
+        const SegEntry seg = splitRow ? SegEntry{(int)blockIdx.x - a.unitCtas, 0, -1, 0}
+                             : (int)blockIdx.x < a.longUnits ? a.segs[blockIdx.x]
+                                                             : a.segsEnd[a.longUnits - 1 - (int)blockIdx.x];
+        const LongRow lr = seg.longIdx < 0 ? LongRow{seg.row, 0, 1, 0} : a.longRows[seg.longIdx];
+        const int rowStart = a.rowPtr[seg.row];
+        const int rowEnd = a.rowPtr[seg.row + 1];
+        if (splitRow && rowEnd - rowStart > a.rowLimit) return;
+        const int segStart = rowStart + seg.seg * kSegNnz;
+        const int segEnd = rowEnd - segStart > kSegNnz ? segStart + kSegNnz : rowEnd;
+        // inside a warp the lane groups take interleaved kLanes-wide chunks of the warp's quarter
+        const int quarter = ((segEnd - segStart + 4 * kWarps - 1) / (4 * kWarps)) * 4;
+        int ws = segStart + warp * quarter;
+        int we = ws + quarter;
+        if (ws > segEnd) ws = segEnd;
+        if (we > segEnd) we = segEnd;
+        const int g = lane / kLanes;
+        Acc *partial = static_cast<Acc *>(a.partials) + (long long)(lr.partBase + seg.seg) * a.n;
+        auto storeSlice = [&](int col, const Acc (&v)[E]) {
+            if constexpr (kGenC) {
 #pragma unroll
                 for (int i = 0; i < E; ++i)
-                    if (!kGenC || col + i < a.n) partial[col + i] = tot[i];
+                    if (col + i < a.n) storeOne(seg.row, col + i, v[i]);
+            } else {
+                StoreRowSlice(a.C + (long long)seg.row * a.ldc + col, v, alpha, beta);
             }
+        };
+
+        for (int col0 = 0; col0 < a.n; col0 += kTileCols) {
+            const int col = col0 + li * E;
+            const bool colLive = col < a.nB;
+            Acc acc[E];
+#pragma unroll
+            for (int i = 0; i < E; ++i) acc[i] = Acc(0);
+            // group g walks chunks g, g + kRowsPerWarp, ... of [ws, we)
+            const int nChunks = (we - ws + kLanes - 1) / kLanes;
+            for (int ch0 = 0; ch0 < nChunks; ch0 += kRowsPerWarp) {  // same trip count in every group
+                const int ch = ch0 + g;
+                const int cs = ws + ch * kLanes < we ? ws + ch * kLanes : we;
+                const int ce = cs + kLanes < we ? cs + kLanes : we;
+                RowDot8<kLanes>(a.colInd, a.val, a.B + (colLive ? col : 0), a.ldb, cs, ce, 1, acc);
+            }
+#pragma unroll
+            for (int i = 0; i < E; ++i) {
+#pragma unroll
+                for (int off = kLanes; off < 32; off <<= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], off);
+            }
+            if (lane < kLanes) {
+#pragma unroll
+                for (int i = 0; i < E; ++i) sBuf[warp * 32 * E + li * E + i] = acc[i];
+            }
+            __syncthreads();
+            // warp 0 adds the four warps' slices
+            if (warp == 0 && lane < kLanes && colLive) {
+                Acc tot[E];
+#pragma unroll
+                for (int i = 0; i < E; ++i) {
+                    tot[i] = sBuf[li * E + i];
+#pragma unroll
+                    for (int w = 1; w < kWarps; ++w) tot[i] += sBuf[w * 32 * E + li * E + i];
+                }
+                if (lr.nseg == 1) {
+                    storeSlice(col, tot);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < E; ++i)
+                        if (!kGenC || col + i < a.n) partial[col + i] = tot[i];
+                }
+            }
+            __syncthreads();
+        }
+        if (lr.nseg == 1) return;
+
+        // Arrival: the unit that comes last sums all partial rows.
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int32_t *counter = a.counters + (long long)seg.longIdx * a.arrivals;
+            const int old = atomicAdd(counter, 1);
+            sLast = (old == lr.nseg - 1);
+            if (sLast) *counter = 0;  // ready for the next launch
         }
         __syncthreads();
-    }
-    if (lr.nseg == 1) return;
-
-    // Arrival: the segment that comes last sums all partial rows in segment order.
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int old = atomicAdd(a.counters + seg.longIdx, 1);
-        sLast = (old == lr.nseg - 1);
-        if (sLast) a.counters[seg.longIdx] = 0;  // ready for the next launch
-    }
-    __syncthreads();
-    if (!sLast) return;
-    __threadfence();
-    const Acc *first = static_cast<const Acc *>(a.partials) + (long long)lr.partBase * a.n;
-    for (int col = threadIdx.x * E; col < a.n; col += kThreads * E) {
-        Acc tot[E];
+        if (!sLast) return;
+        __threadfence();
+        const Acc *first = static_cast<const Acc *>(a.partials) + (long long)lr.partBase * a.n;
+        for (int col = threadIdx.x * E; col < a.n; col += kThreads * E) {
+            Acc tot[E];
 #pragma unroll
-        for (int i = 0; i < E; ++i) tot[i] = Acc(0);
-        for (int sgi = 0; sgi < lr.nseg; ++sgi) {
+            for (int i = 0; i < E; ++i) tot[i] = Acc(0);
+            for (int sgi = 0; sgi < lr.nseg; ++sgi) {
 #pragma unroll
-            for (int i = 0; i < E; ++i)
-                if (!kGenC || col + i < a.n) tot[i] += __ldcg(first + (long long)sgi * a.n + col + i);
+                for (int i = 0; i < E; ++i)
+                    if (!kGenC || col + i < a.n) tot[i] += __ldcg(first + (long long)sgi * a.n + col + i);
+            }
+            storeSlice(col, tot);
         }
-        storeSlice(col, tot);
     }
 }
 
@@ -1194,6 +1420,7 @@ struct StreamArgs {
     const ValT *B;
     OutT *C;
     int m;
+    int rowLimit;
     long long ldb;
     long long ldc;
     ScalarsF sc;
@@ -1246,7 +1473,7 @@ __global__ void __launch_bounds__(kStreamThreads) SpmmRowStreamKernel(const Stre
     if (myRow < a.m) {
         s = a.rowPtr[myRow];
         len = a.rowPtr[myRow + 1] - s;
-        mine = len <= kLongRow;  // longer rows are written by the segment CTAs
+        mine = len <= a.rowLimit;  // longer rows are units
         if (!mine) len = 0;
     }
     int off = len;  // inclusive scan over the lanes, then made exclusive
@@ -1377,6 +1604,7 @@ template <typename ValT>
 __global__ void __launch_bounds__(256) SpmmRepackRowsKernel(const ValT *__restrict__ B, long long ldb, long long k, int n,
                                                             int vecs, uint4 *__restrict__ out)
 {
+    b200sp::WaitForPrevious();
     constexpr int E = 16 / (int)sizeof(ValT);
     const long long total = k * vecs;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -1395,6 +1623,7 @@ template <typename ValT>
 __global__ void __launch_bounds__(256) SpmmRepackColsKernel(const ValT *__restrict__ B, long long ldb, long long k, int n,
                                                             int vecs, uint4 *__restrict__ out)
 {
+    b200sp::WaitForPrevious();
     constexpr int E = 16 / (int)sizeof(ValT);
     constexpr int kCols = 64;                            // columns per step
     constexpr int kVecs = kCols / E;
@@ -1440,6 +1669,7 @@ __global__ void __launch_bounds__(256) SpmmGenericFloatKernel(const int32_t *__r
                                                                const ValT *__restrict__ B, OutT *__restrict__ C,
                                                                GenericShape g, ScalarsF sc)
 {
+    b200sp::WaitForPrevious();
     const float alpha = sc.Alpha();
     const float beta = sc.Beta();
     const long long total = g.m * g.n;
@@ -1468,6 +1698,7 @@ __global__ void __launch_bounds__(256) SpmmGenericInt8Kernel(const int32_t *__re
                                                               const int8_t *__restrict__ B, int32_t *__restrict__ C,
                                                               GenericShape g, ScalarsI sc)
 {
+    b200sp::WaitForPrevious();
     const int32_t alpha = sc.Alpha();
     const int32_t beta = sc.Beta();
     const long long total = g.m * g.n;
@@ -1560,15 +1791,15 @@ int LaunchGeneric(const int32_t *rowPtr, const int32_t *colInd, const void *val,
     const long long cap = (long long)b200sp_sm_count() * 32;
     const unsigned grid = (unsigned)(want < cap ? want : cap);
     const auto sc = MakeScalars<typename Arith<ValT>::Scalars>(s);
+    cudaError_t e;
     if constexpr (std::is_same_v<ValT, int8_t>)
-        SpmmGenericInt8Kernel<<<grid, 256, 0, stream>>>(rowPtr, colInd, static_cast<const ValT *>(val),
-                                                        static_cast<const ValT *>(B), static_cast<OutT *>(C), g, sc);
+        e = b200sp::LaunchChained(SpmmGenericInt8Kernel, grid, 256, 0, stream, rowPtr, colInd, static_cast<const ValT *>(val),
+                                  static_cast<const ValT *>(B), static_cast<OutT *>(C), g, sc);
     else
-        SpmmGenericFloatKernel<ValT, OutT><<<grid, 256, 0, stream>>>(rowPtr, colInd, static_cast<const ValT *>(val),
-                                                                     static_cast<const ValT *>(B),
-                                                                     static_cast<OutT *>(C), g, sc);
+        e = b200sp::LaunchChained(SpmmGenericFloatKernel<ValT, OutT>, grid, 256, 0, stream, rowPtr, colInd,
+                                  static_cast<const ValT *>(val), static_cast<const ValT *>(B), static_cast<OutT *>(C), g, sc);
     b200sp_note_launches(1);
-    return (int)cudaGetLastError();
+    return (int)e;
 }
 
 template <typename ValT, typename OutT>
@@ -1579,7 +1810,9 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
     constexpr bool kInt8 = std::is_same_v<ValT, int8_t>;
     constexpr int E = Pack<ValT>::kElems;
     const size_t repack = RepackBytes(sh, (int)sizeof(ValT));
-    const bool bReady = repack == 0 ? Aligned16(B) : (sh->repack_bytes >= (int64_t)repack && WorthRepacking(sh));
+    // A product of one wave, with no row above MidRowLimit, takes less time than the second launch.
+    const bool small = sh->m * sh->n < 148ll * 2048 && segments + sh->mid_units == 0;
+    const bool bReady = repack == 0 ? Aligned16(B) : (sh->repack_bytes >= (int64_t)repack && WorthRepacking(sh) && !small);
     if (plan == nullptr || !bReady)
         return LaunchGeneric<ValT, OutT>(rowPtr, colInd, val, B, C, sh, s, stream);
     if (sh->m == 0 || sh->n == 0) return 0;
@@ -1602,47 +1835,59 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
     a.sc = MakeScalars<typename Arith<ValT>::Scalars>(s);
     a.longRows = reinterpret_cast<const LongRow *>(p + L.offLong);
     a.segs = reinterpret_cast<const SegEntry *>(p + L.offSegs);
+    a.segsEnd = a.segs + L.capSegs;
     a.counters = reinterpret_cast<int32_t *>(p + L.offCounters);
     a.partials = p + L.offPartials;
-    a.nsegs = segments;
+    a.arrivals = (int)ArrivalsPerRow(sh->n);
+    a.rowLimit = sh->mid_units > 0 ? MidRowLimit(sh->m, sh->nnz, sh->n) : kLongRow;
     a.splitRows = 0;
     a.negZeros = kNegZeros;
     if (repack > 0) {
         const int vecs = (int)((sh->n + E - 1) / E);
         auto *out = reinterpret_cast<uint4 *>(p + L.total);
+        cudaError_t e;
         if (RowsContiguous(sh->op_b, sh->order_b)) {
             const long long want = (sh->k * vecs + 255) / 256;
             const long long cap = (long long)b200sp_sm_count() * 32;
-            SpmmRepackRowsKernel<ValT><<<(unsigned)(want < cap ? want : cap), 256, 0, stream>>>(a.B, sh->ldb, sh->k, a.n,
-                                                                                              vecs, out);
+            e = b200sp::LaunchChained(SpmmRepackRowsKernel<ValT>, (unsigned)(want < cap ? want : cap), 256, 0, stream, a.B,
+                                      sh->ldb, sh->k, a.n, vecs, out);
         } else {
-            SpmmRepackColsKernel<ValT><<<(unsigned)((sh->k + kRepackRows - 1) / kRepackRows), 256, 0, stream>>>(
-                a.B, sh->ldb, sh->k, a.n, vecs, out);
+            e = b200sp::LaunchChained(SpmmRepackColsKernel<ValT>, (unsigned)((sh->k + kRepackRows - 1) / kRepackRows), 256, 0,
+                                      stream, a.B, sh->ldb, sh->k, a.n, vecs, out);
         }
         b200sp_note_launches(1);
-        const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return (int)e;
         a.B = reinterpret_cast<const ValT *>(out);
         a.ldb = (long long)vecs * E;
         a.nB = vecs * E;
     }
+    int midUnits = sh->mid_units;
     constexpr int kMinLanes = kInt8 ? 4 : 1;
     int lanes_ = kMinLanes;  // lanes side by side on a row of B
     while (lanes_ < 32 && lanes_ * E < sh->n) lanes_ <<= 1;
-    // Grid of SpmmFastKernel: `segs` segment CTAs, then CTAs for all rows when `rowCtas` is set.
-    auto launchFast = [&](int segs, bool rowCtas, cudaStream_t st) {
-        a.nsegs = segs;
+    // Grid of SpmmFastKernel: CTAs for the units of long rows, for those of one row each, and for all rows.
+    auto launchFast = [&](int longUnits, int midUnits, bool rowCtas, cudaStream_t st) {
+        const int units = longUnits + midUnits;
+        cudaError_t err = cudaSuccess;
         auto launch = [&]<int kLanes>() {
             using Shape = FastShape<ValT, kLanes>;
-            const long long rows = a.splitRows ? 1 : cPlain ? Shape::kCtaRows : Shape::kGenRows;
-            const long long grid = segs + (rowCtas ? (sh->m + rows - 1) / rows : 0);
+            constexpr int kPieces = UnitShape<kLanes>::kPieces;
+            a.longUnits = longUnits;
+            a.nUnits = units;
+            a.slices = (a.nB / E + kPieces - 1) / kPieces;
+            const long long unitCtas = kInt8 ? units : ((long long)units * a.slices + kWarps - 1) / kWarps;
+            a.unitCtas = (int)unitCtas;
+            a.genRows = sh->m < 2ll * Shape::kGenRows * b200sp_sm_count() ? Shape::kCtaRows : Shape::kGenRows;
+            const long long rows = a.splitRows ? 1 : sh->order_c == 0 ? Shape::kCtaRows : a.genRows;
+            const long long grid = unitCtas + (rowCtas ? (sh->m + rows - 1) / rows : 0);
             if (grid == 0) return;
+            auto go = [&](auto kernel) { err = b200sp::LaunchChained(kernel, (unsigned)grid, kThreads, 0, st, a); };
             if constexpr (std::is_same_v<ValT, float>) {
-                if (sh->kahan && cPlain) SpmmFastKernel<ValT, OutT, true, kLanes, false><<<(unsigned)grid, kThreads, 0, st>>>(a);
-                else if (sh->kahan) SpmmFastKernel<ValT, OutT, true, kLanes, true><<<(unsigned)grid, kThreads, 0, st>>>(a);
+                if (sh->kahan && cPlain) go(SpmmFastKernel<ValT, OutT, true, kLanes, false>);
+                else if (sh->kahan) go(SpmmFastKernel<ValT, OutT, true, kLanes, true>);
             }
-            if (!sh->kahan && cPlain) SpmmFastKernel<ValT, OutT, false, kLanes, false><<<(unsigned)grid, kThreads, 0, st>>>(a);
-            else if (!sh->kahan) SpmmFastKernel<ValT, OutT, false, kLanes, true><<<(unsigned)grid, kThreads, 0, st>>>(a);
+            if (!sh->kahan && cPlain) go(SpmmFastKernel<ValT, OutT, false, kLanes, false>);
+            else if (!sh->kahan) go(SpmmFastKernel<ValT, OutT, false, kLanes, true>);
             b200sp_note_launches(1);
         };
         switch (lanes_) {
@@ -1653,15 +1898,15 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             case 16: launch.template operator()<16>(); break;
             default: launch.template operator()<32>(); break;
         }
-        return cudaGetLastError();
+        return err;
     };
     if constexpr (kInt8) {
         // Integer sums may be regrouped: where a warp per row would not fill the SMs and rows are long enough to be
         // shared, a CTA takes a row (4096 rows of 410 entries, N = 512: 104 us with a warp per row, 74 us so).
         a.splitRows = cPlain && sh->nnz >= 128 * sh->m && sh->m * lanes_ / 32 < 64ll * b200sp_sm_count();
-        return (int)launchFast(segments, true, stream);
+        return (int)launchFast(segments, midUnits, true, stream);
     } else {
-        if (!cPlain) return (int)launchFast(segments, true, stream);
+        if (!cPlain) return (int)launchFast(segments, midUnits, true, stream);
         // B rows of 512 / 1024 bytes: rows of up to kLongRow entries go to the row-stream kernel,
         // and SpmmFastKernel is launched for its segment CTAs only.
         const long long rowBytes = sh->n * (long long)sizeof(ValT);
@@ -1670,6 +1915,10 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
         const bool byBlocks = sh->block_units > 0 && sh->long_rows > 0 && !sh->kahan && rowBytes >= kBlockMinRowBytes &&
                               sh->block_units <= L.capBlockSlots;
         if (byBlocks) segments = 0;
+        if (stream_) {  // which has enough copies in flight for any row it takes
+            a.rowLimit = kLongRow;
+            midUnits = 0;
+        }
         // With both kernels to run, the long rows (few CTAs, each with much work) are forked onto the side stream
         // first and the other rows' kernel shares the SMs with them.
         b200sp::SideLanes *lanes = nullptr;
@@ -1694,7 +1943,7 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
                 b200sp_note_launches(1);
                 if (cudaGetLastError() != cudaSuccess) return (int)cudaErrorLaunchFailure;
             } else if (lanes != nullptr) {
-                if (launchFast(segments, false, longStream) != cudaSuccess) return (int)cudaErrorLaunchFailure;
+                if (launchFast(segments, 0, false, longStream) != cudaSuccess) return (int)cudaErrorLaunchFailure;
                 segments = 0;
             }
             if (lanes != nullptr && cudaEventRecord(lanes->join[0], longStream) != cudaSuccess)
@@ -1708,6 +1957,7 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             sa.B = a.B;
             sa.C = a.C;
             sa.m = a.m;
+            sa.rowLimit = a.rowLimit;
             sa.ldb = a.ldb;
             sa.ldc = sh->ldc;
             sa.sc = a.sc;
@@ -1721,7 +1971,7 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
         // What is left for SpmmFastKernel on the caller's stream: the segment CTAs unless they were forked (or
         // replaced by the column-block kernel), and the rows of up to kLongRow entries unless the row-stream
         // kernel took them.
-        if (launchFast(segments, !stream_, stream) != cudaSuccess) return (int)cudaErrorLaunchFailure;
+        if (launchFast(segments, midUnits, !stream_, stream) != cudaSuccess) return (int)cudaErrorLaunchFailure;
         if (lanes != nullptr)  // the long rows are already running beside: join them
             return (int)cudaStreamWaitEvent(stream, lanes->join[0], 0);
         return 0;
@@ -1762,6 +2012,13 @@ size_t b200sp_spmm_repack_bytes(const b200spSpmmShape *shape, int val_type)
 int b200sp_spmm_analyze(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,
                         size_t plan_bytes, int32_t *segments, void *stream)
 {
+    int32_t mid = 0;
+    return b200sp_spmm_analyze_units(row_ptr, rows, nnz, n, plan, plan_bytes, segments, &mid, stream);
+}
+
+int b200sp_spmm_analyze_units(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,
+                              size_t plan_bytes, int32_t *segments, int32_t *mid_units, void *stream)
+{
     const PlanLayout L = LayoutFor(rows, nnz, n);
     if (plan == nullptr || segments == nullptr || plan_bytes < L.total) return (int)cudaErrorInvalidValue;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -1772,19 +2029,21 @@ int b200sp_spmm_analyze(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64
         const long long want = (rows + 255) / 256;
         const long long cap = (long long)b200sp_sm_count() * 16;
         SpmmFindLongRowsKernel<<<(unsigned)(want < cap ? want : cap), 256, 0, st>>>(
-            row_ptr, (int)rows, reinterpret_cast<int32_t *>(p + L.offCounts),
+            row_ptr, (int)rows, MidRowLimit(rows, nnz, n), (int)ArrivalsPerRow(n), (int)L.capSegs,
+            reinterpret_cast<int32_t *>(p + L.offCounts),
             reinterpret_cast<LongRow *>(p + L.offLong), reinterpret_cast<SegEntry *>(p + L.offSegs),
             reinterpret_cast<int32_t *>(p + L.offCounters));
         b200sp_note_launches(1);
         e = cudaGetLastError();
         if (e != cudaSuccess) return (int)e;
     }
-    int32_t counts[2] = {0, 0};
+    int32_t counts[6] = {};
     e = cudaMemcpyAsync(counts, p + L.offCounts, sizeof(counts), cudaMemcpyDeviceToHost, st);
     if (e != cudaSuccess) return (int)e;
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return (int)e;
     *segments = counts[1];
+    *mid_units = counts[5];
     return 0;
 }
 
@@ -1799,7 +2058,8 @@ int b200sp_spmm_analyze_blocks(const int32_t *row_ptr, const int32_t *col_ind, i
     *long_rows = 0;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     char *p = static_cast<char *>(plan);
-    // counts: long rows, segments, partial slots of the segments, "a long row's columns do not ascend", units
+    // counts: long rows, their units, partial slots of the long rows' units, "a long row's columns do not ascend", units (and
+    // the rows that are a unit each)
     int32_t counts[5] = {0, 0, 0, 0, 0};
     cudaError_t e = cudaMemcpyAsync(counts, p + L.offCounts, sizeof(counts), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);

@@ -1,0 +1,79 @@
+"""GPU: SpMM at the row lengths and widths where its kernels change (rows summed apart from their neighbours, rows cut
+every 1024 entries, 64-byte slices of B, repacked layouts)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from test_spmm_gpu import check_compact, compact_case, run_spmm
+
+pytestmark = pytest.mark.gpu
+
+EDGES = [0, 1, 15, 16, 17, 31, 32, 33, 48, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 1023, 1024, 1025, 2048, 2049, 9000]
+# one lane to several tiles of 32 per row of B, whole and ragged 64-byte slices and 16-byte pieces
+WIDTHS = [1, 4, 5, 8, 12, 16, 31, 40, 64, 100, 136, 300]
+
+
+def case(oracle, vt, ot, n, filler):
+    rng = np.random.default_rng(n + filler)
+    # few rows: every row above 16 entries is a unit; enough for the SMs: those above 64, or above four times the mean
+    extra = 300 if filler == 3 else 148 * 2048 // n + 1
+    lengths = rng.permutation(np.concatenate([EDGES, np.full(extra, filler)]))
+    m, k = lengths.size, 9000
+    return m, k, *compact_case(oracle, rng, m, k, n, lengths, vt, ot, 1.5, -0.5)
+
+
+@pytest.mark.parametrize("vt,ot", [("f32", "f32"), ("f16", "f16"), ("bf16", "bf16"), ("bf16", "f32")])
+@pytest.mark.parametrize("order", ["row", "col"])
+@pytest.mark.parametrize("n", WIDTHS)
+@pytest.mark.parametrize("filler", [3, 30])
+def test_row_lengths(handle, device, oracle, filler, n, order, vt, ot):
+    """The golden's bits for rows of up to 1024 entries, its tolerance for the others."""
+    if n == 1 and filler != 3:
+        filler = 4  # rows enough for the SMs are many here
+    m, k, rp, ci, val, B, C = case(oracle, vt, ot, n, filler)
+    stored = (lambda a: a) if order == "row" else (lambda a: np.ascontiguousarray(a.T))
+    ldb, ldc = (n, n) if order == "row" else (k, m)
+    got = run_spmm(handle, device, rp, ci, val, vt, stored(B), stored(C), ot, m, k, n, ldb, ldc, 1.5, -0.5,
+                   b_order=order, c_order=order)
+    got = got.reshape(m, n) if order == "row" else np.ascontiguousarray(got.reshape(n, m).T)
+    check_compact(oracle, rp, ci, val, B, C, vt, ot, 1.5, -0.5, got, f"{vt}->{ot} n={n} {order} filler={filler}")
+    if vt == "f32":
+        gold = oracle.spmm_f32_layout(m, n, rp, ci, val, B, n, True, False, C, n, True, 1.5, -0.5)
+    else:
+        gold = oracle.spmm_16(rp, ci, val, B, C, 1.5, -0.5, vt, ot)
+    short = np.diff(rp) <= 1024
+    assert np.array_equal(got[short].view(np.uint8), np.asarray(gold).reshape(m, n)[short].view(np.uint8))
+
+
+@pytest.mark.parametrize("n", [3, 16, 150])
+def test_compensated_sums(handle, device, oracle, n):
+    from ops_sparse_b200 import ACL_SPARSE_SPMM_CSR_FP32_HIGH_PRECISION_ALG as KAHAN
+    m, k, rp, ci, val, B, C = case(oracle, "f32", "f32", n, 5)
+    got = run_spmm(handle, device, rp, ci, val, "f32", B, C, "f32", m, k, n, n, n, 1.5, -0.5, alg=KAHAN).reshape(m, n)
+    exact = 1.5 * np.stack([val[s:e].astype(np.float64) @ B[ci[s:e]].astype(np.float64) for s, e in zip(rp, rp[1:])]) - 0.5 * C
+    scale = 1.5 * oracle.spmm_abs_sum(rp, ci, val, B, "f32") + np.abs(0.5 * C)
+    # compensated: 2 eps and a term in eps^2 n per unit, plus the rounding of at most nine units' sums and of the epilogue
+    assert np.all(np.abs(got - exact) <= 16 * 2.0 ** -24 * scale + 1e-30)
+
+
+@pytest.mark.parametrize("order", ["row", "col"])
+@pytest.mark.parametrize("n", [1, 8, 16, 17, 32, 33, 64, 100, 300])
+@pytest.mark.parametrize("filler", [3, 60, 200])
+def test_int8(handle, device, oracle, filler, n, order):
+    rng = np.random.default_rng(n + filler)
+    lengths = rng.permutation(np.concatenate([EDGES, np.full(300 if filler == 3 else 148 * 2048 // n + 1, filler)]))
+    m, k = lengths.size, 2500
+    rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    ci = rng.integers(0, k, rp[-1]).astype(np.int32)
+    val = rng.integers(-128, 128, rp[-1]).astype(np.int8)
+    B = rng.integers(-128, 128, (k, n)).astype(np.int8)
+    C = rng.integers(-1000, 1000, (m, n)).astype(np.int32)
+    stored = (lambda a: a) if order == "row" else (lambda a: np.ascontiguousarray(a.T))
+    ldb, ldc = (n, n) if order == "row" else (k, m)
+    got = run_spmm(handle, device, rp, ci, val, "i8", stored(B), stored(C), "i32", m, k, n, ldb, ldc, 2, -1,
+                   b_order=order, c_order=order)
+    got = got.reshape(m, n) if order == "row" else got.reshape(n, m).T
+    import scipy.sparse
+    A = scipy.sparse.csr_matrix((val.astype(np.int64), ci, rp), shape=(m, k))
+    assert np.array_equal(got, (2 * (A @ B.astype(np.int64)) - C).astype(np.int32))
