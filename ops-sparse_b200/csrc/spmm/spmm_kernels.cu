@@ -85,7 +85,7 @@ constexpr int kUnitNnz = B200SP_SPMM_UNIT_NNZ;   // a (row, block) piece longer 
 // up to 16,384, N = 16: 694 and 362 us.
 inline int MidRowLimit(int64_t rows, int64_t nnz, int64_t n)
 {
-    if (rows * n < 148ll * 2048) return 16;
+    if (rows * (n < 16 ? 16 : n) < 148ll * 512) return 16;  // all units (a warp per 16 to 32 columns) resident at once
     const int64_t four = 4 * (nnz / (rows > 0 ? rows : 1));
     return (int)(four < 64 ? 64 : four > kLongRow ? kLongRow : four);
 }
@@ -183,11 +183,26 @@ __device__ __forceinline__ uint4 LoadB16(const void *p)
 #endif
 }
 
-// The same for lanes with `on` set; the others keep what q held (and request nothing).
-__device__ __forceinline__ void LoadB16If(bool on, const void *p, uint4 &q)
+__device__ __forceinline__ uint32_t LoadB4(const void *p)
 {
-    if (on) q = LoadB16(p);
+    uint64_t pol;
+    asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
+    uint32_t q;
+    asm volatile("ld.global.nc.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(q) : "l"(p), "l"(pol));
+    return q;
 }
+
+// What a lane reads of a row of B: 16 bytes side by side, or (kWords: rows that do not start on 16-byte boundaries) four
+// words a lane group apart, so that a group still reads consecutive words.  first[] in elements from the row's start.
+template <typename ValT, bool kWords> struct Slice {
+    static constexpr int kCols = 4 / (int)sizeof(ValT);  // columns of a word (fp types)
+    int first[kWords ? 4 : 1];
+    __device__ __forceinline__ uint4 Load(const ValT *row) const
+    {
+        if constexpr (kWords) return make_uint4(LoadB4(row + first[0]), LoadB4(row + first[1]), LoadB4(row + first[2]), LoadB4(row + first[3]));
+        else return LoadB16(row + first[0]);
+    }
+};
 
 // 16 bytes of a B row as fp32 values: 4 floats, or 8 half / bf16.
 template <typename T> struct Pack;
@@ -485,9 +500,9 @@ template <int kLanes> struct Chunk {
     static constexpr int kChunk = kLanes * kHold;
 };
 
-template <typename ValT, bool kKahan, int kLanes>
+template <typename ValT, bool kKahan, int kLanes, bool kWords>
 __device__ __forceinline__ void RowDot(const int32_t *__restrict__ colInd, const ValT *__restrict__ val,
-                                       const ValT *__restrict__ Bslice, long long ldb, int s, int e, int trips,
+                                       const ValT *__restrict__ B, const Slice<ValT, kWords> &slice, long long ldb, int s, int e, int trips,
                                        unsigned long long negZeros, float (&acc)[Pack<ValT>::kElems],
                                        float (&comp)[Pack<ValT>::kElems])
 {
@@ -520,7 +535,7 @@ __device__ __forceinline__ void RowDot(const int32_t *__restrict__ colInd, const
                 for (int u = 0; u < kBatch; ++u) {
                     const int c = __shfl_sync(0xffffffffu, myCol[(q0 + u) / kLanes], (q0 + u) % kLanes, kLanes);
                     v[u] = __shfl_sync(0xffffffffu, myVal[(q0 + u) / kLanes], (q0 + u) % kLanes, kLanes);
-                    q[u] = LoadB16(Bslice + (long long)c * ldb);
+                    q[u] = slice.Load(B + (long long)c * ldb);
                 }
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u) {
@@ -548,7 +563,7 @@ __device__ __forceinline__ void RowDot(const int32_t *__restrict__ colInd, const
                 const int c = __shfl_sync(0xffffffffu, myCol[(q0 + u) / kLanes], (q0 + u) % kLanes, kLanes);
                 v[u] = __shfl_sync(0xffffffffu, myVal[(q0 + u) / kLanes], (q0 + u) % kLanes, kLanes);
                 q[u] = make_uint4(0, 0, 0, 0);
-                LoadB16If(q0 + u < rem, Bslice + (long long)c * ldb, q[u]);
+                if (q0 + u < rem) q[u] = slice.Load(B + (long long)c * ldb);
             }
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
@@ -571,47 +586,89 @@ __device__ __forceinline__ void RowDot(const int32_t *__restrict__ colInd, const
 // transposed (eight byte permutes) so that one __dp4a adds four products: 12 instructions for 16 products instead
 // of 32 (16 extractions and 16 multiply-adds).  Entries past a row's end carry value 0 and column 0, which adds
 // nothing.  int32 addition wraps the same in any order, so the result is the golden's whatever the grouping.
+// Up to four lanes side by side are too few for a row of their own: eight lanes share one, kShare sets of kLanes lanes
+// that take every kShare-th entry; their sums are added when the row ends.
+template <int kLanes> struct Group8 {
+    static constexpr int kLanesOfRow = kLanes < 8 ? 8 : kLanes;
+    static constexpr int kShare = kLanesOfRow / kLanes;
+    static constexpr int kChunk = kShare > 1 ? 8 * kShare : kLanes;
+};
+
+__device__ __forceinline__ void DotQuad(const uint32_t (&x)[4], const uint32_t (&y)[4], const uint32_t (&z)[4], const uint32_t (&t)[4],
+                                        int v, int32_t (&acc)[16])
+{
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t lo01 = __byte_perm(x[j], y[j], 0x5140), lo23 = __byte_perm(z[j], t[j], 0x5140);
+        const uint32_t hi01 = __byte_perm(x[j], y[j], 0x7362), hi23 = __byte_perm(z[j], t[j], 0x7362);
+        acc[4 * j] = __dp4a((int)__byte_perm(lo01, lo23, 0x5410), v, acc[4 * j]);
+        acc[4 * j + 1] = __dp4a((int)__byte_perm(lo01, lo23, 0x7632), v, acc[4 * j + 1]);
+        acc[4 * j + 2] = __dp4a((int)__byte_perm(hi01, hi23, 0x5410), v, acc[4 * j + 2]);
+        acc[4 * j + 3] = __dp4a((int)__byte_perm(hi01, hi23, 0x7632), v, acc[4 * j + 3]);
+    }
+}
+
 template <int kLanes>
 __device__ __forceinline__ void RowDot8(const int32_t *__restrict__ colInd, const int8_t *__restrict__ val,
                                         const int8_t *__restrict__ Bslice, long long ldb, int s, int e, int trips,
                                         int32_t (&acc)[16])
 {
-    static_assert(kLanes >= 4, "a lane group holds whole quads of entries");
-    const int li = threadIdx.x & (kLanes - 1);
+    using Shape = Group8<kLanes>;
+    const int li = threadIdx.x & (Shape::kLanesOfRow - 1);
     for (int chunk = 0; chunk < trips; ++chunk) {
-        const int p0 = s + chunk * kLanes;
+        const int p0 = s + chunk * Shape::kChunk;
         const int rem = e - p0;
-        int myCol = 0, quad = 0;
-        if (li < rem) {
-            myCol = __ldcs(colInd + p0 + li);
-            quad = (int)(unsigned char)__ldcs(reinterpret_cast<const signed char *>(val) + p0 + li);
-        }
-        quad |= __shfl_down_sync(0xffffffffu, quad, 1, kLanes) << 8;
-        quad = (quad & 0xffff) | (__shfl_down_sync(0xffffffffu, quad, 2, kLanes) << 16);  // lanes 0, 4, 8, ...: four values
-        constexpr int kQuads = kLanes >= 8 ? 2 : 1;  // quads of B rows in flight per lane
+        if constexpr (Shape::kShare > 1) {
+            auto quadOf = [&](int first, int(&c)[4]) {  // columns and values of four entries of this lane
+                int quad = 0;
 #pragma unroll
-        for (int q0 = 0; q0 < kLanes; q0 += 4 * kQuads) {
-            if (!__any_sync(0xffffffffu, q0 < rem)) break;
-            uint32_t w[4 * kQuads][4];
-#pragma unroll
-            for (int u = 0; u < 4 * kQuads; ++u) {
-                const int c = __shfl_sync(0xffffffffu, myCol, q0 + u, kLanes);
-                const uint4 q = LoadB16(Bslice + (long long)c * ldb);
-                w[u][0] = q.x; w[u][1] = q.y; w[u][2] = q.z; w[u][3] = q.w;
-            }
-#pragma unroll
-            for (int h = 0; h < kQuads; ++h) {
-                const int v = __shfl_sync(0xffffffffu, quad, q0 + 4 * h, kLanes);
-                uint32_t(&x)[4] = w[4 * h], (&y)[4] = w[4 * h + 1], (&z)[4] = w[4 * h + 2], (&t)[4] = w[4 * h + 3];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint32_t lo01 = __byte_perm(x[j], y[j], 0x5140), lo23 = __byte_perm(z[j], t[j], 0x5140);
-                    const uint32_t hi01 = __byte_perm(x[j], y[j], 0x7362), hi23 = __byte_perm(z[j], t[j], 0x7362);
-                    acc[4 * j] = __dp4a((int)__byte_perm(lo01, lo23, 0x5410), v, acc[4 * j]);
-                    acc[4 * j + 1] = __dp4a((int)__byte_perm(lo01, lo23, 0x7632), v, acc[4 * j + 1]);
-                    acc[4 * j + 2] = __dp4a((int)__byte_perm(hi01, hi23, 0x5410), v, acc[4 * j + 2]);
-                    acc[4 * j + 3] = __dp4a((int)__byte_perm(hi01, hi23, 0x7632), v, acc[4 * j + 3]);
+                for (int u = 0; u < 4; ++u) {
+                    const int i = (first + u) * Shape::kShare + li / kLanes;
+                    c[u] = i < rem ? __ldcs(colInd + p0 + i) : 0;
+                    if (i < rem) quad |= (int)(unsigned char)__ldcs(reinterpret_cast<const signed char *>(val) + p0 + i) << (8 * u);
                 }
+                return quad;
+            };
+            auto rowsOf = [&](const int(&c)[4], uint32_t(&w)[4][4]) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const uint4 q = LoadB16(Bslice + (long long)c[u] * ldb);
+                    w[u][0] = q.x; w[u][1] = q.y; w[u][2] = q.z; w[u][3] = q.w;
+                }
+            };
+            int c0[4], c1[4];
+            uint32_t w0[4][4], w1[4][4];
+            const int v0 = quadOf(0, c0);
+            if (__any_sync(0xffffffffu, rem > 4 * Shape::kShare)) {
+                const int v1 = quadOf(4, c1);
+                rowsOf(c0, w0);
+                rowsOf(c1, w1);
+                DotQuad(w0[0], w0[1], w0[2], w0[3], v0, acc);
+                DotQuad(w1[0], w1[1], w1[2], w1[3], v1, acc);
+            } else {
+                rowsOf(c0, w0);
+                DotQuad(w0[0], w0[1], w0[2], w0[3], v0, acc);
+            }
+        } else {
+            int myCol = 0, quad = 0;
+            if (li < rem) {
+                myCol = __ldcs(colInd + p0 + li);
+                quad = (int)(unsigned char)__ldcs(reinterpret_cast<const signed char *>(val) + p0 + li);
+            }
+            quad |= __shfl_down_sync(0xffffffffu, quad, 1, kLanes) << 8;
+            quad = (quad & 0xffff) | (__shfl_down_sync(0xffffffffu, quad, 2, kLanes) << 16);  // lanes 0, 4, 8, ...: four values
+#pragma unroll
+            for (int q0 = 0; q0 < kLanes; q0 += 8) {  // two quads of B rows in flight per lane
+                if (!__any_sync(0xffffffffu, q0 < rem)) break;
+                uint32_t w[8][4];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int c = __shfl_sync(0xffffffffu, myCol, q0 + u, kLanes);
+                    const uint4 q = LoadB16(Bslice + (long long)c * ldb);
+                    w[u][0] = q.x; w[u][1] = q.y; w[u][2] = q.z; w[u][3] = q.w;
+                }
+                DotQuad(w[0], w[1], w[2], w[3], __shfl_sync(0xffffffffu, quad, q0, kLanes), acc);
+                DotQuad(w[4], w[5], w[6], w[7], __shfl_sync(0xffffffffu, quad, q0 + 4, kLanes), acc);
             }
         }
     }
@@ -671,10 +728,13 @@ __device__ __forceinline__ void StoreRowSlice(OutT *dst, const int32_t (&acc)[16
     }
 }
 
-__device__ __forceinline__ void CopyAsync16(void *dst, const void *src, bool on)  // zeros where not `on`
+template <int kBytes> __device__ __forceinline__ void CopyAsync(void *dst, const void *src, bool on)  // zeros where not `on`
 {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
-                 "r"(on ? 16 : 0) : "memory");
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if constexpr (kBytes == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(on ? 16 : 0) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(on ? 4 : 0) : "memory");
 }
 
 // A unit: a row of up to kLongRow entries, or that many of a longer one.  A warp sums kPieces * 16 bytes of the B rows of
@@ -687,18 +747,19 @@ template <int kLanes> struct UnitShape {
     static constexpr int kPieces = kLanes < 4 ? kLanes : 4;
     static constexpr int kRound = kPieces == 4 ? 16 : 32;            // entries per round
     static constexpr int kStages = 4;
-    static constexpr int kCopies = kRound * kPieces / 32;            // of a lane per round
     static constexpr int kStageBytes = kRound * kPieces * 16;
     static constexpr int kWarpBytes = kStages * (kStageBytes + kRound * 4);
 };
 
-template <typename ValT, typename OutT, bool kKahan, int kLanes>
+template <typename ValT, typename OutT, bool kKahan, int kLanes, bool kWords>
 __device__ void UnitSum(const FastArgs<ValT, OutT> &a, unsigned char *sWarp)
 {
     using Shape = UnitShape<kLanes>;
-    constexpr int kPieces = Shape::kPieces, kRound = Shape::kRound, kStages = Shape::kStages, kCopies = Shape::kCopies;
-    constexpr int E = Pack<ValT>::kElems;
+    constexpr int kPieces = Shape::kPieces, kRound = Shape::kRound, kStages = Shape::kStages;
     constexpr int kCols = 4 / (int)sizeof(ValT);  // columns of a word
+    constexpr int kCopyBytes = kWords ? 4 : 16;
+    constexpr int kPerEntry = kPieces * 16 / kCopyBytes;
+    constexpr int kCopies = kRound * kPerEntry / 32;  // of a lane per round
     const int lane = threadIdx.x & 31;
     const long long at = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
     const int unit = (int)(at / a.slices), slice = (int)(at - (long long)unit * a.slices);
@@ -710,9 +771,9 @@ __device__ void UnitSum(const FastArgs<ValT, OutT> &a, unsigned char *sWarp)
     const int rounds = (length + kRound - 1) / kRound;
     unsigned char *sData = sWarp;                                                                     // [kStages][kStageBytes]
     float *sVal = reinterpret_cast<float *>(sWarp + kStages * Shape::kStageBytes);                    // [kStages][kRound]
-    const int piece = lane & (kPieces - 1);
-    const bool live = (slice * kPieces + piece) * E < a.nB;
-    const ValT *Bs = a.B + (live ? (slice * kPieces + piece) * E : 0);
+    const int first = slice * kPieces * 4 * kCols + (lane & (kPerEntry - 1)) * (kCopyBytes / (int)sizeof(ValT));
+    const bool live = first < a.nB;
+    const ValT *Bs = a.B + (live ? first : 0);
 
     struct Batch {  // of kStages rounds; lane l holds entry l of each
         int col[kStages];
@@ -731,10 +792,10 @@ __device__ void UnitSum(const FastArgs<ValT, OutT> &a, unsigned char *sWarp)
         if (round < rounds) {
 #pragma unroll
             for (int u = 0; u < kCopies; ++u) {
-                const int entry = u * (32 / kPieces) + lane / kPieces;
+                const int entry = u * (32 / kPerEntry) + lane / kPerEntry;
                 const int c = __shfl_sync(0xffffffffu, b.col[i], entry);
-                CopyAsync16(sData + i * Shape::kStageBytes + (u * 32 + lane) * 16, Bs + c * a.ldb,
-                            live && round * kRound + entry < length);
+                CopyAsync<kCopyBytes>(sData + i * Shape::kStageBytes + (u * 32 + lane) * kCopyBytes, Bs + c * a.ldb,
+                                      live && round * kRound + entry < length);
             }
             if (lane < kRound) sVal[i * kRound + lane] = b.val[i];
         }
@@ -849,25 +910,33 @@ __device__ void UnitSum(const FastArgs<ValT, OutT> &a, unsigned char *sWarp)
 // CSR order; longer rows are units, at the front of the grid.  A lane past the end of a B row works on the
 // row's first columns once more and stores nothing.
 //
-// kGenC: C is column-major or not 16-byte aligned.  Sums then go through shared memory and are written along the
+// kLayout: kPlain wants C row-major with 16-byte aligned rows, like B; kAnyC takes any C, kAnyCWords also rows of B on
+// any 4-byte boundaries, by words (see WorthRepacking).  Sums of kAnyC go through shared memory and are written along the
 // contiguous direction of C: by a warp where that is the row's, else by the CTA, which takes a.genRows rows (of
 // column-major fp16 C, 32 rows are 64 bytes; straight from registers every element would be a 32-byte sector of its
 // own) unless there are too few rows to give every SM a CTA.
 template <typename ValT, int kLanes> struct FastShape {
     static constexpr int kTileCols = kLanes * Pack<ValT>::kElems;
-    static constexpr int kCtaRows = kWarps * (32 / kLanes);                   // rows of A per pass of the CTA
+    static constexpr int kGroup = std::is_same_v<ValT, int8_t> ? Group8<kLanes>::kLanesOfRow : kLanes;  // lanes of a row of A
+    static constexpr int kCtaRows = kWarps * (32 / kGroup);                   // rows of A per pass of the CTA
     static constexpr int kFit = 8192 / kTileCols < 32 ? 8192 / kTileCols : 32;  // at most 32 KB of tile
     static constexpr int kGenRows = kCtaRows > kFit ? kCtaRows : kFit;
 };
 
-template <typename ValT, typename OutT, bool kKahan, int kLanes, bool kGenC>
-__global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, OutT> a)
+enum { kPlain, kAnyC, kAnyCWords };
+// Rows of a few entries are a chain of dependent loads (row offsets, columns, B, C): warps hide it, so registers are held to
+// what 36 warps per SM leave (24 for wide int8 rows, whose quads of B rows need more).
+template <typename ValT, int kLanes> constexpr int kFastCtas = std::is_same_v<ValT, int8_t> && kLanes >= 8 ? 6 : 9;
+template <typename ValT, typename OutT, bool kKahan, int kLanes, int kLayout>
+__global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKernel(const FastArgs<ValT, OutT> a)
 {
     using Acc = typename Arith<ValT>::Acc;
     using Shape = FastShape<ValT, kLanes>;
     constexpr bool kInt8 = std::is_same_v<ValT, int8_t>;
+    constexpr bool kGenC = kLayout != kPlain, kWords = kLayout == kAnyCWords;
     constexpr int E = Pack<ValT>::kElems;
-    constexpr int kRowsPerWarp = 32 / kLanes;
+    constexpr int kGroup = Shape::kGroup;
+    constexpr int kRowsPerWarp = 32 / kGroup;
     constexpr int kTileCols = Shape::kTileCols;
     constexpr int kTileStride = kTileCols + 1;
     constexpr int kWarpWords = kInt8 ? 32 * E : UnitShape<kLanes>::kWarpBytes / 4;  // what a warp keeps of a unit
@@ -880,10 +949,11 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int li = lane & (kLanes - 1);
+    const bool owner = (lane & (kGroup - 1)) < kLanes;  // of the row's sums once they are joined
     const bool isUnit = (int)blockIdx.x < a.unitCtas;
     if constexpr (!kInt8) {
         if (isUnit) {
-            UnitSum<ValT, OutT, kKahan, kLanes>(a, reinterpret_cast<unsigned char *>(sBuf + warp * kWarpWords));
+            UnitSum<ValT, OutT, kKahan, kLanes, kWords>(a, reinterpret_cast<unsigned char *>(sBuf + warp * kWarpWords));
             return;
         }
     }
@@ -895,17 +965,22 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
         *dst = Finish<OutT>(v, alpha, beta, dst);
     };
 
+    constexpr int kCols = kInt8 ? 1 : 4 / (int)sizeof(ValT);
+    auto columnOf = [&](int colT, int i) {  // that acc[i] of this lane is for
+        return kWords ? colT + (i / kCols * kLanes + li) * kCols + i % kCols : colT + li * E + i;
+    };
+
     const bool splitRow = kInt8 && a.splitRows && !isUnit;
     if (!isUnit && !splitRow) {
         // ---- one lane group per row ----
-        constexpr int kChunk = kInt8 ? kLanes : Chunk<kLanes>::kChunk;
+        constexpr int kChunk = kInt8 ? Group8<kLanes>::kChunk : Chunk<kLanes>::kChunk;
         const bool rowsRun = kGenC && a.cCol != 1;  // column-major C
         const int blockRows = rowsRun ? a.genRows : Shape::kCtaRows;
         const long long row0 = (long long)(blockIdx.x - a.unitCtas) * blockRows;
         for (int col0 = 0; col0 < (rowsRun ? a.n : 1); col0 += kTileCols) {  // column-major C: a tile of columns at a time
 #pragma unroll 1
             for (int pass = 0; pass < blockRows; pass += Shape::kCtaRows) {
-                const int rowIn = pass + warp * kRowsPerWarp + lane / kLanes;
+                const int rowIn = pass + warp * kRowsPerWarp + lane / kGroup;
                 const long long row = row0 + rowIn;
                 int s = 0, e = 0;
                 bool skip = row >= a.m;
@@ -919,7 +994,7 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
                 }
                 int trips = (e - s + kChunk - 1) / kChunk;
 #pragma unroll
-                for (int off = kLanes; off < 32; off <<= 1) {
+                for (int off = kGroup; off < 32; off <<= 1) {
                     const int other = __shfl_xor_sync(0xffffffffu, trips, off);
                     trips = other > trips ? other : trips;
                 }
@@ -930,9 +1005,24 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
                     Acc acc[E], comp[E];
 #pragma unroll
                     for (int i = 0; i < E; ++i) acc[i] = comp[i] = Acc(0);
-                    const ValT *Bs = a.B + (colLive ? col : 0);
-                    if constexpr (kInt8) RowDot8<kLanes>(a.colInd, a.val, Bs, a.ldb, s, e, trips, acc);
-                    else RowDot<ValT, kKahan, kLanes>(a.colInd, a.val, Bs, a.ldb, s, e, trips, a.negZeros, acc, comp);
+                    if constexpr (kInt8) {
+                        RowDot8<kLanes>(a.colInd, a.val, a.B + (colLive ? col : 0), a.ldb, s, e, trips, acc);
+#pragma unroll
+                        for (int i = 0; i < E; ++i) {
+                            if (kLanes == 1 && i >= a.n) break;
+#pragma unroll
+                            for (int off = kLanes; off < kGroup; off <<= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], off);
+                        }
+                    } else {
+                        Slice<ValT, kWords> slice;
+                        if constexpr (kWords) {
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) slice.first[j] = columnOf(colT, j * kCols) < a.n ? columnOf(colT, j * kCols) : 0;
+                        } else {
+                            slice.first[0] = colLive ? col : 0;
+                        }
+                        RowDot<ValT, kKahan, kLanes, kWords>(a.colInd, a.val, a.B, slice, a.ldb, s, e, trips, a.negZeros, acc, comp);
+                    }
                     if (kKahan) {
 #pragma unroll
                         for (int i = 0; i < E; ++i) acc[i] -= comp[i];
@@ -940,23 +1030,29 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
                     if constexpr (kGenC) {
                         if (rowsRun) {
 #pragma unroll
-                            for (int i = 0; i < E; ++i) sBuf[rowIn * kTileStride + li * E + i] = acc[i];
+                            for (int i = 0; i < E; ++i)
+                                if (owner) sBuf[rowIn * kTileStride + columnOf(0, i)] = acc[i];
                             if (li == 0) sSkip[rowIn] = skip;
+                        } else if constexpr (kWords && kLanes >= 8) {  // a group writes whole sectors: consecutive lanes hold consecutive words
+#pragma unroll
+                            for (int i = 0; i < E; ++i)
+                                if (!skip && columnOf(colT, i) < a.n) storeOne(row, columnOf(colT, i), acc[i]);
                         } else {
                             Acc *sWarp = sBuf + warp * 32 * E;
                             const unsigned skipped = __ballot_sync(0xffffffffu, skip);
                             __syncwarp();
 #pragma unroll
-                            for (int i = 0; i < E; ++i) sWarp[lane * E + i] = acc[i];
+                            for (int i = 0; i < E; ++i)
+                                if (owner) sWarp[lane / kGroup * kTileCols + columnOf(0, i)] = acc[i];
                             __syncwarp();
 #pragma unroll
-                            for (int i = lane; i < 32 * E; i += 32) {
+                            for (int i = lane; i < kRowsPerWarp * kTileCols; i += 32) {
                                 const int g = i / kTileCols, c = colT + i % kTileCols;
-                                if (c < a.n && !(skipped >> (g * kLanes) & 1)) storeOne(row0 + warp * kRowsPerWarp + g, c, sWarp[i]);
+                                if (c < a.n && !(skipped >> (g * kGroup) & 1)) storeOne(row0 + warp * kRowsPerWarp + g, c, sWarp[i]);
                             }
                         }
                     } else {
-                        if (!skip && colLive) StoreRowSlice(a.C + row * a.ldc + col, acc, alpha, beta);
+                        if (!skip && colLive && owner) StoreRowSlice(a.C + row * a.ldc + col, acc, alpha, beta);
                     }
                 }
             }
@@ -983,13 +1079,14 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
         if (splitRow && rowEnd - rowStart > a.rowLimit) return;
         const int segStart = rowStart + seg.seg * kSegNnz;
         const int segEnd = rowEnd - segStart > kSegNnz ? segStart + kSegNnz : rowEnd;
-        // inside a warp the lane groups take interleaved kLanes-wide chunks of the warp's quarter
+        // inside a warp the lane groups take interleaved chunks of the warp's quarter
         const int quarter = ((segEnd - segStart + 4 * kWarps - 1) / (4 * kWarps)) * 4;
         int ws = segStart + warp * quarter;
         int we = ws + quarter;
         if (ws > segEnd) ws = segEnd;
         if (we > segEnd) we = segEnd;
-        const int g = lane / kLanes;
+        constexpr int kChunk = Group8<kLanes>::kChunk;
+        const int g = lane / kGroup;
         Acc *partial = static_cast<Acc *>(a.partials) + (long long)(lr.partBase + seg.seg) * a.n;
         auto storeSlice = [&](int col, const Acc (&v)[E]) {
             if constexpr (kGenC) {
@@ -1008,11 +1105,11 @@ __global__ void __launch_bounds__(kThreads) SpmmFastKernel(const FastArgs<ValT, 
 #pragma unroll
             for (int i = 0; i < E; ++i) acc[i] = Acc(0);
             // group g walks chunks g, g + kRowsPerWarp, ... of [ws, we)
-            const int nChunks = (we - ws + kLanes - 1) / kLanes;
+            const int nChunks = (we - ws + kChunk - 1) / kChunk;
             for (int ch0 = 0; ch0 < nChunks; ch0 += kRowsPerWarp) {  // same trip count in every group
                 const int ch = ch0 + g;
-                const int cs = ws + ch * kLanes < we ? ws + ch * kLanes : we;
-                const int ce = cs + kLanes < we ? cs + kLanes : we;
+                const int cs = ws + ch * kChunk < we ? ws + ch * kChunk : we;
+                const int ce = cs + kChunk < we ? cs + kChunk : we;
                 RowDot8<kLanes>(a.colInd, a.val, a.B + (colLive ? col : 0), a.ldb, cs, ce, 1, acc);
             }
 #pragma unroll
@@ -1765,6 +1862,11 @@ int LaunchRowStream(const StreamArgs<ValT, OutT> &sa, cudaStream_t stream)
 // B rows contiguous in memory: (N, row-major) or (T, column-major).
 bool RowsContiguous(int opB, int orderB) { return (opB != 0) == (orderB != 0); }
 
+bool RowsOfWords(const b200spSpmmShape *sh, int valBytes)  // fp types only: int8 products take 16 bytes at a time
+{
+    return RowsContiguous(sh->op_b, sh->order_b) && (valBytes == 4 || (valBytes == 2 && sh->n % 2 == 0 && sh->ldb % 2 == 0));
+}
+
 // Bytes of a repacked B, 0 when its layout is the kernels' own.  From sizes and layout alone, never from the pointer:
 // a caller may size the buffer before B exists (an unaligned B then goes to the generic kernel).
 size_t RepackBytes(const b200spSpmmShape *sh, int valBytes)
@@ -1774,11 +1876,17 @@ size_t RepackBytes(const b200spSpmmShape *sh, int valBytes)
     return (size_t)sh->k * (size_t)((sh->n + E - 1) / E) * 16;
 }
 
-// Repacking reads and writes k * n elements; the generic kernel touches nnz * n of them, a sector each when the
-// columns of B are the contiguous ones and otherwise with one load per product instead of one per 16 bytes.  From
-// two entries per row of B on the copy is the cheaper side by far (65,537 x 50,001 with 24 entries a row, fp16,
-// N = 40 in column-major order: generic 257 us, copy + product 57 us).
-bool WorthRepacking(const b200spSpmmShape *sh) { return sh->nnz >= 2 * sh->k; }
+// Repacking reads and writes k * n elements; the generic kernel reads nnz * n of them, with a load per product instead
+// of one per 16 bytes, and a 32-byte sector per load where the columns of B are the contiguous ones: there the copy is
+// fewer bytes from nnz = k * valBytes / 16 on (65,537 x 50,001 with 24 entries a row, fp16, N = 40: generic 257 us, copy
+// and product 50 us).  Rows on 4-byte boundaries can be read where they are: 298,261 rows of 6 entries, fp32, N = 150, k =
+// 737,797: 579 us with the copy, 408 us without; 415,892 power-law rows of 10, bf16, N = 50: 203 and 245 us.
+bool WorthRepacking(const b200spSpmmShape *sh, int valBytes)
+{
+    if (RowsOfWords(sh, valBytes)) return sh->nnz >= 8 * sh->k;
+    if (RowsContiguous(sh->op_b, sh->order_b)) return sh->nnz >= sh->k;
+    return 16 * sh->nnz >= sh->k * valBytes;
+}
 
 template <typename ValT, typename OutT>
 int LaunchGeneric(const int32_t *rowPtr, const int32_t *colInd, const void *val, const void *B, void *C,
@@ -1810,13 +1918,19 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
     constexpr bool kInt8 = std::is_same_v<ValT, int8_t>;
     constexpr int E = Pack<ValT>::kElems;
     const size_t repack = RepackBytes(sh, (int)sizeof(ValT));
-    // A product of one wave, with no row above MidRowLimit, takes less time than the second launch.
-    const bool small = sh->m * sh->n < 148ll * 2048 && segments + sh->mid_units == 0;
-    const bool bReady = repack == 0 ? Aligned16(B) : (sh->repack_bytes >= (int64_t)repack && WorthRepacking(sh) && !small);
+    // A product of one wave of short rows takes less time than the second launch.
+    const bool small = sh->m * sh->n < 148ll * 2048 && segments + sh->mid_units == 0 && sh->nnz <= 16 * sh->m;
+    const bool vectors = RowsContiguous(sh->op_b, sh->order_b) && sh->n % E == 0 && sh->ldb % E == 0 && Aligned16(B);
+    const bool copy = repack > 0 && sh->repack_bytes >= (int64_t)repack && WorthRepacking(sh, (int)sizeof(ValT)) && !small;
+    const bool words = !vectors && !copy && RowsOfWords(sh, (int)sizeof(ValT)) && reinterpret_cast<uintptr_t>(B) % 4 == 0;
+    // Rows of four entries leave the generic kernel, with a thread per output, nothing to wait for one after the other
+    // (695,764 of them, fp32, N = 11: 70 us; by words 79).
+    const bool few = words && sh->n <= 16 && sh->nnz <= 4 * sh->m && segments + sh->mid_units == 0;
+    const bool bReady = vectors || (words && !few) || copy;
     if (plan == nullptr || !bReady)
         return LaunchGeneric<ValT, OutT>(rowPtr, colInd, val, B, C, sh, s, stream);
     if (sh->m == 0 || sh->n == 0) return 0;
-    const bool cPlain = sh->order_c == 0 && sh->n % E == 0 && sh->ldc % E == 0 && Aligned16(C);
+    const bool cPlain = !words && sh->order_c == 0 && sh->n % E == 0 && sh->ldc % E == 0 && Aligned16(C);
     const PlanLayout L = LayoutFor(sh->m, sh->nnz, sh->n);
     char *p = static_cast<char *>(plan);
     FastArgs<ValT, OutT> a;
@@ -1842,7 +1956,7 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
     a.rowLimit = sh->mid_units > 0 ? MidRowLimit(sh->m, sh->nnz, sh->n) : kLongRow;
     a.splitRows = 0;
     a.negZeros = kNegZeros;
-    if (repack > 0) {
+    if (copy) {
         const int vecs = (int)((sh->n + E - 1) / E);
         auto *out = reinterpret_cast<uint4 *>(p + L.total);
         cudaError_t e;
@@ -1862,9 +1976,16 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
         a.nB = vecs * E;
     }
     int midUnits = sh->mid_units;
-    constexpr int kMinLanes = kInt8 ? 4 : 1;
-    int lanes_ = kMinLanes;  // lanes side by side on a row of B
+    int lanes_ = 1;  // lanes side by side on a row of B
     while (lanes_ < 32 && lanes_ * E < sh->n) lanes_ <<= 1;
+    // Rows of several tiles: half as wide a group where that leaves a fifth fewer lanes idle in the last one (bf16, N = 277,
+    // 35,891 rows of 27: 162 us with 32 lanes, 122 with 16).  Narrower still loses more to rows of different lengths in one
+    // warp than it gains, except by words, which wait for more loads (N = 150 above: 542, 460 and 408 us).
+    if (!kInt8 && lanes_ == 32) {
+        auto padded = [&](int l) { return (sh->n + l * E - 1) / (l * E) * l; };
+        if (10 * padded(16) <= 8 * padded(32)) lanes_ = 16;
+        if (words && 10 * padded(8) < 9 * padded(lanes_)) lanes_ = 8;
+    }
     // Grid of SpmmFastKernel: CTAs for the units of long rows, for those of one row each, and for all rows.
     auto launchFast = [&](int longUnits, int midUnits, bool rowCtas, cudaStream_t st) {
         const int units = longUnits + midUnits;
@@ -1874,7 +1995,7 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             constexpr int kPieces = UnitShape<kLanes>::kPieces;
             a.longUnits = longUnits;
             a.nUnits = units;
-            a.slices = (a.nB / E + kPieces - 1) / kPieces;
+            a.slices = ((a.nB + E - 1) / E + kPieces - 1) / kPieces;
             const long long unitCtas = kInt8 ? units : ((long long)units * a.slices + kWarps - 1) / kWarps;
             a.unitCtas = (int)unitCtas;
             a.genRows = sh->m < 2ll * Shape::kGenRows * b200sp_sm_count() ? Shape::kCtaRows : Shape::kGenRows;
@@ -1882,17 +2003,23 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             const long long grid = unitCtas + (rowCtas ? (sh->m + rows - 1) / rows : 0);
             if (grid == 0) return;
             auto go = [&](auto kernel) { err = b200sp::LaunchChained(kernel, (unsigned)grid, kThreads, 0, st, a); };
+            auto pick = [&]<bool kKahan>() {
+                if (cPlain) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kPlain>);
+                if constexpr (!kInt8)
+                    if (words) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyCWords>);
+                go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyC>);
+            };
             if constexpr (std::is_same_v<ValT, float>) {
-                if (sh->kahan && cPlain) go(SpmmFastKernel<ValT, OutT, true, kLanes, false>);
-                else if (sh->kahan) go(SpmmFastKernel<ValT, OutT, true, kLanes, true>);
+                if (sh->kahan) pick.template operator()<true>();
+                else pick.template operator()<false>();
+            } else {
+                pick.template operator()<false>();
             }
-            if (!sh->kahan && cPlain) go(SpmmFastKernel<ValT, OutT, false, kLanes, false>);
-            else if (!sh->kahan) go(SpmmFastKernel<ValT, OutT, false, kLanes, true>);
             b200sp_note_launches(1);
         };
         switch (lanes_) {
-            case 1: if constexpr (kMinLanes <= 1) launch.template operator()<1>(); break;
-            case 2: if constexpr (kMinLanes <= 2) launch.template operator()<2>(); break;
+            case 1: launch.template operator()<1>(); break;
+            case 2: launch.template operator()<2>(); break;
             case 4: launch.template operator()<4>(); break;
             case 8: launch.template operator()<8>(); break;
             case 16: launch.template operator()<16>(); break;
@@ -1901,6 +2028,10 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
         return err;
     };
     if constexpr (kInt8) {
+        if (lanes_ <= 4) {  // 16 to 64 entries of a row are in flight as it is
+            a.rowLimit = kLongRow;
+            midUnits = 0;
+        }
         // Integer sums may be regrouped: where a warp per row would not fill the SMs and rows are long enough to be
         // shared, a CTA takes a row (4096 rows of 410 entries, N = 512: 104 us with a warp per row, 74 us so).
         a.splitRows = cPlain && sh->nnz >= 128 * sh->m && sh->m * lanes_ / 32 < 64ll * b200sp_sm_count();
@@ -2006,7 +2137,7 @@ size_t b200sp_spmm_plan_bytes(int64_t rows, int64_t nnz, int64_t n) { return Lay
 size_t b200sp_spmm_repack_bytes(const b200spSpmmShape *shape, int val_type)
 {
     const int bytes = val_type == B200SP_F32 ? 4 : val_type == B200SP_I8 ? 1 : 2;
-    return WorthRepacking(shape) ? RepackBytes(shape, bytes) : 0;
+    return WorthRepacking(shape, bytes) ? RepackBytes(shape, bytes) : 0;
 }
 
 int b200sp_spmm_analyze(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,

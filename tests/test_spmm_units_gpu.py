@@ -16,8 +16,8 @@ WIDTHS = [1, 4, 5, 8, 12, 16, 31, 40, 64, 100, 136, 300]
 
 def case(oracle, vt, ot, n, filler):
     rng = np.random.default_rng(n + filler)
-    # few rows: every row above 16 entries is a unit; enough for the SMs: those above 64, or above four times the mean
-    extra = 300 if filler == 3 else 148 * 2048 // n + 1
+    # few rows: every row above 16 entries is a unit; more: those above 64, or above four times the mean
+    extra = 300 if filler == 3 else 148 * 512 // max(n, 16) + 1
     lengths = rng.permutation(np.concatenate([EDGES, np.full(extra, filler)]))
     m, k = lengths.size, 9000
     return m, k, *compact_case(oracle, rng, m, k, n, lengths, vt, ot, 1.5, -0.5)
@@ -62,7 +62,7 @@ def test_compensated_sums(handle, device, oracle, n):
 @pytest.mark.parametrize("filler", [3, 60, 200])
 def test_int8(handle, device, oracle, filler, n, order):
     rng = np.random.default_rng(n + filler)
-    lengths = rng.permutation(np.concatenate([EDGES, np.full(300 if filler == 3 else 148 * 2048 // n + 1, filler)]))
+    lengths = rng.permutation(np.concatenate([EDGES, np.full(300 if filler == 3 else 148 * 512 // max(n, 16) + 1, filler)]))
     m, k = lengths.size, 2500
     rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
     ci = rng.integers(0, k, rp[-1]).astype(np.int32)
