@@ -288,7 +288,6 @@ def config_list(args, world: int) -> list[str]:
 NCU_TRAFFIC = {
     "c2": {"bytes": 280_800_000, "kernels": "SpmvLongBlockKernel + SpmvMediumShortKernel",
            "source": "profiles/spmv_binned_c2_powerlaw_f32.md"},
-    "c3": {"bytes": 352_300_000, "kernels": "SpmvShortRowsKernel", "source": "profiles/spmv_binned_c3_stencil27_f16.md"},
     "c4": {"bytes": 635_600_000, "kernels": "SpmmFastKernel", "source": "profiles/spmm_fast_c4_f32_n64.md"},
     "c5": {"bytes": 13_460_000_000, "kernels": "SpmmRowStreamKernel + SpmmLongBlockKernel",
            "source": "profiles/spmm_rowstream_c5_bf16_n256.md"},
@@ -324,7 +323,7 @@ def kernels_of(is_spmm: bool, launches_per_step: float, b_row_bytes: int, world:
         if plan[1] > 0:
             long_rows = " + SpmmLongBlockKernel (rows > 1024 nnz, block by block of B through L2, side stream)"
         elif plan[0] > 0:
-            long_rows = " + SpmmFastKernel (segment CTAs of rows > 1024 nnz, side stream)"
+            long_rows = " + SpmmFastKernel (units of rows > 1024 nnz, side stream)"
         else:
             long_rows = ""
         if b_row_bytes in (512, 1024):
@@ -332,7 +331,7 @@ def kernels_of(is_spmm: bool, launches_per_step: float, b_row_bytes: int, world:
         return "SpmmFastKernel" + (long_rows if plan[1] > 0 else "")
     if launches_per_step >= 2 + (world > 1):
         return "SpmvLongBlockKernel (side stream) + SpmvMediumShortKernel"
-    return "SpmvShortRowsKernel | SpmvMediumShortKernel | SpmvAllBinsKernel"
+    return "SpmvShortRowsKernel | SpmvStagedRowsKernel | SpmvMediumShortKernel | SpmvAllBinsKernel"
 
 
 def measure_config(name: str, args, env, head: bool) -> dict:
@@ -716,7 +715,7 @@ def aux_arm(args, synth, oracle):
         alg = 4 * (m + 1) + 16 * nnz  # col_ind and P: read once, written once
         workload = {"workload": "csrsort of the c2 pattern, columns shuffled inside every row", "rows": m, "nnz": nnz,
                     "workspace_bytes": int(size.value)}
-        kernels = "SegSortWarpKernel + SegSortCtaKernel (keys formed and split inside the sort)"
+        kernels = "RowSort{Short,Warp,Cta,Huge}Kernel"
     elif args.op == "csr2csc":
         d_v = to(A.values)
         o_v, o_ri = torch.empty_like(d_v), torch.empty_like(d_ci)
@@ -736,8 +735,7 @@ def aux_arm(args, synth, oracle):
         alg = 4 * (m + 1) + 8 * nnz + 4 * (n + 1) + 8 * nnz
         workload = {"workload": "csr2csc (numeric, fp32) of the c2 matrix", "rows": m, "cols": n, "nnz": nnz,
                     "workspace_bytes": int(size.value)}
-        kernels = ("ColumnHistogramKernel + Scan{BlockSums,Sums,Apply}Kernel + ScatterKeysKernel + "
-                   "SegSort{Warp,Cta}Kernel")
+        kernels = "radix sort by column: HistogramKernel + Scan{Tiles,Chunks}Kernel + ScatterKernel per pass"
     elif args.op in ("spmvop-alg1", "spmvop-alg2"):
         # the SpMVOp plan API (compensated row sums) on the c2 matrix, Z aliasing Y
         cfg = synth.config2()
@@ -799,7 +797,7 @@ def aux_arm(args, synth, oracle):
                     "gather_bytes": int(nnz) * 2 * k * 2,
                     "note": "the Y row of every entry is its own 512-byte read: the gather (nnz * 1 KB with X) is what "
                             "moves, the algorithmic bytes count X and Y once"}
-        kernels = "SddmmVecKernel"
+        kernels = "SddmmRowsKernel"
     ms = float(np.median(t))
     line = {"op": args.op, "metric": f"{args.op}_ms", "value": ms, "unit": "ms", "higher_is_better": False, "n_gpus": 1,
             "steps": K, "warmup": 3, "per_step_ms": {"min": float(t.min()), "median": ms, "max": float(t.max())},
