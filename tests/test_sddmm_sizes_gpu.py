@@ -1,0 +1,41 @@
+"""GPU: aclsparseSDDMM at the widths and entry counts where its row kernel changes (lanes and pieces of a row, several
+turns, odd fp16 widths, ends of a warp's tile of entries)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from test_sddmm_gpu import dense_operand, golden, run_sddmm
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+@pytest.mark.parametrize("pad", [0, 1])  # 1: rows that start on any element
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 7, 8, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 256, 257, 511, 512, 513, 1024, 1100])
+def test_widths(pkg, handle, device, k, pad, dtype):
+    rng = np.random.default_rng(k)
+    check(pkg, handle, device, rng, rng.integers(0, 9, 90), k, pad, dtype)
+
+
+@pytest.mark.parametrize("nnz", [1, 3, 4, 5, 31, 32, 33, 63, 64, 65, 129, 148 * 16 * 128 + 1])  # the last: tiles of 64 entries
+def test_entry_counts(pkg, handle, device, nnz):
+    rng = np.random.default_rng(nnz)
+    lengths = np.bincount(rng.integers(0, 50, nnz), minlength=50)
+    check(pkg, handle, device, rng, lengths, 24, 0, "f16")
+
+
+def check(pkg, handle, device, rng, lengths, k, pad, dtype):
+    m, n = lengths.size, 300
+    rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    ci = rng.integers(0, n, rp[-1]).astype(np.int32)
+    X, xs, ldx = dense_operand(rng, m, k, "row", pad, dtype)
+    Yt, ys, ldy = dense_operand(rng, n, k, "row", pad, dtype)
+    c0 = rng.uniform(-1.0, 1.0, ci.size).astype(np.float32)
+    if dtype == "f16":
+        c0 = c0.astype(np.float16).astype(np.float32)
+    got = run_sddmm(pkg, handle, device, rp, ci, c0, (xs, m, k, ldx), (ys, n, k, ldy), 1.5, -0.5, m, n, False, True,
+                    "row", "row", dtype)
+    want, scale = golden(rp, ci, c0, X, np.ascontiguousarray(Yt.T), 1.5, -0.5)
+    tol = 1e-5 * scale + 1e-30 if dtype == "f32" else 2e-3 * scale + np.abs(want) * 2.0 ** -11 + 2.0 ** -25
+    assert np.all(np.abs(got - want) <= tol)
