@@ -86,8 +86,8 @@ int b200sp_spmv_launch(const int32_t *row_ptr, const int32_t *col_ind, const voi
 
 /* The same product for a matrix that was not analysed, with nothing to analyse first: a kernel over the rows and a second
  * one for the segments of the rows above 1024 entries, which the first lists in `scratch`
- * (b200sp_spmv_rows_bytes(nnz) bytes, contents arbitrary).  `state` is two ints of device memory that are zero before the
- * first product; every product leaves them zero.  Two products that can overlap need a scratch and a state each. */
+ * (b200sp_spmv_rows_bytes(nnz) bytes, contents arbitrary).  Two products that can overlap need a scratch each.  `state` is
+ * not used (the list needs no counter) and may be NULL. */
 size_t b200sp_spmv_rows_bytes(int64_t nnz);
 int b200sp_spmv_rows_launch(const int32_t *row_ptr, const int32_t *col_ind, const void *val, const void *x, void *y, int64_t rows,
                             int64_t nnz, const b200spScalars *scalars, int comp_type, int val_type, int out_type, void *scratch,

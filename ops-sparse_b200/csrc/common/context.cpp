@@ -66,20 +66,12 @@ aclsparseStatus_t aclsparseCreate(aclsparseHandle_t *handle)
         delete ctx;
         return ACL_SPARSE_STATUS_NOT_INITIALIZED;
     }
-    if (cudaMalloc(&ctx->ownedWorkspace, b200sp::kDefaultWorkspaceBytes + b200sp::kStateBytes) != cudaSuccess) {
+    if (cudaMalloc(&ctx->ownedWorkspace, b200sp::kDefaultWorkspaceBytes) != cudaSuccess) {
         (void)cudaGetLastError();
         delete ctx;
         return ACL_SPARSE_STATUS_ALLOC_FAILED;
     }
     ctx->ownedWorkspaceBytes = b200sp::kDefaultWorkspaceBytes;
-    ctx->productState = reinterpret_cast<int32_t *>(static_cast<char *>(ctx->ownedWorkspace) + b200sp::kDefaultWorkspaceBytes);
-    // on a stream of its own order: done before any product of this handle can be enqueued, on whatever stream
-    if (cudaMemset(ctx->productState, 0, b200sp::kStateBytes) != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess) {
-        (void)cudaGetLastError();
-        (void)cudaFree(ctx->ownedWorkspace);
-        delete ctx;
-        return ACL_SPARSE_STATUS_ALLOC_FAILED;
-    }
     *handle = ctx;
     return ACL_SPARSE_STATUS_SUCCESS;
 }

@@ -19,7 +19,6 @@
 namespace b200sp {
 
 constexpr size_t kDefaultWorkspaceBytes = 4u << 20;  // reference: ACLSPARSE_DEFAULT_WORKSPACE_SIZE, 4 MiB
-constexpr size_t kStateBytes = 256;                  // behind the owned workspace, see productState
 constexpr int kLibraryVersion = 10000;               // reference: ACLSPARSE_VERSION
 constexpr uint32_t kDnVecMagic = 0xD0D2D4D6u;        // reference: kDnVecSignature, aclsparse_descr.cpp:29
 
@@ -86,7 +85,6 @@ struct aclsparseContext {
     size_t userWorkspaceBytes = 0;
     bool userWorkspaceActive = false;
     int device = 0;
-    int32_t *productState = nullptr;  // behind the owned workspace: zero between products (b200sp_spmv_rows_launch)
 
     void *Workspace() const { return userWorkspaceActive ? userWorkspace : ownedWorkspace; }
     size_t WorkspaceBytes() const { return userWorkspaceActive ? userWorkspaceBytes : ownedWorkspaceBytes; }

@@ -282,18 +282,11 @@ aclsparseStatus_t aclsparseSpMV(aclsparseHandle_t handle, aclsparseOperation_t o
             // kernel with a plan per call.
             const size_t listBytes = b200sp_spmv_rows_bytes(matA->nnz);
             char *scratch = static_cast<char *>(externalBuffer);
-            int32_t *state = handle->productState;
-            if (scratch != nullptr) {  // nothing of the handle is shared then: its stream may change between products
-                state = reinterpret_cast<int32_t *>(scratch);
-                scratch += b200sp::kStateBytes;
-                if (cudaMemsetAsync(state, 0, b200sp::kStateBytes, stream) != cudaSuccess) return ACL_SPARSE_STATUS_EXECUTION_FAILED;
-            } else if (handle->WorkspaceBytes() >= listBytes) {
-                scratch = static_cast<char *>(handle->Workspace());
-            }
+            if (scratch == nullptr && handle->WorkspaceBytes() >= listBytes) scratch = static_cast<char *>(handle->Workspace());
             if (scratch != nullptr) {
-                (void)b200sp::NoteBufferWrite(externalBuffer != nullptr ? externalBuffer : scratch);  // a plan recorded for this buffer, of any matrix, is stale now
+                (void)b200sp::NoteBufferWrite(scratch);  // a plan recorded for this buffer, of any matrix, is stale now
                 rc = b200sp_spmv_rows_launch(rowPtr, colInd, matA->values, vecX->values, vecY->values, matA->rows, matA->nnz, &sc,
-                                             c.compType, c.valType, c.outType, scratch, state, stream);
+                                             c.compType, c.valType, c.outType, scratch, nullptr, stream);
                 if (rc != 0) {
                     B200SP_LOGE("aclsparseSpMV: kernel launch failed (cuda error %d)", rc);
                     return ACL_SPARSE_STATUS_EXECUTION_FAILED;

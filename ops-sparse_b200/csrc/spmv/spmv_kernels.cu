@@ -1127,19 +1127,25 @@ __global__ void __launch_bounds__(256, 6) SpmvAllBinsKernel(const int32_t *__res
 // two launches.  7.2 M gathers at one per clock and SM are 26 us.
 constexpr int kGroupTrips = 4;
 constexpr int kListedRow = 1024;
+// A listed row writes its segments into the slots of the multiples of kListedRow among its entry numbers: it has one at
+// least, and enough for its segments, and no other row has them.  So there is no counter that a product would have to find
+// at zero, and whatever an earlier product (one cut short, or of another matrix) left in the slots is harmless: the second
+// kernel takes an item only if the row offsets bear it out, and then it is what the first kernel wrote there.
 struct RowList {              // what the first kernel leaves for the second
-    int32_t *state;           // {segments listed, CTAs of the second kernel done}; zero between products
     int2 *items;              // {row, segment}; a row's segments are consecutive
     int32_t *counters;        // arrivals, at the first segment of a row
     void *partials;           // one compute-type value per segment
+    int slots;
 };
-inline int64_t RowListItems(int64_t nnz) { return nnz / kListedRow + 1; }  // a row of n > kListedRow entries has n / kSegLen + 1 segments
+inline int64_t RowListItems(int64_t nnz) { return nnz / kListedRow + 1; }
+__device__ __forceinline__ int RowListSlot(int start) { return (int)(((unsigned)start + (kListedRow - 1)) / kListedRow); }
 inline size_t RowListBytes(int64_t nnz) { return (size_t)RowListItems(nnz) * 16 + 512; }
-inline RowList RowListIn(void *scratch, int32_t *state, int64_t nnz)
+inline RowList RowListIn(void *scratch, int64_t nnz)
 {
     const size_t n = AlignUp((size_t)RowListItems(nnz) * 8, 256);
-    char *p = static_cast<char *>(scratch);
-    return {state, reinterpret_cast<int2 *>(p), reinterpret_cast<int32_t *>(p + n), p + n + (size_t)RowListItems(nnz) * 4};
+    char *p = reinterpret_cast<char *>(AlignUp(reinterpret_cast<size_t>(scratch), 8));  // the caller's may start on any word
+    return {reinterpret_cast<int2 *>(p), reinterpret_cast<int32_t *>(p + n), p + n + (size_t)RowListItems(nnz) * 4,
+            (int)RowListItems(nnz)};
 }
 
 // kList false: rows of kLongLen entries and more are somebody else's and not listed.
@@ -1161,7 +1167,7 @@ __global__ void __launch_bounds__(128, 16) SpmvRowsKernel(const int32_t *__restr
     const int len = e - s;
     if (kList && len > kListedRow && li == 0) {
         const int n = (len + kSegLen - 1) / kSegLen;
-        const int at = atomicAdd(list.state, n);
+        const int at = RowListSlot(s);
         list.counters[at] = 0;
         for (int k = 0; k < n; ++k) list.items[at + k] = make_int2((int)r, k);
     }
@@ -1219,75 +1225,84 @@ __global__ void __launch_bounds__(128, 16) SpmvRowsKernel(const int32_t *__restr
     }
 }
 
-// The listed segments, by CTAs that take them in turn.  The last CTA leaves the state as it was found: zero.
+// The listed segments.  Every CTA looks through its share of the slots, 256 at a time and strided, so that the segments of
+// one row go to different CTAs, and sums what it finds.
 template <typename CompT, typename ValT, typename OutT>
 __global__ void __launch_bounds__(256) SpmvListedKernel(const int32_t *__restrict__ rowPtr, const int32_t *__restrict__ colInd,
                                                         const ValT *__restrict__ val, const ValT *__restrict__ x,
-                                                        OutT *__restrict__ y, Scalars<CompT> sc, RowList list)
+                                                        OutT *__restrict__ y, int rows, Scalars<CompT> sc, RowList list)
 {
     __shared__ CompT sWarp[8];
-    __shared__ int sCount;
+    __shared__ int2 sItem[256];
+    __shared__ int sFound;
     const int tid = threadIdx.x;
     b200sp::WaitForPrevious();
-    const int count = *static_cast<volatile int32_t *>(list.state);
-    if (count == 0) return;
     const CompT beta = sc.Beta();
-    for (int i = blockIdx.x; i < count; i += gridDim.x) {
-        const int2 item = list.items[i];
-        const int rowStart = __ldg(rowPtr + item.x), rowEnd = __ldg(rowPtr + item.x + 1);
-        const int s = rowStart + item.y * kSegLen, e = s + kSegLen < rowEnd ? s + kSegLen : rowEnd;
-        const int segments = (rowEnd - rowStart + kSegLen - 1) / kSegLen;
-        CompT sum = CompT(0);
-        for (int p = s + tid; p < e; p += 8 * 256) {
-            int c[8];
-            ValT v[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const bool in = p + u * 256 < e;
-                c[u] = in ? __ldcs(colInd + p + u * 256) : 0;
-                v[u] = in ? __ldcs(val + p + u * 256) : ValT(0);
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const ValT xv = p + u * 256 < e ? __ldg(x + c[u]) : ValT(0);
-                sum += Widen<CompT>(v[u]) * Widen<CompT>(xv);
+    for (long long slot0 = blockIdx.x; slot0 < list.slots; slot0 += 256ll * gridDim.x) {
+        const long long slot = slot0 + (long long)tid * gridDim.x;
+        int2 found = make_int2(0, 0);
+        bool mine = false;
+        if (slot < list.slots) {
+            found = list.items[slot];
+            if (found.x >= 0 && found.x < rows && found.y >= 0) {
+                const int rowStart = __ldg(rowPtr + found.x), len = __ldg(rowPtr + found.x + 1) - rowStart;
+                mine = len > kListedRow && found.y < (len + kSegLen - 1) / kSegLen && RowListSlot(rowStart) + found.y == slot;
             }
         }
-        sum = GroupSum(sum, 32);
-        __syncthreads();  // sWarp may still be read for the segment before
-        if ((tid & 31) == 0) sWarp[tid >> 5] = sum;
+        if (tid == 0) sFound = 0;
+        if (__syncthreads_or(mine) == 0) continue;
+        if (mine) sItem[atomicAdd(&sFound, 1)] = found;
         __syncthreads();
-        if (tid == 0) {
-            CompT tot = CompT(0);
+        for (int i = 0; i < sFound; ++i) {
+            const int2 item = sItem[i];
+            const int rowStart = __ldg(rowPtr + item.x), rowEnd = __ldg(rowPtr + item.x + 1);
+            const int s = rowStart + item.y * kSegLen, e = rowEnd - s > kSegLen ? s + kSegLen : rowEnd;
+            const int segments = (rowEnd - rowStart + kSegLen - 1) / kSegLen;
+            CompT sum = CompT(0);
+            for (int p = s + tid; p < e; p += 8 * 256) {
+                int c[8];
+                ValT v[8];
 #pragma unroll
-            for (int w = 0; w < 8; ++w) tot += sWarp[w];
-            bool last = true;
-            if (segments > 1) {
-                const int first = i - item.y;
-                CompT *part = static_cast<CompT *>(list.partials) + first;
-                part[item.y] = tot;
-                __threadfence();
-                last = atomicAdd(list.counters + first, 1) == segments - 1;
-                if (last) {
-                    __threadfence();
-                    tot = CompT(0);
-                    for (int k = 0; k < segments; ++k) tot += __ldcg(part + k);  // segment order: the sum does not depend on timing
+                for (int u = 0; u < 8; ++u) {
+                    const bool in = p + u * 256 < e;
+                    c[u] = in ? __ldcs(colInd + p + u * 256) : 0;
+                    v[u] = in ? __ldcs(val + p + u * 256) : ValT(0);
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const ValT xv = p + u * 256 < e ? __ldg(x + c[u]) : ValT(0);
+                    sum += Widen<CompT>(v[u]) * Widen<CompT>(xv);
                 }
             }
-            if (last) {
-                CompT z = sc.Alpha() * tot;
-                if (beta != CompT(0)) z += beta * Widen<CompT>(y[item.x]);
-                y[item.x] = Narrow<OutT>(z);
+            sum = GroupSum(sum, 32);
+            __syncthreads();  // sWarp may still be read for the segment before
+            if ((tid & 31) == 0) sWarp[tid >> 5] = sum;
+            __syncthreads();
+            if (tid == 0) {
+                CompT tot = CompT(0);
+#pragma unroll
+                for (int w = 0; w < 8; ++w) tot += sWarp[w];
+                bool last = true;
+                if (segments > 1) {
+                    const int first = RowListSlot(rowStart);
+                    CompT *part = static_cast<CompT *>(list.partials) + first;
+                    part[item.y] = tot;
+                    __threadfence();
+                    last = atomicAdd(list.counters + first, 1) == segments - 1;
+                    if (last) {
+                        __threadfence();
+                        tot = CompT(0);
+                        for (int k = 0; k < segments; ++k) tot += __ldcg(part + k);  // segment order: the sum does not depend on timing
+                    }
+                }
+                if (last) {
+                    CompT z = sc.Alpha() * tot;
+                    if (beta != CompT(0)) z += beta * Widen<CompT>(y[item.x]);
+                    y[item.x] = Narrow<OutT>(z);
+                }
             }
         }
-    }
-    if (tid == 0) {
-        __threadfence();
-        sCount = atomicAdd(list.state + 1, 1);
-        if (sCount == (int)gridDim.x - 1) {
-            list.state[0] = 0;
-            list.state[1] = 0;
-        }
+        __syncthreads();  // sItem and sFound may be written again
     }
 }
 
@@ -1772,10 +1787,10 @@ int LaunchTransTyped(const int32_t *rowPtr, const int32_t *colInd, const void *v
 
 template <typename CompT, typename ValT, typename OutT>
 int LaunchRows(const int32_t *rowPtr, const int32_t *colInd, const void *val, const void *x, void *y, int64_t rows, int64_t nnz,
-               const b200spScalars *s, void *scratch, int32_t *state, cudaStream_t stream)
+               const b200spScalars *s, void *scratch, cudaStream_t stream)
 {
     const Scalars<CompT> sc = MakeScalars<CompT>(s);
-    const RowList list = RowListIn(scratch, state, nnz);
+    const RowList list = RowListIn(scratch, nnz);
     const auto *v = static_cast<const ValT *>(val), *xv = static_cast<const ValT *>(x);
     auto *yv = static_cast<OutT *>(y);
     if (rows == 0) return 0;
@@ -1796,7 +1811,7 @@ int LaunchRows(const int32_t *rowPtr, const int32_t *colInd, const void *val, co
     const int64_t most = nnz / (kListedRow + 1), cap = (int64_t)b200sp_sm_count() * 4;
     b200sp_note_launches(1);
     return (int)b200sp::LaunchChained(SpmvListedKernel<CompT, ValT, OutT>, (unsigned)(most < 1 ? 1 : most < cap ? most : cap), 256, 0,
-                                      stream, rowPtr, colInd, v, xv, yv, sc, list);
+                                      stream, rowPtr, colInd, v, xv, yv, (int)rows, sc, list);
 }
 
 // Calls f.template operator()<CompT, ValT, OutT>() for a supported type triple, or returns -1.
@@ -1943,9 +1958,10 @@ int b200sp_spmv_rows_launch(const int32_t *row_ptr, const int32_t *col_ind, cons
                             int64_t nnz, const b200spScalars *scalars, int comp_type, int val_type, int out_type, void *scratch,
                             int32_t *state, void *stream)
 {
+    (void)state;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int rc = DispatchTypes(comp_type, val_type, out_type, [&]<typename C, typename V, typename O>() {
-        return LaunchRows<C, V, O>(row_ptr, col_ind, val, x, y, rows, nnz, scalars, scratch, state, st);
+        return LaunchRows<C, V, O>(row_ptr, col_ind, val, x, y, rows, nnz, scalars, scratch, st);
     });
     return rc < 0 ? (int)cudaErrorInvalidValue : rc;
 }

@@ -71,3 +71,73 @@ def test_tile_sizes_of_the_entry_point_without_scratch(pkg, device, oracle, item
     want = oracle.spmv(rp, ci, val, x, y, 1.5, -0.5)
     scale = 1.5 * oracle.spmv_abs_rowsum(rp, ci, val, x) + 0.5 * np.abs(y) + 1e-12
     helpers.assert_rowwise(d[4].cpu().numpy().astype(np.float64), want.astype(np.float64), scale, helpers.TOL["f32"], "tiles")
+
+
+def whole_case(device, seed):
+    """An int32 matrix with listed rows of one and of several segments, and the product of it, on the GPU and exact."""
+    from ops_sparse_b200 import api, synth
+    rng = np.random.default_rng(seed)
+    lengths = np.concatenate([rng.integers(0, 9, 3000), [1025, 8193, 20000] * 3])
+    rng.shuffle(lengths)
+    m, n = lengths.size, 30000
+    A = synth.csr_from_lengths(rng, lengths, n, lambda r, k: r.integers(-9, 10, k))
+    val, x, y = A.values.astype(np.int32), rng.integers(-9, 10, n).astype(np.int32), rng.integers(-9, 10, m).astype(np.int32)
+    total = np.concatenate([[0], np.cumsum(val.astype(np.int64) * x[A.col_ind])])
+    want = (2 * (total[A.row_ptr[1:]] - total[A.row_ptr[:-1]]) - y).astype(np.int32)
+    dA = helpers.make_csr(device, A.row_ptr, A.col_ind, val, "i32", m, n)
+    return dA, api.DnVec(helpers.to_device(x, "i32", device)), lambda: api.DnVec(helpers.to_device(y, "i32", device)), want
+
+
+@pytest.mark.parametrize("offset", [0, 4])  # bytes from an aligned address: any word will do
+def test_scratch_with_anything_in_it(pkg, handle, device, offset):
+    """The list may hold whatever an unfinished product, or one of another matrix, left there."""
+    from ctypes import Structure, byref, c_float, c_int, c_int32, c_int64, c_size_t, c_void_p
+    from ops_sparse_b200 import api
+
+    class Scalars(Structure):  # b200spScalars
+        _fields_ = [("alpha_f", c_float), ("beta_f", c_float), ("alpha_i", c_int32), ("beta_i", c_int32),
+                    ("alpha_dev", c_void_p), ("beta_dev", c_void_p)]
+    dA, dx, make_y, want = whole_case(device, 1)
+    rows_bytes, launch = pkg.lib().b200sp_spmv_rows_bytes, pkg.lib().b200sp_spmv_rows_launch
+    rows_bytes.restype, rows_bytes.argtypes = c_size_t, [c_int64]
+    launch.restype = c_int
+    launch.argtypes = [c_void_p] * 5 + [c_int64] * 2 + [c_void_p] + [c_int] * 3 + [c_void_p] * 3
+    ptr = lambda t: c_void_p(t.data_ptr())
+    i32 = 3  # B200SP_I32
+    dB, dv, make_w, other = whole_case(device, 2)
+    bytes_ = max(rows_bytes(dA.nnz), rows_bytes(dB.nnz)) + offset
+    for fill in (0x00, 0x5A, 0xFF):
+        scratch = torch.full((bytes_,), fill, dtype=torch.uint8, device=device)[offset:]
+        state = torch.full((2,), 0x5A5A5A5A, dtype=torch.int32, device=device)
+        for M, dense, make, result in ((dA, dx, make_y, want), (dB, dv, make_w, other), (dA, dx, make_y, want)):
+            dy = make()
+            assert launch(ptr(M.row_ptr), ptr(M.col_ind), ptr(M.values), ptr(dense.values), ptr(dy.values), M.rows, M.nnz,
+                          byref(Scalars(alpha_i=2, beta_i=-1)), i32, i32, i32, ptr(scratch), ptr(state),
+                          c_void_p(handle.stream.cuda_stream)) == 0
+            assert np.array_equal(helpers.to_host(dy.values, "i32"), result)
+    dy = make_y()  # and through the interface, with a buffer of that alignment
+    buf = torch.full((api.spmv_buffer_size(handle, dA, dx, dy) + offset,), 0x5A, dtype=torch.uint8, device=device)[offset:]
+    api.spmv(handle, dA, dx, dy, 2, -1, buffer=buf)
+    assert np.array_equal(helpers.to_host(dy.values, "i32"), want)
+
+
+def test_handle_that_changes_its_stream(pkg, handle, device):
+    """Products without a buffer share the handle's workspace; in order, whatever the stream, each finds its own list."""
+    from ctypes import c_void_p
+    from ops_sparse_b200 import api
+    cases = [whole_case(device, seed) for seed in range(3)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    results = []
+    for i in range(12):
+        dA, dx, make_y, want = cases[i % 3]
+        dy = make_y()
+        torch.cuda.synchronize()
+        s, before = streams[i % 2], streams[(i + 1) % 2]
+        s.wait_stream(before)
+        assert pkg.lib().aclsparseSetStream(handle.raw, c_void_p(s.cuda_stream)) == 0
+        api.spmv(handle, dA, dx, dy, 2, -1)
+        results.append((dy, want))
+    torch.cuda.synchronize()
+    for dy, want in results:
+        assert np.array_equal(helpers.to_host(dy.values, "i32"), want)
