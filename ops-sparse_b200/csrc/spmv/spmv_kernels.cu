@@ -745,20 +745,24 @@ __global__ void __maxnreg__(48) SpmvLongBlockKernel(const LongBlockArgs<CompT, V
                         if (vv < ve) {
                             c[u] = __ldcs(reinterpret_cast<const int4 *>(a.colInd) + vv);
                             q[u] = LoadQuad(a.val + 4 * vv);
+                        } else {
+                            c[u] = make_int4(x0, x0, x0, x0);
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) q[u].v[k] = ValT(0);
                         }
                     }
+                    // Where a lane has no entry both factors are 0: x[x0] may be an infinity or a NaN.  (Selected, not
+                    // branched over: the power-law product takes 1.3 % longer with branches.)
 #pragma unroll
                     for (int u = 0; u < kUnroll; ++u) {
-                        if (v + kPieceLanes * u < ve) {  // not 0 * x[x0] instead: x[x0] may be an infinity or a NaN
-                            sum += Widen<CompT>(q[u].v[0]) * Widen<CompT>(xrel[c[u].x]);
-                            sum += Widen<CompT>(q[u].v[1]) * Widen<CompT>(xrel[c[u].y]);
-                            sum += Widen<CompT>(q[u].v[2]) * Widen<CompT>(xrel[c[u].z]);
-                            sum += Widen<CompT>(q[u].v[3]) * Widen<CompT>(xrel[c[u].w]);
-                        }
+                        const bool in = v + kPieceLanes * u < ve;
+                        const ValT xv[4] = {xrel[c[u].x], xrel[c[u].y], xrel[c[u].z], xrel[c[u].w]};
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) sum += Widen<CompT>(q[u].v[k]) * Widen<CompT>(in ? xv[k] : ValT(0));
                     }
                 }
-                if (doHead) sum += Widen<CompT>(vh) * Widen<CompT>(xrel[ch]);
-                if (doTail) sum += Widen<CompT>(vt) * Widen<CompT>(xrel[ct]);
+                const ValT xh = xrel[ch], xt = xrel[ct];
+                sum += Widen<CompT>(vh) * Widen<CompT>(doHead ? xh : ValT(0)) + Widen<CompT>(vt) * Widen<CompT>(doTail ? xt : ValT(0));
             } else {
                 for (int p = s + pl; p < e; p += kPieceLanes)
                     sum += Widen<CompT>(a.val[p]) * Widen<CompT>(xrel[a.colInd[p]]);
