@@ -181,21 +181,22 @@ __global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(
     }
     __syncwarp();
 
-    const int pieces = kOdd ? (k + 1) / 2 : k * (int)sizeof(T) / kBytes;
+    // unsigned: a row may hold 2^31 - 1 elements, and the last turn ends beyond its last piece
+    const unsigned pieces = kOdd ? ((unsigned)k + 1) / 2 : (unsigned)((long long)k * (int)sizeof(T) / kBytes);
     const int perGroup = tile / (32 / kLanes);
     const int t0 = group * perGroup;
     const int batches = perGroup / kBatch;
-    for (int piece0 = 0; piece0 < pieces; piece0 += kLanes * kSlabs - (kOdd ? 1 : 0)) {
+    for (unsigned piece0 = 0; piece0 < pieces; piece0 += kLanes * kSlabs - (kOdd ? 1 : 0)) {
         const int width = kLanes * kSlabs - (kOdd ? 1 : 0);
         auto copyRow = [&](Piece *slot, const char *row) {
 #pragma unroll
             for (int s = 0; s < kSlabs; ++s) {
-                const int q = piece0 + s * kLanes + li;
+                const unsigned q = piece0 + s * kLanes + li;
                 if constexpr (kOdd) {  // words from the one that holds the first element on, zeros after the row's last
                     const int off = (int)(reinterpret_cast<uintptr_t>(row) & 2);
-                    const int left = 2 * k + off - 4 * q;
-                    const int bytes = left >= 4 ? 4 : left > 0 ? left : 0;
-                    CopyAsync<4>(slot + s * 32 + lane, row - off + (bytes > 0 ? 4 * q : 0), bytes);
+                    const unsigned end = (unsigned)k + (unsigned)off / 2;  // of the row, in elements from the first word on
+                    const int bytes = end >= 2 * q + 2 ? 4 : end > 2 * q ? 2 : 0;
+                    CopyAsync<4>(slot + s * 32 + lane, row - off + (bytes > 0 ? 4ll * q : 0), bytes);
                 } else {
                     const bool in = q < pieces;
                     CopyAsync<kCopy>(slot + s * 32 + lane, row + (in ? (long long)q * kBytes : 0), in ? kCopy : 0);
@@ -382,7 +383,7 @@ int LaunchRows(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const
 {
     const int nnz = (int)C->nnz;
     // pieces of a row, one more where they start in the middle of a word
-    const int pieces = kBytes == 2 ? (k + 1) / 2 + 1 : (int)((long long)k * (long long)sizeof(T) / kBytes);
+    const long long pieces = kBytes == 2 ? ((long long)k + 1) / 2 + 1 : (long long)k * (long long)sizeof(T) / kBytes;
     // The longer the tile the longer the runs of copies in flight, as long as every SM gets some 16 warps.
     int tile = 32;
     while (tile < kSddmmTile && nnz / (2 * tile) >= 16 * b200sp_sm_count()) tile *= 2;

@@ -39,3 +39,22 @@ def check(pkg, handle, device, rng, lengths, k, pad, dtype):
     want, scale = golden(rp, ci, c0, X, np.ascontiguousarray(Yt.T), 1.5, -0.5)
     tol = 1e-5 * scale + 1e-30 if dtype == "f32" else 2e-3 * scale + np.abs(want) * 2.0 ** -11 + 2.0 ** -25
     assert np.all(np.abs(got - want) <= tol)
+
+
+def test_odd_rows_of_two_gigabytes(pkg, handle, device):
+    """A width whose bytes do not fit 31 bits: an element at either end of the row and one in the middle count."""
+    import torch
+    from ops_sparse_b200 import api
+    from ctypes import addressof, c_uint16, c_void_p
+    k = (1 << 30) + 1
+    X, Y = (make(1, k, dtype=torch.float16, device=device) for make in (torch.zeros, torch.ones))
+    X[0, 0], X[0, k // 2], X[0, k - 1] = 2, 3, 5
+    C = api.CsrMatrix(torch.tensor([0, 1], dtype=torch.int32, device=device), torch.zeros(1, dtype=torch.int32, device=device),
+                      torch.full((1,), 4.0, dtype=torch.float16, device=device), 1, 1)
+    dX, dY = api.DnMat.row_major(X), api.DnMat.row_major(Y)
+    alpha, beta = (c_uint16(int(np.float16(v).view(np.uint16))) for v in (1.0, 0.5))
+    buf = torch.empty(256, dtype=torch.uint8, device=device)
+    pkg.check(pkg.lib().aclsparseSDDMM(handle.raw, 0, pkg.ACL_SPARSE_OP_TRANSPOSE, c_void_p(addressof(alpha)), dX.raw, dY.raw,
+                                       c_void_p(addressof(beta)), C.raw, pkg.ACL_FLOAT16, 0, c_void_p(buf.data_ptr())),
+              "aclsparseSDDMM")
+    assert C.values.item() == 12.0
