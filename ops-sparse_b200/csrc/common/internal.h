@@ -105,6 +105,9 @@ struct aclsparseSpMatDescr {
     // Written by *Preprocess through a const descriptor, as in the reference
     // (spmm_host.cpp:341,360): the compute call compares its buffer argument against it.
     mutable b200sp::ActivePlan active;
+    // What aclsparseSpMMGetBufferSize last said for this matrix: room for a copy of B, and for how many columns.
+    mutable int64_t spmmSizedRepack = 0;
+    mutable int64_t spmmSizedN = -1;
 };
 
 struct aclsparseDnVecDescr {

@@ -133,7 +133,10 @@ aclsparseStatus_t aclsparseSpMMGetBufferSize(aclsparseHandle_t handle, aclsparse
     if (size == nullptr) return ACL_SPARSE_STATUS_INVALID_VALUE;
     const aclsparseStatus_t st = ValidateSpmm(opA, opB, matA, matB, matC, computeType, alg);
     if (st != ACL_SPARSE_STATUS_SUCCESS) return st;
-    *size = b200sp_spmm_plan_bytes(matA->rows, matA->nnz, matC->cols) + RepackBytes(matA, matB, matC, opB);
+    const size_t repack = RepackBytes(matA, matB, matC, opB);
+    *size = b200sp_spmm_plan_bytes(matA->rows, matA->nnz, matC->cols) + repack;
+    matA->spmmSizedRepack = (int64_t)repack;
+    matA->spmmSizedN = matC->cols;
     return ACL_SPARSE_STATUS_SUCCESS;
 }
 
@@ -173,7 +176,10 @@ aclsparseStatus_t aclsparseSpMMPreprocess(aclsparseHandle_t handle, aclsparseOpe
     p.longRows = found.longRows;
     p.colInd = matA->indices;
     p.valueType = (int32_t)matA->valueType;
-    p.repackBytes = (int64_t)RepackBytes(matA, matB, matC, opB);  // the buffer holds what GetBufferSize said for these operands
+    // Room for a copy of B is there if GetBufferSize, too, was asked for a B that wants one.  A caller who sized the buffer
+    // with B in another layout (the rest of the size does not depend on it) has none.
+    const int64_t repack = (int64_t)RepackBytes(matA, matB, matC, opB);
+    p.repackBytes = matA->spmmSizedN == matC->cols && matA->spmmSizedRepack >= repack ? repack : 0;
     p.generation = b200sp::BufferGeneration(buffer);
     matA->active = p;
     return ACL_SPARSE_STATUS_SUCCESS;
