@@ -1921,7 +1921,8 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
     // A product of one wave of short rows takes less time than the second launch.
     const bool small = sh->m * sh->n < 148ll * 2048 && segments + sh->mid_units == 0 && sh->nnz <= 16 * sh->m;
     const bool vectors = RowsContiguous(sh->op_b, sh->order_b) && sh->n % E == 0 && sh->ldb % E == 0 && Aligned16(B);
-    const bool copy = repack > 0 && sh->repack_bytes >= (int64_t)repack && WorthRepacking(sh, (int)sizeof(ValT)) && !small;
+    // The copy follows the plan (a multiple of 256 bytes) and is stored 16 bytes at a time; the plan itself may start on any word.
+    const bool copy = repack > 0 && sh->repack_bytes >= (int64_t)repack && WorthRepacking(sh, (int)sizeof(ValT)) && !small && Aligned16(plan);
     const bool words = !vectors && !copy && RowsOfWords(sh, (int)sizeof(ValT)) && reinterpret_cast<uintptr_t>(B) % 4 == 0;
     // Rows of four entries leave the generic kernel, with a thread per output, nothing to wait for one after the other
     // (695,764 of them, fp32, N = 11: 70 us; by words 79).

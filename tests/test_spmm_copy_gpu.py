@@ -57,3 +57,14 @@ def test_buffer_sized_for_another_layout(pkg, handle, device):
     api.spmm(handle, case.A, case.B[0], case.C[0], 1.0, 0.0, buffer=arena[:size])
     assert case.right(0)
     assert bool((arena[size:] == 0x5A).all())
+
+
+def test_buffer_on_any_word(pkg, handle, device):
+    """A buffer that does not start on a 16-byte boundary holds the plan, but no copy."""
+    from ops_sparse_b200 import api
+    case = Case(device)
+    size = api.spmm_buffer_size(handle, case.A, case.B[0], case.C[0])
+    buffer = torch.empty(size + 4, dtype=torch.uint8, device=device)[4:]
+    preprocess(pkg, handle, case, buffer)
+    api.spmm(handle, case.A, case.B[0], case.C[0], 1.0, 0.0, buffer=buffer)
+    assert case.right(0)
