@@ -195,6 +195,10 @@ size_t b200sp_spmm_plan_bytes(int64_t rows, int64_t nnz, int64_t n);
  * product runs a slower kernel that takes any layout.  Only the sizes and the layout of B are read. */
 size_t b200sp_spmm_repack_bytes(const b200spSpmmShape *shape, int val_type);
 
+/* 1 if b200sp_spmm_launch with this shape (room for a copy in shape.repack_bytes) and plan copies B behind the plan.  Two
+ * launches then belong together: products that share the plan must not overlap, nor be enqueued by two threads at once. */
+int b200sp_spmm_copies(const b200spSpmmShape *shape, int val_type, int32_t segments, const void *plan);
+
 /* Analysis pass: finds rows too long for one warp, cuts them into segments and writes
  * the segment table into `plan`, and lists the rows that are better summed apart from
  * their neighbours.  This call synchronises `stream` once to read back the two counts,

@@ -6,6 +6,7 @@
 // with the analysis-plan bookkeeping the B200 kernels need.
 #pragma once
 
+#include <mutex>
 #include <cstddef>
 #include <cstdint>
 #include <cstdio>
@@ -62,7 +63,9 @@ struct ActivePlan {
     int32_t longRows = 0;   // SpMM only: rows listed as long
     const void *colInd = nullptr;  // SpMM with column blocks: the cut table was made from these column indices
     int32_t valueType = -1;        // ... and for B rows of this element type
-    int64_t repackBytes = 0;       // SpMM only: bytes after the plan that a repacked B may use
+    int64_t repackBytes = 0;       // SpMM only: bytes after the plan that a repacked B may use ...
+    bool copyBound = false;        // ... by products on the stream of the first that did
+    unsigned long long copyStream = 0;
     int32_t spmvInfo[B200SP_SPMV_PLAN_INFO_INTS] = {};  // SpMV only: plan_info written by b200sp_spmv_analyze
     uint64_t generation = 0;  // BufferGeneration(buffer) when the analysis was written
 };
@@ -108,6 +111,7 @@ struct aclsparseSpMatDescr {
     // What aclsparseSpMMGetBufferSize last said for this matrix: room for a copy of B, and for how many columns.
     mutable int64_t spmmSizedRepack = 0;
     mutable int64_t spmmSizedN = -1;
+    mutable std::mutex copyMutex;  // held while a product that copies B into the analysed buffer is enqueued
 };
 
 struct aclsparseDnVecDescr {

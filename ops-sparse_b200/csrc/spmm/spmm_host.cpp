@@ -117,6 +117,27 @@ bool PlanMatches(const ActivePlan &p, const void *buffer, const aclsparseSpMatDe
            (p.blockUnits == 0 || (p.colInd == A->indices && p.valueType == (int32_t)A->valueType));
 }
 
+// Whether this product may copy B into the analysed buffer.  Products that share a buffer may otherwise overlap (as long
+// as no row exceeds 1024 entries they only read it), so the copies are kept in order: they are made on one stream,
+// that of the first product after the analysis, and not in a graph, which may be launched beside anything.  The other
+// products read B where it lies.
+bool MayCopy(ActivePlan &p, cudaStream_t stream)
+{
+    if (stream == cudaStreamPerThread) return false;  // as many streams as threads
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;  // never given to a second stream, as a handle may be
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
+        cudaStreamGetId(stream, &id) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    if (!p.copyBound) {
+        p.copyBound = true;
+        p.copyStream = id;
+    }
+    return p.copyStream == id;
+}
+
 }  // namespace
 
 extern "C" {
@@ -230,6 +251,12 @@ aclsparseStatus_t aclsparseSpMM(aclsparseHandle_t handle, aclsparseOperation_t o
     sh.long_rows = found.longRows;
     sh.kahan = (alg == ACL_SPARSE_SPMM_CSR_FP32_HIGH_PRECISION_ALG && matA->valueType == ACL_FLOAT) ? 1 : 0;
 
+    // The copy and the kernel that reads it are two launches: nothing of another thread may come between them.
+    std::unique_lock<std::mutex> copying(matA->copyMutex, std::defer_lock);
+    if (sh.repack_bytes > 0 && b200sp_spmm_copies(&sh, b200sp::KernelTypeOf(matA->valueType), found.segments, buffer) != 0) {
+        copying.lock();
+        if (!MayCopy(matA->active, handle->stream)) sh.repack_bytes = 0;
+    }
     const int rc = b200sp_spmm_launch(static_cast<const int32_t *>(matA->offsets),
                                       static_cast<const int32_t *>(matA->indices), matA->values, matB->values,
                                       matC->values, &sh, &sc, b200sp::KernelTypeOf(matA->valueType),

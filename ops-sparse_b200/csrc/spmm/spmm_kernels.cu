@@ -1888,6 +1888,16 @@ bool WorthRepacking(const b200spSpmmShape *sh, int valBytes)
     return 16 * sh->nnz >= sh->k * valBytes;
 }
 
+// Whether a product with this much room for a copy makes one.
+bool Copies(const b200spSpmmShape *sh, int valBytes, int32_t segments, const void *plan)
+{
+    const size_t repack = RepackBytes(sh, valBytes);
+    // A product of one wave of short rows takes less time than the second launch.
+    const bool small = sh->m * sh->n < 148ll * 2048 && segments + sh->mid_units == 0 && sh->nnz <= 16 * sh->m;
+    // The copy follows the plan (a multiple of 256 bytes) and is stored 16 bytes at a time; the plan itself may start on any word.
+    return repack > 0 && sh->repack_bytes >= (int64_t)repack && WorthRepacking(sh, valBytes) && !small && plan != nullptr && Aligned16(plan);
+}
+
 template <typename ValT, typename OutT>
 int LaunchGeneric(const int32_t *rowPtr, const int32_t *colInd, const void *val, const void *B, void *C,
                   const b200spSpmmShape *sh, const b200spScalars *s, cudaStream_t stream)
@@ -1917,12 +1927,8 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
 {
     constexpr bool kInt8 = std::is_same_v<ValT, int8_t>;
     constexpr int E = Pack<ValT>::kElems;
-    const size_t repack = RepackBytes(sh, (int)sizeof(ValT));
-    // A product of one wave of short rows takes less time than the second launch.
-    const bool small = sh->m * sh->n < 148ll * 2048 && segments + sh->mid_units == 0 && sh->nnz <= 16 * sh->m;
     const bool vectors = RowsContiguous(sh->op_b, sh->order_b) && sh->n % E == 0 && sh->ldb % E == 0 && Aligned16(B);
-    // The copy follows the plan (a multiple of 256 bytes) and is stored 16 bytes at a time; the plan itself may start on any word.
-    const bool copy = repack > 0 && sh->repack_bytes >= (int64_t)repack && WorthRepacking(sh, (int)sizeof(ValT)) && !small && Aligned16(plan);
+    const bool copy = Copies(sh, (int)sizeof(ValT), segments, plan);
     const bool words = !vectors && !copy && RowsOfWords(sh, (int)sizeof(ValT)) && reinterpret_cast<uintptr_t>(B) % 4 == 0;
     // Rows of four entries leave the generic kernel, with a thread per output, nothing to wait for one after the other
     // (695,764 of them, fp32, N = 11: 70 us; by words 79).
@@ -2143,6 +2149,11 @@ size_t b200sp_spmm_repack_bytes(const b200spSpmmShape *shape, int val_type)
 {
     const int bytes = val_type == B200SP_F32 ? 4 : val_type == B200SP_I8 ? 1 : 2;
     return WorthRepacking(shape, bytes) ? RepackBytes(shape, bytes) : 0;
+}
+
+int b200sp_spmm_copies(const b200spSpmmShape *shape, int val_type, int32_t segments, const void *plan)
+{
+    return Copies(shape, val_type == B200SP_F32 ? 4 : val_type == B200SP_I8 ? 1 : 2, segments, plan) ? 1 : 0;
 }
 
 int b200sp_spmm_analyze(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,

@@ -68,3 +68,80 @@ def test_buffer_on_any_word(pkg, handle, device):
     preprocess(pkg, handle, case, buffer)
     api.spmm(handle, case.A, case.B[0], case.C[0], 1.0, 0.0, buffer=buffer)
     assert case.right(0)
+
+
+@pytest.fixture()
+def shared(pkg, handle, device):
+    """A matrix analysed once, four B, and a graph of the product with the last of them."""
+    from ops_sparse_b200 import api
+    case = Case(device, seed=1, matrices=4)
+    buffer = torch.empty(api.spmm_buffer_size(handle, case.A, case.B[0], case.C[0]), dtype=torch.uint8, device=device)
+    preprocess(pkg, handle, case, buffer)
+    return case, buffer
+
+
+def test_products_on_two_streams(pkg, handle, device, shared):
+    """Products that share the buffer may overlap: each uses its own B."""
+    from ops_sparse_b200 import api
+    case, buffer = shared
+    handles = [api.Handle(torch.cuda.Stream()) for _ in range(3)]
+    for _ in range(20):
+        for c in case.C:
+            c.values.zero_()
+        torch.cuda.synchronize()
+        for i, h in enumerate(handles):
+            for _ in range(3):
+                api.spmm(h, case.A, case.B[i], case.C[i], 1.0, 0.0, buffer=buffer)
+        torch.cuda.synchronize()
+        assert all(case.right(i) for i in range(3))
+    for h in handles:
+        h.close()
+
+
+def test_products_of_two_threads(pkg, handle, device, shared):
+    """The copy and its product stay together when threads enqueue on one stream."""
+    from ops_sparse_b200 import api
+    case, buffer = shared
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(i):
+        h = api.Handle(stream)
+        with torch.cuda.stream(stream):
+            for _ in range(200):
+                api.spmm(h, case.A, case.B[i], case.C[i], 1.0, 0.0, buffer=buffer)
+                wrong.append(not case.right(i))
+        h.close()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(wrong) == 600 and not any(wrong)
+
+
+def test_graph_beside_a_product(pkg, handle, device, shared):
+    """A recorded product may be launched beside others that share the buffer."""
+    from ops_sparse_b200 import api
+    case, buffer = shared
+    record, beside = torch.cuda.Stream(), torch.cuda.Stream()
+    h = api.Handle(record)
+    api.spmm(h, case.A, case.B[3], case.C[3], 1.0, 0.0, buffer=buffer)  # what is created at first use must exist
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=record):
+        api.spmm(h, case.A, case.B[3], case.C[3], 1.0, 0.0, buffer=buffer)
+    for _ in range(20):
+        for c in case.C:
+            c.values.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(beside):
+            graph.replay()
+        for i in range(3):
+            api.spmm(h, case.A, case.B[i], case.C[i], 1.0, 0.0, buffer=buffer)
+        torch.cuda.synchronize()
+        assert all(case.right(i) for i in range(4))
+    del graph
+    h.close()
