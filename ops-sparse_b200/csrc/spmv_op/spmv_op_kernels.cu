@@ -112,23 +112,32 @@ __device__ __forceinline__ float Combine(const Triple &t, float alpha, float bet
 __device__ __forceinline__ Triple SumEntries(const OpArgs &a, long long first, long long e, int step)
 {
     Triple t{0.0f, 0.0f, 0.0f};
-    for (long long p = first; p < e; p += 4 * step) {
-        int c[4];
-        float v[4], xv[4];
+    long long p = first;
+    int c[4];
+    float v[4], xv[4];
+    for (; p + 3 * step < e; p += 4 * step) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
+            c[u] = __ldcs(a.colInd + p + u * step) - a.indexBase;
+            v[u] = __ldcs(a.val + p + u * step);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) xv[u] = __ldg(a.x + c[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) PriestStep(t, v[u], xv[u]);
+    }
+    if (p < e) {  // up to three more
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
             const bool in = p + u * step < e;
             c[u] = in ? __ldcs(a.colInd + p + u * step) - a.indexBase : 0;
             v[u] = in ? __ldcs(a.val + p + u * step) : 0.0f;
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) xv[u] = p + u * step < e ? __ldg(a.x + c[u]) : 0.0f;
-        // a step that no lane needs is branched over: rows are short, a step is some twenty instructions
+        for (int u = 0; u < 3; ++u) xv[u] = p + u * step < e ? __ldg(a.x + c[u]) : 0.0f;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            if (u > 0 && !__any_sync(__activemask(), p + u * step < e)) break;
+        for (int u = 0; u < 3; ++u)
             if (p + u * step < e) PriestStep(t, v[u], xv[u]);
-        }
     }
     return t;
 }
