@@ -17,12 +17,14 @@
 // need c bits; a histogram and a scatter, the counterpart of the reference's reorder / bin_edge tables,
 // spmv_op_kernel.cpp:425-540), and a class gets as many lanes per row as leave each of them four to eight entries; rows of
 // 512 entries and more get a CTA.  One grid, longest rows first.
+// SpmvOpLongRowsKernel (ALG2): rows that either grid would wait for, a wider CTA each, beside it on the side stream.
 #include <cstdint>
 
 #include <cuda_runtime.h>
 
 #include "b200sp_kernels.h"
 #include "../common/chained.cuh"
+#include "../common/side_stream.h"
 
 namespace {
 
@@ -108,39 +110,38 @@ __device__ __forceinline__ float Combine(const Triple &t, float alpha, float bet
     return __fmaf_rn(alpha, t.hi, __fmaf_rn(alpha, corr, betaY));
 }
 
-// Entries first, first + step, ... below e, in that order; four are requested before the first of them is used.
+// kCount entries p, p + step, ...: all of them requested before the first is used.  kWhole: none of them lies beyond e.
+template <int kCount, bool kWhole>
+__device__ __forceinline__ void SumSome(const OpArgs &a, Triple &t, long long p, long long e, int step)
+{
+    int c[kCount];
+    float v[kCount], xv[kCount];
+#pragma unroll
+    for (int u = 0; u < kCount; ++u) {
+        const bool in = kWhole || p + u * step < e;
+        c[u] = in ? __ldcs(a.colInd + p + u * step) - a.indexBase : 0;
+        v[u] = in ? __ldcs(a.val + p + u * step) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < kCount; ++u) xv[u] = kWhole || p + u * step < e ? __ldg(a.x + c[u]) : 0.0f;
+#pragma unroll
+    for (int u = 0; u < kCount; ++u)
+        if (kWhole || p + u * step < e) PriestStep(t, v[u], xv[u]);
+}
+
+// Entries first, first + step, ... below e, in that order, four in flight; kLong: eight as long as there are so many.
+template <bool kLong = false>
 __device__ __forceinline__ Triple SumEntries(const OpArgs &a, long long first, long long e, int step)
 {
     Triple t{0.0f, 0.0f, 0.0f};
     long long p = first;
-    int c[4];
-    float v[4], xv[4];
-    for (; p + 3 * step < e; p += 4 * step) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            c[u] = __ldcs(a.colInd + p + u * step) - a.indexBase;
-            v[u] = __ldcs(a.val + p + u * step);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) xv[u] = __ldg(a.x + c[u]);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) PriestStep(t, v[u], xv[u]);
-    }
-    if (p < e) {  // up to three more
-#pragma unroll
-        for (int u = 0; u < 3; ++u) {
-            const bool in = p + u * step < e;
-            c[u] = in ? __ldcs(a.colInd + p + u * step) - a.indexBase : 0;
-            v[u] = in ? __ldcs(a.val + p + u * step) : 0.0f;
-        }
-#pragma unroll
-        for (int u = 0; u < 3; ++u) xv[u] = p + u * step < e ? __ldg(a.x + c[u]) : 0.0f;
-#pragma unroll
-        for (int u = 0; u < 3; ++u)
-            if (p + u * step < e) PriestStep(t, v[u], xv[u]);
-    }
+    if constexpr (kLong)
+        for (; p + 7 * step < e; p += 8 * step) SumSome<8, true>(a, t, p, e, step);
+    for (; p + 3 * step < e; p += 4 * step) SumSome<4, true>(a, t, p, e, step);
+    if (p < e) SumSome<3, false>(a, t, p, e, step);
     return t;
 }
+
 template <int kLanes> __device__ __forceinline__ void JoinLanes(Triple &t)  // lane 0 of every group gets the sum
 {
 #pragma unroll
@@ -153,43 +154,57 @@ template <int kLanes> __device__ __forceinline__ void JoinLanes(Triple &t)  // l
     }
 }
 
-// A row per CTA: thread t runs the recurrence on entries t, t + kThreads, ...; the lanes of a warp are joined on the butterfly,
-// then warp 0 joins the warps' triples the same way: a fixed shape again.
-template <bool kIs64>
+// A row per CTA: thread t runs the recurrence on entries t, t + kRowThreads, ...; the lanes of a warp are joined on the
+// butterfly, then warp 0 joins the warps' triples the same way: a fixed shape again.
+template <bool kIs64, int kRowThreads>
 __device__ __forceinline__ void LongRow(const OpArgs &a, long long row, float alpha, float beta)
 {
-    __shared__ Triple sWarp[kThreads / 32];
+    __shared__ Triple sWarp[kRowThreads / 32];
     const int tid = threadIdx.x;
     const long long s = LoadOffset(a.rowOffsets, kIs64, row) - a.indexBase;
     const long long e = LoadOffset(a.rowOffsets, kIs64, row + 1) - a.indexBase;
     float yOld = 0.0f;
     if (tid == 0 && beta != 0.0f) yOld = a.y[row];
-    Triple t = SumEntries(a, s + tid, e, kThreads);
+    Triple t = SumEntries<true>(a, s + tid, e, kRowThreads);
     JoinLanes<32>(t);
     if ((tid & 31) == 0) sWarp[tid >> 5] = t;
     __syncthreads();
     if (tid < 32) {
-        Triple w = tid < kThreads / 32 ? sWarp[tid] : Triple{0.0f, 0.0f, 0.0f};
-        JoinLanes<kThreads / 32>(w);
+        Triple w = tid < kRowThreads / 32 ? sWarp[tid] : Triple{0.0f, 0.0f, 0.0f};
+        JoinLanes<kRowThreads / 32>(w);
         if (tid == 0) a.z[row] = Combine(w, alpha, __fmul_rn(beta, yOld));
     }
+}
+
+// Rows so long that a grid of lane groups or of CTAs of kThreads would wait for them: wider CTAs, on the side stream (see
+// OutlierBits).  The rows come from the front of the row order.
+template <bool kIs64, int kRowThreads>
+__global__ void __launch_bounds__(kRowThreads) SpmvOpLongRowsKernel(const OpArgs a, int first)
+{
+    const float alpha = a.alphaDev ? *a.alphaDev : a.alpha;
+    const float beta = a.betaDev ? *a.betaDev : a.beta;
+    LongRow<kIs64, kRowThreads>(a, a.reorder[first + blockIdx.x], alpha, beta);
 }
 
 // Light on registers and without barriers: it lives on warps in flight (the gathers of x go to L2, one sector per clock and
 // SM).  CTAs of 128 threads: 466,673 rows of 51 entries 69 us, with 256 threads 78.
 template <int G, bool kIs64>
-__global__ void __launch_bounds__(kThreads, 12) SpmvOpRowsKernel(const OpArgs a)
+__global__ void __launch_bounds__(kThreads, 12) SpmvOpRowsKernel(const OpArgs a, long long outlier)  // rows from there on are others' work
 {
     b200sp::WaitForPrevious();
     const float alpha = a.alphaDev ? *a.alphaDev : a.alpha;
     const float beta = a.betaDev ? *a.betaDev : a.beta;
     const int lane = threadIdx.x & 31, li = lane & (G - 1);
     const long long row = ((long long)blockIdx.x * kThreads + threadIdx.x) / G;
-    const bool mine = row < a.rows;
+    bool mine = row < a.rows;
     long long s = 0, e = 0;
     if (mine) {
         s = LoadOffset(a.rowOffsets, kIs64, row) - a.indexBase;
         e = LoadOffset(a.rowOffsets, kIs64, row + 1) - a.indexBase;
+        if (e - s >= outlier) {
+            mine = false;
+            e = s;
+        }
     }
     const bool wide = e - s > 16 * G;
     float yOld = 0.0f;
@@ -202,7 +217,7 @@ __global__ void __launch_bounds__(kThreads, 12) SpmvOpRowsKernel(const OpArgs a)
         const int owner = __ffs(todo) - 1;
         todo &= todo - 1;
         const long long ws = __shfl_sync(0xffffffffu, s, owner), we = __shfl_sync(0xffffffffu, e, owner);
-        Triple w = SumEntries(a, ws + lane, we, 32);
+        Triple w = SumEntries<true>(a, ws + lane, we, 32);
         JoinLanes<32>(w);
         w.hi = __shfl_sync(0xffffffffu, w.hi, 0);
         w.md = __shfl_sync(0xffffffffu, w.md, 0);
@@ -253,7 +268,7 @@ __global__ void __launch_bounds__(kThreads, 12) SpmvOpClassesKernel(const OpArgs
     const float alpha = a.alphaDev ? *a.alphaDev : a.alpha;
     const float beta = a.betaDev ? *a.betaDev : a.beta;
     const int b = blockIdx.x;
-    if (b < ranges.r[1].firstBlock) LongRow<kIs64>(a, a.reorder[b], alpha, beta);
+    if (b < ranges.r[1].firstBlock) LongRow<kIs64, kThreads>(a, a.reorder[ranges.r[0].first + b], alpha, beta);
     else if (b < ranges.r[2].firstBlock) ClassRow<32, kIs64>(a, ranges.r[1], alpha, beta);
     else if (b < ranges.r[3].firstBlock) ClassRow<16, kIs64>(a, ranges.r[2], alpha, beta);
     else if (b < ranges.r[4].firstBlock) ClassRow<8, kIs64>(a, ranges.r[3], alpha, beta);
@@ -327,13 +342,15 @@ __global__ void SpmvOpScatterKernel(const void *rowOffsets, long long rows, int3
 }
 
 template <bool kIs64>
-cudaError_t LaunchRows(const OpArgs &a, double mean, cudaStream_t st)
+cudaError_t LaunchRows(const OpArgs &a, double mean, long long outlier, cudaStream_t st)
 {
     auto launch = [&]<int G>() {
         b200sp_note_launches(1);
-        return b200sp::LaunchChained(SpmvOpRowsKernel<G, kIs64>, (unsigned)((a.rows * G + kThreads - 1) / kThreads), kThreads, 0, st, a);
+        return b200sp::LaunchChained(SpmvOpRowsKernel<G, kIs64>, (unsigned)((a.rows * G + kThreads - 1) / kThreads), kThreads, 0, st, a,
+                                     outlier);
     };
     // lanes for which rows of the mean length give each of them four to eight entries: fewer idle the memory, more the lanes
+    if (mean <= 1) return launch.template operator()<1>();  // mostly empty rows: 2 M of them, 20,000 entries: 18.9 us with two lanes
     if (mean <= 6) return launch.template operator()<2>();
     if (mean <= 28) return launch.template operator()<4>();
     if (mean <= 64) return launch.template operator()<8>();
@@ -355,6 +372,78 @@ bool Skewed(const int32_t *class_start, double mean)
         if ((double)(1ll << (c - 1)) >= 4 * mean) heavy += entries;
     }
     return heavy > 0.15 * all;
+}
+
+// Bits of a length from which a row gets a CTA of SpmvOpLongRowsKernel.  A warp takes 128 entries of a row per round trip to
+// memory (0.9 us), a CTA of kThreads 512, while a grid that is full takes some 220 entries per ns.  So a row of nnz / 8192
+// entries costs a warp, which may come to it late, a quarter of what the whole grid takes (half is fair for rows below twice
+// the mean), and one of nnz / 512 entries a CTA, which comes to it first, as long as the grid takes; the rows beyond are
+// few, by their number.  With a warp each, and so: 300,000 rows of 20 and 40 of 16,000: 136 and 31 us; 1 M rows of 30 and
+// one of a million: 10.5 and 0.35 ms; 2000 rows of up to 8000: 71 and 37 us; 5000 rows of 1100: 23 and 27, left to warps.
+int OutlierBits(int64_t nnz, double mean, bool skewed)
+{
+    double least = skewed ? 4096 : 1024, share = (double)nnz / (skewed ? 512 : 8192);
+    if (!skewed && least < 2 * mean) least = 2 * mean < 2 * share ? 2 * mean : 2 * share > least ? 2 * share : least;
+    int bits = 1;
+    while (bits < 62 && (double)(1ll << (bits - 1)) < (share > least ? share : least)) ++bits;
+    return bits;  // the shortest length of that many bits is 2^(bits - 1)
+}
+constexpr int kHugeBits = 15;  // rows of 16384 entries and more: CTAs of 1024 threads, the others of 256
+
+// The rows of `bits` bits and more, count of them at the front of the row order; long ones first.
+template <bool kIs64>
+cudaError_t LaunchOutliers(const OpArgs &a, const int32_t *class_start, int count, cudaStream_t st)
+{
+    const int huge = class_start[kClasses - kHugeBits] < count ? class_start[kClasses - kHugeBits] : count;
+    if (huge > 0) SpmvOpLongRowsKernel<kIs64, 1024><<<(unsigned)huge, 1024, 0, st>>>(a, 0);
+    if (count > huge) SpmvOpLongRowsKernel<kIs64, 256><<<(unsigned)(count - huge), 256, 0, st>>>(a, huge);
+    b200sp_note_launches((huge > 0) + (count > huge));
+    return cudaGetLastError();
+}
+
+template <bool kIs64>
+cudaError_t LaunchAll(const OpArgs &a, int64_t nnz, const int32_t *class_start, cudaStream_t st)
+{
+    const double mean = (double)nnz / (double)a.rows;
+    if (class_start == nullptr) return LaunchRows<kIs64>(a, mean, INT64_MAX, st);
+    const bool skewed = Skewed(class_start, mean);
+    const int bits = OutlierBits(nnz, mean, skewed);
+    const int outliers = bits < kClasses ? class_start[kClasses - bits] : 0;
+    if (outliers == a.rows) return LaunchOutliers<kIs64>(a, class_start, outliers, st);
+    // They write rows of z of their own: forked onto the side stream, ahead of the grid for the others.
+    b200sp::SideLanes *lanes = outliers > 0 ? b200sp::GetSideLanes() : nullptr;
+    cudaError_t e = cudaSuccess;
+    if (outliers > 0) {
+        if (lanes != nullptr) e = cudaEventRecord(lanes->fork, st);
+        if (lanes != nullptr && e == cudaSuccess) e = cudaStreamWaitEvent(lanes->stream[0], lanes->fork, 0);
+        if (e == cudaSuccess) e = LaunchOutliers<kIs64>(a, class_start, outliers, lanes != nullptr ? lanes->stream[0] : st);
+        if (lanes != nullptr && e == cudaSuccess) e = cudaEventRecord(lanes->join[0], lanes->stream[0]);
+        if (e != cudaSuccess) return e;
+    }
+    if (!skewed) {
+        e = LaunchRows<kIs64>(a, mean, outliers > 0 ? 1ll << (bits - 1) : INT64_MAX, st);
+    } else {
+        Ranges ranges;
+        long long blocks = 0;
+        for (int i = 0; i < kRanges; ++i) {
+            Range &r = ranges.r[i];
+            r.firstBlock = (int)blocks;
+            r.first = i == 0 ? outliers : ranges.r[i - 1].first + ranges.r[i - 1].count;
+            const int end = class_start[kClasses - kRangeBits[i]];
+            r.count = end > r.first ? end - r.first : 0;
+            const int perBlock = kRangeLanes[i] == 0 ? 1 : kThreads / kRangeLanes[i];
+            blocks += (r.count + perBlock - 1) / perBlock;
+        }
+        if (blocks > 0) {
+            b200sp_note_launches(1);
+            e = b200sp::LaunchChained(SpmvOpClassesKernel<kIs64>, (unsigned)blocks, kThreads, 0, st, a, ranges);
+        }
+    }
+    if (lanes != nullptr) {
+        const cudaError_t joined = cudaStreamWaitEvent(st, lanes->join[0], 0);
+        if (e == cudaSuccess) e = joined;
+    }
+    return e;
 }
 
 }  // namespace
@@ -429,22 +518,8 @@ int b200sp_spmvop_launch(const void *row_offsets, int offsets_are_64, const int3
     a.betaDev = beta_dev;
     a.reorder = static_cast<const int32_t *>(plan);
     a.rows = rows;
-    const double mean = (double)nnz / (double)rows;
-    if (plan == nullptr || class_start == nullptr || !Skewed(class_start, mean))
-        return (int)(offsets_are_64 ? LaunchRows<true>(a, mean, st) : LaunchRows<false>(a, mean, st));
-    Ranges ranges;
-    long long blocks = 0;
-    for (int i = 0; i < kRanges; ++i) {
-        Range &r = ranges.r[i];
-        r.firstBlock = (int)blocks;
-        r.first = i == 0 ? 0 : ranges.r[i - 1].first + ranges.r[i - 1].count;
-        r.count = class_start[kClasses - kRangeBits[i]] - r.first;
-        const int perBlock = kRangeLanes[i] == 0 ? 1 : kThreads / kRangeLanes[i];
-        blocks += (r.count + perBlock - 1) / perBlock;
-    }
-    b200sp_note_launches(1);
-    return (int)(offsets_are_64 ? b200sp::LaunchChained(SpmvOpClassesKernel<true>, (unsigned)blocks, kThreads, 0, st, a, ranges)
-                                : b200sp::LaunchChained(SpmvOpClassesKernel<false>, (unsigned)blocks, kThreads, 0, st, a, ranges));
+    const int32_t *classes = plan != nullptr ? class_start : nullptr;
+    return (int)(offsets_are_64 ? LaunchAll<true>(a, nnz, classes, st) : LaunchAll<false>(a, nnz, classes, st));
 }
 
 int b200sp_spmvop_scale(const float *y, float *z, int64_t rows, float beta, const float *beta_dev, void *stream)
