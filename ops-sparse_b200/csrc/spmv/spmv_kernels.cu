@@ -1373,26 +1373,36 @@ __global__ void SpmvMaxRowLengthKernel(const int32_t *__restrict__ rowPtr, int r
 
 // acc[col] += (alpha * x[row]) * a_ij, cut by non-zeros: a warp takes chunks of kTransChunk consecutive entries, whatever
 // rows they belong to (a scatter needs no per-row reduction, so a row of 16384 entries is simply spread over 64 warps).  All
-// columns and values of a chunk are requested at once; the rows it touches lie one per lane with their alpha * x, and an
-// entry finds its row among them by five shuffles.  Bound by the additions: one request per entry on the path from the
-// SM to L2 and one operation there.
-// Measured, fp32, 11.5 M entries in 500,009 power-law rows: 72 us with a search of the row offsets per entry,
-// 66 us so (0.65 of them per clock and SM); rows of like length gain more
-// (a 67^3 stencil in bf16: 56 -> 34 us with both passes over y).
+// columns and values of a chunk are requested at once.  The rows it touches are read side by side, a lane each: every
+// non-empty one marks its first entry in a bitmap in shared memory and leaves alpha * x there, and an entry finds its row
+// at the last mark at or before it.  A chunk that spans more than kTransSpan rows (stretches of empty ones) searches the
+// offsets for its entries instead, eight of a lane at a time.  Bound by the additions: one request per entry on the
+// path from the SM to L2 and one operation there.
+// Measured, fp32: 11.5 M entries in 500,009 power-law rows: 72 us with a search of the row offsets per entry, 67 with the rows
+// held by the lanes and found by shuffles, 65 so (0.68 of them per clock and SM); 4 M entries in 100,000 rows after 400,000
+// rows of one entry: 37 with a lane group per row, 49 held by the lanes, 31 so; a million empty rows inside a chunk: 12 us
+// with a search per entry, 8.1 ms when the lanes walked through them, 15 so.
 constexpr int kTransChunk = 256;
+constexpr int kTransSpan = 1024;
+constexpr int kTransWarps = 8;
 template <typename CompT, typename ValT, typename AccT>
-__global__ void __launch_bounds__(256) SpmvTransScatterKernel(const int32_t *__restrict__ rowPtr, const int32_t *__restrict__ colInd,
-                                                              const ValT *__restrict__ val, const ValT *__restrict__ x,
-                                                              AccT *__restrict__ acc, int rows, int nnz, int chunksPerWarp,
-                                                              Scalars<CompT> sc)
+__global__ void __launch_bounds__(32 * kTransWarps, 5) SpmvTransScatterKernel(const int32_t *__restrict__ rowPtr,
+                                                                           const int32_t *__restrict__ colInd,
+                                                                           const ValT *__restrict__ val, const ValT *__restrict__ x,
+                                                                           AccT *__restrict__ acc, int rows, int nnz, int chunksPerWarp,
+                                                                           Scalars<CompT> sc)
 {
     constexpr int kSteps = kTransChunk / 32;
+    __shared__ uint32_t sBits[kTransWarps][kSteps];
+    __shared__ CompT sFactor[kTransWarps][kTransChunk];
     b200sp::WaitForPrevious();
     const CompT alpha = sc.Alpha();
-    const int lane = threadIdx.x & 31;
-    long long c0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * chunksPerWarp * kTransChunk;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t *bits = sBits[warp];
+    CompT *factor = sFactor[warp];
+    long long c0 = ((long long)blockIdx.x * kTransWarps + warp) * chunksPerWarp * kTransChunk;
     if (c0 >= nnz) return;
-    int r0 = b200sp::WarpRowOf(rowPtr, rows, c0, lane);
+    int r0 = b200sp::WarpRowOf(rowPtr, rows, c0, lane);  // a row that starts at or before the chunk's first entry
     for (int chunk = 0; chunk < chunksPerWarp && c0 < nnz; ++chunk, c0 += kTransChunk) {
         int c[kSteps];
         ValT v[kSteps];
@@ -1402,48 +1412,72 @@ __global__ void __launch_bounds__(256) SpmvTransScatterKernel(const int32_t *__r
             c[u] = p < nnz ? __ldcs(colInd + p) : -1;
             v[u] = p < nnz ? __ldcs(val + p) : ValT(0);
         }
-        // Starts of the rows r0 + lane, and their factors; `held` of them in order, from the row of the chunk's first entry on.
-        int start = r0 + lane < rows ? __ldg(rowPtr + r0 + lane) : nnz;
-        CompT f = r0 + lane < rows ? alpha * Widen<CompT>(__ldg(x + r0 + lane)) : CompT(0);
-        int at = 0;
+        const int first = (int)c0, last = (int)(c0 + kTransChunk < nnz ? c0 + kTransChunk - 1 : nnz - 1);
+        auto add = [&](int u, CompT f) {
+            if (c[u] >= 0 && f != CompT(0)) atomicAdd(acc + c[u], static_cast<AccT>(f * Widen<CompT>(v[u])));
+        };
+        // Bounds of the rows r0 + 32 k + lane; beyond the last row both lie behind every entry.
+        int s[4], e[4];
+        auto load = [&](int k) {
+            const unsigned r = (unsigned)r0 + 32 * k + lane;
+            s[k] = r < (unsigned)rows ? __ldg(rowPtr + r) : 0x7fffffff;
+            e[k] = r < (unsigned)rows ? __ldg(rowPtr + r + 1) : 0x7fffffff;
+        };
+        load(0);
+        if (r0 < rows - kTransSpan && __ldg(rowPtr + r0 + kTransSpan) <= last) {  // the same in every lane
+            const int rEnd = r0 + b200sp::WarpRowOf(rowPtr + r0, rows - r0, last, lane);
+            int at[kSteps];  // each entry's row lies in [at, at + left]
+#pragma unroll
+            for (int u = 0; u < kSteps; ++u) at[u] = r0;
+            for (int left = rEnd - r0; left > 0;) {
+                const int step = (left + 3) / 4;  // three probes at once: half as many round trips as with one
+#pragma unroll
+                for (int u = 0; u < kSteps; ++u) {
+                    const int entry = u * 32 + lane < last - first ? first + u * 32 + lane : last;
+                    int below = 0;
+#pragma unroll
+                    for (int k = 1; k <= 3; ++k) below += k * step <= rEnd - at[u] && __ldg(rowPtr + at[u] + k * step) <= entry;
+                    at[u] += below * step;
+                }
+                left = step - 1 > left - 3 * step ? step - 1 : left - 3 * step;
+            }
+#pragma unroll
+            for (int u = 0; u < kSteps; ++u) add(u, alpha * Widen<CompT>(__ldg(x + at[u])));
+            r0 = rEnd;
+            continue;
+        }
+        if (lane < kSteps) bits[lane] = 0;
+        __syncwarp();
+        // Returns how many of the 32 rows start at or before the chunk's last entry: a prefix, as starts ascend.
+        auto mark = [&](int k) {
+            const int from = s[k] > first ? s[k] : first;
+            if (s[k] <= last && e[k] > from) {  // holds entries of the chunk
+                factor[from - first] = alpha * Widen<CompT>(__ldg(x + r0 + 32 * k + lane));
+                atomicOr(bits + ((from - first) >> 5), 1u << ((from - first) & 31));
+            }
+            return __popc(__ballot_sync(0xffffffffu, s[k] <= last));
+        };
+        int n = mark(0);
+        int end = __shfl_sync(0xffffffffu, e[0], 31);
+        for (int rowsRead = 32; end <= last; rowsRead = 128) {  // more rows: four times 32 at a time
+            r0 += rowsRead;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) load(k);
+            n = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) n += mark(k);
+            end = __shfl_sync(0xffffffffu, e[3], 31);
+        }
+        r0 += n - 1;  // the last row that starts within the chunk, or before it
+        __syncwarp();
+        int before = 0;  // the last mark in the words before
 #pragma unroll
         for (int u = 0; u < kSteps; ++u) {
-            const int p = (int)(c0 + u * 32 < nnz ? c0 + u * 32 : nnz - 1);          // first entry of the step ...
-            const int q = (int)(c0 + u * 32 + 31 < nnz ? c0 + u * 32 + 31 : nnz - 1);  // ... and its last
-            // Does the row after the 32 held begin within the step?  Then hold the rows from the step's first entry on.
-            while (__shfl_sync(0xffffffffu, start, 31) <= q) {
-                const int n = __popc(__ballot_sync(0xffffffffu, start <= p));  // starts ascend: the first n begin at or before p
-                r0 += n - 1;
-                start = r0 + lane < rows ? __ldg(rowPtr + r0 + lane) : nnz;
-                f = r0 + lane < rows ? alpha * Widen<CompT>(__ldg(x + r0 + lane)) : CompT(0);
-                if (n == 1) break;  // more rows in one step than lanes: searched below
-                if (n < 32) break;
-            }
-            const int e = lane <= q - p ? p + lane : q;
-            at = 0;
-#pragma unroll
-            for (int step = 16; step > 0; step >>= 1) {
-                const int s = __shfl_sync(0xffffffffu, start, at + step);
-                if (s <= e) at += step;
-            }
-            CompT mine = __shfl_sync(0xffffffffu, f, at);
-            const int lastStart = __shfl_sync(0xffffffffu, start, 31);
-            if (lastStart <= e && r0 + 32 < rows) {  // perhaps in a row beyond the 32 held (a stretch of empty rows)
-                int lo = r0 + 31, hi = rows - 1;
-                while (lo < hi) {
-                    const int mid = lo + ((hi - lo + 1) >> 1);
-                    if (__ldg(rowPtr + mid) <= e) lo = mid;
-                    else hi = mid - 1;
-                }
-                mine = alpha * Widen<CompT>(__ldg(x + lo));
-            }
-            if (c[u] >= 0 && mine != CompT(0)) atomicAdd(acc + c[u], static_cast<AccT>(mine * Widen<CompT>(v[u])));
+            const uint32_t word = bits[u], upTo = word & (0xffffffffu >> (31 - lane));
+            add(u, factor[upTo != 0 ? u * 32 + 31 - __clz(upTo) : before]);
+            if (word != 0) before = u * 32 + 31 - __clz(word);
         }
-        const int q = (int)(c0 + kTransChunk < nnz ? c0 + kTransChunk : nnz - 1);  // the next chunk's first entry
-        if (chunk + 1 < chunksPerWarp && c0 + kTransChunk < nnz) {
-            if (__shfl_sync(0xffffffffu, start, 31) <= q) r0 = b200sp::WarpRowOf(rowPtr, rows, q, lane);
-            else r0 += __popc(__ballot_sync(0xffffffffu, start <= q)) - 1;
-        }
+        __syncwarp();  // bits and factors may be written again
     }
 }
 
@@ -1764,7 +1798,7 @@ int LaunchTransTyped(const int32_t *rowPtr, const int32_t *colInd, const void *v
     // Consecutive chunks share a warp (and its first search), as long as every SM gets its 64 warps twice.
     const int64_t chunks = (nnz + kTransChunk - 1) / kTransChunk;
     const int perWarp = chunks >= 4 * 128ll * sms ? 4 : chunks >= 2 * 128ll * sms ? 2 : 1;
-    const unsigned blocks = (unsigned)((chunks + 8 * perWarp - 1) / (8 * perWarp));
+    const unsigned blocks = (unsigned)((chunks + kTransWarps * perWarp - 1) / (kTransWarps * perWarp));
     const auto *v = static_cast<const ValT *>(val), *xv = static_cast<const ValT *>(x);
     // A 16-bit y accumulates in scratch and is rounded once.
     constexpr bool kNarrowOut = sizeof(OutT) == 2;
@@ -1777,7 +1811,7 @@ int LaunchTransTyped(const int32_t *rowPtr, const int32_t *colInd, const void *v
                                           (int)cols, sc);
     if (e == cudaSuccess && rows > 0 && nnz > 0) {
         b200sp_note_launches(1);
-        e = b200sp::LaunchChained(SpmvTransScatterKernel<CompT, ValT, AccT>, blocks, 256, 0, stream, rowPtr, colInd, v, xv, acc,
+        e = b200sp::LaunchChained(SpmvTransScatterKernel<CompT, ValT, AccT>, blocks, 32 * kTransWarps, 0, stream, rowPtr, colInd, v, xv, acc,
                                   (int)rows, (int)nnz, perWarp, sc);
     }
     if constexpr (kNarrowOut) {

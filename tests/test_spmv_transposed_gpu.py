@@ -15,6 +15,10 @@ PATTERNS = {
     "33 rows a step": lambda rng: np.tile([1] * 31 + [0, 0, 2], 40),
     "long and short": lambda rng: np.concatenate([[5000], rng.integers(0, 3, 500), [256, 255, 257, 1]]),
     "a single row": lambda rng: np.array([777]),
+    # the offsets are searched where a chunk of 256 entries spans more than 1024 rows
+    "a long stretch inside a chunk": lambda rng: np.concatenate([[5] * 30, np.zeros(300_000, np.int64), [7] * 40]),
+    "around the limit": lambda rng: np.concatenate([[100, *[0] * k, 200] for k in range(1019, 1028)]),
+    "one row in a hundred": lambda rng: (rng.random(300_000) < 0.01).astype(np.int64),
 }
 
 
