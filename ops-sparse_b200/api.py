@@ -55,8 +55,8 @@ class _PackedCalls(dict):
         if len(self) >= self.MOST:
             self.clear()
         struct = _PackedCall(**fields)
-        self[key] = struct, addressof(struct)
-        return self[key]
+        call = self[key] = struct, addressof(struct)
+        return call  # not looked up again: another thread may have emptied the table
 
 
 class Handle:

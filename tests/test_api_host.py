@@ -5,7 +5,7 @@ from __future__ import annotations
 
 import re
 import subprocess
-from ctypes import byref, c_int, c_int64, c_size_t, c_void_p
+from ctypes import addressof, byref, c_int, c_int64, c_size_t, c_void_p
 from pathlib import Path
 
 import pytest
@@ -332,3 +332,17 @@ def test_sddmm_argument_checks_without_device(pkg):
         assert L.aclsparseDestroyDnMat(d) == 0
     for d in (C, C64, C1):
         assert L.aclsparseDestroySpMat(d) == 0
+
+
+def test_packed_call_outlives_the_table(pkg):
+    """A product packs its arguments while another thread, whose product found the table full, empties it."""
+    from ops_sparse_b200 import api
+
+    class Emptied(api._PackedCalls):
+        def __setitem__(self, key, value):
+            super().__setitem__(key, value)
+            self.clear()
+
+    struct, address = Emptied().pack((1, 2), handle=0x10, a=0x20, opB=1)
+    assert (struct.handle, struct.a, struct.x, struct.opB) == (0x10, 0x20, None, 1)
+    assert address == addressof(struct)
