@@ -286,9 +286,9 @@ def config_list(args, world: int) -> list[str]:
 # the kernels of one product), with the summary under profiles/ they were read from.  A figure is attached to a
 # line only when the kernels that ran are the ones the capture covers.
 NCU_TRAFFIC = {
-    "c2": {"bytes": 280_800_000, "kernels": "SpmvLongBlockKernel + SpmvMediumShortKernel",
-           "source": "profiles/spmv_binned_c2_powerlaw_f32.md"},
-    "c4": {"bytes": 635_600_000, "kernels": "SpmmFastKernel", "source": "profiles/spmm_fast_c4_f32_n64.md"},
+    "c2": {"bytes": 282_700_000, "kernels": "SpmvLongBlockKernel + SpmvMediumShortKernel",
+           "source": "profiles/kernels_of_the_cases.md"},
+    "c4": {"bytes": 606_900_000, "kernels": "SpmmFastKernel", "source": "profiles/kernels_of_the_cases.md"},
     "c5": {"bytes": 13_460_000_000, "kernels": "SpmmRowStreamKernel + SpmmLongBlockKernel",
            "source": "profiles/spmm_rowstream_c5_bf16_n256.md"},
 }

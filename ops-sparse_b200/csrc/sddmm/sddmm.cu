@@ -86,8 +86,8 @@ __global__ void __launch_bounds__(256) SddmmKernel(const int32_t *__restrict__ r
 //     carries costs as many shuffles as values are left (6 instead of 20 for four sums over 32 lanes).
 // fp16 rows that start on odd 2-byte addresses (kBytes = 2) are copied as the 4-byte words that cover them and
 // realigned when they are read from shared memory.
-// Measured (1 M nodes, 16.0 M entries, fp16, k = 256): 2091 us with the rows in registers, four entries in flight and a full butterfly per
-// entry; 1384 us here, 8.2 GB of Y rows at 5.9 TB/s.
+// Measured (1 M nodes, 16.0 M entries, fp16, k = 256, inputs that alternate): 2103 us with the rows in registers, four entries in flight
+// and a full butterfly per entry; 1477 us here.  The kernel alone moves 7.6 GB of Y rows in 1261 us, 6.1 TB/s.
 template <int kBytes> struct Words { using Type = uint32_t; };  // 4, and the words of kBytes = 2
 template <> struct Words<16> { using Type = uint4; };
 template <> struct Words<8> { using Type = uint2; };
@@ -130,7 +130,7 @@ template <int kSize> __device__ __forceinline__ void CopyAsync(void *dst, const 
 __device__ __forceinline__ void CopyCommit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int kPending> __device__ __forceinline__ void CopyWait() { asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory"); }
 
-// 1384 us with 4 warps and tiles of 128, 1286 with 2 and 64 on the same GPU; one warp or longer tiles gain nothing more.
+// The same inputs again and again: 1384 us with 4 warps and tiles of 128, 1286 with 2 and 64 on the same GPU; one warp or longer tiles gain nothing more.
 constexpr int kSddmmWarps = 2;
 constexpr int kSddmmTile = 64;  // entries a warp owns at most
 template <int kBytes, int kLanes, int kSlabs> struct SddmmShape {

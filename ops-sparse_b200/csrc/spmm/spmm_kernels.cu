@@ -1933,7 +1933,7 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
     // Rows of four entries leave the generic kernel, with a thread per output, nothing to wait for one after the other
     // (695,764 of them, fp32, N = 11: 70 us; by words 79).
     // So do int8 rows of up to 32 entries whose B rows are eight bytes at most: eight lanes of 16 columns join more sums
-    // than they save loads (275,178 rows of 26, N = 8: 53 us; by lane groups 63).
+    // than they save loads (275,178 rows of 26, N = 8: 51 to 53 us; by lane groups 63).
     const bool alike = segments + sh->mid_units == 0;
     const bool few = kInt8 ? sh->n <= 8 && sh->nnz <= 32 * sh->m && alike && RowsContiguous(sh->op_b, sh->order_b)
                            : words && sh->n <= 16 && sh->nnz <= 4 * sh->m && alike;

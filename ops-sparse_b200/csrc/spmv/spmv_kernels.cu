@@ -5,7 +5,7 @@
 // walks them one at a time.  Two designs replace it here, chosen by what the caller set up.
 //
 // Binned path (a buffer analysed once by aclsparseSpMVPreprocess / b200sp_spmv_analyze with
-// plan_info).  The analysis lists the rows of 33..1023 entries ("medium") and of >= 1024
+// plan_info).  The analysis lists the rows of 33..511 entries ("medium") and of >= 512
 // entries ("long", ordered by descending length) as {row, start, end}; a product is then two
 // launches over disjoint rows of y, the first forked onto a side stream so that they share
 // the SMs:
@@ -19,7 +19,8 @@
 //                           loads first, then the medium and short rows as below; no side stream.
 //   SpmvMediumShortKernel   one grid: first a warp per listed medium row, then every row gets
 //                           a group of G = 2 or 4 lanes (rows longer than 32 entries are
-//                           skipped).  SpmvShortRowsKernel alone when no row is medium.
+//                           skipped).  SpmvShortRowsKernel, or SpmvStagedRowsKernel for
+//                           banded matrices, alone when no row is medium.
 // Gathers of x from scattered columns cost one L2 sector request each, and an SM issues one
 // request per clock: many light warps, each with a few independent gathers in flight, keep
 // that port busy for the medium and short rows, and the long rows stay off it altogether.
@@ -1379,7 +1380,7 @@ __global__ void SpmvMaxRowLengthKernel(const int32_t *__restrict__ rowPtr, int r
 // offsets for its entries instead, eight of a lane at a time.  Bound by the additions: one request per entry on the
 // path from the SM to L2 and one operation there.
 // Measured, fp32: 11.5 M entries in 500,009 power-law rows: 72 us with a search of the row offsets per entry, 67 with the rows
-// held by the lanes and found by shuffles, 65 so (0.68 of them per clock and SM); 4 M entries in 100,000 rows after 400,000
+// held by the lanes and found by shuffles, 65 so (0.65 of them per clock and SM); 4 M entries in 100,000 rows after 400,000
 // rows of one entry: 37 with a lane group per row, 49 held by the lanes, 31 so; a million empty rows inside a chunk: 12 us
 // with a search per entry, 8.1 ms when the lanes walked through them, 15 so.
 constexpr int kTransChunk = 256;

@@ -259,7 +259,7 @@ __device__ __forceinline__ void ClassRow(const OpArgs &a, const Range &range, fl
 }
 
 // 31.2 M entries in 1 M power-law rows: a warp per row from 64 entries and four lanes below, long rows on a side stream:
-// 165 us; 133 us so.  The long rows wait for their gathers (L2 delivers one sector per clock and SM), the others
+// 165 us; 138 to 141 us so.  The long rows wait for their gathers (L2 delivers one sector per clock and SM), the others
 // for issue slots: an entry is some twenty instructions and a join of two lanes' sums as many, so lanes must not idle.
 template <bool kIs64>
 __global__ void __launch_bounds__(kThreads, 12) SpmvOpClassesKernel(const OpArgs a, const Ranges ranges)
