@@ -1386,25 +1386,25 @@ __global__ void SpmvMaxRowLengthKernel(const int32_t *__restrict__ rowPtr, int r
 constexpr int kTransChunk = 256;
 constexpr int kTransSpan = 1024;
 constexpr int kTransWarps = 8;
-template <typename CompT, typename ValT, typename AccT>
+template <typename CompT, typename ValT, typename AccT, int kChunk>
 __global__ void __launch_bounds__(32 * kTransWarps, 5) SpmvTransScatterKernel(const int32_t *__restrict__ rowPtr,
                                                                            const int32_t *__restrict__ colInd,
                                                                            const ValT *__restrict__ val, const ValT *__restrict__ x,
                                                                            AccT *__restrict__ acc, int rows, int nnz, int chunksPerWarp,
                                                                            Scalars<CompT> sc)
 {
-    constexpr int kSteps = kTransChunk / 32;
+    constexpr int kSteps = kChunk / 32;
     __shared__ uint32_t sBits[kTransWarps][kSteps];
-    __shared__ CompT sFactor[kTransWarps][kTransChunk];
+    __shared__ CompT sFactor[kTransWarps][kChunk];
     b200sp::WaitForPrevious();
     const CompT alpha = sc.Alpha();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t *bits = sBits[warp];
     CompT *factor = sFactor[warp];
-    long long c0 = ((long long)blockIdx.x * kTransWarps + warp) * chunksPerWarp * kTransChunk;
+    long long c0 = ((long long)blockIdx.x * kTransWarps + warp) * chunksPerWarp * kChunk;
     if (c0 >= nnz) return;
     int r0 = b200sp::WarpRowOf(rowPtr, rows, c0, lane);  // a row that starts at or before the chunk's first entry
-    for (int chunk = 0; chunk < chunksPerWarp && c0 < nnz; ++chunk, c0 += kTransChunk) {
+    for (int chunk = 0; chunk < chunksPerWarp && c0 < nnz; ++chunk, c0 += kChunk) {
         int c[kSteps];
         ValT v[kSteps];
 #pragma unroll
@@ -1413,7 +1413,7 @@ __global__ void __launch_bounds__(32 * kTransWarps, 5) SpmvTransScatterKernel(co
             c[u] = p < nnz ? __ldcs(colInd + p) : -1;
             v[u] = p < nnz ? __ldcs(val + p) : ValT(0);
         }
-        const int first = (int)c0, last = (int)(c0 + kTransChunk < nnz ? c0 + kTransChunk - 1 : nnz - 1);
+        const int first = (int)c0, last = (int)(c0 + kChunk < nnz ? c0 + kChunk - 1 : nnz - 1);
         auto add = [&](int u, CompT f) {
             if (c[u] >= 0 && f != CompT(0)) atomicAdd(acc + c[u], static_cast<AccT>(f * Widen<CompT>(v[u])));
         };
@@ -1796,9 +1796,13 @@ int LaunchTransTyped(const int32_t *rowPtr, const int32_t *colInd, const void *v
     if (cols == 0) return 0;
     const int sms = b200sp_sm_count();
     const unsigned eltBlocks = (unsigned)((cols + 255) / 256 < (int64_t)sms * 16 ? (cols + 255) / 256 : sms * 16);
-    // Consecutive chunks share a warp (and its first search), as long as every SM gets its 64 warps twice.
-    const int64_t chunks = (nnz + kTransChunk - 1) / kTransChunk;
-    const int perWarp = chunks >= 4 * 128ll * sms ? 4 : chunks >= 2 * 128ll * sms ? 2 : 1;
+    // Consecutive chunks share a warp (and its first search), as long as every SM gets its 64 warps twice.  Few entries are
+    // shared by as many warps as the SMs hold, which then wait for one step's searches and loads instead of eight (2 M rows
+    // with 20,000 entries: 40 us with chunks of 256, 8 so).
+    const bool small = nnz <= 32ll * 5 * kTransWarps * sms;
+    const int chunkLen = small ? 32 : kTransChunk;
+    const int64_t chunks = (nnz + chunkLen - 1) / chunkLen;
+    const int perWarp = small ? 1 : chunks >= 4 * 128ll * sms ? 4 : chunks >= 2 * 128ll * sms ? 2 : 1;
     const unsigned blocks = (unsigned)((chunks + kTransWarps * perWarp - 1) / (kTransWarps * perWarp));
     const auto *v = static_cast<const ValT *>(val), *xv = static_cast<const ValT *>(x);
     // A 16-bit y accumulates in scratch and is rounded once.
@@ -1812,8 +1816,8 @@ int LaunchTransTyped(const int32_t *rowPtr, const int32_t *colInd, const void *v
                                           (int)cols, sc);
     if (e == cudaSuccess && rows > 0 && nnz > 0) {
         b200sp_note_launches(1);
-        e = b200sp::LaunchChained(SpmvTransScatterKernel<CompT, ValT, AccT>, blocks, 32 * kTransWarps, 0, stream, rowPtr, colInd, v, xv, acc,
-                                  (int)rows, (int)nnz, perWarp, sc);
+        e = b200sp::LaunchChained(small ? SpmvTransScatterKernel<CompT, ValT, AccT, 32> : SpmvTransScatterKernel<CompT, ValT, AccT, kTransChunk>,
+                                  blocks, 32 * kTransWarps, 0, stream, rowPtr, colInd, v, xv, acc, (int)rows, (int)nnz, perWarp, sc);
     }
     if constexpr (kNarrowOut) {
         if (e == cudaSuccess) {
