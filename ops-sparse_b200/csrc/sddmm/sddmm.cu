@@ -118,11 +118,12 @@ template <typename T> __device__ __forceinline__ float DotPiece(uint32_t x, uint
     return DotWord(x, y, acc, T());
 }
 
-// kSize bytes from global to shared memory; `bytes` of them are read, the rest is zero.
-template <int kSize> __device__ __forceinline__ void CopyAsync(void *dst, const void *src, int bytes)
+// kSize bytes from global to shared memory; `bytes` of them are read, the rest is zero.  Copies of 16 bytes go past L1
+// (.cg) or, kNear, through it.
+template <int kSize, bool kNear = true> __device__ __forceinline__ void CopyAsync(void *dst, const void *src, int bytes)
 {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    if constexpr (kSize == 16)
+    if constexpr (!kNear)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
     else
         asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(kSize), "r"(bytes) : "memory");
@@ -143,7 +144,7 @@ template <int kBytes, int kLanes, int kSlabs> struct SddmmShape {
     static constexpr int kCtaBytes = kSddmmWarps * kWarpBytes;
 };
 
-template <typename T, int kBytes, int kLanes, int kSlabs>
+template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear>
 __global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(
     const int32_t *__restrict__ rowPtr, const int32_t *__restrict__ colInd, T *__restrict__ cVal, const char *__restrict__ X,
     const char *__restrict__ Y, int m, int k, int nnz, int tile, long long xRowBytes, long long yRowBytes, float alpha,
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(
                     CopyAsync<4>(slot + s * 32 + lane, row - off + (bytes > 0 ? 4ll * q : 0), bytes);
                 } else {
                     const bool in = q < pieces;
-                    CopyAsync<kCopy>(slot + s * 32 + lane, row + (in ? (long long)q * kBytes : 0), in ? kCopy : 0);
+                    CopyAsync<kCopy, kNear || kCopy != 16>(slot + s * 32 + lane, row + (in ? (long long)q * kBytes : 0), in ? kCopy : 0);
                 }
             }
         };
@@ -357,7 +358,7 @@ aclsparseStatus_t ValidateCall(aclsparseHandle_t handle, const aclsparseDnMatDes
     return ACL_SPARSE_STATUS_SUCCESS;
 }
 
-template <typename T, int kBytes, int kLanes, int kSlabs, typename... Args>
+template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear, typename... Args>
 int LaunchRowsShape(int nnz, int tile, cudaStream_t stream, Args... args)
 {
     using Shape = SddmmShape<kBytes, kLanes, kSlabs>;
@@ -365,17 +366,22 @@ int LaunchRowsShape(int nnz, int tile, cudaStream_t stream, Args... args)
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
     if (!configured[dev].load(std::memory_order_relaxed)) {
-        const cudaError_t e = cudaFuncSetAttribute(SddmmRowsKernel<T, kBytes, kLanes, kSlabs>,
+        const cudaError_t e = cudaFuncSetAttribute(SddmmRowsKernel<T, kBytes, kLanes, kSlabs, kNear>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::kCtaBytes);
         if (e != cudaSuccess) return (int)e;
         configured[dev].store(true, std::memory_order_relaxed);
     }
     const long long warps = ((long long)nnz + tile - 1) / tile;
     b200sp_note_launches(1);
-    return (int)b200sp::LaunchChained(SddmmRowsKernel<T, kBytes, kLanes, kSlabs>,
+    return (int)b200sp::LaunchChained(SddmmRowsKernel<T, kBytes, kLanes, kSlabs, kNear>,
                                       (unsigned)((warps + kSddmmWarps - 1) / kSddmmWarps), 32 * kSddmmWarps, Shape::kCtaBytes,
                                       stream, args...);
 }
+
+// 300,000 rows of up to eight entries, 16-byte copies past L1 and through it, us, by the size of Y: 9 columns, fp16, k = 16 (0.3 KB) 298
+// and 31, k = 200 (3.5 KB) 543 and 108, fp32, k = 300 (10.5 KB) 1085 and 304; 100 columns, fp16, k = 64 (12.5 KB) 36 and 39, fp32,
+// k = 64 (25 KB) 55 and 63; 1 M columns, fp16, k = 256, 16 M entries: 1404 and 1618.
+constexpr long long kNearBytes = 12 << 10;
 
 template <typename T, int kBytes>
 int LaunchRows(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const aclsparseDnMatDescr *Y, int k, Strides st,
@@ -387,12 +393,19 @@ int LaunchRows(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const
     // The longer the tile the longer the runs of copies in flight, as long as every SM gets some 16 warps.
     int tile = 32;
     while (tile < kSddmmTile && nnz / (2 * tile) >= 16 * b200sp_sm_count()) tile *= 2;
-    auto launch = [&]<int kLanes, int kSlabs>() {
-        return LaunchRowsShape<T, kBytes, kLanes, kSlabs>(
+    // A Y of a few lines that all entries want is asked of a few slices of L2 by every SM at once: it comes through L1.
+    const bool near = kBytes == 16 && (long long)C->cols * st.yj * (long long)sizeof(T) <= kNearBytes;
+    auto launchAs = [&]<int kLanes, int kSlabs, bool kNear>() {
+        return LaunchRowsShape<T, kBytes, kLanes, kSlabs, kNear>(
             nnz, tile, stream, static_cast<const int32_t *>(C->offsets), static_cast<const int32_t *>(C->indices),
             static_cast<T *>(C->values), static_cast<const char *>(X->values), static_cast<const char *>(Y->values),
             (int)C->rows, k, nnz, tile, st.xi * (long long)sizeof(T), st.yj * (long long)sizeof(T), alpha, beta,
             static_cast<const T *>(alphaDev), static_cast<const T *>(betaDev));
+    };
+    auto launch = [&]<int kLanes, int kSlabs>() {
+        if constexpr (kBytes == 16)
+            if (near) return launchAs.template operator()<kLanes, kSlabs, true>();
+        return launchAs.template operator()<kLanes, kSlabs, false>();
     };
     if (pieces <= 4) return launch.template operator()<4, 1>();
     if (pieces <= 8) return launch.template operator()<8, 1>();

@@ -25,8 +25,15 @@ def test_entry_counts(pkg, handle, device, nnz):
     check(pkg, handle, device, rng, lengths, 24, 0, "f16")
 
 
-def check(pkg, handle, device, rng, lengths, k, pad, dtype):
-    m, n = lengths.size, 300
+@pytest.mark.parametrize("dtype,k,n", [("f32", 64, 47), ("f32", 64, 48), ("f32", 64, 49), ("f16", 16, 9), ("f16", 1024, 6), ("f16", 1024, 7)])
+def test_few_rows_of_y(pkg, handle, device, dtype, k, n):
+    """Y up to 12 KB comes through L1, a larger one past it."""
+    rng = np.random.default_rng(n)
+    check(pkg, handle, device, rng, rng.integers(0, 9, 90), k, 0, dtype, n)
+
+
+def check(pkg, handle, device, rng, lengths, k, pad, dtype, n=300):
+    m = lengths.size
     rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
     ci = rng.integers(0, n, rp[-1]).astype(np.int32)
     X, xs, ldx = dense_operand(rng, m, k, "row", pad, dtype)
