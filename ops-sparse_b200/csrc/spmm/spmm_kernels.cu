@@ -1888,6 +1888,26 @@ bool WorthRepacking(const b200spSpmmShape *sh, int valBytes)
     return 16 * sh->nnz >= sh->k * valBytes;
 }
 
+// Products whose rows are a few entries, on a few columns of B that do not lie in 16-byte rows: a thread per output (the generic
+// kernel) has nothing to wait for one after the other, and a copy of B or a lane group per row costs more than it saves
+// unless the copy is read back very often.  Thread per output / lane groups, us:
+//   columns of B contiguous: 500,000 rows of one entry, fp32, N = 1, 3 and 8: 8 / 32, 14 / 33 and 30 / 43; a million of three, 18 / 62,
+//     42 / 64 and 113 / 86; 700,000 of three, N = 5: 50 / 62; of three on 43,750 columns, N = 3: 28 / 24; of one, N = 13: 63 / 54;
+//   rows of B contiguous: a million rows of three, fp16, N = 1 and 3: 18 / 33 and 24 / 33;
+//   int8: 500,000 rows of one entry, columns, N = 1, 8 and 33: 8 / 78, 30 / 94 and 171 / 132; 700,000 of four, N = 9 and 13: 111 / 137 and
+//     162 / 148, rows, N = 9: 41 / 115.  Rows of up to 32 entries whose B rows are eight bytes at most go the same way: eight lanes of 16 columns join more
+//     sums than they save loads (275,178 rows of 26, N = 8: 51 to 53 / 63).
+bool FewEntries(const b200spSpmmShape *sh, int valBytes, int32_t segments)
+{
+    if (segments + sh->mid_units != 0) return false;
+    const bool rows = RowsContiguous(sh->op_b, sh->order_b);
+    if (valBytes == 1)
+        return (sh->n <= 16 && sh->nnz <= 4 * sh->m && (rows || sh->nnz * sh->n <= 40 * sh->m)) ||
+               (rows && sh->n <= 8 && sh->nnz <= 32 * sh->m);
+    if (sh->nnz > 24 * sh->k) return false;
+    return rows ? sh->n <= 4 && sh->nnz <= 4 * sh->m : sh->n <= 12 && sh->nnz * sh->n <= 16 * sh->m;
+}
+
 // Whether a product with this much room for a copy makes one.
 bool Copies(const b200spSpmmShape *sh, int valBytes, int32_t segments, const void *plan)
 {
@@ -1895,7 +1915,8 @@ bool Copies(const b200spSpmmShape *sh, int valBytes, int32_t segments, const voi
     // A product of one wave of short rows takes less time than the second launch.
     const bool small = sh->m * sh->n < 148ll * 2048 && segments + sh->mid_units == 0 && sh->nnz <= 16 * sh->m;
     // The copy follows the plan (a multiple of 256 bytes) and is stored 16 bytes at a time; the plan itself may start on any word.
-    return repack > 0 && sh->repack_bytes >= (int64_t)repack && WorthRepacking(sh, valBytes) && !small && plan != nullptr && Aligned16(plan);
+    return repack > 0 && sh->repack_bytes >= (int64_t)repack && WorthRepacking(sh, valBytes) && !small &&
+           !FewEntries(sh, valBytes, segments) && plan != nullptr && Aligned16(plan);
 }
 
 template <typename ValT, typename OutT>
@@ -1930,13 +1951,9 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
     const bool vectors = RowsContiguous(sh->op_b, sh->order_b) && sh->n % E == 0 && sh->ldb % E == 0 && Aligned16(B);
     const bool copy = Copies(sh, (int)sizeof(ValT), segments, plan);
     const bool words = !vectors && !copy && RowsOfWords(sh, (int)sizeof(ValT)) && reinterpret_cast<uintptr_t>(B) % 4 == 0;
-    // Rows of four entries leave the generic kernel, with a thread per output, nothing to wait for one after the other
-    // (695,764 of them, fp32, N = 11: 70 us; by words 79).
-    // So do int8 rows of up to 32 entries whose B rows are eight bytes at most: eight lanes of 16 columns join more sums
-    // than they save loads (275,178 rows of 26, N = 8: 51 to 53 us; by lane groups 63).
-    const bool alike = segments + sh->mid_units == 0;
-    const bool few = kInt8 ? sh->n <= 8 && sh->nnz <= 32 * sh->m && alike && RowsContiguous(sh->op_b, sh->order_b)
-                           : words && sh->n <= 16 && sh->nnz <= 4 * sh->m && alike;
+    // By words, rows of up to four entries: 695,764 of them, fp32, N = 11: 70 us, by lane groups 79.
+    const bool few = !vectors && (FewEntries(sh, (int)sizeof(ValT), segments) ||
+                                  (words && sh->n <= 16 && sh->nnz <= 4 * sh->m && segments + sh->mid_units == 0));
     const bool bReady = !few && (vectors || words || copy);
     if (plan == nullptr || !bReady)
         return LaunchGeneric<ValT, OutT>(rowPtr, colInd, val, B, C, sh, s, stream);

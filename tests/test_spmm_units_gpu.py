@@ -77,3 +77,36 @@ def test_int8(handle, device, oracle, filler, n, order):
     import scipy.sparse
     A = scipy.sparse.csr_matrix((val.astype(np.int64), ci, rp), shape=(m, k))
     assert np.array_equal(got, (2 * (A @ B.astype(np.int64)) - C).astype(np.int32))
+
+
+@pytest.mark.parametrize("order", ["row", "col"])
+@pytest.mark.parametrize("vt,ot", [("f32", "f32"), ("f16", "f16"), ("i8", "i32")])
+@pytest.mark.parametrize("m,k,entries", [(4000, 4000, 1), (4000, 4000, 4), (4000, 4000, 5), (40_000, 1666, 1), (40_000, 1667, 1)])
+def test_rows_of_a_few_entries(handle, device, oracle, m, k, entries, vt, ot, order):
+    """Both sides of the rule that gives such rows a thread per output: entries of a row, columns of B, uses of a row of B."""
+    rng = np.random.default_rng(m + k + entries)
+    lengths = np.full(m, entries)
+    for n in (1, 3, 4, 5, 8, 9, 10, 11, 12, 13, 16, 17):
+        if vt == "i8":
+            rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+            ci = rng.integers(0, k, rp[-1]).astype(np.int32)
+            val, B = (rng.integers(-128, 128, shape).astype(np.int8) for shape in (ci.size, (k, n)))
+            C = rng.integers(-1000, 1000, (m, n)).astype(np.int32)
+            alpha, beta = 2, -1
+        else:
+            alpha, beta = 1.5, -0.5
+            rp, ci, val, B, C = compact_case(oracle, rng, m, k, n, lengths, vt, ot, alpha, beta)
+        stored = (lambda a: a) if order == "row" else (lambda a: np.ascontiguousarray(a.T))
+        ldb, ldc = (n, n) if order == "row" else (k, m)
+        got = run_spmm(handle, device, rp, ci, val, vt, stored(B), stored(C), ot, m, k, n, ldb, ldc, alpha, beta,
+                       b_order=order, c_order=order)
+        got = got.reshape(m, n) if order == "row" else np.ascontiguousarray(got.reshape(n, m).T)
+        if vt == "i8":
+            want = 2 * np.add.reduceat(val.astype(np.int64)[:, None] * B[ci].astype(np.int64), rp[:-1]) - C
+            assert np.array_equal(got, want.astype(np.int32))
+            continue
+        if vt == "f32":
+            gold = oracle.spmm_f32_layout(m, n, rp, ci, val, B, n, True, False, C, n, True, alpha, beta)
+        else:
+            gold = oracle.spmm_16(rp, ci, val, B, C, alpha, beta, vt, ot)
+        assert np.array_equal(got.view(np.uint8), np.asarray(gold).reshape(m, n).view(np.uint8))
