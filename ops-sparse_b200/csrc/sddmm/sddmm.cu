@@ -8,6 +8,7 @@
 #include <atomic>
 #include <climits>
 #include <cstdint>
+#include <type_traits>
 
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -76,46 +77,52 @@ __global__ void __launch_bounds__(256) SddmmKernel(const int32_t *__restrict__ r
 // two short rows, so the work is fetching a row of Y per entry; what counts is how many of them an SM has in flight
 // and how few instructions go into each.
 //   - kLanes lanes lie side by side on a row, kBytes bytes each (the widest the rows' alignment allows) and kSlabs pieces
-//     apart; a warp therefore works on 32 / kLanes entries at a time, and rows wider than 32 * kSlabs pieces take
+//     apart; a warp therefore works on 32 / kLanes entries at a time, and rows wider than kLanes * kSlabs pieces take
 //     several turns.
-//   - Rows come through shared memory by cp.async, kStages batches of kBatch entries deep per lane group: no registers
-//     hold data in flight.  A row of X is copied only when it differs from the entry before.
+//   - Rows come through shared memory by cp.async, two batches of kBatch entries deep per lane group: no registers
+//     hold data in flight.  The batches are as short as the sums allow, for what a warp's ring leaves free are more warps, and those
+//     keep more copies in flight than longer rings do: 100,000 rows of up to 40 entries, fp16, k = 400, two pieces a lane: 265 us
+//     with four entries a batch, 225 with two; f32, k = 512, four pieces: 327 with two, 273 with one; three or four batches deep, with as
+//     many copies in flight per warp, 1.1 to 1.6 times as long.
+//   - A row of X is copied only when it differs from the entry before, and stays in registers, converted, until then.  Two products
+//     share an instruction (packed fp32): a row of 512 bytes in fp16 takes some 30 instead of 47 instructions.
 //   - A warp owns a tile of consecutive entries.  What is done once per entry (row, column, old value, store) is done
 //     for the whole tile with coalesced accesses; lane group g works on the tile's g-th part.
-//   - The kBatch sums of a batch are reduced together: every butterfly step that halves the number of values a lane
-//     carries costs as many shuffles as values are left (6 instead of 20 for four sums over 32 lanes).
+//   - The kBatch sums of a batch are reduced together: a butterfly step that halves the number of values a lane
+//     carries costs as many shuffles as values are left.
 // fp16 rows that start on odd 2-byte addresses (kBytes = 2) are copied as the 4-byte words that cover them and
 // realigned when they are read from shared memory.
-// Measured (1 M nodes, 16.0 M entries, fp16, k = 256, inputs that alternate): 2103 us with the rows in registers, four entries in flight
-// and a full butterfly per entry; 1477 us here.  The kernel alone moves 7.6 GB of Y rows in 1261 us, 6.1 TB/s.
+// Measured (1 M nodes, 16.0 M entries, fp16, k = 256): 1242 us with 32 lanes a row and scalar products, 1166 us here, which is the 7.6 GB
+// of Y rows that come from DRAM at 6.5 TB/s.  Working through Y by blocks of columns that stay in L2 (the pieces of rows of 64 entries and
+// more that lie in a block taken together) cut that to 5.6 GB and cost 1930 us and more: short pieces, and X rows fetched anew for each.
 template <int kBytes> struct Words { using Type = uint32_t; };  // 4, and the words of kBytes = 2
 template <> struct Words<16> { using Type = uint4; };
 template <> struct Words<8> { using Type = uint2; };
 
-__device__ __forceinline__ float DotWord(uint32_t x, uint32_t y, float acc, float)
+// The fp32 values of a piece, in pairs: packed arithmetic takes two of them per instruction.
+template <typename T, typename Piece> struct Pairs {
+    static constexpr int kCount = sizeof(Piece) / (2 * sizeof(T)) > 0 ? sizeof(Piece) / (2 * sizeof(T)) : 1;
+    float2 v[kCount];
+    __device__ __forceinline__ void Set(const Piece &p)
+    {
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(&p);
+        if constexpr (sizeof(T) == 2) {
+#pragma unroll
+            for (int i = 0; i < kCount; ++i) v[i] = __half22float2(reinterpret_cast<const __half2 *>(w)[i]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < kCount; ++i)
+                v[i] = make_float2(__uint_as_float(w[2 * i]), sizeof(Piece) > 4 ? __uint_as_float(w[2 * i + 1]) : 0.0f);
+        }
+    }
+};
+__device__ __forceinline__ void FmaPair(float2 &acc, const float2 &x, const float2 &y)
 {
-    return fmaf(__uint_as_float(x), __uint_as_float(y), acc);
-}
-__device__ __forceinline__ float DotWord(uint32_t x, uint32_t y, float acc, __half)
-{
-    const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&x)), b = __half22float2(*reinterpret_cast<const __half2 *>(&y));
-    return fmaf(a.y, b.y, fmaf(a.x, b.x, acc));
-}
-template <typename T> __device__ __forceinline__ float DotPiece(const uint4 &x, const uint4 &y, float acc)
-{
-    acc = DotWord(x.x, y.x, acc, T());
-    acc = DotWord(x.y, y.y, acc, T());
-    acc = DotWord(x.z, y.z, acc, T());
-    return DotWord(x.w, y.w, acc, T());
-}
-template <typename T> __device__ __forceinline__ float DotPiece(const uint2 &x, const uint2 &y, float acc)
-{
-    acc = DotWord(x.x, y.x, acc, T());
-    return DotWord(x.y, y.y, acc, T());
-}
-template <typename T> __device__ __forceinline__ float DotPiece(uint32_t x, uint32_t y, float acc)
-{
-    return DotWord(x, y, acc, T());
+    asm("{\n\t.reg .b64 a, b, c;\n\t"
+        "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%0, %1};\n\t"
+        "fma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
+        : "+f"(acc.x), "+f"(acc.y)
+        : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
 }
 
 // kSize bytes from global to shared memory; `bytes` of them are read, the rest is zero.  Copies of 16 bytes go past L1
@@ -133,22 +140,26 @@ template <int kPending> __device__ __forceinline__ void CopyWait() { asm volatil
 
 // The same inputs again and again: 1384 us with 4 warps and tiles of 128, 1286 with 2 and 64 on the same GPU; one warp or longer tiles gain nothing more.
 constexpr int kSddmmWarps = 2;
-constexpr int kSddmmTile = 64;  // entries a warp owns at most
+constexpr int kSddmmTile = 64;  // entries a warp works on at a time, at most
 template <int kBytes, int kLanes, int kSlabs> struct SddmmShape {
-    static constexpr int kBatch = kSlabs >= 4 ? 2 : 4;
+    static constexpr int kBatch = kSlabs <= 2 ? 2 : 1;
     static constexpr int kStages = 2;
     static constexpr int kCopy = kBytes == 2 ? 4 : kBytes;
     static constexpr int kSlotBytes = 32 * kSlabs * kCopy;                       // one entry of every lane group
     static constexpr int kRing = 2 * kStages * kBatch * kSlotBytes;              // rows of Y, rows of X
-    static constexpr int kWarpBytes = kRing + kSddmmTile * 12;                   // and row, column, sum per entry
-    static constexpr int kCtaBytes = kSddmmWarps * kWarpBytes;
+    static constexpr int kTileBytes = kSddmmTile * 12;                           // row, column, sum per entry
 };
 
+struct RowsOf {  // the operands' rows and how far apart they are
+    const char *X, *Y;
+    long long xRowBytes, yRowBytes;
+    int k;
+};
+
+// The dot products of a tile of entries: sDot[t] = X row sRow[t] . Y row sCol[t].  tile: a multiple of 32.
 template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear>
-__global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(
-    const int32_t *__restrict__ rowPtr, const int32_t *__restrict__ colInd, T *__restrict__ cVal, const char *__restrict__ X,
-    const char *__restrict__ Y, int m, int k, int nnz, int tile, long long xRowBytes, long long yRowBytes, float alpha,
-    float beta, const T *alphaDev, const T *betaDev)
+__device__ __forceinline__ void TileDots(const RowsOf &rows, unsigned char *ring, const int *sRow, const int *sCol, float *sDot,
+                                         int tile, int lane)
 {
     using Shape = SddmmShape<kBytes, kLanes, kSlabs>;
     using Piece = typename Words<kBytes>::Type;
@@ -157,31 +168,11 @@ __global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(
     constexpr int kCopy = Shape::kCopy;
     constexpr bool kOdd = kBytes == 2;
     static_assert(kLanes >= 4, "the sums of a batch are spread over four lanes");
-    extern __shared__ __align__(16) unsigned char sRaw[];
-    b200sp::WaitForPrevious();
-    const float a = alphaDev ? Load<T>(alphaDev) : alpha;
-    const float b = betaDev ? Load<T>(betaDev) : beta;
-    const int lane = threadIdx.x & 31;
+    using Ints = std::conditional_t<kBatch == 4, int4, std::conditional_t<kBatch == 2, int2, int>>;
     const int li = lane & (kLanes - 1);
     const int group = lane / kLanes;
-    const long long p0 = ((long long)blockIdx.x * kSddmmWarps + (threadIdx.x >> 5)) * tile;
-    if (p0 >= nnz) return;
-    unsigned char *sWarp = sRaw + (threadIdx.x >> 5) * Shape::kWarpBytes;
-    Piece *sY = reinterpret_cast<Piece *>(sWarp), *sX = sY + kStages * kBatch * kSlabs * 32;
-    int *sRow = reinterpret_cast<int *>(sWarp + Shape::kRing), *sCol = sRow + kSddmmTile;
-    float *sDot = reinterpret_cast<float *>(sCol + kSddmmTile);
-
-    int r0 = b200sp::WarpRowOf(rowPtr, m, p0, lane);
-    for (int t = lane; t < tile; t += 32) {
-        const int p = p0 + t < nnz ? (int)p0 + t : nnz - 1;  // past the end: the last entry again, not stored
-        const int r = b200sp::RowOfLane(rowPtr, m, r0, p, lane);
-        sRow[t] = r;
-        sCol[t] = __ldg(colInd + p);
-        sDot[t] = 0.0f;
-        r0 = __shfl_sync(0xffffffffu, r, 31);
-    }
-    __syncwarp();
-
+    Piece *const sY = reinterpret_cast<Piece *>(ring) + lane, *const sX = sY + kStages * kBatch * kSlabs * 32;
+    const int k = rows.k;
     // unsigned: a row may hold 2^31 - 1 elements, and the last turn ends beyond its last piece
     const unsigned pieces = kOdd ? ((unsigned)k + 1) / 2 : (unsigned)((long long)k * (int)sizeof(T) / kBytes);
     const int perGroup = tile / (32 / kLanes);
@@ -189,32 +180,40 @@ __global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(
     const int batches = perGroup / kBatch;
     for (unsigned piece0 = 0; piece0 < pieces; piece0 += kLanes * kSlabs - (kOdd ? 1 : 0)) {
         const int width = kLanes * kSlabs - (kOdd ? 1 : 0);
+        [[maybe_unused]] int inside[kSlabs];  // bytes of the lane's pieces that lie in the row, ...
+        [[maybe_unused]] long long offset[kSlabs];  // ... and where they start
+#pragma unroll
+        for (int s = 0; s < kSlabs; ++s) {
+            const unsigned q = piece0 + s * kLanes + li;
+            inside[s] = q < pieces ? kCopy : 0;
+            offset[s] = q < pieces ? (long long)q * kBytes : 0;
+        }
         auto copyRow = [&](Piece *slot, const char *row) {
 #pragma unroll
             for (int s = 0; s < kSlabs; ++s) {
-                const unsigned q = piece0 + s * kLanes + li;
                 if constexpr (kOdd) {  // words from the one that holds the first element on, zeros after the row's last
+                    const unsigned q = piece0 + s * kLanes + li;
                     const int off = (int)(reinterpret_cast<uintptr_t>(row) & 2);
                     const unsigned end = (unsigned)k + (unsigned)off / 2;  // of the row, in elements from the first word on
                     const int bytes = end >= 2 * q + 2 ? 4 : end > 2 * q ? 2 : 0;
-                    CopyAsync<4>(slot + s * 32 + lane, row - off + (bytes > 0 ? 4ll * q : 0), bytes);
+                    CopyAsync<4>(slot + s * 32, row - off + (bytes > 0 ? 4ll * q : 0), bytes);
                 } else {
-                    const bool in = q < pieces;
-                    CopyAsync<kCopy, kNear || kCopy != 16>(slot + s * 32 + lane, row + (in ? (long long)q * kBytes : 0), in ? kCopy : 0);
+                    CopyAsync<kCopy, kNear || kCopy != 16>(slot + s * 32, row + offset[s], inside[s]);
                 }
             }
         };
+        int asked = -1;  // the row of X copied last
         auto request = [&](int batch) {
             if (batch < batches) {
-                const int stage = batch % kStages;
-                int before = batch > 0 ? sRow[t0 + batch * kBatch - 1] : -1;
+                const int slot0 = (batch % kStages) * kBatch * kSlabs * 32;
+                const Ints rowOf = *reinterpret_cast<const Ints *>(sRow + t0 + batch * kBatch);
+                const Ints colOf = *reinterpret_cast<const Ints *>(sCol + t0 + batch * kBatch);
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u) {
-                    const int t = t0 + batch * kBatch + u;
-                    const int row = sRow[t];
-                    copyRow(sY + (stage * kBatch + u) * kSlabs * 32, Y + sCol[t] * yRowBytes);
-                    if (row != before) copyRow(sX + (stage * kBatch + u) * kSlabs * 32, X + row * xRowBytes);
-                    before = row;
+                    const int row = reinterpret_cast<const int *>(&rowOf)[u];
+                    copyRow(sY + slot0 + u * kSlabs * 32, rows.Y + reinterpret_cast<const int *>(&colOf)[u] * rows.yRowBytes);
+                    if (row != asked) copyRow(sX + slot0 + u * kSlabs * 32, rows.X + row * rows.xRowBytes);
+                    asked = row;
                 }
             }
             CopyCommit();
@@ -224,18 +223,18 @@ __global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(
             if constexpr (kOdd) {
                 const int i = s * kLanes + li;  // word of the turn; the last one only completes its neighbour
                 const int next = i + 1 < kLanes * kSlabs ? i + 1 : i;
-                const uint32_t w0 = slot[s * 32 + lane];
-                const uint32_t w1 = slot[(next / kLanes) * 32 + group * kLanes + (next & (kLanes - 1))];
+                const uint32_t w0 = slot[s * 32];
+                const uint32_t w1 = slot[(next / kLanes) * 32 + group * kLanes + (next & (kLanes - 1)) - lane];
                 const uint32_t v = __funnelshift_r(w0, w1, (uint32_t)(reinterpret_cast<uintptr_t>(row) & 2) * 8);
                 return i < width ? v : 0u;
             } else {
-                return slot[s * 32 + lane];
+                return slot[s * 32];
             }
         };
-        Piece x[kSlabs];
+        Pairs<T, Piece> x[kSlabs];
 #pragma unroll
-        for (int s = 0; s < kSlabs; ++s) x[s] = Piece{};
-        int before = -1;
+        for (int s = 0; s < kSlabs; ++s) x[s].Set(Piece{});
+        int held = -1;  // the row of X in x
 #pragma unroll
         for (int i = 0; i < kStages - 1; ++i) request(i);
 #pragma unroll 1
@@ -243,24 +242,31 @@ __global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(
             request(batch + kStages - 1);
             CopyWait<kStages - 1>();
             __syncwarp();
-            const int stage = batch % kStages;
+            const int slot0 = (batch % kStages) * kBatch * kSlabs * 32;
+            const Ints rowOf = *reinterpret_cast<const Ints *>(sRow + t0 + batch * kBatch);
+            Ints colOf{};
+            if constexpr (kOdd) colOf = *reinterpret_cast<const Ints *>(sCol + t0 + batch * kBatch);
             float acc[kBatch];
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
-                const int t = t0 + batch * kBatch + u;
-                const int row = sRow[t];
-                if (row != before) {
+                const int row = reinterpret_cast<const int *>(&rowOf)[u];
+                if (row != held) {
 #pragma unroll
-                    for (int s = 0; s < kSlabs; ++s) x[s] = read(sX + (stage * kBatch + u) * kSlabs * 32, X + row * xRowBytes, s);
-                    before = row;
+                    for (int s = 0; s < kSlabs; ++s) x[s].Set(read(sX + slot0 + u * kSlabs * 32, rows.X + row * rows.xRowBytes, s));
+                    held = row;
                 }
-                acc[u] = 0.0f;
+                float2 sum = make_float2(0.0f, 0.0f);
 #pragma unroll
-                for (int s = 0; s < kSlabs; ++s)
-                    acc[u] = DotPiece<T>(x[s], read(sY + (stage * kBatch + u) * kSlabs * 32, Y + sCol[t] * yRowBytes, s), acc[u]);
+                for (int s = 0; s < kSlabs; ++s) {
+                    Pairs<T, Piece> y;
+                    y.Set(read(sY + slot0 + u * kSlabs * 32, rows.Y + reinterpret_cast<const int *>(&colOf)[u] * rows.yRowBytes, s));
+#pragma unroll
+                    for (int i = 0; i < Pairs<T, Piece>::kCount; ++i) FmaPair(sum, x[s].v[i], y.v[i]);
+                }
+                acc[u] = sum.x + sum.y;
             }
             // Lanes with bit kLanes/2 set keep the upper half of the values, then those with bit kLanes/4 the odd ones.
-            const bool up = (li & (kLanes / 2)) != 0;
+            [[maybe_unused]] const bool up = (li & (kLanes / 2)) != 0;
             float v;
             int u;  // the value this lane ends up with
             if constexpr (kBatch == 4) {
@@ -271,18 +277,56 @@ __global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(
 #pragma unroll
                 for (int off = kLanes / 8; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
                 u = (up ? 2 : 0) + (odd ? 1 : 0);
+            } else if constexpr (kBatch == 1) {
+                v = acc[0];
+#pragma unroll
+                for (int off = kLanes / 2; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+                u = 0;
             } else {
                 v = (up ? acc[1] : acc[0]) + __shfl_xor_sync(0xffffffffu, up ? acc[0] : acc[1], kLanes / 2);
 #pragma unroll
                 for (int off = kLanes / 4; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
                 u = up ? 1 : 0;
             }
-            if ((li & (kLanes / kBatch - 1)) == 0) sDot[t0 + batch * kBatch + u] += v;
+            if ((li & (kLanes / kBatch - 1)) == 0) {
+                float *dot = sDot + t0 + batch * kBatch + u;
+                *dot = piece0 == 0 ? v : *dot + v;
+            }
             __syncwarp();  // this stage's slots may be written again
         }
         CopyWait<0>();
         __syncwarp();
     }
+}
+
+template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear>
+__global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(const int32_t *__restrict__ rowPtr,
+                                                                    const int32_t *__restrict__ colInd, T *__restrict__ cVal,
+                                                                    const RowsOf rows, int m, int nnz, int tile, float alpha,
+                                                                    float beta, const T *alphaDev, const T *betaDev)
+{
+    using Shape = SddmmShape<kBytes, kLanes, kSlabs>;
+    extern __shared__ __align__(16) unsigned char sRaw[];
+    b200sp::WaitForPrevious();
+    const float a = alphaDev ? Load<T>(alphaDev) : alpha;
+    const float b = betaDev ? Load<T>(betaDev) : beta;
+    const int lane = threadIdx.x & 31;
+    const long long p0 = ((long long)blockIdx.x * kSddmmWarps + (threadIdx.x >> 5)) * tile;
+    if (p0 >= nnz) return;
+    unsigned char *ring = sRaw + (threadIdx.x >> 5) * (Shape::kRing + Shape::kTileBytes);
+    int *sRow = reinterpret_cast<int *>(ring + Shape::kRing), *sCol = sRow + kSddmmTile;
+    float *sDot = reinterpret_cast<float *>(sCol + kSddmmTile);
+    int r0 = b200sp::WarpRowOf(rowPtr, m, p0, lane);
+    for (int t = lane; t < tile; t += 32) {
+        const int p = p0 + t < nnz ? (int)p0 + t : nnz - 1;  // past the end: the last entry again, not stored
+        const int r = b200sp::RowOfLane(rowPtr, m, r0, p, lane);
+        sRow[t] = r;
+        sCol[t] = __ldg(colInd + p);
+        sDot[t] = 0.0f;
+        r0 = __shfl_sync(0xffffffffu, r, 31);
+    }
+    __syncwarp();
+    TileDots<T, kBytes, kLanes, kSlabs, kNear>(rows, ring, sRow, sCol, sDot, tile, lane);
     for (int t = lane; t < tile && p0 + t < nnz; t += 32) {
         float z = a * sDot[t];
         if (b != 0.0f) z += b * Load<T>(cVal + p0 + t);
@@ -358,23 +402,30 @@ aclsparseStatus_t ValidateCall(aclsparseHandle_t handle, const aclsparseDnMatDes
     return ACL_SPARSE_STATUS_SUCCESS;
 }
 
+// Whether the kernel may use the shared memory it wants on the current device: the attribute is set once per device.
+template <auto kKernel> cudaError_t AllowSharedMemory(int bytes, int *device)
+{
+    static std::atomic<bool> done[64] = {};
+    const cudaError_t got = cudaGetDevice(device);
+    if (got != cudaSuccess || *device < 0 || *device >= 64) return cudaErrorInvalidDevice;
+    if (done[*device].load(std::memory_order_relaxed)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done[*device].store(true, std::memory_order_relaxed);
+    return e;
+}
+
 template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear, typename... Args>
 int LaunchRowsShape(int nnz, int tile, cudaStream_t stream, Args... args)
 {
     using Shape = SddmmShape<kBytes, kLanes, kSlabs>;
-    static std::atomic<bool> configured[64] = {};  // per device: this instantiation may use kCtaBytes of shared memory
+    constexpr int kShared = kSddmmWarps * (Shape::kRing + Shape::kTileBytes);
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
-    if (!configured[dev].load(std::memory_order_relaxed)) {
-        const cudaError_t e = cudaFuncSetAttribute(SddmmRowsKernel<T, kBytes, kLanes, kSlabs, kNear>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::kCtaBytes);
-        if (e != cudaSuccess) return (int)e;
-        configured[dev].store(true, std::memory_order_relaxed);
-    }
+    const cudaError_t e = AllowSharedMemory<SddmmRowsKernel<T, kBytes, kLanes, kSlabs, kNear>>(kShared, &dev);
+    if (e != cudaSuccess) return (int)e;
     const long long warps = ((long long)nnz + tile - 1) / tile;
     b200sp_note_launches(1);
     return (int)b200sp::LaunchChained(SddmmRowsKernel<T, kBytes, kLanes, kSlabs, kNear>,
-                                      (unsigned)((warps + kSddmmWarps - 1) / kSddmmWarps), 32 * kSddmmWarps, Shape::kCtaBytes,
+                                      (unsigned)((warps + kSddmmWarps - 1) / kSddmmWarps), 32 * kSddmmWarps, kShared,
                                       stream, args...);
 }
 
@@ -396,22 +447,33 @@ int LaunchRows(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const
     // A Y of a few lines that all entries want is asked of a few slices of L2 by every SM at once: it comes through L1.
     const bool near = kBytes == 16 && (long long)C->cols * st.yj * (long long)sizeof(T) <= kNearBytes;
     auto launchAs = [&]<int kLanes, int kSlabs, bool kNear>() {
+        const RowsOf rows{static_cast<const char *>(X->values), static_cast<const char *>(Y->values),
+                          st.xi * (long long)sizeof(T), st.yj * (long long)sizeof(T), k};
         return LaunchRowsShape<T, kBytes, kLanes, kSlabs, kNear>(
             nnz, tile, stream, static_cast<const int32_t *>(C->offsets), static_cast<const int32_t *>(C->indices),
-            static_cast<T *>(C->values), static_cast<const char *>(X->values), static_cast<const char *>(Y->values),
-            (int)C->rows, k, nnz, tile, st.xi * (long long)sizeof(T), st.yj * (long long)sizeof(T), alpha, beta,
-            static_cast<const T *>(alphaDev), static_cast<const T *>(betaDev));
+            static_cast<T *>(C->values), rows, (int)C->rows, nnz, tile, alpha, beta, static_cast<const T *>(alphaDev),
+            static_cast<const T *>(betaDev));
     };
     auto launch = [&]<int kLanes, int kSlabs>() {
         if constexpr (kBytes == 16)
             if (near) return launchAs.template operator()<kLanes, kSlabs, true>();
         return launchAs.template operator()<kLanes, kSlabs, false>();
     };
+    // Few lanes and several pieces each: a warp then works on more entries per instruction.  16-byte pieces, us with 8 to 32 lanes of
+    // one piece (four entries a batch) and as here: 10 pieces 46.5 and 36.8, 12 123 and 93, 16 228 and 209, 20 147 and 110, 24 77.6 and
+    // 58.1, 32 (100,000 rows of up to 40 entries) 142 and 124; with 32 lanes of two or four pieces: 33 561 and 344, 50 300 and 212, 64
+    // (f32) 544 and 490, 75 622 and 450.  Up to 8 pieces and from 13 to 15 fewer lanes gain nothing (8 pieces: 52.8 and 60.7).
     if (pieces <= 4) return launch.template operator()<4, 1>();
     if (pieces <= 8) return launch.template operator()<8, 1>();
-    if (pieces <= 16) return launch.template operator()<16, 1>();
-    if (pieces <= 32) return launch.template operator()<32, 1>();
+    if (pieces <= 12) return launch.template operator()<4, 3>();
+    if (pieces < 16) return launch.template operator()<8, 2>();
+    if (pieces == 16) return launch.template operator()<4, 4>();
+    if (pieces <= 24) return launch.template operator()<8, 3>();
+    if (pieces <= 32) return launch.template operator()<8, 4>();
+    if (pieces <= 48) return launch.template operator()<16, 3>();
+    if (pieces <= 64) return launch.template operator()<16, 4>();
     if (pieces <= 64) return launch.template operator()<32, 2>();
+    if (pieces <= 96) return launch.template operator()<32, 3>();
     return launch.template operator()<32, 4>();
 }
 

@@ -18,6 +18,14 @@ def test_widths(pkg, handle, device, k, pad, dtype):
     check(pkg, handle, device, rng, rng.integers(0, 9, 90), k, pad, dtype)
 
 
+# pieces of 16 bytes in a row on either side of every change of lanes per row and pieces per lane
+@pytest.mark.parametrize("pieces", [4, 5, 8, 9, 12, 13, 15, 16, 17, 24, 25, 32, 33, 48, 49, 64, 65, 96, 97, 128, 129])
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+def test_pieces(pkg, handle, device, pieces, dtype):
+    rng = np.random.default_rng(pieces)
+    check(pkg, handle, device, rng, rng.integers(0, 9, 90), pieces * (4 if dtype == "f32" else 8), 0, dtype)
+
+
 @pytest.mark.parametrize("nnz", [1, 3, 4, 5, 31, 32, 33, 63, 64, 65, 129, 148 * 16 * 128 + 1])  # the last: tiles of 64 entries
 def test_entry_counts(pkg, handle, device, nnz):
     rng = np.random.default_rng(nnz)
