@@ -182,22 +182,28 @@ typedef struct b200spSpmmShape {
     int32_t kahan;      /* 1 = compensated fp32 accumulation */
     int32_t block_units; /* from b200sp_spmm_analyze_blocks: units of the column-block path, 0 = not in use */
     int32_t long_rows;  /* from b200sp_spmm_analyze_blocks: rows the analysis listed as long */
-    int64_t repack_bytes; /* bytes of the plan buffer beyond b200sp_spmm_plan_bytes that a repacked B may use
+    int64_t repack_bytes; /* bytes of the plan buffer beyond b200sp_spmm_plan_bytes that copies of the operands may use
                            * (b200sp_spmm_repack_bytes), 0 = none */
     int32_t mid_units;  /* from b200sp_spmm_analyze_units; 0 = rows of up to 1024 entries are all treated alike */
+    int32_t ascending;  /* from b200sp_spmm_columns_ascend */
 } b200spSpmmShape;
 
 /* Bytes of workspace for the SpMM analysis + long-row partial sums. */
 size_t b200sp_spmm_plan_bytes(int64_t rows, int64_t nnz, int64_t n);
 
-/* Bytes wanted after the plan for a copy of B in rows the kernels can read with 16-byte loads: 0 when B lies in
- * such rows already, or when it is read too seldom for a copy to pay.  Without them (shape.repack_bytes smaller) the
- * product runs a slower kernel that takes any layout.  Only the sizes and the layout of B are read. */
+/* Bytes wanted after the plan: for a copy of B in rows the kernels can read with 16-byte loads, unless B lies in
+ * such rows already or is read too seldom for a copy to pay, and for the rows of a dense int8 A written out for the tensor
+ * cores.  Without them (shape.repack_bytes smaller) the product runs a slower kernel.  Only sizes and layouts are read. */
 size_t b200sp_spmm_repack_bytes(const b200spSpmmShape *shape, int val_type);
 
-/* 1 if b200sp_spmm_launch with this shape (room for a copy in shape.repack_bytes) and plan copies B behind the plan.  Two
+/* 1 if b200sp_spmm_launch with this shape (room for a copy in shape.repack_bytes) and plan copies B or A behind the plan.  Its
  * launches then belong together: products that share the plan must not overlap, nor be enqueued by two threads at once. */
 int b200sp_spmm_copies(const b200spSpmmShape *shape, int val_type, int32_t segments, const void *plan);
+
+/* After b200sp_spmm_analyze_units: *ascending = 1 if this is an int8 product for the tensor cores (by its sizes) and the
+ * columns of every row of A ascend without repetition; synchronises `stream` to say so.  0, without a launch, otherwise. */
+int b200sp_spmm_columns_ascend(const int32_t *row_ptr, const int32_t *col_ind, const b200spSpmmShape *shape, int val_type,
+                               void *plan, size_t plan_bytes, int32_t *ascending, void *stream);
 
 /* Analysis pass: finds rows too long for one warp, cuts them into segments and writes
  * the segment table into `plan`, and lists the rows that are better summed apart from

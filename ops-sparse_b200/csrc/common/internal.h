@@ -61,9 +61,10 @@ struct ActivePlan {
     int32_t midUnits = 0;  // SpMM only: shorter rows summed apart from their neighbours
     int32_t blockUnits = 0;  // SpMM only: units of the column-block path for the long rows (0 = summed by segments)
     int32_t longRows = 0;   // SpMM only: rows listed as long
-    const void *colInd = nullptr;  // SpMM with column blocks: the cut table was made from these column indices
+    bool ascending = false;  // SpMM only: columns found to ascend, which an int8 product on the tensor cores wants
+    const void *colInd = nullptr;  // SpMM: the cut table of the column blocks was made, the order found, for these column indices
     int32_t valueType = -1;        // ... and for B rows of this element type
-    int64_t repackBytes = 0;       // SpMM only: bytes after the plan that a repacked B may use ...
+    int64_t repackBytes = 0;       // SpMM only: bytes after the plan that copies of B and A may use ...
     bool copyBound = false;        // ... by products on the stream of the first that did
     unsigned long long copyStream = 0;
     int32_t spmvInfo[B200SP_SPMV_PLAN_INFO_INTS] = {};  // SpMV only: plan_info written by b200sp_spmv_analyze
@@ -108,10 +109,10 @@ struct aclsparseSpMatDescr {
     // Written by *Preprocess through a const descriptor, as in the reference
     // (spmm_host.cpp:341,360): the compute call compares its buffer argument against it.
     mutable b200sp::ActivePlan active;
-    // What aclsparseSpMMGetBufferSize last said for this matrix: room for a copy of B, and for how many columns.
+    // What aclsparseSpMMGetBufferSize last said for this matrix: room for copies of B and A, and for how many columns.
     mutable int64_t spmmSizedRepack = 0;
     mutable int64_t spmmSizedN = -1;
-    mutable std::mutex copyMutex;  // held while a product that copies B into the analysed buffer is enqueued
+    mutable std::mutex copyMutex;  // held while a product that copies into the analysed buffer is enqueued
 };
 
 struct aclsparseDnVecDescr {

@@ -50,6 +50,7 @@ aclsparseStatus_t ValidateSpmm(aclsparseOperation_t opA, aclsparseOperation_t op
 struct Analysis {
     int32_t segments = 0, midUnits = 0, blockUnits = 0, longRows = 0;
     int64_t repackBytes = 0;
+    bool ascending = false;
 };
 
 size_t ElemBytes(aclDataType t)
@@ -102,7 +103,8 @@ b200spSpmmShape ShapeOf(const aclsparseSpMatDescr *A, const aclsparseDnMatDescr 
     return sh;
 }
 
-// What a buffer analysed for these operands holds after the plan: room for a copy of B in the kernels' layout.
+// What a buffer analysed for these operands holds after the plan: room for a copy of B in the kernels' layout, and for a
+// dense int8 A.
 size_t RepackBytes(const aclsparseSpMatDescr *A, const aclsparseDnMatDescr *B, const aclsparseDnMatDescr *C,
                    aclsparseOperation_t opB)
 {
@@ -114,13 +116,13 @@ bool PlanMatches(const ActivePlan &p, const void *buffer, const aclsparseSpMatDe
 {
     return p.kind == PlanKind::kSpmm && p.buffer == buffer && p.rowPtr == A->offsets && p.rows == A->rows &&
            p.nnz == A->nnz && p.n == n && p.generation == b200sp::BufferGeneration(buffer) &&
-           (p.blockUnits == 0 || (p.colInd == A->indices && p.valueType == (int32_t)A->valueType));
+           ((p.blockUnits == 0 && !p.ascending) || (p.colInd == A->indices && p.valueType == (int32_t)A->valueType));
 }
 
-// Whether this product may copy B into the analysed buffer.  Products that share a buffer may otherwise overlap (as long
+// Whether this product may copy B (or a dense int8 A) into the analysed buffer.  Products that share a buffer may otherwise overlap (as long
 // as no row exceeds 1024 entries they only read it), so the copies are kept in order: they are made on one stream,
 // that of the first product after the analysis, and not in a graph, which may be launched beside anything.  The other
-// products read B where it lies.
+// products read the operands where they lie.
 bool MayCopy(ActivePlan &p, cudaStream_t stream)
 {
     if (stream == cudaStreamPerThread) return false;  // as many streams as threads
@@ -197,10 +199,24 @@ aclsparseStatus_t aclsparseSpMMPreprocess(aclsparseHandle_t handle, aclsparseOpe
     p.longRows = found.longRows;
     p.colInd = matA->indices;
     p.valueType = (int32_t)matA->valueType;
-    // Room for a copy of B is there if GetBufferSize, too, was asked for a B that wants one.  A caller who sized the buffer
+    // Room for copies is there if GetBufferSize, too, was asked for a B that wants as much.  A caller who sized the buffer
     // with B in another layout (the rest of the size does not depend on it) has none.
     const int64_t repack = (int64_t)RepackBytes(matA, matB, matC, opB);
     p.repackBytes = matA->spmmSizedN == matC->cols && matA->spmmSizedRepack >= repack ? repack : 0;
+    if (p.repackBytes > 0) {
+        const b200spSpmmShape sh = ShapeOf(matA, matB, matC, opB);
+        int32_t ascending = 0;
+        const int rc = b200sp_spmm_columns_ascend(static_cast<const int32_t *>(matA->offsets),
+                                                  static_cast<const int32_t *>(matA->indices), &sh,
+                                                  b200sp::KernelTypeOf(matA->valueType), buffer,
+                                                  b200sp_spmm_plan_bytes(matA->rows, matA->nnz, matC->cols), &ascending,
+                                                  handle != nullptr ? handle->stream : nullptr);
+        if (rc != 0) {
+            B200SP_LOGE("aclsparseSpMMPreprocess: analysis of the columns failed (cuda error %d)", rc);
+            return ACL_SPARSE_STATUS_EXECUTION_FAILED;
+        }
+        p.ascending = ascending != 0;
+    }
     p.generation = b200sp::BufferGeneration(buffer);
     matA->active = p;
     return ACL_SPARSE_STATUS_SUCCESS;
@@ -225,6 +241,7 @@ aclsparseStatus_t aclsparseSpMM(aclsparseHandle_t handle, aclsparseOperation_t o
         found.blockUnits = matA->active.blockUnits;
         found.longRows = matA->active.longRows;
         found.repackBytes = matA->active.repackBytes;
+        found.ascending = matA->active.ascending;
     } else {
         // Not the active buffer: analyse into it now, as the reference rebuilds its tiling
         // in place (spmm_host.cpp:310-321).  This path synchronises the stream once.
@@ -246,6 +263,7 @@ aclsparseStatus_t aclsparseSpMM(aclsparseHandle_t handle, aclsparseOperation_t o
 
     b200spSpmmShape sh = ShapeOf(matA, matB, matC, opB);
     sh.repack_bytes = found.repackBytes;
+    sh.ascending = found.ascending ? 1 : 0;
     sh.mid_units = found.midUnits;
     sh.block_units = found.blockUnits;
     sh.long_rows = found.longRows;

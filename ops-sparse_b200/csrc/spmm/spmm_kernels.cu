@@ -28,9 +28,11 @@
 // 125-200): inputs widened to fp32 (int32), products accumulated in fp32 (int32),
 // C = alpha*acc + beta*C with C not read when beta == 0; fp16 output is clamped to
 // +-65504 before rounding; int32 output is computed in int64 and saturated.
+#include <atomic>
 #include <cstdint>
 #include <type_traits>
 
+#include <cuda.h>  // tensor maps: types only
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -1700,6 +1702,10 @@ __global__ void __launch_bounds__(kStreamThreads) SpmmRowStreamKernel(const Stre
     }
 }
 
+// ---------------------------------------------------------------- int8 on the tensor cores
+
+#include "int8_tensor.cuh"
+
 // ---------------------------------------------------------------- repacking B
 
 // Copies op(B) (k rows of n elements, any layout) into rows of `vecs` 16-byte pieces, zeros after element n.  One
@@ -1926,6 +1932,31 @@ bool Copies(const b200spSpmmShape *sh, int valBytes, int32_t segments, const voi
            !FewEntries(sh, valBytes, segments) && plan != nullptr && Aligned16(plan);
 }
 
+// Whether an int8 product of rows whose columns ascend is one for the tensor cores: A at least one twelfth full, and work enough for the
+// two passes over it.  Lane groups / tensor cores, us: rows of C and B in 16-byte pieces, 4096 x 4096 at 0.1, N = 512: 69 / 24; 1278 rows, 24 / 20;
+// 40,000 x 2000 at 0.15, N = 16: 116 / 73; 700 x 1500 at 0.2, N = 128: 6.1 / 12.7; 1500 x 1100 at 0.18, N = 64: 8.1 / 13.2;
+// 20,000 x 1500 at 0.07, N = 100: 34 / 47; other layouts: 2000 x 1200 at 0.21, N = 40: 31 / 16; 1500 x 2500 at 0.15, N = 200: 61 / 24;
+// 4000 x 1050 at 0.11, N = 9: 11.5 / 18.
+bool TensorPays(const b200spSpmmShape *sh)
+{
+    const bool plain = RowsContiguous(sh->op_b, sh->order_b) && sh->order_c == 0 && sh->n % 16 == 0;
+    return sh->k <= kTcMaxK && 12 * sh->nnz >= sh->m * sh->k && sh->nnz * sh->n >= (plain ? 96ll : 24ll) << 20 && (plain || sh->n >= 24);
+}
+
+// What an analysed buffer holds after the plan: a copy of B (from a multiple of 256 bytes) and an A written out.
+size_t ExtraBytes(const b200spSpmmShape *sh, int valBytes)
+{
+    const size_t repack = WorthRepacking(sh, valBytes) ? RepackBytes(sh, valBytes) : 0;
+    if (valBytes != 1 || !TensorPays(sh)) return repack;
+    return AlignUp(repack, 256) + DenseBytes(sh->m, sh->k);
+}
+
+// Whether an int8 product with this much room, on rows found to ascend, writes A out.
+bool OnTensorCores(const b200spSpmmShape *sh, const void *plan)
+{
+    return sh->ascending != 0 && TensorPays(sh) && sh->repack_bytes >= (int64_t)ExtraBytes(sh, 1) && plan != nullptr && Aligned16(plan);
+}
+
 template <typename ValT, typename OutT>
 int LaunchGeneric(const int32_t *rowPtr, const int32_t *colInd, const void *val, const void *B, void *C,
                   const b200spSpmmShape *sh, const b200spScalars *s, cudaStream_t stream)
@@ -1946,6 +1977,93 @@ int LaunchGeneric(const int32_t *rowPtr, const int32_t *colInd, const void *val,
                                   static_cast<const ValT *>(val), static_cast<const ValT *>(B), static_cast<OutT *>(C), g, sc);
     b200sp_note_launches(1);
     return (int)e;
+}
+
+// A matrix of bytes, `rows` rows of `cols` with `stride` bytes between them, in tiles of 128 rows by 128, 64 or 32 columns, swizzled
+// over their whole width.
+using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                 const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+bool ByteTiles(EncodeTiled encode, const void *at, long long rows, long long cols, long long stride, int tileCols, CUtensorMap *map)
+{
+    const cuuint64_t size[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)stride};
+    const cuuint32_t box[2] = {(cuuint32_t)tileCols, 128}, step[2] = {1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(at), size, strides, box, step,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  tileCols == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : tileCols == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// dense: DenseBytes(m, k), 16-byte aligned
+int LaunchInt8Tensor(const FastArgs<int8_t, int32_t> &f, const b200spSpmmShape *sh, unsigned char *dense, cudaStream_t stream)
+{
+    static const EncodeTiled encode = [] {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found{};
+        const cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found);
+        return e == cudaSuccess && found == cudaDriverEntryPointSuccess ? reinterpret_cast<EncodeTiled>(fn) : nullptr;
+    }();
+    static std::atomic<bool> allowed[64] = {};  // per device: the kernel may use kTcSmem bytes of shared memory
+    int dev = 0;
+    if (encode == nullptr) return (int)cudaErrorNotSupported;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
+    if (!allowed[dev].load(std::memory_order_relaxed)) {
+        const cudaError_t e = cudaFuncSetAttribute(SpmmInt8TensorKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
+        if (e != cudaSuccess) return (int)e;
+        allowed[dev].store(true, std::memory_order_relaxed);
+    }
+    const long long denseCols = DenseCols(sh->k);
+    TcArgs t{};
+    t.dense = dense;
+    t.odd = dense + AlignUp((size_t)sh->m * (size_t)denseCols, 256);
+    t.rowPtr = f.rowPtr;
+    t.colInd = f.colInd;
+    t.val = f.val;
+    t.B = f.B;
+    t.C = f.C;
+    t.m = f.m;
+    t.n = f.n;
+    t.chunks = (int)(denseCols / kTcDepth);
+    t.ldb = f.ldb;
+    t.cRow = f.cRow;
+    t.cCol = f.cCol;
+    t.cVectors = f.cCol == 1 && f.cRow % 4 == 0 && Aligned16(f.C);
+    t.sc = f.sc;
+    t.waitCycles = gHostStreamWaitCycles;
+    t.extraTx = gHostStreamExtraTx;
+    const long long rowTiles = (sh->m + kTcRows - 1) / kTcRows;
+    // Narrower tiles where the widest leave half of the SMs without work.  Clusters of eight find their SMs free only where they are few:
+    // 10 of them 19.7 us against 23.8 with 4 CTAs each, 16 of them 27.9 against 18.1.
+    const int cluster = rowTiles <= 12 ? 2 * kTcCluster : kTcCluster;
+    t.cols = kTcCols;
+    while (t.cols > 32 && (2 * sh->n <= t.cols || (2 * sh->n <= cluster * t.cols &&
+                                                   2 * rowTiles * ((sh->n + t.cols - 1) / t.cols) <= b200sp_sm_count())))
+        t.cols /= 2;
+    CUtensorMap mapA, mapB;
+    if (!ByteTiles(encode, dense, sh->m, denseCols, denseCols, kTcDepth, &mapA) ||
+        !ByteTiles(encode, f.B, sh->k, f.nB, f.ldb, t.cols, &mapB))
+        return (int)cudaErrorInvalidValue;
+    for (; t.firstCol < t.n; t.firstCol += cluster * t.cols) {  // a launch for every 512 or 1024 columns
+        const int left = t.n - t.firstCol;
+        t.colTiles = left < cluster * t.cols ? (left + t.cols - 1) / t.cols : cluster;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)(rowTiles * t.colTiles));
+        cfg.blockDim = dim3(kTcThreads);
+        cfg.dynamicSmemBytes = kTcSmem;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2] = {};
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = (unsigned)t.colTiles;
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        b200sp_note_launches(1);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, SpmmInt8TensorKernel, t, mapA, mapB);
+        if (e != cudaSuccess) return (int)e;
+    }
+    return 0;
 }
 
 template <typename ValT, typename OutT>
@@ -2063,6 +2181,9 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
         return err;
     };
     if constexpr (kInt8) {
+        if (OnTensorCores(sh, plan))
+            return LaunchInt8Tensor(a, sh, reinterpret_cast<unsigned char *>(p + L.total + ExtraBytes(sh, 1) - DenseBytes(sh->m, sh->k)),
+                                    stream);
         if (lanes_ <= 4) {  // 16 to 64 entries of a row are in flight as it is
             a.rowLimit = kLongRow;
             midUnits = 0;
@@ -2172,12 +2293,34 @@ size_t b200sp_spmm_plan_bytes(int64_t rows, int64_t nnz, int64_t n) { return Lay
 size_t b200sp_spmm_repack_bytes(const b200spSpmmShape *shape, int val_type)
 {
     const int bytes = val_type == B200SP_F32 ? 4 : val_type == B200SP_I8 ? 1 : 2;
-    return WorthRepacking(shape, bytes) ? RepackBytes(shape, bytes) : 0;
+    return ExtraBytes(shape, bytes);
 }
 
 int b200sp_spmm_copies(const b200spSpmmShape *shape, int val_type, int32_t segments, const void *plan)
 {
-    return Copies(shape, val_type == B200SP_F32 ? 4 : val_type == B200SP_I8 ? 1 : 2, segments, plan) ? 1 : 0;
+    const int bytes = val_type == B200SP_F32 ? 4 : val_type == B200SP_I8 ? 1 : 2;
+    return Copies(shape, bytes, segments, plan) || (bytes == 1 && OnTensorCores(shape, plan)) ? 1 : 0;
+}
+
+int b200sp_spmm_columns_ascend(const int32_t *row_ptr, const int32_t *col_ind, const b200spSpmmShape *shape, int val_type,
+                               void *plan, size_t plan_bytes, int32_t *ascending, void *stream)
+{
+    *ascending = 0;
+    if (val_type != B200SP_I8 || !TensorPays(shape) || col_ind == nullptr) return 0;
+    const PlanLayout L = LayoutFor(shape->m, shape->nnz, shape->n);
+    if (plan == nullptr || plan_bytes < L.total) return (int)cudaErrorInvalidValue;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    int32_t *flag = reinterpret_cast<int32_t *>(static_cast<char *>(plan) + L.offCounts) + 6;  // zero since the analysis of the rows
+    const long long want = (shape->m + 7) / 8, cap = (long long)b200sp_sm_count() * 8;
+    SpmmAscendingKernel<<<(unsigned)(want < cap ? want : cap), 256, 0, st>>>(row_ptr, col_ind, (int)shape->m, flag);
+    b200sp_note_launches(1);
+    int32_t bad = 1;
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, flag, sizeof(bad), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return (int)e;
+    *ascending = bad == 0;
+    return 0;
 }
 
 int b200sp_spmm_analyze(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,

@@ -1,0 +1,112 @@
+"""GPU: int8 SpMM on the tensor cores, at the edges of its tiles, clusters and launches, and on rows it may not write out."""
+from __future__ import annotations
+
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def pattern(rng, m, k, entries):
+    """Ascending columns; rows of about `entries` among empty and full ones."""
+    lengths = np.where(rng.random(m) < 0.05, rng.choice([0, 1, k], m), np.minimum(entries + rng.integers(-5, 6, m), k))
+    rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    ci = np.concatenate([np.sort(rng.permutation(k)[:n]) for n in lengths]).astype(np.int32)
+    return rp, ci, rng.integers(-128, 128, ci.size).astype(np.int8)
+
+
+class Product:
+    def __init__(self, pkg, handle, device, rng, m, k, n, entries, order, align=0):
+        from ops_sparse_b200 import api
+        self.handle, self.shape, self.order = handle, (m, k, n), order
+        self.rp, self.ci, self.val = pattern(rng, m, k, entries)
+        self.B = rng.integers(-128, 128, (k, n)).astype(np.int8)
+        self.C = rng.integers(-1000, 1000, (m, n)).astype(np.int32)
+        dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(device)
+        stored = (lambda a: a) if order == "row" else (lambda a: a.T)
+        self.A = api.CsrMatrix(dev(self.rp), dev(self.ci), dev(self.val), m, k)
+        self.dB = api.DnMat(dev(stored(self.B)), k, n, n if order == "row" else k, order)
+        self.dC = api.DnMat(dev(stored(self.C)), m, n, n if order == "row" else m, order)
+        size = api.spmm_buffer_size(handle, self.A, self.dB, self.dC)
+        assert size >= m * k  # room for A as it is written out
+        self.buffer = torch.empty(size + 256, dtype=torch.uint8, device=device)[align:]
+        pkg.check(pkg.lib().aclsparseSpMMPreprocess(handle.raw, 0, 0, None, self.A.raw, self.dB.raw, None, self.dC.raw, pkg.ACL_INT32, 0,
+                                                    ctypes.c_void_p(self.buffer.data_ptr())), "aclsparseSpMMPreprocess")
+
+    def run(self, alpha, beta, handle=None):
+        from ops_sparse_b200 import api
+        api.spmm(handle or self.handle, self.A, self.dB, self.dC, alpha, beta, buffer=self.buffer)
+        torch.cuda.synchronize()
+        m, k, n = self.shape
+        got = self.dC.values.cpu().numpy()
+        return got.reshape(m, n) if self.order == "row" else got.reshape(n, m).T
+
+    def want(self, alpha, beta, ci=None):
+        import scipy.sparse
+        m, k, n = self.shape
+        A = scipy.sparse.csr_matrix((self.val.astype(np.int64), self.ci if ci is None else ci, self.rp), shape=(m, k))
+        exact = alpha * (A @ self.B.astype(np.int64)) + beta * self.C.astype(np.int64)
+        return np.clip(exact, -2 ** 31, 2 ** 31 - 1).astype(np.int32)
+
+
+# columns of A on either side of a step and the most a row may have; one to eight column tiles of 32, 64 and 128, several launches;
+# last rows and columns of a tile
+@pytest.mark.parametrize("m,k,n,entries,order", [
+    (4100, 128, 130, 60, "row"), (4097, 129, 132, 60, "col"), (1000, 257, 300, 120, "col"), (220, 12288, 112, 1200, "col"),
+    (2000, 512, 256, 256, "row"), (5000, 700, 64, 350, "row"), (20000, 320, 32, 180, "row"), (1700, 400, 1100, 100, "col"),
+    (1500, 200, 1030, 100, "row"), (1280, 1000, 512, 200, "row"), (2049, 900, 24, 700, "col"), (257, 3000, 136, 1000, "col"),
+])
+@pytest.mark.parametrize("alpha,beta", [(1, 0), (70000, -3)])
+def test_edges(pkg, handle, device, m, k, n, entries, order, alpha, beta):
+    p = Product(pkg, handle, device, np.random.default_rng(m + k + n), m, k, n, entries, order)
+    assert np.array_equal(p.run(alpha, beta), p.want(alpha, beta))
+
+
+def test_rows_that_ascend_no_longer(pkg, handle, device):
+    """Columns written over in place after the analysis: repeated and unordered ones are summed entry by entry."""
+    p = Product(pkg, handle, device, np.random.default_rng(5), 1500, 600, 150, 270, "col")
+    ci = p.ci.copy()
+    for i, r in enumerate((0, 3, 127, 128, 700, 1499)):
+        row = ci[p.rp[r]:p.rp[r + 1]]
+        if i % 2 and row.size > 257:
+            row[255] = row[256]  # across two requests
+        else:
+            row[:] = row[::-1]
+    p.A.col_ind.copy_(torch.from_numpy(ci))
+    assert np.array_equal(p.run(2, -1), p.want(2, -1, ci))
+
+
+@pytest.mark.parametrize("align", [4, 8])
+def test_buffer_on_any_word(pkg, handle, device, align):
+    p = Product(pkg, handle, device, np.random.default_rng(6), 1500, 600, 150, 270, "col", align)
+    assert np.array_equal(p.run(2, -1), p.want(2, -1))
+
+
+def test_second_stream(pkg, handle, device):
+    """The first product's stream may write A into the shared buffer, a product on another reads it as it lies."""
+    from ops_sparse_b200 import api
+    p = Product(pkg, handle, device, np.random.default_rng(8), 1500, 600, 150, 270, "col")
+    assert np.array_equal(p.run(1, 0), p.want(1, 0))
+    other = api.Handle(torch.cuda.Stream())
+    assert np.array_equal(p.run(3, 0, other), p.want(3, 0))
+    other.close()
+
+
+def test_wait_that_runs_out(pkg, handle, device):
+    """As in the row-stream kernel's test: a few bytes more expected than are copied, two milliseconds to wait for them."""
+    L = pkg.lib()
+    L.b200sp_spmm_stream_wait_test.argtypes = [ctypes.c_longlong, ctypes.c_uint]
+    L.b200sp_spmm_stream_wait_test.restype = None
+    p = Product(pkg, handle, device, np.random.default_rng(9), 1500, 600, 150, 270, "col")
+    assert L.b200sp_spmm_stream_error() == 0
+    try:
+        L.b200sp_spmm_stream_wait_test(1 << 22, 16)
+        assert np.array_equal(p.run(1, 0), p.C)  # nothing written
+        assert L.b200sp_spmm_stream_error() == 1
+    finally:
+        L.b200sp_spmm_stream_wait_test(0, 0)
+    assert L.b200sp_spmm_stream_error_clear() == 0
+    assert np.array_equal(p.run(1, 0), p.want(1, 0))
