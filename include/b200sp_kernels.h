@@ -186,6 +186,7 @@ typedef struct b200spSpmmShape {
                            * (b200sp_spmm_repack_bytes), 0 = none */
     int32_t mid_units;  /* from b200sp_spmm_analyze_units; 0 = rows of up to 1024 entries are all treated alike */
     int32_t ascending;  /* from b200sp_spmm_columns_ascend */
+    int64_t longest_row; /* from b200sp_spmm_analyze_units: entries of the longest row that is neither cut nor listed */
 } b200spSpmmShape;
 
 /* Bytes of workspace for the SpMM analysis + long-row partial sums. */
@@ -208,9 +209,10 @@ int b200sp_spmm_columns_ascend(const int32_t *row_ptr, const int32_t *col_ind, c
 /* Analysis pass: finds rows too long for one warp, cuts them into segments and writes
  * the segment table into `plan`, and lists the rows that are better summed apart from
  * their neighbours.  This call synchronises `stream` once to read back the two counts,
- * returned in *segments and *mid_units. */
+ * returned in *segments and *mid_units, and the entries of the longest other row. */
 int b200sp_spmm_analyze_units(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,
-                              size_t plan_bytes, int32_t *segments, int32_t *mid_units, void *stream);
+                              size_t plan_bytes, int32_t *segments, int32_t *mid_units, int32_t *longest_row,
+                              void *stream);
 /* The same without the second count. */
 int b200sp_spmm_analyze(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,
                         size_t plan_bytes, int32_t *segments, void *stream);

@@ -49,6 +49,7 @@ aclsparseStatus_t ValidateSpmm(aclsparseOperation_t opA, aclsparseOperation_t op
 
 struct Analysis {
     int32_t segments = 0, midUnits = 0, blockUnits = 0, longRows = 0;
+    int32_t longestRow = 0;
     int64_t repackBytes = 0;
     bool ascending = false;
 };
@@ -69,7 +70,7 @@ aclsparseStatus_t Analyse(const aclsparseSpMatDescr *A, int64_t n, void *buffer,
     // Whatever plan this buffer held is overwritten now; an active plan that is not re-recorded below goes stale.
     (void)b200sp::NoteBufferWrite(buffer);
     const int rc = b200sp_spmm_analyze_units(static_cast<const int32_t *>(A->offsets), A->rows, A->nnz, n, buffer, bytes,
-                                             segments, &out->midUnits, stream);
+                                             segments, &out->midUnits, &out->longestRow, stream);
     if (rc != 0) {
         B200SP_LOGE("aclsparseSpMM: analysis failed (cuda error %d)", rc);
         return ACL_SPARSE_STATUS_EXECUTION_FAILED;
@@ -195,6 +196,7 @@ aclsparseStatus_t aclsparseSpMMPreprocess(aclsparseHandle_t handle, aclsparseOpe
     p.n = matC->cols;
     p.segments = found.segments;
     p.midUnits = found.midUnits;
+    p.longestRow = found.longestRow;
     p.blockUnits = found.blockUnits;
     p.longRows = found.longRows;
     p.colInd = matA->indices;
@@ -238,6 +240,7 @@ aclsparseStatus_t aclsparseSpMM(aclsparseHandle_t handle, aclsparseOperation_t o
     if (PlanMatches(matA->active, buffer, matA, matC->cols)) {
         found.segments = matA->active.segments;
         found.midUnits = matA->active.midUnits;
+        found.longestRow = matA->active.longestRow;
         found.blockUnits = matA->active.blockUnits;
         found.longRows = matA->active.longRows;
         found.repackBytes = matA->active.repackBytes;
@@ -265,6 +268,7 @@ aclsparseStatus_t aclsparseSpMM(aclsparseHandle_t handle, aclsparseOperation_t o
     sh.repack_bytes = found.repackBytes;
     sh.ascending = found.ascending ? 1 : 0;
     sh.mid_units = found.midUnits;
+    sh.longest_row = found.longestRow;
     sh.block_units = found.blockUnits;
     sh.long_rows = found.longRows;
     sh.kahan = (alg == ACL_SPARSE_SPMM_CSR_FP32_HIGH_PRECISION_ALG && matA->valueType == ACL_FLOAT) ? 1 : 0;

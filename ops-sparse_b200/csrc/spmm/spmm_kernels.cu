@@ -279,10 +279,14 @@ __device__ __forceinline__ OutT Finish(int32_t acc, int32_t alpha, int32_t beta,
 __global__ void SpmmFindLongRowsKernel(const int32_t *__restrict__ rowPtr, int rows, int limit, int arrivals, int capSegs, int32_t *counts,
                                        LongRow *longRows, SegEntry *segs, int32_t *counters)
 {
+    int longest = 0;  // of the ordinary rows
     for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < rows;
          r += (long long)gridDim.x * blockDim.x) {
         const int len = rowPtr[r + 1] - rowPtr[r];
-        if (len <= limit) continue;
+        if (len <= limit) {
+            longest = len > longest ? len : longest;
+            continue;
+        }
         if (len <= kLongRow) {
             segs[capSegs - 1 - atomicAdd(&counts[5], 1)] = {(int32_t)r, 0, -1, 0};
             continue;
@@ -295,6 +299,9 @@ __global__ void SpmmFindLongRowsKernel(const int32_t *__restrict__ rowPtr, int r
         for (int s = 0; s < arrivals; ++s) counters[(long long)li * arrivals + s] = 0;
         for (int s = 0; s < nseg; ++s) segs[sb + s] = {(int32_t)r, s, li, 0};
     }
+    __syncwarp();
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if ((threadIdx.x & 31) == 0 && longest > 0) atomicMax(&counts[7], longest);
 }
 
 // A warp per long row: checks that its columns ascend, finds where it crosses the boundaries of the column
@@ -450,6 +457,8 @@ struct FastArgs {
     int slices;           // fp: warps a unit takes, 64 bytes of a B row each
     int splitRows;        // int8 only: a CTA per row
     int genRows;          // column-major C: rows of a CTA
+    int ctaRows;          // other C: rows of a CTA
+    int byLength;         // the 32 rows of a CTA are taken in order of their lengths
     const LongRow *longRows;
     const SegEntry *segs, *segsEnd;
     int32_t *counters;    // [long row][ArrivalsPerRow]
@@ -513,18 +522,46 @@ __device__ __forceinline__ void RowDot(const int32_t *__restrict__ colInd, const
     constexpr int kChunk = Chunk<kLanes>::kChunk;
     constexpr int kBatch = kChunk < B200SP_SPMM_BATCH ? kChunk : B200SP_SPMM_BATCH;  // B rows in flight per lane
     const int li = threadIdx.x & (kLanes - 1);
+    [[maybe_unused]] int nextCol[kHold];
+    [[maybe_unused]] ValT nextVal[kHold];
+    [[maybe_unused]] auto request = [&](int p0) {
+#pragma unroll
+        for (int h = 0; h < kHold; ++h) {
+            nextCol[h] = 0;
+            nextVal[h] = FromF32<ValT>(0.0f);
+            if (p0 + h * kLanes + li < e) {
+                nextCol[h] = __ldcs(colInd + p0 + h * kLanes + li);
+                nextVal[h] = __ldcs(val + p0 + h * kLanes + li);
+            }
+        }
+    };
+    // The entries of the next chunk are asked for before this one's rows of B.  us without and with, f32 and f16 of N = 64 in rows of 20 to 64: 264.5
+    // and 259.6, 72.5 and 70.4; f32, N = 32: 39.9 and 38.4.  Other widths pay for the registers: f16, N = 8: 53 and 70; bf16, N = 128: 127 and 133.
+    // f16 and bf16, N = 32: 52.3 and 54.0, 87.5 and 90.7.
+    constexpr bool kEarly = kLanes == 8 || ((kLanes == 4 || kLanes == 16) && sizeof(ValT) == 4);
+    if constexpr (kEarly)
+        if (trips > 0) request(s);
     for (int chunk = 0; chunk < trips; ++chunk) {
         const int p0 = s + chunk * kChunk;
         const int rem = e - p0;  // entries of this group's row left; <= 0 once the row is done
         int myCol[kHold];
         float myVal[kHold];
+        if constexpr (kEarly) {
 #pragma unroll
-        for (int h = 0; h < kHold; ++h) {
-            myCol[h] = 0;
-            myVal[h] = 0.0f;
-            if (h * kLanes + li < rem) {
-                myCol[h] = __ldcs(colInd + p0 + h * kLanes + li);
-                myVal[h] = ToF32(__ldcs(val + p0 + h * kLanes + li));
+            for (int h = 0; h < kHold; ++h) {
+                myCol[h] = nextCol[h];
+                myVal[h] = ToF32(nextVal[h]);
+            }
+            if (chunk + 1 < trips) request(p0 + kChunk);
+        } else {
+#pragma unroll
+            for (int h = 0; h < kHold; ++h) {
+                myCol[h] = 0;
+                myVal[h] = 0.0f;
+                if (h * kLanes + li < rem) {
+                    myCol[h] = __ldcs(colInd + p0 + h * kLanes + li);
+                    myVal[h] = ToF32(__ldcs(val + p0 + h * kLanes + li));
+                }
             }
         }
         // Whole warp on full chunks: straight-line code, no predicate per entry.
@@ -930,6 +967,8 @@ template <typename ValT, int kLanes> struct FastShape {
     static constexpr int kCtaRows = kWarps * (32 / kGroup);                   // rows of A per pass of the CTA
     static constexpr int kFit = 8192 / kTileCols < 32 ? 8192 / kTileCols : 32;  // at most 32 KB of tile
     static constexpr int kGenRows = kCtaRows > kFit ? kCtaRows : kFit;
+    // 32 rows of a CTA may be taken in order of their lengths (int8 loses: 44.6 and 50.3 us on 55,686 rows of 0 to 232 entries, N = 16).
+    static constexpr bool kOrdered = !std::is_same_v<ValT, int8_t> && kCtaRows <= 32 && kGroup < 32;
 };
 
 enum { kPlain, kAnyC, kAnyCWords };
@@ -952,6 +991,8 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
     constexpr int kTileWords = kGenC ? (Shape::kGenRows * kTileStride > kThreads * E ? Shape::kGenRows * kTileStride : kThreads * E) : 0;
     __shared__ __align__(16) Acc sBuf[kWarps * kWarpWords > kTileWords ? kWarps * kWarpWords : kTileWords];
     __shared__ unsigned char sSkip[kGenC ? Shape::kGenRows : 1];
+    constexpr bool kOrdered = Shape::kOrdered;
+    __shared__ unsigned char sOrder[kOrdered ? kWarps : 1][32];
     __shared__ int sLast;
 
     b200sp::WaitForPrevious();
@@ -984,12 +1025,29 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
         // ---- one lane group per row ----
         constexpr int kChunk = kInt8 ? Group8<kLanes>::kChunk : Chunk<kLanes>::kChunk;
         const bool rowsRun = kGenC && a.cCol != 1;  // column-major C
-        const int blockRows = rowsRun ? a.genRows : Shape::kCtaRows;
+        const int blockRows = rowsRun ? a.genRows : a.ctaRows;
         const long long row0 = (long long)(blockIdx.x - a.unitCtas) * blockRows;
+        if constexpr (kOrdered) {
+            if (a.byLength) {  // sOrder[i]: the row with the i-th most entries (every warp has its own copy: no barrier)
+                int len = row0 + lane < a.m ? a.rowPtr[row0 + lane + 1] - a.rowPtr[row0 + lane] : 0;
+                if (len > a.rowLimit) len = 0;
+                const int key = len << 5 | (31 - lane);
+                int rank = 0;
+#pragma unroll
+                for (int j = 1; j < 32; ++j) rank += __shfl_xor_sync(0xffffffffu, key, j) > key;
+                sOrder[warp][rank] = (unsigned char)lane;
+                __syncwarp();
+            }
+        }
         for (int col0 = 0; col0 < (rowsRun ? a.n : 1); col0 += kTileCols) {  // column-major C: a tile of columns at a time
 #pragma unroll 1
             for (int pass = 0; pass < blockRows; pass += Shape::kCtaRows) {
-                const int rowIn = pass + warp * kRowsPerWarp + lane / kGroup;
+                int rowIn = pass + warp * kRowsPerWarp + lane / kGroup;
+                if constexpr (kOrdered) {
+                    // every other pass the other way round: the warp with the longest rows of one has the shortest of the next
+                    const int turn = pass & Shape::kCtaRows ? kWarps - 1 - warp : warp;
+                    if (a.byLength) rowIn = sOrder[warp][pass + turn * kRowsPerWarp + lane / kGroup];
+                }
                 const long long row = row0 + rowIn;
                 int s = 0, e = 0;
                 bool skip = row >= a.m;
@@ -1057,7 +1115,8 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
 #pragma unroll
                             for (int i = lane; i < kRowsPerWarp * kTileCols; i += 32) {
                                 const int g = i / kTileCols, c = colT + i % kTileCols;
-                                if (c < a.n && !(skipped >> (g * kGroup) & 1)) storeOne(row0 + warp * kRowsPerWarp + g, c, sWarp[i]);
+                                const int r = kOrdered ? __shfl_sync(0xffffffffu, rowIn, g * kGroup) : warp * kRowsPerWarp + g;
+                                if (c < a.n && !(skipped >> (g * kGroup) & 1)) storeOne(row0 + r, c, sWarp[i]);
                             }
                         }
                     } else {
@@ -2152,7 +2211,15 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             const long long unitCtas = kInt8 ? units : ((long long)units * a.slices + kWarps - 1) / kWarps;
             a.unitCtas = (int)unitCtas;
             a.genRows = sh->m < 2ll * Shape::kGenRows * b200sp_sm_count() ? Shape::kCtaRows : Shape::kGenRows;
-            const long long rows = a.splitRows ? 1 : sh->order_c == 0 ? Shape::kCtaRows : a.genRows;
+            // The rows that a warp takes together wait for the longest of them: a CTA takes 32 rows in order of their lengths where
+            // that leaves every SM four CTAs.  Rows of 0 to twice the mean, us in their own order and so: f16, N = 64: 98.8 and 72.5; f32, N = 32: 49.4
+            // and 39.9; bf16, N = 128: 163 and 127; f16, N = 37: 65 and 51; columns of C, N = 40: 53 and 41; power-law rows, bf16,
+            // N = 64: 186 and 175.  Not where the longest has less than a quarter more entries than the mean: rows of 30, bf16, N = 128,
+            // take 102 us eight to a CTA and 108 with 32, which makes for a longer last wave.
+            const bool uneven = Shape::kOrdered && 4 * sh->longest_row * sh->m >= 5 * sh->nnz;
+            a.ctaRows = uneven && sh->m >= 4 * 32ll * b200sp_sm_count() ? 32 : Shape::kCtaRows;
+            a.byLength = uneven && (sh->order_c == 0 ? a.ctaRows : a.genRows) == 32;
+            const long long rows = a.splitRows ? 1 : sh->order_c == 0 ? a.ctaRows : a.genRows;
             const long long grid = unitCtas + (rowCtas ? (sh->m + rows - 1) / rows : 0);
             if (grid == 0) return;
             auto go = [&](auto kernel) { err = b200sp::LaunchChained(kernel, (unsigned)grid, kThreads, 0, st, a); };
@@ -2326,12 +2393,13 @@ int b200sp_spmm_columns_ascend(const int32_t *row_ptr, const int32_t *col_ind, c
 int b200sp_spmm_analyze(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,
                         size_t plan_bytes, int32_t *segments, void *stream)
 {
-    int32_t mid = 0;
-    return b200sp_spmm_analyze_units(row_ptr, rows, nnz, n, plan, plan_bytes, segments, &mid, stream);
+    int32_t mid = 0, longest = 0;
+    return b200sp_spmm_analyze_units(row_ptr, rows, nnz, n, plan, plan_bytes, segments, &mid, &longest, stream);
 }
 
 int b200sp_spmm_analyze_units(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,
-                              size_t plan_bytes, int32_t *segments, int32_t *mid_units, void *stream)
+                              size_t plan_bytes, int32_t *segments, int32_t *mid_units, int32_t *longest_row,
+                              void *stream)
 {
     const PlanLayout L = LayoutFor(rows, nnz, n);
     if (plan == nullptr || segments == nullptr || plan_bytes < L.total) return (int)cudaErrorInvalidValue;
@@ -2351,13 +2419,14 @@ int b200sp_spmm_analyze_units(const int32_t *row_ptr, int64_t rows, int64_t nnz,
         e = cudaGetLastError();
         if (e != cudaSuccess) return (int)e;
     }
-    int32_t counts[6] = {};
+    int32_t counts[8] = {};
     e = cudaMemcpyAsync(counts, p + L.offCounts, sizeof(counts), cudaMemcpyDeviceToHost, st);
     if (e != cudaSuccess) return (int)e;
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return (int)e;
     *segments = counts[1];
     *mid_units = counts[5];
+    *longest_row = counts[7];
     return 0;
 }
 

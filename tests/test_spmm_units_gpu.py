@@ -110,3 +110,25 @@ def test_rows_of_a_few_entries(handle, device, oracle, m, k, entries, vt, ot, or
         else:
             gold = oracle.spmm_16(rp, ci, val, B, C, alpha, beta, vt, ot)
         assert np.array_equal(got.view(np.uint8), np.asarray(gold).reshape(m, n).view(np.uint8))
+
+
+@pytest.mark.parametrize("order", ["row", "col"])
+@pytest.mark.parametrize("vt,ot,n", [("f32", "f32", 16), ("f16", "f16", 37), ("bf16", "f32", 64), ("f32", "f32", 64), ("bf16", "bf16", 120)])
+def test_rows_in_order_of_their_lengths(handle, device, oracle, vt, ot, n, order):
+    """Rows enough for CTAs of 32 that take them by length (4 to 16 lanes a row): the golden's bits, ties and empty rows among them."""
+    rng = np.random.default_rng(n)
+    m, k = 4 * 32 * 148 + 13, 3000
+    lengths = rng.integers(0, 12, m)
+    lengths[64:128] = 7                      # CTAs of equal rows
+    lengths[rng.integers(0, m, 200)] = 100   # rows summed apart
+    rp, ci, val, B, C = compact_case(oracle, rng, m, k, n, lengths, vt, ot, 1.5, -0.5)
+    stored = (lambda a: a) if order == "row" else (lambda a: np.ascontiguousarray(a.T))
+    ldb, ldc = (n, n) if order == "row" else (k, m)
+    got = run_spmm(handle, device, rp, ci, val, vt, stored(B), stored(C), ot, m, k, n, ldb, ldc, 1.5, -0.5,
+                   b_order=order, c_order=order)
+    got = got.reshape(m, n) if order == "row" else np.ascontiguousarray(got.reshape(n, m).T)
+    if vt == "f32":
+        gold = oracle.spmm_f32_layout(m, n, rp, ci, val, B, n, True, False, C, n, True, 1.5, -0.5)
+    else:
+        gold = oracle.spmm_16(rp, ci, val, B, C, 1.5, -0.5, vt, ot)
+    assert np.array_equal(got.view(np.uint8), np.asarray(gold).reshape(m, n).view(np.uint8))
