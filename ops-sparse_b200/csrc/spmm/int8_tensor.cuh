@@ -42,8 +42,9 @@ __global__ void __launch_bounds__(256) SpmmAscendingKernel(const int32_t *__rest
     const int lane = threadIdx.x & 31;
     bool bad = false;
     for (long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * 8) {
-        const int e = rowPtr[r + 1];
-        for (int p = rowPtr[r] + lane; p + 1 < e; p += 32) bad |= colInd[p] >= colInd[p + 1];
+        const int s = rowPtr[r], len = rowPtr[r + 1] - s;
+        // unsigned, from the row's start: a row may end at the last entry that 31 bits count
+        for (unsigned i = lane; i + 1 < (unsigned)len; i += 32) bad |= colInd[s + i] >= colInd[s + i + 1];
     }
     if (__any_sync(0xffffffffu, bad) && lane == 0) atomicExch(notAscending, 1);
 }
@@ -112,16 +113,17 @@ constexpr int kTcWindows = 8;
 struct TcEntries {
     uint32_t col[kTcWindows];
     int8_t val[kTcWindows];
-    __device__ __forceinline__ void Request(const TcArgs &a, int from, int end, int lane)
+    // len: entries from `from` on.  Lengths are compared, not positions: from + 32 * h + lane may not fit 31 bits.
+    __device__ __forceinline__ void Request(const TcArgs &a, int from, int len, int lane)
     {
 #pragma unroll
         for (int h = 0; h < kTcWindows; ++h) {
-            const int p = from + 32 * h + lane;
-            col[h] = 0x80000000u + 32 * h + lane;  // past the end: ascending too, and in no row
+            const int i = 32 * h + lane;
+            col[h] = 0x80000000u + i;  // past the end: ascending too, and in no row
             val[h] = 0;
-            if (p < end) {
-                col[h] = (uint32_t)__ldg(a.colInd + p);
-                val[h] = __ldg(a.val + p);
+            if (i < len) {
+                col[h] = (uint32_t)__ldg(a.colInd + from + i);
+                val[h] = __ldg(a.val + from + i);
             }
         }
     }
@@ -141,7 +143,7 @@ struct TcEntries {
 };
 
 // Row `row` of A as bytes, through a row of zeros in shared memory; its first entries are in hand.
-__device__ __forceinline__ void TcExpandRow(const TcArgs &a, int row, int from, int end, const TcEntries &first, unsigned char *sRow,
+__device__ __forceinline__ void TcExpandRow(const TcArgs &a, int row, int from, int len, const TcEntries &first, unsigned char *sRow,
                                             int lane)
 {
     const int width = a.chunks * kTcDepth;
@@ -150,9 +152,9 @@ __device__ __forceinline__ void TcExpandRow(const TcArgs &a, int row, int from, 
     __syncwarp();
     uint32_t least = 0;
     bool bad = first.Write(sRow, width, least, lane);
-    for (int p0 = from + 32 * kTcWindows; p0 < end; p0 += 32 * kTcWindows) {
+    for (int left = len - 32 * kTcWindows; left > 0; left -= 32 * kTcWindows) {
         TcEntries more;
-        more.Request(a, p0, end, lane);
+        more.Request(a, from + (len - left), left, lane);
         bad |= more.Write(sRow, width, least, lane);
     }
     bad = __any_sync(0xffffffffu, bad);
@@ -184,21 +186,21 @@ __global__ void __launch_bounds__(kTcThreads, 1) SpmmInt8TensorKernel(const TcAr
     const int rank = blockIdx.x % a.colTiles;
     const int row0 = (int)(blockIdx.x / a.colTiles) * kTcRows;
     const int n0 = a.firstCol + rank * a.cols;
-    {  // lane t has the ends of the warp's t-th row; two rows at a time
+    {  // lane t has the start and the length of the warp's t-th row; two rows at a time
         unsigned char *const sRow = tiles + warp * a.chunks * kTcDepth;
         const int first = rank * kTcWarps + warp, step = a.colTiles * kTcWarps;  // rows of the tile: first, first + step, ...
         const int own = row0 + first + lane * step;
         const bool some = first + lane * step < kTcRows && own < a.m;
-        const int ownFrom = some ? __ldg(a.rowPtr + own) : 0, ownEnd = some ? __ldg(a.rowPtr + own + 1) : 0;
+        const int ownFrom = some ? __ldg(a.rowPtr + own) : 0, ownLen = some ? __ldg(a.rowPtr + own + 1) - ownFrom : 0;
         for (int t = 0; first + t * step < kTcRows && row0 + first + t * step < a.m; t += 2) {
             const int row = row0 + first + t * step;
-            const int from0 = __shfl_sync(0xffffffffu, ownFrom, t), end0 = __shfl_sync(0xffffffffu, ownEnd, t);
-            const int from1 = __shfl_sync(0xffffffffu, ownFrom, t + 1), end1 = __shfl_sync(0xffffffffu, ownEnd, t + 1);
+            const int from0 = __shfl_sync(0xffffffffu, ownFrom, t), len0 = __shfl_sync(0xffffffffu, ownLen, t);
+            const int from1 = __shfl_sync(0xffffffffu, ownFrom, t + 1), len1 = __shfl_sync(0xffffffffu, ownLen, t + 1);
             TcEntries e0, e1;
-            e0.Request(a, from0, end0, lane);
-            e1.Request(a, from1, end1, lane);
-            TcExpandRow(a, row, from0, end0, e0, sRow, lane);
-            if (first + (t + 1) * step < kTcRows && row + step < a.m) TcExpandRow(a, row + step, from1, end1, e1, sRow, lane);
+            e0.Request(a, from0, len0, lane);
+            e1.Request(a, from1, len1, lane);
+            TcExpandRow(a, row, from0, len0, e0, sRow, lane);
+            if (first + (t + 1) * step < kTcRows && row + step < a.m) TcExpandRow(a, row + step, from1, len1, e1, sRow, lane);
         }
     }
     // What was stored, here and by the rest of the cluster, is read, and the shared memory written, by TMA from here on.

@@ -522,46 +522,18 @@ __device__ __forceinline__ void RowDot(const int32_t *__restrict__ colInd, const
     constexpr int kChunk = Chunk<kLanes>::kChunk;
     constexpr int kBatch = kChunk < B200SP_SPMM_BATCH ? kChunk : B200SP_SPMM_BATCH;  // B rows in flight per lane
     const int li = threadIdx.x & (kLanes - 1);
-    [[maybe_unused]] int nextCol[kHold];
-    [[maybe_unused]] ValT nextVal[kHold];
-    [[maybe_unused]] auto request = [&](int p0) {
-#pragma unroll
-        for (int h = 0; h < kHold; ++h) {
-            nextCol[h] = 0;
-            nextVal[h] = FromF32<ValT>(0.0f);
-            if (p0 + h * kLanes + li < e) {
-                nextCol[h] = __ldcs(colInd + p0 + h * kLanes + li);
-                nextVal[h] = __ldcs(val + p0 + h * kLanes + li);
-            }
-        }
-    };
-    // The entries of the next chunk are asked for before this one's rows of B.  us without and with, f32 and f16 of N = 64 in rows of 20 to 64: 264.5
-    // and 259.6, 72.5 and 70.4; f32, N = 32: 39.9 and 38.4.  Other widths pay for the registers: f16, N = 8: 53 and 70; bf16, N = 128: 127 and 133.
-    // f16 and bf16, N = 32: 52.3 and 54.0, 87.5 and 90.7.
-    constexpr bool kEarly = kLanes == 8 || ((kLanes == 4 || kLanes == 16) && sizeof(ValT) == 4);
-    if constexpr (kEarly)
-        if (trips > 0) request(s);
     for (int chunk = 0; chunk < trips; ++chunk) {
         const int p0 = s + chunk * kChunk;
         const int rem = e - p0;  // entries of this group's row left; <= 0 once the row is done
         int myCol[kHold];
         float myVal[kHold];
-        if constexpr (kEarly) {
 #pragma unroll
-            for (int h = 0; h < kHold; ++h) {
-                myCol[h] = nextCol[h];
-                myVal[h] = ToF32(nextVal[h]);
-            }
-            if (chunk + 1 < trips) request(p0 + kChunk);
-        } else {
-#pragma unroll
-            for (int h = 0; h < kHold; ++h) {
-                myCol[h] = 0;
-                myVal[h] = 0.0f;
-                if (h * kLanes + li < rem) {
-                    myCol[h] = __ldcs(colInd + p0 + h * kLanes + li);
-                    myVal[h] = ToF32(__ldcs(val + p0 + h * kLanes + li));
-                }
+        for (int h = 0; h < kHold; ++h) {
+            myCol[h] = 0;
+            myVal[h] = 0.0f;
+            if (h * kLanes + li < rem) {
+                myCol[h] = __ldcs(colInd + p0 + h * kLanes + li);
+                myVal[h] = ToF32(__ldcs(val + p0 + h * kLanes + li));
             }
         }
         // Whole warp on full chunks: straight-line code, no predicate per entry.
