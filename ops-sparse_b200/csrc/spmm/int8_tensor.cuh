@@ -158,6 +158,7 @@ __device__ __forceinline__ void TcExpandRow(const TcArgs &a, int row, int from, 
         bad |= more.Write(sRow, width, least, lane);
     }
     bad = __any_sync(0xffffffffu, bad);
+    __syncwarp();  // bytes of other lanes are read from here on: votes order no memory
     uint4 *const out = reinterpret_cast<uint4 *>(a.dense + (long long)row * width);
     for (int i = lane; i < width / 16; i += 32) out[i] = sPieces[i];
     if (lane == 0) a.odd[row] = bad;
