@@ -28,6 +28,7 @@ constexpr int kTcTileBytes = kTcRows * kTcDepth;                     // of A, an
 constexpr int kTcSmem = 2 * kTcStages * kTcTileBytes + 1024;         // tiles start on multiples of 1024 bytes
 constexpr int kTcPitch = kTcCols + 4;       // of the sums in shared memory
 constexpr long long kTcMaxK = 12288;        // every warp has a row of A, written out, in the stages' shared memory
+constexpr long long kTcMaxDense = 4ll << 30;  // bytes of A written out
 static_assert(kTcMaxK * kTcWarps <= 2 * kTcStages * kTcTileBytes);
 static_assert(kTcRows * kTcPitch * 4 <= 2 * kTcStages * kTcTileBytes);
 

@@ -206,7 +206,8 @@ aclsparseStatus_t aclsparseSpMMPreprocess(aclsparseHandle_t handle, aclsparseOpe
     const int64_t repack = (int64_t)RepackBytes(matA, matB, matC, opB);
     p.repackBytes = matA->spmmSizedN == matC->cols && matA->spmmSizedRepack >= repack ? repack : 0;
     if (p.repackBytes > 0) {
-        const b200spSpmmShape sh = ShapeOf(matA, matB, matC, opB);
+        b200spSpmmShape sh = ShapeOf(matA, matB, matC, opB);
+        sh.longest_row = found.longestRow;
         int32_t ascending = 0;
         const int rc = b200sp_spmm_columns_ascend(static_cast<const int32_t *>(matA->offsets),
                                                   static_cast<const int32_t *>(matA->indices), &sh,

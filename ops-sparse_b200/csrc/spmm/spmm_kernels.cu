@@ -29,6 +29,7 @@
 // C = alpha*acc + beta*C with C not read when beta == 0; fp16 output is clamped to
 // +-65504 before rounding; int32 output is computed in int64 and saturated.
 #include <atomic>
+#include <cmath>
 #include <cstdint>
 #include <type_traits>
 
@@ -1920,6 +1921,14 @@ size_t RepackBytes(const b200spSpmmShape *sh, int valBytes)
     return (size_t)sh->k * (size_t)((sh->n + E - 1) / E) * 16;
 }
 
+// Lanes side by side on a row of B of n elements, `perLane` of them a lane.
+int LanesOf(int64_t n, int perLane)
+{
+    int lanes = 1;
+    while (lanes < 32 && (int64_t)lanes * perLane < n) lanes <<= 1;
+    return lanes;
+}
+
 // Repacking reads and writes k * n elements; the generic kernel reads nnz * n of them, with a load per product instead
 // of one per 16 bytes, and a 32-byte sector per load where the columns of B are the contiguous ones: there the copy is
 // fewer bytes from nnz = k * valBytes / 16 on (65,537 x 50,001 with 24 entries a row, fp16, N = 40: generic 257 us, copy
@@ -1963,29 +1972,56 @@ bool Copies(const b200spSpmmShape *sh, int valBytes, int32_t segments, const voi
            !FewEntries(sh, valBytes, segments) && plan != nullptr && Aligned16(plan);
 }
 
-// Whether an int8 product of rows whose columns ascend is one for the tensor cores: A at least one twelfth full, and work enough for the
-// two passes over it.  Lane groups / tensor cores, us: rows of C and B in 16-byte pieces, 4096 x 4096 at 0.1, N = 512: 69 / 24; 1278 rows, 24 / 20;
-// 40,000 x 2000 at 0.15, N = 16: 116 / 73; 700 x 1500 at 0.2, N = 128: 6.1 / 12.7; 1500 x 1100 at 0.18, N = 64: 8.1 / 13.2;
-// 20,000 x 1500 at 0.07, N = 100: 34 / 47; other layouts: 2000 x 1200 at 0.21, N = 40: 31 / 16; 1500 x 2500 at 0.15, N = 200: 61 / 24;
-// 4000 x 1050 at 0.11, N = 9: 11.5 / 18.
-bool TensorPays(const b200spSpmmShape *sh)
+// Whether an int8 product of rows whose columns ascend is one for the tensor cores.
+//   - A is at least one twelfth full as it is written out, in rows of a multiple of 128 bytes, and takes at most 4 GB so.
+//   - There is work enough for the two passes over it: 700 x 1500 at 0.2, N = 128, takes 6.1 us in lane groups and 12.7 on the tensor
+//     cores, 1500 x 1100 at 0.18, N = 64, 8.1 and 13.2, 4000 x 1050 at 0.11, N = 9, in columns, 11.5 and 18.
+//   - With rows enough to fill the SMs either way the two times are estimated, in us.  Lane groups cost by the entry, half as much
+//     again for rows of 0 to twice the mean, and by the row: mostly so where a CTA takes one; where C is not in rows of
+//     16-byte pieces, by the element of C too.  The tensor cores cost by the tile of 128 rows, of which an SM has one at a time.  Fitted
+//     to 523 products of 3,000 to 800,000 rows, k = 64 to 4096, N = 16 to 512; for 514 the choice is within 10 % of the better
+//     one.  Lane groups / tensor cores, us, 100,000 rows: 19 entries on 128 columns, N = 64: 25 / 65; 38 on 256, N = 256: 91 / 99; 60
+//     on 200, N = 256: 124 / 100; 77 on 512, N = 64: 60 / 78, N = 128: 87 / 78; 154 on 1024, N = 16: 274 / 94, N = 128: 166 / 94; in columns,
+//     200,000 rows, 50 on 256, N = 40: 100 / 141, N = 128: 174 / 167, 120 on 768, N = 40: 185 / 169, N = 128: 310 / 196.
+// longest: entries of the longest row, 0 while it is not known.
+bool TensorPays(const b200spSpmmShape *sh, long long longest)
 {
     const bool plain = RowsContiguous(sh->op_b, sh->order_b) && sh->order_c == 0 && sh->n % 16 == 0;
-    return sh->k <= kTcMaxK && 12 * sh->nnz >= sh->m * sh->k && sh->nnz * sh->n >= (plain ? 96ll : 24ll) << 20 && (plain || sh->n >= 24);
+    const long long denseCols = DenseCols(sh->k);
+    if (sh->m == 0 || sh->k > kTcMaxK || 12 * sh->nnz < sh->m * denseCols || sh->m * denseCols > kTcMaxDense) return false;
+    if (sh->nnz * sh->n < (plain ? 96ll : 24ll) << 20 || (!plain && sh->n < 24)) return false;
+    const long long sms = b200sp_sm_count();
+    if (sh->m < 64 * sms || sh->nnz > kLongRow * sh->m) return true;
+    const double n = (double)sh->n, mean = (double)sh->nnz / (double)sh->m, rows = 1e-5 * (double)sh->m;
+    const double spread = longest > 0 ? 0.525 * (1 + fmin((double)longest / mean, 2.0)) : 1.575;
+    const int across = LanesOf(sh->n, 16);
+    double lanes;
+    if (!plain)
+        lanes = 5 + 0.05 * n + rows * (8 + (sh->order_c != 0 ? 0.28 : 0.1) * n + spread * mean * (0.2 + 0.006 * fmax(n, 16.0 * across)));
+    else if (sh->nnz >= 128 * sh->m && sh->m * across / 32 < 64 * sms)
+        lanes = 4 + rows * fmax(265, 230 + 0.0069 * n * mean);
+    else
+        lanes = 4 + rows * spread * (8 + mean * (0.2 + 0.006 * n));
+    const long long tiles = (sh->m + kTcRows - 1) / kTcRows * ((sh->n + kTcCols - 1) / kTcCols);
+    const double turns = tiles <= sms ? 1 : (double)tiles / (double)sms + 0.65;  // of an SM: the last is short, on average
+    const double share = fmin(ceil(n / kTcCols), kTcCluster);                    // CTAs that write the rows of A out together
+    const double tile = 5.1 + 4.9 / share + (double)denseCols * (0.0033 + 0.0027 / share) +
+                        4 / share * floor(mean / (32 * kTcWindows)) + (sh->order_c != 0 ? 0.027 * fmin(n, kTcCols) : 0);
+    return lanes > tile * turns;
 }
 
 // What an analysed buffer holds after the plan: a copy of B (from a multiple of 256 bytes) and an A written out.
 size_t ExtraBytes(const b200spSpmmShape *sh, int valBytes)
 {
     const size_t repack = WorthRepacking(sh, valBytes) ? RepackBytes(sh, valBytes) : 0;
-    if (valBytes != 1 || !TensorPays(sh)) return repack;
+    if (valBytes != 1 || !TensorPays(sh, 0)) return repack;
     return AlignUp(repack, 256) + DenseBytes(sh->m, sh->k);
 }
 
 // Whether an int8 product with this much room, on rows found to ascend, writes A out.
 bool OnTensorCores(const b200spSpmmShape *sh, const void *plan)
 {
-    return sh->ascending != 0 && TensorPays(sh) && sh->repack_bytes >= (int64_t)ExtraBytes(sh, 1) && plan != nullptr && Aligned16(plan);
+    return sh->ascending != 0 && TensorPays(sh, sh->longest_row) && sh->repack_bytes >= (int64_t)ExtraBytes(sh, 1) && plan != nullptr && Aligned16(plan);
 }
 
 template <typename ValT, typename OutT>
@@ -2160,8 +2196,7 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
         a.nB = vecs * E;
     }
     int midUnits = sh->mid_units;
-    int lanes_ = 1;  // lanes side by side on a row of B
-    while (lanes_ < 32 && lanes_ * E < sh->n) lanes_ <<= 1;
+    int lanes_ = LanesOf(sh->n, E);
     // Rows of several tiles: half as wide a group where that leaves a fifth fewer lanes idle in the last one (bf16, N = 277,
     // 35,891 rows of 27: 162 us with 32 lanes, 122 with 16).  Narrower still loses more to rows of different lengths in one
     // warp than it gains, except by words, which wait for more loads (N = 150 above: 542, 460 and 408 us).
@@ -2345,7 +2380,7 @@ int b200sp_spmm_columns_ascend(const int32_t *row_ptr, const int32_t *col_ind, c
                                void *plan, size_t plan_bytes, int32_t *ascending, void *stream)
 {
     *ascending = 0;
-    if (val_type != B200SP_I8 || !TensorPays(shape) || col_ind == nullptr) return 0;
+    if (val_type != B200SP_I8 || !TensorPays(shape, shape->longest_row) || col_ind == nullptr) return 0;
     const PlanLayout L = LayoutFor(shape->m, shape->nnz, shape->n);
     if (plan == nullptr || plan_bytes < L.total) return (int)cudaErrorInvalidValue;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
