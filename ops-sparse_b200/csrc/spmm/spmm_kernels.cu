@@ -458,8 +458,6 @@ struct FastArgs {
     int slices;           // fp: warps a unit takes, 64 bytes of a B row each
     int splitRows;        // int8 only: a CTA per row
     int genRows;          // column-major C: rows of a CTA
-    int ctaRows;          // other C: rows of a CTA
-    int byLength;         // the 32 rows of a CTA are taken in order of their lengths
     const LongRow *longRows;
     const SegEntry *segs, *segsEnd;
     int32_t *counters;    // [long row][ArrivalsPerRow]
@@ -512,7 +510,7 @@ template <int kLanes> struct Chunk {
     static constexpr int kChunk = kLanes * kHold;
 };
 
-template <typename ValT, bool kKahan, int kLanes, bool kWords>
+template <typename ValT, bool kKahan, int kLanes, bool kWords, bool kOrdered>
 __device__ __forceinline__ void RowDot(const int32_t *__restrict__ colInd, const ValT *__restrict__ val,
                                        const ValT *__restrict__ B, const Slice<ValT, kWords> &slice, long long ldb, int s, int e, int trips,
                                        unsigned long long negZeros, float (&acc)[Pack<ValT>::kElems],
@@ -523,18 +521,49 @@ __device__ __forceinline__ void RowDot(const int32_t *__restrict__ colInd, const
     constexpr int kChunk = Chunk<kLanes>::kChunk;
     constexpr int kBatch = kChunk < B200SP_SPMM_BATCH ? kChunk : B200SP_SPMM_BATCH;  // B rows in flight per lane
     const int li = threadIdx.x & (kLanes - 1);
-    for (int chunk = 0; chunk < trips; ++chunk) {
-        const int p0 = s + chunk * kChunk;
-        const int rem = e - p0;  // entries of this group's row left; <= 0 once the row is done
-        int myCol[kHold];
-        float myVal[kHold];
+    [[maybe_unused]] int nextCol[kHold];
+    [[maybe_unused]] ValT nextVal[kHold];
+    // rem: entries of the row from p on, <= 0 past its end; p itself may then be past what an int counts
+    [[maybe_unused]] auto request = [&](int p, int rem) {
 #pragma unroll
         for (int h = 0; h < kHold; ++h) {
-            myCol[h] = 0;
-            myVal[h] = 0.0f;
+            nextCol[h] = 0;
+            nextVal[h] = FromF32<ValT>(0.0f);
             if (h * kLanes + li < rem) {
-                myCol[h] = __ldcs(colInd + p0 + h * kLanes + li);
-                myVal[h] = ToF32(__ldcs(val + p0 + h * kLanes + li));
+                nextCol[h] = __ldcs(colInd + p + h * kLanes + li);
+                nextVal[h] = __ldcs(val + p + h * kLanes + li);
+            }
+        }
+    };
+    // The entries of the next chunk are asked for before this one's rows of B.  us without and with: f32, 64 entries a row, N = 64, 262 and 252;
+    // f32, N = 16, power-law rows of 100, 172 and 157, ragged rows of 16, 6.6 and 5.9; N = 32, 3000 rows of 60, 9.0 and 8.1.  Not for
+    // fp32 rows of eight lanes and more that are taken by length (N = 64, ragged rows of 12, 52 and 56), nor for other widths (f16, N = 8: 53 and
+    // 70; bf16, N = 128: 127 and 133; f16 and bf16, N = 32: 52 and 54, 88 and 91).
+    constexpr bool kWide = sizeof(ValT) == 4;
+    constexpr bool kEarly = (kLanes == 4 && kWide) || (kLanes == 8 && !(kWide && kOrdered)) || (kLanes == 16 && kWide && !kOrdered);
+    if constexpr (kEarly)
+        if (trips > 0) request(s, e - s);
+    for (int chunk = 0; chunk < trips; ++chunk) {
+        const int p0 = (int)((unsigned)s + chunk * kChunk);
+        const int rem = e - s - chunk * kChunk;  // entries of this group's row left; <= 0 once the row is done
+        int myCol[kHold];
+        float myVal[kHold];
+        if constexpr (kEarly) {
+#pragma unroll
+            for (int h = 0; h < kHold; ++h) {
+                myCol[h] = nextCol[h];
+                myVal[h] = ToF32(nextVal[h]);
+            }
+            if (chunk + 1 < trips) request((int)((unsigned)p0 + kChunk), rem - kChunk);
+        } else {
+#pragma unroll
+            for (int h = 0; h < kHold; ++h) {
+                myCol[h] = 0;
+                myVal[h] = 0.0f;
+                if (h * kLanes + li < rem) {
+                    myCol[h] = __ldcs(colInd + p0 + h * kLanes + li);
+                    myVal[h] = ToF32(__ldcs(val + p0 + h * kLanes + li));
+                }
             }
         }
         // Whole warp on full chunks: straight-line code, no predicate per entry.
@@ -941,14 +970,14 @@ template <typename ValT, int kLanes> struct FastShape {
     static constexpr int kFit = 8192 / kTileCols < 32 ? 8192 / kTileCols : 32;  // at most 32 KB of tile
     static constexpr int kGenRows = kCtaRows > kFit ? kCtaRows : kFit;
     // 32 rows of a CTA may be taken in order of their lengths (int8 loses: 44.6 and 50.3 us on 55,686 rows of 0 to 232 entries, N = 16).
-    static constexpr bool kOrdered = !std::is_same_v<ValT, int8_t> && kCtaRows <= 32 && kGroup < 32;
+    static constexpr bool kMayOrder = !std::is_same_v<ValT, int8_t> && kCtaRows <= 32 && kGroup < 32;
 };
 
 enum { kPlain, kAnyC, kAnyCWords };
 // Rows of a few entries are a chain of dependent loads (row offsets, columns, B, C): warps hide it, so registers are held to
 // what 36 warps per SM leave (24 for wide int8 rows, whose quads of B rows need more).
 template <typename ValT, int kLanes> constexpr int kFastCtas = std::is_same_v<ValT, int8_t> && kLanes >= 8 ? 6 : 9;
-template <typename ValT, typename OutT, bool kKahan, int kLanes, int kLayout>
+template <typename ValT, typename OutT, bool kKahan, int kLanes, int kLayout, bool kOrdered>
 __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKernel(const FastArgs<ValT, OutT> a)
 {
     using Acc = typename Arith<ValT>::Acc;
@@ -964,7 +993,6 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
     constexpr int kTileWords = kGenC ? (Shape::kGenRows * kTileStride > kThreads * E ? Shape::kGenRows * kTileStride : kThreads * E) : 0;
     __shared__ __align__(16) Acc sBuf[kWarps * kWarpWords > kTileWords ? kWarps * kWarpWords : kTileWords];
     __shared__ unsigned char sSkip[kGenC ? Shape::kGenRows : 1];
-    constexpr bool kOrdered = Shape::kOrdered;
     __shared__ unsigned char sOrder[kOrdered ? kWarps : 1][32];
     __shared__ int sLast;
 
@@ -998,19 +1026,17 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
         // ---- one lane group per row ----
         constexpr int kChunk = kInt8 ? Group8<kLanes>::kChunk : Chunk<kLanes>::kChunk;
         const bool rowsRun = kGenC && a.cCol != 1;  // column-major C
-        const int blockRows = rowsRun ? a.genRows : a.ctaRows;
+        const int blockRows = kOrdered ? 32 : rowsRun ? a.genRows : Shape::kCtaRows;
         const long long row0 = (long long)(blockIdx.x - a.unitCtas) * blockRows;
-        if constexpr (kOrdered) {
-            if (a.byLength) {  // sOrder[i]: the row with the i-th most entries (every warp has its own copy: no barrier)
-                int len = row0 + lane < a.m ? a.rowPtr[row0 + lane + 1] - a.rowPtr[row0 + lane] : 0;
-                if (len > a.rowLimit) len = 0;
-                const int key = len << 5 | (31 - lane);
-                int rank = 0;
+        if constexpr (kOrdered) {  // sOrder[i]: the row with the i-th most entries (every warp has its own copy: no barrier)
+            int len = row0 + lane < a.m ? a.rowPtr[row0 + lane + 1] - a.rowPtr[row0 + lane] : 0;
+            if (len > a.rowLimit) len = 0;
+            const int key = len << 5 | (31 - lane);
+            int rank = 0;
 #pragma unroll
-                for (int j = 1; j < 32; ++j) rank += __shfl_xor_sync(0xffffffffu, key, j) > key;
-                sOrder[warp][rank] = (unsigned char)lane;
-                __syncwarp();
-            }
+            for (int j = 1; j < 32; ++j) rank += __shfl_xor_sync(0xffffffffu, key, j) > key;
+            sOrder[warp][rank] = (unsigned char)lane;
+            __syncwarp();
         }
         for (int col0 = 0; col0 < (rowsRun ? a.n : 1); col0 += kTileCols) {  // column-major C: a tile of columns at a time
 #pragma unroll 1
@@ -1019,7 +1045,7 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
                 if constexpr (kOrdered) {
                     // every other pass the other way round: the warp with the longest rows of one has the shortest of the next
                     const int turn = pass & Shape::kCtaRows ? kWarps - 1 - warp : warp;
-                    if (a.byLength) rowIn = sOrder[warp][pass + turn * kRowsPerWarp + lane / kGroup];
+                    rowIn = sOrder[warp][pass + turn * kRowsPerWarp + lane / kGroup];
                 }
                 const long long row = row0 + rowIn;
                 int s = 0, e = 0;
@@ -1061,7 +1087,7 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
                         } else {
                             slice.first[0] = colLive ? col : 0;
                         }
-                        RowDot<ValT, kKahan, kLanes, kWords>(a.colInd, a.val, a.B, slice, a.ldb, s, e, trips, a.negZeros, acc, comp);
+                        RowDot<ValT, kKahan, kLanes, kWords, kOrdered>(a.colInd, a.val, a.B, slice, a.ldb, s, e, trips, a.negZeros, acc, comp);
                     }
                     if (kKahan) {
 #pragma unroll
@@ -2010,6 +2036,28 @@ bool TensorPays(const b200spSpmmShape *sh, long long longest)
     return lanes > tile * turns;
 }
 
+// Whether a CTA takes its 32 rows in order of their lengths (ctaRows, genRows: those it takes otherwise, of row- and of column-major
+// C): the rows that a warp takes together wait for the longest of them.  It costs a pass over the lengths and fewer CTAs.  Never where the
+// longest row has less than a quarter more entries than the mean.  Rows in their own order and so, us; ragged: rows of 0 to twice the mean,
+// 150,000 of them where not said.
+//   - Column-major C, whose CTAs have 32 rows anyway: ragged rows of 3, f16, N = 64, 53 and 43; of 40, 166 and 111.
+//   - Eight lanes a row and more, with four CTAs of 32 rows for every SM (six where that takes four passes instead of one) and 1700
+//     entries: ragged rows of 3, bf16, N = 128, 45 and 38, of 40, 182 and 138; power-law rows of 16, f32, N = 64, 103 and 94; but 30,000 rows of 6, 9.3
+//     and 10.3, 20,000 of 24, 15.6 and 17.1.
+//   - Four lanes, where 32 rows are one pass and a warp's eight rows are not shared out better: rows of like lengths, or long ones, in 16-bit
+//     types from 8 entries on (f16, N = 32: ragged rows of 6 17.3 and 18.0, of 9 23.1 and 22.6, of 40 74 and 61; 4000 power-law rows of 16 22.6 and 27.1,
+//     150,000 of 24 74 and 72), in fp32, whose rows of B take twice as long, from 64 (N = 16: ragged rows of 5 13.6 and 15.1, of 16 25.7
+//     and 26.5, of 100 130 and 125).
+bool OrderPays(const b200spSpmmShape *sh, int valBytes, int ctaRows, int genRows)
+{
+    if (4 * sh->longest_row * sh->m < 5 * sh->nnz) return false;
+    if (sh->order_c != 0) return genRows == 32;
+    const long long sms = b200sp_sm_count();
+    const bool many = sh->m >= (ctaRows < 16 ? 6 : 4) * 32 * sms;
+    if (ctaRows < 32) return many && sh->nnz >= 1700 * sms;
+    return sh->nnz >= (valBytes == 2 ? 8 : 64) * sh->m && (sh->longest_row * sh->m <= 4 * sh->nnz || (many && sh->nnz >= 24 * sh->m));
+}
+
 // What an analysed buffer holds after the plan: a copy of B (from a multiple of 256 bytes) and an A written out.
 size_t ExtraBytes(const b200spSpmmShape *sh, int valBytes)
 {
@@ -2218,29 +2266,27 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             const long long unitCtas = kInt8 ? units : ((long long)units * a.slices + kWarps - 1) / kWarps;
             a.unitCtas = (int)unitCtas;
             a.genRows = sh->m < 2ll * Shape::kGenRows * b200sp_sm_count() ? Shape::kCtaRows : Shape::kGenRows;
-            // The rows that a warp takes together wait for the longest of them: a CTA takes 32 rows in order of their lengths where
-            // that leaves every SM four CTAs.  Rows of 0 to twice the mean, us in their own order and so: f16, N = 64: 98.8 and 72.5; f32, N = 32: 49.4
-            // and 39.9; bf16, N = 128: 163 and 127; f16, N = 37: 65 and 51; columns of C, N = 40: 53 and 41; power-law rows, bf16,
-            // N = 64: 186 and 175.  Not where the longest has less than a quarter more entries than the mean: rows of 30, bf16, N = 128,
-            // take 102 us eight to a CTA and 108 with 32, which makes for a longer last wave.
-            const bool uneven = Shape::kOrdered && 4 * sh->longest_row * sh->m >= 5 * sh->nnz;
-            a.ctaRows = uneven && sh->m >= 4 * 32ll * b200sp_sm_count() ? 32 : Shape::kCtaRows;
-            a.byLength = uneven && (sh->order_c == 0 ? a.ctaRows : a.genRows) == 32;
-            const long long rows = a.splitRows ? 1 : sh->order_c == 0 ? a.ctaRows : a.genRows;
+            const bool byLength = Shape::kMayOrder && rowCtas && OrderPays(sh, (int)sizeof(ValT), Shape::kCtaRows, a.genRows);
+            const long long rows = a.splitRows ? 1 : byLength ? 32 : sh->order_c == 0 ? Shape::kCtaRows : a.genRows;
             const long long grid = unitCtas + (rowCtas ? (sh->m + rows - 1) / rows : 0);
             if (grid == 0) return;
             auto go = [&](auto kernel) { err = b200sp::LaunchChained(kernel, (unsigned)grid, kThreads, 0, st, a); };
-            auto pick = [&]<bool kKahan>() {
-                if (cPlain) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kPlain>);
+            auto pick = [&]<bool kKahan, bool kOrdered>() {
+                if (cPlain) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kPlain, kOrdered>);
                 if constexpr (!kInt8)
-                    if (words) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyCWords>);
-                go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyC>);
+                    if (words) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyCWords, kOrdered>);
+                go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyC, kOrdered>);
+            };
+            auto pickOrder = [&]<bool kKahan>() {
+                if constexpr (Shape::kMayOrder)
+                    if (byLength) return pick.template operator()<kKahan, true>();
+                pick.template operator()<kKahan, false>();
             };
             if constexpr (std::is_same_v<ValT, float>) {
-                if (sh->kahan) pick.template operator()<true>();
-                else pick.template operator()<false>();
+                if (sh->kahan) pickOrder.template operator()<true>();
+                else pickOrder.template operator()<false>();
             } else {
-                pick.template operator()<false>();
+                pickOrder.template operator()<false>();
             }
             b200sp_note_launches(1);
         };

@@ -4,6 +4,8 @@ from __future__ import annotations
 
 import numpy as np
 import pytest
+import scipy.sparse
+import torch
 
 from test_spmm_gpu import check_compact, compact_case, run_spmm
 
@@ -127,6 +129,45 @@ def test_rows_in_order_of_their_lengths(handle, device, oracle, vt, ot, n, order
     got = run_spmm(handle, device, rp, ci, val, vt, stored(B), stored(C), ot, m, k, n, ldb, ldc, 1.5, -0.5,
                    b_order=order, c_order=order)
     got = got.reshape(m, n) if order == "row" else np.ascontiguousarray(got.reshape(n, m).T)
+    if vt == "f32":
+        gold = oracle.spmm_f32_layout(m, n, rp, ci, val, B, n, True, False, C, n, True, 1.5, -0.5)
+    else:
+        gold = oracle.spmm_16(rp, ci, val, B, C, 1.5, -0.5, vt, ot)
+    assert np.array_equal(got.view(np.uint8), np.asarray(gold).reshape(m, n).view(np.uint8))
+
+
+# lanes a row and what the kernel is asked for beside: compensated sums, B by words, C in rows of any width, scalars on the device
+@pytest.mark.parametrize("vt,ot,m,k,n,most,kind", [
+    ("f32", "f32", 18957, 3000, 32, 40, "plain"), ("f32", "f32", 18957, 3000, 32, 40, "kahan"),
+    ("f32", "f32", 28423, 90000, 37, 40, "plain"), ("f16", "f16", 28423, 90000, 74, 40, "plain"), ("f32", "f32", 18957, 60000, 21, 40, "kahan"),
+    ("f16", "f16", 18957, 3000, 32, 40, "plain"), ("bf16", "bf16", 5003, 3000, 24, 40, "device"), ("f32", "f32", 5003, 3000, 16, 140, "plain"),
+    ("f32", "f32", 5003, 3000, 13, 140, "kahan"), ("bf16", "f32", 18957, 3000, 64, 40, "wide"), ("f32", "f32", 28423, 3000, 64, 40, "device"),
+])
+def test_uneven_rows_in_order_of_their_lengths(handle, device, oracle, vt, ot, m, k, n, most, kind):
+    """The rules' own ranges: four lanes from 8 (64) entries on, more lanes from 1700 entries for every SM on; the golden's bits."""
+    from ops_sparse_b200 import ACL_SPARSE_SPMM_CSR_FP32_HIGH_PRECISION_ALG as KAHAN
+    rng = np.random.default_rng(n)
+    lengths = rng.integers(0, most + 1, m)
+    lengths[64:128] = most // 2              # CTAs of equal rows
+    lengths[128:160] = 0                     # ... and of empty ones
+    rp, ci, val, B, C = compact_case(oracle, rng, m, k, n, lengths, vt, ot, 1.5, -0.5)
+    ldc = n + 1 if kind == "wide" else n
+    stored = np.zeros((m, ldc), C.dtype)
+    stored[:, :n] = C
+    alpha, beta = 1.5, -0.5
+    if kind == "device":
+        handle.set_pointer_mode_device(True)
+        alpha, beta = (torch.tensor(v, dtype=torch.float32, device=device) for v in (1.5, -0.5))
+    got = run_spmm(handle, device, rp, ci, val, vt, B, stored, ot, m, k, n, n, ldc, alpha, beta, alg=KAHAN if kind == "kahan" else 0)
+    got = got.reshape(m, ldc)
+    assert not got[:, n:].any()
+    got = np.ascontiguousarray(got[:, :n])
+    if kind == "kahan":
+        exact = 1.5 * np.asarray(scipy.sparse.csr_matrix((val.astype(np.float64), ci, rp), shape=(m, k)) @ B.astype(np.float64)) - 0.5 * C
+        scale = 1.5 * oracle.spmm_abs_sum(rp, ci, val, B, vt) + 0.5 * np.abs(C)
+        # products one rounding, compensated sums two, alpha, beta and the last sum one each
+        assert np.all(np.abs(got - exact) <= 6 * 2.0 ** -24 * scale)
+        return
     if vt == "f32":
         gold = oracle.spmm_f32_layout(m, n, rp, ci, val, B, n, True, False, C, n, True, 1.5, -0.5)
     else:
