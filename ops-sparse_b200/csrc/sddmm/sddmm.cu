@@ -80,10 +80,12 @@ __global__ void __launch_bounds__(256) SddmmKernel(const int32_t *__restrict__ r
 //     apart; a warp therefore works on 32 / kLanes entries at a time, and rows wider than kLanes * kSlabs pieces take
 //     several turns.
 //   - Rows come through shared memory by cp.async, two batches of kBatch entries deep per lane group: no registers
-//     hold data in flight.  The batches are as short as the sums allow, for what a warp's ring leaves free are more warps, and those
-//     keep more copies in flight than longer rings do: 100,000 rows of up to 40 entries, fp16, k = 400, two pieces a lane: 265 us
-//     with four entries a batch, 225 with two; f32, k = 512, four pieces: 327 with two, 273 with one; three or four batches deep, with as
-//     many copies in flight per warp, 1.1 to 1.6 times as long.
+//     hold data in flight.  With warps enough the batches are short (kShortBatch), for what a warp's ring leaves free are more warps, and
+//     those keep more copies in flight than longer rings do: 2.4 M entries, fp16, k = 400, 248 us with one entry a batch, k = 512, 258, 310 and
+//     404 with one, two and four; but pieces of 4 bytes, fp32, k = 211, 593, 499 and 477.  Three or four batches deep, with as many copies
+//     in flight per warp, take 1.1 to 1.6 times as long.  Where all warps find room on the SMs with a longer batch, it is as long as that: a small
+//     product waits for one copy after the other.  2000 entries, fp16, k = 64, 4.2 us with two entries a batch, 3.5 with four; fp32, k = 512, 13.1
+//     with one, 8.3 with four; 38,400 entries, 14.9 and, with two, 11.9.
 //   - A row of X is copied only when it differs from the entry before, and stays in registers, converted, until then.  Two products
 //     share an instruction (packed fp32): a row of 512 bytes in fp16 takes some 30 instead of 47 instructions.
 //   - A warp owns a tile of consecutive entries.  What is done once per entry (row, column, old value, store) is done
@@ -92,8 +94,8 @@ __global__ void __launch_bounds__(256) SddmmKernel(const int32_t *__restrict__ r
 //     carries costs as many shuffles as values are left.
 // fp16 rows that start on odd 2-byte addresses (kBytes = 2) are copied as the 4-byte words that cover them and
 // realigned when they are read from shared memory.
-// Measured (1 M nodes, 16.0 M entries, fp16, k = 256): 1242 us with 32 lanes a row and scalar products, 1166 us here, which is the 7.6 GB
-// of Y rows that come from DRAM at 6.5 TB/s.  Working through Y by blocks of columns that stay in L2 (the pieces of rows of 64 entries and
+// Measured (1 M nodes, 16.0 M entries, fp16, k = 256): 1256 us with 32 lanes a row and scalar products, 1139 us here, which is the 7.6 GB
+// of Y rows that come from DRAM at 6.7 TB/s.  Working through Y by blocks of columns that stay in L2 (the pieces of rows of 64 entries and
 // more that lie in a block taken together) cut that to 5.6 GB and cost 1930 us and more: short pieces, and X rows fetched anew for each.
 template <int kBytes> struct Words { using Type = uint32_t; };  // 4, and the words of kBytes = 2
 template <> struct Words<16> { using Type = uint4; };
@@ -138,16 +140,24 @@ template <int kSize, bool kNear = true> __device__ __forceinline__ void CopyAsyn
 __device__ __forceinline__ void CopyCommit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int kPending> __device__ __forceinline__ void CopyWait() { asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory"); }
 
-// The same inputs again and again: 1384 us with 4 warps and tiles of 128, 1286 with 2 and 64 on the same GPU; one warp or longer tiles gain nothing more.
-constexpr int kSddmmWarps = 2;
+constexpr int kSddmmWarps = 2;  // the same with 4 (1 M nodes: 1139 and 1148 us) and with tiles of 128 (1147)
 constexpr int kSddmmTile = 64;  // entries a warp works on at a time, at most
-template <int kBytes, int kLanes, int kSlabs> struct SddmmShape {
-    static constexpr int kBatch = kSlabs <= 2 ? 2 : 1;
+// Entries of a batch where there are warps enough: about 2 KB of copies a batch, half as much of the widest pieces.  Four lanes of three
+// pieces have few entries a group, and warps enough from the start (fp16, k = 36, 320,000 entries: 11.5 us with one, 13.9 with two).
+template <int kBytes, int kLanes, int kSlabs>
+constexpr int kShortBatch = kLanes == 4 && kSlabs == 3 ? 1
+                            : kBytes < 8  ? 4
+                            : kBytes == 8 ? (kSlabs <= 2 ? 4 : kSlabs == 3 || kLanes == 16 ? 2 : 1)
+                                          : (kSlabs <= 2 ? 2 : 1);
+
+template <int kBytes, int kSlabs, int kBatch> struct SddmmShape {
     static constexpr int kStages = 2;
     static constexpr int kCopy = kBytes == 2 ? 4 : kBytes;
     static constexpr int kSlotBytes = 32 * kSlabs * kCopy;                       // one entry of every lane group
     static constexpr int kRing = 2 * kStages * kBatch * kSlotBytes;              // rows of Y, rows of X
     static constexpr int kTileBytes = kSddmmTile * 12;                           // row, column, sum per entry
+    static constexpr int kShared = kSddmmWarps * (kRing + kTileBytes);
+    static constexpr int kWarpsPerSm = kSddmmWarps * ((228 << 10) / (kShared + 1024));  // that find room at once
 };
 
 struct RowsOf {  // the operands' rows and how far apart they are
@@ -157,13 +167,12 @@ struct RowsOf {  // the operands' rows and how far apart they are
 };
 
 // The dot products of a tile of entries: sDot[t] = X row sRow[t] . Y row sCol[t].  tile: a multiple of 32.
-template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear>
+template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear, int kBatch>
 __device__ __forceinline__ void TileDots(const RowsOf &rows, unsigned char *ring, const int *sRow, const int *sCol, float *sDot,
                                          int tile, int lane)
 {
-    using Shape = SddmmShape<kBytes, kLanes, kSlabs>;
+    using Shape = SddmmShape<kBytes, kSlabs, kBatch>;
     using Piece = typename Words<kBytes>::Type;
-    constexpr int kBatch = Shape::kBatch;
     constexpr int kStages = Shape::kStages;
     constexpr int kCopy = Shape::kCopy;
     constexpr bool kOdd = kBytes == 2;
@@ -288,10 +297,7 @@ __device__ __forceinline__ void TileDots(const RowsOf &rows, unsigned char *ring
                 for (int off = kLanes / 4; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
                 u = up ? 1 : 0;
             }
-            if ((li & (kLanes / kBatch - 1)) == 0) {
-                float *dot = sDot + t0 + batch * kBatch + u;
-                *dot = piece0 == 0 ? v : *dot + v;
-            }
+            if ((li & (kLanes / kBatch - 1)) == 0) sDot[t0 + batch * kBatch + u] += v;
             __syncwarp();  // this stage's slots may be written again
         }
         CopyWait<0>();
@@ -299,13 +305,13 @@ __device__ __forceinline__ void TileDots(const RowsOf &rows, unsigned char *ring
     }
 }
 
-template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear>
+template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear, int kBatch>
 __global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(const int32_t *__restrict__ rowPtr,
                                                                     const int32_t *__restrict__ colInd, T *__restrict__ cVal,
                                                                     const RowsOf rows, int m, int nnz, int tile, float alpha,
                                                                     float beta, const T *alphaDev, const T *betaDev)
 {
-    using Shape = SddmmShape<kBytes, kLanes, kSlabs>;
+    using Shape = SddmmShape<kBytes, kSlabs, kBatch>;
     extern __shared__ __align__(16) unsigned char sRaw[];
     b200sp::WaitForPrevious();
     const float a = alphaDev ? Load<T>(alphaDev) : alpha;
@@ -326,7 +332,7 @@ __global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(const int32_
         r0 = __shfl_sync(0xffffffffu, r, 31);
     }
     __syncwarp();
-    TileDots<T, kBytes, kLanes, kSlabs, kNear>(rows, ring, sRow, sCol, sDot, tile, lane);
+    TileDots<T, kBytes, kLanes, kSlabs, kNear, kBatch>(rows, ring, sRow, sCol, sDot, tile, lane);
     for (int t = lane; t < tile && p0 + t < nnz; t += 32) {
         float z = a * sDot[t];
         if (b != 0.0f) z += b * Load<T>(cVal + p0 + t);
@@ -414,24 +420,23 @@ template <auto kKernel> cudaError_t AllowSharedMemory(int bytes, int *device)
     return e;
 }
 
-template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear, typename... Args>
+template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear, int kBatch, typename... Args>
 int LaunchRowsShape(int nnz, int tile, cudaStream_t stream, Args... args)
 {
-    using Shape = SddmmShape<kBytes, kLanes, kSlabs>;
-    constexpr int kShared = kSddmmWarps * (Shape::kRing + Shape::kTileBytes);
+    using Shape = SddmmShape<kBytes, kSlabs, kBatch>;
     int dev = 0;
-    const cudaError_t e = AllowSharedMemory<SddmmRowsKernel<T, kBytes, kLanes, kSlabs, kNear>>(kShared, &dev);
+    const cudaError_t e = AllowSharedMemory<SddmmRowsKernel<T, kBytes, kLanes, kSlabs, kNear, kBatch>>(Shape::kShared, &dev);
     if (e != cudaSuccess) return (int)e;
     const long long warps = ((long long)nnz + tile - 1) / tile;
     b200sp_note_launches(1);
-    return (int)b200sp::LaunchChained(SddmmRowsKernel<T, kBytes, kLanes, kSlabs, kNear>,
-                                      (unsigned)((warps + kSddmmWarps - 1) / kSddmmWarps), 32 * kSddmmWarps, kShared,
+    return (int)b200sp::LaunchChained(SddmmRowsKernel<T, kBytes, kLanes, kSlabs, kNear, kBatch>,
+                                      (unsigned)((warps + kSddmmWarps - 1) / kSddmmWarps), 32 * kSddmmWarps, Shape::kShared,
                                       stream, args...);
 }
 
-// 300,000 rows of up to eight entries, 16-byte copies past L1 and through it, us, by the size of Y: 9 columns, fp16, k = 16 (0.3 KB) 298
-// and 31, k = 200 (3.5 KB) 543 and 108, fp32, k = 300 (10.5 KB) 1085 and 304; 100 columns, fp16, k = 64 (12.5 KB) 36 and 39, fp32,
-// k = 64 (25 KB) 55 and 63; 1 M columns, fp16, k = 256, 16 M entries: 1404 and 1618.
+// 300,000 rows of four entries, 16-byte copies past L1 and through it, us, by the size of Y: 9 columns, fp16, k = 16 (0.3 KB) 292 and
+// 24, k = 200 (3.5 KB) 542 and 89, fp32, k = 300 (10.5 KB) 823 and 245; 100 columns, fp16, k = 64 (12.5 KB) 34 and 37, fp32,
+// k = 64 (25 KB) 63 and 69; 1 M columns, fp16, k = 256, 16 M entries: 1140 and 1737.
 constexpr long long kNearBytes = 12 << 10;
 
 template <typename T, int kBytes>
@@ -446,33 +451,44 @@ int LaunchRows(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const
     while (tile < kSddmmTile && nnz / (2 * tile) >= 16 * b200sp_sm_count()) tile *= 2;
     // A Y of a few lines that all entries want is asked of a few slices of L2 by every SM at once: it comes through L1.
     const bool near = kBytes == 16 && (long long)C->cols * st.yj * (long long)sizeof(T) <= kNearBytes;
-    auto launchAs = [&]<int kLanes, int kSlabs, bool kNear>() {
+    auto launchAs = [&]<int kLanes, int kSlabs, bool kNear, int kBatch>() {
         const RowsOf rows{static_cast<const char *>(X->values), static_cast<const char *>(Y->values),
                           st.xi * (long long)sizeof(T), st.yj * (long long)sizeof(T), k};
-        return LaunchRowsShape<T, kBytes, kLanes, kSlabs, kNear>(
-            nnz, tile, stream, static_cast<const int32_t *>(C->offsets), static_cast<const int32_t *>(C->indices),
-            static_cast<T *>(C->values), rows, (int)C->rows, nnz, tile, alpha, beta, static_cast<const T *>(alphaDev),
+        // Rows of more than 32 pieces are long enough work for a last wave that is nearly empty to show.  320,000 entries, fp32, tiles of 64 and
+        // 32: k = 400 80 and 66 us, k = 512 68 and 58, fp16, k = 640 66 and 56; narrower rows lose (fp16, k = 80: 17.2 and 19.0).
+        const long long room = (long long)SddmmShape<kBytes, kSlabs, kBatch>::kWarpsPerSm * b200sp_sm_count(), warps = nnz / kSddmmTile;
+        const int entries = kLanes * kSlabs > 32 && warps > room && warps < 3 * room ? 32 : tile;
+        return LaunchRowsShape<T, kBytes, kLanes, kSlabs, kNear, kBatch>(
+            nnz, entries, stream, static_cast<const int32_t *>(C->offsets), static_cast<const int32_t *>(C->indices),
+            static_cast<T *>(C->values), rows, (int)C->rows, nnz, entries, alpha, beta, static_cast<const T *>(alphaDev),
             static_cast<const T *>(betaDev));
     };
-    auto launch = [&]<int kLanes, int kSlabs>() {
+    auto launchDeep = [&]<int kLanes, int kSlabs, int kBatch>() {
         if constexpr (kBytes == 16)
-            if (near) return launchAs.template operator()<kLanes, kSlabs, true>();
-        return launchAs.template operator()<kLanes, kSlabs, false>();
+            if (near) return launchAs.template operator()<kLanes, kSlabs, true, kBatch>();
+        return launchAs.template operator()<kLanes, kSlabs, false, kBatch>();
     };
-    // Few lanes and several pieces each: a warp then works on more entries per instruction.  16-byte pieces, us with 8 to 32 lanes of
-    // one piece (four entries a batch) and as here: 10 pieces 46.5 and 36.8, 12 123 and 93, 16 228 and 209, 20 147 and 110, 24 77.6 and
-    // 58.1, 32 (100,000 rows of up to 40 entries) 142 and 124; with 32 lanes of two or four pieces: 33 561 and 344, 50 300 and 212, 64
-    // (f32) 544 and 490, 75 622 and 450.  Up to 8 pieces and from 13 to 15 fewer lanes gain nothing (8 pieces: 52.8 and 60.7).
+    auto launch = [&]<int kLanes, int kSlabs>() {
+        constexpr int kShort = kShortBatch<kBytes, kLanes, kSlabs>;
+        const long long warps = (nnz + 31ll) / 32 / b200sp_sm_count();  // for every SM, with the shortest tiles
+        if constexpr (kShort < 4)
+            if (warps < SddmmShape<kBytes, kSlabs, 4>::kWarpsPerSm) return launchDeep.template operator()<kLanes, kSlabs, 4>();
+        if constexpr (kShort < 2)
+            if (warps < SddmmShape<kBytes, kSlabs, 2>::kWarpsPerSm) return launchDeep.template operator()<kLanes, kSlabs, 2>();
+        return launchDeep.template operator()<kLanes, kSlabs, kShort>();
+    };
+    // Few lanes and several pieces each: a warp then works on more entries per instruction.  2.4 M entries, 16-byte pieces, us with 16 or 32
+    // lanes of one piece, or 32 of two and four, and as here: 10 pieces 113 and 71, 16 109 and 83, 20 185 and 110, 24 183 and 111, 32
+    // 183 and 131, 50 352 and 248, 80 576 and 371, 128 (fp16) 631 and 584.  Up to 8 pieces fewer lanes gain nothing.  Rows of 14 and 16 pieces start on
+    // 32-byte sectors, which four lanes side by side fill: 84 and 83 us, by eight lanes 90 and 89; of 13 and 15: 94 and 101, by eight 91 and 92.
     if (pieces <= 4) return launch.template operator()<4, 1>();
     if (pieces <= 8) return launch.template operator()<8, 1>();
     if (pieces <= 12) return launch.template operator()<4, 3>();
-    if (pieces < 16) return launch.template operator()<8, 2>();
-    if (pieces == 16) return launch.template operator()<4, 4>();
+    if (pieces <= 16) return pieces % 2 != 0 ? launch.template operator()<8, 2>() : launch.template operator()<4, 4>();
     if (pieces <= 24) return launch.template operator()<8, 3>();
     if (pieces <= 32) return launch.template operator()<8, 4>();
     if (pieces <= 48) return launch.template operator()<16, 3>();
     if (pieces <= 64) return launch.template operator()<16, 4>();
-    if (pieces <= 64) return launch.template operator()<32, 2>();
     if (pieces <= 96) return launch.template operator()<32, 3>();
     return launch.template operator()<32, 4>();
 }

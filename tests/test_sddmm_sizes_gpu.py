@@ -26,6 +26,17 @@ def test_pieces(pkg, handle, device, pieces, dtype):
     check(pkg, handle, device, rng, rng.integers(0, 9, 90), pieces * (4 if dtype == "f32" else 8), 0, dtype)
 
 
+# one to four entries a batch, tiles of 32 and 64 entries: every shape at entry counts on either side of where they change, which depends
+# on the shared memory of a shape; pieces of 16, 8, 4 and 2 bytes
+@pytest.mark.parametrize("nnz", [18944, 37889, 75777, 151553, 260003])
+@pytest.mark.parametrize("dtype,k", [("f16", 32), ("f16", 64), ("f16", 80), ("f16", 104), ("f16", 112), ("f16", 192), ("f16", 256), ("f16", 384),
+                                     ("f32", 256), ("f16", 768), ("f32", 512), ("f32", 600), ("f16", 20), ("f16", 36), ("f16", 100), ("f16", 204),
+                                     ("f16", 300), ("f16", 500), ("f16", 18), ("f32", 129), ("f16", 23), ("f16", 401)])
+def test_entries_in_flight(pkg, handle, device, dtype, k, nnz):
+    rng = np.random.default_rng(nnz + k)
+    check(pkg, handle, device, rng, np.bincount(rng.integers(0, 9000, nnz), minlength=9000), k, 0, dtype)
+
+
 @pytest.mark.parametrize("nnz", [1, 3, 4, 5, 31, 32, 33, 63, 64, 65, 129, 148 * 16 * 128 + 1])  # the last: tiles of 64 entries
 def test_entry_counts(pkg, handle, device, nnz):
     rng = np.random.default_rng(nnz)
