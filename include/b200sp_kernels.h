@@ -243,7 +243,8 @@ int b200sp_spmm_stream_error(void);
 int b200sp_spmm_stream_error_clear(void);
 /* For tests of that path: later row-stream launches wait at most wait_cycles SM clocks on a copy barrier
  * (0 = the default, about a second) and expect extra_tx bytes more than they copy on every barrier, so that with
- * extra_tx > 0 every wait runs out: the kernel must set the flag, stop writing C and return.  (0, 0) restores the
+ * extra_tx > 0 every wait runs out: the kernel must set the flag, stop writing C and return.  The int8 kernel for the
+ * tensor cores takes both as well; it sums its part of C entry by entry then and sets no flag.  (0, 0) restores the
  * normal behaviour.  Not thread-safe; nothing faults or hangs in either setting. */
 void b200sp_spmm_stream_wait_test(long long wait_cycles, unsigned extra_tx);
 

@@ -14,7 +14,8 @@
 // and the cluster has met, 12 for the megabyte every SM fetches from L2 (52 of the 62 bytes per clock and SM that L2 delivers), 3 to write C.
 // Writing the rows of A straight into the swizzled tiles, by every CTA for itself, took 68 us (some hundred
 // instructions per row and step), tiles by cp.async, which wants a proxy fence before every step, 28 us.
-// Every wait is bounded, as in the row-stream kernel: one that runs out raises gStreamError, and C is not written.
+// Every wait is bounded, as in the row-stream kernel.  After one that ran out the CTA sums its part of C entry by entry, straight from
+// A and B: no output is lost, and none comes from shared or tensor memory that a copy or a product may still be writing.
 #pragma once
 
 constexpr int kTcRows = 128;                // rows of a CTA: the lanes of tensor memory
@@ -166,6 +167,15 @@ __device__ __forceinline__ void TcExpandRow(const TcArgs &a, int row, int from, 
     __syncwarp();
 }
 
+// One element of A * B, entry by entry.
+__device__ __forceinline__ int32_t TcSum(const TcArgs &a, int row, int col)
+{
+    int32_t sum = 0;
+    for (int p = a.rowPtr[row]; p < a.rowPtr[row + 1]; ++p)
+        sum += (int32_t)a.val[p] * (int32_t)a.B[(long long)a.colInd[p] * a.ldb + col];
+    return sum;
+}
+
 __global__ void __launch_bounds__(kTcThreads, 1) SpmmInt8TensorKernel(const TcArgs a, const __grid_constant__ CUtensorMap mapA,
                                                                       const __grid_constant__ CUtensorMap mapB)
 {
@@ -252,14 +262,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) SpmmInt8TensorKernel(const TcAr
     __syncwarp();
     if (!MbarWait(&sDone, 0, 4 * a.waitCycles)) failed = true;  // longer than the waits above may take one after the other
     failed = __syncthreads_or(failed) != 0;
+    const int32_t alpha = a.sc.Alpha(), beta = a.sc.Beta();
+    const int live = min(a.cols, a.n - n0);  // columns
     if (failed && tid == 0) {
-        atomicExch(&gStreamError, 1);
         for (int c = asked > kTcStages ? asked - kTcStages : 0; c < asked; ++c)  // copies on their way: a bounded chance to land
             (void)MbarWait(sFull + c % kTcStages, (uint32_t)(c / kTcStages) & 1u, a.waitCycles);
     }
     if (!failed) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int32_t alpha = a.sc.Alpha(), beta = a.sc.Beta();
         // The sums go through shared memory (the stages are done with), so that rows of C are written whole.
         const int quarter = warp & 3;  // a warp reads the lanes of tensor memory that are its rank modulo four
         int32_t *const sSums = reinterpret_cast<int32_t *>(tiles);
@@ -271,18 +281,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) SpmmInt8TensorKernel(const TcAr
             for (int i = 0; i < 4; ++i) to[i] = make_int4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
         }
         __syncthreads();
-        const int live = min(a.cols, a.n - n0);  // columns
         const bool plain = alpha == 1 && beta == 0;
         for (int r = warp; r < kTcRows && row0 + r < a.m; r += kTcWarps) {
             const int row = row0 + r;
             int32_t *const sums = sSums + r * kTcPitch;
             if (odd >> (r / kTcWarps) & 1) {
-                for (int j = lane; j < live; j += 32) {
-                    int32_t sum = 0;
-                    for (int p = a.rowPtr[row]; p < a.rowPtr[row + 1]; ++p)
-                        sum += (int32_t)a.val[p] * (int32_t)a.B[(long long)a.colInd[p] * a.ldb + n0 + j];
-                    sums[j] = sum;
-                }
+                for (int j = lane; j < live; j += 32) sums[j] = TcSum(a, row, n0 + j);
                 __syncwarp();
             }
             if (a.cCol != 1) continue;
@@ -315,6 +319,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) SpmmInt8TensorKernel(const TcAr
                     int32_t *const at = out + (row0 + r) * a.cRow;
                     *at = Finish<int32_t>(sSums[r * kTcPitch + j], alpha, beta, at);
                 }
+            }
+        }
+    } else {
+        for (int r = warp; r < kTcRows && row0 + r < a.m; r += kTcWarps) {
+            for (int j = lane; j < live; j += 32) {
+                int32_t *const at = a.C + (row0 + r) * a.cRow + (n0 + j) * a.cCol;
+                *at = Finish<int32_t>(TcSum(a, row0 + r, n0 + j), alpha, beta, at);
             }
         }
     }

@@ -1434,7 +1434,7 @@ constexpr long long kStreamWaitCycles = 1ll << 31;           // SM clocks (about
 long long gHostStreamWaitCycles = kStreamWaitCycles;
 unsigned gHostStreamExtraTx = 0;
 
-__device__ int gStreamError;  // set when a wait ran out (never observed; the kernel then stops writing C)
+__device__ int gStreamError;  // set when a wait of the row-stream kernel ran out (never observed; it then stops writing C)
 
 __device__ __forceinline__ uint32_t SmemAddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void MbarInit(uint64_t *bar, int count)
@@ -2109,9 +2109,11 @@ bool ByteTiles(EncodeTiled encode, const void *at, long long rows, long long col
                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// dense: DenseBytes(m, k), 16-byte aligned
-int LaunchInt8Tensor(const FastArgs<int8_t, int32_t> &f, const b200spSpmmShape *sh, unsigned char *dense, cudaStream_t stream)
+// dense: DenseBytes(m, k), 16-byte aligned.  False, with nothing launched, where tensor maps or the shared memory are not to be had;
+// else *error is the launches' status.
+bool LaunchInt8Tensor(const FastArgs<int8_t, int32_t> &f, const b200spSpmmShape *sh, unsigned char *dense, cudaStream_t stream, int *error)
 {
+    *error = 0;
     static const EncodeTiled encode = [] {
         void *fn = nullptr;
         cudaDriverEntryPointQueryResult found{};
@@ -2120,11 +2122,12 @@ int LaunchInt8Tensor(const FastArgs<int8_t, int32_t> &f, const b200spSpmmShape *
     }();
     static std::atomic<bool> allowed[64] = {};  // per device: the kernel may use kTcSmem bytes of shared memory
     int dev = 0;
-    if (encode == nullptr) return (int)cudaErrorNotSupported;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
+    if (encode == nullptr || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     if (!allowed[dev].load(std::memory_order_relaxed)) {
-        const cudaError_t e = cudaFuncSetAttribute(SpmmInt8TensorKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
-        if (e != cudaSuccess) return (int)e;
+        if (cudaFuncSetAttribute(SpmmInt8TensorKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
         allowed[dev].store(true, std::memory_order_relaxed);
     }
     const long long denseCols = DenseCols(sh->k);
@@ -2157,7 +2160,7 @@ int LaunchInt8Tensor(const FastArgs<int8_t, int32_t> &f, const b200spSpmmShape *
     CUtensorMap mapA, mapB;
     if (!ByteTiles(encode, dense, sh->m, denseCols, denseCols, kTcDepth, &mapA) ||
         !ByteTiles(encode, f.B, sh->k, f.nB, f.ldb, t.cols, &mapB))
-        return (int)cudaErrorInvalidValue;
+        return false;
     for (; t.firstCol < t.n; t.firstCol += cluster * t.cols) {  // a launch for every 512 or 1024 columns
         const int left = t.n - t.firstCol;
         t.colTiles = left < cluster * t.cols ? (left + t.cols - 1) / t.cols : cluster;
@@ -2175,10 +2178,10 @@ int LaunchInt8Tensor(const FastArgs<int8_t, int32_t> &f, const b200spSpmmShape *
         cfg.attrs = attr;
         cfg.numAttrs = 2;
         b200sp_note_launches(1);
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, SpmmInt8TensorKernel, t, mapA, mapB);
-        if (e != cudaSuccess) return (int)e;
+        *error = (int)cudaLaunchKernelEx(&cfg, SpmmInt8TensorKernel, t, mapA, mapB);
+        if (*error != 0) break;
     }
-    return 0;
+    return true;
 }
 
 template <typename ValT, typename OutT>
@@ -2301,9 +2304,11 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
         return err;
     };
     if constexpr (kInt8) {
-        if (OnTensorCores(sh, plan))
-            return LaunchInt8Tensor(a, sh, reinterpret_cast<unsigned char *>(p + L.total + ExtraBytes(sh, 1) - DenseBytes(sh->m, sh->k)),
-                                    stream);
+        if (OnTensorCores(sh, plan)) {
+            auto *dense = reinterpret_cast<unsigned char *>(p + L.total + ExtraBytes(sh, 1) - DenseBytes(sh->m, sh->k));
+            int error = 0;
+            if (LaunchInt8Tensor(a, sh, dense, stream, &error)) return error;
+        }
         if (lanes_ <= 4) {  // 16 to 64 entries of a row are in flight as it is
             a.rowLimit = kLongRow;
             midUnits = 0;

@@ -95,18 +95,24 @@ def test_second_stream(pkg, handle, device):
     other.close()
 
 
-def test_wait_that_runs_out(pkg, handle, device):
-    """As in the row-stream kernel's test: a few bytes more expected than are copied, two milliseconds to wait for them."""
+@pytest.mark.parametrize("order,n", [("col", 150), ("row", 256), ("row", 150)])  # rows of 16-byte pieces: from 96 M products on
+def test_wait_that_runs_out(pkg, handle, device, order, n):
+    """A few bytes more expected than are copied, two milliseconds to wait for them: C is whole all the same, entry by entry."""
     L = pkg.lib()
     L.b200sp_spmm_stream_wait_test.argtypes = [ctypes.c_longlong, ctypes.c_uint]
     L.b200sp_spmm_stream_wait_test.restype = None
-    p = Product(pkg, handle, device, np.random.default_rng(9), 1500, 600, 150, 270, "col")
-    assert L.b200sp_spmm_stream_error() == 0
+    p = Product(pkg, handle, device, np.random.default_rng(9), 1500, 600, n, 270, order)
+    start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
     try:
         L.b200sp_spmm_stream_wait_test(1 << 22, 16)
-        assert np.array_equal(p.run(1, 0), p.C)  # nothing written
-        assert L.b200sp_spmm_stream_error() == 1
+        start.record()
+        got = p.run(3, -2)
+        end.record()
+        end.synchronize()
     finally:
         L.b200sp_spmm_stream_wait_test(0, 0)
-    assert L.b200sp_spmm_stream_error_clear() == 0
-    assert np.array_equal(p.run(1, 0), p.want(1, 0))
+    assert start.elapsed_time(end) > 1.0  # it did wait
+    assert np.array_equal(got, p.want(3, -2))
+    assert L.b200sp_spmm_stream_error() == 0
+    p.dC.values.copy_(torch.from_numpy(np.ascontiguousarray(p.C if order == "row" else p.C.T)))
+    assert np.array_equal(p.run(3, -2), p.want(3, -2))
