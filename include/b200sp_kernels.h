@@ -183,39 +183,51 @@ typedef struct b200spSpmmShape {
     int32_t block_units; /* from b200sp_spmm_analyze_blocks: units of the column-block path, 0 = not in use */
     int32_t long_rows;  /* from b200sp_spmm_analyze_blocks: rows the analysis listed as long */
     int64_t repack_bytes; /* bytes of the plan buffer beyond b200sp_spmm_plan_bytes that copies of the operands may use
-                           * (b200sp_spmm_repack_bytes), 0 = none */
+                           * (b200sp_spmm_repack_bytes or b200sp_spmm_operand_bytes), 0 = none */
     int32_t mid_units;  /* from b200sp_spmm_analyze_units; 0 = rows of up to 1024 entries are all treated alike */
-    int32_t ascending;  /* from b200sp_spmm_columns_ascend */
-    int64_t longest_row; /* from b200sp_spmm_analyze_units: entries of the longest row that is neither cut nor listed */
 } b200spSpmmShape;
+
+/* What the analysis may find out beyond that.  Callers of the functions without it lose speed, nothing else. */
+typedef struct b200spSpmmFound {
+    int64_t longest_row; /* from b200sp_spmm_analyze_rows: entries of the longest row that is neither cut nor listed, 0 = not known */
+    int32_t ascending;   /* from b200sp_spmm_columns_ascend */
+} b200spSpmmFound;
 
 /* Bytes of workspace for the SpMM analysis + long-row partial sums. */
 size_t b200sp_spmm_plan_bytes(int64_t rows, int64_t nnz, int64_t n);
 
-/* Bytes wanted after the plan: for a copy of B in rows the kernels can read with 16-byte loads, unless B lies in
- * such rows already or is read too seldom for a copy to pay, and for the rows of a dense int8 A written out for the tensor
- * cores.  Without them (shape.repack_bytes smaller) the product runs a slower kernel.  Only sizes and layouts are read. */
+/* Bytes wanted after the plan for a copy of B in rows the kernels can read with 16-byte loads: 0 when B lies in
+ * such rows already, or when it is read too seldom for a copy to pay.  Without them (shape.repack_bytes smaller) the
+ * product runs a slower kernel that takes any layout.  Only the sizes and the layout of B are read. */
 size_t b200sp_spmm_repack_bytes(const b200spSpmmShape *shape, int val_type);
+/* The same, and room for the rows of a dense int8 A written out for the tensor cores (at most 4 GB). */
+size_t b200sp_spmm_operand_bytes(const b200spSpmmShape *shape, int val_type);
 
-/* 1 if b200sp_spmm_launch with this shape (room for a copy in shape.repack_bytes) and plan copies B or A behind the plan.  Its
+/* 1 if b200sp_spmm_launch with this shape (room for a copy in shape.repack_bytes) and plan copies B behind the plan.  Two
  * launches then belong together: products that share the plan must not overlap, nor be enqueued by two threads at once. */
 int b200sp_spmm_copies(const b200spSpmmShape *shape, int val_type, int32_t segments, const void *plan);
-
-/* After b200sp_spmm_analyze_units: *ascending = 1 if this is an int8 product for the tensor cores (by its sizes) and the
- * columns of every row of A ascend without repetition; synchronises `stream` to say so.  0, without a launch, otherwise. */
-int b200sp_spmm_columns_ascend(const int32_t *row_ptr, const int32_t *col_ind, const b200spSpmmShape *shape, int val_type,
-                               void *plan, size_t plan_bytes, int32_t *ascending, void *stream);
+/* The same for b200sp_spmm_launch_found, which may write A out as well. */
+int b200sp_spmm_copies_found(const b200spSpmmShape *shape, const b200spSpmmFound *found, int val_type, int32_t segments,
+                             const void *plan);
 
 /* Analysis pass: finds rows too long for one warp, cuts them into segments and writes
  * the segment table into `plan`, and lists the rows that are better summed apart from
  * their neighbours.  This call synchronises `stream` once to read back the two counts,
- * returned in *segments and *mid_units, and the entries of the longest other row. */
+ * returned in *segments and *mid_units. */
 int b200sp_spmm_analyze_units(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,
-                              size_t plan_bytes, int32_t *segments, int32_t *mid_units, int32_t *longest_row,
-                              void *stream);
+                              size_t plan_bytes, int32_t *segments, int32_t *mid_units, void *stream);
 /* The same without the second count. */
 int b200sp_spmm_analyze(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,
                         size_t plan_bytes, int32_t *segments, void *stream);
+/* The same with both counts; found (may be NULL) is set to the longest row and to columns not known to ascend. */
+int b200sp_spmm_analyze_rows(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,
+                             size_t plan_bytes, int32_t *segments, int32_t *mid_units, b200spSpmmFound *found,
+                             void *stream);
+
+/* After b200sp_spmm_analyze_rows: found->ascending = 1 if this is an int8 product for the tensor cores (by its sizes) and the
+ * columns of every row of A ascend without repetition; synchronises `stream` to say so.  0, without a launch, otherwise. */
+int b200sp_spmm_columns_ascend(const int32_t *row_ptr, const int32_t *col_ind, const b200spSpmmShape *shape, int val_type,
+                               void *plan, size_t plan_bytes, b200spSpmmFound *found, void *stream);
 
 /* Second, optional analysis pass, after b200sp_spmm_analyze on the same plan: decides whether the long rows are
  * better summed block by block of B (B much larger than L2, rows of B of `b_row_bytes` >= 512 bytes, every long
@@ -232,6 +244,10 @@ int b200sp_spmm_analyze_blocks(const int32_t *row_ptr, const int32_t *col_ind, i
 int b200sp_spmm_launch(const int32_t *row_ptr, const int32_t *col_ind, const void *val, const void *B, void *C,
                        const b200spSpmmShape *shape, const b200spScalars *scalars, int val_type, int out_type,
                        void *plan, int32_t segments, void *stream);
+/* The same with what the analysis found beside (NULL = nothing). */
+int b200sp_spmm_launch_found(const int32_t *row_ptr, const int32_t *col_ind, const void *val, const void *B, void *C,
+                             const b200spSpmmShape *shape, const b200spSpmmFound *found, const b200spScalars *scalars,
+                             int val_type, int out_type, void *plan, int32_t segments, void *stream);
 
 /* 1 when a wait on the copy engine ran out of time in the SpMM row-stream kernel since the library was
  * loaded or the flag was last cleared (the affected rows of C were then not written), 0 when none did, -1 when

@@ -59,10 +59,9 @@ struct ActivePlan {
     int64_t n = 0;         // SpMM only: dense column count the partial-sum area was sized for
     int32_t segments = 0;  // SpMM only: long-row segments found by the analysis
     int32_t midUnits = 0;  // SpMM only: shorter rows summed apart from their neighbours
-    int32_t longestRow = 0;  // SpMM only: entries of the longest of the others
     int32_t blockUnits = 0;  // SpMM only: units of the column-block path for the long rows (0 = summed by segments)
     int32_t longRows = 0;   // SpMM only: rows listed as long
-    bool ascending = false;  // SpMM only: columns found to ascend, which an int8 product on the tensor cores wants
+    b200spSpmmFound spmmFound{};  // SpMM only: the longest of the other rows; whether the columns ascend, as an int8 product on the tensor cores wants
     const void *colInd = nullptr;  // SpMM: the cut table of the column blocks was made, the order found, for these column indices
     int32_t valueType = -1;        // ... and for B rows of this element type
     int64_t repackBytes = 0;       // SpMM only: bytes after the plan that copies of B and A may use ...

@@ -49,9 +49,8 @@ aclsparseStatus_t ValidateSpmm(aclsparseOperation_t opA, aclsparseOperation_t op
 
 struct Analysis {
     int32_t segments = 0, midUnits = 0, blockUnits = 0, longRows = 0;
-    int32_t longestRow = 0;
+    b200spSpmmFound more{};
     int64_t repackBytes = 0;
-    bool ascending = false;
 };
 
 size_t ElemBytes(aclDataType t)
@@ -69,8 +68,8 @@ aclsparseStatus_t Analyse(const aclsparseSpMatDescr *A, int64_t n, void *buffer,
     const size_t bytes = b200sp_spmm_plan_bytes(A->rows, A->nnz, n);
     // Whatever plan this buffer held is overwritten now; an active plan that is not re-recorded below goes stale.
     (void)b200sp::NoteBufferWrite(buffer);
-    const int rc = b200sp_spmm_analyze_units(static_cast<const int32_t *>(A->offsets), A->rows, A->nnz, n, buffer, bytes,
-                                             segments, &out->midUnits, &out->longestRow, stream);
+    const int rc = b200sp_spmm_analyze_rows(static_cast<const int32_t *>(A->offsets), A->rows, A->nnz, n, buffer, bytes,
+                                            segments, &out->midUnits, &out->more, stream);
     if (rc != 0) {
         B200SP_LOGE("aclsparseSpMM: analysis failed (cuda error %d)", rc);
         return ACL_SPARSE_STATUS_EXECUTION_FAILED;
@@ -110,14 +109,14 @@ size_t RepackBytes(const aclsparseSpMatDescr *A, const aclsparseDnMatDescr *B, c
                    aclsparseOperation_t opB)
 {
     const b200spSpmmShape sh = ShapeOf(A, B, C, opB);
-    return b200sp_spmm_repack_bytes(&sh, b200sp::KernelTypeOf(A->valueType));
+    return b200sp_spmm_operand_bytes(&sh, b200sp::KernelTypeOf(A->valueType));
 }
 
 bool PlanMatches(const ActivePlan &p, const void *buffer, const aclsparseSpMatDescr *A, int64_t n)
 {
     return p.kind == PlanKind::kSpmm && p.buffer == buffer && p.rowPtr == A->offsets && p.rows == A->rows &&
            p.nnz == A->nnz && p.n == n && p.generation == b200sp::BufferGeneration(buffer) &&
-           ((p.blockUnits == 0 && !p.ascending) || (p.colInd == A->indices && p.valueType == (int32_t)A->valueType));
+           ((p.blockUnits == 0 && p.spmmFound.ascending == 0) || (p.colInd == A->indices && p.valueType == (int32_t)A->valueType));
 }
 
 // Whether this product may copy B (or a dense int8 A) into the analysed buffer.  Products that share a buffer may otherwise overlap (as long
@@ -196,7 +195,6 @@ aclsparseStatus_t aclsparseSpMMPreprocess(aclsparseHandle_t handle, aclsparseOpe
     p.n = matC->cols;
     p.segments = found.segments;
     p.midUnits = found.midUnits;
-    p.longestRow = found.longestRow;
     p.blockUnits = found.blockUnits;
     p.longRows = found.longRows;
     p.colInd = matA->indices;
@@ -206,20 +204,18 @@ aclsparseStatus_t aclsparseSpMMPreprocess(aclsparseHandle_t handle, aclsparseOpe
     const int64_t repack = (int64_t)RepackBytes(matA, matB, matC, opB);
     p.repackBytes = matA->spmmSizedN == matC->cols && matA->spmmSizedRepack >= repack ? repack : 0;
     if (p.repackBytes > 0) {
-        b200spSpmmShape sh = ShapeOf(matA, matB, matC, opB);
-        sh.longest_row = found.longestRow;
-        int32_t ascending = 0;
+        const b200spSpmmShape sh = ShapeOf(matA, matB, matC, opB);
         const int rc = b200sp_spmm_columns_ascend(static_cast<const int32_t *>(matA->offsets),
                                                   static_cast<const int32_t *>(matA->indices), &sh,
                                                   b200sp::KernelTypeOf(matA->valueType), buffer,
-                                                  b200sp_spmm_plan_bytes(matA->rows, matA->nnz, matC->cols), &ascending,
+                                                  b200sp_spmm_plan_bytes(matA->rows, matA->nnz, matC->cols), &found.more,
                                                   handle != nullptr ? handle->stream : nullptr);
         if (rc != 0) {
             B200SP_LOGE("aclsparseSpMMPreprocess: analysis of the columns failed (cuda error %d)", rc);
             return ACL_SPARSE_STATUS_EXECUTION_FAILED;
         }
-        p.ascending = ascending != 0;
     }
+    p.spmmFound = found.more;
     p.generation = b200sp::BufferGeneration(buffer);
     matA->active = p;
     return ACL_SPARSE_STATUS_SUCCESS;
@@ -241,11 +237,10 @@ aclsparseStatus_t aclsparseSpMM(aclsparseHandle_t handle, aclsparseOperation_t o
     if (PlanMatches(matA->active, buffer, matA, matC->cols)) {
         found.segments = matA->active.segments;
         found.midUnits = matA->active.midUnits;
-        found.longestRow = matA->active.longestRow;
         found.blockUnits = matA->active.blockUnits;
         found.longRows = matA->active.longRows;
         found.repackBytes = matA->active.repackBytes;
-        found.ascending = matA->active.ascending;
+        found.more = matA->active.spmmFound;
     } else {
         // Not the active buffer: analyse into it now, as the reference rebuilds its tiling
         // in place (spmm_host.cpp:310-321).  This path synchronises the stream once.
@@ -267,23 +262,22 @@ aclsparseStatus_t aclsparseSpMM(aclsparseHandle_t handle, aclsparseOperation_t o
 
     b200spSpmmShape sh = ShapeOf(matA, matB, matC, opB);
     sh.repack_bytes = found.repackBytes;
-    sh.ascending = found.ascending ? 1 : 0;
     sh.mid_units = found.midUnits;
-    sh.longest_row = found.longestRow;
     sh.block_units = found.blockUnits;
     sh.long_rows = found.longRows;
     sh.kahan = (alg == ACL_SPARSE_SPMM_CSR_FP32_HIGH_PRECISION_ALG && matA->valueType == ACL_FLOAT) ? 1 : 0;
 
     // The copy and the kernel that reads it are two launches: nothing of another thread may come between them.
     std::unique_lock<std::mutex> copying(matA->copyMutex, std::defer_lock);
-    if (sh.repack_bytes > 0 && b200sp_spmm_copies(&sh, b200sp::KernelTypeOf(matA->valueType), found.segments, buffer) != 0) {
+    if (sh.repack_bytes > 0 &&
+        b200sp_spmm_copies_found(&sh, &found.more, b200sp::KernelTypeOf(matA->valueType), found.segments, buffer) != 0) {
         copying.lock();
         if (!MayCopy(matA->active, handle->stream)) sh.repack_bytes = 0;
     }
-    const int rc = b200sp_spmm_launch(static_cast<const int32_t *>(matA->offsets),
-                                      static_cast<const int32_t *>(matA->indices), matA->values, matB->values,
-                                      matC->values, &sh, &sc, b200sp::KernelTypeOf(matA->valueType),
-                                      b200sp::KernelTypeOf(matC->valueType), buffer, found.segments, handle->stream);
+    const int rc = b200sp_spmm_launch_found(static_cast<const int32_t *>(matA->offsets),
+                                            static_cast<const int32_t *>(matA->indices), matA->values, matB->values,
+                                            matC->values, &sh, &found.more, &sc, b200sp::KernelTypeOf(matA->valueType),
+                                            b200sp::KernelTypeOf(matC->valueType), buffer, found.segments, handle->stream);
     if (rc != 0) {
         B200SP_LOGE("aclsparseSpMM: kernel launch failed (cuda error %d)", rc);
         return ACL_SPARSE_STATUS_EXECUTION_FAILED;

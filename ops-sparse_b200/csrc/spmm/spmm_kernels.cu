@@ -2048,14 +2048,14 @@ bool TensorPays(const b200spSpmmShape *sh, long long longest)
 //     types from 8 entries on (f16, N = 32: ragged rows of 6 17.3 and 18.0, of 9 23.1 and 22.6, of 40 74 and 61; 4000 power-law rows of 16 22.6 and 27.1,
 //     150,000 of 24 74 and 72), in fp32, whose rows of B take twice as long, from 64 (N = 16: ragged rows of 5 13.6 and 15.1, of 16 25.7
 //     and 26.5, of 100 130 and 125).
-bool OrderPays(const b200spSpmmShape *sh, int valBytes, int ctaRows, int genRows)
+bool OrderPays(const b200spSpmmShape *sh, long long longest, int valBytes, int ctaRows, int genRows)
 {
-    if (4 * sh->longest_row * sh->m < 5 * sh->nnz) return false;
+    if (4 * longest * sh->m < 5 * sh->nnz) return false;
     if (sh->order_c != 0) return genRows == 32;
     const long long sms = b200sp_sm_count();
     const bool many = sh->m >= (ctaRows < 16 ? 6 : 4) * 32 * sms;
     if (ctaRows < 32) return many && sh->nnz >= 1700 * sms;
-    return sh->nnz >= (valBytes == 2 ? 8 : 64) * sh->m && (sh->longest_row * sh->m <= 4 * sh->nnz || (many && sh->nnz >= 24 * sh->m));
+    return sh->nnz >= (valBytes == 2 ? 8 : 64) * sh->m && (longest * sh->m <= 4 * sh->nnz || (many && sh->nnz >= 24 * sh->m));
 }
 
 // What an analysed buffer holds after the plan: a copy of B (from a multiple of 256 bytes) and an A written out.
@@ -2067,9 +2067,10 @@ size_t ExtraBytes(const b200spSpmmShape *sh, int valBytes)
 }
 
 // Whether an int8 product with this much room, on rows found to ascend, writes A out.
-bool OnTensorCores(const b200spSpmmShape *sh, const void *plan)
+bool OnTensorCores(const b200spSpmmShape *sh, const b200spSpmmFound &found, const void *plan)
 {
-    return sh->ascending != 0 && TensorPays(sh, sh->longest_row) && sh->repack_bytes >= (int64_t)ExtraBytes(sh, 1) && plan != nullptr && Aligned16(plan);
+    return found.ascending != 0 && TensorPays(sh, found.longest_row) && sh->repack_bytes >= (int64_t)ExtraBytes(sh, 1) && plan != nullptr &&
+           Aligned16(plan);
 }
 
 template <typename ValT, typename OutT>
@@ -2186,7 +2187,7 @@ bool LaunchInt8Tensor(const FastArgs<int8_t, int32_t> &f, const b200spSpmmShape 
 
 template <typename ValT, typename OutT>
 int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, const void *B, void *C,
-                const b200spSpmmShape *sh, const b200spScalars *s, void *plan, int32_t segments,
+                const b200spSpmmShape *sh, const b200spSpmmFound &found, const b200spScalars *s, void *plan, int32_t segments,
                 cudaStream_t stream)
 {
     constexpr bool kInt8 = std::is_same_v<ValT, int8_t>;
@@ -2269,7 +2270,7 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             const long long unitCtas = kInt8 ? units : ((long long)units * a.slices + kWarps - 1) / kWarps;
             a.unitCtas = (int)unitCtas;
             a.genRows = sh->m < 2ll * Shape::kGenRows * b200sp_sm_count() ? Shape::kCtaRows : Shape::kGenRows;
-            const bool byLength = Shape::kMayOrder && rowCtas && OrderPays(sh, (int)sizeof(ValT), Shape::kCtaRows, a.genRows);
+            const bool byLength = Shape::kMayOrder && rowCtas && OrderPays(sh, found.longest_row, (int)sizeof(ValT), Shape::kCtaRows, a.genRows);
             const long long rows = a.splitRows ? 1 : byLength ? 32 : sh->order_c == 0 ? Shape::kCtaRows : a.genRows;
             const long long grid = unitCtas + (rowCtas ? (sh->m + rows - 1) / rows : 0);
             if (grid == 0) return;
@@ -2304,7 +2305,7 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
         return err;
     };
     if constexpr (kInt8) {
-        if (OnTensorCores(sh, plan)) {
+        if (OnTensorCores(sh, found, plan)) {
             auto *dense = reinterpret_cast<unsigned char *>(p + L.total + ExtraBytes(sh, 1) - DenseBytes(sh->m, sh->k));
             int error = 0;
             if (LaunchInt8Tensor(a, sh, dense, stream, &error)) return error;
@@ -2415,23 +2416,33 @@ void b200sp_spmm_stream_wait_test(long long wait_cycles, unsigned extra_tx)
 
 size_t b200sp_spmm_plan_bytes(int64_t rows, int64_t nnz, int64_t n) { return LayoutFor(rows, nnz, n).total; }
 
+static int BytesOf(int val_type) { return val_type == B200SP_F32 ? 4 : val_type == B200SP_I8 ? 1 : 2; }
+
 size_t b200sp_spmm_repack_bytes(const b200spSpmmShape *shape, int val_type)
 {
-    const int bytes = val_type == B200SP_F32 ? 4 : val_type == B200SP_I8 ? 1 : 2;
-    return ExtraBytes(shape, bytes);
+    return WorthRepacking(shape, BytesOf(val_type)) ? RepackBytes(shape, BytesOf(val_type)) : 0;
 }
+
+size_t b200sp_spmm_operand_bytes(const b200spSpmmShape *shape, int val_type) { return ExtraBytes(shape, BytesOf(val_type)); }
 
 int b200sp_spmm_copies(const b200spSpmmShape *shape, int val_type, int32_t segments, const void *plan)
 {
-    const int bytes = val_type == B200SP_F32 ? 4 : val_type == B200SP_I8 ? 1 : 2;
-    return Copies(shape, bytes, segments, plan) || (bytes == 1 && OnTensorCores(shape, plan)) ? 1 : 0;
+    return b200sp_spmm_copies_found(shape, nullptr, val_type, segments, plan);
+}
+
+int b200sp_spmm_copies_found(const b200spSpmmShape *shape, const b200spSpmmFound *found, int val_type, int32_t segments,
+                             const void *plan)
+{
+    const bool dense = found != nullptr && val_type == B200SP_I8 && OnTensorCores(shape, *found, plan);
+    return dense || Copies(shape, BytesOf(val_type), segments, plan) ? 1 : 0;
 }
 
 int b200sp_spmm_columns_ascend(const int32_t *row_ptr, const int32_t *col_ind, const b200spSpmmShape *shape, int val_type,
-                               void *plan, size_t plan_bytes, int32_t *ascending, void *stream)
+                               void *plan, size_t plan_bytes, b200spSpmmFound *found, void *stream)
 {
-    *ascending = 0;
-    if (val_type != B200SP_I8 || !TensorPays(shape, shape->longest_row) || col_ind == nullptr) return 0;
+    if (found == nullptr) return (int)cudaErrorInvalidValue;
+    found->ascending = 0;
+    if (val_type != B200SP_I8 || !TensorPays(shape, found->longest_row) || col_ind == nullptr) return 0;
     const PlanLayout L = LayoutFor(shape->m, shape->nnz, shape->n);
     if (plan == nullptr || plan_bytes < L.total) return (int)cudaErrorInvalidValue;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -2444,23 +2455,29 @@ int b200sp_spmm_columns_ascend(const int32_t *row_ptr, const int32_t *col_ind, c
     if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, flag, sizeof(bad), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return (int)e;
-    *ascending = bad == 0;
+    found->ascending = bad == 0;
     return 0;
 }
 
 int b200sp_spmm_analyze(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,
                         size_t plan_bytes, int32_t *segments, void *stream)
 {
-    int32_t mid = 0, longest = 0;
-    return b200sp_spmm_analyze_units(row_ptr, rows, nnz, n, plan, plan_bytes, segments, &mid, &longest, stream);
+    int32_t mid = 0;
+    return b200sp_spmm_analyze_rows(row_ptr, rows, nnz, n, plan, plan_bytes, segments, &mid, nullptr, stream);
 }
 
 int b200sp_spmm_analyze_units(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,
-                              size_t plan_bytes, int32_t *segments, int32_t *mid_units, int32_t *longest_row,
-                              void *stream)
+                              size_t plan_bytes, int32_t *segments, int32_t *mid_units, void *stream)
+{
+    return b200sp_spmm_analyze_rows(row_ptr, rows, nnz, n, plan, plan_bytes, segments, mid_units, nullptr, stream);
+}
+
+int b200sp_spmm_analyze_rows(const int32_t *row_ptr, int64_t rows, int64_t nnz, int64_t n, void *plan,
+                             size_t plan_bytes, int32_t *segments, int32_t *mid_units, b200spSpmmFound *found,
+                             void *stream)
 {
     const PlanLayout L = LayoutFor(rows, nnz, n);
-    if (plan == nullptr || segments == nullptr || plan_bytes < L.total) return (int)cudaErrorInvalidValue;
+    if (plan == nullptr || segments == nullptr || mid_units == nullptr || plan_bytes < L.total) return (int)cudaErrorInvalidValue;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     char *p = static_cast<char *>(plan);
     cudaError_t e = cudaMemsetAsync(p + L.offCounts, 0, 256, st);
@@ -2484,7 +2501,7 @@ int b200sp_spmm_analyze_units(const int32_t *row_ptr, int64_t rows, int64_t nnz,
     if (e != cudaSuccess) return (int)e;
     *segments = counts[1];
     *mid_units = counts[5];
-    *longest_row = counts[7];
+    if (found != nullptr) *found = {counts[7], 0};
     return 0;
 }
 
@@ -2541,9 +2558,17 @@ int b200sp_spmm_launch(const int32_t *row_ptr, const int32_t *col_ind, const voi
                        const b200spSpmmShape *shape, const b200spScalars *scalars, int val_type, int out_type,
                        void *plan, int32_t segments, void *stream)
 {
+    return b200sp_spmm_launch_found(row_ptr, col_ind, val, B, C, shape, nullptr, scalars, val_type, out_type, plan, segments, stream);
+}
+
+int b200sp_spmm_launch_found(const int32_t *row_ptr, const int32_t *col_ind, const void *val, const void *B, void *C,
+                             const b200spSpmmShape *shape, const b200spSpmmFound *found, const b200spScalars *scalars,
+                             int val_type, int out_type, void *plan, int32_t segments, void *stream)
+{
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     auto go = [&]<typename ValT, typename OutT>() {
-        return LaunchTyped<ValT, OutT>(row_ptr, col_ind, val, B, C, shape, scalars, plan, segments, st);
+        return LaunchTyped<ValT, OutT>(row_ptr, col_ind, val, B, C, shape, found != nullptr ? *found : b200spSpmmFound{}, scalars, plan, segments,
+                                         st);
     };
     if (val_type == B200SP_F32 && out_type == B200SP_F32) return go.template operator()<float, float>();
     if (val_type == B200SP_F16 && out_type == B200SP_F16) return go.template operator()<__half, __half>();
