@@ -19,16 +19,20 @@ def pattern(rng, m, k, entries):
 
 
 class Product:
-    def __init__(self, pkg, handle, device, rng, m, k, n, entries, order, align=0):
+    def __init__(self, pkg, handle, device, rng, m, k, n, entries, order, align=0, ascending=True, pad=0):
         from ops_sparse_b200 import api
         self.handle, self.shape, self.order = handle, (m, k, n), order
         self.rp, self.ci, self.val = pattern(rng, m, k, entries)
         self.B = rng.integers(-128, 128, (k, n)).astype(np.int8)
         self.C = rng.integers(-1000, 1000, (m, n)).astype(np.int32)
+        if not ascending:  # one row of many
+            r = m // 2
+            self.ci[self.rp[r]:self.rp[r + 1]] = self.ci[self.rp[r]:self.rp[r + 1]][::-1]
         dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(device)
         stored = (lambda a: a) if order == "row" else (lambda a: a.T)
         self.A = api.CsrMatrix(dev(self.rp), dev(self.ci), dev(self.val), m, k)
-        self.dB = api.DnMat(dev(stored(self.B)), k, n, n if order == "row" else k, order)
+        padded = np.pad(stored(self.B), ((0, 0), (0, pad)), constant_values=99)  # rows (columns) of B further apart
+        self.dB = api.DnMat(dev(padded), k, n, (n if order == "row" else k) + pad, order)
         self.dC = api.DnMat(dev(stored(self.C)), m, n, n if order == "row" else m, order)
         size = api.spmm_buffer_size(handle, self.A, self.dB, self.dC)
         assert size >= m * k  # room for A as it is written out
@@ -77,6 +81,58 @@ def test_rows_that_ascend_no_longer(pkg, handle, device):
             row[:] = row[::-1]
     p.A.col_ind.copy_(torch.from_numpy(ci))
     assert np.array_equal(p.run(2, -1), p.want(2, -1, ci))
+
+
+@pytest.mark.parametrize("m,k,n,entries,order", [(9001, 100, 64, 60, "col"), (9001, 127, 40, 80, "col"), (9401, 64, 256, 50, "row")])
+def test_fewer_columns_than_a_step(pkg, handle, device, m, k, n, entries, order):
+    p = Product(pkg, handle, device, np.random.default_rng(k), m, k, n, entries, order)
+    assert np.array_equal(p.run(2, -1), p.want(2, -1))
+
+
+@pytest.mark.parametrize("m,k,n,entries,order,pad", [(2000, 512, 256, 256, "row", 16), (2000, 512, 256, 256, "row", 5), (1500, 600, 150, 270, "col", 3)])
+def test_wider_leading_dimension(pkg, handle, device, m, k, n, entries, order, pad):
+    p = Product(pkg, handle, device, np.random.default_rng(pad), m, k, n, entries, order, pad=pad)
+    assert np.array_equal(p.run(2, -1), p.want(2, -1))
+
+
+def test_rows_that_never_ascended(pkg, handle, device):
+    """The analysis finds a row that descends: lane groups."""
+    p = Product(pkg, handle, device, np.random.default_rng(12), 1500, 600, 150, 270, "col", ascending=False)
+    assert np.array_equal(p.run(2, -1), p.want(2, -1))
+
+
+def test_replaced_column_array(pkg, handle, device):
+    """Other arrays drop the plan, which is analysed again in the product or, for the products after it, by a Preprocess."""
+    p = Product(pkg, handle, device, np.random.default_rng(13), 1500, 600, 150, 270, "col")
+    columns = p.A.col_ind.clone()
+    p.A.col_ind.zero_()
+    L = pkg.lib()
+    pointer = lambda t: ctypes.c_void_p(t.data_ptr())
+    pkg.check(L.aclsparseCsrSetPointers(p.A.raw, pointer(p.A.row_ptr), pointer(columns), pointer(p.A.values)), "aclsparseCsrSetPointers")
+    assert np.array_equal(p.run(1, 0), p.want(1, 0))
+    pkg.check(L.aclsparseSpMMPreprocess(p.handle.raw, 0, 0, None, p.A.raw, p.dB.raw, None, p.dC.raw, pkg.ACL_INT32, 0, pointer(p.buffer)),
+              "aclsparseSpMMPreprocess")
+    assert np.array_equal(p.run(3, 0), p.want(3, 0))
+
+
+def test_in_a_graph(pkg, handle, device):
+    """A captured product leaves the shared buffer alone and gives the same, also with other values and beside later ones."""
+    from ops_sparse_b200 import api
+    p = Product(pkg, handle, device, np.random.default_rng(14), 1500, 600, 150, 270, "col")
+    assert np.array_equal(p.run(1, 0), p.want(1, 0))
+    record = torch.cuda.Stream()
+    recorder = api.Handle(record)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=record):
+        api.spmm(recorder, p.A, p.dB, p.dC, 3, 0, buffer=p.buffer)
+    p.val = np.roll(p.val, 1)
+    p.A.values.copy_(torch.from_numpy(p.val))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(p.dC.values.cpu().numpy().reshape(150, 1500).T, p.want(3, 0))
+    assert np.array_equal(p.run(5, 0), p.want(5, 0))
+    del graph
+    recorder.close()
 
 
 @pytest.mark.parametrize("align", [4, 8])
