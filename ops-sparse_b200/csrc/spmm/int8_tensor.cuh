@@ -10,8 +10,9 @@
 //     row that fails is marked, and its outputs are summed entry by entry instead.
 //   - Tiles of 128 columns of A and as many rows of B come through seven stages of shared memory by TMA, requested by one thread; another
 //     starts the products.
-// 4096 x 4096 at one tenth, N = 512: 69 us with the lane groups of SpmmFastKernel, 24 here: some 6 us until the rows are written out
-// and the cluster has met, 12 for the megabyte every SM fetches from L2 (52 of the 62 bytes per clock and SM that L2 delivers), 3 to write C.
+// 4096 x 4096 at one tenth, N = 512: 69 us with the lane groups of SpmmFastKernel, 24 here: every SM fetches 1.1 MB from L2, at least 9.4 us
+// at the 62 bytes per clock that it gets; before that the rows are written out and the cluster meets, and the tensor cores
+// work in 19 % of the cycles.
 // Writing the rows of A straight into the swizzled tiles, by every CTA for itself, took 68 us (some hundred
 // instructions per row and step), tiles by cp.async, which wants a proxy fence before every step, 28 us.
 // Every wait is bounded, as in the row-stream kernel.  After one that ran out the CTA sums its part of C entry by entry, straight from
