@@ -457,7 +457,7 @@ struct FastArgs {
     int unitCtas;         // CTAs at the front of the grid that work on them
     int slices;           // fp: warps a unit takes, 64 bytes of a B row each
     int splitRows;        // int8 only: a CTA per row
-    int genRows;          // column-major C: rows of a CTA
+    int genRows;          // rows of a CTA: column-major C, and int8 as a loop
     const LongRow *longRows;
     const SegEntry *segs, *segsEnd;
     int32_t *counters;    // [long row][ArrivalsPerRow]
@@ -971,6 +971,9 @@ template <typename ValT, int kLanes> struct FastShape {
     static constexpr int kGenRows = kCtaRows > kFit ? kCtaRows : kFit;
     // 32 rows of a CTA may be taken in order of their lengths (int8 loses: 44.6 and 50.3 us on 55,686 rows of 0 to 232 entries, N = 16).
     static constexpr bool kMayOrder = !std::is_same_v<ValT, int8_t> && kCtaRows <= 32 && kGroup < 32;
+    // int8 instead: the pass over the rows compiled as a loop, although it has one turn.  More of a row's loads are then asked for together, at
+    // some spilled registers: faster where the SMs wait for single rows, slower where they have warps enough (see launchFast).
+    static constexpr bool kMayLoop = std::is_same_v<ValT, int8_t> && (kLanes == 2 || kLanes == 4);
 };
 
 enum { kPlain, kAnyC, kAnyCWords };
@@ -993,7 +996,8 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
     constexpr int kTileWords = kGenC ? (Shape::kGenRows * kTileStride > kThreads * E ? Shape::kGenRows * kTileStride : kThreads * E) : 0;
     __shared__ __align__(16) Acc sBuf[kWarps * kWarpWords > kTileWords ? kWarps * kWarpWords : kTileWords];
     __shared__ unsigned char sSkip[kGenC ? Shape::kGenRows : 1];
-    __shared__ unsigned char sOrder[kOrdered ? kWarps : 1][32];
+    constexpr bool kByLength = kOrdered && !kInt8;
+    __shared__ unsigned char sOrder[kByLength ? kWarps : 1][32];
     __shared__ int sLast;
 
     b200sp::WaitForPrevious();
@@ -1026,9 +1030,9 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
         // ---- one lane group per row ----
         constexpr int kChunk = kInt8 ? Group8<kLanes>::kChunk : Chunk<kLanes>::kChunk;
         const bool rowsRun = kGenC && a.cCol != 1;  // column-major C
-        const int blockRows = kOrdered ? 32 : rowsRun ? a.genRows : Shape::kCtaRows;
+        const int blockRows = kByLength ? 32 : rowsRun || kOrdered ? a.genRows : Shape::kCtaRows;
         const long long row0 = (long long)(blockIdx.x - a.unitCtas) * blockRows;
-        if constexpr (kOrdered) {  // sOrder[i]: the row with the i-th most entries (every warp has its own copy: no barrier)
+        if constexpr (kByLength) {  // sOrder[i]: the row with the i-th most entries (every warp has its own copy: no barrier)
             int len = row0 + lane < a.m ? a.rowPtr[row0 + lane + 1] - a.rowPtr[row0 + lane] : 0;
             if (len > a.rowLimit) len = 0;
             const int key = len << 5 | (31 - lane);
@@ -1042,7 +1046,7 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
 #pragma unroll 1
             for (int pass = 0; pass < blockRows; pass += Shape::kCtaRows) {
                 int rowIn = pass + warp * kRowsPerWarp + lane / kGroup;
-                if constexpr (kOrdered) {
+                if constexpr (kByLength) {
                     // every other pass the other way round: the warp with the longest rows of one has the shortest of the next
                     const int turn = pass & Shape::kCtaRows ? kWarps - 1 - warp : warp;
                     rowIn = sOrder[warp][pass + turn * kRowsPerWarp + lane / kGroup];
@@ -1114,7 +1118,7 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
 #pragma unroll
                             for (int i = lane; i < kRowsPerWarp * kTileCols; i += 32) {
                                 const int g = i / kTileCols, c = colT + i % kTileCols;
-                                const int r = kOrdered ? __shfl_sync(0xffffffffu, rowIn, g * kGroup) : warp * kRowsPerWarp + g;
+                                const int r = kByLength ? __shfl_sync(0xffffffffu, rowIn, g * kGroup) : warp * kRowsPerWarp + g;
                                 if (c < a.n && !(skipped >> (g * kGroup) & 1)) storeOne(row0 + r, c, sWarp[i]);
                             }
                         }
@@ -2271,6 +2275,12 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             a.unitCtas = (int)unitCtas;
             a.genRows = sh->m < 2ll * Shape::kGenRows * b200sp_sm_count() ? Shape::kCtaRows : Shape::kGenRows;
             const bool byLength = Shape::kMayOrder && rowCtas && OrderPays(sh, found.longest_row, (int)sizeof(ValT), Shape::kCtaRows, a.genRows);
+            // int8, where rows above four times the mean (which units would take in other types) or few rows are waited for; N = 32 / 64, us
+            // straight and as a loop: power-law rows, 20,000 of 30, 50 / 81 and 40 / 67, 100,000 of 40, 84 / 131 and 76 / 117; 3,000
+            // ragged rows of 60, 9.8 / 15.4 and 8.3 / 12.7; but 100,000 equal rows of 40, 31 / 42 and 35 / 43, 20,000 of 150, a CTA each, 57 / 58 and 59 / 61.
+            const bool loop = Shape::kMayLoop && cPlain && rowCtas &&
+                              (sh->mid_units > 0 || (!a.splitRows && sh->m < 4ll * Shape::kCtaRows * b200sp_sm_count()));
+            if (loop) a.genRows = Shape::kCtaRows;
             const long long rows = a.splitRows ? 1 : byLength ? 32 : sh->order_c == 0 ? Shape::kCtaRows : a.genRows;
             const long long grid = unitCtas + (rowCtas ? (sh->m + rows - 1) / rows : 0);
             if (grid == 0) return;
@@ -2284,6 +2294,8 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             auto pickOrder = [&]<bool kKahan>() {
                 if constexpr (Shape::kMayOrder)
                     if (byLength) return pick.template operator()<kKahan, true>();
+                if constexpr (Shape::kMayLoop)
+                    if (loop) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kPlain, true>);
                 pick.template operator()<kKahan, false>();
             };
             if constexpr (std::is_same_v<ValT, float>) {
