@@ -173,3 +173,18 @@ def test_uneven_rows_in_order_of_their_lengths(handle, device, oracle, vt, ot, m
     else:
         gold = oracle.spmm_16(rp, ci, val, B, C, 1.5, -0.5, vt, ot)
     assert np.array_equal(got.view(np.uint8), np.asarray(gold).reshape(m, n).view(np.uint8))
+
+
+@pytest.mark.parametrize("n", [17, 32, 48, 64])
+@pytest.mark.parametrize("m,outliers", [(500, 0), (9471, 0), (9473, 0), (9473, 7)])  # few rows; enough; enough with a few long ones
+def test_int8_rows_that_are_waited_for(handle, device, oracle, m, n, outliers):
+    rng = np.random.default_rng(m + n)
+    k = 2000
+    lengths = rng.integers(0, 40, m)
+    lengths[rng.integers(0, m, outliers)] = 900
+    rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    ci = rng.integers(0, k, rp[-1]).astype(np.int32)
+    val, B = (rng.integers(-128, 128, shape).astype(np.int8) for shape in (rp[-1], (k, n)))
+    C = rng.integers(-1000, 1000, (m, n)).astype(np.int32)
+    got = run_spmm(handle, device, rp, ci, val, "i8", B, C, "i32", m, k, n, n, n, 3, -2)
+    assert np.array_equal(got.reshape(-1), oracle.spmm_i8(m, n, rp, ci, val, B, n, True, False, C, n, True, 3, -2))
