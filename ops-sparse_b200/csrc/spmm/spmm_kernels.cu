@@ -96,7 +96,7 @@ inline int MidRowLimit(int64_t rows, int64_t nnz, int64_t n)
 struct PlanLayout {
     int64_t capLong, capSegs, capBlockSlots;
     size_t offCounts, offLong, offSegs, offCounters, offPartials;
-    size_t offCuts, offRowSlots, offBlockCounters, offBlockMeta, offUnits, offBlockPartials, total;
+    size_t offCuts, offRowSlots, offBlockMeta, offUnits, offBlockPartials, total;
 };
 
 inline int64_t ArrivalsPerRow(int64_t n) { return (n + 15) / 16; }  // slices of 64 bytes in a B row, at most
@@ -120,8 +120,7 @@ inline PlanLayout LayoutFor(int64_t rows, int64_t nnz, int64_t n)
     L.capBlockSlots = n >= 128 ? nnz / 128 + kMaxBlocks : 0;
     const bool on = L.capBlockSlots > 0;
     L.offRowSlots = AlignUp(L.offCuts + (on ? sizeof(int32_t) * (size_t)L.capLong * (kMaxBlocks + 1) : 0), 256);
-    L.offBlockCounters = AlignUp(L.offRowSlots + (on ? sizeof(int2) * (size_t)L.capLong : 0), 256);
-    L.offBlockMeta = AlignUp(L.offBlockCounters + (on ? sizeof(int32_t) * (size_t)L.capLong : 0), 256);
+    L.offBlockMeta = AlignUp(L.offRowSlots + (on ? sizeof(int2) * (size_t)L.capLong : 0), 256);
     L.offUnits = AlignUp(L.offBlockMeta + (on ? sizeof(int32_t) * 3 * kMaxBlocks : 0), 256);
     L.offBlockPartials = AlignUp(L.offUnits + (on ? sizeof(int4) * (size_t)L.capBlockSlots : 0), 256);
     L.total = AlignUp(L.offBlockPartials + sizeof(float) * (size_t)L.capBlockSlots * (size_t)n, 256);
@@ -312,8 +311,8 @@ __global__ void __launch_bounds__(256) SpmmCutBlocksKernel(const int32_t *__rest
                                                            const int32_t *__restrict__ colInd,
                                                            const LongRow *__restrict__ longRows, int nLong,
                                                            long long blockCols, int blocks, int32_t *__restrict__ cuts,
-                                                           int2 *__restrict__ rowSlots, int32_t *__restrict__ counters,
-                                                           int32_t *__restrict__ blockUnits, int32_t *unsorted)
+                                                           int2 *__restrict__ rowSlots, int32_t *__restrict__ blockUnits,
+                                                           int32_t *unsorted)
 {
     const int lane = threadIdx.x & 31;
     const int li = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -347,10 +346,7 @@ __global__ void __launch_bounds__(256) SpmmCutBlocksKernel(const int32_t *__rest
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) units += __shfl_xor_sync(0xffffffffu, units, off);
-    if (lane == 0) {
-        rowSlots[li] = make_int2(0, units);
-        counters[li] = 0;
-    }
+    if (lane == 0) rowSlots[li] = make_int2(0, units);
 }
 
 // One CTA: first slot of every long row (exclusive scan of the rows' unit counts, in list order) and first unit
@@ -1250,14 +1246,15 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
 // is being worked on, every long row gathers from the same few megabytes, which the first touch brings into L2
 // and the evict-last policy of the B loads keeps there.  Pieces are cut into units of at most kUnitNnz entries so
 // that all units take about the same time and the grid stays inside a window of one or two blocks.  A warp sums
-// one unit in CSR order into one partial row; the warp that completes a row adds its partial rows in column
-// order (fixed order: the same bits every run) and applies the epilogue.
+// one unit in CSR order into one partial row; SpmmLongSumKernel then adds the partial rows of a row in column order (fixed
+// order: the same bits every run) and applies the epilogue.
 struct BlockArgs {
     int nUnits;
     const BlockUnit *units;   // ordered by column block
     const int2 *rowSlots;     // [long row] {first partial slot, slots}
-    int32_t *counters;        // [long row] arrivals
+    int nLong;
     float *partials;          // [slot][n]
+    unsigned long long share; // of the units in the row-stream kernel's grid, times 2^32
 };
 
 // Packed fp32 arithmetic of sm_100: one instruction, two fused multiply-adds.  The long rows are not bound to the
@@ -1303,106 +1300,6 @@ template <> struct FusedRow<__half> {
     }
 };
 
-// Measured on the 2 M x 2 M graph matrix with 512-byte rows of B (2,767 long rows, 14.0 M entries), this kernel
-// alone, microseconds: the segment CTAs it replaces 1067 (DRAM-bound: every B row fetched from DRAM);
-// blocks of 16 / 24 / 32 / 48 / 64 MB 848 / 729 / 727 / 715 / 725; units of 128 / 256 / 512 entries
-// 851 / 727 / 813; 2 / 4 / 8 / 16 rows in flight per lane 879 / 727 / 752 / 857; a fixed grid of 4 CTAs per SM
-// walking the units with a stride 1739 (its warps drift apart and the window of blocks in use outgrows L2).
-// At 714 us: 1.9 GB of DRAM traffic instead of 7.2, issue slots 54 % busy (28 warp instructions per B row).
-#ifndef B200SP_SPMM_BLOCK_BATCH
-#define B200SP_SPMM_BLOCK_BATCH 4   // B rows a lane has in flight
-#endif
-#ifndef B200SP_SPMM_BLOCK_CTAS
-#define B200SP_SPMM_BLOCK_CTAS 0    // > 0: a fixed grid of that many CTAs per SM walks the units; 0: a CTA per 4 units
-#endif
-
-template <typename ValT, typename OutT>
-__global__ void __launch_bounds__(kThreads) SpmmLongBlockKernel(const FastArgs<ValT, OutT> a, const BlockArgs b)
-{
-    constexpr int E = Pack<ValT>::kElems;
-    constexpr int kTileCols = 32 * E;
-    constexpr int kBatch = B200SP_SPMM_BLOCK_BATCH;
-    const int lane = threadIdx.x & 31;
-    const long long warpsTotal = (long long)gridDim.x * kWarps;
-    for (long long unit = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5); unit < b.nUnits; unit += warpsTotal) {
-        const int4 raw = __ldg(reinterpret_cast<const int4 *>(b.units) + unit);
-        const int s = raw.x, e = raw.y, li = raw.z, slot = raw.w;
-        float *partial = b.partials + (long long)slot * a.n;
-        for (int col0 = 0; col0 < a.n; col0 += kTileCols) {
-            const int col = col0 + lane * E;
-            const bool colLive = col < a.n;
-            const ValT *Bs = a.B + (colLive ? col : 0);
-            float2 acc[E / 2];
-#pragma unroll
-            for (int i = 0; i < E / 2; ++i) acc[i] = make_float2(0.0f, 0.0f);
-            for (int p0 = s; p0 < e; p0 += 32) {
-                const int cnt = e - p0 < 32 ? e - p0 : 32;
-                int myCol = 0;
-                float myVal = 0.0f;
-                if (lane < cnt) {
-                    myCol = __ldcs(a.colInd + p0 + lane);
-                    myVal = ToF32(__ldcs(a.val + p0 + lane));
-                }
-                int j = 0;
-                for (; j + kBatch <= cnt; j += kBatch) {  // cnt is the same in every lane
-                    uint4 q[kBatch];
-                    float v[kBatch];
-#pragma unroll
-                    for (int u = 0; u < kBatch; ++u) {
-                        const int c = __shfl_sync(0xffffffffu, myCol, j + u);
-                        v[u] = __shfl_sync(0xffffffffu, myVal, j + u);
-                        q[u] = LoadB16(Bs + (long long)c * a.ldb);
-                    }
-#pragma unroll
-                    for (int u = 0; u < kBatch; ++u) FusedRow<ValT>::Add(q[u], v[u], acc);
-                }
-                for (; j < cnt; ++j) {
-                    const int c = __shfl_sync(0xffffffffu, myCol, j);
-                    const float v = __shfl_sync(0xffffffffu, myVal, j);
-                    const uint4 q = LoadB16(Bs + (long long)c * a.ldb);
-                    FusedRow<ValT>::Add(q, v, acc);
-                }
-            }
-            if (colLive) {
-#pragma unroll
-                for (int i = 0; i < E / 2; i += 2)
-                    __stcg(reinterpret_cast<float4 *>(partial + col + 2 * i),
-                           make_float4(acc[i].x, acc[i].y, acc[i + 1].x, acc[i + 1].y));
-            }
-        }
-        // Arrival: the unit that comes last adds the row's partial rows in slot (= column) order.
-        const int2 rs = __ldg(b.rowSlots + li);
-        __threadfence();
-        int last = 0;
-        if (lane == 0) {
-            const int old = atomicAdd(b.counters + li, 1);
-            last = old == rs.y - 1;
-            if (last) b.counters[li] = 0;  // ready for the next launch
-        }
-        last = __shfl_sync(0xffffffffu, last, 0);
-        if (!last) continue;
-        __threadfence();
-        const float alpha = a.sc.Alpha();
-        const float beta = a.sc.Beta();
-        const int row = a.longRows[li].row;
-        const float *first = b.partials + (long long)rs.x * a.n;
-        for (int col = lane * E; col < a.n; col += kTileCols) {
-            float tot[E];
-#pragma unroll
-            for (int i = 0; i < E; ++i) tot[i] = 0.0f;
-#pragma unroll 4
-            for (int sl = 0; sl < rs.y; ++sl) {
-#pragma unroll
-                for (int i = 0; i < E; i += 4) {
-                    const float4 v = __ldcg(reinterpret_cast<const float4 *>(first + (long long)sl * a.n + col + i));
-                    tot[i] += v.x; tot[i + 1] += v.y; tot[i + 2] += v.z; tot[i + 3] += v.w;
-                }
-            }
-            StoreRowSlice<OutT, E>(a.C + (long long)row * a.ldc + col, tot, alpha, beta);
-        }
-    }
-}
-
 // ---------------------------------------------------------------- row-stream path
 
 // For B rows of 512 or 1024 bytes.  A warp owns 32 consecutive rows of A and walks their
@@ -1414,11 +1311,15 @@ __global__ void __launch_bounds__(kThreads) SpmmLongBlockKernel(const FastArgs<V
 // Every lane owns kRowBytes / 32 bytes of the row; each output keeps one fp32 accumulator
 // that takes its products in CSR order with separate multiply and add, as in the kernel above,
 // so the results are the same bits.  Rows above kLongRow entries are left to the segment CTAs
-// of SpmmFastKernel.
+// of SpmmFastKernel or, by column blocks of B, are units of the same grid.
 // Measured on the 2 M x 2 M graph matrix with 512-byte rows (ms per product, segment CTAs included):
 // 3 buffers x 16 rows x 4 warps per CTA 5.28; 2 x 16 x 4 3.97; 2 x 8 x 4 3.29; 2 x 4 x 4 3.38;
 // 2 x 8 x 2 2.99; 2 x 8 x 1 2.91.  Less shared memory per warp means more warps per SM, and
 // one warp per CTA gives the memory of a finished warp back at once.
+// The rows are bound by DRAM, the units of long rows by the latency of L2.  One kernel after the other (two streams do not
+// help: the first takes every SM until its last CTA has started) they took 2610 us; in one grid, units spread evenly
+// among the rows, 2300, with 13.5 GB of DRAM traffic either way (2070 us at the copy rate).  The entries are looked up 32 at a time,
+// not one batch at a time, which is 120 of those 310 us: issue slots 57 % busy.
 #ifndef B200SP_SPMM_STREAM_BUFFERS
 #define B200SP_SPMM_STREAM_BUFFERS 2
 #endif
@@ -1471,29 +1372,145 @@ __device__ __forceinline__ bool MbarWait(uint64_t *bar, uint32_t parity, long lo
     }
     return true;
 }
-// One row: global -> shared through the copy engine; both addresses 16-byte aligned, bytes a multiple of 16.
-// B200SP_SPMM_STREAM_B_POLICY 1: the copies carry an L2 evict-first policy, so that the rows this kernel streams
-// through L2 once do not displace the block of B rows that SpmmLongBlockKernel, running beside it, keeps there.
-// Measured: the row-stream kernel alone slows from 1.90 to 2.01 ms with it and the pair gains nothing; off.
-#ifndef B200SP_SPMM_STREAM_B_POLICY
-#define B200SP_SPMM_STREAM_B_POLICY 0
-#endif
-__device__ __forceinline__ void BulkLoadRow(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
+// One row: global -> shared through the copy engine; both addresses 16-byte aligned, bytes a multiple of 16.  `once`: with an
+// L2 evict-first policy, so that rows that stream through L2 do not displace the block of B that units of long rows in the
+// same grid gather from (2 M x 2 M graph matrix, 512-byte rows: 2290 us with it, 2390 without; by itself the row stream
+// loses 5 % to it).
+__device__ __forceinline__ void BulkLoadRow(void *dst, const void *src, uint32_t bytes, uint64_t *bar, bool once)
 {
-#if B200SP_SPMM_STREAM_B_POLICY == 1
-    uint64_t pol;
-    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
-            SmemAddr(dst)),
-        "l"(src), "r"(bytes), "r"(SmemAddr(bar)), "l"(pol)
-        : "memory");
-#else
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     SmemAddr(dst)),
-                 "l"(src), "r"(bytes), "r"(SmemAddr(bar))
-                 : "memory");
-#endif
+    if (once) {
+        uint64_t pol;
+        asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
+                SmemAddr(dst)),
+            "l"(src), "r"(bytes), "r"(SmemAddr(bar)), "l"(pol)
+            : "memory");
+    } else {
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         SmemAddr(dst)),
+                     "l"(src), "r"(bytes), "r"(SmemAddr(bar))
+                     : "memory");
+    }
+}
+
+// What bounds a unit is the latency of its gathers from L2: the rows of B come through shared memory by cp.async, three
+// requests of four rows in flight per warp, and a lane reads back what it asked for itself.  (The copy engine starts a row
+// per 20 clocks and SM, which the ordinary rows of the same grid use up; plain loads into registers leave a warp without
+// any in flight while it sums.)
+constexpr int kUnitRows = 4;      // rows of B per request
+constexpr int kUnitRequests = 4;  // three in flight, one being summed
+constexpr int kUnitTile = 512;    // bytes of a row of B that a warp takes at a time
+constexpr int kUnitRing = kUnitRequests * kUnitRows * kUnitTile;
+
+// One unit by one warp; ring: kUnitRing bytes of shared memory of its own.
+template <typename ValT, typename OutT>
+__device__ __forceinline__ void LongUnit(const FastArgs<ValT, OutT> &a, const BlockArgs &b, int unit, unsigned char *ring)
+{
+    constexpr int E = Pack<ValT>::kElems;
+    constexpr int kTileCols = kUnitTile / (int)sizeof(ValT);
+    constexpr int kChunkRequests = 32 / kUnitRows;
+    static_assert(kUnitTile == 32 * 16 && kUnitRequests - 1 <= kChunkRequests && kChunkRequests % kUnitRequests == 0);
+    const int lane = threadIdx.x & 31;
+    const int4 raw = __ldg(reinterpret_cast<const int4 *>(b.units) + unit);
+    const int s = raw.x, total = raw.y - raw.x, slot = raw.w;
+    float *partial = b.partials + (long long)slot * a.n;
+    unsigned char *const mine = ring + lane * 16;
+    uint64_t policy;
+    asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(policy));
+    for (int col0 = 0; col0 < a.n; col0 += kTileCols) {
+        const int col = col0 + lane * E;
+        const bool colLive = col < a.n;
+        const ValT *Bs = a.B + (colLive ? col : 0);
+        float2 acc[E / 2];
+#pragma unroll
+        for (int i = 0; i < E / 2; ++i) acc[i] = make_float2(0.0f, 0.0f);
+        // 32 entries at a time, one per lane (column -1 after the last), and the next 32 on their way
+        auto fetch = [&](int first, int &c, float &v) {
+            c = -1;
+            v = 0.0f;
+            if (first + lane < total) {
+                c = __ldcs(a.colInd + s + first + lane);
+                v = ToF32(__ldcs(a.val + s + first + lane));
+            }
+        };
+        int colNow, colNext;
+        float valNow, valNext;
+        fetch(0, colNow, valNow);
+        fetch(32, colNext, valNext);
+        auto request = [&](int from, int first, int place) {  // past the last entry: zeros, nothing is read
+#pragma unroll
+            for (int u = 0; u < kUnitRows; ++u) {
+                const int c = __shfl_sync(0xffffffffu, from, first + u);
+                asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;" ::"r"(
+                                 SmemAddr(mine + (place * kUnitRows + u) * kUnitTile)),
+                             "l"(Bs + (long long)(c < 0 ? 0 : c) * a.ldb), "r"(c < 0 ? 0 : 16), "l"(policy)
+                             : "memory");
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+#pragma unroll
+        for (int r = 0; r < kUnitRequests - 1; ++r) request(colNow, kUnitRows * r, r);
+        for (int done = 0; done < total; done += 32) {
+#pragma unroll
+            for (int r = 0; r < kChunkRequests; ++r) {
+                if (done + kUnitRows * r >= total) break;
+                constexpr int kAhead = kUnitRequests - 1;
+                __syncwarp();  // the place asked for next has been read
+                if (r + kAhead < kChunkRequests) request(colNow, kUnitRows * (r + kAhead), (r + kAhead) % kUnitRequests);
+                else request(colNext, kUnitRows * (r + kAhead - kChunkRequests), (r + kAhead) % kUnitRequests);
+                asm volatile("cp.async.wait_group %0;" ::"n"(kAhead) : "memory");
+#pragma unroll
+                for (int u = 0; u < kUnitRows; ++u) {
+                    const float v = __shfl_sync(0xffffffffu, valNow, kUnitRows * r + u);
+                    const uint4 q = *reinterpret_cast<const uint4 *>(mine + ((r % kUnitRequests) * kUnitRows + u) * kUnitTile);
+                    FusedRow<ValT>::Add(q, v, acc);
+                }
+            }
+            colNow = colNext;
+            valNow = valNext;
+            fetch(done + 64, colNext, valNext);
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+        if (colLive) {
+#pragma unroll
+            for (int i = 0; i < E / 2; i += 2)
+                __stcg(reinterpret_cast<float4 *>(partial + col + 2 * i),
+                       make_float4(acc[i].x, acc[i].y, acc[i + 1].x, acc[i + 1].y));
+        }
+    }
+}
+
+// The units alone, beside SpmmFastKernel for the other rows.  A CTA per kBlockWarps units, in their order: a fixed grid that walks them with a
+// stride drifts apart until the window of blocks in use outgrows L2 (1739 us instead of 714).
+constexpr int kBlockWarps = 2;
+template <typename ValT, typename OutT>
+__global__ void __launch_bounds__(32 * kBlockWarps) SpmmLongBlockKernel(const FastArgs<ValT, OutT> a, const BlockArgs b)
+{
+    __shared__ __align__(16) unsigned char ring[kBlockWarps][kUnitRing];
+    const long long unit = (long long)blockIdx.x * kBlockWarps + (threadIdx.x >> 5);
+    if (unit < b.nUnits) LongUnit<ValT, OutT>(a, b, (int)unit, ring[threadIdx.x >> 5]);
+}
+
+// C of the long rows from their partial rows: a warp per 32 columns of a row, which are added up in slot (= column) order.
+template <typename OutT, typename ArgsT>
+__global__ void __launch_bounds__(256) SpmmLongSumKernel(const ArgsT a, const BlockArgs b)
+{
+    b200sp::WaitForPrevious();
+    const int slices = (a.n + 31) / 32;
+    const long long w = (long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+    if (w >= (long long)b.nLong * slices) return;
+    const int li = (int)(w / slices);
+    const int col = (int)(w % slices) * 32 + (threadIdx.x & 31);
+    if (col >= a.n) return;
+    const int2 rs = __ldg(b.rowSlots + li);
+    const float *at = b.partials + (long long)rs.x * a.n + col;
+    float tot = 0.0f;
+#pragma unroll 16
+    for (int sl = 0; sl < rs.y; ++sl) tot += __ldcs(at + (long long)sl * a.n);
+    OutT *dst = a.C + (long long)a.longRows[li].row * a.ldc + col;
+    *dst = Finish(tot, a.sc.Alpha(), a.sc.Beta(), dst);
 }
 
 template <int kBytes> struct LaneWords {  // kBytes of shared memory as 32-bit words
@@ -1571,7 +1588,7 @@ __device__ __forceinline__ void StoreSlice(OutT *dst, const float (&acc)[E], con
     if constexpr (kBytes % 16 == 0) {
 #pragma unroll
         for (int i = 0; i < kBytes / 16; ++i)
-            reinterpret_cast<uint4 *>(dst)[i] = reinterpret_cast<const uint4 *>(o)[i];
+            __stcs(reinterpret_cast<uint4 *>(dst) + i, reinterpret_cast<const uint4 *>(o)[i]);
     } else if constexpr (kBytes == 8) {
         *reinterpret_cast<uint2 *>(dst) = *reinterpret_cast<const uint2 *>(o);
     } else {
@@ -1588,6 +1605,7 @@ struct StreamArgs {
     const ValT *B;
     OutT *C;
     int m;
+    int warpRows;            // rows of A per warp, up to 32
     int rowLimit;
     long long ldb;
     long long ldc;
@@ -1605,7 +1623,8 @@ template <int kRowBytes> struct StreamShape {
 };
 
 template <typename ValT, typename OutT, int kRowBytes>
-__global__ void __launch_bounds__(kStreamThreads) SpmmRowStreamKernel(const StreamArgs<ValT, OutT> a)
+__global__ void __launch_bounds__(kStreamThreads) SpmmRowStreamKernel(const StreamArgs<ValT, OutT> a, const FastArgs<ValT, OutT> fa,
+                                                                      const BlockArgs ba)
 {
     using Shape = StreamShape<kRowBytes>;
     constexpr int kBatch = Shape::kBatch;
@@ -1613,9 +1632,16 @@ __global__ void __launch_bounds__(kStreamThreads) SpmmRowStreamKernel(const Stre
     constexpr int kWords = kLaneBytes / 4;
     constexpr int E = WordsToF32<ValT, kWords>::kElems;
     extern __shared__ __align__(128) unsigned char sRaw[];
+    static_assert(kStreamWarps == 1 && Shape::kCtaBytes >= kUnitRing, "a unit takes the place of a warp");
 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
+    // Units of long rows, spread evenly over the grid
+    const unsigned before = (unsigned)((blockIdx.x * ba.share) >> 32);
+    if ((unsigned)(((blockIdx.x + 1ull) * ba.share) >> 32) != before) {
+        LongUnit<ValT, OutT>(fa, ba, (int)before, sRaw);
+        return;
+    }
     unsigned char *base = sRaw + (size_t)warp * Shape::kWarpBytes;
     unsigned char *sData = base;                                                          // [buffers][kBatch][kRowBytes]
     float *sVal = reinterpret_cast<float *>(base + kStreamBuffers * kBatch * kRowBytes);  // [buffers][kBatch]
@@ -1631,14 +1657,14 @@ __global__ void __launch_bounds__(kStreamThreads) SpmmRowStreamKernel(const Stre
 
     const float alpha = a.sc.Alpha();
     const float beta = a.sc.Beta();
-    const long long r0 = ((long long)blockIdx.x * kStreamWarps + warp) * kStreamRows;
+    const long long r0 = ((blockIdx.x - before) * kStreamWarps + warp) * a.warpRows;
     if (r0 >= a.m) return;
 
     // This lane's row: bounds, length, and where its entries start in the warp's stream.
     const long long myRow = r0 + lane;
     int s = 0, len = 0;
     bool mine = false;
-    if (myRow < a.m) {
+    if (lane < a.warpRows && myRow < a.m) {
         s = a.rowPtr[myRow];
         len = a.rowPtr[myRow + 1] - s;
         mine = len <= a.rowLimit;  // longer rows are units
@@ -1670,12 +1696,13 @@ __global__ void __launch_bounds__(kStreamThreads) SpmmRowStreamKernel(const Stre
     const unsigned liveMask = __ballot_sync(0xffffffffu, len > 0);
 
     const int nBatches = (total + kBatch - 1) / kBatch;
-    // Entry q of the stream (held by lane q % kBatch of its batch): column, value, and which row it
-    // belongs to / whether it ends that row.
-    int eCol = 0, eMeta = 0;
-    float eVal = 0.0f;
-    auto fetchEntries = [&](int k) {
-        const int q = k * kBatch + lane;
+    // The stream's entries, 32 at a time, an entry per lane: column, value, and which row it belongs to / whether it ends
+    // that row.  The chunk in use, and the next one, on its way.
+    constexpr int kPerChunk = 32 / kBatch;
+    int eCol = 0, eMeta = 0, nCol = 0, nMeta = 0;
+    float eVal = 0.0f, nVal = 0.0f;
+    auto fetchChunk = [&](int chunk) {
+        const int q = chunk * 32 + lane;
         // last lane whose stream offset is <= q: the row that holds entry q
         int lo = 0;
 #pragma unroll
@@ -1687,33 +1714,37 @@ __global__ void __launch_bounds__(kStreamThreads) SpmmRowStreamKernel(const Stre
         const int sL = __shfl_sync(0xffffffffu, s, lo);
         const int offL = __shfl_sync(0xffffffffu, off, lo);
         const int lenL = __shfl_sync(0xffffffffu, len, lo);
-        if (lane < kBatch && q < total) {
+        if (q < total) {
             const int p = sL + (q - offL);
-            eCol = __ldcs(a.colInd + p);
-            eVal = ToF32(__ldcs(a.val + p));
-            eMeta = lo | ((q - offL == lenL - 1) ? 0x100 : 0);
+            nCol = __ldcs(a.colInd + p);
+            nVal = ToF32(__ldcs(a.val + p));
+            nMeta = lo | ((q - offL == lenL - 1) ? 0x100 : 0);
         }
     };
     auto issueBatch = [&](int k) {
+        if (k % kPerChunk == 0) {
+            eCol = nCol;
+            eVal = nVal;
+            eMeta = nMeta;
+            if ((k + kPerChunk) * kBatch < total) fetchChunk(k / kPerChunk + 1);
+        }
         const int buf = k % kStreamBuffers;
         const int live = total - k * kBatch < kBatch ? total - k * kBatch : kBatch;
         if (lane == 0) MbarExpectTx(sBar + buf, (uint32_t)live * kRowBytes + a.extraTx);
         __syncwarp();
-        if (lane < live) {
-            sVal[buf * kBatch + lane] = eVal;
-            sMeta[buf * kBatch + lane] = eMeta;
-            BulkLoadRow(sData + ((size_t)buf * kBatch + lane) * kRowBytes, a.B + (long long)eCol * a.ldb, kRowBytes,
-                        sBar + buf);
+        const int i = lane - (k % kPerChunk) * kBatch;
+        if (i >= 0 && i < live) {
+            sVal[buf * kBatch + i] = eVal;
+            sMeta[buf * kBatch + i] = eMeta;
+            BulkLoadRow(sData + ((size_t)buf * kBatch + i) * kRowBytes, a.B + (long long)eCol * a.ldb, kRowBytes, sBar + buf,
+                        ba.share != 0);
         }
     };
 
     // prologue: all but one buffer in flight
     const int ahead = kStreamBuffers - 1;
-    for (int k = 0; k < ahead && k < nBatches; ++k) {
-        fetchEntries(k);
-        issueBatch(k);
-    }
-    if (ahead < nBatches) fetchEntries(ahead);
+    fetchChunk(0);
+    for (int k = 0; k < ahead && k < nBatches; ++k) issueBatch(k);
 
     float acc[E], old[E];
 #pragma unroll
@@ -1723,8 +1754,7 @@ __global__ void __launch_bounds__(kStreamThreads) SpmmRowStreamKernel(const Stre
 
     int failedAt = -1;
     for (int k = 0; k < nBatches; ++k) {
-        if (k + ahead < nBatches) issueBatch(k + ahead);           // uses the entries fetched one trip ago
-        if (k + ahead + 1 < nBatches) fetchEntries(k + ahead + 1);  // lands while this batch is summed
+        if (k + ahead < nBatches) issueBatch(k + ahead);
         const int buf = k % kStreamBuffers;
         __syncwarp();
         if (!MbarWait(sBar + buf, (uint32_t)(k / kStreamBuffers) & 1u, a.waitCycles)) {
@@ -1915,7 +1945,7 @@ bool Aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0;
 // 128-bit loads and stay with SpmmFastKernel (256-byte rows, 64 per row of A: 1249 us against 265 us).
 
 template <typename ValT, typename OutT, int kRowBytes>
-int LaunchRowStream(const StreamArgs<ValT, OutT> &sa, cudaStream_t stream)
+int LaunchRowStream(const StreamArgs<ValT, OutT> &sa, const FastArgs<ValT, OutT> &fa, BlockArgs ba, cudaStream_t stream)
 {
     constexpr int kSmem = StreamShape<kRowBytes>::kCtaBytes;
     static bool configured[64] = {};  // per device: this instantiation uses kSmem bytes of dynamic shared memory
@@ -1927,9 +1957,10 @@ int LaunchRowStream(const StreamArgs<ValT, OutT> &sa, cudaStream_t stream)
         if (e != cudaSuccess) return (int)e;
         configured[dev] = true;
     }
-    const long long rowsPerBlock = (long long)kStreamWarps * kStreamRows;
-    const unsigned grid = (unsigned)((sa.m + rowsPerBlock - 1) / rowsPerBlock);
-    SpmmRowStreamKernel<ValT, OutT, kRowBytes><<<grid, kStreamThreads, kSmem, stream>>>(sa);
+    const unsigned grid = (unsigned)(((long long)sa.m + sa.warpRows - 1) / sa.warpRows);
+    const unsigned long long all = (unsigned long long)grid + (unsigned)ba.nUnits;
+    ba.share = (((unsigned long long)(unsigned)ba.nUnits << 32) + all - 1) / all;  // rounded up: the last CTA's count is nUnits
+    SpmmRowStreamKernel<ValT, OutT, kRowBytes><<<(unsigned)all, kStreamThreads, kSmem, stream>>>(sa, fa, ba);
     b200sp_note_launches(1);
     return (int)cudaGetLastError();
 }
@@ -2348,7 +2379,20 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
         // first and the other rows' kernel shares the SMs with them.
         b200sp::SideLanes *lanes = nullptr;
         cudaStream_t longStream = stream;
-        if ((stream_ && segments > 0) || byBlocks) {
+        BlockArgs ba{};
+        if (byBlocks) {
+            ba.nUnits = sh->block_units;
+            ba.nLong = sh->long_rows;
+            ba.units = reinterpret_cast<const BlockUnit *>(p + L.offUnits);
+            ba.rowSlots = reinterpret_cast<const int2 *>(p + L.offRowSlots);
+            ba.partials = reinterpret_cast<float *>(p + L.offBlockPartials);
+        }
+        auto sumLongRows = [&](cudaStream_t st) {
+            const long long warps = (long long)ba.nLong * ((sh->n + 31) / 32);
+            b200sp_note_launches(1);
+            return b200sp::LaunchChained(SpmmLongSumKernel<OutT, FastArgs<ValT, OutT>>, (unsigned)((warps + 7) / 8), 256, 0, st, a, ba);
+        };
+        if ((stream_ && segments > 0) || (byBlocks && !stream_)) {
             lanes = b200sp::GetSideLanes();
             if (lanes != nullptr) {
                 if (cudaEventRecord(lanes->fork, stream) != cudaSuccess ||
@@ -2357,16 +2401,10 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
                 longStream = lanes->stream[0];
             }
             if (byBlocks) {
-                BlockArgs ba{};
-                ba.nUnits = sh->block_units;
-                ba.units = reinterpret_cast<const BlockUnit *>(p + L.offUnits);
-                ba.rowSlots = reinterpret_cast<const int2 *>(p + L.offRowSlots);
-                ba.counters = reinterpret_cast<int32_t *>(p + L.offBlockCounters);
-                ba.partials = reinterpret_cast<float *>(p + L.offBlockPartials);
-                const unsigned grid = (unsigned)(((long long)ba.nUnits + kWarps - 1) / kWarps);
-                SpmmLongBlockKernel<ValT, OutT><<<grid, kThreads, 0, longStream>>>(a, ba);
+                const unsigned grid = (unsigned)(((long long)ba.nUnits + kBlockWarps - 1) / kBlockWarps);
+                SpmmLongBlockKernel<ValT, OutT><<<grid, 32 * kBlockWarps, 0, longStream>>>(a, ba);
                 b200sp_note_launches(1);
-                if (cudaGetLastError() != cudaSuccess) return (int)cudaErrorLaunchFailure;
+                if (cudaGetLastError() != cudaSuccess || sumLongRows(longStream) != cudaSuccess) return (int)cudaErrorLaunchFailure;
             } else if (lanes != nullptr) {
                 if (launchFast(segments, 0, false, longStream) != cudaSuccess) return (int)cudaErrorLaunchFailure;
                 segments = 0;
@@ -2383,15 +2421,17 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             sa.C = a.C;
             sa.m = a.m;
             sa.rowLimit = a.rowLimit;
+            sa.warpRows = kStreamRows;
             sa.ldb = a.ldb;
             sa.ldc = sh->ldc;
             sa.sc = a.sc;
             sa.negZeros = kNegZeros;
             sa.waitCycles = gHostStreamWaitCycles;
             sa.extraTx = gHostStreamExtraTx;
-            const int rc = rowBytes == 512 ? LaunchRowStream<ValT, OutT, 512>(sa, stream)
-                                           : LaunchRowStream<ValT, OutT, 1024>(sa, stream);
+            const int rc = rowBytes == 512 ? LaunchRowStream<ValT, OutT, 512>(sa, a, ba, stream)
+                                           : LaunchRowStream<ValT, OutT, 1024>(sa, a, ba, stream);
             if (rc != 0) return rc;
+            if (byBlocks && sumLongRows(stream) != cudaSuccess) return (int)cudaErrorLaunchFailure;
         }
         // What is left for SpmmFastKernel on the caller's stream: the segment CTAs unless they were forked (or
         // replaced by the column-block kernel), and the rows of up to kLongRow entries unless the row-stream
@@ -2551,7 +2591,7 @@ int b200sp_spmm_analyze_blocks(const int32_t *row_ptr, const int32_t *col_ind, i
     if (e != cudaSuccess) return (int)e;
     SpmmCutBlocksKernel<<<(unsigned)((nLong + 7) / 8), 256, 0, st>>>(
         row_ptr, col_ind, reinterpret_cast<const LongRow *>(p + L.offLong), nLong, blockCols, (int)blocks, cuts,
-        rowSlots, reinterpret_cast<int32_t *>(p + L.offBlockCounters), meta, countsDev + 3);
+        rowSlots, meta, countsDev + 3);
     SpmmBlockScanKernel<<<1, 1024, 0, st>>>(rowSlots, nLong, meta, (int)blocks, countsDev + 4);
     SpmmFillUnitsKernel<<<(unsigned)((nLong + 7) / 8), 256, 0, st>>>(
         cuts, rowSlots, nLong, (int)blocks, meta, reinterpret_cast<BlockUnit *>(p + L.offUnits),
