@@ -1302,7 +1302,7 @@ template <> struct FusedRow<__half> {
 
 // ---------------------------------------------------------------- row-stream path
 
-// For B rows of 512 or 1024 bytes.  A warp owns 32 consecutive rows of A and walks their
+// For B rows of 512 or 1024 bytes.  A warp owns up to 32 consecutive rows of A and walks their
 // non-zeros as one stream, in CSR order, across the row boundaries; the B row of every entry
 // is brought into shared memory by the copy engine (cp.async.bulk, one row per copy, completion
 // counted on an mbarrier) several batches ahead of its use, so the chain row_ptr -> col_ind ->
@@ -1332,7 +1332,6 @@ template <> struct FusedRow<__half> {
 constexpr int kStreamBuffers = B200SP_SPMM_STREAM_BUFFERS;  // batches of B rows per warp: one in use, the rest in flight
 constexpr int kStreamWarps = B200SP_SPMM_STREAM_WARPS;
 constexpr int kStreamThreads = kStreamWarps * 32;
-constexpr int kStreamRows = 32;                              // rows of A per warp
 constexpr long long kStreamWaitCycles = 1ll << 31;           // SM clocks (about a second) to wait on one barrier before giving up
 // What the next launches pass to the kernel as its wait limit and as bytes to expect beyond those it copies
 // (b200sp_spmm_stream_wait_test: a test makes a wait run out without any fault by expecting bytes nobody sends).
@@ -1940,6 +1939,25 @@ bool Aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0;
 #ifndef B200SP_SPMM_USE_STREAM
 #define B200SP_SPMM_USE_STREAM 1
 #endif
+// Which of the two takes B rows of 512 or 1024 bytes.  A warp of the row stream sums its rows one after the other: that
+// spares the chain of loads per row, which rows of few entries and a B far from the SMs cost most by, and needs rows enough for
+// all warps; SpmmFastKernel spends fewer instructions per entry and shares out the rows above four times the mean.  bf16,
+// N = 256, us by the stream and by SpmmFastKernel:
+//   few rows: 1000 of 30 11 (a row per warp; 133 with 32) and 7, 16,000 of 32 on 16,000 columns 41 and 30, 16,000 of 12 on 1 M
+//   28 and 26, 30,000 of 12 on 1 M 41 and 45;
+//   B of up to 61 MB: 120,000 of 6 60 and 74, of 12 95 and 99, of 30 209 and 185, 800,000 of 4 226 and 354, of 30 1224 and 1085;
+//   B above: 200,000 of 16 on as many columns 194 and 253, of 60 637 and 613, 800,000 of 30 1575 and 1915;
+//   power-law rows: 60,000 of 16 204 and 100, 200,000 of 24 on 1 M columns 419 and 414, 250,000 of 8 270 and 234, 300,000 of 24
+//   on 1 M 501 and 566, 800,000 of 4 367 and 465.
+constexpr int64_t kStreamMinRows = 16384, kStreamMinSkewed = 262144, kStreamMaxMean = 16;
+bool StreamPays(const b200spSpmmShape *sh, int32_t segments, int64_t rowBytes)
+{
+    if (gHostStreamExtraTx != 0) return true;  // the wait test is about the stream
+    if (sh->m < kStreamMinRows) return false;
+    if (sh->mid_units + (int64_t)segments > sh->m / 1000) return sh->m >= kStreamMinSkewed;
+    return sh->k * rowBytes >= kBlockMinB || sh->nnz < kStreamMaxMean * sh->m;
+}
+
 // The copy engine of an SM starts about one row copy per 20 clocks (measured: 16.8 M copies of
 // 256 bytes took 1.25 ms on 148 SMs), so rows shorter than 512 bytes move faster through plain
 // 128-bit loads and stay with SpmmFastKernel (256-byte rows, 64 per row of A: 1249 us against 265 us).
@@ -2366,7 +2384,7 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
         // B rows of 512 / 1024 bytes: rows of up to kLongRow entries go to the row-stream kernel,
         // and SpmmFastKernel is launched for its segment CTAs only.
         const long long rowBytes = sh->n * (long long)sizeof(ValT);
-        const bool stream_ = !sh->kahan && (rowBytes == 512 || rowBytes == 1024);
+        const bool stream_ = !sh->kahan && (rowBytes == 512 || rowBytes == 1024) && StreamPays(sh, segments, rowBytes);
         // Long rows by column blocks of B (found applicable by b200sp_spmm_analyze_blocks) instead of by segments.
         const bool byBlocks = sh->block_units > 0 && sh->long_rows > 0 && !sh->kahan && rowBytes >= kBlockMinRowBytes &&
                               sh->block_units <= L.capBlockSlots;
@@ -2421,7 +2439,10 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             sa.C = a.C;
             sa.m = a.m;
             sa.rowLimit = a.rowLimit;
-            sa.warpRows = kStreamRows;
+            // Eight rows a warp, fewer where that leaves less than two waves of some 24 warps an SM: 200,000 rows of 16, 32 / 16 / 8 / 4 / 2
+            // a warp, 214 / 200 / 194 / 195 / 208 us, 30,000 of 12 68 / 48 / 46 / 41 / -, 2 M power-law rows 2255 / 2245 / 2230 / 2300 / -.
+            sa.warpRows = 8;
+            while (sa.warpRows > 1 && sh->m < sa.warpRows * 48ll * b200sp_sm_count()) sa.warpRows /= 2;
             sa.ldb = a.ldb;
             sa.ldc = sh->ldc;
             sa.sc = a.sc;
