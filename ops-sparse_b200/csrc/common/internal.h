@@ -71,6 +71,16 @@ struct ActivePlan {
     uint64_t generation = 0;  // BufferGeneration(buffer) when the analysis was written
 };
 
+// SDDMM: an order of the tiles of C's entries that Preprocess left in a buffer.  Any order is right, whatever the pattern: only the
+// number of entries has to be the same.
+struct TileOrderPlan {
+    int64_t sized = 0;             // what aclsparseSDDMMBufferSize last said for this matrix
+    const void *buffer = nullptr;  // nullptr: no order
+    int64_t nnz = 0;
+    int64_t near = 0;              // tiles that are in the order of their columns, before the others
+    uint64_t generation = 0;
+};
+
 // Every library call that writes an analysis or scratch data into a caller buffer stamps that buffer with a new
 // generation; a recorded plan is valid only while its generation is still the buffer's current one.  Without it
 // a stale plan would be trusted after its bytes were overwritten: Preprocess(A, buf), then a call that re-analyses
@@ -112,6 +122,7 @@ struct aclsparseSpMatDescr {
     // What aclsparseSpMMGetBufferSize last said for this matrix: room for copies of B and A, and for how many columns.
     mutable int64_t spmmSizedRepack = 0;
     mutable int64_t spmmSizedN = -1;
+    b200sp::TileOrderPlan sddmm;  // of the SDDMM products that write this matrix
     mutable std::mutex copyMutex;  // held while a product that copies into the analysed buffer is enqueued
 };
 

@@ -3,8 +3,10 @@
 // (the reference's device arithmetic, sparse/sddmm/arch35/sddmm_kernel.cpp:26-27, 424-437).  Checks, their
 // order and status codes follow the reference host layer (sparse/sddmm/arch35/sddmm_host.cpp:145-320, 478-510,
 // 660-764).  The reference reorders rows greedily over its cores in Preprocess; here the work is cut by
-// non-zeros (a warp per 32 consecutive entries of C, the lanes splitting k), which needs no analysis:
-// BufferSize reports a token 256 bytes (the API wants a buffer), Preprocess only checks its arguments.
+// non-zeros (a warp per 32 or 64 consecutive entries of C), which needs no analysis.  For a Y that L2 does not hold Preprocess looks for an
+// order of these tiles that finds more of it there; otherwise BufferSize reports a token 256 bytes (the API wants a buffer)
+// and Preprocess only checks its arguments.
+#include <algorithm>
 #include <atomic>
 #include <climits>
 #include <cstdint>
@@ -94,9 +96,9 @@ __global__ void __launch_bounds__(256) SddmmKernel(const int32_t *__restrict__ r
 //     carries costs as many shuffles as values are left.
 // fp16 rows that start on odd 2-byte addresses (kBytes = 2) are copied as the 4-byte words that cover them and
 // realigned when they are read from shared memory.
-// Measured (1 M nodes, 16.0 M entries, fp16, k = 256): 1256 us with 32 lanes a row and scalar products, 1139 us here, which is the 7.6 GB
-// of Y rows that come from DRAM at 6.7 TB/s.  Working through Y by blocks of columns that stay in L2 (the pieces of rows of 64 entries and
-// more that lie in a block taken together) cut that to 5.6 GB and cost 1930 us and more: short pieces, and X rows fetched anew for each.
+// Measured (1 M nodes, 16.0 M entries, fp16, k = 256): 1256 us with 32 lanes a row and scalar products, 1157 us as it is here, which is the 7.6 GB
+// of Y rows that come from DRAM at 6.6 TB/s, 934 us with the tiles in an order (see TileOrder): 5.4 GB.  Cutting rows of 64 entries and more into
+// the pieces that lie in a block of columns cost 1930 us and more: short pieces, and X rows fetched anew for each.
 template <int kBytes> struct Words { using Type = uint32_t; };  // 4, and the words of kBytes = 2
 template <> struct Words<16> { using Type = uint4; };
 template <> struct Words<8> { using Type = uint2; };
@@ -129,10 +131,14 @@ __device__ __forceinline__ void FmaPair(float2 &acc, const float2 &x, const floa
 
 // kSize bytes from global to shared memory; `bytes` of them are read, the rest is zero.  Copies of 16 bytes go past L1
 // (.cg) or, kNear, through it.
-template <int kSize, bool kNear = true> __device__ __forceinline__ void CopyAsync(void *dst, const void *src, int bytes)
+template <int kSize, bool kNear = true, bool kHinted = false>
+__device__ __forceinline__ void CopyAsync(void *dst, const void *src, int bytes, [[maybe_unused]] uint64_t policy = 0)
 {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    if constexpr (!kNear)
+    if constexpr (kHinted)
+        asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;" ::"r"(d), "l"(src), "r"(bytes), "l"(policy)
+                     : "memory");
+    else if constexpr (!kNear)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
     else
         asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(kSize), "r"(bytes) : "memory");
@@ -140,7 +146,6 @@ template <int kSize, bool kNear = true> __device__ __forceinline__ void CopyAsyn
 __device__ __forceinline__ void CopyCommit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int kPending> __device__ __forceinline__ void CopyWait() { asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory"); }
 
-constexpr int kSddmmWarps = 2;  // the same with 4 (1 M nodes: 1139 and 1148 us) and with tiles of 128 (1147)
 constexpr int kSddmmTile = 64;  // entries a warp works on at a time, at most
 // Entries of a batch where there are warps enough: about 2 KB of copies a batch, half as much of the widest pieces.  Four lanes of three
 // pieces have few entries a group, and warps enough from the start (fp16, k = 36, 320,000 entries: 11.5 us with one, 13.9 with two).
@@ -150,14 +155,18 @@ constexpr int kShortBatch = kLanes == 4 && kSlabs == 3 ? 1
                             : kBytes == 8 ? (kSlabs <= 2 ? 4 : kSlabs == 3 || kLanes == 16 ? 2 : 1)
                                           : (kSlabs <= 2 ? 2 : 1);
 
-template <int kBytes, int kSlabs, int kBatch> struct SddmmShape {
+template <int kBytes, int kSlabs, int kBatch, bool kOrdered = false> struct SddmmShape {
     static constexpr int kStages = 2;
     static constexpr int kCopy = kBytes == 2 ? 4 : kBytes;
     static constexpr int kSlotBytes = 32 * kSlabs * kCopy;                       // one entry of every lane group
     static constexpr int kRing = 2 * kStages * kBatch * kSlotBytes;              // rows of Y, rows of X
     static constexpr int kTileBytes = kSddmmTile * 12;                           // row, column, sum per entry
-    static constexpr int kShared = kSddmmWarps * (kRing + kTileBytes);
-    static constexpr int kWarpsPerSm = kSddmmWarps * ((228 << 10) / (kShared + 1024));  // that find room at once
+    // Warps of a CTA.  Ordered tiles of wide rows: one, whose memory is free again as soon as it is done (1 M nodes, k = 256: 966 us with two,
+    // 934 with one; k = 128 602 and 578).  Otherwise two (150,000 nodes, k = 256, no order: 91 and 93; k = 64 56 and 60, where the 32 CTAs of
+    // an SM would not fill it).
+    static constexpr int kWarps = kOrdered && kRing + kTileBytes > 7000 ? 1 : 2;
+    static constexpr int kShared = kWarps * (kRing + kTileBytes);
+    static constexpr int kWarpsPerSm = kWarps * ((228 << 10) / (kShared + 1024));  // that find room at once
 };
 
 struct RowsOf {  // the operands' rows and how far apart they are
@@ -166,10 +175,137 @@ struct RowsOf {  // the operands' rows and how far apart they are
     int k;
 };
 
+// ---------------------------------------------------------------- the order of the tiles
+
+// In a row of many entries a tile of consecutive ones lies on few rows of Y: with ascending columns, 64 of 4096 entries span a
+// sixty-fourth of it.  Worked on in the order of their columns, such tiles of all rows ask for the same few megabytes of Y at any
+// time, and those stay in L2, where the tiles of short rows, in between, fetch every row of Y from DRAM.  The order is found by Preprocess (the
+// values and rows may change afterwards, the product is the same in any order) and kept in the caller's buffer: the near tiles by
+// column, then the others.  Tiles of both kinds take turns in the grid, so that neither L2 nor DRAM waits for the other.
+struct TileOrder {
+    const int2 *tiles = nullptr;       // {tile, row of its first entry}; near tiles by column, then the others; nullptr: as they come
+    long long near = 0;
+    unsigned long long share = 0;      // of the near tiles among all, times 2^32, rounded up
+};
+constexpr int kOrderBuckets = 1024;
+// A smaller Y stays in L2 as a whole.
+constexpr long long kOrderMinY = 96ll << 20;
+// Bytes of Y that a near tile may lie on, a third of Y at most.  1 M nodes, fp16, k = 256 (Y of 537 MB), DRAM traffic 7.6 GB without an order: 32 MB
+// 1046 us and 5.5 GB, 64 MB 1034, 96 MB 1029; with the rows of the tiles found by Preprocess, too, 976, 970 and (160 MB) 966.
+constexpr long long kNearSpan = 160ll << 20;
+// Fewer near tiles than one in so many are not worth the turns.
+constexpr long long kNearShare = 16;
+struct OrderLayout {
+    long long tiles;
+    size_t offCounts, offBucket, offTiles, total;
+};
+inline OrderLayout OrderLayoutFor(long long nnz)
+{
+    OrderLayout L;
+    L.tiles = (nnz + kSddmmTile - 1) / kSddmmTile;
+    L.offCounts = 256;
+    L.offBucket = L.offCounts + sizeof(int32_t) * 2 * (kOrderBuckets + 1);
+    L.offBucket = (L.offBucket + 255) / 256 * 256;
+    L.offTiles = (L.offBucket + sizeof(int16_t) * (size_t)L.tiles + 255) / 256 * 256;
+    L.total = L.offTiles + sizeof(int2) * (size_t)L.tiles;
+    return L;
+}
+
+// A warp per tile: its bucket of columns, kOrderBuckets if it is not near; how many tiles every bucket has.
+__global__ void __launch_bounds__(256) SddmmTileBucketsKernel(const int32_t *__restrict__ colInd, int nnz, int cols, int span,
+                                                              long long tiles, int16_t *__restrict__ bucket, int *__restrict__ counts)
+{
+    __shared__ int sCount[kOrderBuckets + 1];
+    for (int i = threadIdx.x; i <= kOrderBuckets; i += blockDim.x) sCount[i] = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+    for (long long t = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < tiles; t += warps) {
+        int low = INT_MAX, high = INT_MIN;
+        for (int i = lane; i < kSddmmTile; i += 32) {
+            const long long p = t * kSddmmTile + i;
+            if (p >= nnz) continue;
+            const int c = __ldg(colInd + p);
+            low = min(low, c);
+            high = max(high, c);
+        }
+        low = __reduce_min_sync(0xffffffffu, low);
+        high = __reduce_max_sync(0xffffffffu, high);
+        if (lane == 0) {
+            const bool near = low >= 0 && high < cols && high - low <= span;
+            const int b = near ? (int)(((long long)low + (high - low) / 2) * kOrderBuckets / cols) : kOrderBuckets;
+            bucket[t] = (int16_t)b;
+            atomicAdd(sCount + b, 1);
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i <= kOrderBuckets; i += blockDim.x)
+        if (sCount[i] != 0) atomicAdd(counts + i, sCount[i]);
+}
+
+// One CTA: where every bucket starts; what is in the last but one place after it is the number of near tiles.
+__global__ void __launch_bounds__(kOrderBuckets) SddmmBucketStartsKernel(const int *__restrict__ counts, int *__restrict__ starts)
+{
+    __shared__ int sWarp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n = counts[threadIdx.x];
+    int upTo = n;
+    for (int off = 1; off < 32; off <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upTo, off);
+        if (lane >= off) upTo += v;
+    }
+    if (lane == 31) sWarp[warp] = upTo;
+    __syncthreads();
+    if (warp == 0) {
+        int v = sWarp[lane];
+        for (int off = 1; off < 32; off <<= 1) {
+            const int w = __shfl_up_sync(0xffffffffu, v, off);
+            if (lane >= off) v += w;
+        }
+        sWarp[lane] = v;
+    }
+    __syncthreads();
+    upTo += warp > 0 ? sWarp[warp - 1] : 0;
+    starts[threadIdx.x] = upTo - n;
+    if (threadIdx.x == kOrderBuckets - 1) starts[kOrderBuckets] = upTo;
+}
+
+// A CTA per 1024 tiles: their places.  Inside a bucket as the CTAs come, the others nearly as they lie.
+__global__ void __launch_bounds__(256) SddmmOrderTilesKernel(const int32_t *__restrict__ rowPtr, int m, const int16_t *__restrict__ bucket,
+                                                             long long tiles, int *__restrict__ starts, int2 *__restrict__ order)
+{
+    __shared__ int sCount[kOrderBuckets + 1], sStart[kOrderBuckets + 1];
+    for (int i = threadIdx.x; i <= kOrderBuckets; i += blockDim.x) sCount[i] = 0;
+    __syncthreads();
+    const long long t0 = (long long)blockIdx.x * 1024 + threadIdx.x;
+    int mine[4], at[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const long long t = t0 + i * 256;
+        mine[i] = t < tiles ? bucket[t] : -1;
+        at[i] = mine[i] >= 0 ? atomicAdd(sCount + mine[i], 1) : 0;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i <= kOrderBuckets; i += blockDim.x) sStart[i] = sCount[i] != 0 ? atomicAdd(starts + i, sCount[i]) : 0;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (mine[i] >= 0) {
+            const int t = (int)(t0 + i * 256);
+            int lo = 0, hi = m - 1;  // row of its first entry: largest r with rowPtr[r] <= p
+            while (lo < hi) {
+                const int mid = lo + ((hi - lo + 1) >> 1);
+                if ((long long)__ldg(rowPtr + mid) <= (long long)t * kSddmmTile) lo = mid;
+                else hi = mid - 1;
+            }
+            order[sStart[mine[i]] + at[i]] = make_int2(t, lo);
+        }
+}
+
 // The dot products of a tile of entries: sDot[t] = X row sRow[t] . Y row sCol[t].  tile: a multiple of 32.
-template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear, int kBatch>
+template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear, int kBatch, bool kOrdered>
 __device__ __forceinline__ void TileDots(const RowsOf &rows, unsigned char *ring, const int *sRow, const int *sCol, float *sDot,
-                                         int tile, int lane)
+                                         int tile, int lane, [[maybe_unused]] uint64_t policy)
 {
     using Shape = SddmmShape<kBytes, kSlabs, kBatch>;
     using Piece = typename Words<kBytes>::Type;
@@ -207,7 +343,7 @@ __device__ __forceinline__ void TileDots(const RowsOf &rows, unsigned char *ring
                     const int bytes = end >= 2 * q + 2 ? 4 : end > 2 * q ? 2 : 0;
                     CopyAsync<4>(slot + s * 32, row - off + (bytes > 0 ? 4ll * q : 0), bytes);
                 } else {
-                    CopyAsync<kCopy, kNear || kCopy != 16>(slot + s * 32, row + offset[s], inside[s]);
+                    CopyAsync<kCopy, kNear || kCopy != 16, kOrdered>(slot + s * 32, row + offset[s], inside[s], policy);
                 }
             }
         };
@@ -305,24 +441,41 @@ __device__ __forceinline__ void TileDots(const RowsOf &rows, unsigned char *ring
     }
 }
 
-template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear, int kBatch>
-__global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(const int32_t *__restrict__ rowPtr,
+template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear, int kBatch, bool kOrdered>
+__global__ void __launch_bounds__(32 * SddmmShape<kBytes, kSlabs, kBatch, kOrdered>::kWarps) SddmmRowsKernel(const int32_t *__restrict__ rowPtr,
                                                                     const int32_t *__restrict__ colInd, T *__restrict__ cVal,
                                                                     const RowsOf rows, int m, int nnz, int tile, float alpha,
-                                                                    float beta, const T *alphaDev, const T *betaDev)
+                                                                    float beta, const T *alphaDev, const T *betaDev,
+                                                                    [[maybe_unused]] const TileOrder order)
 {
-    using Shape = SddmmShape<kBytes, kSlabs, kBatch>;
+    using Shape = SddmmShape<kBytes, kSlabs, kBatch, kOrdered>;
+    static_assert(!kOrdered || (kBytes == 16 && !kNear));
     extern __shared__ __align__(16) unsigned char sRaw[];
     b200sp::WaitForPrevious();
     const float a = alphaDev ? Load<T>(alphaDev) : alpha;
     const float b = betaDev ? Load<T>(betaDev) : beta;
     const int lane = threadIdx.x & 31;
-    const long long p0 = ((long long)blockIdx.x * kSddmmWarps + (threadIdx.x >> 5)) * tile;
-    if (p0 >= nnz) return;
+    long long p0 = (long long)blockIdx.x * Shape::kWarps + (threadIdx.x >> 5);
+    uint64_t policy = 0;
+    int r0 = -1;
+    if constexpr (kOrdered) {
+        if (p0 * tile >= nnz) return;
+        const unsigned before = (unsigned)((p0 * order.share) >> 32);
+        const bool near = (unsigned)(((p0 + 1) * order.share) >> 32) != before;
+        const int2 at = __ldg(order.tiles + (near ? before : order.near + (p0 - before)));
+        p0 = at.x;
+        r0 = at.y;
+        if (near) asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(policy));
+        else asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+    }
+    p0 *= tile;
+    if (p0 < 0 || p0 >= nnz) return;
     unsigned char *ring = sRaw + (threadIdx.x >> 5) * (Shape::kRing + Shape::kTileBytes);
     int *sRow = reinterpret_cast<int *>(ring + Shape::kRing), *sCol = sRow + kSddmmTile;
     float *sDot = reinterpret_cast<float *>(sCol + kSddmmTile);
-    int r0 = b200sp::WarpRowOf(rowPtr, m, p0, lane);
+    // the row that Preprocess found, if it is still the one
+    if (!kOrdered || (unsigned)r0 >= (unsigned)m || __ldg(rowPtr + r0) > p0 || __ldg(rowPtr + r0 + 1) <= p0)
+        r0 = b200sp::WarpRowOf(rowPtr, m, p0, lane);
     for (int t = lane; t < tile; t += 32) {
         const int p = p0 + t < nnz ? (int)p0 + t : nnz - 1;  // past the end: the last entry again, not stored
         const int r = b200sp::RowOfLane(rowPtr, m, r0, p, lane);
@@ -332,7 +485,7 @@ __global__ void __launch_bounds__(32 * kSddmmWarps) SddmmRowsKernel(const int32_
         r0 = __shfl_sync(0xffffffffu, r, 31);
     }
     __syncwarp();
-    TileDots<T, kBytes, kLanes, kSlabs, kNear, kBatch>(rows, ring, sRow, sCol, sDot, tile, lane);
+    TileDots<T, kBytes, kLanes, kSlabs, kNear, kBatch, kOrdered>(rows, ring, sRow, sCol, sDot, tile, lane, policy);
     for (int t = lane; t < tile && p0 + t < nnz; t += 32) {
         float z = a * sDot[t];
         if (b != 0.0f) z += b * Load<T>(cVal + p0 + t);
@@ -420,17 +573,17 @@ template <auto kKernel> cudaError_t AllowSharedMemory(int bytes, int *device)
     return e;
 }
 
-template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear, int kBatch, typename... Args>
+template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear, int kBatch, bool kOrdered, typename... Args>
 int LaunchRowsShape(int nnz, int tile, cudaStream_t stream, Args... args)
 {
-    using Shape = SddmmShape<kBytes, kSlabs, kBatch>;
+    using Shape = SddmmShape<kBytes, kSlabs, kBatch, kOrdered>;
     int dev = 0;
-    const cudaError_t e = AllowSharedMemory<SddmmRowsKernel<T, kBytes, kLanes, kSlabs, kNear, kBatch>>(Shape::kShared, &dev);
+    const cudaError_t e = AllowSharedMemory<SddmmRowsKernel<T, kBytes, kLanes, kSlabs, kNear, kBatch, kOrdered>>(Shape::kShared, &dev);
     if (e != cudaSuccess) return (int)e;
     const long long warps = ((long long)nnz + tile - 1) / tile;
     b200sp_note_launches(1);
-    return (int)b200sp::LaunchChained(SddmmRowsKernel<T, kBytes, kLanes, kSlabs, kNear, kBatch>,
-                                      (unsigned)((warps + kSddmmWarps - 1) / kSddmmWarps), 32 * kSddmmWarps, Shape::kShared,
+    return (int)b200sp::LaunchChained(SddmmRowsKernel<T, kBytes, kLanes, kSlabs, kNear, kBatch, kOrdered>,
+                                      (unsigned)((warps + Shape::kWarps - 1) / Shape::kWarps), 32 * Shape::kWarps, Shape::kShared,
                                       stream, args...);
 }
 
@@ -441,7 +594,7 @@ constexpr long long kNearBytes = 12 << 10;
 
 template <typename T, int kBytes>
 int LaunchRows(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const aclsparseDnMatDescr *Y, int k, Strides st,
-               float alpha, float beta, const void *alphaDev, const void *betaDev, cudaStream_t stream)
+               float alpha, float beta, const void *alphaDev, const void *betaDev, const TileOrder &order, cudaStream_t stream)
 {
     const int nnz = (int)C->nnz;
     // pieces of a row, one more where they start in the middle of a word
@@ -451,25 +604,27 @@ int LaunchRows(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const
     while (tile < kSddmmTile && nnz / (2 * tile) >= 16 * b200sp_sm_count()) tile *= 2;
     // A Y of a few lines that all entries want is asked of a few slices of L2 by every SM at once: it comes through L1.
     const bool near = kBytes == 16 && (long long)C->cols * st.yj * (long long)sizeof(T) <= kNearBytes;
-    auto launchAs = [&]<int kLanes, int kSlabs, bool kNear, int kBatch>() {
+    auto launchAs = [&]<int kLanes, int kSlabs, bool kNear, int kBatch, bool kOrdered>() {
         const RowsOf rows{static_cast<const char *>(X->values), static_cast<const char *>(Y->values),
                           st.xi * (long long)sizeof(T), st.yj * (long long)sizeof(T), k};
         // Rows of more than 32 pieces are long enough work for a last wave that is nearly empty to show.  320,000 entries, fp32, tiles of 64 and
         // 32: k = 400 80 and 66 us, k = 512 68 and 58, fp16, k = 640 66 and 56; narrower rows lose (fp16, k = 80: 17.2 and 19.0).
         const long long room = (long long)SddmmShape<kBytes, kSlabs, kBatch>::kWarpsPerSm * b200sp_sm_count(), warps = nnz / kSddmmTile;
-        const int entries = kLanes * kSlabs > 32 && warps > room && warps < 3 * room ? 32 : tile;
-        return LaunchRowsShape<T, kBytes, kLanes, kSlabs, kNear, kBatch>(
+        const int entries = !kOrdered && kLanes * kSlabs > 32 && warps > room && warps < 3 * room ? 32 : tile;
+        return LaunchRowsShape<T, kBytes, kLanes, kSlabs, kNear, kBatch, kOrdered>(
             nnz, entries, stream, static_cast<const int32_t *>(C->offsets), static_cast<const int32_t *>(C->indices),
             static_cast<T *>(C->values), rows, (int)C->rows, nnz, entries, alpha, beta, static_cast<const T *>(alphaDev),
-            static_cast<const T *>(betaDev));
+            static_cast<const T *>(betaDev), order);
     };
     auto launchDeep = [&]<int kLanes, int kSlabs, int kBatch>() {
         if constexpr (kBytes == 16)
-            if (near) return launchAs.template operator()<kLanes, kSlabs, true, kBatch>();
-        return launchAs.template operator()<kLanes, kSlabs, false, kBatch>();
+            if (near) return launchAs.template operator()<kLanes, kSlabs, true, kBatch, false>();
+        return launchAs.template operator()<kLanes, kSlabs, false, kBatch, false>();
     };
     auto launch = [&]<int kLanes, int kSlabs>() {
         constexpr int kShort = kShortBatch<kBytes, kLanes, kSlabs>;
+        if constexpr (kBytes == 16)
+            if (order.tiles != nullptr && tile == kSddmmTile && !near) return launchAs.template operator()<kLanes, kSlabs, false, kShort, true>();
         const long long warps = (nnz + 31ll) / 32 / b200sp_sm_count();  // for every SM, with the shortest tiles
         if constexpr (kShort < 4)
             if (warps < SddmmShape<kBytes, kSlabs, 4>::kWarpsPerSm) return launchDeep.template operator()<kLanes, kSlabs, 4>();
@@ -495,19 +650,19 @@ int LaunchRows(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const
 
 template <typename T>
 int Launch(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const aclsparseDnMatDescr *Y, int k, Strides st,
-           float alpha, float beta, const void *alphaDev, const void *betaDev, cudaStream_t stream)
+           float alpha, float beta, const void *alphaDev, const void *betaDev, const TileOrder &order, cudaStream_t stream)
 {
     if (st.xk == 1 && st.yk == 1) {
         // the widest piece that every row starts and ends on
         const unsigned long long all = (unsigned long long)k * sizeof(T) | (unsigned long long)st.xi * sizeof(T) |
                                        (unsigned long long)st.yj * sizeof(T) | reinterpret_cast<uintptr_t>(X->values) |
                                        reinterpret_cast<uintptr_t>(Y->values);
-        if (all % 16 == 0) return LaunchRows<T, 16>(C, X, Y, k, st, alpha, beta, alphaDev, betaDev, stream);
-        if (all % 8 == 0) return LaunchRows<T, 8>(C, X, Y, k, st, alpha, beta, alphaDev, betaDev, stream);
-        if (all % 4 == 0) return LaunchRows<T, 4>(C, X, Y, k, st, alpha, beta, alphaDev, betaDev, stream);
+        if (all % 16 == 0) return LaunchRows<T, 16>(C, X, Y, k, st, alpha, beta, alphaDev, betaDev, order, stream);
+        if (all % 8 == 0) return LaunchRows<T, 8>(C, X, Y, k, st, alpha, beta, alphaDev, betaDev, order, stream);
+        if (all % 4 == 0) return LaunchRows<T, 4>(C, X, Y, k, st, alpha, beta, alphaDev, betaDev, order, stream);
         if constexpr (sizeof(T) == 2)  // the covering words of the first rows start at the arrays
             if (reinterpret_cast<uintptr_t>(X->values) % 4 == 0 && reinterpret_cast<uintptr_t>(Y->values) % 4 == 0)
-                return LaunchRows<T, 2>(C, X, Y, k, st, alpha, beta, alphaDev, betaDev, stream);
+                return LaunchRows<T, 2>(C, X, Y, k, st, alpha, beta, alphaDev, betaDev, order, stream);
     }
     const long long chunks = (C->nnz + 31) / 32;
     const long long want = (chunks + 7) / 8;
@@ -519,6 +674,60 @@ int Launch(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const acl
         alpha, beta, static_cast<const T *>(alphaDev), static_cast<const T *>(betaDev));
     b200sp_note_launches(1);
     return (int)cudaGetLastError();
+}
+
+// Whether Preprocess looks for an order of the tiles: rows of Y that lie side by side, more than L2 holds, and tiles enough.
+bool MayOrder(const aclsparseDnMatDescr *Y, const aclsparseSpMatDescr *C, aclsparseOperation_t opY)
+{
+    const bool rows = (opY == ACL_SPARSE_OP_TRANSPOSE) == (Y->order == ACL_SPARSE_ORDER_ROW);
+    const long long bytes = Y->valueType == ACL_FLOAT16 ? 2 : 4;
+    return rows && (double)C->cols * (double)Y->ld * (double)bytes >= (double)kOrderMinY && C->nnz >= (1 << 20);
+}
+
+cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, aclsparseSpMatDescr *C, void *buffer, cudaStream_t stream)
+{
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        (void)cudaGetLastError();
+        return cudaSuccess;  // a product without an order is as good, only slower
+    }
+    const OrderLayout L = OrderLayoutFor(C->nnz);
+    char *p = static_cast<char *>(buffer);
+    int *counts = reinterpret_cast<int *>(p + L.offCounts), *starts = counts + kOrderBuckets + 1;
+    auto *bucket = reinterpret_cast<int16_t *>(p + L.offBucket);
+    const long long rowBytes = Y->ld * (Y->valueType == ACL_FLOAT16 ? 2ll : 4ll);
+    C->sddmm.generation = b200sp::NoteBufferWrite(buffer);
+    cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(int) * (kOrderBuckets + 1), stream);
+    if (e != cudaSuccess) return e;
+    const long long want = (L.tiles + 7) / 8, cap = (long long)b200sp_sm_count() * 8;
+    SddmmTileBucketsKernel<<<(unsigned)(want < cap ? want : cap), 256, 0, stream>>>(
+        static_cast<const int32_t *>(C->indices), (int)C->nnz, (int)C->cols, (int)std::min<long long>(kNearSpan / rowBytes, C->cols / 3), L.tiles, bucket, counts);
+    SddmmBucketStartsKernel<<<1, kOrderBuckets, 0, stream>>>(counts, starts);
+    int near = 0;
+    e = cudaMemcpyAsync(&near, starts + kOrderBuckets, sizeof(near), cudaMemcpyDeviceToHost, stream);
+    if (e != cudaSuccess) return e;
+    SddmmOrderTilesKernel<<<(unsigned)((L.tiles + 1023) / 1024), 256, 0, stream>>>(
+        static_cast<const int32_t *>(C->offsets), (int)C->rows, bucket, L.tiles, starts, reinterpret_cast<int2 *>(p + L.offTiles));
+    b200sp_note_launches(3);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e != cudaSuccess) return e;
+    C->sddmm.near = near;
+    C->sddmm.nnz = C->nnz;
+    C->sddmm.buffer = buffer;
+    return cudaSuccess;
+}
+
+// The order that Preprocess left in the buffer, if it is still there and worth following.
+TileOrder OrderOf(const aclsparseSpMatDescr *C, const void *buffer)
+{
+    const auto &plan = C->sddmm;
+    const OrderLayout L = OrderLayoutFor(C->nnz);
+    if (plan.buffer == nullptr || plan.buffer != buffer || plan.nnz != C->nnz || plan.generation != b200sp::BufferGeneration(buffer) ||
+        plan.near * kNearShare < L.tiles)
+        return {};
+    return {reinterpret_cast<const int2 *>(static_cast<const char *>(buffer) + L.offTiles), plan.near,
+            (((unsigned long long)plan.near << 32) + (unsigned long long)L.tiles - 1) / (unsigned long long)L.tiles};
 }
 
 }  // namespace
@@ -535,7 +744,8 @@ aclsparseStatus_t aclsparseSDDMMBufferSize(aclsparseHandle_t handle, aclsparseOp
     if (alpha == nullptr || beta == nullptr) return ACL_SPARSE_STATUS_INVALID_VALUE;
     const aclsparseStatus_t st = ValidateInputs(matX, matY, matC, opX, opY, computeType, alg);
     if (st != ACL_SPARSE_STATUS_SUCCESS) return st;
-    *size = 256;
+    *size = MayOrder(matY, matC, opY) ? OrderLayoutFor(matC->nnz).total : 256;
+    matC->sddmm.sized = (int64_t)*size;
     return ACL_SPARSE_STATUS_SUCCESS;
 }
 
@@ -544,7 +754,15 @@ aclsparseStatus_t aclsparseSDDMMPreprocess(aclsparseHandle_t handle, aclsparseOp
                                            aclsparseConstDnMatDescr_t matY, const void *beta, aclsparseSpMatDescr_t matC,
                                            aclDataType computeType, aclsparseSDDMMAlg_t alg, void *buffer)
 {
-    return ValidateCall(handle, matX, matY, matC, alpha, beta, buffer, true, opX, opY, computeType, alg);
+    const aclsparseStatus_t st = ValidateCall(handle, matX, matY, matC, alpha, beta, buffer, true, opX, opY, computeType, alg);
+    if (st != ACL_SPARSE_STATUS_SUCCESS) return st;
+    matC->sddmm.buffer = nullptr;
+    if (!MayOrder(matY, matC, opY) || matC->sddmm.sized < (int64_t)OrderLayoutFor(matC->nnz).total) return ACL_SPARSE_STATUS_SUCCESS;
+    if (OrderTiles(matY, matC, buffer, handle->stream) != cudaSuccess) {
+        B200SP_LOGE("aclsparseSDDMMPreprocess: analysis failed");
+        return ACL_SPARSE_STATUS_EXECUTION_FAILED;
+    }
+    return ACL_SPARSE_STATUS_SUCCESS;
 }
 
 aclsparseStatus_t aclsparseSDDMM(aclsparseHandle_t handle, aclsparseOperation_t opX, aclsparseOperation_t opY,
@@ -572,9 +790,10 @@ aclsparseStatus_t aclsparseSDDMM(aclsparseHandle_t handle, aclsparseOperation_t 
     const float b = host ? ReadScalar(beta, computeType) : 0.0f;
     const void *aDev = host ? nullptr : alpha;
     const void *bDev = host ? nullptr : beta;
+    const TileOrder order = OrderOf(matC, buffer);
     const int rc = computeType == ACL_FLOAT16
-                       ? Launch<__half>(matC, matX, matY, k, s, a, b, aDev, bDev, handle->stream)
-                       : Launch<float>(matC, matX, matY, k, s, a, b, aDev, bDev, handle->stream);
+                       ? Launch<__half>(matC, matX, matY, k, s, a, b, aDev, bDev, order, handle->stream)
+                       : Launch<float>(matC, matX, matY, k, s, a, b, aDev, bDev, order, handle->stream);
     if (rc != 0) {
         B200SP_LOGE("aclsparseSDDMM: kernel launch failed (cuda error %d)", rc);
         return ACL_SPARSE_STATUS_EXECUTION_FAILED;
