@@ -48,6 +48,7 @@
 // compute type, the result is alpha*sum + beta*y rounded once to the output type.
 // beta == 0 never reads y.
 #include <atomic>
+#include <cmath>
 #include <cstdint>
 #include <cstdio>
 #include <type_traits>
@@ -1386,22 +1387,14 @@ __global__ void SpmvMaxRowLengthKernel(const int32_t *__restrict__ rowPtr, int r
 constexpr int kTransChunk = 256;
 constexpr int kTransSpan = 1024;
 constexpr int kTransWarps = 8;
-template <typename CompT, typename ValT, typename AccT, int kChunk>
-__global__ void __launch_bounds__(32 * kTransWarps, 5) SpmvTransScatterKernel(const int32_t *__restrict__ rowPtr,
-                                                                           const int32_t *__restrict__ colInd,
-                                                                           const ValT *__restrict__ val, const ValT *__restrict__ x,
-                                                                           AccT *__restrict__ acc, int rows, int nnz, int chunksPerWarp,
-                                                                           Scalars<CompT> sc)
+// The chunks of one warp, from entry c0 on; put(column, term) adds a term.  bits, factor: shared memory of the warp.
+template <typename CompT, typename ValT, typename AccT, int kChunk, typename Put>
+__device__ __forceinline__ void TransChunks(const int32_t *__restrict__ rowPtr, const int32_t *__restrict__ colInd,
+                                            const ValT *__restrict__ val, const ValT *__restrict__ x, int rows, int nnz, long long c0,
+                                            int chunksPerWarp, CompT alpha, uint32_t *bits, CompT *factor, Put put)
 {
     constexpr int kSteps = kChunk / 32;
-    __shared__ uint32_t sBits[kTransWarps][kSteps];
-    __shared__ CompT sFactor[kTransWarps][kChunk];
-    b200sp::WaitForPrevious();
-    const CompT alpha = sc.Alpha();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t *bits = sBits[warp];
-    CompT *factor = sFactor[warp];
-    long long c0 = ((long long)blockIdx.x * kTransWarps + warp) * chunksPerWarp * kChunk;
+    const int lane = threadIdx.x & 31;
     if (c0 >= nnz) return;
     int r0 = b200sp::WarpRowOf(rowPtr, rows, c0, lane);  // a row that starts at or before the chunk's first entry
     for (int chunk = 0; chunk < chunksPerWarp && c0 < nnz; ++chunk, c0 += kChunk) {
@@ -1415,7 +1408,7 @@ __global__ void __launch_bounds__(32 * kTransWarps, 5) SpmvTransScatterKernel(co
         }
         const int first = (int)c0, last = (int)(c0 + kChunk < nnz ? c0 + kChunk - 1 : nnz - 1);
         auto add = [&](int u, CompT f) {
-            if (c[u] >= 0 && f != CompT(0)) atomicAdd(acc + c[u], static_cast<AccT>(f * Widen<CompT>(v[u])));
+            if (c[u] >= 0 && f != CompT(0)) put(c[u], static_cast<AccT>(f * Widen<CompT>(v[u])));
         };
         // Bounds of the rows r0 + 32 k + lane; beyond the last row both lie behind every entry.
         int s[4], e[4];
@@ -1479,6 +1472,55 @@ __global__ void __launch_bounds__(32 * kTransWarps, 5) SpmvTransScatterKernel(co
             if (word != 0) before = u * 32 + 31 - __clz(word);
         }
         __syncwarp();  // bits and factors may be written again
+    }
+}
+
+template <typename CompT, typename ValT, typename AccT, int kChunk>
+__global__ void __launch_bounds__(32 * kTransWarps, 5) SpmvTransScatterKernel(const int32_t *__restrict__ rowPtr,
+                                                                           const int32_t *__restrict__ colInd,
+                                                                           const ValT *__restrict__ val, const ValT *__restrict__ x,
+                                                                           AccT *__restrict__ acc, int rows, int nnz, int chunksPerWarp,
+                                                                           Scalars<CompT> sc)
+{
+    __shared__ uint32_t sBits[kTransWarps][kChunk / 32];
+    __shared__ CompT sFactor[kTransWarps][kChunk];
+    b200sp::WaitForPrevious();
+    const int warp = threadIdx.x >> 5;
+    const long long c0 = ((long long)blockIdx.x * kTransWarps + warp) * chunksPerWarp * kChunk;
+    TransChunks<CompT, ValT, AccT, kChunk>(rowPtr, colInd, val, x, rows, nnz, c0, chunksPerWarp, sc.Alpha(), sBits[warp],
+                                           sFactor[warp], [&](int c, AccT term) { atomicAdd(acc + c, term); });
+}
+
+// Few columns: the additions of all SMs meet at the few lines of y and wait for one another in L2 (15 M entries, fp32, 1000 columns: 1084 us;
+// 0.05 of them per clock and SM).  A CTA per SM adds up a y of its own in shared memory instead, and that to y: 49 us, 1.1 per
+// clock and SM; 4000 columns 331 and 46, 16,000 193 and 46, 48,000 129 and 52.  (Adding up the parts of 2, 4 or 8 CTAs of a cluster before
+// they go to y: the same for 2, 2 to 18 % slower for more, as not all SMs are in a cluster.)
+constexpr int kTransBlockWarps = 32;
+constexpr int kTransBlockCols = 48 << 10;  // what fits beside the warps' marks and factors
+template <typename CompT, typename ValT, typename AccT>
+__global__ void __launch_bounds__(32 * kTransBlockWarps, 1) SpmvTransBlockKernel(const int32_t *__restrict__ rowPtr,
+                                                                                const int32_t *__restrict__ colInd,
+                                                                                const ValT *__restrict__ val, const ValT *__restrict__ x,
+                                                                                AccT *__restrict__ acc, int rows, int cols, int nnz,
+                                                                                int chunksPerWarp, Scalars<CompT> sc)
+{
+    extern __shared__ __align__(16) unsigned char sRaw[];
+    AccT *sY = reinterpret_cast<AccT *>(sRaw);
+    __shared__ uint32_t sBits[kTransBlockWarps][kTransChunk / 32];
+    __shared__ CompT sFactor[kTransBlockWarps][kTransChunk];
+    for (int j = threadIdx.x; j < cols; j += blockDim.x) sY[j] = AccT(0);
+    __syncthreads();
+    b200sp::WaitForPrevious();
+    const int warp = threadIdx.x >> 5;
+    const long long c0 = ((long long)blockIdx.x * kTransBlockWarps + warp) * chunksPerWarp * kTransChunk;
+    TransChunks<CompT, ValT, AccT, kTransChunk>(rowPtr, colInd, val, x, rows, nnz, c0, chunksPerWarp, sc.Alpha(), sBits[warp],
+                                                sFactor[warp], [&](int c, AccT term) {
+                                                    if (c < cols) atomicAdd(sY + c, term);
+                                                });
+    __syncthreads();
+    for (int j = threadIdx.x; j < cols; j += blockDim.x) {
+        const AccT sum = sY[j];
+        if (sum != AccT(0)) atomicAdd(acc + j, sum);
     }
 }
 
@@ -1787,6 +1829,36 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
     return (int)cudaGetLastError();
 }
 
+// Whether a y per SM pays: estimates of both times in us, from 49 products of 6000 to 15 M entries on 1000 to 48,000 columns.  Additions to y run
+// at some 600 sqrt(columns) per us and all SMs, those to shared memory at 320,000, after the block is cleared and before it is
+// added to y.  600,000 entries on 48,000 columns: 9 us and 16 with a y per SM, 3 M 28 and 23; 150,000 on 1000: 14 and 9.
+bool TransByBlocks(int64_t cols, int64_t nnz)
+{
+    if (cols > kTransBlockCols) return false;
+    const double direct = 3.5 + (double)nnz / (600.0 * sqrt((double)cols));
+    const double blocks = 7.5 + 1.1e-4 * (double)cols + (double)nnz / 320000.0;
+    return direct > 1.1 * blocks;
+}
+
+template <typename CompT, typename ValT, typename AccT>
+cudaError_t LaunchTransBlock(const int32_t *rowPtr, const int32_t *colInd, const ValT *val, const ValT *x, AccT *acc, int rows,
+                             int cols, int nnz, const Scalars<CompT> &sc, cudaStream_t stream)
+{
+    static std::atomic<bool> configured[b200sp::kMaxDevices] = {};  // per device: this instantiation may use a block of shared memory
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= b200sp::kMaxDevices) return cudaErrorInvalidDevice;
+    if (!configured[dev].load(std::memory_order_relaxed)) {
+        const cudaError_t e = cudaFuncSetAttribute(SpmvTransBlockKernel<CompT, ValT, AccT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   kTransBlockCols * (int)sizeof(AccT));
+        if (e != cudaSuccess) return e;
+        configured[dev].store(true, std::memory_order_relaxed);
+    }
+    const long long chunks = ((long long)nnz + kTransChunk - 1) / kTransChunk, warps = (long long)kTransBlockWarps * b200sp_sm_count();
+    const long long perWarp = (chunks + warps - 1) / warps, perCta = perWarp * kTransBlockWarps;
+    return b200sp::LaunchChained(SpmvTransBlockKernel<CompT, ValT, AccT>, (unsigned)((chunks + perCta - 1) / perCta), 32 * kTransBlockWarps,
+                                 (size_t)cols * sizeof(AccT), stream, rowPtr, colInd, val, x, acc, rows, cols, nnz, (int)perWarp, sc);
+}
+
 template <typename CompT, typename ValT, typename OutT>
 int LaunchTransTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, const void *x, void *y,
                      int64_t rows, int64_t cols, int64_t nnz, const b200spScalars *s, void *scratch,
@@ -1816,8 +1888,11 @@ int LaunchTransTyped(const int32_t *rowPtr, const int32_t *colInd, const void *v
                                           (int)cols, sc);
     if (e == cudaSuccess && rows > 0 && nnz > 0) {
         b200sp_note_launches(1);
-        e = b200sp::LaunchChained(small ? SpmvTransScatterKernel<CompT, ValT, AccT, 32> : SpmvTransScatterKernel<CompT, ValT, AccT, kTransChunk>,
-                                  blocks, 32 * kTransWarps, 0, stream, rowPtr, colInd, v, xv, acc, (int)rows, (int)nnz, perWarp, sc);
+        if (TransByBlocks(cols, nnz))
+            e = LaunchTransBlock<CompT, ValT, AccT>(rowPtr, colInd, v, xv, acc, (int)rows, (int)cols, (int)nnz, sc, stream);
+        else
+            e = b200sp::LaunchChained(small ? SpmvTransScatterKernel<CompT, ValT, AccT, 32> : SpmvTransScatterKernel<CompT, ValT, AccT, kTransChunk>,
+                                      blocks, 32 * kTransWarps, 0, stream, rowPtr, colInd, v, xv, acc, (int)rows, (int)nnz, perWarp, sc);
     }
     if constexpr (kNarrowOut) {
         if (e == cudaSuccess) {
