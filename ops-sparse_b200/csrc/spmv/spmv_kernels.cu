@@ -467,6 +467,8 @@ struct BinHeader {  // first 256 bytes of the binned plan
     int32_t segments;         // segments the long rows were cut into
     int32_t longestShort;     // entries of the longest short row
     int32_t pairs, nearPairs; // sampled neighbouring rows, and those whose first and last columns lie within kNear
+    unsigned long long longNnz;   // entries in long rows
+    int32_t longestLong;
 };
 
 // Long rows, second form: x is cut into blocks of kXBlockElems columns and every CTA of
@@ -507,8 +509,11 @@ __global__ void SpmvBinRowsKernel(const int32_t *__restrict__ rowPtr, const int3
             const int rs = rowPtr[r], re = rowPtr[r + 1];
             const int len = re - rs;
             // a list entry carries the row's bounds, so its kernel starts on col_ind / values at once
-            if (len >= kLongLen) listL[atomicAdd(&hdr->longs, 1)] = make_int4((int)r, rs, re, 0);
-            else if (len > kShortMax) listM[atomicAdd(&hdr->medium, 1)] = make_int4((int)r, rs, re, 0);
+            if (len >= kLongLen) {
+                listL[atomicAdd(&hdr->longs, 1)] = make_int4((int)r, rs, re, 0);
+                atomicAdd(&hdr->longNnz, (unsigned long long)len);
+                if (len > *const_cast<volatile int32_t *>(&hdr->longestLong)) atomicMax(&hdr->longestLong, len);
+            } else if (len > kShortMax) listM[atomicAdd(&hdr->medium, 1)] = make_int4((int)r, rs, re, 0);
             else {
                 shortLen = longest = len;
                 isShort = 1;
@@ -667,7 +672,7 @@ struct LongBlockArgs {
 
 // CTA (b, g) keeps block b of x in shared memory and sums, for every long row of its group,
 // the entries whose column falls in that block -- a contiguous piece of the row, because the
-// column indices ascend.  kPieceLanes lanes share a piece (8, 32 or 256: see LongBlockShapeFor); x comes from shared memory, so the
+// column indices ascend.  kPieceLanes lanes share a piece (8, 32 or 256: see LongBlockLanes); x comes from shared memory, so the
 // only global traffic is the col_ind / values stream.  The last CTA of a row group to finish
 // adds each row's partial sums in block order (no wait, fixed order) and writes y.
 // Registers are capped at 48 (not at the 64 a 1024-thread CTA could have): while this kernel holds an SM, the
@@ -1606,32 +1611,32 @@ enum { kPlanTiles = 0, kPlanBinned = 1, kPlanBinnedBlocked = 2 };  // blocked: l
 
 // How SpmvLongBlockKernel shares out the long rows: groups of them, a CTA for each on every block of x (one CTA per SM at
 // most: it holds half of the SM's threads and a block of x), and lanes per piece.  With many blocks the groups are
-// few and large, and eight lanes per piece keep 128 pieces going; with few blocks a group is a handful of rows,
-// and more lanes share a piece.  Estimated per trip: about a microsecond, and a round trip to memory per eight entries
-// of a lane, for the 2048 entries a long row has on average.  (765,345 rows, one block of x, 5,000 long rows: 59 us
-// with eight lanes and 40 groups, 40 us with 32 lanes; 25,544 rows of mean 26: 40 and 10 us.)
-struct LongBlockShape {
-    int groups, lanes;
-};
-LongBlockShape LongBlockShapeFor(int xBlocks, int nLong)
+// few and large, and eight lanes per piece keep 128 pieces going; with few blocks a group is a handful of rows, whose pieces are
+// long, and more lanes share a piece.  Estimated per trip: about a microsecond (two where its warps meet), and a round trip to memory per eight entries
+// of a lane, for the longest rows in the first trip (they are ordered) and the average in the others.  600,000 power-law rows, us with 8
+// and 32 lanes: 100,000 columns (4 blocks) 87 and 55, 250,000 (8) 51 and 53, 1 M (32) 55 and 74; 765,345 rows, one block, 5,000 long rows: 59
+// with eight lanes and 40 groups, 40 with 32; 25,544 rows of mean 26: 40 and 10.
+int LongBlockGroups(int xBlocks, int nLong, int lanes)
 {
-    LongBlockShape best{1, 8};
     int groups = b200sp_sm_count() / xBlocks;
     groups = groups < 1 ? 1 : groups > kMaxLongGroups ? kMaxLongGroups : groups;
-    if (groups > nLong) groups = nLong;
-    const int rows = (nLong + groups - 1) / groups, piece = 2048 / xBlocks;
+    const int slots = kLongBlockThreads / lanes, useful = (nLong + slots - 1) / slots;
+    return groups < useful ? groups : useful;
+}
+int LongBlockLanes(int xBlocks, int nLong, long long longNnz, int longest)
+{
+    int best = 8;
     double least = 1e30;
     for (int lanes : {8, 32, 256}) {
-        const int slots = kLongBlockThreads / lanes;
-        const double cost = ((rows + slots - 1) / slots) * (1.0 + 0.6 * ((piece + 8 * lanes - 1) / (8 * lanes)));
+        const int slots = kLongBlockThreads / lanes, groups = LongBlockGroups(xBlocks, nLong, lanes);
+        const int trips = ((nLong + groups - 1) / groups + slots - 1) / slots;
+        auto trip = [&](double entries) { return (lanes > 32 ? 2.0 : 1.0) + 0.6 * ceil(entries / xBlocks / (8.0 * lanes)); };
+        const double cost = trip(longest) + (trips - 1) * trip((double)longNnz / nLong);
         if (cost < least) {
             least = cost;
-            best.lanes = lanes;
+            best = lanes;
         }
     }
-    const int slots = kLongBlockThreads / best.lanes;
-    const int useful = (nLong + slots - 1) / slots;
-    best.groups = groups < useful ? groups : useful;
     return best;
 }
 
@@ -1715,14 +1720,14 @@ int LaunchBinned(const int32_t *rowPtr, const int32_t *colInd, const ValT *val, 
             la.partials = reinterpret_cast<CompT *>(p + L.offPartials);
             la.nLong = nL;
             la.xBlocks = L.xBlocks;
-            const LongBlockShape shape = LongBlockShapeFor(L.xBlocks, nL);
-            la.groups = shape.groups;
+            const int pieceLanes = info[kInfoSegments];
+            la.groups = LongBlockGroups(L.xBlocks, nL, pieceLanes);
             auto launchLong = [&]<int kPieceLanes>() {
                 return vec ? LaunchLongBlock<CompT, ValT, OutT, true, kPieceLanes>(la, L.xBlocks * la.groups, sL)
                            : LaunchLongBlock<CompT, ValT, OutT, false, kPieceLanes>(la, L.xBlocks * la.groups, sL);
             };
-            const int rcL = shape.lanes == 8 ? launchLong.template operator()<8>()
-                          : shape.lanes == 32 ? launchLong.template operator()<32>() : launchLong.template operator()<256>();
+            const int rcL = pieceLanes == 8 ? launchLong.template operator()<8>()
+                          : pieceLanes == 32 ? launchLong.template operator()<32>() : launchLong.template operator()<256>();
             if (rcL != 0) return rcL;
         } else {
             if (vec) SpmvLongListKernel<CompT, ValT, OutT, true><<<(unsigned)nS, 256, 0, sL>>>(colInd, val, x, y, ls, sc);
@@ -2046,7 +2051,7 @@ int b200sp_spmv_analyze(const int32_t *row_ptr, const int32_t *col_ind, int64_t 
     plan_info[kInfoXBlocks] = useBlocked ? L.xBlocks : 0;
     plan_info[kInfoBlockElems] = useBlocked ? kXBlockElems : host.nearPairs * 4ll > host.pairs * 3ll ? host.longestShort : 0;
     plan_info[kInfoLongLen] = kLongLen;
-    plan_info[kInfoSegments] = host.segments;
+    plan_info[kInfoSegments] = useBlocked ? LongBlockLanes(L.xBlocks, host.longs, (long long)host.longNnz, host.longestLong) : host.segments;
     plan_info[kInfoMedium] = host.medium;
     plan_info[kInfoLong] = host.longs;
 #ifdef B200SP_SPMV_FORCE_SHORT_G
