@@ -6,9 +6,9 @@
 //
 // Here, with kernels of this library only: the entries, taken in CSR order, are sorted by column with a stable radix
 // sort (radix.cuh) that carries row and value along -- stability IS the golden's order.  Two passes for up to a million
-// columns, the second one in shared memory where the first can leave buckets of the right size.
+// columns.
 // Measured on 31.2 M entries in 1 M columns, numeric fp32: 1500 us with entries dropped into their columns by an
-// atomic cursor each (a sector of traffic per entry) and every column sorted afterwards, 745 us with both passes over all entries, 610 us here.
+// atomic cursor each (a sector of traffic per entry) and every column sorted afterwards, 745 us here.
 // A CSC copy of A gives y = A^T x without atomics: aclsparseSpMV (non-transposed) on the CSC arrays read as CSR.
 #include <atomic>
 #include <climits>
@@ -110,21 +110,6 @@ int BitsFor(long long count)  // of the numbers below count
     return bits;
 }
 
-constexpr int kBucketLeast = 6144, kBucketLeastBits = 4, kBucketMost = b200sp_radix::kBucketMax - b200sp_radix::kBucketMax / 20;
-// Upper bits of a column first (buckets that one CTA sorts each) or lower bits first: the whole assembly (COO to CSR, sort, this), us, lower and
-// upper: 1 M columns, 30.5 M entries, 30 K a bucket, 1272 and 1139, 16.8 M 797 and 746, 8.4 M 403 and 392, 4.2 M 232 and 248; 300,000 columns, 9.6 M
-// 443 and 428, power-law rows on 100,000, 15 M, 586 and 562.  Few lower bits are few words for the lanes to meet at: 2000 columns, one
-// lower bit, 842 and 868.
-// The fewest upper bits of a column whose buckets hold at most kBucketMost entries on average; 0 if none do, or they hold too few.
-int BucketBits(int bits, int n, int nnz)
-{
-    using b200sp_radix::kMaxDigitBits;
-    auto entries = [&](int high) { return (double)nnz / n * (double)(1 << (bits - high)); };
-    int high = bits > kMaxDigitBits ? bits - kMaxDigitBits : 1;  // the lower ones are one digit, too
-    while (high < kMaxDigitBits && high + kBucketLeastBits < bits && entries(high) > kBucketMost) ++high;
-    return entries(high) > kBucketMost || entries(high) < kBucketLeast ? 0 : high;
-}
-
 template <int kItems, int kBytes>
 cudaError_t Convert(int m, int n, int nnz, int base, const void *csrVal, const int *csrRowPtr, const int *csrColInd,
                     const Arrays &work, const Arrays &out, int *cscColPtr, int *counts, int *chunks, char *startsBytes,
@@ -148,49 +133,6 @@ cudaError_t Convert(int m, int n, int nnz, int base, const void *csrVal, const i
     a.chunks = chunks;
     a.words = csrColInd;
     a.vals = csrVal;
-    a.rowShift = digit;
-    a.wordShift = digit;
-    a.wordMask = -1;
-    if constexpr (kItems == kItemsLarge) {
-        const int high = passes == 2 ? BucketBits(bits, n, nnz) : 0, low = bits - high;
-        if (high > 0 && BitsFor(m) + low <= 32) {
-            int *starts = reinterpret_cast<int *>(startsBytes), *largeTiles = reinterpret_cast<int *>(startsBytes + kStartsBytes);
-            a.shift = low;
-            a.bins = 1 << high;
-            a.rowShift = low;
-            a.wordShift = 0;
-            a.wordMask = (1 << low) - 1;
-            a.wordBase = base;
-            a.starts = starts;
-            a.outWords = work.keys;
-            a.outVals = work.vals;
-            const int chunkCount = ChunksFor(a.tiles);
-            b200sp_note_launches(4);
-            cudaError_t e = b200sp::LaunchChained(HistogramKernel<kItems>, (unsigned)a.tiles, kThreads, 0, stream, a.words, nnz, a.wordBase,
-                                                  a.shift, a.bins, counts);
-            if (e == cudaSuccess)
-                e = b200sp::LaunchChained(ScanTilesKernel, (unsigned)(((a.bins + 127) / 128) * chunkCount), 128, 0, stream, counts, a.tiles,
-                                          a.bins, chunks);
-            if (e == cudaSuccess)
-                e = b200sp::LaunchChained(ScanChunksKernel, 1, kMaxBins, 0, stream, chunks, chunkCount, a.bins, starts, largeTiles);
-            if (e == cudaSuccess) e = LaunchScatter<kItems, kBytes, true, false, false>(a, stream);
-            if (e != cudaSuccess) return e;
-            const BucketArgs buckets{work.keys, work.vals, starts, out.rows, out.vals, cscColPtr, n, base, low};
-            // What no pass uses here, four bytes an entry each: the counts of the tiles of large buckets, at most 5/4 of a tile for
-            // every kLargeTile entries, and their sums, kMaxBins for every bucket.
-            const LargeArgs large{largeTiles, work.rows, out.keys, a.bins};
-            PassArgs last = a;
-            last.words = work.keys;
-            last.vals = work.vals;
-            last.wordBase = last.shift = 0;
-            last.digitBits = low;
-            last.bins = 1 << low;
-            last.rowPlus = base;
-            last.outRows = out.rows;
-            last.outVals = out.vals;
-            return LaunchBuckets<kBytes>(last, buckets, large, b200sp_sm_count(), stream);
-        }
-    }
     const int chunkCount = ChunksFor(a.tiles);
     const unsigned scanBlocks = (unsigned)(((a.bins + 127) / 128) * chunkCount);
     cudaError_t e = cudaSuccess;
@@ -210,8 +152,7 @@ cudaError_t Convert(int m, int n, int nnz, int base, const void *csrVal, const i
         e = b200sp::LaunchChained(HistogramKernel<kItems>, (unsigned)a.tiles, kThreads, 0, stream, a.words, nnz, a.wordBase, a.shift,
                                   a.bins, counts);
         if (e == cudaSuccess) e = b200sp::LaunchChained(ScanTilesKernel, scanBlocks, 128, 0, stream, counts, a.tiles, a.bins, chunks);
-        if (e == cudaSuccess) e = b200sp::LaunchChained(ScanChunksKernel, 1, kMaxBins, 0, stream, chunks, chunkCount, a.bins, starts,
-                                                        (int *)nullptr);
+        if (e == cudaSuccess) e = b200sp::LaunchChained(ScanChunksKernel, 1, kMaxBins, 0, stream, chunks, chunkCount, a.bins, starts);
         if (e != cudaSuccess) break;
         if (!packed) {
             e = p == 0 ? LaunchScatter<kItems, kBytes, true, false, true>(a, stream)

@@ -7,8 +7,6 @@
 // take two.  The first pass reads the caller's columns and makes the rows from the row offsets; the last one leaves
 // rows and values in the caller's arrays.
 //
-// Where the columns' upper bits can be taken first, a second pass over all entries is not needed: see BucketKernel.
-//
 // What bounds a scatter pass is the number of 32-byte sectors it stores (a tile of 8192 entries meets 1024 digits eight
 // times each, so a run is about a sector long, unaligned: 85 us per 4-byte array of 31 M entries).  So as few arrays
 // as possible move: with up to two passes the first packs the row and the digit of the second into one word where
@@ -146,16 +144,9 @@ static __global__ void __launch_bounds__(128) ScanTilesKernel(int *__restrict__ 
     chunks[(long long)chunk * bins + d] = run;
 }
 
-// Entries of a bucket that one CTA sorts in shared memory (BucketKernel), and of a tile of larger buckets.
-constexpr int kBucketThreads = 1024, kBucketItems = 32;
-constexpr int kBucketMax = kBucketThreads * kBucketItems;
-constexpr int kLargeTile = kThreads * kItemsLarge;
-
 // One CTA, a thread per digit: chunks[chunk][digit] becomes the count in the chunks before it, starts[digit] the first
-// place of the digit in the output (starts[bins] = all).  largeTiles[digit], if wanted: the tiles that buckets above kBucketMax
-// entries before it are cut into (largeTiles[bins] = all).
-static __global__ void __launch_bounds__(kMaxBins) ScanChunksKernel(int *__restrict__ chunks, int count, int bins, int *__restrict__ starts,
-                                                                    int *__restrict__ largeTiles)
+// place of the digit in the output (starts[bins] = all).
+static __global__ void __launch_bounds__(kMaxBins) ScanChunksKernel(int *__restrict__ chunks, int count, int bins, int *__restrict__ starts)
 {
     __shared__ int sWarp[32];
     b200sp::WaitForPrevious();
@@ -176,11 +167,6 @@ static __global__ void __launch_bounds__(kMaxBins) ScanChunksKernel(int *__restr
     const int incl = CtaInclusiveScan<kMaxBins>(run, sWarp);
     if (d < bins) starts[d] = incl - run;
     if (d == bins - 1) starts[bins] = incl;
-    if (largeTiles == nullptr) return;
-    const int tiles = d < bins && run > kBucketMax ? (run + kLargeTile - 1) / kLargeTile : 0;
-    const int upTo = CtaInclusiveScan<kMaxBins>(tiles, sWarp);
-    if (d < bins) largeTiles[d] = upTo - tiles;
-    if (d == bins - 1) largeTiles[bins] = upTo;
 }
 
 template <int kBytes> struct Value { using Type = uint32_t; };  // 4, and a placeholder for 0
@@ -199,7 +185,6 @@ struct PassArgs {
     int wordBase;         // subtracted from the words read: the index base in the first pass
     int rowPlus;          // added to the rows written: the index base in the last pass
     int shift, digitBits, bins, tiles;
-    int rowShift, wordShift, wordMask;  // packing: (row << rowShift) | (column >> wordShift & wordMask)
     const int *prefix;    // counts, chunks and starts after the scans
     const int *chunks;
     const int *starts;
@@ -288,8 +273,8 @@ __device__ __forceinline__ void RowsOfTile(const PassArgs &a, long long first, i
 
 // kKeys: columns travel in an array of their own, beside the rows.  Otherwise a pass that is not the last leaves
 // (row << digitBits) | (column >> digitBits), and the last one leaves rows.
-template <int kItems, int kBytes, bool kFirst, bool kLast, bool kKeys, typename Dest>
-__device__ __forceinline__ void ScatterTile(const PassArgs &a, long long first, int live, Dest destOf)  // destOf(digit): place of the tile's first
+template <int kItems, int kBytes, bool kFirst, bool kLast, bool kKeys>
+static __global__ void __launch_bounds__(kThreads, 2) ScatterKernel(const PassArgs a)
 {
     using Val = typename Value<kBytes>::Type;
     constexpr int kTile = kThreads * kItems;
@@ -305,6 +290,9 @@ __device__ __forceinline__ void ScatterTile(const PassArgs &a, long long first, 
     __shared__ int sWarp[kWarps];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int bins = a.bins;
+    b200sp::WaitForPrevious();
+    const long long first = (long long)blockIdx.x * kTile;
+    const int live = a.nnz - first < kTile ? (int)(a.nnz - first) : kTile;
 
     // A warp's entries are consecutive, lane by lane within a step: their order is (step, lane).
     const int w0 = warp * kPerWarp + lane;
@@ -337,7 +325,8 @@ __device__ __forceinline__ void ScatterTile(const PassArgs &a, long long first, 
             const int d = tid * kPer + k;
             tot[k] = glob[k] = 0;
             if (d < bins) {
-                glob[k] = destOf(d);
+                glob[k] = __ldg(a.starts + d) + __ldg(a.prefix + (long long)blockIdx.x * bins + d) +
+                          __ldg(a.chunks + (long long)(blockIdx.x / kChunk) * bins + d);
 #pragma unroll
                 for (int w = 0; w < kWarps; ++w) {
                     const int c = sCount[w * kMaxBins + d];
@@ -373,7 +362,7 @@ __device__ __forceinline__ void ScatterTile(const PassArgs &a, long long first, 
                 sMove[to] = kFirst ? row[u] : __ldg(a.rows + first + i);
             } else {
                 sDigit[to] = (uint16_t)d;
-                if constexpr (kFirst && !kLast) sMove[to] = (int)((unsigned)row[u] << a.rowShift | ((unsigned)w >> a.wordShift & (unsigned)a.wordMask));
+                if constexpr (kFirst && !kLast) sMove[to] = (int)((unsigned)row[u] << a.digitBits | (unsigned)w >> a.digitBits);
                 else if constexpr (kFirst) sMove[to] = row[u];
                 else sMove[to] = (int)((unsigned)w >> a.digitBits);
             }
@@ -413,229 +402,6 @@ __device__ __forceinline__ void ScatterTile(const PassArgs &a, long long first, 
     }
 }
 
-template <int kItems, int kBytes, bool kFirst, bool kLast, bool kKeys>
-static __global__ void __launch_bounds__(kThreads, 2) ScatterKernel(const PassArgs a)
-{
-    constexpr int kTile = kThreads * kItems;
-    b200sp::WaitForPrevious();
-    const long long first = (long long)blockIdx.x * kTile;
-    const int live = a.nnz - first < kTile ? (int)(a.nnz - first) : kTile;
-    ScatterTile<kItems, kBytes, kFirst, kLast, kKeys>(a, first, live, [&](int d) {
-        return __ldg(a.starts + d) + __ldg(a.prefix + (long long)blockIdx.x * a.bins + d) +
-               __ldg(a.chunks + (long long)(blockIdx.x / kChunk) * a.bins + d);
-    });
-}
-
-// ---------------------------------------------------------------- buckets of columns
-
-// Two passes the other way round: the first scatters the entries into buckets by their columns' upper bits, and a bucket, whose place in
-// the output is a stretch of its own, is sorted by the lower bits by one CTA in shared memory and written out in order: no
-// unaligned runs, no histogram and no scan for the second pass.  What bounds it are the steps between barriers of a CTA that has an SM to
-// itself: a bucket of 30,000 entries takes some 30 us, about 9 of them ranks (shared memory), 2 the places of the digits, 7 entries on their way
-// through shared memory, the rest reading and writing.  30.5 M entries in 1024 buckets: 212 us, where a histogram, scans, a scatter of all
-// entries and the offsets of the columns took 340.  The packed words are read twice, the second time from L2, as registers for
-// rank and word do not go round.
-struct BucketArgs {
-    const int *words;      // (row << lowBits) | low bits of the column, by bucket
-    const void *vals;
-    const int *starts;     // of the buckets
-    int *outRows;
-    void *outVals;
-    int *colPtr;
-    int n, base, lowBits;
-};
-constexpr int BucketSmem() { return kBucketMax * 4 + (kBucketThreads / 32) * kMaxBins * 2; }
-
-template <int kBytes> static __global__ void __launch_bounds__(kBucketThreads, 1) BucketKernel(const BucketArgs a)
-{
-    using Val = typename Value<kBytes>::Type;
-    constexpr int kWarpCount = kBucketThreads / 32;
-    extern __shared__ __align__(16) unsigned char sRaw[];
-    uint32_t *sMask = reinterpret_cast<uint32_t *>(sRaw);           // [warp][digit], then
-    int *sMove = reinterpret_cast<int *>(sRaw);                     // [kBucketMax] an array in its new order
-    uint16_t *sCount = reinterpret_cast<uint16_t *>(sRaw + kBucketMax * 4);  // [warp][digit]
-    __shared__ int sWarp[kWarpCount];
-    static_assert(kWarpCount * kMaxBins <= kBucketMax);
-    b200sp::WaitForPrevious();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int s = __ldg(a.starts + blockIdx.x), count = __ldg(a.starts + blockIdx.x + 1) - s;
-    if (blockIdx.x == 0 && tid == 0) a.colPtr[a.n] = a.base + __ldg(a.starts + gridDim.x);
-    if (count > kBucketMax) return;
-    const int bins = 1 << a.lowBits;
-    const int steps = (count + kBucketThreads - 1) / kBucketThreads;
-    const int w0 = warp * 32 * steps + lane;  // a warp's entries are consecutive
-    const int *words = a.words + s;
-    uint32_t place[kBucketItems];
-#pragma unroll
-    for (int u = 0; u < kBucketItems; ++u) place[u] = u < steps && w0 + u * 32 < count ? (uint32_t)__ldg(words + w0 + u * 32) : 0u;
-    for (int i = tid; i < kWarpCount * bins / 4; i += kBucketThreads) reinterpret_cast<uint4 *>(sMask)[i] = make_uint4(0, 0, 0, 0);
-    for (int i = tid; i < kWarpCount * kMaxBins / 8; i += kBucketThreads) reinterpret_cast<uint4 *>(sCount)[i] = make_uint4(0, 0, 0, 0);
-    __syncthreads();
-    uint16_t *mine = sCount + warp * kMaxBins;
-    uint32_t *masks = sMask + warp * bins;
-#pragma unroll
-    for (int u = 0; u < kBucketItems; ++u) {
-        if (u < steps) {
-            const int d = (int)place[u] & (bins - 1);
-            place[u] = ((uint32_t)d << 16) | (uint32_t)RankStep(masks, mine, d, w0 + u * 32 < count, lane);
-        }
-    }
-    __syncthreads();
-    {   // counts -> first place of (digit, warp) in the bucket; where the columns start
-        int tot = 0;
-        if (tid < bins)
-            for (int w = 0; w < kWarpCount; ++w) tot += sCount[w * kMaxBins + tid];
-        int run = CtaInclusiveScan<kBucketThreads>(tot, sWarp) - tot;
-        if (tid < bins) {
-            const long long c = ((long long)blockIdx.x << a.lowBits) | tid;
-            if (c < a.n) a.colPtr[c] = a.base + s + run;
-            for (int w = 0; w < kWarpCount; ++w) {
-                const int k = sCount[w * kMaxBins + tid];
-                sCount[w * kMaxBins + tid] = (uint16_t)run;
-                run += k;
-            }
-        }
-    }
-    __syncthreads();  // the masks' space serves the rows now
-#pragma unroll
-    for (int u = 0; u < kBucketItems; ++u) {
-        if (u < steps && w0 + u * 32 < count) {
-            const int to = (int)(place[u] & 0xffffu) + mine[place[u] >> 16];
-            place[u] = (uint32_t)to;
-            sMove[to] = (int)((uint32_t)__ldg(words + w0 + u * 32) >> a.lowBits);
-        }
-    }
-    __syncthreads();
-    for (int i = tid; i < count; i += kBucketThreads) a.outRows[s + i] = sMove[i] + a.base;
-    if constexpr (kBytes > 0) {
-        __syncthreads();
-        Val *sVal = reinterpret_cast<Val *>(sRaw);
-        const Val *vals = static_cast<const Val *>(a.vals) + s;
-#pragma unroll
-        for (int u = 0; u < kBucketItems; ++u)
-            if (u < steps && w0 + u * 32 < count) sVal[place[u]] = __ldg(vals + w0 + u * 32);
-        __syncthreads();
-        for (int i = tid; i < count; i += kBucketThreads) static_cast<Val *>(a.outVals)[s + i] = sVal[i];
-    }
-}
-
-// Buckets of more than kBucketMax entries: their tiles are counted, the counts of every bucket's digits are added up over its tiles, and the
-// tiles are scattered as in a pass over all entries.  Where there are none the three kernels return at once.
-struct LargeArgs {
-    const int *largeTiles;  // [bucket] first tile, [buckets] all tiles
-    int *counts;            // [tile][digit]
-    int *totals;            // [bucket][digit]
-    int buckets;
-};
-__device__ __forceinline__ int BucketOfTile(const LargeArgs &l, int tile)  // the last bucket that starts at or before it
-{
-    int lo = 0, hi = l.buckets - 1;
-    while (lo < hi) {
-        const int mid = lo + (hi - lo + 1) / 2;
-        if (__ldg(l.largeTiles + mid) <= tile) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-static __global__ void __launch_bounds__(kThreads) LargeHistogramKernel(const BucketArgs a, const LargeArgs l)
-{
-    __shared__ int sHist[kMaxBins];
-    b200sp::WaitForPrevious();
-    const int tiles = __ldg(l.largeTiles + l.buckets), bins = 1 << a.lowBits;
-    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const int b = BucketOfTile(l, t);
-        const long long first = __ldg(a.starts + b) + (long long)(t - __ldg(l.largeTiles + b)) * kLargeTile;
-        const long long left = __ldg(a.starts + b + 1) - first;
-        const int live = left < kLargeTile ? (int)left : kLargeTile;
-        for (int i = threadIdx.x; i < bins; i += kThreads) sHist[i] = 0;
-        __syncthreads();
-        int k[kItemsLarge];
-#pragma unroll
-        for (int u = 0; u < kItemsLarge; ++u) k[u] = u * kThreads + (int)threadIdx.x < live ? __ldg(a.words + first + u * kThreads + threadIdx.x) : 0;
-#pragma unroll
-        for (int u = 0; u < kItemsLarge; ++u)
-            if (u * kThreads + (int)threadIdx.x < live) atomicAdd(&sHist[k[u] & (bins - 1)], 1);
-        __syncthreads();
-        for (int i = threadIdx.x; i < bins; i += kThreads) l.counts[(long long)t * bins + i] = sHist[i];
-        __syncthreads();
-    }
-}
-
-// Eight parts of a bucket's tiles by 128 digits: counts become the count in the bucket's tiles before.
-static __global__ void __launch_bounds__(1024) LargeScanKernel(const LargeArgs l, int bins)
-{
-    __shared__ int sSum[8][128];
-    b200sp::WaitForPrevious();
-    if (__ldg(l.largeTiles + l.buckets) == 0) return;
-    const int groups = (bins + 127) / 128, column = threadIdx.x & 127, part = threadIdx.x >> 7;
-    for (int item = blockIdx.x; item < l.buckets * groups; item += gridDim.x) {
-        const int b = item / groups, d = (item % groups) * 128 + column;
-        const int first = __ldg(l.largeTiles + b), tiles = __ldg(l.largeTiles + b + 1) - first;
-        if (tiles == 0) continue;
-        const int t0 = first + (int)((long long)tiles * part / 8), t1 = first + (int)((long long)tiles * (part + 1) / 8);
-        int sum = 0;
-        if (d < bins) {
-#pragma unroll 8
-            for (int t = t0; t < t1; ++t) sum += l.counts[(long long)t * bins + d];
-        }
-        sSum[part][column] = sum;
-        __syncthreads();
-        int run = 0;
-        for (int k = 0; k < part; ++k) run += sSum[k][column];
-        if (d < bins) {
-            if (part == 7) l.totals[(long long)b * bins + d] = run + sum;
-            for (int t = t0; t < t1; t += 8) {
-                int v[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) v[u] = t + u < t1 ? l.counts[(long long)(t + u) * bins + d] : 0;
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    if (t + u < t1) l.counts[(long long)(t + u) * bins + d] = run;
-                    run += v[u];
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
-
-template <int kBytes>
-static __global__ void __launch_bounds__(kThreads, 2) LargeScatterKernel(const PassArgs p, const BucketArgs a, const LargeArgs l)
-{
-    __shared__ int sBase[kMaxBins], sScan[kWarps];
-    b200sp::WaitForPrevious();
-    const int tiles = __ldg(l.largeTiles + l.buckets), bins = 1 << a.lowBits;
-    constexpr int kPer = kMaxBins / kThreads;
-    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const int b = BucketOfTile(l, t), tile = t - __ldg(l.largeTiles + b), start = __ldg(a.starts + b);
-        const long long first = start + (long long)tile * kLargeTile, left = __ldg(a.starts + b + 1) - first;
-        int tot[kPer], sum = 0;
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            const int d = (int)threadIdx.x * kPer + k;
-            tot[k] = d < bins ? __ldg(l.totals + (long long)b * bins + d) : 0;
-            sum += tot[k];
-        }
-        int run = CtaInclusiveScan<kThreads>(sum, sScan) - sum;
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            const int d = (int)threadIdx.x * kPer + k;
-            const long long c = ((long long)b << a.lowBits) | d;
-            if (d < bins) {
-                sBase[d] = start + run;
-                if (tile == 0 && c < a.n) a.colPtr[c] = a.base + start + run;
-            }
-            run += tot[k];
-        }
-        __syncthreads();
-        ScatterTile<kItemsLarge, kBytes, false, true, false>(p, first, left < kLargeTile ? (int)left : kLargeTile, [&](int d) {
-            return sBase[d] + l.counts[(long long)t * bins + d];
-        });
-        __syncthreads();
-    }
-}
-
 // Column offsets from the counts of the last of at most two passes.  With one pass the digits are the columns.  With two,
 // column (hi, lo) starts where the entries with digit hi that lie before the first entry with low digit lo end: a CTA
 // per lo counts, in the tile in which that entry lies, the digits before it.
@@ -670,43 +436,21 @@ static __global__ void __launch_bounds__(256) OffsetsFromCountsKernel(const int 
     }
 }
 
-// Once per device and kernel: it may use that many bytes of shared memory.
-template <auto kKernel> inline cudaError_t AllowSharedMemory(int bytes)
-{
-    static std::atomic<bool> configured[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    if (configured[dev].load(std::memory_order_relaxed)) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) configured[dev].store(true, std::memory_order_relaxed);
-    return e;
-}
-
 template <int kItems, int kBytes, bool kFirst, bool kLast, bool kKeys>
 inline cudaError_t LaunchScatter(const PassArgs &a, cudaStream_t stream)
 {
     constexpr int kSmem = ScatterSmem<kItems>();
-    const cudaError_t e = AllowSharedMemory<ScatterKernel<kItems, kBytes, kFirst, kLast, kKeys>>(kSmem);
-    if (e != cudaSuccess) return e;
+    static std::atomic<bool> configured[64] = {};  // per device: this instantiation may use kSmem bytes
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (!configured[dev].load(std::memory_order_relaxed)) {
+        const cudaError_t e = cudaFuncSetAttribute(ScatterKernel<kItems, kBytes, kFirst, kLast, kKeys>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+        if (e != cudaSuccess) return e;
+        configured[dev].store(true, std::memory_order_relaxed);
+    }
     b200sp_note_launches(1);
     return b200sp::LaunchChained(ScatterKernel<kItems, kBytes, kFirst, kLast, kKeys>, (unsigned)a.tiles, kThreads, kSmem, stream, a);
-}
-
-// The buckets that a scatter by the upper bits left, small ones and large ones.  p: the pass that scatters the tiles of large ones.
-template <int kBytes>
-inline cudaError_t LaunchBuckets(const PassArgs &p, const BucketArgs &a, const LargeArgs &l, int sms, cudaStream_t stream)
-{
-    constexpr int kSmem = ScatterSmem<kItemsLarge>();
-    cudaError_t e = AllowSharedMemory<BucketKernel<kBytes>>(BucketSmem());
-    if (e == cudaSuccess) e = AllowSharedMemory<LargeScatterKernel<kBytes>>(kSmem);
-    if (e != cudaSuccess) return e;
-    b200sp_note_launches(4);
-    e = b200sp::LaunchChained(BucketKernel<kBytes>, (unsigned)l.buckets, kBucketThreads, BucketSmem(), stream, a);
-    const unsigned grid = (unsigned)(2 * sms);
-    if (e == cudaSuccess) e = b200sp::LaunchChained(LargeHistogramKernel, grid, kThreads, 0, stream, a, l);
-    if (e == cudaSuccess) e = b200sp::LaunchChained(LargeScanKernel, grid, 1024, 0, stream, l, 1 << a.lowBits);
-    if (e == cudaSuccess) e = b200sp::LaunchChained(LargeScatterKernel<kBytes>, grid, kThreads, kSmem, stream, p, a, l);
-    return e;
 }
 
 }  // namespace b200sp_radix
