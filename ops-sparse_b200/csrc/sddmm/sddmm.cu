@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(256) SddmmKernel(const int32_t *__restrict__ r
 // fp16 rows that start on odd 2-byte addresses (kBytes = 2) are copied as the 4-byte words that cover them and
 // realigned when they are read from shared memory.
 // Measured (1 M nodes, 16.0 M entries, fp16, k = 256): 1256 us with 32 lanes a row and scalar products, 1157 us as it is here, which is the 7.6 GB
-// of Y rows that come from DRAM at 6.6 TB/s, 934 us with the tiles in an order (see TileOrder): 5.4 GB.  Cutting rows of 64 entries and more into
+// of Y rows that come from DRAM at 6.6 TB/s, 881 us with the tiles in an order (see TileOrder): 5.4 GB.  Cutting rows of 64 entries and more into
 // the pieces that lie in a block of columns cost 1930 us and more: short pieces, and X rows fetched anew for each.
 template <int kBytes> struct Words { using Type = uint32_t; };  // 4, and the words of kBytes = 2
 template <> struct Words<16> { using Type = uint4; };
@@ -131,14 +131,10 @@ __device__ __forceinline__ void FmaPair(float2 &acc, const float2 &x, const floa
 
 // kSize bytes from global to shared memory; `bytes` of them are read, the rest is zero.  Copies of 16 bytes go past L1
 // (.cg) or, kNear, through it.
-template <int kSize, bool kNear = true, bool kHinted = false>
-__device__ __forceinline__ void CopyAsync(void *dst, const void *src, int bytes, [[maybe_unused]] uint64_t policy = 0)
+template <int kSize, bool kNear = true> __device__ __forceinline__ void CopyAsync(void *dst, const void *src, int bytes)
 {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    if constexpr (kHinted)
-        asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;" ::"r"(d), "l"(src), "r"(bytes), "l"(policy)
-                     : "memory");
-    else if constexpr (!kNear)
+    if constexpr (!kNear)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
     else
         asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(kSize), "r"(bytes) : "memory");
@@ -191,7 +187,9 @@ constexpr int kOrderBuckets = 1024;
 // A smaller Y stays in L2 as a whole.
 constexpr long long kOrderMinY = 96ll << 20;
 // Bytes of Y that a near tile may lie on, a third of Y at most.  1 M nodes, fp16, k = 256 (Y of 537 MB), DRAM traffic 7.6 GB without an order: 32 MB
-// 1046 us and 5.5 GB, 64 MB 1034, 96 MB 1029; with the rows of the tiles found by Preprocess, too, 976, 970 and (160 MB) 966.
+// 1046 us and 5.5 GB, 64 MB 1034, 96 MB 1029; with the rows of the tiles found by Preprocess, too, 976, 970 and (160 MB) 966.  (Copies with L2 policies, near tiles
+// evict-last and the others evict-first, picked at run time and handed to every copy, ended in an illegal instruction when the code around
+// them changed: no policy here.)
 constexpr long long kNearSpan = 160ll << 20;
 // Fewer near tiles than one in so many are not worth the turns.
 constexpr long long kNearShare = 16;
@@ -303,9 +301,9 @@ __global__ void __launch_bounds__(256) SddmmOrderTilesKernel(const int32_t *__re
 }
 
 // The dot products of a tile of entries: sDot[t] = X row sRow[t] . Y row sCol[t].  tile: a multiple of 32.
-template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear, int kBatch, bool kOrdered>
+template <typename T, int kBytes, int kLanes, int kSlabs, bool kNear, int kBatch>
 __device__ __forceinline__ void TileDots(const RowsOf &rows, unsigned char *ring, const int *sRow, const int *sCol, float *sDot,
-                                         int tile, int lane, [[maybe_unused]] uint64_t policy)
+                                         int tile, int lane)
 {
     using Shape = SddmmShape<kBytes, kSlabs, kBatch>;
     using Piece = typename Words<kBytes>::Type;
@@ -343,7 +341,7 @@ __device__ __forceinline__ void TileDots(const RowsOf &rows, unsigned char *ring
                     const int bytes = end >= 2 * q + 2 ? 4 : end > 2 * q ? 2 : 0;
                     CopyAsync<4>(slot + s * 32, row - off + (bytes > 0 ? 4ll * q : 0), bytes);
                 } else {
-                    CopyAsync<kCopy, kNear || kCopy != 16, kOrdered>(slot + s * 32, row + offset[s], inside[s], policy);
+                    CopyAsync<kCopy, kNear || kCopy != 16>(slot + s * 32, row + offset[s], inside[s]);
                 }
             }
         };
@@ -456,7 +454,6 @@ __global__ void __launch_bounds__(32 * SddmmShape<kBytes, kSlabs, kBatch, kOrder
     const float b = betaDev ? Load<T>(betaDev) : beta;
     const int lane = threadIdx.x & 31;
     long long p0 = (long long)blockIdx.x * Shape::kWarps + (threadIdx.x >> 5);
-    uint64_t policy = 0;
     int r0 = -1;
     if constexpr (kOrdered) {
         if (p0 * tile >= nnz) return;
@@ -465,27 +462,40 @@ __global__ void __launch_bounds__(32 * SddmmShape<kBytes, kSlabs, kBatch, kOrder
         const int2 at = __ldg(order.tiles + (near ? before : order.near + (p0 - before)));
         p0 = at.x;
         r0 = at.y;
-        if (near) asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(policy));
-        else asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
     }
     p0 *= tile;
     if (p0 < 0 || p0 >= nnz) return;
     unsigned char *ring = sRaw + (threadIdx.x >> 5) * (Shape::kRing + Shape::kTileBytes);
     int *sRow = reinterpret_cast<int *>(ring + Shape::kRing), *sCol = sRow + kSddmmTile;
     float *sDot = reinterpret_cast<float *>(sCol + kSddmmTile);
-    // the row that Preprocess found, if it is still the one
-    if (!kOrdered || (unsigned)r0 >= (unsigned)m || __ldg(rowPtr + r0) > p0 || __ldg(rowPtr + r0 + 1) <= p0)
-        r0 = b200sp::WarpRowOf(rowPtr, m, p0, lane);
-    for (int t = lane; t < tile; t += 32) {
+    // All columns, and the bounds of the row that Preprocess found, are asked for at once: one round trip instead of three (1 M nodes, k = 256, in
+    // order 942 us and 881 so; 100,000 rows of 10, fp32, k = 60 47 and 42).
+    int cols[kSddmmTile / 32];
+#pragma unroll
+    for (int i = 0; i < kSddmmTile / 32; ++i) {
+        const int t = i * 32 + lane;
+        cols[i] = t < tile ? __ldg(colInd + (p0 + t < nnz ? p0 + t : nnz - 1)) : 0;
+    }
+    long long end = -1;  // of that row, if the tile's first entry still lies in it
+    if (kOrdered && (unsigned)r0 < (unsigned)m) {
+        const int s = __ldg(rowPtr + r0), e = __ldg(rowPtr + r0 + 1);
+        if (s <= p0 && p0 < e) end = e;
+    }
+    const bool single = end >= p0 + tile;  // one row: a near tile's usual case
+    if (end < 0) r0 = b200sp::WarpRowOf(rowPtr, m, p0, lane);
+#pragma unroll
+    for (int i = 0; i < kSddmmTile / 32; ++i) {
+        const int t = i * 32 + lane;
+        if (i * 32 >= tile) break;
         const int p = p0 + t < nnz ? (int)p0 + t : nnz - 1;  // past the end: the last entry again, not stored
-        const int r = b200sp::RowOfLane(rowPtr, m, r0, p, lane);
+        const int r = single ? r0 : b200sp::RowOfLane(rowPtr, m, r0, p, lane);
         sRow[t] = r;
-        sCol[t] = __ldg(colInd + p);
+        sCol[t] = cols[i];
         sDot[t] = 0.0f;
-        r0 = __shfl_sync(0xffffffffu, r, 31);
+        if (!single) r0 = __shfl_sync(0xffffffffu, r, 31);
     }
     __syncwarp();
-    TileDots<T, kBytes, kLanes, kSlabs, kNear, kBatch, kOrdered>(rows, ring, sRow, sCol, sDot, tile, lane, policy);
+    TileDots<T, kBytes, kLanes, kSlabs, kNear, kBatch>(rows, ring, sRow, sCol, sDot, tile, lane);
     for (int t = lane; t < tile && p0 + t < nnz; t += 32) {
         float z = a * sDot[t];
         if (b != 0.0f) z += b * Load<T>(cVal + p0 + t);
