@@ -3,9 +3,9 @@
 // (the reference's device arithmetic, sparse/sddmm/arch35/sddmm_kernel.cpp:26-27, 424-437).  Checks, their
 // order and status codes follow the reference host layer (sparse/sddmm/arch35/sddmm_host.cpp:145-320, 478-510,
 // 660-764).  The reference reorders rows greedily over its cores in Preprocess; here the work is cut by
-// non-zeros (a warp per 32 or 64 consecutive entries of C), which needs no analysis.  For a Y that L2 does not hold Preprocess looks for an
-// order of these tiles that finds more of it there; otherwise BufferSize reports a token 256 bytes (the API wants a buffer)
-// and Preprocess only checks its arguments.
+// non-zeros (a warp per 32 or 64 consecutive entries of C), which needs no analysis.  Preprocess notes the rows of these tiles and, for a Y that L2
+// does not hold, an order that finds more of it there; for small products BufferSize reports a token 256 bytes (the
+// API wants a buffer) and Preprocess only checks its arguments.
 #include <algorithm>
 #include <atomic>
 #include <climits>
@@ -177,7 +177,8 @@ struct RowsOf {  // the operands' rows and how far apart they are
 // sixty-fourth of it.  Worked on in the order of their columns, such tiles of all rows ask for the same few megabytes of Y at any
 // time, and those stay in L2, where the tiles of short rows, in between, fetch every row of Y from DRAM.  The order is found by Preprocess (the
 // values and rows may change afterwards, the product is the same in any order) and kept in the caller's buffer: the near tiles by
-// column, then the others.  Tiles of both kinds take turns in the grid, so that neither L2 nor DRAM waits for the other.
+// column, then the others.  Tiles of both kinds take turns in the grid, so that neither L2 nor DRAM waits for the other.  With a smaller Y, or few such
+// tiles, what remains of this are the rows of the tiles.
 struct TileOrder {
     const int2 *tiles = nullptr;       // {tile, row of its first entry}; near tiles by column, then the others; nullptr: as they come
     long long near = 0;
@@ -191,6 +192,10 @@ constexpr long long kOrderMinY = 96ll << 20;
 // evict-last and the others evict-first, picked at run time and handed to every copy, ended in an illegal instruction when the code around
 // them changed: no policy here.)
 constexpr long long kNearSpan = 160ll << 20;
+// Entries from which Preprocess notes the rows of the tiles (of 64 entries; fewer entries have shorter ones), in the order they lie in if none is
+// near: a warp's search in the row offsets are four loads one after the other.  200,000 power-law rows of 12, fp16, k = 16 36.5 and 32.7 us, k = 128
+// 87 and 78, 50,000 rows of 8, k = 32, 11.5 and 10.2; k = 384 and more as without.
+constexpr long long kOrderLeast = 1 << 18;
 // Fewer near tiles than one in so many are not worth the turns.
 constexpr long long kNearShare = 16;
 struct OrderLayout {
@@ -686,12 +691,12 @@ int Launch(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const acl
     return (int)cudaGetLastError();
 }
 
-// Whether Preprocess looks for an order of the tiles: rows of Y that lie side by side, more than L2 holds, and tiles enough.
+// Whether Preprocess writes an order of the tiles: rows of Y in whole 16-byte pieces side by side, and tiles enough.
 bool MayOrder(const aclsparseDnMatDescr *Y, const aclsparseSpMatDescr *C, aclsparseOperation_t opY)
 {
     const bool rows = (opY == ACL_SPARSE_OP_TRANSPOSE) == (Y->order == ACL_SPARSE_ORDER_ROW);
     const long long bytes = Y->valueType == ACL_FLOAT16 ? 2 : 4;
-    return rows && (double)C->cols * (double)Y->ld * (double)bytes >= (double)kOrderMinY && C->nnz >= (1 << 20);
+    return rows && Y->ld * bytes % 16 == 0 && C->nnz >= kOrderLeast;
 }
 
 cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, aclsparseSpMatDescr *C, void *buffer, cudaStream_t stream)
@@ -706,12 +711,13 @@ cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, aclsparseSpMatDescr *C, voi
     int *counts = reinterpret_cast<int *>(p + L.offCounts), *starts = counts + kOrderBuckets + 1;
     auto *bucket = reinterpret_cast<int16_t *>(p + L.offBucket);
     const long long rowBytes = Y->ld * (Y->valueType == ACL_FLOAT16 ? 2ll : 4ll);
+    const int span = C->cols * rowBytes >= kOrderMinY ? (int)std::min<long long>(kNearSpan / rowBytes, C->cols / 3) : -1;  // -1: none is near
     C->sddmm.generation = b200sp::NoteBufferWrite(buffer);
     cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(int) * (kOrderBuckets + 1), stream);
     if (e != cudaSuccess) return e;
     const long long want = (L.tiles + 7) / 8, cap = (long long)b200sp_sm_count() * 8;
     SddmmTileBucketsKernel<<<(unsigned)(want < cap ? want : cap), 256, 0, stream>>>(
-        static_cast<const int32_t *>(C->indices), (int)C->nnz, (int)C->cols, (int)std::min<long long>(kNearSpan / rowBytes, C->cols / 3), L.tiles, bucket, counts);
+        static_cast<const int32_t *>(C->indices), (int)C->nnz, (int)C->cols, span, L.tiles, bucket, counts);
     SddmmBucketStartsKernel<<<1, kOrderBuckets, 0, stream>>>(counts, starts);
     int near = 0;
     e = cudaMemcpyAsync(&near, starts + kOrderBuckets, sizeof(near), cudaMemcpyDeviceToHost, stream);
@@ -733,9 +739,9 @@ TileOrder OrderOf(const aclsparseSpMatDescr *C, const void *buffer)
 {
     const auto &plan = C->sddmm;
     const OrderLayout L = OrderLayoutFor(C->nnz);
-    if (plan.buffer == nullptr || plan.buffer != buffer || plan.nnz != C->nnz || plan.generation != b200sp::BufferGeneration(buffer) ||
-        plan.near * kNearShare < L.tiles)
+    if (plan.buffer == nullptr || plan.buffer != buffer || plan.nnz != C->nnz || plan.generation != b200sp::BufferGeneration(buffer))
         return {};
+    if (plan.near * kNearShare < L.tiles) return {reinterpret_cast<const int2 *>(static_cast<const char *>(buffer) + L.offTiles), 0, 0};
     return {reinterpret_cast<const int2 *>(static_cast<const char *>(buffer) + L.offTiles), plan.near,
             (((unsigned long long)plan.near << 32) + (unsigned long long)L.tiles - 1) / (unsigned long long)L.tiles};
 }

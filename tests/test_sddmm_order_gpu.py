@@ -14,14 +14,14 @@ pytestmark = pytest.mark.gpu
 class Case:
     """Rows of 16 to 30,000 entries among short ones; a last tile that is not full."""
 
-    def __init__(self, pkg, handle, device, dtype, k, seed=0, nnz=(1 << 20) + 77):
+    def __init__(self, pkg, handle, device, dtype, k, seed=0, nnz=(1 << 20) + 77, cols=0):
         from ops_sparse_b200 import api
         self.pkg, self.handle, self.device = pkg, handle, device
         half = dtype == "f16"
-        self.cols, tdt = (100 << 20) // (k * (2 if half else 4)) + 3, torch.float16 if half else torch.float32
+        self.cols, tdt = cols or (100 << 20) // (k * (2 if half else 4)) + 3, torch.float16 if half else torch.float32
         rng = np.random.default_rng(seed)
         lengths = np.concatenate([[30000, 16, 1, 0, 2000, 64, 63, 65], rng.integers(100, 3000, 300), rng.integers(0, 9, 40000)])
-        lengths = rng.permutation(lengths)
+        lengths = rng.permutation(lengths[np.cumsum(lengths) < nnz])
         lengths[-1] += nnz - lengths.sum()
         self.m, self.nnz, self.k = lengths.size, nnz, k
         self.row_ptr = torch.from_numpy(np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)).to(device)
@@ -73,12 +73,25 @@ def test_order(pkg, handle, device, dtype, k):
     plain = case.product(torch.empty(256, dtype=torch.uint8, device=device))  # never preprocessed: no order
     case.check(plain)
     buf = case.buffer()
-    assert buf.numel() > 256
+    assert (buf.numel() > 256) == (k != 100)
     assert torch.equal(case.product(buf), plain)    # of the right size, but not preprocessed
     case.preprocess(buf)
     assert torch.equal(case.product(buf), plain)
     other = torch.empty(256, dtype=torch.uint8, device=device)
     assert torch.equal(case.product(other), plain)  # another buffer than the one with the order
+
+
+# a Y that L2 holds, one that comes through L1, and a matrix too small for an order
+@pytest.mark.parametrize("cols,nnz", [(5000, (1 << 18) + 1), (60, 1 << 18), (5000, (1 << 18) - 1), (5000, 1_000_003)])
+@pytest.mark.parametrize("dtype,k", [("f16", 64), ("f32", 256), ("f16", 384)])
+def test_rows_of_tiles(pkg, handle, device, dtype, k, cols, nnz):
+    case = Case(pkg, handle, device, dtype, k, nnz=nnz, cols=cols)
+    plain = case.product(torch.empty(256, dtype=torch.uint8, device=device))
+    case.check(plain)
+    buf = case.buffer()
+    assert (buf.numel() > 256) == (nnz >= 1 << 18)
+    case.preprocess(buf)
+    assert torch.equal(case.product(buf), plain)
 
 
 def test_pattern_and_buffer_that_change(pkg, handle, device):
