@@ -955,7 +955,7 @@ __device__ void UnitSum(const FastArgs<ValT, OutT> &a, unsigned char *sWarp)
 // row's first columns once more and stores nothing.
 //
 // kLayout: kPlain wants C row-major with 16-byte aligned rows, like B; kAnyC takes any C, kAnyCWords also rows of B on
-// any 4-byte boundaries, by words (see WorthRepacking).  Sums of kAnyC go through shared memory and are written along the
+// any 4-byte boundaries, by words (see WorthRepacking); the kinds with Add are for a beta other than 0.  Sums of kAnyC go through shared memory and are written along the
 // contiguous direction of C: by a warp where that is the row's, else by the CTA, which takes a.genRows rows (of
 // column-major fp16 C, 32 rows are 64 bytes; straight from registers every element would be a 32-byte sector of its
 // own) unless there are too few rows to give every SM a CTA.
@@ -972,7 +972,7 @@ template <typename ValT, int kLanes> struct FastShape {
     static constexpr bool kMayLoop = std::is_same_v<ValT, int8_t> && (kLanes == 2 || kLanes == 4);
 };
 
-enum { kPlain, kAnyC, kAnyCWords };
+enum { kPlain, kAnyC, kAnyCWords, kAnyCAdd, kAnyCWordsAdd };
 // Rows of a few entries are a chain of dependent loads (row offsets, columns, B, C): warps hide it, so registers are held to
 // what 36 warps per SM leave (24 for wide int8 rows, whose quads of B rows need more).
 template <typename ValT, int kLanes> constexpr int kFastCtas = std::is_same_v<ValT, int8_t> && kLanes >= 8 ? 6 : 9;
@@ -982,7 +982,8 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
     using Acc = typename Arith<ValT>::Acc;
     using Shape = FastShape<ValT, kLanes>;
     constexpr bool kInt8 = std::is_same_v<ValT, int8_t>;
-    constexpr bool kGenC = kLayout != kPlain, kWords = kLayout == kAnyCWords;
+    constexpr bool kGenC = kLayout != kPlain, kWords = kLayout == kAnyCWords || kLayout == kAnyCWordsAdd;
+    constexpr bool kAdds = kLayout >= kAnyCAdd;  // beta may be other than 0 (fp types)
     constexpr int E = Pack<ValT>::kElems;
     constexpr int kGroup = Shape::kGroup;
     constexpr int kRowsPerWarp = 32 / kGroup;
@@ -1014,6 +1015,27 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
     auto storeOne = [&](long long row, int col, Acc v) {
         OutT *dst = a.C + row * a.cRow + col * a.cCol;
         *dst = Finish<OutT>(v, alpha, beta, dst);
+    };
+
+    // Some of them, beta not 0: what C holds is read for all before any is written, since a load waits for the store before it otherwise, a round
+    // trip to memory per element (column-major, beta = 0.5, bf16, 900,000 rows of 2, N = 100 471 us and 323 in eights, 341 in fours).  In kernels of
+    // their own: with beta = 0, where nothing is read, the code for it costs 1 to 10 %.
+    [[maybe_unused]] constexpr int kStoreBatch = 8;
+    [[maybe_unused]] auto addSome = [&]<int kSome>(auto elementOf) {  // elementOf(u, row, column, value): whether there is such an element
+        OutT *dst[kSome], old[kSome];
+        Acc v[kSome];
+#pragma unroll
+        for (int u = 0; u < kSome; ++u) {
+            long long row = 0;
+            int col = 0;
+            v[u] = Acc(0);
+            dst[u] = elementOf(u, row, col, v[u]) ? a.C + row * a.cRow + col * a.cCol : nullptr;
+            old[u] = OutT{};
+            if (dst[u] != nullptr) old[u] = *dst[u];
+        }
+#pragma unroll
+        for (int u = 0; u < kSome; ++u)
+            if (dst[u] != nullptr) *dst[u] = Finish<OutT>(v[u], alpha, beta, &old[u]);
     };
 
     constexpr int kCols = kInt8 ? 1 : 4 / (int)sizeof(ValT);
@@ -1111,11 +1133,30 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
                             for (int i = 0; i < E; ++i)
                                 if (owner) sWarp[lane / kGroup * kTileCols + columnOf(0, i)] = acc[i];
                             __syncwarp();
-#pragma unroll
-                            for (int i = lane; i < kRowsPerWarp * kTileCols; i += 32) {
-                                const int g = i / kTileCols, c = colT + i % kTileCols;
+                            auto element = [&](int i, long long &toRow, int &toCol, Acc &v) {
+                                const int g = i / kTileCols;
                                 const int r = kByLength ? __shfl_sync(0xffffffffu, rowIn, g * kGroup) : warp * kRowsPerWarp + g;
-                                if (c < a.n && !(skipped >> (g * kGroup) & 1)) storeOne(row0 + r, c, sWarp[i]);
+                                toRow = row0 + r;
+                                toCol = colT + i % kTileCols;
+                                v = sWarp[i];
+                                return toCol < a.n && !(skipped >> (g * kGroup) & 1);
+                            };
+                            constexpr int kElements = kRowsPerWarp * kTileCols;  // a multiple of 32: all lanes take part in every step
+                            if (!kAdds || beta == 0) {
+#pragma unroll
+                                for (int i = lane; i < kElements; i += 32) {
+                                    long long toRow;
+                                    int toCol;
+                                    Acc v;
+                                    if (element(i, toRow, toCol, v)) storeOne(toRow, toCol, v);
+                                }
+                            } else if constexpr (kAdds) {
+                                constexpr int kSome = kElements / 32 < kStoreBatch ? kElements / 32 : kStoreBatch;
+                                static_assert(kElements % (32 * kSome) == 0);
+                                for (int i0 = lane; i0 < kElements; i0 += 32 * kSome)
+                                    addSome.template operator()<kSome>([&](int u, long long &toRow, int &toCol, Acc &v) {
+                                        return element(i0 + u * 32, toRow, toCol, v);
+                                    });
                             }
                         }
                     } else {
@@ -1125,9 +1166,22 @@ __global__ void __launch_bounds__(kThreads, kFastCtas<ValT, kLanes>) SpmmFastKer
             }
             if (rowsRun) {
                 __syncthreads();
-                for (int i = threadIdx.x; i < blockRows * kTileCols; i += kThreads) {  // consecutive threads on consecutive rows
-                    const int c = i / blockRows, r = i - c * blockRows;
-                    if (col0 + c < a.n && !sSkip[r]) storeOne(row0 + r, col0 + c, sBuf[r * kTileStride + c]);
+                if (!kAdds || beta == 0) {
+                    for (int i = threadIdx.x; i < blockRows * kTileCols; i += kThreads) {  // consecutive threads on consecutive rows
+                        const int c = i / blockRows, r = i - c * blockRows;
+                        if (col0 + c < a.n && !sSkip[r]) storeOne(row0 + r, col0 + c, sBuf[r * kTileStride + c]);
+                    }
+                } else if constexpr (kAdds) {
+                    for (int i0 = threadIdx.x; i0 < blockRows * kTileCols; i0 += kThreads * kStoreBatch)
+                        addSome.template operator()<kStoreBatch>([&](int u, long long &toRow, int &toCol, Acc &v) {
+                            const int i = i0 + u * kThreads;
+                            if (i >= blockRows * kTileCols) return false;
+                            const int c = i / blockRows, r = i - c * blockRows;
+                            toRow = row0 + r;
+                            toCol = col0 + c;
+                            v = sBuf[r * kTileStride + c];
+                            return toCol < a.n && !sSkip[r];
+                        });
                 }
                 __syncthreads();
             }
@@ -2336,8 +2390,12 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             auto go = [&](auto kernel) { err = b200sp::LaunchChained(kernel, (unsigned)grid, kThreads, 0, st, a); };
             auto pick = [&]<bool kKahan, bool kOrdered>() {
                 if (cPlain) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kPlain, kOrdered>);
-                if constexpr (!kInt8)
+                if constexpr (!kInt8) {
+                    const bool adds = s->beta_dev != nullptr || s->beta_f != 0.0f;
+                    if (words && adds) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyCWordsAdd, kOrdered>);
                     if (words) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyCWords, kOrdered>);
+                    if (adds) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyCAdd, kOrdered>);
+                }
                 go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyC, kOrdered>);
             };
             auto pickOrder = [&]<bool kKahan>() {
