@@ -228,6 +228,7 @@ aclsparseStatus_t aclsparseCsr2cscEx2(aclsparseHandle_t handle, int m, int n, in
     }
     if (buffer == nullptr) return ACL_SPARSE_STATUS_INSUFFICIENT_RESOURCES;  // csr2csc_ex2_host.cpp:298-310
 
+    (void)b200sp::NoteBufferWrite(buffer);  // an analysis that lies in it is stale now
     const Layout L = LayoutFor(nnz);
     char *p = static_cast<char *>(buffer);
     const Arrays work{reinterpret_cast<int *>(p + L.offKeys), reinterpret_cast<int *>(p + L.offRows), p + L.offVals};

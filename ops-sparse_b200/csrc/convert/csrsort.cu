@@ -108,6 +108,7 @@ aclsparseStatus_t aclsparseXcsrsort(aclsparseHandle_t handle, int m, int n, int 
     if (pBuffer == nullptr) return ACL_SPARSE_STATUS_INVALID_VALUE;
 
     cudaStream_t stream = handle->stream;
+    (void)b200sp::NoteBufferWrite(pBuffer);  // an analysis that lies in it is stale now
     const SortLayout L = SortLayoutFor(m, nnz);
     char *w = static_cast<char *>(pBuffer);
     auto *keys = reinterpret_cast<unsigned long long *>(w + L.offKeys);

@@ -121,6 +121,7 @@ aclsparseStatus_t aclsparseSpMVOp_createDescr(aclsparseHandle_t handle, aclspars
     d->csrValues = matA->values;
     d->alg = alg == ACL_SPARSE_SPMVOP_ALG_DEFAULT ? ACL_SPARSE_SPMVOP_ALG1 : alg;
     if (d->alg == ACL_SPARSE_SPMVOP_ALG2) {
+        (void)b200sp::NoteBufferWrite(buffer);  // an analysis that lies in it is stale now
         const int rc = b200sp_spmvop_analyze(d->csrRowOffsets, d->rowOffsetType == ACL_SPARSE_INDEX_64I, d->m,
                                              buffer, b200sp_spmvop_plan_bytes(d->m), d->classStart, handle->stream);
         if (rc != 0) {

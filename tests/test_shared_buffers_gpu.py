@@ -1,0 +1,91 @@
+"""GPU: one buffer that several operations are given, one after the other: none trusts what another has written over."""
+from __future__ import annotations
+
+from ctypes import byref, c_size_t, c_void_p
+
+import numpy as np
+import pytest
+import torch
+
+from test_sddmm_order_gpu import Case
+
+pytestmark = pytest.mark.gpu
+
+
+def at(t):
+    return c_void_p(t.data_ptr())
+
+
+class Writer:
+    """A library call that writes its buffer: `bytes` it wants, `write(buf)`."""
+
+    def __init__(self, pkg, handle, case, kind):
+        self.pkg, self.L, self.handle, self.kind = pkg, pkg.lib(), handle, kind
+        h, m, n, nnz, size = handle.raw, case.m, case.cols, case.nnz, c_size_t()
+        rp, self.ci = case.row_ptr, case.col_ind.clone()
+        if kind == "csr2csc":
+            self.val = torch.rand(nnz, device=case.device)
+            self.out = [torch.empty(nnz, device=case.device), *(torch.empty(s, dtype=torch.int32, device=case.device) for s in (n + 1, nnz))]
+            self.args = (h, m, n, nnz, at(self.val), at(rp), at(self.ci), *map(at, self.out), pkg.ACL_FLOAT, 1, 0, 0)
+            pkg.check(self.L.aclsparseCsr2cscEx2_bufferSize(*self.args, byref(size)), "size")
+        elif kind == "csrsort":
+            self.descr, self.P = c_void_p(), torch.arange(nnz, dtype=torch.int32, device=case.device)
+            pkg.check(self.L.aclsparseCreateMatDescr(byref(self.descr)), "descr")
+            self.args = (h, m, n, nnz, self.descr, at(rp), at(self.ci), at(self.P))
+            pkg.check(self.L.aclsparseXcsrsort_bufferSizeExt(h, m, n, nnz, at(rp), at(self.ci), byref(size)), "size")
+        else:
+            from ops_sparse_b200 import api
+            self.A = api.CsrMatrix(rp, self.ci, torch.rand(nnz, device=case.device), m, n)
+            self.x, self.y = (api.DnVec(torch.rand(s, device=case.device)) for s in (n, m))
+            self.args = (0, self.A.raw, self.x.raw, self.y.raw, self.y.raw, pkg.ACL_FLOAT, 2)
+            self.descr = c_void_p()
+            pkg.check(self.L.aclsparseSpMVOp_bufferSize(h, *self.args, byref(size)), "size")
+        self.bytes = size.value
+
+    def write(self, buf):
+        if self.kind == "csr2csc":
+            status = self.L.aclsparseCsr2cscEx2(*self.args, at(buf))
+        elif self.kind == "csrsort":
+            status = self.L.aclsparseXcsrsort(*self.args, at(buf))
+        else:
+            status = self.L.aclsparseSpMVOp_createDescr(self.handle.raw, byref(self.descr), *self.args, at(buf))
+        self.pkg.check(status, self.kind)
+
+    def close(self):
+        if self.kind == "csrsort":
+            self.L.aclsparseDestroyMatDescr(self.descr)
+        elif self.kind == "spmvop":
+            self.L.aclsparseSpMVOp_destroyDescr(self.descr)
+
+
+@pytest.mark.parametrize("kind", ["csr2csc", "csrsort", "spmvop"])
+def test_sddmm_order_written_over(pkg, handle, device, kind):
+    case = Case(pkg, handle, device, "f16", 128)
+    writer = Writer(pkg, handle, case, kind)
+    plain = case.product(torch.empty(256, dtype=torch.uint8, device=device))
+    buf = torch.empty(max(case.buffer().numel(), writer.bytes), dtype=torch.uint8, device=device)
+    case.preprocess(buf)
+    writer.write(buf)
+    assert torch.equal(case.product(buf), plain)
+    writer.close()
+
+
+@pytest.mark.parametrize("kind", ["csr2csc", "csrsort", "spmvop"])
+def test_spmv_plan_written_over(pkg, handle, device, kind):
+    from ops_sparse_b200 import api
+    case = Case(pkg, handle, device, "f32", 4, nnz=300_000, cols=50_000)
+    writer = Writer(pkg, handle, case, kind)
+    val, x = torch.rand(case.nnz, device=device), torch.rand(case.cols, device=device)
+    A, dx, dy = api.CsrMatrix(case.row_ptr, case.col_ind, val, case.m, case.cols), api.DnVec(x), api.DnVec(torch.empty(case.m, device=device))
+    size = api.spmv_preprocess(handle, A, dx, dy).numel()
+    buf = torch.empty(max(size, writer.bytes), dtype=torch.uint8, device=device)
+    null = c_void_p()
+    pkg.check(pkg.lib().aclsparseSpMVPreprocess(handle.raw, 0, null, A.raw, dx.raw, null, dy.raw, pkg.ACL_FLOAT, 0, at(buf)), "preprocess")
+    writer.write(buf)
+    api.spmv(handle, A, dx, dy, 1.0, 0.0, buffer=buf)
+    torch.cuda.synchronize()
+    want = torch.zeros(case.m, dtype=torch.float64, device=device).index_add(0, case.rows, val.double() * x.double()[case.col_ind.long()])
+    count = torch.bincount(case.rows, minlength=case.m)
+    # all terms are positive: (additions + 3) half ulps of the sum
+    assert bool(((dy.values.double() - want).abs() <= (count + 3) * 2.0 ** -24 * want).all())
+    writer.close()
