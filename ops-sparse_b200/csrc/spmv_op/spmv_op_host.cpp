@@ -16,6 +16,7 @@ struct aclsparseSpMVOpDescr {
     const void *csrValues = nullptr;
     aclsparseSpMVOpAlg_t alg = ACL_SPARSE_SPMVOP_ALG1;
     void *userBuffer = nullptr;                         // ALG2: the caller's workspace (row order)
+    uint64_t generation = 0;                            // ... BufferGeneration(userBuffer) when it was written
     int32_t classStart[B200SP_SPMVOP_CLASSES + 1] = {};  // ALG2: where each length class starts in it
 };
 
@@ -121,7 +122,7 @@ aclsparseStatus_t aclsparseSpMVOp_createDescr(aclsparseHandle_t handle, aclspars
     d->csrValues = matA->values;
     d->alg = alg == ACL_SPARSE_SPMVOP_ALG_DEFAULT ? ACL_SPARSE_SPMVOP_ALG1 : alg;
     if (d->alg == ACL_SPARSE_SPMVOP_ALG2) {
-        (void)b200sp::NoteBufferWrite(buffer);  // an analysis that lies in it is stale now
+        d->generation = b200sp::NoteBufferWrite(buffer);  // an analysis that lies in it is stale now
         const int rc = b200sp_spmvop_analyze(d->csrRowOffsets, d->rowOffsetType == ACL_SPARSE_INDEX_64I, d->m,
                                              buffer, b200sp_spmvop_plan_bytes(d->m), d->classStart, handle->stream);
         if (rc != 0) {
@@ -210,7 +211,9 @@ aclsparseStatus_t aclsparseSpMVOp(aclsparseHandle_t handle, aclsparseSpMVOpPlan_
     if (d->nnz == 0) {
         rc = b200sp_spmvop_scale(y, z, d->m, b, bDev, handle->stream);
     } else {
-        const bool planned = d->alg == ACL_SPARSE_SPMVOP_ALG2 && d->userBuffer != nullptr;
+        // A row order that another call has written over since is not followed: the rows as they lie, as ALG1 takes them.
+        const bool planned = d->alg == ACL_SPARSE_SPMVOP_ALG2 && d->userBuffer != nullptr &&
+                             d->generation == b200sp::BufferGeneration(d->userBuffer);
         rc = b200sp_spmvop_launch(d->csrRowOffsets, d->rowOffsetType == ACL_SPARSE_INDEX_64I,
                                   static_cast<const int32_t *>(d->csrColInd), static_cast<const float *>(d->csrValues),
                                   static_cast<const float *>(vecX->values), y, z, d->m, d->nnz,

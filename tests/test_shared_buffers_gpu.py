@@ -1,7 +1,7 @@
 """GPU: one buffer that several operations are given, one after the other: none trusts what another has written over."""
 from __future__ import annotations
 
-from ctypes import byref, c_size_t, c_void_p
+from ctypes import addressof, byref, c_float, c_size_t, c_void_p
 
 import numpy as np
 import pytest
@@ -89,3 +89,32 @@ def test_spmv_plan_written_over(pkg, handle, device, kind):
     # all terms are positive: (additions + 3) half ulps of the sum
     assert bool(((dy.values.double() - want).abs() <= (count + 3) * 2.0 ** -24 * want).all())
     writer.close()
+
+
+@pytest.mark.parametrize("kind", ["csr2csc", "csrsort", "spmvop", "spmv"])
+def test_row_order_of_spmvop_written_over(pkg, handle, device, kind):
+    from ops_sparse_b200 import api
+    case = Case(pkg, handle, device, "f32", 4, nnz=300_000, cols=50_000)
+    A = api.CsrMatrix(case.row_ptr, case.col_ind, torch.rand(case.nnz, device=device), case.m, case.cols)
+    x, y, z = (api.DnVec(torch.rand(s, device=device)) for s in (case.cols, case.m, case.m))
+    fewer = Case(pkg, handle, device, "f32", 4, seed=5, nnz=200_000, cols=50_000)
+    other = Writer(pkg, handle, fewer, "csrsort" if kind == "spmv" else kind)
+    args, null, size, descr, plan = (0, A.raw, x.raw, y.raw, z.raw, pkg.ACL_FLOAT, 2), c_void_p(), c_size_t(), c_void_p(), c_void_p()
+    pkg.check(pkg.lib().aclsparseSpMVOp_bufferSize(handle.raw, *args, byref(size)), "size")
+    buf = torch.empty(max(size.value, other.bytes, api.spmv_buffer_size(handle, A, x, y)), dtype=torch.uint8, device=device)
+    pkg.check(pkg.lib().aclsparseSpMVOp_createDescr(handle.raw, byref(descr), *args, at(buf)), "descr")
+    pkg.check(pkg.lib().aclsparseSpMVOp_createPlan(handle.raw, descr, byref(plan), None, 0), "plan")
+    if kind == "spmv":
+        pkg.check(pkg.lib().aclsparseSpMVPreprocess(handle.raw, 0, null, A.raw, x.raw, null, y.raw, pkg.ACL_FLOAT, 0, at(buf)), "preprocess")
+    else:
+        other.write(buf)
+    a, b = c_float(1.0), c_float(0.0)
+    pkg.check(pkg.lib().aclsparseSpMVOp(handle.raw, plan, c_void_p(addressof(a)), c_void_p(addressof(b)), x.raw, y.raw, z.raw), "product")
+    torch.cuda.synchronize()
+    terms = A.values.double() * x.values.double()[case.col_ind.long()]
+    want = torch.zeros(case.m, dtype=torch.float64, device=device).index_add(0, case.rows, terms)
+    # compensated sums of positive terms
+    assert bool(((z.values.double() - want).abs() <= 8 * 2.0 ** -24 * want).all())
+    pkg.lib().aclsparseSpMVOp_destroyPlan(plan)
+    pkg.lib().aclsparseSpMVOp_destroyDescr(descr)
+    other.close()
