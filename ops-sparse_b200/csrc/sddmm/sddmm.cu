@@ -179,9 +179,16 @@ struct RowsOf {  // the operands' rows and how far apart they are
 // values and rows may change afterwards, the product is the same in any order) and kept in the caller's buffer: the near tiles by
 // column, then the others.  Tiles of both kinds take turns in the grid, so that neither L2 nor DRAM waits for the other.  With a smaller Y, or few such
 // tiles, what remains of this are the rows of the tiles.
+//
+// What the buffer holds when a product runs is not known: it may have been written by code that this library does not see, or be other memory at the
+// same address, and a product in a graph may run after any call.  So nothing is taken from it on trust: rows are compared with the row
+// offsets, and before an order is followed a kernel looks whether it names every tile once; if not, the tiles are taken as they lie.  (That kernel takes
+// 4 us of 1000.  A kernel whose warps see for themselves whose tile is whose takes 31 us longer.)
 struct TileOrder {
-    const int2 *tiles = nullptr;       // {tile, row of its first entry}; near tiles by column, then the others; nullptr: as they come
-    long long near = 0;
+    const int2 *tiles = nullptr;       // {tile, row of its first entry}; near tiles by column, then the others; nullptr: no order and no rows
+    const int *place = nullptr;        // [tile] where it stands in `tiles`
+    int *bad = nullptr;                // not 0: not an order.  Preprocess writes 0, a product 1, nobody 0 again
+    long long near = 0;                // 0: all tiles stand where they lie, and there is nothing to look at but rows
     unsigned long long share = 0;      // of the near tiles among all, times 2^32, rounded up
 };
 constexpr int kOrderBuckets = 1024;
@@ -200,7 +207,7 @@ constexpr long long kOrderLeast = 1 << 18;
 constexpr long long kNearShare = 16;
 struct OrderLayout {
     long long tiles;
-    size_t offCounts, offBucket, offTiles, total;
+    size_t offCounts, offBucket, offTiles, offPlace, total;
 };
 inline OrderLayout OrderLayoutFor(long long nnz)
 {
@@ -210,7 +217,8 @@ inline OrderLayout OrderLayoutFor(long long nnz)
     L.offBucket = L.offCounts + sizeof(int32_t) * 2 * (kOrderBuckets + 1);
     L.offBucket = (L.offBucket + 255) / 256 * 256;
     L.offTiles = (L.offBucket + sizeof(int16_t) * (size_t)L.tiles + 255) / 256 * 256;
-    L.total = L.offTiles + sizeof(int2) * (size_t)L.tiles;
+    L.offPlace = L.offTiles + sizeof(int2) * (size_t)L.tiles;
+    L.total = L.offPlace + sizeof(int32_t) * (size_t)L.tiles;
     return L;
 }
 
@@ -273,9 +281,29 @@ __global__ void __launch_bounds__(kOrderBuckets) SddmmBucketStartsKernel(const i
     if (threadIdx.x == kOrderBuckets - 1) starts[kOrderBuckets] = upTo;
 }
 
+// Row of entry p: the last one that starts at or before it.
+__device__ __forceinline__ int RowOfEntry(const int32_t *rowPtr, int m, long long p)
+{
+    int lo = 0, hi = m - 1;
+    while (lo < hi) {
+        const int mid = lo + ((hi - lo + 1) >> 1);
+        if (__ldg(rowPtr + mid) <= p) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// A thread per tile: where it lies, and its row.
+__global__ void __launch_bounds__(256) SddmmTileRowsKernel(const int32_t *__restrict__ rowPtr, int m, long long tiles, int2 *__restrict__ order)
+{
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < tiles) order[t] = make_int2((int)t, RowOfEntry(rowPtr, m, t * kSddmmTile));
+}
+
 // A CTA per 1024 tiles: their places.  Inside a bucket as the CTAs come, the others nearly as they lie.
 __global__ void __launch_bounds__(256) SddmmOrderTilesKernel(const int32_t *__restrict__ rowPtr, int m, const int16_t *__restrict__ bucket,
-                                                             long long tiles, int *__restrict__ starts, int2 *__restrict__ order)
+                                                             long long tiles, int *__restrict__ starts, int2 *__restrict__ order,
+                                                             int *__restrict__ place)
 {
     __shared__ int sCount[kOrderBuckets + 1], sStart[kOrderBuckets + 1];
     for (int i = threadIdx.x; i <= kOrderBuckets; i += blockDim.x) sCount[i] = 0;
@@ -295,14 +323,20 @@ __global__ void __launch_bounds__(256) SddmmOrderTilesKernel(const int32_t *__re
     for (int i = 0; i < 4; ++i)
         if (mine[i] >= 0) {
             const int t = (int)(t0 + i * 256);
-            int lo = 0, hi = m - 1;  // row of its first entry: largest r with rowPtr[r] <= p
-            while (lo < hi) {
-                const int mid = lo + ((hi - lo + 1) >> 1);
-                if ((long long)__ldg(rowPtr + mid) <= (long long)t * kSddmmTile) lo = mid;
-                else hi = mid - 1;
-            }
-            order[sStart[mine[i]] + at[i]] = make_int2(t, lo);
+            const int to = sStart[mine[i]] + at[i];
+            order[to] = make_int2(t, RowOfEntry(rowPtr, m, (long long)t * kSddmmTile));
+            place[t] = to;
         }
+}
+
+// A thread per tile: whether it stands somewhere, and there alone.
+__global__ void __launch_bounds__(256) SddmmOrderCheckKernel(const int2 *__restrict__ order, const int *__restrict__ place, int tiles, int *bad)
+{
+    b200sp::WaitForPrevious();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= tiles) return;
+    const int at = __ldg(place + t);
+    if ((unsigned)at >= (unsigned)tiles || __ldg(&order[at].x) != t) *bad = 1;
 }
 
 // The dot products of a tile of entries: sDot[t] = X row sRow[t] . Y row sCol[t].  tile: a multiple of 32.
@@ -459,17 +493,17 @@ __global__ void __launch_bounds__(32 * SddmmShape<kBytes, kSlabs, kBatch, kOrder
     const float b = betaDev ? Load<T>(betaDev) : beta;
     const int lane = threadIdx.x & 31;
     long long p0 = (long long)blockIdx.x * Shape::kWarps + (threadIdx.x >> 5);
+    if (p0 * tile >= nnz) return;
     int r0 = -1;
     if constexpr (kOrdered) {
-        if (p0 * tile >= nnz) return;
         const unsigned before = (unsigned)((p0 * order.share) >> 32);
         const bool near = (unsigned)(((p0 + 1) * order.share) >> 32) != before;
         const int2 at = __ldg(order.tiles + (near ? before : order.near + (p0 - before)));
-        p0 = at.x;
+        if (order.near != 0 && __ldg(order.bad) == 0) p0 = at.x;
         r0 = at.y;
     }
     p0 *= tile;
-    if (p0 < 0 || p0 >= nnz) return;
+    if (kOrdered && (p0 < 0 || p0 >= nnz)) return;
     unsigned char *ring = sRaw + (threadIdx.x >> 5) * (Shape::kRing + Shape::kTileBytes);
     int *sRow = reinterpret_cast<int *>(ring + Shape::kRing), *sCol = sRow + kSddmmTile;
     float *sDot = reinterpret_cast<float *>(sCol + kSddmmTile);
@@ -639,7 +673,16 @@ int LaunchRows(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const
     auto launch = [&]<int kLanes, int kSlabs>() {
         constexpr int kShort = kShortBatch<kBytes, kLanes, kSlabs>;
         if constexpr (kBytes == 16)
-            if (order.tiles != nullptr && tile == kSddmmTile && !near) return launchAs.template operator()<kLanes, kSlabs, false, kShort, true>();
+            if (order.tiles != nullptr && tile == kSddmmTile && !near) {
+                if (order.near > 0) {
+                    const int tiles = (nnz - 1) / kSddmmTile + 1;
+                    b200sp_note_launches(1);
+                    const cudaError_t e = b200sp::LaunchChained(SddmmOrderCheckKernel, (unsigned)((tiles + 255) / 256), 256, 0, stream, order.tiles,
+                                                                order.place, tiles, order.bad);
+                    if (e != cudaSuccess) return (int)e;
+                }
+                return launchAs.template operator()<kLanes, kSlabs, false, kShort, true>();
+            }
         const long long warps = (nnz + 31ll) / 32 / b200sp_sm_count();  // for every SM, with the shortest tiles
         if constexpr (kShort < 4)
             if (warps < SddmmShape<kBytes, kSlabs, 4>::kWarpsPerSm) return launchDeep.template operator()<kLanes, kSlabs, 4>();
@@ -713,7 +756,7 @@ cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, aclsparseSpMatDescr *C, voi
     const long long rowBytes = Y->ld * (Y->valueType == ACL_FLOAT16 ? 2ll : 4ll);
     const int span = C->cols * rowBytes >= kOrderMinY ? (int)std::min<long long>(kNearSpan / rowBytes, C->cols / 3) : -1;  // -1: none is near
     C->sddmm.generation = b200sp::NoteBufferWrite(buffer);
-    cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(int) * (kOrderBuckets + 1), stream);
+    cudaError_t e = cudaMemsetAsync(p, 0, L.offCounts + sizeof(int) * (kOrderBuckets + 1), stream);  // and TileOrder::bad
     if (e != cudaSuccess) return e;
     const long long want = (L.tiles + 7) / 8, cap = (long long)b200sp_sm_count() * 8;
     SddmmTileBucketsKernel<<<(unsigned)(want < cap ? want : cap), 256, 0, stream>>>(
@@ -723,11 +766,20 @@ cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, aclsparseSpMatDescr *C, voi
     e = cudaMemcpyAsync(&near, starts + kOrderBuckets, sizeof(near), cudaMemcpyDeviceToHost, stream);
     if (e != cudaSuccess) return e;
     SddmmOrderTilesKernel<<<(unsigned)((L.tiles + 1023) / 1024), 256, 0, stream>>>(
-        static_cast<const int32_t *>(C->offsets), (int)C->rows, bucket, L.tiles, starts, reinterpret_cast<int2 *>(p + L.offTiles));
+        static_cast<const int32_t *>(C->offsets), (int)C->rows, bucket, L.tiles, starts, reinterpret_cast<int2 *>(p + L.offTiles),
+        reinterpret_cast<int *>(p + L.offPlace));
     b200sp_note_launches(3);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return e;
+    if (near * kNearShare < L.tiles) {
+        near = 0;
+        SddmmTileRowsKernel<<<(unsigned)((L.tiles + 255) / 256), 256, 0, stream>>>(static_cast<const int32_t *>(C->offsets), (int)C->rows,
+                                                                                   L.tiles, reinterpret_cast<int2 *>(p + L.offTiles));
+        b200sp_note_launches(1);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
     C->sddmm.near = near;
     C->sddmm.nnz = C->nnz;
     C->sddmm.buffer = buffer;
@@ -735,14 +787,14 @@ cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, aclsparseSpMatDescr *C, voi
 }
 
 // The order that Preprocess left in the buffer, if it is still there and worth following.
-TileOrder OrderOf(const aclsparseSpMatDescr *C, const void *buffer)
+TileOrder OrderOf(const aclsparseSpMatDescr *C, void *buffer)
 {
     const auto &plan = C->sddmm;
     const OrderLayout L = OrderLayoutFor(C->nnz);
     if (plan.buffer == nullptr || plan.buffer != buffer || plan.nnz != C->nnz || plan.generation != b200sp::BufferGeneration(buffer))
         return {};
-    if (plan.near * kNearShare < L.tiles) return {reinterpret_cast<const int2 *>(static_cast<const char *>(buffer) + L.offTiles), 0, 0};
-    return {reinterpret_cast<const int2 *>(static_cast<const char *>(buffer) + L.offTiles), plan.near,
+    char *p = static_cast<char *>(buffer);
+    return {reinterpret_cast<const int2 *>(p + L.offTiles), reinterpret_cast<const int *>(p + L.offPlace), reinterpret_cast<int *>(p), plan.near,
             (((unsigned long long)plan.near << 32) + (unsigned long long)L.tiles - 1) / (unsigned long long)L.tiles};
 }
 

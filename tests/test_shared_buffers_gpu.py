@@ -118,3 +118,55 @@ def test_row_order_of_spmvop_written_over(pkg, handle, device, kind):
     pkg.lib().aclsparseSpMVOp_destroyPlan(plan)
     pkg.lib().aclsparseSpMVOp_destroyDescr(descr)
     other.close()
+
+
+def foreign(kind, buf, kept, gen):
+    """Bytes that no call of the library wrote."""
+    n, words = buf.numel(), buf[: buf.numel() // 8 * 8].view(torch.int32)
+    if kind == "zeros":
+        buf.zero_()
+    elif kind == "ones":
+        buf.fill_(255)
+    elif kind == "noise":
+        buf.random_(0, 256, generator=gen)
+    elif kind == "small numbers":  # many are tiles
+        words.random_(0, 20000, generator=gen)
+    elif kind == "shifted":  # every entry is one, but of another place
+        buf.copy_(kept.roll(8))
+    elif kind == "half":  # what was there, up to the middle; the end of the order is another one's
+        buf[n // 2:].random_(0, 256, generator=gen)
+    elif kind == "swapped":  # two entries of the order in each other's place
+        words[-200:] = words[-200:].flip(0)
+    else:  # single words
+        at = torch.randint(words.numel(), (50,), generator=gen, device=buf.device)
+        words[at] = words[at] + 1
+
+
+@pytest.mark.parametrize("kind", ["zeros", "ones", "noise", "small numbers", "shifted", "half", "swapped", "words"])
+@pytest.mark.parametrize("cols", [0, 5000])  # with near tiles, and the rows of the tiles alone
+def test_sddmm_order_written_over_by_others(pkg, handle, device, cols, kind):
+    """Straight into the memory, and into that of a product that a graph repeats: with beta, so that a tile done twice shows."""
+    case = Case(pkg, handle, device, "f16", 128, cols=cols)
+    plain = case.product(torch.empty(256, dtype=torch.uint8, device=device))
+    buf = case.buffer()
+    case.preprocess(buf)
+    assert torch.equal(case.product(buf), plain)
+    kept, gen = buf.clone(), torch.Generator(device=device).manual_seed(3)
+    for _ in range(2):
+        foreign(kind, buf, kept, gen)
+        assert torch.equal(case.product(buf), plain)
+        kept = buf.clone()
+    case.preprocess(buf)
+    kept = buf.clone()
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream(device)
+    with torch.cuda.graph(graph, stream=stream):
+        assert pkg.lib().aclsparseSetStream(handle.raw, c_void_p(stream.cuda_stream)) == 0
+        try:
+            pkg.check(pkg.lib().aclsparseSDDMM(*case.args, at(buf)), "product")
+        finally:
+            assert pkg.lib().aclsparseSetStream(handle.raw, c_void_p(handle.stream.cuda_stream)) == 0
+    foreign(kind, buf, kept, gen)
+    case.C.values.copy_(case.c0)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(case.C.values, plain)
