@@ -187,10 +187,15 @@ struct RowsOf {  // the operands' rows and how far apart they are
 struct TileOrder {
     const int2 *tiles = nullptr;       // {tile, row of its first entry}; near tiles by column, then the others; nullptr: no order and no rows
     const int *place = nullptr;        // [tile] where it stands in `tiles`
-    int *bad = nullptr;                // not 0: not an order.  Preprocess writes 0, a product 1, nobody 0 again
+    unsigned ticket = 0;               // of the product that looks it over
     long long near = 0;                // 0: all tiles stand where they lie, and there is nothing to look at but rows
     unsigned long long share = 0;      // of the near tiles among all, times 2^32, rounded up
 };
+// Products do not write the caller's buffer.  Where the check finds that there is no order, it leaves the product's ticket here, which the product compares; a ticket's
+// place serves another product 65,536 tickets later.  One that a graph repeats has the same ticket each time: once it was left here
+// it may take the tiles as they lie from then on.
+constexpr unsigned kTickets = 1 << 16;
+__device__ unsigned gNoOrder[kTickets];
 constexpr int kOrderBuckets = 1024;
 // A smaller Y stays in L2 as a whole.
 constexpr long long kOrderMinY = 96ll << 20;
@@ -330,13 +335,13 @@ __global__ void __launch_bounds__(256) SddmmOrderTilesKernel(const int32_t *__re
 }
 
 // A thread per tile: whether it stands somewhere, and there alone.
-__global__ void __launch_bounds__(256) SddmmOrderCheckKernel(const int2 *__restrict__ order, const int *__restrict__ place, int tiles, int *bad)
+__global__ void __launch_bounds__(256) SddmmOrderCheckKernel(const int2 *__restrict__ order, const int *__restrict__ place, int tiles, unsigned ticket)
 {
     b200sp::WaitForPrevious();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= tiles) return;
     const int at = __ldg(place + t);
-    if ((unsigned)at >= (unsigned)tiles || __ldg(&order[at].x) != t) *bad = 1;
+    if ((unsigned)at >= (unsigned)tiles || __ldg(&order[at].x) != t) gNoOrder[ticket % kTickets] = ticket;
 }
 
 // The dot products of a tile of entries: sDot[t] = X row sRow[t] . Y row sCol[t].  tile: a multiple of 32.
@@ -499,7 +504,7 @@ __global__ void __launch_bounds__(32 * SddmmShape<kBytes, kSlabs, kBatch, kOrder
         const unsigned before = (unsigned)((p0 * order.share) >> 32);
         const bool near = (unsigned)(((p0 + 1) * order.share) >> 32) != before;
         const int2 at = __ldg(order.tiles + (near ? before : order.near + (p0 - before)));
-        if (order.near != 0 && __ldg(order.bad) == 0) p0 = at.x;
+        if (order.near != 0 && gNoOrder[order.ticket % kTickets] != order.ticket) p0 = at.x;
         r0 = at.y;
     }
     p0 *= tile;
@@ -678,7 +683,7 @@ int LaunchRows(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const
                     const int tiles = (nnz - 1) / kSddmmTile + 1;
                     b200sp_note_launches(1);
                     const cudaError_t e = b200sp::LaunchChained(SddmmOrderCheckKernel, (unsigned)((tiles + 255) / 256), 256, 0, stream, order.tiles,
-                                                                order.place, tiles, order.bad);
+                                                                order.place, tiles, order.ticket);
                     if (e != cudaSuccess) return (int)e;
                 }
                 return launchAs.template operator()<kLanes, kSlabs, false, kShort, true>();
@@ -756,7 +761,7 @@ cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, aclsparseSpMatDescr *C, voi
     const long long rowBytes = Y->ld * (Y->valueType == ACL_FLOAT16 ? 2ll : 4ll);
     const int span = C->cols * rowBytes >= kOrderMinY ? (int)std::min<long long>(kNearSpan / rowBytes, C->cols / 3) : -1;  // -1: none is near
     C->sddmm.generation = b200sp::NoteBufferWrite(buffer);
-    cudaError_t e = cudaMemsetAsync(p, 0, L.offCounts + sizeof(int) * (kOrderBuckets + 1), stream);  // and TileOrder::bad
+    cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(int) * (kOrderBuckets + 1), stream);
     if (e != cudaSuccess) return e;
     const long long want = (L.tiles + 7) / 8, cap = (long long)b200sp_sm_count() * 8;
     SddmmTileBucketsKernel<<<(unsigned)(want < cap ? want : cap), 256, 0, stream>>>(
@@ -787,14 +792,17 @@ cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, aclsparseSpMatDescr *C, voi
 }
 
 // The order that Preprocess left in the buffer, if it is still there and worth following.
-TileOrder OrderOf(const aclsparseSpMatDescr *C, void *buffer)
+TileOrder OrderOf(const aclsparseSpMatDescr *C, const void *buffer)
 {
     const auto &plan = C->sddmm;
     const OrderLayout L = OrderLayoutFor(C->nnz);
     if (plan.buffer == nullptr || plan.buffer != buffer || plan.nnz != C->nnz || plan.generation != b200sp::BufferGeneration(buffer))
         return {};
-    char *p = static_cast<char *>(buffer);
-    return {reinterpret_cast<const int2 *>(p + L.offTiles), reinterpret_cast<const int *>(p + L.offPlace), reinterpret_cast<int *>(p), plan.near,
+    static std::atomic<unsigned> products{0};
+    unsigned ticket = products.fetch_add(1, std::memory_order_relaxed) + 1;
+    if (ticket == 0) ticket = products.fetch_add(1, std::memory_order_relaxed) + 1;  // what every place holds at first
+    const char *p = static_cast<const char *>(buffer);
+    return {reinterpret_cast<const int2 *>(p + L.offTiles), reinterpret_cast<const int *>(p + L.offPlace), ticket, plan.near,
             (((unsigned long long)plan.near << 32) + (unsigned long long)L.tiles - 1) / (unsigned long long)L.tiles};
 }
 
