@@ -205,9 +205,19 @@ constexpr long long kOrderMinY = 96ll << 20;
 // them changed: no policy here.)
 constexpr long long kNearSpan = 160ll << 20;
 // Entries from which Preprocess notes the rows of the tiles (of 64 entries; fewer entries have shorter ones), in the order they lie in if none is
-// near: a warp's search in the row offsets are four loads one after the other.  200,000 power-law rows of 12, fp16, k = 16 36.5 and 32.7 us, k = 128
-// 87 and 78, 50,000 rows of 8, k = 32, 11.5 and 10.2; k = 384 and more as without.
+// near: a warp's search in the row offsets are four loads one after the other.  320,000 to 1.6 M entries of even and power-law rows, without and with
+// them, us: fp16, k = 16 7.8 and 7.2, 26.0 and 24.1, k = 64 17.0 and 16.2, k = 128 55.3 and 51.1, k = 256 22.4 and 21.0, 91 and 86, fp32, k = 64 15.2 and
+// 12.9, k = 128 83 and 76.
 constexpr long long kOrderLeast = 1 << 18;
+// Wider rows are as they were: their tiles are long, one warp a CTA and no tiles of 32 cost more than the search (fp16, k = 512 34.1 and 34.3, k =
+// 640 56.0 and 60.4, 248 and 258; fp32, k = 256 29.7 and 31.8, k = 1024 104 and 113, at best 122 and 114).
+constexpr int kRowsPieces = 32;
+// Entries from which tiles may be near, for rows of up to eight pieces and wider ones: the check costs 2 us or more.  Y of 100 MB, a tenth / 60 % of the entries in rows of
+// thousands, us without an order and with one: fp16, k = 16, 280,000 entries 7.3 / 7.0 and 8.7 / 8.8, 600,000 12.7 / 12.1 and 12.9 / 12.1, 1.5 M 30.0 / 28.4 and
+// 28.3 / 26.3; k = 64 10.1 / 9.7 and 10.6 / 10.3, 17.8 / 16.8 and 17.8 / 17.4, 41 / 40 and 40 / 37; k = 512 39.6 / 37.6 and 43.3 / 39.8,
+// 76 / 73 and 74 / 68, 185 / 165 and 174 / 160; fp32, k = 256 37.6 / 35.4 and 40.9 / 37.5, 75 / 69 and 70 / 62, 175 / 167 and 167 / 154.
+constexpr long long kNearLeast = 1 << 20, kNearLeastWide = 1 << 19;
+constexpr int kNearNarrow = 8;
 // Fewer near tiles than one in so many are not worth the turns.
 constexpr long long kNearShare = 16;
 struct OrderLayout {
@@ -678,7 +688,7 @@ int LaunchRows(const aclsparseSpMatDescr *C, const aclsparseDnMatDescr *X, const
     auto launch = [&]<int kLanes, int kSlabs>() {
         constexpr int kShort = kShortBatch<kBytes, kLanes, kSlabs>;
         if constexpr (kBytes == 16)
-            if (order.tiles != nullptr && tile == kSddmmTile && !near) {
+            if (order.tiles != nullptr && tile == kSddmmTile && !near && (order.near > 0 || kLanes * kSlabs <= kRowsPieces)) {
                 if (order.near > 0) {
                     const int tiles = (nnz - 1) / kSddmmTile + 1;
                     b200sp_note_launches(1);
@@ -747,7 +757,8 @@ bool MayOrder(const aclsparseDnMatDescr *Y, const aclsparseSpMatDescr *C, aclspa
     return rows && Y->ld * bytes % 16 == 0 && C->nnz >= kOrderLeast;
 }
 
-cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, aclsparseSpMatDescr *C, void *buffer, cudaStream_t stream)
+// pieces: the 16-byte pieces of a row of Y.
+cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, long long pieces, aclsparseSpMatDescr *C, void *buffer, cudaStream_t stream)
 {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
@@ -759,7 +770,9 @@ cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, aclsparseSpMatDescr *C, voi
     int *counts = reinterpret_cast<int *>(p + L.offCounts), *starts = counts + kOrderBuckets + 1;
     auto *bucket = reinterpret_cast<int16_t *>(p + L.offBucket);
     const long long rowBytes = Y->ld * (Y->valueType == ACL_FLOAT16 ? 2ll : 4ll);
-    const int span = C->cols * rowBytes >= kOrderMinY ? (int)std::min<long long>(kNearSpan / rowBytes, C->cols / 3) : -1;  // -1: none is near
+    const bool mayBeNear = C->cols * rowBytes >= kOrderMinY && C->nnz >= (pieces <= kNearNarrow ? kNearLeast : kNearLeastWide);
+    if (!mayBeNear && pieces > kRowsPieces) return cudaSuccess;
+    const int span = mayBeNear ? (int)std::min<long long>(kNearSpan / rowBytes, C->cols / 3) : -1;  // -1: none is near
     C->sddmm.generation = b200sp::NoteBufferWrite(buffer);
     cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(int) * (kOrderBuckets + 1), stream);
     if (e != cudaSuccess) return e;
@@ -778,6 +791,7 @@ cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, aclsparseSpMatDescr *C, voi
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return e;
     if (near * kNearShare < L.tiles) {
+        if (pieces > kRowsPieces) return cudaSuccess;
         near = 0;
         SddmmTileRowsKernel<<<(unsigned)((L.tiles + 255) / 256), 256, 0, stream>>>(static_cast<const int32_t *>(C->offsets), (int)C->rows,
                                                                                    L.tiles, reinterpret_cast<int2 *>(p + L.offTiles));
@@ -834,7 +848,8 @@ aclsparseStatus_t aclsparseSDDMMPreprocess(aclsparseHandle_t handle, aclsparseOp
     if (st != ACL_SPARSE_STATUS_SUCCESS) return st;
     matC->sddmm.buffer = nullptr;
     if (!MayOrder(matY, matC, opY) || matC->sddmm.sized < (int64_t)OrderLayoutFor(matC->nnz).total) return ACL_SPARSE_STATUS_SUCCESS;
-    if (OrderTiles(matY, matC, buffer, handle->stream) != cudaSuccess) {
+    const int64_t k = opX == ACL_SPARSE_OP_TRANSPOSE ? matX->rows : matX->cols;
+    if (OrderTiles(matY, (k * (matY->valueType == ACL_FLOAT16 ? 2 : 4) + 15) / 16, matC, buffer, handle->stream) != cudaSuccess) {
         B200SP_LOGE("aclsparseSDDMMPreprocess: analysis failed");
         return ACL_SPARSE_STATUS_EXECUTION_FAILED;
     }

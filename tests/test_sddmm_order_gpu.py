@@ -129,3 +129,17 @@ def test_pattern_and_buffer_that_change(pkg, handle, device):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(case.C.values, want)
+
+
+# rows of 32 pieces and of 33; Y above 96 MB with too few entries for near tiles, by the width of the rows
+@pytest.mark.parametrize("dtype,k,cols,nnz,written", [("f16", 256, 5000, 1 << 18, True), ("f16", 264, 5000, 1 << 18, False), ("f32", 1024, 5000, 300_000, False),
+                                                      ("f32", 136, 0, (1 << 19) - 1, False), ("f32", 136, 0, 1 << 19, True), ("f16", 64, 0, 1 << 19, True)])
+def test_where_an_order_pays(pkg, handle, device, dtype, k, cols, nnz, written):
+    case = Case(pkg, handle, device, dtype, k, nnz=nnz, cols=cols)
+    plain = case.product(torch.empty(256, dtype=torch.uint8, device=device))
+    buf = case.buffer()
+    untouched = buf.clone()
+    case.preprocess(buf)
+    torch.cuda.synchronize()
+    assert (not torch.equal(buf, untouched)) == written
+    assert torch.equal(case.product(buf), plain)
