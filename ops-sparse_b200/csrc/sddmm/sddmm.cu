@@ -772,29 +772,35 @@ cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, long long pieces, aclsparse
     const long long rowBytes = Y->ld * (Y->valueType == ACL_FLOAT16 ? 2ll : 4ll);
     const bool mayBeNear = C->cols * rowBytes >= kOrderMinY && C->nnz >= (pieces <= kNearNarrow ? kNearLeast : kNearLeastWide);
     if (!mayBeNear && pieces > kRowsPieces) return cudaSuccess;
-    const int span = mayBeNear ? (int)std::min<long long>(kNearSpan / rowBytes, C->cols / 3) : -1;  // -1: none is near
+    auto *order = reinterpret_cast<int2 *>(p + L.offTiles);
+    const auto *rowPtr = static_cast<const int32_t *>(C->offsets);
     C->sddmm.generation = b200sp::NoteBufferWrite(buffer);
-    cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(int) * (kOrderBuckets + 1), stream);
-    if (e != cudaSuccess) return e;
-    const long long want = (L.tiles + 7) / 8, cap = (long long)b200sp_sm_count() * 8;
-    SddmmTileBucketsKernel<<<(unsigned)(want < cap ? want : cap), 256, 0, stream>>>(
-        static_cast<const int32_t *>(C->indices), (int)C->nnz, (int)C->cols, span, L.tiles, bucket, counts);
-    SddmmBucketStartsKernel<<<1, kOrderBuckets, 0, stream>>>(counts, starts);
     int near = 0;
-    e = cudaMemcpyAsync(&near, starts + kOrderBuckets, sizeof(near), cudaMemcpyDeviceToHost, stream);
-    if (e != cudaSuccess) return e;
-    SddmmOrderTilesKernel<<<(unsigned)((L.tiles + 1023) / 1024), 256, 0, stream>>>(
-        static_cast<const int32_t *>(C->offsets), (int)C->rows, bucket, L.tiles, starts, reinterpret_cast<int2 *>(p + L.offTiles),
-        reinterpret_cast<int *>(p + L.offPlace));
-    b200sp_note_launches(3);
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess) return e;
-    if (near * kNearShare < L.tiles) {
-        if (pieces > kRowsPieces) return cudaSuccess;
-        near = 0;
-        SddmmTileRowsKernel<<<(unsigned)((L.tiles + 255) / 256), 256, 0, stream>>>(static_cast<const int32_t *>(C->offsets), (int)C->rows,
-                                                                                   L.tiles, reinterpret_cast<int2 *>(p + L.offTiles));
+    cudaError_t e = cudaSuccess;
+    if (mayBeNear) {
+        const int span = (int)std::min<long long>(kNearSpan / rowBytes, C->cols / 3);
+        e = cudaMemsetAsync(counts, 0, sizeof(int) * (kOrderBuckets + 1), stream);
+        if (e != cudaSuccess) return e;
+        const long long want = (L.tiles + 7) / 8, cap = (long long)b200sp_sm_count() * 8;
+        SddmmTileBucketsKernel<<<(unsigned)(want < cap ? want : cap), 256, 0, stream>>>(
+            static_cast<const int32_t *>(C->indices), (int)C->nnz, (int)C->cols, span, L.tiles, bucket, counts);
+        SddmmBucketStartsKernel<<<1, kOrderBuckets, 0, stream>>>(counts, starts);
+        e = cudaMemcpyAsync(&near, starts + kOrderBuckets, sizeof(near), cudaMemcpyDeviceToHost, stream);
+        if (e != cudaSuccess) return e;
+        SddmmOrderTilesKernel<<<(unsigned)((L.tiles + 1023) / 1024), 256, 0, stream>>>(rowPtr, (int)C->rows, bucket, L.tiles, starts, order,
+                                                                                       reinterpret_cast<int *>(p + L.offPlace));
+        b200sp_note_launches(3);
+        e = cudaGetLastError();
+        // Not only for the number of near tiles: a product on another stream must not find the order changed after it has looked it over.
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) return e;
+        if (near * kNearShare < L.tiles) {
+            if (pieces > kRowsPieces) return cudaSuccess;
+            near = 0;
+        }
+    }
+    if (near == 0) {  // nothing is waited for: a product compares the rows with the row offsets
+        SddmmTileRowsKernel<<<(unsigned)((L.tiles + 255) / 256), 256, 0, stream>>>(rowPtr, (int)C->rows, L.tiles, order);
         b200sp_note_launches(1);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;

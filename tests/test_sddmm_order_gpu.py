@@ -143,3 +143,15 @@ def test_where_an_order_pays(pkg, handle, device, dtype, k, cols, nnz, written):
     torch.cuda.synchronize()
     assert (not torch.equal(buf, untouched)) == written
     assert torch.equal(case.product(buf), plain)
+
+
+@pytest.mark.parametrize("cols,launches", [(5000, 1), (0, 3)])  # the rows of the tiles; an order of them
+def test_launches_of_preprocess(pkg, handle, device, cols, launches):
+    """Where no tile can be near, one kernel, which does not wait and does not read the columns: those may not be there yet."""
+    case = Case(pkg, handle, device, "f16", 128, cols=cols)
+    plain = case.product(torch.empty(256, dtype=torch.uint8, device=device))
+    buf = case.buffer()
+    before = pkg.lib().b200sp_kernel_launches()
+    case.preprocess(buf)
+    assert pkg.lib().b200sp_kernel_launches() - before == launches
+    assert torch.equal(case.product(buf), plain)
