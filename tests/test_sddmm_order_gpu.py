@@ -155,3 +155,16 @@ def test_launches_of_preprocess(pkg, handle, device, cols, launches):
     case.preprocess(buf)
     assert pkg.lib().b200sp_kernel_launches() - before == launches
     assert torch.equal(case.product(buf), plain)
+
+
+@pytest.mark.parametrize("cols", [0, 5000])
+@pytest.mark.parametrize("shift", [1, 2, 4, 8, 16])
+def test_buffer_at_any_address(pkg, handle, device, shift, cols):
+    case = Case(pkg, handle, device, "f16", 128, cols=cols)
+    plain = case.product(torch.empty(256, dtype=torch.uint8, device=device))
+    whole = torch.full((case.buffer().numel() + 16,), 255, dtype=torch.uint8, device=device)
+    buf = whole[shift:shift + whole.numel() - 16]
+    case.preprocess(buf)
+    torch.cuda.synchronize()
+    assert bool((buf == 255).all()) == (shift % 8 != 0)  # no order where its entries would not be aligned
+    assert torch.equal(case.product(buf), plain)
