@@ -2,6 +2,7 @@
 // Behaviour follows sparse/common/aclsparse_auxiliary.cpp:64-198, 253-279 of the reference;
 // device memory comes from the CUDA runtime instead of aclrtMalloc.
 #include <atomic>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <unordered_map>
@@ -22,7 +23,11 @@ int LogLevel()
 
 namespace {
 std::mutex gGenerationMutex;
-std::unordered_map<const void *, uint64_t> gGenerations;
+struct BufferNote {
+    uint64_t generation = 0;
+    std::weak_ptr<const void> plan;
+};
+std::unordered_map<const void *, BufferNote> gBuffers;
 uint64_t gNextGeneration = 0;
 }  // namespace
 
@@ -30,15 +35,38 @@ uint64_t NoteBufferWrite(const void *buffer)
 {
     if (buffer == nullptr) return 0;
     std::lock_guard<std::mutex> lock(gGenerationMutex);
-    return gGenerations[buffer] = ++gNextGeneration;
+    BufferNote &note = gBuffers[buffer];
+    note.plan.reset();
+    return note.generation = ++gNextGeneration;
 }
 
 uint64_t BufferGeneration(const void *buffer)
 {
     if (buffer == nullptr) return 0;
     std::lock_guard<std::mutex> lock(gGenerationMutex);
-    const auto it = gGenerations.find(buffer);
-    return it == gGenerations.end() ? 0 : it->second;
+    const auto it = gBuffers.find(buffer);
+    return it == gBuffers.end() ? 0 : it->second.generation;
+}
+
+std::shared_ptr<const void> HoldPlan(const void *buffer)
+{
+    if (buffer == nullptr) return nullptr;
+    try {
+        std::shared_ptr<const void> held = std::make_shared<char>();
+        std::lock_guard<std::mutex> lock(gGenerationMutex);
+        gBuffers[buffer].plan = held;
+        return held;
+    } catch (const std::bad_alloc &) {
+        return nullptr;
+    }
+}
+
+bool HoldsPlan(const void *buffer)
+{
+    if (buffer == nullptr) return false;
+    std::lock_guard<std::mutex> lock(gGenerationMutex);
+    const auto it = gBuffers.find(buffer);
+    return it != gBuffers.end() && !it->second.plan.expired();
 }
 
 }  // namespace b200sp

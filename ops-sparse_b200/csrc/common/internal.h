@@ -6,6 +6,7 @@
 // with the analysis-plan bookkeeping the B200 kernels need.
 #pragma once
 
+#include <memory>
 #include <mutex>
 #include <cstddef>
 #include <cstdint>
@@ -69,6 +70,7 @@ struct ActivePlan {
     unsigned long long copyStream = 0;
     int32_t spmvInfo[B200SP_SPMV_PLAN_INFO_INTS] = {};  // SpMV only: plan_info written by b200sp_spmv_analyze
     uint64_t generation = 0;  // BufferGeneration(buffer) when the analysis was written
+    std::shared_ptr<const void> held;  // see HoldPlan
 };
 
 // SDDMM: an order of the tiles of C's entries that Preprocess left in a buffer.  Any order is right, whatever the pattern: only the
@@ -87,6 +89,11 @@ struct TileOrderPlan {
 // into buf for another operation or another matrix, then a compute call on A with buf.
 uint64_t NoteBufferWrite(const void *buffer);   // returns the new generation (never 0)
 uint64_t BufferGeneration(const void *buffer);  // 0 = no library call has written this buffer
+
+// A buffer that holds what a descriptor needs: from HoldPlan on, as long as a copy of what it returned exists and nothing else is noted to have
+// written the buffer.  A call that can do without its buffer (SDDMM's preprocessing) leaves such a one alone.
+std::shared_ptr<const void> HoldPlan(const void *buffer);  // nullptr without memory for the note
+bool HoldsPlan(const void *buffer);
 
 }  // namespace b200sp
 

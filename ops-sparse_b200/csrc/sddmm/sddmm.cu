@@ -855,6 +855,7 @@ aclsparseStatus_t aclsparseSDDMMPreprocess(aclsparseHandle_t handle, aclsparseOp
     matC->sddmm.buffer = nullptr;
     if (!MayOrder(matY, matC, opY) || matC->sddmm.sized < (int64_t)OrderLayoutFor(matC->nnz).total) return ACL_SPARSE_STATUS_SUCCESS;
     if (reinterpret_cast<uintptr_t>(buffer) % alignof(int2) != 0) return ACL_SPARSE_STATUS_SUCCESS;  // any address is accepted
+    if (b200sp::HoldsPlan(buffer)) return ACL_SPARSE_STATUS_SUCCESS;
     const int64_t k = opX == ACL_SPARSE_OP_TRANSPOSE ? matX->rows : matX->cols;
     if (OrderTiles(matY, (k * (matY->valueType == ACL_FLOAT16 ? 2 : 4) + 15) / 16, matC, buffer, handle->stream) != cudaSuccess) {
         B200SP_LOGE("aclsparseSDDMMPreprocess: analysis failed");

@@ -217,6 +217,7 @@ aclsparseStatus_t aclsparseSpMMPreprocess(aclsparseHandle_t handle, aclsparseOpe
     }
     p.spmmFound = found.more;
     p.generation = b200sp::BufferGeneration(buffer);
+    p.held = b200sp::HoldPlan(buffer);
     matA->active = p;
     return ACL_SPARSE_STATUS_SUCCESS;
 }

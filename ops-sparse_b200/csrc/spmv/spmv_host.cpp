@@ -218,6 +218,7 @@ aclsparseStatus_t aclsparseSpMVPreprocess(aclsparseHandle_t handle, aclsparseOpe
         B200SP_LOGE("aclsparseSpMVPreprocess: analysis failed (cuda error %d)", rc);
         return ACL_SPARSE_STATUS_EXECUTION_FAILED;
     }
+    p.held = b200sp::HoldPlan(externalBuffer);
     p.buffer = externalBuffer;
     p.kind = PlanKind::kSpmv;
     p.rowPtr = matA->offsets;

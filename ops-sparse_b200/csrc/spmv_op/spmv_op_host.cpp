@@ -2,6 +2,7 @@
 // Argument checks, their order and their status codes follow the reference host layer
 // (sparse/spmv_op/arch35/spmv_op_host.cpp:65-297, 496-745); the device work is in spmv_op_kernels.cu.
 #include <climits>
+#include <memory>
 #include <new>
 
 #include "b200sp_kernels.h"
@@ -17,6 +18,7 @@ struct aclsparseSpMVOpDescr {
     aclsparseSpMVOpAlg_t alg = ACL_SPARSE_SPMVOP_ALG1;
     void *userBuffer = nullptr;                         // ALG2: the caller's workspace (row order)
     uint64_t generation = 0;                            // ... BufferGeneration(userBuffer) when it was written
+    std::shared_ptr<const void> held;                   // ... see HoldPlan
     int32_t classStart[B200SP_SPMVOP_CLASSES + 1] = {};  // ALG2: where each length class starts in it
 };
 
@@ -131,6 +133,7 @@ aclsparseStatus_t aclsparseSpMVOp_createDescr(aclsparseHandle_t handle, aclspars
             return ACL_SPARSE_STATUS_EXECUTION_FAILED;
         }
         d->userBuffer = buffer;
+        d->held = b200sp::HoldPlan(buffer);
     }
     *descr = d;
     return ACL_SPARSE_STATUS_SUCCESS;

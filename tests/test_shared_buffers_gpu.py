@@ -173,3 +173,46 @@ def test_sddmm_order_written_over_by_others(pkg, handle, device, cols, kind):
         torch.cuda.synchronize()
         assert torch.equal(case.C.values, plain)
         buf.copy_(kept)
+
+
+@pytest.mark.parametrize("kind", ["spmv", "spmm", "spmvop"])
+def test_sddmm_leaves_the_plans_of_others_alone(pkg, handle, device, kind):
+    from ops_sparse_b200 import api
+    case = Case(pkg, handle, device, "f16", 128, nnz=300_000, cols=5000)
+    plain = case.product(torch.empty(256, dtype=torch.uint8, device=device))
+    A = api.CsrMatrix(case.row_ptr, case.col_ind, torch.rand(case.nnz, device=device), case.m, case.cols)
+    null, descr, size = c_void_p(), c_void_p(), c_size_t()
+    x, y = (api.DnVec(torch.rand(s, device=device)) for s in (case.cols, case.m))
+    B, out = (api.DnMat.row_major(torch.rand((s, 16), device=device)) for s in (case.cols, case.m))
+    need = {"spmv": lambda: api.spmv_preprocess(handle, A, x, y).numel(), "spmm": lambda: api.spmm_preprocess(handle, A, B, out).numel(),
+            "spmvop": lambda: 4 * case.m + 4096}[kind]()
+    buf = torch.full((max(case.buffer().numel(), need),), 255, dtype=torch.uint8, device=device)
+    L = pkg.lib()
+    if kind == "spmv":
+        pkg.check(L.aclsparseSpMVPreprocess(handle.raw, 0, null, A.raw, x.raw, null, y.raw, pkg.ACL_FLOAT, 0, at(buf)), "plan")
+    elif kind == "spmm":
+        pkg.check(L.aclsparseSpMMPreprocess(handle.raw, 0, 0, null, A.raw, B.raw, null, out.raw, pkg.ACL_FLOAT, 0, at(buf)), "plan")
+    else:
+        args = (0, A.raw, x.raw, y.raw, y.raw, pkg.ACL_FLOAT, 2)
+        pkg.check(L.aclsparseSpMVOp_bufferSize(handle.raw, *args, byref(size)), "size")
+        assert size.value <= need
+        pkg.check(L.aclsparseSpMVOp_createDescr(handle.raw, byref(descr), *args, at(buf)), "plan")
+    kept = buf.clone()
+    case.preprocess(buf)
+    assert torch.equal(buf, kept)
+    assert torch.equal(case.product(buf), plain)
+    if kind == "spmm":  # a product with a plan waits for nothing, so a graph may hold it
+        graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream(device)
+        with torch.cuda.graph(graph, stream=stream):
+            assert L.aclsparseSetStream(handle.raw, c_void_p(stream.cuda_stream)) == 0
+            try:
+                api.spmm(handle, A, B, out, 1.0, 0.0, buffer=buf)
+            finally:
+                assert L.aclsparseSetStream(handle.raw, c_void_p(handle.stream.cuda_stream)) == 0
+    A.close()  # nobody needs the plan any more
+    if kind == "spmvop":
+        L.aclsparseSpMVOp_destroyDescr(descr)
+    case.preprocess(buf)
+    torch.cuda.synchronize()
+    assert not torch.equal(buf, kept)
+    assert torch.equal(case.product(buf), plain)
