@@ -757,6 +757,14 @@ bool MayOrder(const aclsparseDnMatDescr *Y, const aclsparseSpMatDescr *C, aclspa
     return rows && Y->ld * bytes % 16 == 0 && C->nnz >= kOrderLeast;
 }
 
+// While another stream is being captured, waiting for one that is not, or loading a kernel, would end that capture with an error unless this
+// thread says that it knows what it does.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // pieces: the 16-byte pieces of a row of Y.
 cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, long long pieces, aclsparseSpMatDescr *C, void *buffer, cudaStream_t stream)
 {
@@ -765,6 +773,7 @@ cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, long long pieces, aclsparse
         (void)cudaGetLastError();
         return cudaSuccess;  // a product without an order is as good, only slower
     }
+    const RelaxedCapture relaxed;
     const OrderLayout L = OrderLayoutFor(C->nnz);
     char *p = static_cast<char *>(buffer);
     int *counts = reinterpret_cast<int *>(p + L.offCounts), *starts = counts + kOrderBuckets + 1;

@@ -168,3 +168,26 @@ def test_buffer_at_any_address(pkg, handle, device, shift, cols):
     torch.cuda.synchronize()
     assert bool((buf == 255).all()) == (shift % 8 != 0)  # no order where its entries would not be aligned
     assert torch.equal(case.product(buf), plain)
+
+
+@pytest.mark.parametrize("cols", [0, 5000])
+@pytest.mark.parametrize("mode", ["global", "thread_local", "relaxed"])
+def test_preprocess_while_another_stream_is_captured(pkg, handle, device, mode, cols):
+    """Nothing of it goes into the graph and the capture goes on, as when Preprocess launched nothing."""
+    case = Case(pkg, handle, device, "f16", 128, cols=cols)
+    plain = case.product(torch.empty(256, dtype=torch.uint8, device=device))
+    buf, data = case.buffer(), torch.ones(1000, device=device)
+    graph, stream, mine = torch.cuda.CUDAGraph(), torch.cuda.Stream(device), torch.cuda.Stream(device)
+    torch.cuda.synchronize()
+    assert pkg.lib().aclsparseSetStream(handle.raw, c_void_p(mine.cuda_stream)) == 0
+    try:
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode=mode):
+            data.add_(1)
+            case.preprocess(buf)
+            data.add_(1)
+    finally:
+        assert pkg.lib().aclsparseSetStream(handle.raw, c_void_p(handle.stream.cuda_stream)) == 0
+    graph.replay()
+    torch.cuda.synchronize()
+    assert bool((data == 3).all())
+    assert torch.equal(case.product(buf), plain)
