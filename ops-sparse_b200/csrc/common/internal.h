@@ -130,6 +130,7 @@ struct aclsparseSpMatDescr {
     mutable int64_t spmmSizedRepack = 0;
     mutable int64_t spmmSizedN = -1;
     b200sp::TileOrderPlan sddmm;  // of the SDDMM products that write this matrix
+    mutable std::mutex sddmmMutex;  // held while it is read or written
     mutable std::mutex copyMutex;  // held while a product that copies into the analysed buffer is enqueued
 };
 

@@ -766,7 +766,8 @@ struct RelaxedCapture {
 };
 
 // pieces: the 16-byte pieces of a row of Y.
-cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, long long pieces, aclsparseSpMatDescr *C, void *buffer, cudaStream_t stream)
+cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, long long pieces, const aclsparseSpMatDescr *C, void *buffer, cudaStream_t stream,
+                       b200sp::TileOrderPlan *plan)
 {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
@@ -783,7 +784,7 @@ cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, long long pieces, aclsparse
     if (!mayBeNear && pieces > kRowsPieces) return cudaSuccess;
     auto *order = reinterpret_cast<int2 *>(p + L.offTiles);
     const auto *rowPtr = static_cast<const int32_t *>(C->offsets);
-    C->sddmm.generation = b200sp::NoteBufferWrite(buffer);
+    plan->generation = b200sp::NoteBufferWrite(buffer);
     int near = 0;
     cudaError_t e = cudaSuccess;
     if (mayBeNear) {
@@ -814,16 +815,20 @@ cudaError_t OrderTiles(const aclsparseDnMatDescr *Y, long long pieces, aclsparse
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    C->sddmm.near = near;
-    C->sddmm.nnz = C->nnz;
-    C->sddmm.buffer = buffer;
+    plan->near = near;
+    plan->nnz = C->nnz;
+    plan->buffer = buffer;
     return cudaSuccess;
 }
 
 // The order that Preprocess left in the buffer, if it is still there and worth following.
 TileOrder OrderOf(const aclsparseSpMatDescr *C, const void *buffer)
 {
-    const auto &plan = C->sddmm;
+    b200sp::TileOrderPlan plan;
+    {
+        std::lock_guard<std::mutex> lock(C->sddmmMutex);
+        plan = C->sddmm;
+    }
     const OrderLayout L = OrderLayoutFor(C->nnz);
     if (plan.buffer == nullptr || plan.buffer != buffer || plan.nnz != C->nnz || plan.generation != b200sp::BufferGeneration(buffer))
         return {};
@@ -850,6 +855,7 @@ aclsparseStatus_t aclsparseSDDMMBufferSize(aclsparseHandle_t handle, aclsparseOp
     const aclsparseStatus_t st = ValidateInputs(matX, matY, matC, opX, opY, computeType, alg);
     if (st != ACL_SPARSE_STATUS_SUCCESS) return st;
     *size = MayOrder(matY, matC, opY) ? OrderLayoutFor(matC->nnz).total : 256;
+    std::lock_guard<std::mutex> lock(matC->sddmmMutex);
     matC->sddmm.sized = (int64_t)*size;
     return ACL_SPARSE_STATUS_SUCCESS;
 }
@@ -861,14 +867,24 @@ aclsparseStatus_t aclsparseSDDMMPreprocess(aclsparseHandle_t handle, aclsparseOp
 {
     const aclsparseStatus_t st = ValidateCall(handle, matX, matY, matC, alpha, beta, buffer, true, opX, opY, computeType, alg);
     if (st != ACL_SPARSE_STATUS_SUCCESS) return st;
-    matC->sddmm.buffer = nullptr;
-    if (!MayOrder(matY, matC, opY) || matC->sddmm.sized < (int64_t)OrderLayoutFor(matC->nnz).total) return ACL_SPARSE_STATUS_SUCCESS;
+    b200sp::TileOrderPlan plan;  // without an order
+    {
+        std::lock_guard<std::mutex> lock(matC->sddmmMutex);
+        plan.sized = matC->sddmm.sized;
+        matC->sddmm = plan;
+    }
+    if (!MayOrder(matY, matC, opY) || plan.sized < (int64_t)OrderLayoutFor(matC->nnz).total) return ACL_SPARSE_STATUS_SUCCESS;
     if (reinterpret_cast<uintptr_t>(buffer) % alignof(int2) != 0) return ACL_SPARSE_STATUS_SUCCESS;  // any address is accepted
     if (b200sp::HoldsPlan(buffer)) return ACL_SPARSE_STATUS_SUCCESS;
     const int64_t k = opX == ACL_SPARSE_OP_TRANSPOSE ? matX->rows : matX->cols;
-    if (OrderTiles(matY, (k * (matY->valueType == ACL_FLOAT16 ? 2 : 4) + 15) / 16, matC, buffer, handle->stream) != cudaSuccess) {
+    if (OrderTiles(matY, (k * (matY->valueType == ACL_FLOAT16 ? 2 : 4) + 15) / 16, matC, buffer, handle->stream, &plan) != cudaSuccess) {
         B200SP_LOGE("aclsparseSDDMMPreprocess: analysis failed");
         return ACL_SPARSE_STATUS_EXECUTION_FAILED;
+    }
+    if (plan.buffer != nullptr) {
+        std::lock_guard<std::mutex> lock(matC->sddmmMutex);
+        plan.sized = matC->sddmm.sized;
+        matC->sddmm = plan;
     }
     return ACL_SPARSE_STATUS_SUCCESS;
 }

@@ -191,3 +191,35 @@ def test_preprocess_while_another_stream_is_captured(pkg, handle, device, mode, 
     torch.cuda.synchronize()
     assert bool((data == 3).all())
     assert torch.equal(case.product(buf), plain)
+
+
+def test_threads(pkg, handle, device):
+    """One thread preprocesses the matrix again and again, into two buffers in turn; others run products of it on the same stream."""
+    import threading
+    case = Case(pkg, handle, device, "f16", 128, nnz=1 << 20)
+    plain = case.product(torch.empty(256, dtype=torch.uint8, device=device))
+    buf, other, failed, done = case.buffer(), case.buffer(), [], threading.Event()
+
+    def products():
+        torch.cuda.set_device(device)
+        while not done.is_set():
+            for b in (buf, other):
+                if pkg.lib().aclsparseSDDMM(*case.args, c_void_p(b.data_ptr())):
+                    failed.append(1)
+
+    case.keep[1].value = 0  # beta: every product writes the same
+    zero = case.product(torch.empty(256, dtype=torch.uint8, device=device))
+    threads = [threading.Thread(target=products) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for i in range(60):
+        case.preprocess((buf, other)[i % 2])
+        size = c_size_t()
+        pkg.check(pkg.lib().aclsparseSDDMMBufferSize(*case.args, byref(size)), "size")
+    done.set()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed
+    assert torch.equal(case.C.values, zero)
+    assert not torch.equal(zero, plain)
