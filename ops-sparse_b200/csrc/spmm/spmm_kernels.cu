@@ -1425,13 +1425,13 @@ __device__ __forceinline__ bool MbarWait(uint64_t *bar, uint32_t parity, long lo
     }
     return true;
 }
-// One row: global -> shared through the copy engine; both addresses 16-byte aligned, bytes a multiple of 16.  `once`: with an
+// One row: global -> shared through the copy engine; both addresses 16-byte aligned, bytes a multiple of 16.  kOnce: with an
 // L2 evict-first policy, so that rows that stream through L2 do not displace the block of B that units of long rows in the
 // same grid gather from (2 M x 2 M graph matrix, 512-byte rows: 2290 us with it, 2390 without; by itself the row stream
-// loses 5 % to it).
-__device__ __forceinline__ void BulkLoadRow(void *dst, const void *src, uint32_t bytes, uint64_t *bar, bool once)
+// loses 5 % to it).  A policy is made where it is used, by one instruction, and is never one of two: see the note at SDDMM's kNearSpan.
+template <bool kOnce> __device__ __forceinline__ void BulkLoadRow(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
 {
-    if (once) {
+    if constexpr (kOnce) {
         uint64_t pol;
         asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
         asm volatile(
@@ -1675,9 +1675,11 @@ template <int kRowBytes> struct StreamShape {
     static constexpr int kCtaBytes = kStreamWarps * kWarpBytes;
 };
 
-template <typename ValT, typename OutT, int kRowBytes>
-__global__ void __launch_bounds__(kStreamThreads) SpmmRowStreamKernel(const StreamArgs<ValT, OutT> a, const FastArgs<ValT, OutT> fa,
-                                                                      const BlockArgs ba)
+// kUnits: units of long rows are CTAs of this grid.
+template <typename ValT, typename OutT, int kRowBytes, bool kUnits>
+__global__ void __launch_bounds__(kStreamThreads) SpmmRowStreamKernel(const StreamArgs<ValT, OutT> a,
+                                                                      [[maybe_unused]] const FastArgs<ValT, OutT> fa,
+                                                                      [[maybe_unused]] const BlockArgs ba)
 {
     using Shape = StreamShape<kRowBytes>;
     constexpr int kBatch = Shape::kBatch;
@@ -1689,11 +1691,13 @@ __global__ void __launch_bounds__(kStreamThreads) SpmmRowStreamKernel(const Stre
 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    // Units of long rows, spread evenly over the grid
-    const unsigned before = (unsigned)((blockIdx.x * ba.share) >> 32);
-    if ((unsigned)(((blockIdx.x + 1ull) * ba.share) >> 32) != before) {
-        LongUnit<ValT, OutT>(fa, ba, (int)before, sRaw);
-        return;
+    unsigned before = 0;
+    if constexpr (kUnits) {  // spread evenly over the grid
+        before = (unsigned)((blockIdx.x * ba.share) >> 32);
+        if ((unsigned)(((blockIdx.x + 1ull) * ba.share) >> 32) != before) {
+            LongUnit<ValT, OutT>(fa, ba, (int)before, sRaw);
+            return;
+        }
     }
     unsigned char *base = sRaw + (size_t)warp * Shape::kWarpBytes;
     unsigned char *sData = base;                                                          // [buffers][kBatch][kRowBytes]
@@ -1789,8 +1793,7 @@ __global__ void __launch_bounds__(kStreamThreads) SpmmRowStreamKernel(const Stre
         if (i >= 0 && i < live) {
             sVal[buf * kBatch + i] = eVal;
             sMeta[buf * kBatch + i] = eMeta;
-            BulkLoadRow(sData + ((size_t)buf * kBatch + i) * kRowBytes, a.B + (long long)eCol * a.ldb, kRowBytes, sBar + buf,
-                        ba.share != 0);
+            BulkLoadRow<kUnits>(sData + ((size_t)buf * kBatch + i) * kRowBytes, a.B + (long long)eCol * a.ldb, kRowBytes, sBar + buf);
         }
     };
 
@@ -2016,7 +2019,7 @@ bool StreamPays(const b200spSpmmShape *sh, int32_t segments, int64_t rowBytes)
 // 256 bytes took 1.25 ms on 148 SMs), so rows shorter than 512 bytes move faster through plain
 // 128-bit loads and stay with SpmmFastKernel (256-byte rows, 64 per row of A: 1249 us against 265 us).
 
-template <typename ValT, typename OutT, int kRowBytes>
+template <typename ValT, typename OutT, int kRowBytes, bool kUnits>
 int LaunchRowStream(const StreamArgs<ValT, OutT> &sa, const FastArgs<ValT, OutT> &fa, BlockArgs ba, cudaStream_t stream)
 {
     constexpr int kSmem = StreamShape<kRowBytes>::kCtaBytes;
@@ -2024,7 +2027,7 @@ int LaunchRowStream(const StreamArgs<ValT, OutT> &sa, const FastArgs<ValT, OutT>
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
     if (!configured[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(SpmmRowStreamKernel<ValT, OutT, kRowBytes>,
+        const cudaError_t e = cudaFuncSetAttribute(SpmmRowStreamKernel<ValT, OutT, kRowBytes, kUnits>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
         if (e != cudaSuccess) return (int)e;
         configured[dev] = true;
@@ -2032,7 +2035,7 @@ int LaunchRowStream(const StreamArgs<ValT, OutT> &sa, const FastArgs<ValT, OutT>
     const unsigned grid = (unsigned)(((long long)sa.m + sa.warpRows - 1) / sa.warpRows);
     const unsigned long long all = (unsigned long long)grid + (unsigned)ba.nUnits;
     ba.share = (((unsigned long long)(unsigned)ba.nUnits << 32) + all - 1) / all;  // rounded up: the last CTA's count is nUnits
-    SpmmRowStreamKernel<ValT, OutT, kRowBytes><<<(unsigned)all, kStreamThreads, kSmem, stream>>>(sa, fa, ba);
+    SpmmRowStreamKernel<ValT, OutT, kRowBytes, kUnits><<<(unsigned)all, kStreamThreads, kSmem, stream>>>(sa, fa, ba);
     b200sp_note_launches(1);
     return (int)cudaGetLastError();
 }
@@ -2507,8 +2510,11 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             sa.negZeros = kNegZeros;
             sa.waitCycles = gHostStreamWaitCycles;
             sa.extraTx = gHostStreamExtraTx;
-            const int rc = rowBytes == 512 ? LaunchRowStream<ValT, OutT, 512>(sa, a, ba, stream)
-                                           : LaunchRowStream<ValT, OutT, 1024>(sa, a, ba, stream);
+            auto launchStream = [&]<bool kUnits>() {
+                return rowBytes == 512 ? LaunchRowStream<ValT, OutT, 512, kUnits>(sa, a, ba, stream)
+                                       : LaunchRowStream<ValT, OutT, 1024, kUnits>(sa, a, ba, stream);
+            };
+            const int rc = ba.nUnits > 0 ? launchStream.template operator()<true>() : launchStream.template operator()<false>();
             if (rc != 0) return rc;
             if (byBlocks && sumLongRows(stream) != cudaSuccess) return (int)cudaErrorLaunchFailure;
         }
