@@ -2393,12 +2393,21 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
             auto go = [&](auto kernel) { err = b200sp::LaunchChained(kernel, (unsigned)grid, kThreads, 0, st, a); };
             auto pick = [&]<bool kKahan, bool kOrdered>() {
                 if (cPlain) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kPlain, kOrdered>);
-                if constexpr (!kInt8) {
-                    const bool adds = s->beta_dev != nullptr || s->beta_f != 0.0f;
+                // Kernels that read C in eights, where beta may be other than 0: into a column-major C only if hardly any of a tile's columns lie past
+                // the last one, or rows are long; these take part in every batch.  Time without them by time with them, 100,000 to 900,000 rows of 2 to
+                // 60, beta = 0.5: row-major N = 3 to 203 0.95 to 1.44, two thirds above 1.05; column-major fp16 / fp32, N = 5 0.89 to 1.13 / 0.88 to
+                // 1.02, 24 0.93 to 1.02 / 0.97 to 1.16, 33 0.85 to 1.08 / 0.90 to 1.03, 60 0.97 to 1.18 / 1.03 to 1.23, 72 0.86 to 1.05 / 0.97 to 1.05, 100
+                // 0.93 to 1.06 / 0.99 to 1.17, 128 0.98 to 1.17 / 1.02 to 1.27, 200 0.98 to 1.22 / 1.01 to 1.20.  Compensated sums lose up to 5 %
+                // and gain up to 10: not worth the kernels.
+                if constexpr (!kInt8 && !kKahan) {
+                    const long long tileCols = kLanes * (16 / (int)sizeof(ValT)), padded = (sh->n + tileCols - 1) / tileCols * tileCols;
+                    const bool adds = (s->beta_dev != nullptr || s->beta_f != 0.0f) &&
+                                      (sh->order_c == 0 || 16 * sh->n >= 15 * padded || sh->n * (long long)sizeof(ValT) >= 384);
                     if (words && adds) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyCWordsAdd, kOrdered>);
-                    if (words) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyCWords, kOrdered>);
-                    if (adds) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyCAdd, kOrdered>);
+                    if (!words && adds) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyCAdd, kOrdered>);
                 }
+                if constexpr (!kInt8)
+                    if (words) return go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyCWords, kOrdered>);
                 go(SpmmFastKernel<ValT, OutT, kKahan, kLanes, kAnyC, kOrdered>);
             };
             auto pickOrder = [&]<bool kKahan>() {

@@ -41,3 +41,9 @@ def test_layouts_and_scalars(handle, device, oracle, m, n, vt, ot):
             handle.set_pointer_mode_device(False)
         got = helpers.to_host(dC.values, ot).reshape((m, n) if order == "row" else (n, m))
         assert np.array_equal((got if order == "row" else flip(got)).view(np.uint8), want.view(np.uint8)), (order, b)
+
+
+@pytest.mark.parametrize("vt,ot", [("f32", "f32"), ("f16", "f16"), ("bf16", "f32")])
+@pytest.mark.parametrize("n", [59, 60, 95, 96, 119, 120, 191, 192])  # fifteen sixteenths of a tile's columns; rows of 384 bytes
+def test_either_side_of_the_rule(handle, device, oracle, n, vt, ot):
+    test_layouts_and_scalars(handle, device, oracle, 9001, n, vt, ot)
