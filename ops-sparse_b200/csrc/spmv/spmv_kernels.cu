@@ -47,6 +47,7 @@
 // values and x are widened to the compute type before the multiply, sums are kept in the
 // compute type, the result is alpha*sum + beta*y rounded once to the output type.
 // beta == 0 never reads y.
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdint>
@@ -1501,6 +1502,11 @@ __global__ void __launch_bounds__(32 * kTransWarps, 5) SpmvTransScatterKernel(co
 // clock and SM; 4000 columns 331 and 46, 16,000 193 and 46, 48,000 129 and 52.  (Adding up the parts of 2, 4 or 8 CTAs of a cluster before
 // they go to y: the same for 2, 2 to 18 % slower for more, as not all SMs are in a cluster.)
 constexpr int kTransBlockWarps = 32;
+// Few entries are spread over more CTAs than they would fill, as long as these have no more than so many columns between them to add to y: an address of
+// shared memory takes an addition per 26 ns.  85,000 entries, half of them in one column, us straight to y, with full CTAs, spread by 16 K and 64 K
+// columns: 30 columns 73, 108, 19 and 19, 395 69, 105, 38 and 20; evenly drawn 21, 14, 7.8 and 7.5, and 17.6, 8.4, 6.9 and 7.1; 30,000 on 30
+// columns 28, 107, 12 and 12, evenly 9.8, 15, 7.2 and 7.0; 200,000 on 1000 158, 107, 106 and 43, evenly 19, 8.5, 8.4 and 7.2.
+constexpr long long kTransSpread = 64 << 10;
 constexpr int kTransBlockCols = 48 << 10;  // what fits beside the warps' marks and factors
 template <typename CompT, typename ValT, typename AccT>
 __global__ void __launch_bounds__(32 * kTransBlockWarps, 1) SpmvTransBlockKernel(const int32_t *__restrict__ rowPtr,
@@ -1517,7 +1523,7 @@ __global__ void __launch_bounds__(32 * kTransBlockWarps, 1) SpmvTransBlockKernel
     __syncthreads();
     b200sp::WaitForPrevious();
     const int warp = threadIdx.x >> 5;
-    const long long c0 = ((long long)blockIdx.x * kTransBlockWarps + warp) * chunksPerWarp * kTransChunk;
+    const long long c0 = ((long long)warp * gridDim.x + blockIdx.x) * chunksPerWarp * kTransChunk;
     TransChunks<CompT, ValT, AccT, kTransChunk>(rowPtr, colInd, val, x, rows, nnz, c0, chunksPerWarp, sc.Alpha(), sBits[warp],
                                                 sFactor[warp], [&](int c, AccT term) {
                                                     if (c < cols) atomicAdd(sY + c, term);
@@ -1858,9 +1864,11 @@ cudaError_t LaunchTransBlock(const int32_t *rowPtr, const int32_t *colInd, const
         if (e != cudaSuccess) return e;
         configured[dev].store(true, std::memory_order_relaxed);
     }
-    const long long chunks = ((long long)nnz + kTransChunk - 1) / kTransChunk, warps = (long long)kTransBlockWarps * b200sp_sm_count();
-    const long long perWarp = (chunks + warps - 1) / warps, perCta = perWarp * kTransBlockWarps;
-    return b200sp::LaunchChained(SpmvTransBlockKernel<CompT, ValT, AccT>, (unsigned)((chunks + perCta - 1) / perCta), 32 * kTransBlockWarps,
+    const long long chunks = ((long long)nnz + kTransChunk - 1) / kTransChunk;
+    const long long full = (chunks + kTransBlockWarps - 1) / kTransBlockWarps, apart = kTransSpread / cols;
+    const long long ctas = std::min<long long>(b200sp_sm_count(), std::max(full, std::min(chunks, apart)));
+    const long long perWarp = (chunks + kTransBlockWarps * ctas - 1) / (kTransBlockWarps * ctas);
+    return b200sp::LaunchChained(SpmvTransBlockKernel<CompT, ValT, AccT>, (unsigned)ctas, 32 * kTransBlockWarps,
                                  (size_t)cols * sizeof(AccT), stream, rowPtr, colInd, val, x, acc, rows, cols, nnz, (int)perWarp, sc);
 }
 

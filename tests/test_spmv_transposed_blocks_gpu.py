@@ -46,3 +46,26 @@ def test_few_columns(handle, device, cols, nnz, vt, ot):
     count = torch.bincount(ci.long(), minlength=cols).double()
     bound = (count + 3) * 2.0 ** -24 * scale + (2.0 ** -8 * want.abs() if ot == "bf16" else 0)
     assert bool(((dy.values.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("vt,ot", [("f32", "f32"), ("i32", "i32")])
+@pytest.mark.parametrize("cols", [1, 30, 395, 1000])
+@pytest.mark.parametrize("nnz", [30_011, 65_536, 65_537, 200_003, 600_007])  # CTAs with one chunk, with a chunk for every warp, and between
+def test_columns_that_many_entries_share(handle, device, cols, nnz, vt, ot):
+    from ops_sparse_b200 import ACL_SPARSE_OP_TRANSPOSE, api
+    gen = torch.Generator(device=device).manual_seed(nnz + cols)
+    m = (nnz + 9) // 10
+    rp = torch.arange(m + 1, device=device).mul_(10).clamp_max_(nnz).to(torch.int32)
+    ci = torch.randint(cols, (nnz,), generator=gen, device=device, dtype=torch.int32)
+    ci[torch.rand(nnz, generator=gen, device=device) < 0.5] = cols // 2
+    draw = lambda n: torch.randint(-9, 10, (n,), generator=gen, device=device, dtype=torch.int32).to(helpers.TORCH_OF[vt])  # sums below 2^24: exact
+    val, x, y = draw(nnz), draw(m), draw(cols)
+    rows = torch.arange(nnz, device=device) // 10
+    want = (-y.to(torch.int64)).index_add(0, ci.long(), 2 * val.to(torch.int64) * x.to(torch.int64)[rows])
+    A = api.CsrMatrix(rp, ci, val, m, cols)
+    dx, dy = api.DnVec(x), api.DnVec(y.clone())
+    buf = api.spmv_preprocess(handle, A, dx, dy, ACL_SPARSE_OP_TRANSPOSE)
+    api.spmv(handle, A, dx, dy, 2, -1, op=ACL_SPARSE_OP_TRANSPOSE, buffer=buf)
+    torch.cuda.synchronize()
+    assert int(want.abs().max()) < 1 << 23
+    assert torch.equal(dy.values.long(), want)
