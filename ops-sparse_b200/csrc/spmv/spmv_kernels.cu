@@ -1618,10 +1618,12 @@ enum { kPlanTiles = 0, kPlanBinned = 1, kPlanBinnedBlocked = 2 };  // blocked: l
 // How SpmvLongBlockKernel shares out the long rows: groups of them, a CTA for each on every block of x (one CTA per SM at
 // most: it holds half of the SM's threads and a block of x), and lanes per piece.  With many blocks the groups are
 // few and large, and eight lanes per piece keep 128 pieces going; with few blocks a group is a handful of rows, whose pieces are
-// long, and more lanes share a piece.  Estimated per trip: about a microsecond (two where its warps meet), and a round trip to memory per eight entries
-// of a lane, for the longest rows in the first trip (they are ordered) and the average in the others.  600,000 power-law rows, us with 8
-// and 32 lanes: 100,000 columns (4 blocks) 87 and 55, 250,000 (8) 51 and 53, 1 M (32) 55 and 74; 765,345 rows, one block, 5,000 long rows: 59
-// with eight lanes and 40 groups, 40 with 32; 25,544 rows of mean 26: 40 and 10.
+// long, and more lanes share a piece.  Estimated in us per trip: a fixed part, more where its warps meet, and a round trip to memory per eight entries of
+// a lane, for the longest rows in the first trip (they are ordered) and the average in the others.  All that is done before the other rows are,
+// which run beside, is early enough: then the fewest lanes, whose CTAs are the fewest.  600,000 power-law rows, us with 8 and 32 lanes: 100,000 columns (4
+// blocks) 87 and 55, 250,000 (8) 51 and 53, 1 M (32) 55 and 74; 86,660 rows, 137,378 columns (5), 433 long rows of up to 68,689, 8, 32 and 256 lanes 109, 36
+// and 21; 583,532 rows of 38 on 29,971 columns (1), 780 long rows, 173, 65 and 82; 25,544 rows of mean 26, one block: 40 with 8, 10 with 32.  Of 250
+// power-law matrices the choice is within 3 % of the best for 238, and at worst 5 % slower than by the number of blocks alone (3.1 times as fast at best).
 int LongBlockGroups(int xBlocks, int nLong, int lanes)
 {
     int groups = b200sp_sm_count() / xBlocks;
@@ -1629,15 +1631,16 @@ int LongBlockGroups(int xBlocks, int nLong, int lanes)
     const int slots = kLongBlockThreads / lanes, useful = (nLong + slots - 1) / slots;
     return groups < useful ? groups : useful;
 }
-int LongBlockLanes(int xBlocks, int nLong, long long longNnz, int longest)
+int LongBlockLanes(int xBlocks, int nLong, long long nnz, long long longNnz, int longest)
 {
     int best = 8;
     double least = 1e30;
+    const double others = 4e-6 * (double)(nnz - longNnz);
     for (int lanes : {8, 32, 256}) {
         const int slots = kLongBlockThreads / lanes, groups = LongBlockGroups(xBlocks, nLong, lanes);
         const int trips = ((nLong + groups - 1) / groups + slots - 1) / slots;
-        auto trip = [&](double entries) { return (lanes > 32 ? 2.0 : 1.0) + 0.6 * ceil(entries / xBlocks / (8.0 * lanes)); };
-        const double cost = trip(longest) + (trips - 1) * trip((double)longNnz / nLong);
+        auto trip = [&](double entries) { return (lanes > 32 ? 3.0 : 1.0) + 0.7 * ceil(entries / xBlocks / (8.0 * lanes)); };
+        const double cost = std::max(others, trip(longest) + (trips - 1) * trip((double)longNnz / nLong));
         if (cost < least) {
             least = cost;
             best = lanes;
@@ -2059,7 +2062,7 @@ int b200sp_spmv_analyze(const int32_t *row_ptr, const int32_t *col_ind, int64_t 
     plan_info[kInfoXBlocks] = useBlocked ? L.xBlocks : 0;
     plan_info[kInfoBlockElems] = useBlocked ? kXBlockElems : host.nearPairs * 4ll > host.pairs * 3ll ? host.longestShort : 0;
     plan_info[kInfoLongLen] = kLongLen;
-    plan_info[kInfoSegments] = useBlocked ? LongBlockLanes(L.xBlocks, host.longs, (long long)host.longNnz, host.longestLong) : host.segments;
+    plan_info[kInfoSegments] = useBlocked ? LongBlockLanes(L.xBlocks, host.longs, nnz, (long long)host.longNnz, host.longestLong) : host.segments;
     plan_info[kInfoMedium] = host.medium;
     plan_info[kInfoLong] = host.longs;
 #ifdef B200SP_SPMV_FORCE_SHORT_G
