@@ -317,11 +317,12 @@ class Env:
     pass
 
 
-def kernels_of(is_spmm: bool, launches_per_step: float, b_row_bytes: int, world: int, plan=(0, 0, 0, 0)) -> str:
-    """The kernels one step launches, as the library's routing rules give them (`plan`: b200spSpMMPlanInfo)."""
+def kernels_of(is_spmm: bool, launches_per_step: float, world: int, plan=(0, 0, 0, 0), stream=False) -> str:
+    """The kernels one step launches, as the library's routing rules give them (`plan`: b200spSpMMPlanInfo, `stream`:
+    b200spSpMMToRowStream)."""
     if is_spmm:
         if plan[1] > 0:
-            if b_row_bytes in (512, 1024):
+            if stream:
                 return ("SpmmRowStreamKernel (rows, and units of rows > 1024 nnz, block by block of B through L2) + "
                         "SpmmLongSumKernel")
             long_rows = " + SpmmLongBlockKernel + SpmmLongSumKernel (rows > 1024 nnz, block by block of B through L2, side stream)"
@@ -329,7 +330,7 @@ def kernels_of(is_spmm: bool, launches_per_step: float, b_row_bytes: int, world:
             long_rows = " + SpmmFastKernel (units of rows > 1024 nnz, side stream)"
         else:
             long_rows = ""
-        if b_row_bytes in (512, 1024):
+        if stream:
             return "SpmmRowStreamKernel" + long_rows
         return "SpmmFastKernel" + (long_rows if plan[1] > 0 else "")
     if launches_per_step >= 2 + (world > 1):
@@ -544,10 +545,11 @@ def measure_config(name: str, args, env, head: bool) -> dict:
         base = cpu_baseline(cfg, oracle, oracle.hardware_threads())
 
     lps = launches / K
-    plan = (ctypes.c_int32 * 4)()
+    plan, stream_on = (ctypes.c_int32 * 4)(), ctypes.c_int32()
     if is_spmm:
         L.b200spSpMMPlanInfo(op.A.raw, plan)
-    kernels = kernels_of(is_spmm, lps, n * dense.element_size() if is_spmm else 0, world, tuple(plan))
+        L.b200spSpMMToRowStream(op.A.raw, ctypes.byref(stream_on))
+    kernels = kernels_of(is_spmm, lps, world, tuple(plan), bool(stream_on.value))
     traffic = NCU_TRAFFIC.get(name) if world == 1 else None
     if traffic is not None and any(k not in kernels for k in traffic["kernels"].split(" + ")):
         traffic = None

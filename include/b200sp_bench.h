@@ -30,6 +30,8 @@ aclsparseStatus_t b200spRepeatSpMM(aclsparseHandle_t handle, aclsparseOperation_
 /* What aclsparseSpMMPreprocess recorded for matA: info = {long-row segments, units of the column-block path
  * (0 = the long rows are summed by segments), long rows, 1 if a plan is recorded}. */
 aclsparseStatus_t b200spSpMMPlanInfo(aclsparseConstSpMatDescr_t matA, int32_t info[4]);
+/* *on = 1 if a product with this plan, with B and C in 16-byte aligned rows, gives its rows to the row-stream kernel. */
+aclsparseStatus_t b200spSpMMToRowStream(aclsparseConstSpMatDescr_t matA, int32_t *on);
 
 /* Row-sharded operator on several GPUs: `reps` steps, step i = b200spMgPush of this rank's slice (`slice`,
  * `offset`, `bytes` as for b200spMgPush) with sequence number firstSeq + i into replica (firstSeq + i) % replicas,

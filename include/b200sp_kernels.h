@@ -209,6 +209,8 @@ int b200sp_spmm_copies(const b200spSpmmShape *shape, int val_type, int32_t segme
 /* The same for b200sp_spmm_launch_found, which may write A out as well. */
 int b200sp_spmm_copies_found(const b200spSpmmShape *shape, const b200spSpmmFound *found, int val_type, int32_t segments,
                              const void *plan);
+/* 1 if the row-stream kernel takes the rows of up to 1024 entries of this product, its B and C being in 16-byte aligned rows. */
+int b200sp_spmm_to_row_stream(const b200spSpmmShape *shape, int val_type, int32_t segments);
 
 /* Analysis pass: finds rows too long for one warp, cuts them into segments and writes
  * the segment table into `plan`, and lists the rows that are better summed apart from

@@ -299,4 +299,18 @@ aclsparseStatus_t b200spSpMMPlanInfo(aclsparseConstSpMatDescr_t matA, int32_t in
     return ACL_SPARSE_STATUS_SUCCESS;
 }
 
+aclsparseStatus_t b200spSpMMToRowStream(aclsparseConstSpMatDescr_t matA, int32_t *on)
+{
+    if (matA == nullptr || on == nullptr) return ACL_SPARSE_STATUS_INVALID_VALUE;
+    const auto &p = matA->active;
+    b200spSpmmShape sh{};
+    sh.m = p.rows;
+    sh.k = matA->cols;
+    sh.n = p.n;
+    sh.nnz = p.nnz;
+    sh.mid_units = p.midUnits;
+    *on = p.kind == PlanKind::kSpmm ? b200sp_spmm_to_row_stream(&sh, b200sp::KernelTypeOf(matA->valueType), p.segments) : 0;
+    return ACL_SPARSE_STATUS_SUCCESS;
+}
+
 }  // extern "C"

@@ -2014,6 +2014,10 @@ bool StreamPays(const b200spSpmmShape *sh, int32_t segments, int64_t rowBytes)
     if (sh->mid_units + (int64_t)segments > sh->m / 1000) return sh->m >= kStreamMinSkewed;
     return sh->k * rowBytes >= kBlockMinB || sh->nnz < kStreamMaxMean * sh->m;
 }
+bool ToRowStream(const b200spSpmmShape *sh, int32_t segments, int64_t rowBytes)  // of B and C in 16-byte aligned rows, not int8
+{
+    return !sh->kahan && (rowBytes == 512 || rowBytes == 1024) && StreamPays(sh, segments, rowBytes);
+}
 
 // The copy engine of an SM starts about one row copy per 20 clocks (measured: 16.8 M copies of
 // 256 bytes took 1.25 ms on 148 SMs), so rows shorter than 512 bytes move faster through plain
@@ -2454,7 +2458,7 @@ int LaunchTyped(const int32_t *rowPtr, const int32_t *colInd, const void *val, c
         // B rows of 512 / 1024 bytes: rows of up to kLongRow entries go to the row-stream kernel,
         // and SpmmFastKernel is launched for its segment CTAs only.
         const long long rowBytes = sh->n * (long long)sizeof(ValT);
-        const bool stream_ = !sh->kahan && (rowBytes == 512 || rowBytes == 1024) && StreamPays(sh, segments, rowBytes);
+        const bool stream_ = ToRowStream(sh, segments, rowBytes);
         // Long rows by column blocks of B (found applicable by b200sp_spmm_analyze_blocks) instead of by segments.
         const bool byBlocks = sh->block_units > 0 && sh->long_rows > 0 && !sh->kahan && rowBytes >= kBlockMinRowBytes &&
                               sh->block_units <= L.capBlockSlots;
@@ -2558,6 +2562,12 @@ void b200sp_spmm_stream_wait_test(long long wait_cycles, unsigned extra_tx)
 {
     gHostStreamWaitCycles = wait_cycles > 0 ? wait_cycles : kStreamWaitCycles;
     gHostStreamExtraTx = extra_tx;
+}
+
+int b200sp_spmm_to_row_stream(const b200spSpmmShape *shape, int val_type, int32_t segments)
+{
+    const int bytes = val_type == B200SP_F32 ? 4 : 2;
+    return shape != nullptr && val_type != B200SP_I8 && ToRowStream(shape, segments, shape->n * bytes) ? 1 : 0;
 }
 
 size_t b200sp_spmm_plan_bytes(int64_t rows, int64_t nnz, int64_t n) { return LayoutFor(rows, nnz, n).total; }
