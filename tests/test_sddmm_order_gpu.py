@@ -223,3 +223,42 @@ def test_threads(pkg, handle, device):
     assert not failed
     assert torch.equal(case.C.values, zero)
     assert not torch.equal(zero, plain)
+
+
+@pytest.mark.parametrize("cols", [0, 5000])
+@pytest.mark.parametrize("dtype", ["f16", "f32"])
+@pytest.mark.parametrize("x,y", [("row", "row"), ("turned", "row"), ("row", "turned"), ("turned", "turned"), ("other", "row")])
+def test_layouts_leading_dimensions_and_device_scalars(pkg, handle, device, dtype, x, y, cols):
+    """The operands as stored rows, as columns of a turned matrix (the same memory), and an X whose rows do not lie together."""
+    from ops_sparse_b200 import api
+    case = Case(pkg, handle, device, dtype, 128, cols=cols)
+    k, tdt, keep, scalars = case.k, case.X.dtype, [], []
+
+    def operand(a, how, pad):
+        rows = a.shape[0]
+        store = torch.full((rows, k + pad), float("nan"), dtype=tdt, device=device)
+        store[:, :k] = a
+        if how == "other":
+            store = a.t().contiguous()
+            mat = api.DnMat(store, rows, k, rows, "col")
+        else:
+            mat = api.DnMat(store, rows, k, k + pad, "row") if how == "row" else api.DnMat(store, k, rows, k + pad, "col")
+        keep.append((store, mat))
+        return mat
+    X, Y = operand(case.X, x, 8), operand(case.Y, y, 16)
+    opx = pkg.ACL_SPARSE_OP_TRANSPOSE if x == "turned" else pkg.ACL_SPARSE_OP_NON_TRANSPOSE
+    opy = pkg.ACL_SPARSE_OP_NON_TRANSPOSE if y == "turned" else pkg.ACL_SPARSE_OP_TRANSPOSE
+    plain_args = case.args
+    case.args = (handle.raw, opx, opy, plain_args[3], X.raw, Y.raw, *plain_args[6:])
+    plain = case.product(torch.empty(256, dtype=torch.uint8, device=device))
+    case.check(plain)
+    buf = case.buffer()
+    case.preprocess(buf)
+    assert torch.equal(case.product(buf), plain)
+    scalars = [torch.tensor([v], dtype=tdt, device=device) for v in (0.75, -0.5)]
+    case.args = (*case.args[:3], c_void_p(scalars[0].data_ptr()), *case.args[4:6], c_void_p(scalars[1].data_ptr()), *case.args[7:])
+    handle.set_pointer_mode_device(True)
+    try:
+        assert torch.equal(case.product(buf), plain)
+    finally:
+        handle.set_pointer_mode_device(False)
