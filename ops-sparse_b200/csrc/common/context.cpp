@@ -31,12 +31,12 @@ std::unordered_map<const void *, BufferNote> gBuffers;
 uint64_t gNextGeneration = 0;
 }  // namespace
 
-uint64_t NoteBufferWrite(const void *buffer)
+uint64_t NoteBufferWrite(const void *buffer, bool byOwner)
 {
     if (buffer == nullptr) return 0;
     std::lock_guard<std::mutex> lock(gGenerationMutex);
     BufferNote &note = gBuffers[buffer];
-    note.plan.reset();
+    if (!byOwner) note.plan.reset();
     return note.generation = ++gNextGeneration;
 }
 

@@ -87,11 +87,11 @@ struct TileOrderPlan {
 // generation; a recorded plan is valid only while its generation is still the buffer's current one.  Without it
 // a stale plan would be trusted after its bytes were overwritten: Preprocess(A, buf), then a call that re-analyses
 // into buf for another operation or another matrix, then a compute call on A with buf.
-uint64_t NoteBufferWrite(const void *buffer);   // returns the new generation (never 0)
+uint64_t NoteBufferWrite(const void *buffer, bool byOwner = false);   // returns the new generation (never 0)
 uint64_t BufferGeneration(const void *buffer);  // 0 = no library call has written this buffer
 
-// A buffer that holds what a descriptor needs: from HoldPlan on, as long as a copy of what it returned exists and nothing else is noted to have
-// written the buffer.  A call that can do without its buffer (SDDMM's preprocessing) leaves such a one alone.
+// A buffer that holds what a descriptor needs: from HoldPlan on, as long as a copy of what it returned exists and nothing else (than a product that
+// writes its own descriptor's buffer, `byOwner`) is noted to have written the buffer.  A call that can do without its buffer (SDDMM's preprocessing) leaves such a one alone.
 std::shared_ptr<const void> HoldPlan(const void *buffer);  // nullptr without memory for the note
 bool HoldsPlan(const void *buffer);
 

@@ -204,6 +204,7 @@ aclsparseStatus_t aclsparseSpMVPreprocess(aclsparseHandle_t handle, aclsparseOpe
         t.rows = matA->rows;
         t.nnz = matA->nnz;
         t.spmvInfo[0] = kTransPlan;
+        t.held = b200sp::HoldPlan(externalBuffer);  // a record that another call made stale would no longer refuse a plain product
         matA->active = t;
         return ACL_SPARSE_STATUS_SUCCESS;
     }
@@ -257,7 +258,7 @@ aclsparseStatus_t aclsparseSpMV(aclsparseHandle_t handle, aclsparseOperation_t o
         // host-side knowledge only, so it survives.)
         const bool mine = PlanMatches(matA->active, externalBuffer, matA) && matA->active.spmvInfo[0] == kTransPlan;
         if (scratch == externalBuffer && scratchBytes > 0) {
-            const uint64_t gen = b200sp::NoteBufferWrite(externalBuffer);
+            const uint64_t gen = b200sp::NoteBufferWrite(externalBuffer, mine);
             if (mine) matA->active.generation = gen;
         }
         rc = b200sp_spmv_trans_launch(rowPtr, colInd, matA->values, vecX->values, vecY->values, matA->rows,

@@ -175,6 +175,30 @@ def test_sddmm_order_written_over_by_others(pkg, handle, device, cols, kind):
         buf.copy_(kept)
 
 
+@pytest.mark.parametrize("dtype", ["f32", "f16"])  # a y of 16 bits accumulates in the buffer
+def test_sddmm_leaves_the_buffer_of_a_transposed_product_alone(pkg, handle, device, dtype):
+    """What was preprocessed for the transposed product, and may be 256 bytes, stays refused for the plain one."""
+    from ops_sparse_b200 import api
+    case = Case(pkg, handle, device, "f16", 128, nnz=300_000, cols=5000)
+    tdt = torch.float16 if dtype == "f16" else torch.float32
+    A = api.CsrMatrix(case.row_ptr, case.col_ind, torch.rand(case.nnz, device=device).to(tdt), case.m, case.cols)
+    x, y = (api.DnVec(torch.rand(s, device=device).to(tdt)) for s in (case.m, case.cols))
+    buf, L, null, T = case.buffer(), pkg.lib(), c_void_p(), pkg.ACL_SPARSE_OP_TRANSPOSE
+    assert buf.numel() >= 4 * case.cols
+    pkg.check(L.aclsparseSpMVPreprocess(handle.raw, T, null, A.raw, x.raw, null, y.raw, pkg.ACL_FLOAT, 0, at(buf)), "plan")
+    a, b = c_float(1.0), c_float(0.0)
+    scalars = c_void_p(addressof(a)), c_void_p(addressof(b))
+    for _ in range(2):  # the second time after a product
+        torch.cuda.synchronize()
+        kept = buf.clone()
+        case.preprocess(buf)
+        torch.cuda.synchronize()
+        assert torch.equal(buf, kept)
+        status = L.aclsparseSpMV(handle.raw, 0, scalars[0], A.raw, y.raw, scalars[1], x.raw, pkg.ACL_FLOAT, 0, at(buf))
+        assert status == pkg.ACL_SPARSE_STATUS_INVALID_VALUE
+        pkg.check(L.aclsparseSpMV(handle.raw, T, scalars[0], A.raw, x.raw, scalars[1], y.raw, pkg.ACL_FLOAT, 0, at(buf)), "product")
+
+
 @pytest.mark.parametrize("kind", ["spmv", "spmm", "spmvop"])
 def test_sddmm_leaves_the_plans_of_others_alone(pkg, handle, device, kind):
     from ops_sparse_b200 import api
