@@ -289,7 +289,7 @@ NCU_TRAFFIC = {
     "c2": {"bytes": 282_700_000, "kernels": "SpmvLongBlockKernel + SpmvMediumShortKernel",
            "source": "profiles/kernels_of_the_cases.md"},
     "c4": {"bytes": 606_900_000, "kernels": "SpmmFastKernel", "source": "profiles/kernels_of_the_cases.md"},
-    "c5": {"bytes": 13_460_000_000, "kernels": "SpmmRowStreamKernel + SpmmLongSumKernel",
+    "c5": {"bytes": 13_000_000_000, "kernels": "SpmmRowStreamKernel + SpmmLongSumKernel",
            "source": "profiles/spmm_rowstream_c5_bf16_n256.md"},
 }
 # What the counters show to be the busy resource where it is not DRAM.
@@ -302,7 +302,7 @@ BOUND_NOTES = {
     "c4": "B (67 MB) is gathered from L2: 4.3 GB move L2->SM per product and that path delivers 18.1-18.4 TB/s "
           "(62-63 B per clock and SM, measured with a pure row-gather probe), so 236 us is the floor of any "
           "formulation that fetches a B row per non-zero",
-    "c5": "B (1.07 GB) exceeds L2: the rows of up to 1024 entries gather their B rows from DRAM (11.6 GB of the 13.5 GB "
+    "c5": "B (1.07 GB) exceeds L2: the rows of up to 1024 entries gather their B rows from DRAM (most of the 13.0 GB "
           "per product); the longer rows (43 % of the non-zeros) gather block by block of B through L2 in the same grid, "
           "so that their latency hides behind the DRAM traffic of the others",
 }

@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(256) SddmmKernel(const int32_t *__restrict__ r
 // fp16 rows that start on odd 2-byte addresses (kBytes = 2) are copied as the 4-byte words that cover them and
 // realigned when they are read from shared memory.
 // Measured (1 M nodes, 16.0 M entries, fp16, k = 256): 1256 us with 32 lanes a row and scalar products, 1157 us as it is here, which is the 7.6 GB
-// of Y rows that come from DRAM at 6.6 TB/s, 881 us with the tiles in an order (see TileOrder): 5.4 GB.  Cutting rows of 64 entries and more into
+// of Y rows that come from DRAM at 6.6 TB/s, 890 us with the tiles in an order (see TileOrder): 5.0 GB.  Cutting rows of 64 entries and more into
 // the pieces that lie in a block of columns cost 1930 us and more: short pieces, and X rows fetched anew for each.
 template <int kBytes> struct Words { using Type = uint32_t; };  // 4, and the words of kBytes = 2
 template <> struct Words<16> { using Type = uint4; };

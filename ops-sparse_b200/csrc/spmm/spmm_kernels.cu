@@ -1372,7 +1372,7 @@ template <> struct FusedRow<__half> {
 // one warp per CTA gives the memory of a finished warp back at once.
 // The rows are bound by DRAM, the units of long rows by the latency of L2.  One kernel after the other (two streams do not
 // help: the first takes every SM until its last CTA has started) they took 2610 us; in one grid, units spread evenly
-// among the rows, 2300, with 13.5 GB of DRAM traffic either way (2070 us at the copy rate).  The entries are looked up 32 at a time,
+// among the rows, 2300; 13.0 GB of DRAM traffic now (1985 us at the copy rate), 13.5 as two.  The entries are looked up 32 at a time,
 // not one batch at a time, which is 120 of those 310 us: issue slots 57 % busy.
 #ifndef B200SP_SPMM_STREAM_BUFFERS
 #define B200SP_SPMM_STREAM_BUFFERS 2
